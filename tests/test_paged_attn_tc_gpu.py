@@ -1,0 +1,141 @@
+"""The tcgen05 attention of the hybrid decoders (grouped heads and latent rows) against plain 64-bit attention, at the sizes
+where its tiles end: groups that do not divide 128 rows, key rows with a 32-wide tail, several passes over the value columns,
+queries kept in tensor memory, split keys, windows and chunks that start inside a page, cache rows that hold NaN."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+D64 = torch.float64
+
+
+def _i32(x):
+    return torch.tensor(x, dtype=torch.int32, device="cuda")
+
+
+def _pages(g, ctxs, shape):
+    """A cache of scattered pages filled with NaN, its block table, and a writer of a sequence's rows."""
+    need = [-(-c // 64) for c in ctxs]
+    perm = torch.randperm(sum(need) + 2, generator=g).tolist()
+    cache = torch.full((len(perm), 64, *shape), float("nan"), dtype=torch.bfloat16)
+    bt = torch.zeros(len(ctxs), max(need), dtype=torch.int32)
+    at = 0
+    for b, n in enumerate(need):
+        bt[b, :n] = torch.tensor(perm[at:at + n])
+        at += n
+
+    def put(c, b, rows):
+        for i in range(0, rows.shape[0], 64):
+            c[int(bt[b, i // 64]), :min(64, rows.shape[0] - i)] = rows[i:i + 64]
+    return cache, bt, put
+
+
+def _want(q, k, v, pos, scale, window, keep, chunk, cap, sink, gate, slopes, table):
+    """(result, sum of weights times |values|): q [n, H, d], k [m, G, d], v [m, Gv, e], pos [n]; 64 bits."""
+    n, H, _ = q.shape
+    m, G, Gv = k.shape[0], k.shape[1], v.shape[1]
+    i, j = pos[:, None], torch.arange(m)[None]
+    lo = (i - window + 1 if window else torch.zeros_like(i)).clamp(min=0)
+    if chunk:
+        lo = torch.maximum(lo, i // chunk * chunk)
+    ok = (j <= i) & ((j >= lo) | (j < keep))
+    out, mag = torch.zeros(n, H, v.shape[2], dtype=D64), torch.zeros(n, H, v.shape[2], dtype=D64)
+    for h in range(H):
+        g = h // (H // G)
+        s = q[:, h] @ k[:, g].T * scale
+        if cap:
+            s = cap * torch.tanh(s / cap)
+        if slopes is not None:
+            s = s - slopes[h] * (i - j)
+        if table is not None:
+            s = s + table[h][(i - j).clamp(0, table.shape[1] - 1)]
+        s = s.masked_fill(~ok, -math.inf)
+        if sink is not None:
+            s = torch.cat([s, sink[h].expand(n, 1)], 1)
+        w = torch.softmax(s, 1)[:, :m]
+        out[:, h], mag[:, h] = w @ v[:, g % Gv], w @ v[:, g % Gv].abs()
+    gt = torch.sigmoid(gate) if gate is not None else torch.ones(n, H, dtype=D64)
+    gt = gt.reshape(n, H, -1)
+    return out * gt, mag * gt
+
+
+def _check(out, want, mag):
+    # weights are rounded to bf16 once (unit roundoff 2^-8 for its 8 significant bits) and the result once more; the fp32 sums
+    # and exponentials of scores up to ~50 add a few 1e-6 of the same sum
+    err = (out.double().cpu() - want).abs()
+    assert torch.isfinite(out).all()
+    assert bool((err <= mag * (2.0 ** -7) * 1.02 + 1e-6).all()), (err / mag.clamp(min=1e-9)).max().item()
+
+
+LENS = [([1], [1]), ([1, 1, 1], [64, 129, 700]), ([5, 1, 70], [5, 65, 333]), ([130, 257], [130, 300])]
+
+
+@pytest.mark.parametrize("lens,ctxs", LENS)
+@pytest.mark.parametrize("H,G,Gv,dk,dv,opt", [
+    (16, 4, 4, 128, 128, dict(window=100, keep=3, cap=9.0, sink=True, gate="head")),
+    (16, 4, 4, 128, 128, dict()),
+    (6, 2, 2, 96, 64, dict(window=64, sink=True, f32=True)),
+    (8, 1, 1, 64, 192, dict(window=1, gate="elem")),
+    (5, 5, 5, 256, 256, dict(chunk=96, slopes=True)),
+    (8, 4, 2, 64, 64, dict(chunk=50, table=40, f32=True)),
+    (40, 1, 1, 160, 320, dict(window=333, keep=70, table=90, cap=20.0)),
+])
+def test_grouped_heads(lib, H, G, Gv, dk, dv, opt, lens, ctxs):
+    from vllm_rs_b200 import ops
+    g = torch.Generator().manual_seed(H * dk + sum(ctxs))
+    kc, bt, put = _pages(g, ctxs, (G, dk))
+    vc = torch.full((kc.shape[0], 64, Gv, dv), float("nan"), dtype=torch.bfloat16)
+    T = sum(lens)
+    q = (torch.randn(T, H, dk, generator=g) * 1.5).bfloat16()
+    f = lambda name, *shape: torch.randn(*shape, generator=g) if opt.get(name) else None      # noqa: E731
+    sink, slopes = f("sink", H), f("slopes", H)
+    slopes = slopes.abs() * 0.02 if slopes is not None else None
+    table = torch.randn(H, opt["table"], generator=g) if opt.get("table") else None
+    gate = {"head": torch.randn(T, H, generator=g), "elem": torch.randn(T, H * dv, generator=g)}.get(opt.get("gate"))
+    scale, window, keep, chunk, cap = dk ** -0.5, opt.get("window", 0), opt.get("keep", 0), opt.get("chunk", 0), opt.get("cap", 0.0)
+    d = lambda t: None if t is None else t.double()                                           # noqa: E731
+    want, mag, at = [], [], 0
+    for b, (n, c) in enumerate(zip(lens, ctxs)):
+        k, v = torch.randn(c, G, dk, generator=g).bfloat16(), torch.randn(c, Gv, dv, generator=g).bfloat16()
+        put(kc, b, k)
+        put(vc, b, v)
+        w, m = _want(q[at:at + n].double(), k.double(), v.double(), torch.arange(c - n, c), scale, window, keep, chunk, cap,
+                     d(sink), None if gate is None else gate[at:at + n].double(), d(slopes), d(table))
+        want.append(w)
+        mag.append(m)
+        at += n
+    cu = _i32([0] + [sum(lens[:i + 1]) for i in range(len(lens))])
+    c_ = lambda t: None if t is None else t.cuda().contiguous()                               # noqa: E731
+    for split in (True, False):
+        out = ops.window_attn(q.float().cuda(), kc.cuda(), vc.cuda(), c_(sink), c_(gate), cu, _i32(ctxs), bt.cuda(), window=window,
+                              keep_first=keep, scale=scale, softcap=cap, split=split, dist_slopes=c_(slopes), chunk=chunk,
+                              out_f32=opt.get("f32", False), dist_bias=c_(table))
+        _check(out, torch.cat(want), torch.cat(mag))
+
+
+@pytest.mark.parametrize("lens,ctxs", LENS + [([420], [420])])
+@pytest.mark.parametrize("H,rank,rot,window", [(16, 256, 32, 100), (32, 512, 32, 0), (24, 512, 64, 129), (20, 320, 32, 64),
+                                               (3, 64, 0, 1), (128, 128, 32, 77), (9, 448, 32, 0)])
+def test_latent_rows(lib, H, rank, rot, window, lens, ctxs):
+    from vllm_rs_b200 import ops
+    g = torch.Generator().manual_seed(H * rank + sum(ctxs))
+    R, T = rank + rot, sum(lens)
+    cache, bt, put = _pages(g, ctxs, (R,))
+    q = (torch.randn(T, H, R, generator=g) * 0.7).bfloat16()
+    sink, gate = torch.randn(H, generator=g), torch.randn(T, H, generator=g)
+    want, mag, at = [], [], 0
+    for b, (n, c) in enumerate(zip(lens, ctxs)):
+        k = torch.randn(c, R, generator=g).bfloat16()
+        put(cache, b, k)
+        k = k.double()[:, None]
+        w, m = _want(q[at:at + n].double(), k, k[..., :rank], torch.arange(c - n, c), 0.1, window, 0, 0, 0.0, sink.double(),
+                     gate[at:at + n].double(), None, None)
+        want.append(w)
+        mag.append(m)
+        at += n
+    cu = _i32([0] + [sum(lens[:i + 1]) for i in range(len(lens))])
+    for split in (True, False):
+        out = ops.latent_attn(q.float().cuda(), cache.cuda(), sink.cuda(), cu, _i32(ctxs), bt.cuda(), kv_rank=rank, rot_dim=rot,
+                              window=window, scale=0.1, split=split, gate=gate.cuda())
+        _check(out, torch.cat(want), torch.cat(mag))

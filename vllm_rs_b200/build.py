@@ -5,8 +5,8 @@
     python -m vllm_rs_b200.build --target hybrid
 
 Output: vllm_rs_b200/libb200_vllm.so (git-ignored).  The `hybrid` target builds
-vllm_rs_b200/libb200_hybrid.so from the sources the fp32-residual hybrid decoders need and nothing else (no tcgen05
-GEMM / attention kernels): what a fresh checkout compiles when it is first asked to serve such a model.
+vllm_rs_b200/libb200_hybrid.so from the sources the fp32-residual hybrid decoders need and nothing else (none of the
+dense decoders' GEMM / attention kernels): what a fresh checkout compiles when it is first asked to serve such a model.
 """
 from __future__ import annotations
 
@@ -35,7 +35,7 @@ NVCC_FLAGS = [
 ] + os.environ.get("B200_NVCC_EXTRA", "").split()   # e.g. -DB200_DEC_TRACE (tools/dec_trace.py)
 
 
-HYBRID_SOURCES = ["runtime.cu", "glue.cu", "sampler.cu", "seq_norms.cu", "latent_attn.cu", "window_attn.cu",
+HYBRID_SOURCES = ["runtime.cu", "glue.cu", "sampler.cu", "seq_norms.cu", "latent_attn.cu", "window_attn.cu", "paged_attn_tc.cu",
                   "linear_recurrence.cu",
                   "moe.cu", "gemm_lib.cu", "host/scheduler.cpp", "host/hybrid_runner.cpp"]
 HYBRID_LIB = PKG / "libb200_hybrid.so"

@@ -26,6 +26,8 @@ void count_launch(int n);
   } while (0)
 
 int sm_count();
+// Device address of a host-visible word that a kernel sets when a wait ran out (read by b200_last_error); NULL: not to be had.
+int* wait_error_flag();
 
 // ---------------------------------------------------------------- programmatic dependent launch
 // Every kernel of the decode step is launched with programmaticStreamSerialization: its
@@ -553,6 +555,22 @@ __device__ __forceinline__ void mbar_wait_bounded(uint64_t* bar, uint32_t parity
   const long long t0 = clock64();
   while (!mbar_try_wait(bar, parity))
     if (clock64() - t0 > 4000000000LL) __trap();     // ~2 s: no legitimate wait is that long
+}
+
+// A wait that gives up: after about a second, or as soon as another wait of the block has given up (`fail`, may be NULL).
+// The caller then leaves its loop; false is returned and *err (host-visible) and *fail are set.
+__device__ __forceinline__ bool mbar_wait_limited(uint64_t* bar, uint32_t parity, volatile int* fail, int* err) {
+  if (mbar_try_wait(bar, parity)) return true;
+  const long long t0 = clock64();
+  while (!mbar_try_wait(bar, parity)) {
+    if (fail && *fail) return false;
+    if (clock64() - t0 > 2000000000LL) {
+      *reinterpret_cast<volatile int*>(err) = 1;
+      if (fail) *fail = 1;
+      return false;
+    }
+  }
+  return true;
 }
 
 }  // namespace b200

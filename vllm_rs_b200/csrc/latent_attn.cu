@@ -27,7 +27,7 @@
 #include <algorithm>
 #include <cstdlib>
 
-#include "seqmix.cuh"
+#include "paged_attn_tc.cuh"
 
 namespace b200 {
 using namespace seqmix;
@@ -501,6 +501,8 @@ static bool launch_latent_attn_mma(void* out, const float* q_full, const void* c
   return true;
 }
 
+// steps of few rows (decoding): the keys of a row are split over several blocks
+static bool few_rows(int T) { return T <= 2 * sm_count() / 4; }
 int latent_attn_splits(int T, int heads, int window) {
   const int nw = heads >= 8 ? 8 : (heads >= 4 ? 4 : (heads >= 2 ? 2 : 1));
   const int blocks = T * ((heads + nw - 1) / nw);
@@ -509,7 +511,8 @@ int latent_attn_splits(int T, int heads, int window) {
   return std::max(1, std::min(n, 16));
 }
 size_t latent_attn_workspace_bytes(int T, int heads, int kv_rank, int window) {
-  const int n = std::max(latent_attn_splits(T, heads, window), latent_attn_mma_splits(T, heads, window));
+  const int n = std::max({latent_attn_splits(T, heads, window), latent_attn_mma_splits(T, heads, window),
+                          few_rows(T) ? attn_tc_splits(T, 1, kv_rank, 1, window, 0) : 1});
   return n == 1 ? 0 : static_cast<size_t>(T) * heads * n * (kv_rank + 2) * 4;
 }
 
@@ -518,9 +521,26 @@ void launch_latent_attn(void* out, const float* q_full, const void* cache, const
                         int max_blocks, int num_seqs, int T, int heads, int kv_rank, int rot_dim, int window, float scale,
                         int dt, void* workspace, cudaStream_t st_) {
   if (T <= 0) return;
-  // steps of many rows in bf16: the tensor-core kernel (small steps keep the split form below)
+  // bf16: the tcgen05 form takes ranks that are multiples of 64 (rows: of 32) and up to 128 heads
+  if (!dt && latent_mma_enabled()) {
+    const int nsplit = few_rows(T) && workspace ? attn_tc_splits(T, 1, kv_rank, 1, window, 0) : 1;
+    float* po = reinterpret_cast<float*>(workspace);
+    const AttnTcProblem p{out, q_full, cache, nullptr, sink, gate, ld_gate, 0, cu, ctx, block_tables, max_blocks, num_seqs, T,
+                          heads, 1, 1, kv_rank + rot_dim, kv_rank, window, 0, 0, scale, 0.f, nullptr, nullptr, 0, 0, nsplit,
+                          po, po ? po + static_cast<size_t>(T) * heads * nsplit * kv_rank : nullptr};
+    if (attn_tc_takes(p)) {
+      launch_attn_tc(p, st_);
+      if (nsplit > 1) {
+        latent_attn_merge_kernel<__nv_bfloat16><<<T * heads, kv_rank >= 256 ? 256 : 128, 0, st_>>>(
+            (__nv_bfloat16*)out, p.part_o, p.part_ml, sink, gate, ld_gate, heads, kv_rank, nsplit);
+        B200_CUDA_LAUNCH_CHECK();
+      }
+      return;
+    }
+  }
+  // other sizes in bf16: mma.sync
   if (!dt && launch_latent_attn_mma(out, q_full, cache, sink, gate, ld_gate, cu, ctx, block_tables, max_blocks, num_seqs, T, heads,
-                                    kv_rank, rot_dim, window, scale, /*hrows=*/T <= 2 * sm_count() / 4, workspace, st_))
+                                    kv_rank, rot_dim, window, scale, /*hrows=*/few_rows(T), workspace, st_))
     return;
   const int R = kv_rank + rot_dim, Rp = R | 1;
   const int nw = heads >= 8 ? 8 : (heads >= 4 ? 4 : (heads >= 2 ? 2 : 1));

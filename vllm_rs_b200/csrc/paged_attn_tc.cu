@@ -1,0 +1,682 @@
+// Softmax attention over paged bf16 caches on tcgen05 tensor cores, for the hybrid decoders: windowed grouped-head
+// attention (window_attn.cu has the list of options) and latent attention (one shared row per token whose first vdim
+// entries are the values).  Queries, scores, softmax and sums are fp32; the operands of both products are bf16.
+//
+// A block owns 128 rows = (128 / group) tokens x the `group` query heads of ONE key head (latent attention: all heads),
+// so that every key page is fetched once for all of them, and walks the pages (64 tokens) that its rows see: first those
+// that hold kept tokens outside the window, then the window.
+//   S  = Q K^T    fp32 [128 x 64] in TMEM.  Q was rounded to bf16 once: in shared memory (SW128, K-major) or, where the key
+//                 rows are so long that Q and the page ring do not fit together, its first q_tm blocks of 64 in TMEM
+//   P  = softmax  thread = row: options and mask on the fp32 scores, lazy running maximum (the accumulator is rescaled
+//                 when the maximum grows by more than 2^8; exact, since the last division uses the same reference),
+//                 bf16 P to TMEM
+//   O += P V      fp32 [128 x up to 256] in TMEM; V = page as an MN-major operand
+// Warp 0 fetches pages by block-table index (TMA, K ring | V ring), warp 1 issues the MMAs (S of page j + 1 before P V of
+// page j), warps 2-5 own the rows.  Latent rows (kv_rank 512: O would need all 512 TMEM columns) are walked in passes of up to
+// 256 value columns; the scores are computed again in every pass (1.5x the products, still far from the 8 mma.sync
+// warps' rate that made 128-row tiles of 16 rows x 1 head re-read every page 64 times).  In a pass the page blocks that are
+// also values stay until P V has read them (V ring), the rest is released after S (K ring).
+//
+// Bound: tensor cores for prompts (per page 2 * 128 * 64 * (dim * passes + vdim) flop against 64 * dim * 2 bytes from L2),
+// HBM for steps of few rows, whose keys are split over blocks; window_attn_merge / latent_attn_merge then finish.
+#include "paged_attn_tc.cuh"
+
+#include <algorithm>
+
+namespace b200 {
+using namespace seqmix;
+namespace hat {
+
+constexpr int kRows = 128, kTok = 64, kThreads = 192;
+constexpr int kBlk = kTok * 128;          // a page's 64 x 64 block: 64 swizzled rows of 128 bytes
+constexpr int kTailBlk = kTok * 64;       // the last 32 columns: 64 rows of 64 bytes
+constexpr int kQBlk = kRows * 128, kQTail = kRows * 64;
+constexpr int kMaxStages = 4;
+constexpr float kLog2e = 1.4426950408889634f, kLn2 = 0.6931471805599453f;
+constexpr float kRescale = 8.f;           // log2 units
+constexpr float kNone = -1e30f;           // a reference maximum before any key was seen
+
+struct Args {
+  AttnTcProblem p;
+  int group, tq;                          // query heads per key head; tokens per block
+  int kblk, tail, vblk, passes, ppc;      // 64-wide blocks of a key row (+ 32-wide tail), of a value row; passes; passes per block
+  int shared, q_tm, sk, sv;               // values inside the key rows; query blocks in TMEM; ring stages
+  int k_stage, v_stage, q_bytes, tmem_cols;
+  int* err;
+};
+
+__device__ __forceinline__ uint64_t desc_mn_sw128(uint32_t saddr) {       // chunks of 64 MN elements 8 KB apart
+  uint64_t d = 0;
+  d |= uint64_t((saddr & 0x3FFFF) >> 4);
+  d |= uint64_t(kBlk >> 4) << 16;
+  d |= uint64_t(1024 >> 4) << 32;
+  d |= uint64_t(1) << 46;
+  d |= uint64_t(2) << 61;
+  return d;
+}
+__device__ __forceinline__ uint64_t desc_k_sw64(uint32_t saddr) {         // rows of 64 bytes, 8-row groups 512 bytes apart
+  uint64_t d = 0;
+  d |= uint64_t((saddr & 0x3FFFF) >> 4);
+  d |= uint64_t(1) << 16;
+  d |= uint64_t(512 >> 4) << 32;
+  d |= uint64_t(1) << 46;
+  d |= uint64_t(4) << 61;
+  return d;
+}
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+      "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
+      "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};" ::"r"(taddr),
+      "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
+      "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]),
+      "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]),
+      "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
+      : "memory");
+}
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float rcp(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ int first_seen(int pos, int window, int chunk) {
+  const int lo = window > 0 ? max(0, pos - window + 1) : 0;
+  return chunk > 0 ? max(lo, pos / chunk * chunk) : lo;
+}
+
+// Ring position: stage and the parity of its current use.
+struct Ring {
+  int s = 0;
+  uint32_t ph = 0;
+  __device__ __forceinline__ void next(int stages) {
+    if (++s == stages) { s = 0; ph ^= 1; }
+  }
+};
+
+// CAP: scores are capped; BIAS: a distance bias (slopes or table) joins them.
+template <bool CAP, bool BIAS>
+__global__ void __launch_bounds__(kThreads, 2)
+attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap tmap,
+               const __grid_constant__ CUtensorMap vmap, const __grid_constant__ Args a) {
+  const AttnTcProblem& p = a.p;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int G = a.group, kvh = blockIdx.y, vh = kvh % p.v_heads;
+  // ---- which tokens: tile (gridDim.x - 1 - blockIdx.x) of the sequences' tiles, so that the latest (longest) go first
+  int b = -1, tile = 0;
+  {
+    const int want = static_cast<int>(gridDim.x - 1 - blockIdx.x);
+    int before = 0;
+    for (int s0 = 0; s0 < p.num_seqs && b < 0; s0 += 32) {
+      const int s = s0 + lane;
+      const int n = s < p.num_seqs ? static_cast<int>(p.cu[s + 1] - p.cu[s]) : 0;
+      const int mine = (n + a.tq - 1) / a.tq;
+      int inc = mine;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += v;
+      }
+      const bool here = want >= before + inc - mine && want < before + inc;
+      const unsigned hit = __ballot_sync(0xffffffffu, here);
+      if (hit) {
+        const int src = __ffs(hit) - 1;
+        b = s0 + src;
+        tile = want - before - __shfl_sync(0xffffffffu, inc - mine, src);
+      }
+      before += __shfl_sync(0xffffffffu, inc, 31);
+    }
+    if (b < 0) return;
+  }
+  const int seq0 = static_cast<int>(p.cu[b]), nq = static_cast<int>(p.cu[b + 1]) - seq0;
+  const int row0 = seq0 + tile * a.tq;                       // first token row
+  const int nt = min(a.tq, nq - tile * a.tq), nrows = nt * G;
+  const int pos0 = static_cast<int>(p.ctx[b]) - nq + tile * a.tq, pos_last = pos0 + nt - 1;
+  const int key_lo = first_seen(pos0, p.window, p.chunk);
+  const int wpage = key_lo / kTok;
+  const int nkept = min(wpage, (min(max(p.keep_first, 0), key_lo) + kTok - 1) / kTok);
+  const int ntiles = nkept + pos_last / kTok - wpage + 1;
+  const int npz = a.passes / a.ppc, sp = blockIdx.z / npz, pass0 = (blockIdx.z % npz) * a.ppc;
+  const int per = (ntiles + p.nsplit - 1) / p.nsplit;
+  const int j0 = sp * per, n = min(ntiles, j0 + per) - j0;   // this block's pages
+  const int vcols = a.vblk * 64;                             // value columns of a pass (the last one may have fewer)
+
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* q_smem = smem;
+  uint8_t* k_smem = q_smem + a.q_bytes;
+  uint8_t* v_smem = k_smem + a.sk * a.k_stage;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(v_smem + a.sv * a.v_stage);
+  uint64_t* k_full = bars;
+  uint64_t* k_empty = k_full + kMaxStages;
+  uint64_t* v_full = k_empty + kMaxStages;
+  uint64_t* v_empty = v_full + kMaxStages;
+  uint64_t* q_full = v_empty + kMaxStages;
+  uint64_t* s_full = q_full + 1;
+  uint64_t* s_free = q_full + 2;
+  uint64_t* p_full = q_full + 3;
+  uint64_t* pv_done = q_full + 4;
+  uint64_t* drained = q_full + 5;
+  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(q_full + 6);
+  volatile int* fail = reinterpret_cast<volatile int*>(tmem_ptr + 1);
+
+  if (n <= 0) {                            // a split without keys leaves an empty part
+    for (int e = threadIdx.x; e < nrows * a.ppc * vcols; e += kThreads) {
+      const int r = e / (a.ppc * vcols), c = pass0 * vcols + e % (a.ppc * vcols);
+      const size_t pi = (static_cast<size_t>(row0 + r / G) * p.heads + kvh * G + r % G) * p.nsplit + sp;
+      if (c < p.vdim) p.part_o[pi * p.vdim + c] = 0.f;
+      if (c == 0) {
+        p.part_ml[pi * 2] = kNone;
+        p.part_ml[pi * 2 + 1] = 0.f;
+      }
+    }
+    return;
+  }
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < a.sk; ++s) { mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 1); }
+    for (int s = 0; s < a.sv; ++s) { mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 1); }
+    mbar_init(q_full, 4);
+    mbar_init(s_full, 1);
+    mbar_init(s_free, 4);
+    mbar_init(p_full, 4);
+    mbar_init(pv_done, 1);
+    mbar_init(drained, 1);
+    *fail = 0;
+    fence_barrier_init();
+    prefetch_tmap(&kmap);
+    prefetch_tmap(&vmap);
+    if (a.tail) prefetch_tmap(&tmap);
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_ptr, a.tmem_cols);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_ptr;
+  const uint32_t o_tm = tmem, s_tm = tmem + vcols, p_tm = s_tm + 64, q_tm = p_tm + 32;
+  const int total = a.ppc * n;
+  // blocks of value columns in pass x, and the first of them
+  auto v_first = [&](int x) { return x * a.vblk; };
+  auto v_count = [&](int x) { return min(a.vblk, p.vdim / 64 - x * a.vblk); };
+  auto page_of = [&](int j) { return j < nkept ? j : wpage + j - nkept; };
+
+  if (warp == 0) {
+    // ------------------------------------------------------------ pages
+    bool ok = true;
+    if (a.q_tm) ok = mbar_wait_limited(q_full, 0, fail, a.err);      // the rings lend their space to the staging of Q
+    const uint32_t* bt = p.block_tables + static_cast<size_t>(b) * p.max_blocks;
+    Ring kr, vr;
+    int armed_k = 0, armed_v = 0;
+    for (int pi = 0; pi < a.ppc && ok; ++pi) {
+      const int vf = v_first(pass0 + pi), vn = v_count(pass0 + pi);
+      for (int base = 0; base < n && ok; base += 32) {
+        const int mine = base + lane < n ? static_cast<int>(bt[page_of(j0 + base + lane)]) : 0;
+        const int cnt = min(32, n - base);
+        for (int jj = 0; jj < cnt && ok; ++jj) {
+          const int page = __shfl_sync(0xffffffffu, mine, jj);
+          if (lane == 0) {
+            ok = mbar_wait_limited(&k_empty[kr.s], kr.ph ^ 1, fail, a.err);
+            if (ok) {
+              uint8_t* dst = k_smem + kr.s * a.k_stage;
+              const int kn = a.shared ? a.kblk - vn : a.kblk;
+              mbar_arrive_expect_tx(&k_full[kr.s], kn * kBlk + a.tail * kTailBlk);
+              for (int i = 0; i < kn; ++i) {
+                const int blk = a.shared && i >= vf ? i + vn : i;
+                tma_load_4d(dst + i * kBlk, &kmap, &k_full[kr.s], blk * 64, kvh, 0, page);
+              }
+              if (a.tail) tma_load_4d(dst + kn * kBlk, &tmap, &k_full[kr.s], a.kblk * 64, kvh, 0, page);
+              ++armed_k;
+              ok = mbar_wait_limited(&v_empty[vr.s], vr.ph ^ 1, fail, a.err);
+            }
+            if (ok) {
+              uint8_t* dst = v_smem + vr.s * a.v_stage;
+              mbar_arrive_expect_tx(&v_full[vr.s], vn * kBlk);
+              for (int i = 0; i < vn; ++i)
+                tma_load_4d(dst + i * kBlk, &vmap, &v_full[vr.s], (vf + i) * 64, vh, 0, page);
+              ++armed_v;
+            }
+            kr.next(a.sk);
+            vr.next(a.sv);
+          }
+          ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+        }
+      }
+    }
+    if (!ok && lane == 0) {                 // copies in flight land before the block ends
+      for (int s = 0; s < a.sk; ++s) {
+        const int uses = (armed_k + a.sk - 1 - s) / a.sk;
+        if (uses > 0) mbar_wait_limited(&k_full[s], (uses - 1) & 1, nullptr, a.err);
+      }
+      for (int s = 0; s < a.sv; ++s) {
+        const int uses = (armed_v + a.sv - 1 - s) / a.sv;
+        if (uses > 0) mbar_wait_limited(&v_full[s], (uses - 1) & 1, nullptr, a.err);
+      }
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------------------ products
+    if (lane == 0) {
+      constexpr uint32_t kBf16 = (1u << 7) | (1u << 10);
+      const uint32_t idesc_s = make_idesc_f16(kRows, kTok) | kBf16;
+      const uint32_t q_addr = smem_u32(q_smem);
+      Ring kr, vr, vr_pv;
+      bool ok = mbar_wait_limited(q_full, 0, fail, a.err);
+      tc_fence_after();
+      auto qk_block = [&](int blk, uint32_t kaddr, uint32_t acc) {
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks) {
+          const uint64_t bd = make_smem_desc_sw128(kaddr + ks * 32);
+          if (blk < a.q_tm)
+            tc_mma_ts(s_tm, q_tm + blk * 32 + ks * 8, bd, idesc_s, (acc | ks) ? 1u : 0u);
+          else
+            tc_mma_ss(s_tm, make_smem_desc_sw128(q_addr + (blk - a.q_tm) * kQBlk + ks * 32), bd, idesc_s, (acc | ks) ? 1u : 0u);
+        }
+      };
+      auto issue_qk = [&](int it) {
+        const int pass = pass0 + it / n, vf = v_first(pass), vn = v_count(pass);
+        ok = ok && mbar_wait_limited(&k_full[kr.s], kr.ph, fail, a.err);
+        if (it > 0) ok = ok && mbar_wait_limited(s_free, (it - 1) & 1, fail, a.err);     // the rows hold S of the page before
+        if (!ok) return;
+        tc_fence_after();
+        const uint32_t kaddr = smem_u32(k_smem + kr.s * a.k_stage);
+        const int kn = a.shared ? a.kblk - vn : a.kblk;
+        uint32_t acc = 0;
+        for (int i = 0; i < kn; ++i, acc = 1) qk_block(a.shared && i >= vf ? i + vn : i, kaddr + i * kBlk, acc);
+        if (a.tail) {
+#pragma unroll
+          for (int ks = 0; ks < 2; ++ks, acc = 1)
+            tc_mma_ss(s_tm, desc_k_sw64(q_addr + (a.kblk - a.q_tm) * kQBlk + ks * 32), desc_k_sw64(kaddr + kn * kBlk + ks * 32),
+                      idesc_s, acc);
+        }
+        if (a.shared) {
+          tc_commit(&k_empty[kr.s]);        // (the blocks of this ring were read by the products so far)
+          ok = mbar_wait_limited(&v_full[vr.s], vr.ph, fail, a.err);
+          if (!ok) return;
+          const uint32_t vaddr = smem_u32(v_smem + vr.s * a.v_stage);
+          for (int i = 0; i < vn; ++i, acc = 1) qk_block(vf + i, vaddr + i * kBlk, acc);
+          vr.next(a.sv);
+        } else {
+          tc_commit(&k_empty[kr.s]);
+        }
+        tc_commit(s_full);
+        kr.next(a.sk);
+      };
+      issue_qk(0);
+      for (int it = 0; it < total && ok; ++it) {
+        if (it + 1 < total) issue_qk(it + 1);
+        ok = ok && mbar_wait_limited(p_full, it & 1, fail, a.err);
+        if (!a.shared) ok = ok && mbar_wait_limited(&v_full[vr_pv.s], vr_pv.ph, fail, a.err);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t vaddr = smem_u32(v_smem + vr_pv.s * a.v_stage);
+        const uint32_t idesc_o = make_idesc_f16(kRows, v_count(pass0 + it / n) * 64) | (1u << 16) | kBf16;     // B is MN-major
+#pragma unroll
+        for (int ks = 0; ks < kTok / 16; ++ks)
+          tc_mma_ts(o_tm, p_tm + ks * 8, desc_mn_sw128(vaddr + ks * 2048), idesc_o, (it % n > 0 || ks > 0) ? 1u : 0u);
+        tc_commit(&v_empty[vr_pv.s]);
+        tc_commit(pv_done);
+        vr_pv.next(a.sv);
+      }
+      if (!ok) {                            // products in flight end before TMEM is given back
+        tc_commit(drained);
+        mbar_wait_limited(drained, 0, nullptr, a.err);
+      }
+    }
+    __syncwarp();
+  } else {
+    // ------------------------------------------------------------ rows
+    const int q4 = warp & 3, r = q4 * 32 + lane;             // row = TMEM lane
+    const int tid = threadIdx.x - 64;
+    const uint32_t lane_base = static_cast<uint32_t>(q4 * 32) << 16;
+    // ---- stage Q as bf16: coalesced 32-byte reads, chunks of 8 entries
+    {
+      const int cpr = p.dim / 8, pitch = a.q_tm * 128 + 16;
+      const int dr = kRows / cpr, dc = kRows % cpr;          // what 128 chunks on are: dr rows and dc chunks
+      int row = tid / cpr, c = tid % cpr;
+      while (row < kRows) {
+        float4 lo[4], hi[4];
+        int rw[4], cc[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          rw[u] = row;
+          cc[u] = c;
+          lo[u] = hi[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (row < nrows) {
+            const int t = row / G;
+            const float4* src = reinterpret_cast<const float4*>(
+                p.q + (static_cast<size_t>(row0 + t) * p.heads + kvh * G + (row - t * G)) * p.dim + c * 8);
+            lo[u] = __ldg(src);
+            hi[u] = __ldg(src + 1);
+          }
+          row += dr;
+          c += dc;
+          if (c >= cpr) { c -= cpr; ++row; }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          if (rw[u] >= kRows) continue;
+          uint4 w;
+          w.x = pack16x2<true>(lo[u].x, lo[u].y);
+          w.y = pack16x2<true>(lo[u].z, lo[u].w);
+          w.z = pack16x2<true>(hi[u].x, hi[u].y);
+          w.w = pack16x2<true>(hi[u].z, hi[u].w);
+          const int blk = cc[u] >> 3, c8 = cc[u] & 7;
+          uint8_t* dst;
+          if (blk < a.q_tm) dst = k_smem + rw[u] * pitch + cc[u] * 16;
+          else if (blk < a.kblk) dst = q_smem + (blk - a.q_tm) * kQBlk + rw[u] * 128 + ((c8 ^ (rw[u] & 7)) << 4);
+          else dst = q_smem + (a.kblk - a.q_tm) * kQBlk + rw[u] * 64 + ((c8 ^ ((rw[u] >> 1) & 3)) << 4);
+          *reinterpret_cast<uint4*>(dst) = w;
+        }
+      }
+      __syncwarp();
+      if (a.q_tm) {
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        for (int blk = 0; blk < a.q_tm; ++blk) {
+          uint32_t w[32];
+          const uint4* src = reinterpret_cast<const uint4*>(k_smem + r * pitch + blk * 128);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const uint4 v = src[i];
+            w[4 * i] = v.x; w[4 * i + 1] = v.y; w[4 * i + 2] = v.z; w[4 * i + 3] = v.w;
+          }
+          tmem_st32(q_tm + lane_base + blk * 32, w);
+        }
+        tc_wait_st();
+        tc_fence_before();
+      }
+      fence_proxy_async();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(q_full);
+    }
+    // ---- this row
+    const int tl = min(r / G, nt - 1), h = kvh * G + (r - (r / G) * G);      // rows past nrows repeat the last token's limits
+    const bool valid = r < nrows;
+    const int pos = pos0 + tl, lo = first_seen(pos, p.window, p.chunk);
+    const int lo_last = first_seen(pos_last, p.window, p.chunk);
+    const bool with_sink = p.sink && p.nsplit == 1;          // split runs add the sink when the parts are merged
+    const float sl = CAP ? p.scale / p.softcap * (2.f * kLog2e) : p.scale * kLog2e;
+    const float cap2 = p.softcap * kLog2e;
+    float slope = 0.f, far_bias = 0.f;
+    const float* table = nullptr;
+    if (BIAS) {
+      slope = (p.slopes && valid) ? p.slopes[h] * kLog2e : 0.f;
+      if (p.dist_bias) {
+        table = p.dist_bias + static_cast<size_t>(valid ? h : kvh * G) * p.dist_n;
+        far_bias = table[p.dist_n - 1] * kLog2e;
+      }
+    }
+    Ring vr;
+    bool ok = true;
+    int it = 0;
+    for (int pi = 0; pi < a.ppc && ok; ++pi) {
+      float m_ref = with_sink && valid ? p.sink[h] * kLog2e : kNone, l = with_sink ? 1.f : 0.f;
+      const int vn = v_count(pass0 + pi);
+      for (int j = 0; j < n; ++j, ++it) {
+        const int base = page_of(j0 + j) * kTok;
+        ok = mbar_wait_limited(s_full, it & 1, fail, a.err);
+        if (__any_sync(0xffffffffu, !ok)) { ok = false; break; }
+        tc_fence_after();
+        float x[kTok];
+        {
+          uint32_t v0[32], v1[32];
+          tmem_ld_x32(s_tm + lane_base, v0);
+          tmem_ld_x32(s_tm + lane_base + 32, v1);
+          tc_wait_ld();
+#pragma unroll
+          for (int i = 0; i < 32; ++i) {
+            x[i] = __uint_as_float(v0[i]);
+            x[32 + i] = __uint_as_float(v1[i]);
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(s_free);
+        // x becomes the score in log2 units (plain scores keep their scale for the exponent's multiply-add)
+        if (CAP) {
+          // cap tanh(s / cap) = cap - 2 cap / (e^(2 s / cap) + 1)
+#pragma unroll
+          for (int i = 0; i < kTok; ++i) x[i] = fmaf(-2.f * cap2, rcp(ex2(x[i] * sl) + 1.f), cap2);
+        }
+        if (BIAS) {
+          if (!CAP) {
+#pragma unroll
+            for (int i = 0; i < kTok; ++i) x[i] *= sl;
+          }
+          const float d0 = static_cast<float>(pos - base);
+          if (table && pos - (base + kTok - 1) < p.dist_n - 1) {
+#pragma unroll
+            for (int i = 0; i < kTok; ++i)
+              x[i] += fmaf(__ldg(table + max(0, min(pos - base - i, p.dist_n - 1))), kLog2e, -slope * (d0 - i));
+          } else {
+#pragma unroll
+            for (int i = 0; i < kTok; ++i) x[i] += far_bias - slope * (d0 - i);
+          }
+        }
+        if (base + kTok - 1 > pos0 || base < lo_last) {       // the diagonal, the window's edge, kept tokens
+#pragma unroll
+          for (int i = 0; i < kTok; ++i) {
+            const int k = base + i;
+            x[i] = (k <= pos && (k >= lo || k < p.keep_first)) ? x[i] : -INFINITY;
+          }
+        }
+        float mx = fmaxf(x[0], x[1]);
+#pragma unroll
+        for (int i = 2; i < kTok; ++i) mx = fmaxf(mx, x[i]);
+        const float mult = (CAP || BIAS) ? 1.f : sl;
+        mx *= mult;
+        float corr = 1.f;
+        bool grow = false;
+        if (mx - m_ref > kRescale) {
+          corr = ex2(m_ref - mx);
+          m_ref = mx;
+          grow = true;
+        }
+        float ps0 = 0.f, ps1 = 0.f;
+        uint32_t pk[32];
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+          const float e0 = ex2(fmaf(x[2 * i], mult, -m_ref)), e1 = ex2(fmaf(x[2 * i + 1], mult, -m_ref));
+          ps0 += e0;
+          ps1 += e1;
+          pk[i] = pack16x2<true>(e0, e1);
+        }
+        l = fmaf(l, corr, ps0 + ps1);
+        // value rows that no row of the block sees (past the last key, before the window) may hold anything: 0 * NaN
+        if (base + kTok - 1 > pos_last || (base < key_lo && base + kTok > p.keep_first)) {
+          ok = mbar_wait_limited(&v_full[vr.s], vr.ph, fail, a.err);
+          if (__any_sync(0xffffffffu, !ok)) { ok = false; break; }
+          uint8_t* vt = v_smem + vr.s * a.v_stage;
+          for (int e = tid; e < kTok * vn * 8; e += 128) {
+            const int row = e / (vn * 8), c = e - row * (vn * 8), k = base + row;
+            if (k > pos_last || (k < key_lo && k >= p.keep_first))
+              *reinterpret_cast<uint4*>(vt + (c >> 3) * kBlk + row * 128 + (c & 7) * 16) = make_uint4(0, 0, 0, 0);
+          }
+          fence_proxy_async();
+        }
+        vr.next(a.sv);
+        if (it > 0) {
+          ok = mbar_wait_limited(pv_done, (it - 1) & 1, fail, a.err);      // P and O are the rows' again
+          if (__any_sync(0xffffffffu, !ok)) { ok = false; break; }
+          tc_fence_after();
+          if (j > 0 && __any_sync(0xffffffffu, grow)) {
+#pragma unroll 1
+            for (int c0 = 0; c0 < vn * 64; c0 += 32) {
+              uint32_t o[32];
+              tmem_ld_x32(o_tm + lane_base + c0, o);
+              tc_wait_ld();
+#pragma unroll
+              for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * corr);
+              tmem_st32(o_tm + lane_base + c0, o);
+            }
+          }
+        }
+        tmem_st32(p_tm + lane_base, pk);
+        tc_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(p_full);
+      }
+      if (!ok) break;
+      ok = mbar_wait_limited(pv_done, (it - 1) & 1, fail, a.err);
+      if (__any_sync(0xffffffffu, !ok)) { ok = false; break; }
+      tc_fence_after();
+      // ---- the pass's columns of this row
+      const size_t trow = static_cast<size_t>(row0 + tl), orow = trow * p.heads + h;
+      const int col0 = v_first(pass0 + pi) * 64;
+      float inv = l > 0.f ? 1.f / l : 0.f;
+      if (p.nsplit == 1 && p.gate && !p.gate_elems && valid) inv *= sigmoid_f(p.gate[trow * p.ld_gate + h]);
+      const float* ge = p.gate && p.gate_elems ? p.gate + trow * p.ld_gate + static_cast<size_t>(h) * p.vdim + col0 : nullptr;
+#pragma unroll 1
+      for (int c0 = 0; c0 < vn * 64; c0 += 32) {
+        uint32_t o[32];
+        tmem_ld_x32(o_tm + lane_base + c0, o);
+        tc_wait_ld();
+        if (valid && p.nsplit > 1) {
+          float* dst = p.part_o + (orow * p.nsplit + sp) * p.vdim + col0 + c0;
+#pragma unroll
+          for (int i = 0; i < 32; i += 4) *reinterpret_cast<uint4*>(dst + i) = make_uint4(o[i], o[i + 1], o[i + 2], o[i + 3]);
+        } else if (valid) {
+          if (ge) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * sigmoid_f(ge[c0 + i]));
+          }
+          if (p.out_f32) {
+            float* dst = reinterpret_cast<float*>(p.out) + orow * p.vdim + col0 + c0;
+#pragma unroll
+            for (int i = 0; i < 32; i += 4)
+              *reinterpret_cast<float4*>(dst + i) = make_float4(__uint_as_float(o[i]) * inv, __uint_as_float(o[i + 1]) * inv,
+                                                                __uint_as_float(o[i + 2]) * inv, __uint_as_float(o[i + 3]) * inv);
+          } else {
+            __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.out) + orow * p.vdim + col0 + c0;
+#pragma unroll
+            for (int i = 0; i < 32; i += 8) {
+              uint4 w;
+              w.x = pack16x2<true>(__uint_as_float(o[i]) * inv, __uint_as_float(o[i + 1]) * inv);
+              w.y = pack16x2<true>(__uint_as_float(o[i + 2]) * inv, __uint_as_float(o[i + 3]) * inv);
+              w.z = pack16x2<true>(__uint_as_float(o[i + 4]) * inv, __uint_as_float(o[i + 5]) * inv);
+              w.w = pack16x2<true>(__uint_as_float(o[i + 6]) * inv, __uint_as_float(o[i + 7]) * inv);
+              *reinterpret_cast<uint4*>(dst + i) = w;
+            }
+          }
+        }
+        __syncwarp();
+      }
+      if (p.nsplit > 1 && valid && col0 == 0) {
+        float* ml = p.part_ml + (orow * p.nsplit + sp) * 2;
+        ml[0] = m_ref * kLn2;
+        ml[1] = l;
+      }
+      tc_fence_before();
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem, a.tmem_cols);
+  }
+}
+
+constexpr int kSmemMax = 227 * 1024, kBarBytes = 256, kAlign = 1024;
+
+// Sizes of one launch; false: the shape does not fit.
+static bool plan(const AttnTcProblem& p, Args& a) {
+  a.p = p;
+  a.shared = p.v_cache == nullptr;
+  a.group = p.heads / p.kv_heads;
+  if (a.group > kRows || p.dim % 32 != 0 || p.dim < 64 || p.vdim % 64 != 0 || p.vdim <= 0) return false;
+  if (a.shared && (p.vdim > p.dim || p.kv_heads != 1)) return false;
+  a.tq = kRows / a.group;
+  a.kblk = p.dim / 64;
+  a.tail = (p.dim % 64) / 32;
+  const int vb = p.vdim / 64;
+  a.passes = (vb + 3) / 4;
+  a.vblk = (vb + a.passes - 1) / a.passes;
+  a.passes = (vb + a.vblk - 1) / a.vblk;
+  const int last = vb - (a.passes - 1) * a.vblk;              // value blocks of the last pass: the most key blocks beside them
+  a.v_stage = a.vblk * kBlk;
+  a.k_stage = (a.shared ? a.kblk - last : a.kblk) * kBlk + a.tail * kTailBlk;
+  const int tm_room = (512 - a.vblk * 64 - 96) / 32;          // query blocks that TMEM can hold
+  // Latent rows want three V stages (a page's value blocks stay until P V, one page after S); queries move to TMEM until
+  // that fits, and with the last one moved two stages have to do.
+  const int want_v = a.shared ? 3 : 2;
+  for (a.sv = want_v; a.sv >= 2; --a.sv)
+    for (a.q_tm = 0; a.q_tm <= (a.shared ? std::min(tm_room, a.kblk) : 0); ++a.q_tm) {
+      a.sk = 2;
+      a.q_bytes = (a.kblk - a.q_tm) * kQBlk + a.tail * kQTail;
+      const int rings = a.sk * a.k_stage + a.sv * a.v_stage;
+      if (a.q_bytes + rings + kBarBytes + kAlign > kSmemMax) continue;
+      if (a.q_tm && kRows * (a.q_tm * 128 + 16) > rings) continue;
+      const int cols = a.vblk * 64 + 96 + a.q_tm * 32;
+      a.tmem_cols = cols <= 128 ? 128 : (cols <= 256 ? 256 : 512);
+      return true;
+    }
+  return false;
+}
+
+static bool page_map(CUtensorMap* m, const void* base, int row, int heads, int box_cols, CUtensorMapSwizzle swz) {
+  // the page count is not known here: block tables hold valid pages only, so the outer extent is left open
+  const uint64_t dims[4] = {static_cast<uint64_t>(row), static_cast<uint64_t>(heads), kTok, 1u << 25};
+  const uint64_t tok = static_cast<uint64_t>(row) * heads * 2;
+  const uint64_t strides[3] = {static_cast<uint64_t>(row) * 2, tok, tok * kTok};
+  const uint32_t box[4] = {static_cast<uint32_t>(box_cols), 1, kTok, 1}, es[4] = {1, 1, 1, 1};
+  return encode_tensor_map(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, es, swz,
+                           CU_TENSOR_MAP_L2_PROMOTION_L2_256B) == CUDA_SUCCESS;
+}
+
+}  // namespace hat
+
+bool attn_tc_takes(const AttnTcProblem& p) {
+  hat::Args a;
+  const uintptr_t ptrs = reinterpret_cast<uintptr_t>(p.q) | reinterpret_cast<uintptr_t>(p.k_cache) |
+                         reinterpret_cast<uintptr_t>(p.v_cache) | reinterpret_cast<uintptr_t>(p.out) |
+                         reinterpret_cast<uintptr_t>(p.part_o);
+  return (ptrs & 15) == 0 && p.scale > 0.f && hat::plan(p, a);
+}
+
+int attn_tc_splits(int T, int kv_heads, int vdim, int shared_kv, int window, int keep_first) {
+  // every row is a tile of its own (one token per sequence), or a few of one sequence share one; a block per pass
+  const int passes = shared_kv ? (vdim + 255) / 256 : 1;
+  const int blocks = T * kv_heads * passes;
+  int n = ((shared_kv ? 1 : 2) * sm_count()) / std::max(1, blocks);
+  if (window > 0) n = std::min(n, (window + std::max(keep_first, 0) + hat::kTok - 1) / hat::kTok + 1);
+  return std::max(1, std::min(n, 16));
+}
+
+void launch_attn_tc(const AttnTcProblem& p, cudaStream_t st) {
+  using namespace hat;
+  Args a;
+  if (!plan(p, a)) {
+    set_error(1, "attn_tc: shape not supported");
+    return;
+  }
+  CUtensorMap kmap, tmap, vmap;
+  bool ok = page_map(&kmap, p.k_cache, p.dim, p.kv_heads, 64, CU_TENSOR_MAP_SWIZZLE_128B);
+  tmap = vmap = kmap;
+  if (a.tail) ok = ok && page_map(&tmap, p.k_cache, p.dim, p.kv_heads, 32, CU_TENSOR_MAP_SWIZZLE_64B);
+  if (!a.shared) ok = ok && page_map(&vmap, p.v_cache, p.vdim, p.v_heads, 64, CU_TENSOR_MAP_SWIZZLE_128B);
+  a.err = wait_error_flag();
+  if (!ok || !a.err) {
+    set_error(2, "attn_tc: cuTensorMapEncodeTiled failed");
+    return;
+  }
+  const int smem = a.q_bytes + a.sk * a.k_stage + a.sv * a.v_stage + kBarBytes + kAlign;
+  const int tiles = (p.T + a.tq - 1) / a.tq + p.num_seqs;
+  // all passes in one block (Q is staged once) where that still gives every SM two blocks; otherwise a block per pass
+  a.ppc = p.nsplit == 1 && tiles * p.kv_heads >= 2 * sm_count() ? a.passes : 1;
+  const dim3 grid(tiles, p.kv_heads, p.nsplit * (a.passes / a.ppc));
+  const bool cap = p.softcap > 0.f, bias = p.slopes || p.dist_bias;
+  auto kern = cap ? (bias ? attn_tc_kernel<true, true> : attn_tc_kernel<true, false>)
+                  : (bias ? attn_tc_kernel<false, true> : attn_tc_kernel<false, false>);
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  kern<<<grid, kThreads, smem, st>>>(kmap, tmap, vmap, a);
+  B200_CUDA_LAUNCH_CHECK();
+}
+
+}  // namespace b200

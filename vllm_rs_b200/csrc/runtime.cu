@@ -48,6 +48,26 @@ int sm_count() {
   return cached;
 }
 
+static int* g_wait_host = nullptr;      // pinned; written by kernels through its device address
+int* wait_error_flag() {
+  static std::once_flag once;
+  static int* dev = nullptr;
+  std::call_once(once, [] {
+    // the first use may lie inside a stream capture of this thread: an allocation is no part of it
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    void *h = nullptr, *d = nullptr;
+    if (cudaHostAlloc(&h, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) == cudaSuccess &&
+        cudaHostGetDevicePointer(&d, h, 0) == cudaSuccess) {
+      *static_cast<volatile int*>(h) = 0;
+      g_wait_host = static_cast<int*>(h);
+      dev = static_cast<int*>(d);
+    }
+    cudaThreadExchangeStreamCaptureMode(&mode);
+  });
+  return dev;
+}
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
                                   const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
                                   const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
@@ -76,6 +96,10 @@ CUresult encode_tensor_map(CUtensorMap* map, CUtensorMapDataType dt, uint32_t ra
 
 extern "C" {
 int b200_last_error(void) {
+  if (b200::g_wait_host && *static_cast<volatile int*>(b200::g_wait_host)) {
+    *static_cast<volatile int*>(b200::g_wait_host) = 0;
+    b200::set_error(3, "a kernel gave up waiting for its data; the results of that launch are not valid");
+  }
   std::lock_guard<std::mutex> lk(b200::g_err_mu);
   return b200::g_err_code;
 }

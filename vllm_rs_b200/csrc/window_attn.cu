@@ -43,7 +43,7 @@
 #include <algorithm>
 #include <cstdlib>
 
-#include "seqmix.cuh"
+#include "paged_attn_tc.cuh"
 
 namespace b200 {
 using namespace seqmix;
@@ -887,6 +887,8 @@ static size_t window_mma_smem(int dim, int vdim, int maps = 1) {
 static bool window_mma_shape_ok(int dim, int vdim, int maps = 1) {
   return dim % 16 == 0 && vdim % 32 == 0 && vdim <= 256 && maps <= WQ && window_mma_smem(dim, vdim, maps) <= 200 * 1024;
 }
+// steps of few rows (decoding): the keys of a row are split over several blocks
+static bool few_rows(int T) { return T <= 2 * sm_count() / 4; }
 // blocks per token of the heads-as-rows form: a value head's group takes ceil(per_group / hpg) blocks
 static int window_mma_row_blocks(int heads, int kv_heads, int v_heads) {
   const int maps = std::max(1, kv_heads / v_heads), per_group = heads / kv_heads;
@@ -914,8 +916,9 @@ static int window_attn_mma_splits(int T, int heads, int kv_heads, int window, in
 }
 size_t window_attn_workspace_bytes(int T, int heads, int kv_heads, int vdim, int window, int keep_first, int v_heads) {
   if (v_heads <= 0 || kv_heads % v_heads != 0) v_heads = kv_heads;
-  const int n = std::max(window_attn_splits(T, heads, kv_heads, window, keep_first),
-                         window_attn_mma_splits(T, heads, kv_heads, window, keep_first, v_heads));
+  const int n = std::max({window_attn_splits(T, heads, kv_heads, window, keep_first),
+                          window_attn_mma_splits(T, heads, kv_heads, window, keep_first, v_heads),
+                          few_rows(T) ? attn_tc_splits(T, kv_heads, vdim, 0, window, keep_first) : 1});
   return n == 1 ? 0 : static_cast<size_t>(T) * heads * n * (vdim + 2) * 4;
 }
 
@@ -939,8 +942,25 @@ void launch_window_attn(void* out, const float* q, const void* k_cache, const vo
     set_error(1, "window_attn: kv_heads is a multiple of v_heads");
     return;
   }
-  // bf16, steps of many rows, value sizes up to 128: the tensor-core form with 64 token rows per block
-  if (!dt && window_mma_enabled() && T > 2 * sm_count() / 4 && window_rows_enabled() && dim % 16 == 0 && vdim % 16 == 0 &&
+  // bf16: the tcgen05 form takes key sizes that are multiples of 32 and value sizes that are multiples of 64
+  if (!dt && window_mma_enabled()) {
+    const int nsplit = few_rows(T) && workspace ? attn_tc_splits(T, kv_heads, vdim, 0, window, keep_first) : 1;
+    float* po = reinterpret_cast<float*>(workspace);
+    const AttnTcProblem p{out, q, k_cache, v_cache, sink, gate, ld_gate, gate_elems, cu, ctx, block_tables, max_blocks, num_seqs,
+                          T, heads, kv_heads, v_heads, dim, vdim, window, keep_first, chunk, scale, softcap, slopes, dist_bias,
+                          dist_n, out_f32, nsplit, po, po ? po + static_cast<size_t>(T) * heads * nsplit * vdim : nullptr};
+    if (attn_tc_takes(p)) {
+      launch_attn_tc(p, st_);
+      if (nsplit > 1) {
+        window_attn_merge_kernel<__nv_bfloat16><<<T * heads, vdim >= 128 ? 128 : 64, 0, st_>>>(
+            (__nv_bfloat16*)out, p.part_o, p.part_ml, sink, gate, ld_gate, heads, vdim, nsplit, gate_elems, out_f32);
+        B200_CUDA_LAUNCH_CHECK();
+      }
+      return;
+    }
+  }
+  // other sizes, steps of many rows, value sizes up to 128: the mma.sync form with 64 token rows per block
+  if (!dt && window_mma_enabled() && !few_rows(T) && window_rows_enabled() && dim % 16 == 0 && vdim % 16 == 0 &&
       vdim <= 128) {
     const int stage_bias = dist_bias && dist_n <= 2048;
     const size_t smem = (static_cast<size_t>(WKT + RQ) * (dim + 8) + static_cast<size_t>(WKT) * (vdim + 8)) * 2 +
@@ -975,7 +995,7 @@ void launch_window_attn(void* out, const float* q, const void* k_cache, const vo
     }
   }
   // bf16: the tensor-core kernel; steps of few rows take its heads-as-rows form with the keys split over blocks
-  const bool hrows = T <= 2 * sm_count() / 4;
+  const bool hrows = few_rows(T);
   if (!dt && window_mma_enabled() && window_mma_shape_ok(dim, vdim, hrows ? kv_heads / v_heads : 1)) {
     const size_t smem = window_mma_smem(dim, vdim, hrows ? kv_heads / v_heads : 1);
     const int nsplit = hrows && workspace ? window_attn_mma_splits(T, heads, kv_heads, window, keep_first, v_heads) : 1;
