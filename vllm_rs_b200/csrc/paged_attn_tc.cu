@@ -45,24 +45,65 @@ struct Args {
   int* err;
 };
 
-__device__ __forceinline__ uint64_t desc_mn_sw128(uint32_t saddr) {       // chunks of 64 MN elements 8 KB apart
-  uint64_t d = 0;
-  d |= uint64_t((saddr & 0x3FFFF) >> 4);
-  d |= uint64_t(kBlk >> 4) << 16;
-  d |= uint64_t(1024 >> 4) << 32;
-  d |= uint64_t(1) << 46;
-  d |= uint64_t(2) << 61;
-  return d;
+// Operand descriptors, upper words (version 1, SBO; layout 2 = SW128, 4 = SW64).  The lower word is the address in 16-byte
+// units under the LBO: unused for K-major rows (1); 8 KB between the 64-column chunks of the MN-major values.
+constexpr uint32_t kHiSw128 = (1024 >> 4) | (1u << 14) | (2u << 29), kHiSw64 = (512 >> 4) | (1u << 14) | (4u << 29);
+__device__ __forceinline__ uint32_t desc_k(uint32_t saddr) { return (saddr >> 4) | (1u << 16); }
+__device__ __forceinline__ uint32_t desc_mn(uint32_t saddr) { return (saddr >> 4) | (uint32_t(kBlk >> 4) << 16); }
+// One lane (lead != 0) issues; the warp runs the loop around it together, so that addresses stay uniform.
+__device__ __forceinline__ void mma_ss(uint32_t lead, uint32_t d, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi,
+                                       uint32_t idesc, uint32_t acc) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"
+      "setp.ne.b32 q, %0, 0;\n\tsetp.ne.b32 p, %7, 0;\n\t"
+      "mov.b64 da, {%2, %3};\n\tmov.b64 db, {%4, %5};\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%1], da, db, %6, p;\n\t}\n" ::"r"(lead),
+      "r"(d), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(acc)
+      : "memory");
 }
-__device__ __forceinline__ uint64_t desc_k_sw64(uint32_t saddr) {         // rows of 64 bytes, 8-row groups 512 bytes apart
-  uint64_t d = 0;
-  d |= uint64_t((saddr & 0x3FFFF) >> 4);
-  d |= uint64_t(1) << 16;
-  d |= uint64_t(512 >> 4) << 32;
-  d |= uint64_t(1) << 46;
-  d |= uint64_t(4) << 61;
-  return d;
+__device__ __forceinline__ void mma_ts(uint32_t lead, uint32_t d, uint32_t a_tmem, uint32_t b_lo, uint32_t b_hi, uint32_t idesc,
+                                       uint32_t acc) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t.reg .b64 db;\n\t"
+      "setp.ne.b32 q, %0, 0;\n\tsetp.ne.b32 p, %6, 0;\n\t"
+      "mov.b64 db, {%3, %4};\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%1], [%2], db, %5, p;\n\t}\n" ::"r"(lead),
+      "r"(d), "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(acc)
+      : "memory");
 }
+__device__ __forceinline__ void commit(uint32_t lead, uint64_t* bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %0, 0;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%1];\n\t}\n" ::"r"(lead),
+      "r"(smem_u32(bar))
+      : "memory");
+}
+// two fp32 values in a 64-bit register, one instruction for both
+using f2 = unsigned long long;
+__device__ __forceinline__ f2 pack2(float lo, float hi) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
+  f2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+// tanh(y) = y P(y^2) for |y| <= kTanhMax: minimax fit of tanh(y) / y in y^2, relative error 3e-8 before rounding
+constexpr float kTanhMax = 0.75f;
+constexpr float kT0 = 1.f, kT1 = -0.33332958817481995f, kT2 = 0.1332540661096573f, kT3 = -0.05334442853927612f,
+                kT4 = 0.019582903012633324f, kT5 = -0.004716253839433193f;
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32]) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
@@ -89,6 +130,8 @@ __device__ __forceinline__ int first_seen(int pos, int window, int chunk) {
   return chunk > 0 ? max(lo, pos / chunk * chunk) : lo;
 }
 
+// Waits do not end the loops around them: once one has given up (*fail), every other returns at once and the loops run out,
+// over shared memory and TMEM that stay the block's; what is still in flight then is waited for at the end.
 // Ring position: stage and the parity of its current use.
 struct Ring {
   int s = 0;
@@ -104,7 +147,7 @@ __global__ void __launch_bounds__(kThreads, 2)
 attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap tmap,
                const __grid_constant__ CUtensorMap vmap, const __grid_constant__ Args a) {
   const AttnTcProblem& p = a.p;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int G = a.group, kvh = blockIdx.y, vh = kvh % p.v_heads;
   // ---- which tokens: tile (gridDim.x - 1 - blockIdx.x) of the sequences' tiles, so that the latest (longest) go first
   int b = -1, tile = 0;
@@ -135,14 +178,16 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
   const int seq0 = static_cast<int>(p.cu[b]), nq = static_cast<int>(p.cu[b + 1]) - seq0;
   const int row0 = seq0 + tile * a.tq;                       // first token row
   const int nt = min(a.tq, nq - tile * a.tq), nrows = nt * G;
-  const int pos0 = static_cast<int>(p.ctx[b]) - nq + tile * a.tq, pos_last = pos0 + nt - 1;
+  const int p_ctx = static_cast<int>(p.ctx[b]);
+  const int pos0 = p_ctx - nq + tile * a.tq, pos_last = pos0 + nt - 1;
   const int key_lo = first_seen(pos0, p.window, p.chunk);
   const int wpage = key_lo / kTok;
   const int nkept = min(wpage, (min(max(p.keep_first, 0), key_lo) + kTok - 1) / kTok);
   const int ntiles = nkept + pos_last / kTok - wpage + 1;
   const int npz = a.passes / a.ppc, sp = blockIdx.z / npz, pass0 = (blockIdx.z % npz) * a.ppc;
   const int per = (ntiles + p.nsplit - 1) / p.nsplit;
-  const int j0 = sp * per, n = min(ntiles, j0 + per) - j0;   // this block's pages
+  const int j0 = sp * per, n = __shfl_sync(0xffffffffu, min(ntiles, j0 + per) - j0, 0);   // this block's pages
+  const int nwarps = (nrows + 31) / 32;                      // row warps that have a row
   const int vcols = a.vblk * 64;                             // value columns of a pass (the last one may have fewer)
 
   extern __shared__ uint8_t smem_raw[];
@@ -182,8 +227,8 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
     for (int s = 0; s < a.sv; ++s) { mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 1); }
     mbar_init(q_full, 4);
     mbar_init(s_full, 1);
-    mbar_init(s_free, 4);
-    mbar_init(p_full, 4);
+    mbar_init(s_free, nwarps);
+    mbar_init(p_full, nwarps);
     mbar_init(pv_done, 1);
     mbar_init(drained, 1);
     *fail = 0;
@@ -199,7 +244,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_ptr;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_ptr, 0);
   const uint32_t o_tm = tmem, s_tm = tmem + vcols, p_tm = s_tm + 64, q_tm = p_tm + 32;
   const int total = a.ppc * n;
   // blocks of value columns in pass x, and the first of them
@@ -209,124 +254,124 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
 
   if (warp == 0) {
     // ------------------------------------------------------------ pages
-    bool ok = true;
-    if (a.q_tm) ok = mbar_wait_limited(q_full, 0, fail, a.err);      // the rings lend their space to the staging of Q
+    if (a.q_tm) mbar_wait_limited(q_full, 0, fail, a.err);      // the rings lend their space to the staging of Q
     const uint32_t* bt = p.block_tables + static_cast<size_t>(b) * p.max_blocks;
     Ring kr, vr;
-    int armed_k = 0, armed_v = 0;
-    for (int pi = 0; pi < a.ppc && ok; ++pi) {
+    int armed_k = 0, armed_v = 0;           // (a stage that did not come free is not armed again, nor any after it)
+    bool free_ = true;
+    for (int pi = 0; pi < a.ppc; ++pi) {
       const int vf = v_first(pass0 + pi), vn = v_count(pass0 + pi);
-      for (int base = 0; base < n && ok; base += 32) {
+      const int kn = a.shared ? a.kblk - vn : a.kblk;
+      for (int base = 0; base < n; base += 32) {
         const int mine = base + lane < n ? static_cast<int>(bt[page_of(j0 + base + lane)]) : 0;
         const int cnt = min(32, n - base);
-        for (int jj = 0; jj < cnt && ok; ++jj) {
+        for (int jj = 0; jj < cnt; ++jj) {
           const int page = __shfl_sync(0xffffffffu, mine, jj);
           if (lane == 0) {
-            ok = mbar_wait_limited(&k_empty[kr.s], kr.ph ^ 1, fail, a.err);
-            if (ok) {
-              uint8_t* dst = k_smem + kr.s * a.k_stage;
-              const int kn = a.shared ? a.kblk - vn : a.kblk;
+            free_ = free_ && mbar_wait_limited(&k_empty[kr.s], kr.ph ^ 1, fail, a.err);
+            if (free_) {
+              uint8_t* kd = k_smem + kr.s * a.k_stage;
               mbar_arrive_expect_tx(&k_full[kr.s], kn * kBlk + a.tail * kTailBlk);
               for (int i = 0; i < kn; ++i) {
                 const int blk = a.shared && i >= vf ? i + vn : i;
-                tma_load_4d(dst + i * kBlk, &kmap, &k_full[kr.s], blk * 64, kvh, 0, page);
+                tma_load_4d(kd + i * kBlk, &kmap, &k_full[kr.s], blk * 64, kvh, 0, page);
               }
-              if (a.tail) tma_load_4d(dst + kn * kBlk, &tmap, &k_full[kr.s], a.kblk * 64, kvh, 0, page);
+              if (a.tail) tma_load_4d(kd + kn * kBlk, &tmap, &k_full[kr.s], a.kblk * 64, kvh, 0, page);
               ++armed_k;
-              ok = mbar_wait_limited(&v_empty[vr.s], vr.ph ^ 1, fail, a.err);
             }
-            if (ok) {
-              uint8_t* dst = v_smem + vr.s * a.v_stage;
+            free_ = free_ && mbar_wait_limited(&v_empty[vr.s], vr.ph ^ 1, fail, a.err);
+            if (free_) {
+              uint8_t* vd = v_smem + vr.s * a.v_stage;
               mbar_arrive_expect_tx(&v_full[vr.s], vn * kBlk);
               for (int i = 0; i < vn; ++i)
-                tma_load_4d(dst + i * kBlk, &vmap, &v_full[vr.s], (vf + i) * 64, vh, 0, page);
+                tma_load_4d(vd + i * kBlk, &vmap, &v_full[vr.s], (vf + i) * 64, vh, 0, page);
               ++armed_v;
             }
-            kr.next(a.sk);
-            vr.next(a.sv);
           }
-          ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+          kr.next(a.sk);
+          vr.next(a.sv);
         }
       }
     }
-    if (!ok && lane == 0) {                 // copies in flight land before the block ends
-      for (int s = 0; s < a.sk; ++s) {
-        const int uses = (armed_k + a.sk - 1 - s) / a.sk;
-        if (uses > 0) mbar_wait_limited(&k_full[s], (uses - 1) & 1, nullptr, a.err);
-      }
-      for (int s = 0; s < a.sv; ++s) {
-        const int uses = (armed_v + a.sv - 1 - s) / a.sv;
-        if (uses > 0) mbar_wait_limited(&v_full[s], (uses - 1) & 1, nullptr, a.err);
-      }
+    if (lane == 0 && *fail) {               // copies in flight land before the block ends
+      for (int s = 0; s < a.sk && s < armed_k; ++s)
+        mbar_wait_limited(&k_full[s], ((armed_k - 1 - s) / a.sk) & 1, nullptr, a.err);
+      for (int s = 0; s < a.sv && s < armed_v; ++s)
+        mbar_wait_limited(&v_full[s], ((armed_v - 1 - s) / a.sv) & 1, nullptr, a.err);
     }
+    __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------------------ products
-    if (lane == 0) {
-      constexpr uint32_t kBf16 = (1u << 7) | (1u << 10);
-      const uint32_t idesc_s = make_idesc_f16(kRows, kTok) | kBf16;
-      const uint32_t q_addr = smem_u32(q_smem);
-      Ring kr, vr, vr_pv;
-      bool ok = mbar_wait_limited(q_full, 0, fail, a.err);
+    constexpr uint32_t kBf16 = (1u << 7) | (1u << 10);
+    constexpr uint32_t idesc_s = make_idesc_f16(kRows, kTok) | kBf16;
+    const uint32_t lead = elect_one() ? 1u : 0u;
+    const uint32_t q_lo = desc_k(smem_u32(q_smem));
+    Ring kr, vr, vr_pv;
+    auto wait = [&](uint64_t* bar, uint32_t parity) { mbar_wait_limited(bar, parity, fail, a.err); };
+    // S (+)= the queries of block `blk` times a page's block of 64 columns
+    auto qk_block = [&](int blk, uint32_t b_lo, uint32_t acc) {
+      if (blk < a.q_tm) {
+        const uint32_t qa = q_tm + blk * 32;
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks) mma_ts(lead, s_tm, qa + ks * 8, b_lo + ks * 2, kHiSw128, idesc_s, ks ? 1u : acc);
+      } else {
+        const uint32_t a_lo = q_lo + (blk - a.q_tm) * (kQBlk >> 4);
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks)
+          mma_ss(lead, s_tm, a_lo + ks * 2, kHiSw128, b_lo + ks * 2, kHiSw128, idesc_s, ks ? 1u : acc);
+      }
+    };
+    const uint32_t k_base = desc_k(smem_u32(k_smem)), v_base = desc_k(smem_u32(v_smem)), vm_base = desc_mn(smem_u32(v_smem));
+    const uint32_t k_step = a.k_stage >> 4, v_step = a.v_stage >> 4;
+    auto issue_qk = [&](int it, int vf, int vn) {
+      wait(&k_full[kr.s], kr.ph);
+      if (it > 0) wait(s_free, (it - 1) & 1);           // the rows hold S of the page before
       tc_fence_after();
-      auto qk_block = [&](int blk, uint32_t kaddr, uint32_t acc) {
+      const uint32_t k_lo = k_base + kr.s * k_step;
+      const int kn = a.shared ? a.kblk - vn : a.kblk;
+      uint32_t acc = 0;
+      for (int i = 0; i < kn; ++i, acc = 1) qk_block(a.shared && i >= vf ? i + vn : i, k_lo + i * (kBlk >> 4), acc);
+      if (a.tail) {
+        const uint32_t a_lo = q_lo + (a.kblk - a.q_tm) * (kQBlk >> 4), b_lo = k_lo + kn * (kBlk >> 4);
 #pragma unroll
-        for (int ks = 0; ks < 4; ++ks) {
-          const uint64_t bd = make_smem_desc_sw128(kaddr + ks * 32);
-          if (blk < a.q_tm)
-            tc_mma_ts(s_tm, q_tm + blk * 32 + ks * 8, bd, idesc_s, (acc | ks) ? 1u : 0u);
-          else
-            tc_mma_ss(s_tm, make_smem_desc_sw128(q_addr + (blk - a.q_tm) * kQBlk + ks * 32), bd, idesc_s, (acc | ks) ? 1u : 0u);
-        }
-      };
-      auto issue_qk = [&](int it) {
-        const int pass = pass0 + it / n, vf = v_first(pass), vn = v_count(pass);
-        ok = ok && mbar_wait_limited(&k_full[kr.s], kr.ph, fail, a.err);
-        if (it > 0) ok = ok && mbar_wait_limited(s_free, (it - 1) & 1, fail, a.err);     // the rows hold S of the page before
-        if (!ok) return;
+        for (int ks = 0; ks < 2; ++ks, acc = 1)
+          mma_ss(lead, s_tm, a_lo + ks * 2, kHiSw64, b_lo + ks * 2, kHiSw64, idesc_s, acc);
+      }
+      commit(lead, &k_empty[kr.s]);
+      kr.next(a.sk);
+      if (a.shared) {
+        wait(&v_full[vr.s], vr.ph);
         tc_fence_after();
-        const uint32_t kaddr = smem_u32(k_smem + kr.s * a.k_stage);
-        const int kn = a.shared ? a.kblk - vn : a.kblk;
-        uint32_t acc = 0;
-        for (int i = 0; i < kn; ++i, acc = 1) qk_block(a.shared && i >= vf ? i + vn : i, kaddr + i * kBlk, acc);
-        if (a.tail) {
-#pragma unroll
-          for (int ks = 0; ks < 2; ++ks, acc = 1)
-            tc_mma_ss(s_tm, desc_k_sw64(q_addr + (a.kblk - a.q_tm) * kQBlk + ks * 32), desc_k_sw64(kaddr + kn * kBlk + ks * 32),
-                      idesc_s, acc);
-        }
-        if (a.shared) {
-          tc_commit(&k_empty[kr.s]);        // (the blocks of this ring were read by the products so far)
-          ok = mbar_wait_limited(&v_full[vr.s], vr.ph, fail, a.err);
-          if (!ok) return;
-          const uint32_t vaddr = smem_u32(v_smem + vr.s * a.v_stage);
-          for (int i = 0; i < vn; ++i, acc = 1) qk_block(vf + i, vaddr + i * kBlk, acc);
-          vr.next(a.sv);
-        } else {
-          tc_commit(&k_empty[kr.s]);
-        }
-        tc_commit(s_full);
-        kr.next(a.sk);
-      };
-      issue_qk(0);
-      for (int it = 0; it < total && ok; ++it) {
-        if (it + 1 < total) issue_qk(it + 1);
-        ok = ok && mbar_wait_limited(p_full, it & 1, fail, a.err);
-        if (!a.shared) ok = ok && mbar_wait_limited(&v_full[vr_pv.s], vr_pv.ph, fail, a.err);
-        if (!ok) break;
+        const uint32_t v_lo = v_base + vr.s * v_step;
+        for (int i = 0; i < vn; ++i, acc = 1) qk_block(vf + i, v_lo + i * (kBlk >> 4), acc);
+        vr.next(a.sv);
+      }
+      commit(lead, s_full);
+    };
+    wait(q_full, 0);
+    int it = 0;
+    issue_qk(0, v_first(pass0), v_count(pass0));
+    for (int pi = 0; pi < a.ppc; ++pi) {
+      const int vf = v_first(pass0 + pi), vn = v_count(pass0 + pi);
+      const uint32_t idesc_o = make_idesc_f16(kRows, vn * 64) | (1u << 16) | kBf16;     // B is MN-major
+      for (int j = 0; j < n; ++j, ++it) {
+        if (j + 1 < n) issue_qk(it + 1, vf, vn);
+        else if (pi + 1 < a.ppc) issue_qk(it + 1, v_first(pass0 + pi + 1), v_count(pass0 + pi + 1));
+        wait(p_full, it & 1);
+        if (!a.shared) wait(&v_full[vr_pv.s], vr_pv.ph);
         tc_fence_after();
-        const uint32_t vaddr = smem_u32(v_smem + vr_pv.s * a.v_stage);
-        const uint32_t idesc_o = make_idesc_f16(kRows, v_count(pass0 + it / n) * 64) | (1u << 16) | kBf16;     // B is MN-major
+        const uint32_t v_lo = vm_base + vr_pv.s * v_step;
 #pragma unroll
         for (int ks = 0; ks < kTok / 16; ++ks)
-          tc_mma_ts(o_tm, p_tm + ks * 8, desc_mn_sw128(vaddr + ks * 2048), idesc_o, (it % n > 0 || ks > 0) ? 1u : 0u);
-        tc_commit(&v_empty[vr_pv.s]);
-        tc_commit(pv_done);
+          mma_ts(lead, o_tm, p_tm + ks * 8, v_lo + ks * (2048 >> 4), kHiSw128, idesc_o, (j > 0 || ks > 0) ? 1u : 0u);
+        commit(lead, &v_empty[vr_pv.s]);
+        commit(lead, pv_done);
         vr_pv.next(a.sv);
       }
-      if (!ok) {                            // products in flight end before TMEM is given back
-        tc_commit(drained);
-        mbar_wait_limited(drained, 0, nullptr, a.err);
-      }
+    }
+    if (*fail) {                            // products in flight end before TMEM is given back
+      commit(lead, drained);
+      mbar_wait_limited(drained, 0, nullptr, a.err);
     }
     __syncwarp();
   } else {
@@ -336,16 +381,15 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
     const uint32_t lane_base = static_cast<uint32_t>(q4 * 32) << 16;
     // ---- stage Q as bf16: coalesced 32-byte reads, chunks of 8 entries
     {
-      const int cpr = p.dim / 8, pitch = a.q_tm * 128 + 16;
+      const int cpr = p.dim / 8;
       const int dr = kRows / cpr, dc = kRows % cpr;          // what 128 chunks on are: dr rows and dc chunks
       int row = tid / cpr, c = tid % cpr;
       while (row < kRows) {
-        float4 lo[4], hi[4];
-        int rw[4], cc[4];
+        constexpr int U = 8;                                 // chunks in flight per thread: 32 KB per block
+        float4 lo[U], hi[U];
+        const int row_first = row, c_first = c;
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          rw[u] = row;
-          cc[u] = c;
+        for (int u = 0; u < U; ++u) {
           lo[u] = hi[u] = make_float4(0.f, 0.f, 0.f, 0.f);
           if (row < nrows) {
             const int t = row / G;
@@ -358,20 +402,26 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
           c += dc;
           if (c >= cpr) { c -= cpr; ++row; }
         }
+        row = row_first;
+        c = c_first;
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          if (rw[u] >= kRows) continue;
-          uint4 w;
-          w.x = pack16x2<true>(lo[u].x, lo[u].y);
-          w.y = pack16x2<true>(lo[u].z, lo[u].w);
-          w.z = pack16x2<true>(hi[u].x, hi[u].y);
-          w.w = pack16x2<true>(hi[u].z, hi[u].w);
-          const int blk = cc[u] >> 3, c8 = cc[u] & 7;
-          uint8_t* dst;
-          if (blk < a.q_tm) dst = k_smem + rw[u] * pitch + cc[u] * 16;
-          else if (blk < a.kblk) dst = q_smem + (blk - a.q_tm) * kQBlk + rw[u] * 128 + ((c8 ^ (rw[u] & 7)) << 4);
-          else dst = q_smem + (a.kblk - a.q_tm) * kQBlk + rw[u] * 64 + ((c8 ^ ((rw[u] >> 1) & 3)) << 4);
-          *reinterpret_cast<uint4*>(dst) = w;
+        for (int u = 0; u < U; ++u) {
+          if (row < kRows) {
+            uint4 w;
+            w.x = pack16x2<true>(lo[u].x, lo[u].y);
+            w.y = pack16x2<true>(lo[u].z, lo[u].w);
+            w.z = pack16x2<true>(hi[u].x, hi[u].y);
+            w.w = pack16x2<true>(hi[u].z, hi[u].w);
+            const int blk = c >> 3, c8 = c & 7;
+            uint8_t* dst;
+            if (blk < a.q_tm) dst = k_smem + blk * kQBlk + row * 128 + ((c8 ^ (row & 7)) << 4);
+            else if (blk < a.kblk) dst = q_smem + (blk - a.q_tm) * kQBlk + row * 128 + ((c8 ^ (row & 7)) << 4);
+            else dst = q_smem + (a.kblk - a.q_tm) * kQBlk + row * 64 + ((c8 ^ ((row >> 1) & 3)) << 4);
+            *reinterpret_cast<uint4*>(dst) = w;
+          }
+          row += dr;
+          c += dc;
+          if (c >= cpr) { c -= cpr; ++row; }
         }
       }
       __syncwarp();
@@ -379,10 +429,10 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
         asm volatile("bar.sync 1, 128;" ::: "memory");
         for (int blk = 0; blk < a.q_tm; ++blk) {
           uint32_t w[32];
-          const uint4* src = reinterpret_cast<const uint4*>(k_smem + r * pitch + blk * 128);
+          const uint8_t* src = k_smem + blk * kQBlk + r * 128;          // (eight lanes' rows lie in different banks)
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
-            const uint4 v = src[i];
+            const uint4 v = *reinterpret_cast<const uint4*>(src + ((i ^ (r & 7)) << 4));
             w[4 * i] = v.x; w[4 * i + 1] = v.y; w[4 * i + 2] = v.z; w[4 * i + 3] = v.w;
           }
           tmem_st32(q_tm + lane_base + blk * 32, w);
@@ -400,7 +450,8 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
     const int pos = pos0 + tl, lo = first_seen(pos, p.window, p.chunk);
     const int lo_last = first_seen(pos_last, p.window, p.chunk);
     const bool with_sink = p.sink && p.nsplit == 1;          // split runs add the sink when the parts are merged
-    const float sl = CAP ? p.scale / p.softcap * (2.f * kLog2e) : p.scale * kLog2e;
+    // what a product becomes a score (or, capped, the argument of tanh) by; scores are in log2 units
+    const float sl = CAP ? p.scale / p.softcap : p.scale * kLog2e;
     const float cap2 = p.softcap * kLog2e;
     float slope = 0.f, far_bias = 0.f;
     const float* table = nullptr;
@@ -412,64 +463,82 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
       }
     }
     Ring vr;
-    bool ok = true;
     int it = 0;
-    for (int pi = 0; pi < a.ppc && ok; ++pi) {
+    const int passes = q4 < nwarps ? a.ppc : 0;              // a warp without rows is done
+    for (int pi = 0; pi < passes; ++pi) {
       float m_ref = with_sink && valid ? p.sink[h] * kLog2e : kNone, l = with_sink ? 1.f : 0.f;
       const int vn = v_count(pass0 + pi);
       for (int j = 0; j < n; ++j, ++it) {
         const int base = page_of(j0 + j) * kTok;
-        ok = mbar_wait_limited(s_full, it & 1, fail, a.err);
-        if (__any_sync(0xffffffffu, !ok)) { ok = false; break; }
+        mbar_wait_limited(s_full, it & 1, fail, a.err);
+        __syncwarp();
         tc_fence_after();
-        float x[kTok];
-        {
-          uint32_t v0[32], v1[32];
-          tmem_ld_x32(s_tm + lane_base, v0);
-          tmem_ld_x32(s_tm + lane_base + 32, v1);
-          tc_wait_ld();
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            x[i] = __uint_as_float(v0[i]);
-            x[32 + i] = __uint_as_float(v1[i]);
-          }
-        }
+        uint32_t v0[32], v1[32];
+        tmem_ld_x32(s_tm + lane_base, v0);
+        tmem_ld_x32(s_tm + lane_base + 32, v1);
+        tc_wait_ld();
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(s_free);
-        // x becomes the score in log2 units (plain scores keep their scale for the exponent's multiply-add)
-        if (CAP) {
-          // cap tanh(s / cap) = cap - 2 cap / (e^(2 s / cap) + 1)
+        float x[kTok];
 #pragma unroll
-          for (int i = 0; i < kTok; ++i) x[i] = fmaf(-2.f * cap2, rcp(ex2(x[i] * sl) + 1.f), cap2);
+        for (int i = 0; i < 32; ++i) {
+          x[i] = __uint_as_float(v0[i]);
+          x[32 + i] = __uint_as_float(v1[i]);
+        }
+        // x times `mult` is the score; keys outside the mask become -inf
+        float mult = sl;
+        if (CAP) {
+          float big0 = fabsf(x[0]), big1 = fabsf(x[1]);
+#pragma unroll
+          for (int i = 2; i < kTok - 2; i += 4) {
+            big0 = max3(big0, fabsf(x[i]), fabsf(x[i + 1]));
+            big1 = max3(big1, fabsf(x[i + 2]), fabsf(x[i + 3]));
+          }
+          big0 = max3(big0, fabsf(x[kTok - 2]), fabsf(x[kTok - 1]));
+          mult = cap2;
+          if (__all_sync(0xffffffffu, fmaxf(big0, big1) * sl <= kTanhMax)) {
+#pragma unroll
+            for (int i = 0; i < kTok; i += 2) {
+              const f2 y = mul2(pack2(x[i], x[i + 1]), pack2(sl, sl)), t = mul2(y, y);
+              f2 q = fma2(t, pack2(kT5, kT5), pack2(kT4, kT4));
+              q = fma2(t, q, pack2(kT3, kT3));
+              q = fma2(t, q, pack2(kT2, kT2));
+              q = fma2(t, q, pack2(kT1, kT1));
+              q = mul2(y, fma2(t, q, pack2(kT0, kT0)));
+              asm("mov.b64 {%0, %1}, %2;" : "=f"(x[i]), "=f"(x[i + 1]) : "l"(q));
+            }
+          } else {
+            // tanh(y) = 1 - 2 / (e^(2 y) + 1)
+            const float e2 = sl * (2.f * kLog2e);
+#pragma unroll
+            for (int i = 0; i < kTok; ++i) x[i] = fmaf(-2.f, rcp(ex2(x[i] * e2) + 1.f), 1.f);
+          }
         }
         if (BIAS) {
-          if (!CAP) {
-#pragma unroll
-            for (int i = 0; i < kTok; ++i) x[i] *= sl;
-          }
           const float d0 = static_cast<float>(pos - base);
           if (table && pos - (base + kTok - 1) < p.dist_n - 1) {
 #pragma unroll
             for (int i = 0; i < kTok; ++i)
-              x[i] += fmaf(__ldg(table + max(0, min(pos - base - i, p.dist_n - 1))), kLog2e, -slope * (d0 - i));
+              x[i] = fmaf(x[i], mult, fmaf(-slope, d0 - i, __ldg(table + max(0, min(pos - base - i, p.dist_n - 1))) * kLog2e));
           } else {
 #pragma unroll
-            for (int i = 0; i < kTok; ++i) x[i] += far_bias - slope * (d0 - i);
+            for (int i = 0; i < kTok; ++i) x[i] = fmaf(x[i], mult, fmaf(-slope, d0 - i, far_bias));
           }
+          mult = 1.f;
         }
         if (base + kTok - 1 > pos0 || base < lo_last) {       // the diagonal, the window's edge, kept tokens
+          const int last = pos - base, first = lo - base, kept = p.keep_first - base;
 #pragma unroll
-          for (int i = 0; i < kTok; ++i) {
-            const int k = base + i;
-            x[i] = (k <= pos && (k >= lo || k < p.keep_first)) ? x[i] : -INFINITY;
-          }
+          for (int i = 0; i < kTok; ++i) x[i] = i <= last && (i >= first || i < kept) ? x[i] : -INFINITY;
         }
-        float mx = fmaxf(x[0], x[1]);
+        float mx0 = max3(x[0], x[1], x[2]), mx1 = max3(x[3], x[4], x[5]);
 #pragma unroll
-        for (int i = 2; i < kTok; ++i) mx = fmaxf(mx, x[i]);
-        const float mult = (CAP || BIAS) ? 1.f : sl;
-        mx *= mult;
+        for (int i = 6; i < kTok - 2; i += 4) {
+          mx0 = max3(mx0, x[i], x[i + 1]);
+          mx1 = max3(mx1, x[i + 2], x[i + 3]);
+        }
+        const float mx = max3(mx0, mx1, fmaxf(x[kTok - 2], x[kTok - 1])) * mult;
         float corr = 1.f;
         bool grow = false;
         if (mx - m_ref > kRescale) {
@@ -477,32 +546,31 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
           m_ref = mx;
           grow = true;
         }
-        float ps0 = 0.f, ps1 = 0.f;
+        // the sum takes the weights as the product does, rounded to bf16: their roundings cancel in the quotient
+        float sum[4] = {0.f, 0.f, 0.f, 0.f};
         uint32_t pk[32];
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
-          const float e0 = ex2(fmaf(x[2 * i], mult, -m_ref)), e1 = ex2(fmaf(x[2 * i + 1], mult, -m_ref));
-          ps0 += e0;
-          ps1 += e1;
-          pk[i] = pack16x2<true>(e0, e1);
+          pk[i] = pack16x2<true>(ex2(fmaf(x[2 * i], mult, -m_ref)), ex2(fmaf(x[2 * i + 1], mult, -m_ref)));
+          sum[(2 * i) & 3] += __uint_as_float(pk[i] << 16);
+          sum[(2 * i + 1) & 3] += __uint_as_float(pk[i] & 0xFFFF0000u);
         }
-        l = fmaf(l, corr, ps0 + ps1);
-        // value rows that no row of the block sees (past the last key, before the window) may hold anything: 0 * NaN
-        if (base + kTok - 1 > pos_last || (base < key_lo && base + kTok > p.keep_first)) {
-          ok = mbar_wait_limited(&v_full[vr.s], vr.ph, fail, a.err);
-          if (__any_sync(0xffffffffu, !ok)) { ok = false; break; }
-          uint8_t* vt = v_smem + vr.s * a.v_stage;
-          for (int e = tid; e < kTok * vn * 8; e += 128) {
-            const int row = e / (vn * 8), c = e - row * (vn * 8), k = base + row;
-            if (k > pos_last || (k < key_lo && k >= p.keep_first))
-              *reinterpret_cast<uint4*>(vt + (c >> 3) * kBlk + row * 128 + (c & 7) * 16) = make_uint4(0, 0, 0, 0);
-          }
+        l = fmaf(l, corr, (sum[0] + sum[1]) + (sum[2] + sum[3]));
+        // Value rows past the sequence's end may hold anything, and 0 * NaN is no 0; a single token does not even meet the
+        // rows before its window.
+        const int v_end = p_ctx - base, v_lo = nt == 1 && base + kTok > p.keep_first ? key_lo - base : 0;
+        if (v_end < kTok || v_lo > 0) {
+          mbar_wait_limited(&v_full[vr.s], vr.ph, fail, a.err);
+          uint8_t* vt = v_smem + vr.s * a.v_stage + (r & 7) * 16;
+          for (int row = r >> 3; row < kTok; row += nwarps * 4)
+            if (row >= v_end || (row < v_lo && base + row >= p.keep_first))
+              for (int i = 0; i < vn; ++i) *reinterpret_cast<uint4*>(vt + i * kBlk + row * 128) = make_uint4(0, 0, 0, 0);
           fence_proxy_async();
         }
         vr.next(a.sv);
         if (it > 0) {
-          ok = mbar_wait_limited(pv_done, (it - 1) & 1, fail, a.err);      // P and O are the rows' again
-          if (__any_sync(0xffffffffu, !ok)) { ok = false; break; }
+          mbar_wait_limited(pv_done, (it - 1) & 1, fail, a.err);           // P and O are the rows' again
+          __syncwarp();
           tc_fence_after();
           if (j > 0 && __any_sync(0xffffffffu, grow)) {
 #pragma unroll 1
@@ -522,9 +590,8 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
         __syncwarp();
         if (lane == 0) mbar_arrive(p_full);
       }
-      if (!ok) break;
-      ok = mbar_wait_limited(pv_done, (it - 1) & 1, fail, a.err);
-      if (__any_sync(0xffffffffu, !ok)) { ok = false; break; }
+      mbar_wait_limited(pv_done, (it - 1) & 1, fail, a.err);
+      __syncwarp();
       tc_fence_after();
       // ---- the pass's columns of this row
       const size_t trow = static_cast<size_t>(row0 + tl), orow = trow * p.heads + h;
@@ -612,7 +679,7 @@ static bool plan(const AttnTcProblem& p, Args& a) {
       a.q_bytes = (a.kblk - a.q_tm) * kQBlk + a.tail * kQTail;
       const int rings = a.sk * a.k_stage + a.sv * a.v_stage;
       if (a.q_bytes + rings + kBarBytes + kAlign > kSmemMax) continue;
-      if (a.q_tm && kRows * (a.q_tm * 128 + 16) > rings) continue;
+      if (a.q_tm * kQBlk > rings) continue;
       const int cols = a.vblk * 64 + 96 + a.q_tm * 32;
       a.tmem_cols = cols <= 128 ? 128 : (cols <= 256 ? 256 : 512);
       return true;
