@@ -246,7 +246,6 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
   tc_fence_after();
   const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_ptr, 0);
   const uint32_t o_tm = tmem, s_tm = tmem + vcols, p_tm = s_tm + 64, q_tm = p_tm + 32;
-  const int total = a.ppc * n;
   // blocks of value columns in pass x, and the first of them
   auto v_first = [&](int x) { return x * a.vblk; };
   auto v_count = [&](int x) { return min(a.vblk, p.vdim / 64 - x * a.vblk); };
