@@ -1,0 +1,56 @@
+"""The tcgen05 grouped products of routed experts against 64-bit experts: buckets that are empty, hold one row, end inside a tile
+or take several; features and inner sizes that end inside a tile; every activation; identity experts; all three tile widths."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("act", ["silu_gate", "relu2", "clamped"])
+@pytest.mark.parametrize("T,E,top,D,F,skew", [
+    (1, 4, 2, 64, 32, 0), (37, 5, 3, 72, 40, 0), (3, 64, 1, 512, 8, 0), (300, 3, 2, 136, 264, 0), (700, 16, 4, 64, 520, 3),
+    (513, 2, 1, 264, 1032, 0), (2100, 20, 2, 96, 4100 // 8 * 8, 0), (129, 1, 1, 8, 16, 0)])
+def test_experts(lib, act, T, E, top, D, F, skew):
+    from vllm_rs_b200 import ops
+    g = torch.Generator().manual_seed(T * E + F)
+    bf, dev = torch.bfloat16, "cuda"
+    ident = 2 if T == 37 else 0
+    h = torch.randn(T, D, generator=g).to(bf)
+    wu = (torch.randn(E, F if act == "relu2" else 2 * F, D, generator=g) / D ** 0.5).to(bf)
+    wd = (torch.randn(E, D, F, generator=g) / F ** 0.5).to(bf)
+    z = torch.randn(T, E + ident, generator=g) - skew * torch.arange(E + ident).float()       # skew leaves buckets empty
+    w, idx = torch.softmax(z, 1).topk(top, 1)
+    x = torch.randn(T, D, generator=g)
+    limit, alpha, add = 1.5, 1.702, 1.0
+    want, tol = x.double().to(dev), torch.zeros(T, D, dtype=torch.float64, device=dev)
+    H, u24 = h.double().to(dev), 2.0 ** -24
+    for e in range(E):
+        t, j = (idx == e).nonzero(as_tuple=True)
+        if not len(t):
+            continue
+        t, wt = t.to(dev), w[t, j].double().to(dev)[:, None]
+        a, b, m = H[t], wu[e].double().to(dev), wd[e].double().to(dev)
+        y, dy = a @ b.T, D * u24 * (a.abs() @ b.abs().T)          # a product and what its fp32 sum may be off by
+        if act == "relu2":
+            r = torch.relu(y)
+            y, dy = r * r, 2 * r * dy + dy * dy
+        else:
+            gt, up, dg, du = *y.chunk(2, 1), *dy.chunk(2, 1)
+            if act == "clamped":
+                gt, up = gt.clamp(max=limit), up.clamp(-limit, limit)
+                s = gt * torch.sigmoid(alpha * gt)
+                y, dy = s * (up + add), 1.2 * (up + add).abs() * dg + s.abs() * du
+            else:
+                s = torch.nn.functional.silu(gt)
+                y, dy = s * up, 1.2 * up.abs() * dg + s.abs() * du          # |d silu| < 1.1
+        want.index_add_(0, t, wt * (y @ m.T))
+        # the activation is rounded to bf16 (2^-8 of itself), the second product sums F terms in fp32
+        tol.index_add_(0, t, wt * (((2.0 ** -8 + F * u24) * y.abs() + dy) @ m.abs().T))
+    for e in range(E, E + ident):
+        t, j = (idx == e).nonzero(as_tuple=True)
+        want.index_add_(0, t.to(dev), w[t, j].double().to(dev)[:, None] * H[t.to(dev)])
+    kw = dict(limit=limit, alpha=alpha, up_add=add) if act == "clamped" else {}
+    c = lambda v: v.to(dev).contiguous()                                     # noqa: E731
+    out = ops.moe_experts_ex(c(x), c(h), c(idx.int()), c(w), c(wu), c(wd), act=act, identity=ident, **kw)
+    err = (out.double() - want).abs()
+    assert bool((err <= 1.02 * tol + 1e-5 * want.abs().clamp(min=1.0)).all()), (err - tol).max().item()

@@ -17,10 +17,10 @@
 //   down     : y[slot, d] = act[slot] . Wd[e, d];  W_down [E, width, F]; fp32 out.
 //   combine  : x[token] (+)= sum_choice w[token, choice] * y[slot(token, choice)], choices added in order (no atomics).
 //              Router outputs past the last real expert are identity experts: y = the token's own input row.
-// The grouped products run on the tensor cores (mma.sync m16n8k16, bf16 x bf16 -> fp32) for bf16 activations and as
-// plain fp32 FMAs for fp32 activations; both walk K in the same order for a row wherever the row sits in a tile.
+// The grouped products run on the tensor cores for bf16 activations (moe_tc.cu; mma.sync where sizes are no multiples of 8)
+// and as plain fp32 FMAs for fp32 activations; all walk K in the same order for a row wherever the row sits in a tile.
 #include "../../include/b200_vllm.h"
-#include "seqmix.cuh"
+#include "moe_tc.cuh"
 
 namespace b200 {
 using namespace seqmix;
@@ -120,27 +120,46 @@ __global__ void moe_route_kernel(const float* __restrict__ logits, const float* 
     for (int j = lane; j < top; j += 32) top_w[static_cast<size_t>(t) * top + j] /= total + (score == 2 ? 0.f : 1e-20f);
 }
 
-// single block: histogram, exclusive scan, scatter
-__global__ void moe_sort_kernel(const int32_t* __restrict__ top_idx, int pairs, int E, int32_t* __restrict__ expert_off,
-                                int32_t* __restrict__ pair_of_slot, int32_t* __restrict__ slot_of_pair) {
+// Single block: histogram, exclusive scan, scatter.  Lanes with the same expert count as one: thousands of pairs meet on few
+// counters (16384 pairs of 16 experts, 14.5 us with an atomic per pair).
+__global__ void __launch_bounds__(1024)
+moe_sort_kernel(const int32_t* __restrict__ top_idx, int pairs, int E, int32_t* __restrict__ expert_off,
+                int32_t* __restrict__ pair_of_slot, int32_t* __restrict__ slot_of_pair) {
   extern __shared__ int cnt[];       // [E] counts, then cursors
+  const int lane = threadIdx.x & 31;
   for (int e = threadIdx.x; e < E; e += blockDim.x) cnt[e] = 0;
   __syncthreads();
-  for (int p = threadIdx.x; p < pairs; p += blockDim.x) atomicAdd(&cnt[top_idx[p]], 1);
+  for (int p = threadIdx.x; p < pairs; p += blockDim.x) {
+    const unsigned act = __activemask();
+    const int e = top_idx[p];
+    const unsigned same = __match_any_sync(act, e);
+    if (lane == __ffs(same) - 1) atomicAdd(&cnt[e], __popc(same));
+  }
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (threadIdx.x < 32) {            // one warp scans the counts, 32 at a time
     int run = 0;
-    for (int e = 0; e < E; ++e) {
-      const int c = cnt[e];
-      expert_off[e] = run;
-      cnt[e] = run;
-      run += c;
+    for (int e0 = 0; e0 < E; e0 += 32) {
+      const int e = e0 + lane, c = e < E ? cnt[e] : 0;
+      int inc = c;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += v;
+      }
+      if (e < E) expert_off[e] = cnt[e] = run + inc - c;
+      run += __shfl_sync(0xffffffffu, inc, 31);
     }
-    expert_off[E] = run;
+    if (lane == 0) expert_off[E] = run;
   }
   __syncthreads();
   for (int p = threadIdx.x; p < pairs; p += blockDim.x) {
-    const int slot = atomicAdd(&cnt[top_idx[p]], 1);
+    const unsigned act = __activemask();
+    const int e = top_idx[p];
+    const unsigned same = __match_any_sync(act, e);
+    const int head = __ffs(same) - 1;
+    int slot = 0;
+    if (lane == head) slot = atomicAdd(&cnt[e], __popc(same));
+    slot = __shfl_sync(act, slot, head) + __popc(same & ((1u << lane) - 1));
     pair_of_slot[slot] = p;
     slot_of_pair[p] = slot;
   }
@@ -170,13 +189,6 @@ __device__ __forceinline__ bool find_tile(const int32_t* __restrict__ off, int E
 // ACT: 0 = plain product over slot rows, fp32 out (the down projection); 1 = gathered token rows, two weight matrices,
 // SiLU(gate) * up; 2 = gathered token rows, one matrix, relu(.)^2; 3 = as 1 with the clamped gate.  ACT != 0 stores the
 // activation dtype.
-template <int ACT>
-__device__ __forceinline__ float expert_gate(float g, float u, const b200_expert_act& p) {
-  if (ACT != 3) return silu_exact(g) * u;
-  g = fminf(g, p.limit);
-  u = fminf(fmaxf(u, -p.limit), p.limit);
-  return g / (1.f + expf(-p.alpha * g)) * (u + p.up_add);
-}
 // fp32 path (and the generic one): 256 threads, each 2 rows x 2 columns (x 2 matrices when gated)
 template <typename T, int ACT>
 __global__ void __launch_bounds__(256)
@@ -374,23 +386,42 @@ grouped_linear_mma_kernel(void* __restrict__ out_, const __nv_bfloat16* __restri
       }
 }
 
-// choices >= E are identity experts: their row is the token's own input (ident, fp32 or the activation dtype)
-template <typename TI>
-__global__ void moe_combine_kernel(float* __restrict__ x, const float* __restrict__ down,
-                                   const int32_t* __restrict__ slot_of_pair, const int32_t* __restrict__ top_idx,
-                                   const float* __restrict__ top_w, int top, int width, int E,
-                                   const TI* __restrict__ ident, int accumulate) {
-  const int t = blockIdx.x;
-  for (int d = threadIdx.x; d < width; d += blockDim.x) {
-    float acc = 0.f;
-    for (int j = 0; j < top; ++j) {
-      const size_t p = static_cast<size_t>(t) * top + j;
-      const float row = (ident && top_idx[p] >= E) ? ld(ident + static_cast<size_t>(t) * width + d)
-                                                   : down[static_cast<size_t>(slot_of_pair[p]) * width + d];
-      acc += top_w[p] * row;
+// choices >= E are identity experts: their row is the token's own input (ident, fp32 or the activation dtype).
+// grid = (tokens, runs of 1024 columns): a thread owns V neighbouring columns (V = 4 where the rows allow 16-byte accesses).
+template <typename TI, int V>
+__global__ void __launch_bounds__(256)
+moe_combine_kernel(float* __restrict__ x, const float* __restrict__ down, const int32_t* __restrict__ slot_of_pair,
+                   const int32_t* __restrict__ top_idx, const float* __restrict__ top_w, int top, int width, int E,
+                   const TI* __restrict__ ident, int accumulate) {
+  const int t = blockIdx.x, d = (blockIdx.y * 256 + threadIdx.x) * V;
+  if (d >= width) return;
+  float acc[V] = {};
+  for (int j = 0; j < top; ++j) {
+    const size_t p = static_cast<size_t>(t) * top + j;
+    float row[V];
+    if (ident && top_idx[p] >= E) {
+#pragma unroll
+      for (int i = 0; i < V; ++i) row[i] = ld(ident + static_cast<size_t>(t) * width + d + i);
+    } else {
+      const float* src = down + static_cast<size_t>(slot_of_pair[p]) * width + d;
+      if constexpr (V == 4) {
+        const float4 v = *reinterpret_cast<const float4*>(src);
+        row[0] = v.x; row[1] = v.y; row[2] = v.z; row[3] = v.w;
+      } else {
+        row[0] = src[0];
+      }
     }
-    float* o = x + static_cast<size_t>(t) * width + d;
-    *o = accumulate ? *o + acc : acc;
+    const float w = top_w[p];
+#pragma unroll
+    for (int i = 0; i < V; ++i) acc[i] += w * row[i];
+  }
+  float* o = x + static_cast<size_t>(t) * width + d;
+  if constexpr (V == 4) {
+    float4 v = accumulate ? *reinterpret_cast<const float4*>(o) : make_float4(0.f, 0.f, 0.f, 0.f);
+    v.x += acc[0]; v.y += acc[1]; v.z += acc[2]; v.w += acc[3];
+    *reinterpret_cast<float4*>(o) = v;
+  } else {
+    o[0] = accumulate ? o[0] + acc[0] : acc[0];
   }
 }
 
@@ -449,6 +480,8 @@ static void grouped_linear(void* out, const void* a, const void* w, const int32_
   if (dt) {
     grouped_linear_fma_kernel<float, ACT><<<dim3(tiles, (N + TN - 1) / TN), 256, 0, st_>>>(
         out, (const float*)a, (const float*)w, off, pair_of_slot, top, E, K, N, act);
+  } else if (use_mma() && grouped_linear_tc(ACT, out, a, w, off, pair_of_slot, pairs, top, E, K, N, act, st_)) {
+    return;
   } else if (use_mma()) {
     grouped_linear_mma_kernel<ACT><<<dim3(tiles, (N + MN - 1) / MN), 128, 0, st_>>>(
         out, (const __nv_bfloat16*)a, (const __nv_bfloat16*)w, off, pair_of_slot, top, E, K, N, act);
@@ -477,12 +510,15 @@ void launch_moe_combine(float* x, const float* down, const int32_t* slot_of_pair
                         const float* top_w, int T, int top, int width, int E, const void* ident, int ident_f32, int dt,
                         int accumulate, cudaStream_t st_) {
   if (T <= 0) return;
+  const bool vec = width % 4 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(down)) & 15) == 0;
+  const dim3 grid(T, (width + (vec ? 1024 : 256) - 1) / (vec ? 1024 : 256));
+  auto run = [&](auto kern, auto* id) {
+    kern<<<grid, 256, 0, st_>>>(x, down, slot_of_pair, top_idx, top_w, top, width, E, id, accumulate);
+  };
   if (!ident || ident_f32 || dt)
-    moe_combine_kernel<float><<<T, 256, 0, st_>>>(x, down, slot_of_pair, top_idx, top_w, top, width, E,
-                                                  (const float*)ident, accumulate);
+    run(vec ? moe_combine_kernel<float, 4> : moe_combine_kernel<float, 1>, (const float*)ident);
   else
-    moe_combine_kernel<__nv_bfloat16><<<T, 256, 0, st_>>>(x, down, slot_of_pair, top_idx, top_w, top, width, E,
-                                                          (const __nv_bfloat16*)ident, accumulate);
+    run(vec ? moe_combine_kernel<__nv_bfloat16, 4> : moe_combine_kernel<__nv_bfloat16, 1>, (const __nv_bfloat16*)ident);
   B200_CUDA_LAUNCH_CHECK();
 }
 

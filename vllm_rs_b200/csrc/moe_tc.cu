@@ -1,0 +1,317 @@
+// The grouped matrix products of routed experts on tcgen05 tensor cores (bf16 operands, fp32 accumulation; moe.cu has the
+// formulas, the buckets and the fp32 / odd-size forms).
+//
+// Persistent blocks, one per SM, walk tiles of 128 slots (rows of ONE expert's bucket) x BN weight rows.  Warp 0 fetches
+// 64-wide K blocks: the weights by TMA boxes, the slots' token rows by TMA gathers of four rows each (an ungathered operand by
+// one box), only as many rows as the bucket has.  Warp 1 issues the products into one of two TMEM accumulators, warps 2-5
+// apply the activation and store under the products of the next tile.  A gated tile holds BN / 2 gate and BN / 2 up rows of
+// the same features side by side, so the activation needs no second pass.
+//
+// Bound: tensor cores where experts get hundreds of rows, HBM (every hit expert's weights once) where they get few; BN is the
+// largest of 256 / 128 / 64 that gives every SM two tiles (fewer tiles leave SMs without weights to fetch).
+#include "../../include/b200_vllm.h"
+#include "moe_tc.cuh"
+
+namespace b200 {
+using namespace seqmix;
+namespace moetc {
+
+constexpr int kM = 128, kK = 64, kThreads = 192, kMaxExperts = 1024;
+constexpr int kABytes = kM * 128;
+constexpr uint32_t kHiSw128 = (1024 >> 4) | (1u << 14) | (2u << 29);
+
+template <int BN> struct Cfg {
+  static constexpr int kStage = kABytes + BN * 128;
+  static constexpr int kStages = 192 * 1024 / kStage;          // 4 / 6 / 8
+  static constexpr int kBarOff = kStages * kStage;
+  static constexpr int kSmem = kBarOff + (2 * kStages + 5) * 8 + 16 + (kMaxExperts + 1) * 4 + 1024;
+};
+
+struct Args {
+  void* out;
+  const int32_t *off, *pair_of_slot;
+  int top, E, KB, N, ntiles_n;          // KB: K blocks; N: output features; ntiles_n: tiles along them
+  b200_expert_act act;
+  int* err;
+};
+
+__device__ __forceinline__ void tma_gather4(void* dst, const CUtensorMap* m, uint64_t* bar, int col, int r0, int r1, int r2, int r3) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cta.global.tile::gather4.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
+      ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)), "r"(col), "r"(r0), "r"(r1), "r"(r2), "r"(r3)
+      : "memory");
+}
+__device__ __forceinline__ void mma_ss(uint32_t lead, uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t acc) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"
+      "setp.ne.b32 q, %0, 0;\n\tsetp.ne.b32 p, %6, 0;\n\t"
+      "mov.b64 da, {%2, %5};\n\tmov.b64 db, {%3, %5};\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%1], da, db, %4, p;\n\t}\n" ::"r"(lead),
+      "r"(d), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(kHiSw128), "r"(acc)
+      : "memory");
+}
+__device__ __forceinline__ void commit(uint32_t lead, uint64_t* bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %0, 0;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%1];\n\t}\n" ::"r"(lead),
+      "r"(smem_u32(bar))
+      : "memory");
+}
+
+// ACT as in moe.cu: 0 plain product of slot rows, fp32 out; 1 SiLU gate, 2 squared ReLU, 3 clamped gate: gathered token rows,
+// bf16 out.  After a wait has given up (*fail) all others return at once and the loops run out.
+template <int ACT, int BN>
+__global__ void __launch_bounds__(kThreads, 1)
+grouped_linear_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap wmap, const Args a) {
+  constexpr bool GATED = ACT == 1 || ACT == 3, GATHER = ACT != 0;
+  constexpr int FN = GATED ? BN / 2 : BN;          // output features of a tile
+  using C = Cfg<BN>;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + C::kBarOff);
+  uint64_t* empty = full + C::kStages;
+  uint64_t* tfull = empty + C::kStages;            // [2] accumulator complete
+  uint64_t* tempty = tfull + 2;                    // [2] accumulator stored
+  uint64_t* drained = tempty + 2;
+  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(drained + 1);
+  volatile int* fail = reinterpret_cast<volatile int*>(tmem_ptr + 1);
+  int* first = reinterpret_cast<int*>(tmem_ptr + 4);         // [E + 1] first row tile of every expert
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < C::kStages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+    for (int s = 0; s < 2; ++s) { mbar_init(&tfull[s], 1); mbar_init(&tempty[s], 4); }
+    mbar_init(drained, 1);
+    *fail = 0;
+    fence_barrier_init();
+    prefetch_tmap(&amap);
+    prefetch_tmap(&wmap);
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_ptr, 2 * BN);
+    tmem_relinquish();
+  }
+  if (warp == 2) {                                 // row tiles before every expert: a scan over the buckets' sizes
+    int before = 0;
+    for (int e0 = 0; e0 < a.E; e0 += 32) {
+      const int e = e0 + lane;
+      const int mine = e < a.E ? (a.off[e + 1] - a.off[e] + kM - 1) / kM : 0;
+      int inc = mine;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += v;
+      }
+      if (e < a.E) first[e] = before + inc - mine;
+      before += __shfl_sync(0xffffffffu, inc, 31);
+    }
+    if (lane == 0) first[a.E] = before;
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_ptr, 0);
+  const int ntiles = first[a.E] * a.ntiles_n;
+  // tile -> expert, first slot, rows, first feature
+  struct Tile { int e, s0, rows, n0; };
+  auto tile_at = [&](int t) {
+    const int m = t / a.ntiles_n;
+    int lo = 0, hi = a.E - 1;                      // the last expert whose first tile is <= m (empty ones share their successor's)
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (first[mid] <= m) lo = mid; else hi = mid - 1;
+    }
+    const int b = a.off[lo], k = m - first[lo];
+    return Tile{lo, b + k * kM, min(kM, a.off[lo + 1] - b - k * kM), (t - m * a.ntiles_n) * FN};
+  };
+
+  if (warp == 0) {
+    // ------------------------------------------------------------ operands
+    int s = 0, armed = 0;
+    uint32_t ph = 0;
+    bool free_ = true;
+    for (int t = blockIdx.x; t < ntiles && free_; t += gridDim.x) {
+      const Tile w = tile_at(t);
+      int r[4] = {0, 0, 0, 0};
+      const int quads = (w.rows + 3) >> 2;
+      if (GATHER) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) r[i] = a.pair_of_slot[w.s0 + min(lane * 4 + i, w.rows - 1)] / a.top;
+      }
+      const uint32_t bytes = (GATHER ? quads * 512 : kABytes) + BN * 128;
+      const int wrow = w.e * (GATED ? 2 : 1) * a.N + w.n0;
+      for (int kb = 0; kb < a.KB; ++kb) {
+        free_ = __all_sync(0xffffffffu, mbar_wait_limited(&empty[s], ph ^ 1, fail, a.err));
+        if (!free_) break;                         // a stage that did not come free is not armed again
+        uint8_t* ad = smem + s * C::kStage;
+        uint8_t* wd = ad + kABytes;
+        if (lane == 0) {
+          mbar_arrive_expect_tx(&full[s], bytes);
+          if (GATED) {
+            tma_load_2d(wd, &wmap, &full[s], kb * kK, wrow);
+            tma_load_2d(wd + FN * 128, &wmap, &full[s], kb * kK, wrow + a.N);
+          } else {
+            tma_load_2d(wd, &wmap, &full[s], kb * kK, wrow);
+          }
+          if (!GATHER) tma_load_2d(ad, &amap, &full[s], kb * kK, w.s0);
+        }
+        __syncwarp();
+        if (GATHER && lane < quads) tma_gather4(ad + lane * 512, &amap, &full[s], kb * kK, r[0], r[1], r[2], r[3]);
+        ++armed;
+        if (++s == C::kStages) { s = 0; ph ^= 1; }
+      }
+    }
+    if (lane == 0 && *fail)                        // copies in flight land before the block ends
+      for (int i = 0; i < C::kStages && i < armed; ++i)
+        mbar_wait_limited(&full[i], ((armed - 1 - i) / C::kStages) & 1, nullptr, a.err);
+    __syncwarp();
+  } else if (warp == 1) {
+    // ------------------------------------------------------------ products
+    constexpr uint32_t idesc = make_idesc_f16(kM, BN) | (1u << 7) | (1u << 10);        // bf16 operands
+    const uint32_t lead = elect_one() ? 1u : 0u;
+    const uint32_t base = (smem_u32(smem) >> 4) | (1u << 16);
+    int s = 0, it = 0;
+    uint32_t ph = 0;
+    for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++it) {
+      const int buf = it & 1;
+      mbar_wait_limited(&tempty[buf], ((it >> 1) & 1) ^ 1, fail, a.err);
+      tc_fence_after();
+      const uint32_t d = tmem + buf * BN;
+      for (int kb = 0; kb < a.KB; ++kb) {
+        mbar_wait_limited(&full[s], ph, fail, a.err);
+        tc_fence_after();
+        const uint32_t a_lo = base + s * (C::kStage >> 4), b_lo = a_lo + (kABytes >> 4);
+#pragma unroll
+        for (int ks = 0; ks < kK / 16; ++ks) mma_ss(lead, d, a_lo + ks * 2, b_lo + ks * 2, idesc, (kb | ks) ? 1u : 0u);
+        commit(lead, &empty[s]);
+        if (++s == C::kStages) { s = 0; ph ^= 1; }
+      }
+      commit(lead, &tfull[buf]);
+    }
+    if (*fail) {                                   // products in flight end before TMEM is given back
+      commit(lead, drained);
+      mbar_wait_limited(drained, 0, nullptr, a.err);
+    }
+    __syncwarp();
+  } else {
+    // ------------------------------------------------------------ activation and stores: a thread per row
+    const int q4 = warp & 3, r = q4 * 32 + lane;
+    const uint32_t lanes = static_cast<uint32_t>(q4 * 32) << 16;
+    int it = 0;
+    for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++it) {
+      const Tile w = tile_at(t);
+      const int buf = it & 1;
+      mbar_wait_limited(&tfull[buf], (it >> 1) & 1, fail, a.err);
+      __syncwarp();
+      tc_fence_after();
+      const uint32_t src = tmem + lanes + buf * BN;
+      const bool mine = r < w.rows;
+      const size_t o = static_cast<size_t>(w.s0 + r) * a.N + w.n0;
+      if (q4 * 32 < w.rows) {
+#pragma unroll 1
+        for (int c = 0; c < FN; c += 32) {
+          uint32_t v[32], u[GATED ? 32 : 1];
+          tmem_ld_x32(src + c, v);
+          if constexpr (GATED) tmem_ld_x32(src + FN + c, u);
+          tc_wait_ld();
+          if (mine) {
+            if constexpr (ACT == 0) {
+              float* dst = reinterpret_cast<float*>(a.out) + o + c;
+#pragma unroll
+              for (int i = 0; i < 32; i += 4)
+                if (w.n0 + c + i < a.N) *reinterpret_cast<uint4*>(dst + i) = make_uint4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+            } else {
+#pragma unroll
+              for (int i = 0; i < 32; ++i) {
+                float x = __uint_as_float(v[i]);
+                if constexpr (GATED) {
+                  x = expert_gate<ACT>(x, __uint_as_float(u[i]), a.act);
+                } else {
+                  x = fmaxf(x, 0.f);
+                  x *= x;
+                }
+                v[i] = __float_as_uint(x);
+              }
+              __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(a.out) + o + c;
+#pragma unroll
+              for (int i = 0; i < 32; i += 8)
+                if (w.n0 + c + i < a.N)
+                  *reinterpret_cast<uint4*>(dst + i) =
+                      make_uint4(pack16x2<true>(__uint_as_float(v[i]), __uint_as_float(v[i + 1])),
+                                 pack16x2<true>(__uint_as_float(v[i + 2]), __uint_as_float(v[i + 3])),
+                                 pack16x2<true>(__uint_as_float(v[i + 4]), __uint_as_float(v[i + 5])),
+                                 pack16x2<true>(__uint_as_float(v[i + 6]), __uint_as_float(v[i + 7])));
+            }
+          }
+          __syncwarp();
+        }
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&tempty[buf]);
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem, 2 * BN);
+  }
+}
+
+static bool map_2d(CUtensorMap* m, const void* base, uint64_t rows, int K, uint32_t box_rows) {
+  const uint64_t dims[2] = {static_cast<uint64_t>(K), rows}, strides[1] = {static_cast<uint64_t>(K) * 2};
+  const uint32_t box[2] = {kK, box_rows}, es[2] = {1, 1};
+  return encode_tensor_map(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, es,
+                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B) == CUDA_SUCCESS;
+}
+
+template <int ACT, int BN>
+static void launch(void* out, const void* a, const void* w, const int32_t* off, const int32_t* pair_of_slot, int pairs, int top,
+                   int E, int K, int N, const b200_expert_act& act, cudaStream_t st) {
+  constexpr bool GATED = ACT == 1 || ACT == 3;
+  constexpr int FN = GATED ? BN / 2 : BN;
+  Args g{out, off, pair_of_slot, top, E, (K + kK - 1) / kK, N, (N + FN - 1) / FN, act, wait_error_flag()};
+  CUtensorMap amap, wmap;
+  const bool ok = map_2d(&amap, a, ACT ? pairs / top : pairs, K, ACT ? 1 : kM) &&
+                  map_2d(&wmap, w, static_cast<uint64_t>(E) * (GATED ? 2 : 1) * N, K, FN);
+  if (!ok || !g.err) {
+    set_error(2, "grouped_linear_tc: cuTensorMapEncodeTiled failed");
+    return;
+  }
+  auto kern = grouped_linear_tc_kernel<ACT, BN>;
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BN>::kSmem);
+  const int most = std::min(pairs, E + pairs / kM) * g.ntiles_n;        // no step has more tiles
+  kern<<<std::min(most, sm_count()), kThreads, Cfg<BN>::kSmem, st>>>(amap, wmap, g);
+  B200_CUDA_LAUNCH_CHECK();
+}
+
+template <int ACT>
+static void launch_bn(void* out, const void* a, const void* w, const int32_t* off, const int32_t* pair_of_slot, int pairs,
+                      int top, int E, int K, int N, const b200_expert_act& act, cudaStream_t st) {
+  constexpr int G = ACT == 1 || ACT == 3 ? 2 : 1;
+  const int row_tiles = std::max(std::min(E, pairs), pairs / kM);
+  const int want = 2 * sm_count();
+  if (row_tiles * ((N * G + 255) / 256) >= want) launch<ACT, 256>(out, a, w, off, pair_of_slot, pairs, top, E, K, N, act, st);
+  else if (row_tiles * ((N * G + 127) / 128) >= want) launch<ACT, 128>(out, a, w, off, pair_of_slot, pairs, top, E, K, N, act, st);
+  else launch<ACT, 64>(out, a, w, off, pair_of_slot, pairs, top, E, K, N, act, st);
+}
+
+}  // namespace moetc
+
+bool grouped_linear_tc(int act_kind, void* out, const void* a, const void* w, const int32_t* off, const int32_t* pair_of_slot,
+                       int pairs, int top, int E, int K, int N, const b200_expert_act& act, cudaStream_t st) {
+  using namespace moetc;
+  const uintptr_t ptrs = reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w);
+  if (K % 8 != 0 || N % 8 != 0 || E > kMaxExperts || (ptrs & 15)) return false;
+  switch (act_kind) {
+    case 0: launch_bn<0>(out, a, w, off, pair_of_slot, pairs, top, E, K, N, act, st); break;
+    case 1: launch_bn<1>(out, a, w, off, pair_of_slot, pairs, top, E, K, N, act, st); break;
+    case 2: launch_bn<2>(out, a, w, off, pair_of_slot, pairs, top, E, K, N, act, st); break;
+    default: launch_bn<3>(out, a, w, off, pair_of_slot, pairs, top, E, K, N, act, st); break;
+  }
+  return true;
+}
+
+}  // namespace b200
