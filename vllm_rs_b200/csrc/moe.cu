@@ -120,20 +120,45 @@ __global__ void moe_route_kernel(const float* __restrict__ logits, const float* 
     for (int j = lane; j < top; j += 32) top_w[static_cast<size_t>(t) * top + j] /= total + (score == 2 ? 0.f : 1e-20f);
 }
 
+// The lanes of `act` that hold the same number below 2^bits: a vote per bit (match.any took longer than the atomics that it
+// saves).  The whole warp takes part.
+__device__ __forceinline__ unsigned same_lanes(unsigned act, int v, int bits) {
+  unsigned m = act;
+  for (int i = 0; i < bits; ++i) {
+    const unsigned b = __ballot_sync(0xffffffffu, (v >> i) & 1);
+    m &= ((v >> i) & 1) ? b : ~b;
+  }
+  return m;
+}
 // Single block: histogram, exclusive scan, scatter.  Lanes with the same expert count as one: thousands of pairs meet on few
-// counters (16384 pairs of 16 experts, 14.5 us with an atomic per pair).
+// counters (16384 pairs of 16 experts: 14.5 us with an atomic per pair).
 __global__ void __launch_bounds__(1024)
 moe_sort_kernel(const int32_t* __restrict__ top_idx, int pairs, int E, int32_t* __restrict__ expert_off,
                 int32_t* __restrict__ pair_of_slot, int32_t* __restrict__ slot_of_pair) {
   extern __shared__ int cnt[];       // [E] counts, then cursors
-  const int lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, bits = 32 - __clz(E - 1 | 1);
   for (int e = threadIdx.x; e < E; e += blockDim.x) cnt[e] = 0;
   __syncthreads();
-  for (int p = threadIdx.x; p < pairs; p += blockDim.x) {
-    const unsigned act = __activemask();
-    const int e = top_idx[p];
-    const unsigned same = __match_any_sync(act, e);
-    if (lane == __ffs(same) - 1) atomicAdd(&cnt[e], __popc(same));
+  // every thread reads kBatch choices at a time (the loads are what a round waits for); -1 past the last one
+  constexpr int kBatch = 8;
+  auto batch = [&](int p0, int (&e)[kBatch]) {
+#pragma unroll
+    for (int i = 0; i < kBatch; ++i) {
+      const int p = p0 + i * blockDim.x + threadIdx.x;
+      e[i] = p < pairs ? top_idx[p] : -1;
+    }
+  };
+  const int step = kBatch * blockDim.x;
+  for (int p0 = 0; p0 < pairs; p0 += step) {
+    int e[kBatch];
+    batch(p0, e);
+#pragma unroll
+    for (int i = 0; i < kBatch; ++i) {
+      if (p0 + i * blockDim.x >= pairs) break;
+      const unsigned act = __ballot_sync(0xffffffffu, e[i] >= 0);
+      const unsigned same = same_lanes(act, e[i], bits);
+      if (e[i] >= 0 && lane == __ffs(same) - 1) atomicAdd(&cnt[e[i]], __popc(same));
+    }
   }
   __syncthreads();
   if (threadIdx.x < 32) {            // one warp scans the counts, 32 at a time
@@ -152,16 +177,24 @@ moe_sort_kernel(const int32_t* __restrict__ top_idx, int pairs, int E, int32_t* 
     if (lane == 0) expert_off[E] = run;
   }
   __syncthreads();
-  for (int p = threadIdx.x; p < pairs; p += blockDim.x) {
-    const unsigned act = __activemask();
-    const int e = top_idx[p];
-    const unsigned same = __match_any_sync(act, e);
-    const int head = __ffs(same) - 1;
-    int slot = 0;
-    if (lane == head) slot = atomicAdd(&cnt[e], __popc(same));
-    slot = __shfl_sync(act, slot, head) + __popc(same & ((1u << lane) - 1));
-    pair_of_slot[slot] = p;
-    slot_of_pair[p] = slot;
+  for (int p0 = 0; p0 < pairs; p0 += step) {
+    int e[kBatch];
+    batch(p0, e);
+#pragma unroll
+    for (int i = 0; i < kBatch; ++i) {
+      if (p0 + i * blockDim.x >= pairs) break;
+      const unsigned act = __ballot_sync(0xffffffffu, e[i] >= 0);
+      const unsigned same = same_lanes(act, e[i], bits);
+      const int head = max(__ffs(same) - 1, 0);
+      int slot = 0;
+      if (e[i] >= 0 && lane == head) slot = atomicAdd(&cnt[e[i]], __popc(same));
+      slot = __shfl_sync(0xffffffffu, slot, head) + __popc(same & ((1u << lane) - 1));
+      if (e[i] >= 0) {
+        const int p = p0 + i * blockDim.x + threadIdx.x;
+        pair_of_slot[slot] = p;
+        slot_of_pair[p] = slot;
+      }
+    }
   }
 }
 
@@ -473,14 +506,14 @@ static bool use_mma() {
 
 template <int ACT>
 static void grouped_linear(void* out, const void* a, const void* w, const int32_t* off, const int32_t* pair_of_slot,
-                           int pairs, int top, int E, int K, int N, int dt, cudaStream_t st_,
+                           void* rows, int pairs, int top, int E, int K, int N, int dt, cudaStream_t st_,
                            const b200_expert_act& act = b200_expert_act{}) {
   if (pairs <= 0) return;
   const int tiles = (pairs + TM - 1) / TM + E;
   if (dt) {
     grouped_linear_fma_kernel<float, ACT><<<dim3(tiles, (N + TN - 1) / TN), 256, 0, st_>>>(
         out, (const float*)a, (const float*)w, off, pair_of_slot, top, E, K, N, act);
-  } else if (use_mma() && grouped_linear_tc(ACT, out, a, w, off, pair_of_slot, pairs, top, E, K, N, act, st_)) {
+  } else if (use_mma() && grouped_linear_tc(ACT, out, a, w, off, pair_of_slot, rows, pairs, top, E, K, N, act, st_)) {
     return;
   } else if (use_mma()) {
     grouped_linear_mma_kernel<ACT><<<dim3(tiles, (N + MN - 1) / MN), 128, 0, st_>>>(
@@ -493,18 +526,18 @@ static void grouped_linear(void* out, const void* a, const void* w, const int32_
 }
 
 void launch_moe_gate_up(void* act_out, const void* h, const void* w_up, const int32_t* expert_off,
-                        const int32_t* pair_of_slot, int pairs, int top, int E, int width, int ff,
+                        const int32_t* pair_of_slot, void* rows, int pairs, int top, int E, int width, int ff,
                         const b200_expert_act& act, int dt, cudaStream_t st_) {
   if (act.kind == B200_EXPERT_SILU)
-    grouped_linear<1>(act_out, h, w_up, expert_off, pair_of_slot, pairs, top, E, width, ff, dt, st_);
+    grouped_linear<1>(act_out, h, w_up, expert_off, pair_of_slot, rows, pairs, top, E, width, ff, dt, st_);
   else if (act.kind == B200_EXPERT_CLAMPED)
-    grouped_linear<3>(act_out, h, w_up, expert_off, pair_of_slot, pairs, top, E, width, ff, dt, st_, act);
+    grouped_linear<3>(act_out, h, w_up, expert_off, pair_of_slot, rows, pairs, top, E, width, ff, dt, st_, act);
   else
-    grouped_linear<2>(act_out, h, w_up, expert_off, pair_of_slot, pairs, top, E, width, ff, dt, st_);
+    grouped_linear<2>(act_out, h, w_up, expert_off, pair_of_slot, rows, pairs, top, E, width, ff, dt, st_);
 }
 void launch_moe_down(float* out, const void* act, const void* w_down, const int32_t* expert_off, int pairs, int E,
                      int width, int ff, int dt, cudaStream_t st_) {
-  grouped_linear<0>(out, act, w_down, expert_off, nullptr, pairs, 1, E, ff, width, dt, st_);
+  grouped_linear<0>(out, act, w_down, expert_off, nullptr, nullptr, pairs, 1, E, ff, width, dt, st_);
 }
 void launch_moe_combine(float* x, const float* down, const int32_t* slot_of_pair, const int32_t* top_idx,
                         const float* top_w, int T, int top, int width, int E, const void* ident, int ident_f32, int dt,
@@ -568,7 +601,7 @@ static void moe_expert_rows(const void* h, const int32_t* top_idx, const void* w
   float* down = reinterpret_cast<float*>(p);
   // identity experts take buckets past the real ones; the grouped products walk the first `experts` buckets only
   launch_moe_sort(top_idx, P, all, off, pos, sop, st_);
-  launch_moe_gate_up(actb, h, w_up, off, pos, P, top, experts, width, ff, act, dt, st_);
+  launch_moe_gate_up(actb, h, w_up, off, pos, down, P, top, experts, width, ff, act, dt, st_);
   launch_moe_down(down, actb, w_down, off, P, experts, width, ff, dt, st_);
   *down_out = down;
   *slot_out = sop;

@@ -1,11 +1,14 @@
 // The grouped matrix products of routed experts on tcgen05 tensor cores (bf16 operands, fp32 accumulation; moe.cu has the
 // formulas, the buckets and the fp32 / odd-size forms).
 //
-// Persistent blocks, one per SM, walk tiles of 128 slots (rows of ONE expert's bucket) x BN weight rows.  Warp 0 fetches
-// 64-wide K blocks: the weights by TMA boxes, the slots' token rows by TMA gathers of four rows each (an ungathered operand by
-// one box), only as many rows as the bucket has.  Warp 1 issues the products into one of two TMEM accumulators, warps 2-5
-// apply the activation and store under the products of the next tile.  A gated tile holds BN / 2 gate and BN / 2 up rows of
-// the same features side by side, so the activation needs no second pass.
+// Persistent blocks, one per SM, walk tiles of 128 slots (rows of ONE expert's bucket) x BN weight rows.  Warp 0 fetches 64-wide
+// K blocks of both operands by TMA, of the rows only as many 32-row boxes as the bucket has.  Warp 1 issues the products into
+// one of two TMEM accumulators, warps 2-9 apply the activation and store, through shared memory so that rows leave in whole
+// sectors, under the products of the next tile.  A gated tile holds BN / 2 gate and BN / 2 up rows of the same features side by
+// side, so the activation needs no second pass.  Token rows are first gathered into bucket order by a copy of their own (in
+// space that the second product's results take later): gathering inside the product took longer than the product, by TMA
+// gathers of four rows (~90 cycles each) as by cp.async, whose blocks need a wait and a fence on their way to the tensor core
+// (prompt of 4096 rows, 16 experts, first product: 183 us and 103-139 us).
 //
 // Bound: tensor cores where experts get hundreds of rows, HBM (every hit expert's weights once) where they get few; BN is the
 // largest of 256 / 128 / 64 that gives every SM two tiles (fewer tiles leave SMs without weights to fetch).
@@ -16,32 +19,27 @@ namespace b200 {
 using namespace seqmix;
 namespace moetc {
 
-constexpr int kM = 128, kK = 64, kThreads = 192, kMaxExperts = 1024;
+constexpr int kM = 128, kK = 64, kBox = 32, kThreads = 320, kEpiWarps = 8, kMaxExperts = 1024;
 constexpr int kABytes = kM * 128;
+constexpr int kPitch = 80, kOutBytes = kEpiWarps * 32 * kPitch;      // a warp's 32 rows x 64 bytes on their way out
 constexpr uint32_t kHiSw128 = (1024 >> 4) | (1u << 14) | (2u << 29);
 
 template <int BN> struct Cfg {
   static constexpr int kStage = kABytes + BN * 128;
   static constexpr int kStages = 192 * 1024 / kStage;          // 4 / 6 / 8
-  static constexpr int kBarOff = kStages * kStage;
+  static constexpr int kOutOff = kStages * kStage;
+  static constexpr int kBarOff = kOutOff + kOutBytes;
   static constexpr int kSmem = kBarOff + (2 * kStages + 5) * 8 + 16 + (kMaxExperts + 1) * 4 + 1024;
 };
 
 struct Args {
   void* out;
-  const int32_t *off, *pair_of_slot;
-  int top, E, KB, N, ntiles_n;          // KB: K blocks; N: output features; ntiles_n: tiles along them
+  const int32_t* off;
+  int E, KB, N, ntiles_n;          // KB: K blocks; N: output features; ntiles_n: tiles along them
   b200_expert_act act;
   int* err;
 };
 
-__device__ __forceinline__ void tma_gather4(void* dst, const CUtensorMap* m, uint64_t* bar, int col, int r0, int r1, int r2, int r3) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cta.global.tile::gather4.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
-      ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)), "r"(col), "r"(r0), "r"(r1), "r"(r2), "r"(r3)
-      : "memory");
-}
 __device__ __forceinline__ void mma_ss(uint32_t lead, uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t acc) {
   asm volatile(
       "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"
@@ -59,12 +57,11 @@ __device__ __forceinline__ void commit(uint32_t lead, uint64_t* bar) {
       : "memory");
 }
 
-// ACT as in moe.cu: 0 plain product of slot rows, fp32 out; 1 SiLU gate, 2 squared ReLU, 3 clamped gate: gathered token rows,
-// bf16 out.  After a wait has given up (*fail) all others return at once and the loops run out.
+// ACT as in moe.cu: 0 plain product, fp32 out; 1 SiLU gate, 2 squared ReLU, 3 clamped gate, bf16 out.  Rows in bucket order.  After a wait has given up (*fail) all others return at once and the loops run out.
 template <int ACT, int BN>
 __global__ void __launch_bounds__(kThreads, 1)
 grouped_linear_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap wmap, const Args a) {
-  constexpr bool GATED = ACT == 1 || ACT == 3, GATHER = ACT != 0;
+  constexpr bool GATED = ACT == 1 || ACT == 3;
   constexpr int FN = GATED ? BN / 2 : BN;          // output features of a tile
   using C = Cfg<BN>;
   extern __shared__ uint8_t smem_raw[];
@@ -81,7 +78,7 @@ grouped_linear_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::kStages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-    for (int s = 0; s < 2; ++s) { mbar_init(&tfull[s], 1); mbar_init(&tempty[s], 4); }
+    for (int s = 0; s < 2; ++s) { mbar_init(&tfull[s], 1); mbar_init(&tempty[s], kEpiWarps); }
     mbar_init(drained, 1);
     *fail = 0;
     fence_barrier_init();
@@ -133,13 +130,7 @@ grouped_linear_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_
     bool free_ = true;
     for (int t = blockIdx.x; t < ntiles && free_; t += gridDim.x) {
       const Tile w = tile_at(t);
-      int r[4] = {0, 0, 0, 0};
-      const int quads = (w.rows + 3) >> 2;
-      if (GATHER) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) r[i] = a.pair_of_slot[w.s0 + min(lane * 4 + i, w.rows - 1)] / a.top;
-      }
-      const uint32_t bytes = (GATHER ? quads * 512 : kABytes) + BN * 128;
+      const int boxes = (w.rows + kBox - 1) / kBox;
       const int wrow = w.e * (GATED ? 2 : 1) * a.N + w.n0;
       for (int kb = 0; kb < a.KB; ++kb) {
         free_ = __all_sync(0xffffffffu, mbar_wait_limited(&empty[s], ph ^ 1, fail, a.err));
@@ -147,17 +138,15 @@ grouped_linear_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_
         uint8_t* ad = smem + s * C::kStage;
         uint8_t* wd = ad + kABytes;
         if (lane == 0) {
-          mbar_arrive_expect_tx(&full[s], bytes);
+          mbar_arrive_expect_tx(&full[s], boxes * (kBox * 128) + BN * 128);
           if (GATED) {
             tma_load_2d(wd, &wmap, &full[s], kb * kK, wrow);
             tma_load_2d(wd + FN * 128, &wmap, &full[s], kb * kK, wrow + a.N);
           } else {
             tma_load_2d(wd, &wmap, &full[s], kb * kK, wrow);
           }
-          if (!GATHER) tma_load_2d(ad, &amap, &full[s], kb * kK, w.s0);
+          for (int i = 0; i < boxes; ++i) tma_load_2d(ad + i * (kBox * 128), &amap, &full[s], kb * kK, w.s0 + i * kBox);
         }
-        __syncwarp();
-        if (GATHER && lane < quads) tma_gather4(ad + lane * 512, &amap, &full[s], kb * kK, r[0], r[1], r[2], r[3]);
         ++armed;
         if (++s == C::kStages) { s = 0; ph ^= 1; }
       }
@@ -195,9 +184,12 @@ grouped_linear_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_
     }
     __syncwarp();
   } else {
-    // ------------------------------------------------------------ activation and stores: a thread per row
-    const int q4 = warp & 3, r = q4 * 32 + lane;
+    // ------------------------------------------------------------ activation and stores
+    // A warp reads its quarter of the rows, every other 32 columns; four lanes then write 64 bytes of a row.
+    const int q4 = warp & 3;
     const uint32_t lanes = static_cast<uint32_t>(q4 * 32) << 16;
+    uint8_t* stage = smem + C::kOutOff + (warp - 2) * 32 * kPitch;
+    const int sub = (lane & 3) * 16;
     int it = 0;
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++it) {
       const Tile w = tile_at(t);
@@ -206,45 +198,59 @@ grouped_linear_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_
       __syncwarp();
       tc_fence_after();
       const uint32_t src = tmem + lanes + buf * BN;
-      const bool mine = r < w.rows;
-      const size_t o = static_cast<size_t>(w.s0 + r) * a.N + w.n0;
-      if (q4 * 32 < w.rows) {
+      const int rows = w.rows - q4 * 32;               // of this warp
+      // the staged rows' bytes [b, b + 64) of a tile row whose first column is n0
+      auto store = [&](int b, int elem) {
+        __syncwarp();
+        uint8_t* dst = static_cast<uint8_t*>(a.out) + (static_cast<size_t>(w.s0 + q4 * 32) * a.N + w.n0) * elem + b + sub;
+        if (w.n0 * elem + b + sub < a.N * elem) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int rw = i * 8 + (lane >> 2);
+            if (rw < rows)
+              *reinterpret_cast<uint4*>(dst + static_cast<size_t>(rw) * a.N * elem) =
+                  *reinterpret_cast<const uint4*>(stage + rw * kPitch + sub);
+          }
+        }
+        __syncwarp();
+      };
+      if (rows > 0) {
 #pragma unroll 1
-        for (int c = 0; c < FN; c += 32) {
+        for (int c = warp < 6 ? 0 : 32; c < FN; c += 64) {
           uint32_t v[32], u[GATED ? 32 : 1];
           tmem_ld_x32(src + c, v);
           if constexpr (GATED) tmem_ld_x32(src + FN + c, u);
           tc_wait_ld();
-          if (mine) {
-            if constexpr (ACT == 0) {
-              float* dst = reinterpret_cast<float*>(a.out) + o + c;
+          if constexpr (ACT == 0) {
 #pragma unroll
-              for (int i = 0; i < 32; i += 4)
-                if (w.n0 + c + i < a.N) *reinterpret_cast<uint4*>(dst + i) = make_uint4(v[i], v[i + 1], v[i + 2], v[i + 3]);
-            } else {
+            for (int hf = 0; hf < 2; ++hf) {
 #pragma unroll
-              for (int i = 0; i < 32; ++i) {
-                float x = __uint_as_float(v[i]);
-                if constexpr (GATED) {
-                  x = expert_gate<ACT>(x, __uint_as_float(u[i]), a.act);
-                } else {
-                  x = fmaxf(x, 0.f);
-                  x *= x;
-                }
-                v[i] = __float_as_uint(x);
-              }
-              __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(a.out) + o + c;
-#pragma unroll
-              for (int i = 0; i < 32; i += 8)
-                if (w.n0 + c + i < a.N)
-                  *reinterpret_cast<uint4*>(dst + i) =
-                      make_uint4(pack16x2<true>(__uint_as_float(v[i]), __uint_as_float(v[i + 1])),
-                                 pack16x2<true>(__uint_as_float(v[i + 2]), __uint_as_float(v[i + 3])),
-                                 pack16x2<true>(__uint_as_float(v[i + 4]), __uint_as_float(v[i + 5])),
-                                 pack16x2<true>(__uint_as_float(v[i + 6]), __uint_as_float(v[i + 7])));
+              for (int i = 0; i < 16; i += 4)
+                *reinterpret_cast<uint4*>(stage + lane * kPitch + i * 4) =
+                    make_uint4(v[hf * 16 + i], v[hf * 16 + i + 1], v[hf * 16 + i + 2], v[hf * 16 + i + 3]);
+              store((c + hf * 16) * 4, 4);
             }
+          } else {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+              float x = __uint_as_float(v[i]);
+              if constexpr (GATED) {
+                x = expert_gate<ACT>(x, __uint_as_float(u[i]), a.act);
+              } else {
+                x = fmaxf(x, 0.f);
+                x *= x;
+              }
+              v[i] = __float_as_uint(x);
+            }
+#pragma unroll
+            for (int i = 0; i < 32; i += 8)
+              *reinterpret_cast<uint4*>(stage + lane * kPitch + i * 2) =
+                  make_uint4(pack16x2<true>(__uint_as_float(v[i]), __uint_as_float(v[i + 1])),
+                             pack16x2<true>(__uint_as_float(v[i + 2]), __uint_as_float(v[i + 3])),
+                             pack16x2<true>(__uint_as_float(v[i + 4]), __uint_as_float(v[i + 5])),
+                             pack16x2<true>(__uint_as_float(v[i + 6]), __uint_as_float(v[i + 7])));
+            store(c * 2, 2);
           }
-          __syncwarp();
         }
       }
       tc_fence_before();
@@ -267,15 +273,15 @@ static bool map_2d(CUtensorMap* m, const void* base, uint64_t rows, int K, uint3
                            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B) == CUDA_SUCCESS;
 }
 
+// a [pairs, K] in bucket order
 template <int ACT, int BN>
-static void launch(void* out, const void* a, const void* w, const int32_t* off, const int32_t* pair_of_slot, int pairs, int top,
-                   int E, int K, int N, const b200_expert_act& act, cudaStream_t st) {
+static void launch(void* out, const void* a, const void* w, const int32_t* off, int pairs, int E, int K, int N,
+                   const b200_expert_act& act, cudaStream_t st) {
   constexpr bool GATED = ACT == 1 || ACT == 3;
   constexpr int FN = GATED ? BN / 2 : BN;
-  Args g{out, off, pair_of_slot, top, E, (K + kK - 1) / kK, N, (N + FN - 1) / FN, act, wait_error_flag()};
+  Args g{out, off, E, (K + kK - 1) / kK, N, (N + FN - 1) / FN, act, wait_error_flag()};
   CUtensorMap amap, wmap;
-  const bool ok = map_2d(&amap, a, ACT ? pairs / top : pairs, K, ACT ? 1 : kM) &&
-                  map_2d(&wmap, w, static_cast<uint64_t>(E) * (GATED ? 2 : 1) * N, K, FN);
+  const bool ok = map_2d(&amap, a, pairs, K, kBox) && map_2d(&wmap, w, static_cast<uint64_t>(E) * (GATED ? 2 : 1) * N, K, FN);
   if (!ok || !g.err) {
     set_error(2, "grouped_linear_tc: cuTensorMapEncodeTiled failed");
     return;
@@ -288,28 +294,55 @@ static void launch(void* out, const void* a, const void* w, const int32_t* off, 
 }
 
 template <int ACT>
-static void launch_bn(void* out, const void* a, const void* w, const int32_t* off, const int32_t* pair_of_slot, int pairs,
-                      int top, int E, int K, int N, const b200_expert_act& act, cudaStream_t st) {
+static void launch_bn(void* out, const void* a, const void* w, const int32_t* off, int pairs, int E, int K, int N,
+                      const b200_expert_act& act, cudaStream_t st) {
   constexpr int G = ACT == 1 || ACT == 3 ? 2 : 1;
   const int row_tiles = std::max(std::min(E, pairs), pairs / kM);
   const int want = 2 * sm_count();
-  if (row_tiles * ((N * G + 255) / 256) >= want) launch<ACT, 256>(out, a, w, off, pair_of_slot, pairs, top, E, K, N, act, st);
-  else if (row_tiles * ((N * G + 127) / 128) >= want) launch<ACT, 128>(out, a, w, off, pair_of_slot, pairs, top, E, K, N, act, st);
-  else launch<ACT, 64>(out, a, w, off, pair_of_slot, pairs, top, E, K, N, act, st);
+  if (row_tiles * ((N * G + 255) / 256) >= want) launch<ACT, 256>(out, a, w, off, pairs, E, K, N, act, st);
+  else if (row_tiles * ((N * G + 127) / 128) >= want) launch<ACT, 128>(out, a, w, off, pairs, E, K, N, act, st);
+  else launch<ACT, 64>(out, a, w, off, pairs, E, K, N, act, st);
+}
+
+// out[slot] = h[pair_of_slot[slot] / top], rows of n16 16-byte pieces
+__global__ void __launch_bounds__(256)
+bucket_rows_kernel(uint4* __restrict__ out, const uint4* __restrict__ h, const int32_t* __restrict__ pair_of_slot, int pairs,
+                   int top, int n16) {
+  const int per = 256 / 32, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;       // a warp per row
+  const int slot = blockIdx.x * per + warp;
+  if (slot >= pairs) return;
+  const uint4* src = h + static_cast<size_t>(pair_of_slot[slot] / top) * n16;
+  uint4* dst = out + static_cast<size_t>(slot) * n16;
+  for (int i0 = lane; i0 < n16; i0 += 128) {
+    uint4 v[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (i0 + 32 * i < n16) v[i] = __ldg(src + i0 + 32 * i);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (i0 + 32 * i < n16) dst[i0 + 32 * i] = v[i];
+  }
 }
 
 }  // namespace moetc
 
 bool grouped_linear_tc(int act_kind, void* out, const void* a, const void* w, const int32_t* off, const int32_t* pair_of_slot,
-                       int pairs, int top, int E, int K, int N, const b200_expert_act& act, cudaStream_t st) {
+                       void* rows, int pairs, int top, int E, int K, int N, const b200_expert_act& act, cudaStream_t st) {
   using namespace moetc;
-  const uintptr_t ptrs = reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w);
-  if (K % 8 != 0 || N % 8 != 0 || E > kMaxExperts || (ptrs & 15)) return false;
+  const uintptr_t ptrs = reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w) |
+                         reinterpret_cast<uintptr_t>(rows);
+  if (K % 8 != 0 || N % 8 != 0 || E > kMaxExperts || (ptrs & 15) || (act_kind != 0 && !rows)) return false;
+  if (act_kind != 0) {
+    bucket_rows_kernel<<<(pairs + 7) / 8, 256, 0, st>>>(static_cast<uint4*>(rows), static_cast<const uint4*>(a), pair_of_slot,
+                                                        pairs, top, K / 8);
+    B200_CUDA_LAUNCH_CHECK();
+    a = rows;
+  }
   switch (act_kind) {
-    case 0: launch_bn<0>(out, a, w, off, pair_of_slot, pairs, top, E, K, N, act, st); break;
-    case 1: launch_bn<1>(out, a, w, off, pair_of_slot, pairs, top, E, K, N, act, st); break;
-    case 2: launch_bn<2>(out, a, w, off, pair_of_slot, pairs, top, E, K, N, act, st); break;
-    default: launch_bn<3>(out, a, w, off, pair_of_slot, pairs, top, E, K, N, act, st); break;
+    case 0: launch_bn<0>(out, a, w, off, pairs, E, K, N, act, st); break;
+    case 1: launch_bn<1>(out, a, w, off, pairs, E, K, N, act, st); break;
+    case 2: launch_bn<2>(out, a, w, off, pairs, E, K, N, act, st); break;
+    default: launch_bn<3>(out, a, w, off, pairs, E, K, N, act, st); break;
   }
   return true;
 }

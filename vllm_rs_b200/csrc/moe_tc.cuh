@@ -15,8 +15,9 @@ __device__ __forceinline__ float expert_gate(float g, float u, const b200_expert
   return g / (1.f + expf(-p.alpha * g)) * (u + p.up_add);
 }
 
-// A grouped product in bf16 on the tensor cores (act_kind as ACT in moe.cu); false: sizes or alignment it does not take.
+// A grouped product in bf16 on the tensor cores (act_kind as ACT in moe.cu).  Token rows (act_kind != 0) are first copied to
+// `rows` [pairs, K] in bucket order.  false: sizes or alignment it does not take, or no space for the rows.
 bool grouped_linear_tc(int act_kind, void* out, const void* a, const void* w, const int32_t* off, const int32_t* pair_of_slot,
-                       int pairs, int top, int E, int K, int N, const b200_expert_act& act, cudaStream_t st);
+                       void* rows, int pairs, int top, int E, int K, int N, const b200_expert_act& act, cudaStream_t st);
 
 }  // namespace b200

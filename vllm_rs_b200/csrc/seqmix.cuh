@@ -163,9 +163,9 @@ void launch_moe_route(const float* logits, const float* bias, int T, int E, int 
                       int group_top, int renorm, float scale, int32_t* top_idx, float* top_w, cudaStream_t st);
 void launch_moe_sort(const int32_t* top_idx, int pairs, int E, int32_t* expert_off, int32_t* pair_of_slot,
                      int32_t* slot_of_pair, cudaStream_t st);
-// act.kind: B200_EXPERT_*
+// act.kind: B200_EXPERT_*; rows: space for the token rows in bucket order [pairs, width] (bf16)
 void launch_moe_gate_up(void* act_out, const void* h, const void* w_up, const int32_t* expert_off,
-                        const int32_t* pair_of_slot, int pairs, int top, int E, int width, int ff,
+                        const int32_t* pair_of_slot, void* rows, int pairs, int top, int E, int width, int ff,
                         const b200_expert_act& act, int dt, cudaStream_t st);
 void launch_moe_down(float* out, const void* act, const void* w_down, const int32_t* expert_off, int pairs, int E,
                      int width, int ff, int dt, cudaStream_t st);
