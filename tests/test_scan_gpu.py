@@ -1,0 +1,79 @@
+"""The recurrent scans (gated delta rule, decayed linear attention, state-space scan) against the recurrence token by token in 64
+bits: sequences that end at, just before and just after a block of eight tokens and a staged pass of sixteen, single tokens
+on a kept state, sizes with padding, unaligned rows, decays near zero and one, several sequences at once."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _i32(x):
+    return torch.tensor(x, dtype=torch.int32, device="cuda")
+
+
+def _walk(q, k, v, decay, w, S, corrected):
+    """q, k [T, H, d], v [T, H, e], decay [T, H, d or 1], w [T, H] write strengths, S [H, d, e]."""
+    out = torch.empty_like(v)
+    for t in range(v.shape[0]):
+        S = S * decay[t][:, :, None]
+        u = v[t] - (torch.einsum("hd,hde->he", k[t], S) if corrected else 0)
+        S = S + torch.einsum("hd,he->hde", k[t], w[t][:, None] * u)
+        out[t] = torch.einsum("hd,hde->he", q[t], S)
+    return out, S
+
+
+@pytest.mark.parametrize("lens", [[1], [1, 1, 1], [7, 8, 9], [15, 16, 17], [33, 1, 130]])
+@pytest.mark.parametrize("H,G,d,e", [(2, 1, 128, 128), (3, 3, 20, 50), (2, 2, 33, 16), (1, 1, 200, 36), (2, 2, 64, 40)])
+@pytest.mark.parametrize("kind", ["delta", "delta_chan", "decay", "decay_chan", "ssd"])
+def test_scans(lib, kind, H, G, d, e, lens):
+    from vllm_rs_b200 import ops
+    if kind.startswith("decay"):
+        G = H
+    g = torch.Generator().manual_seed(d * e + sum(lens))
+    T, n, D = sum(lens), len(lens), torch.float64
+    r = lambda *s: torch.randn(*s, generator=g)                               # noqa: E731
+    q, k, v, state = r(T, G, d), r(T, G, d), r(T, H, e), r(n + 1, H, d, e)
+    slots = torch.randperm(n + 1, generator=g)[:n]
+    past = [0 if i % 2 else 5 for i in range(n)]                              # every other sequence starts here
+    cu, ctx = _i32([0] + [sum(lens[:i + 1]) for i in range(n)]), _i32([a + b for a, b in zip(lens, past)])
+    c = lambda t: t.cuda().contiguous()                                       # noqa: E731
+    dev_state, rep = c(state), H // G
+    wide = lambda t: t.double().repeat_interleave(rep, 1)                     # noqa: E731
+    corrected, skip = kind.startswith("delta"), 0.0
+    chan = torch.sigmoid(4 * r(T, H, d)) ** 0.5
+    chan[::5, :, 0] = 0.0                                                     # a channel that forgets everything
+    if corrected:
+        braw, araw, alog, dtb = r(T, H), r(T, H), r(H) * 0.5, r(H)
+        unit = lambda t: t / torch.sqrt((t * t).sum(-1, keepdim=True) + 1e-6)      # noqa: E731
+        Q, K, w = unit(wide(q)) * d ** -0.5, unit(wide(k)), torch.sigmoid(braw.double())
+        dec = torch.exp(-torch.exp(alog.double()) * torch.nn.functional.softplus(araw.double() + dtb.double()))[..., None]
+        if kind == "delta":
+            got = ops.delta_rule(c(q), c(k), c(v), c(braw), c(araw), c(alog), c(dtb), dev_state, c(slots.int()), cu, ctx)
+        else:
+            dec = chan.double()
+            got = ops.delta_rule_chan(c(q), c(k), c(v), c(braw), c(chan), dev_state, c(slots.int()), cu, ctx)
+        V = v.double()
+    elif kind == "ssd":
+        dt, alog, dtb, dsk = r(T, H), r(H) * 0.5, r(H), r(H)
+        w = torch.nn.functional.softplus(dt.double() + dtb.double())
+        Q, K, V, skip = wide(q), wide(k), v.double(), dsk.double()[:, None] * v.double()
+        dec = torch.exp(-torch.exp(alog.double()) * w)[..., None]
+        got = ops.ssd_scan(c(v), c(k), c(q), c(dt), c(alog), c(dtb), c(dsk), dev_state, c(slots.int()), cu, ctx)
+    else:
+        act = kind == "decay_chan"
+        f = torch.nn.functional.silu if act else (lambda t: t)
+        Q, K, V, w = f(q.double()) * 0.3, f(k.double()), f(v.double()), torch.full((T, H), 0.7, dtype=D)
+        hd = torch.linspace(0.3, 1.0, H)
+        dec = chan.double() if act else hd.double()[None, :, None].expand(T, H, 1)
+        got = ops.decay_attn(c(q), c(k), c(v), dev_state, c(slots.int()), cu, ctx, q_scale=0.3, k_scale=0.7, act=act,
+                             **(dict(chan_decay=c(chan)) if act else dict(head_decay=c(hd))))
+    want, want_state, at = torch.empty(T, H, e, dtype=D), state.double().clone(), 0
+    for i, m in enumerate(lens):
+        sl, s = slice(at, at + m), int(slots[i])
+        S0 = state[s].double() if past[i] else torch.zeros(H, d, e, dtype=D)
+        want[sl], want_state[s] = _walk(Q[sl], K[sl], V[sl], dec[sl], w[sl], S0, corrected)
+        at += m
+    want = want + skip
+    # fp32 sums of up to d terms, thousands of them below 2^-24 of the largest entries each
+    assert (got.double().cpu() - want).abs().max() <= 1e-5 * want.abs().max()
+    assert (dev_state.double().cpu() - want_state).abs().max() <= 1e-5 * want_state.abs().max()

@@ -19,11 +19,16 @@
 //                     one value per key channel and token (gated linear attention; lowrank_decay makes it from a
 //                     low-rank projection: sigmoid(z)^(1/tau)).  Optional SiLU on q, k, v and scales on q and k.
 //                     state [slots, heads, dim, vdim].
-// In the scans eight lanes share one column of S (one value channel), each holding every eighth row in registers,
-// and walk the sequence's tokens in order: the exact recurrence, no chunked reformulation, so a portion boundary
-// cannot change the arithmetic.  The tokens' inputs are staged in shared memory a pass at a time through two buffers
-// filled by cp.async, so the walk never waits for global memory.
+// The three scans share two kernels.  scan_one_kernel takes the sequences that bring one token.  scan_kernel walks longer portions
+// in blocks of eight tokens, within which the recurrence is unrolled exactly: with G_t the product of the block's decays up to
+// token t and S0 the state before it,
+//   k_t^T S_(t-1) = G_t k_t^T S0 + sum_(j<t) (G_t / G_j) (k_t . k_j) u_j,   S_t^T q_t likewise,   S_8 = G_8 S0 + sum_j (G_8 / G_j) k_j u_j^T
+// so that the eight tokens' products with the state are independent of each other and their sums over the lanes meet in one
+// exchange; the u_t follow from a product with the inverse of an 8 x 8 unit triangle.  Decay ratios are products of decays,
+// never quotients.  All fp32.
 #include "../../include/b200_vllm.h"
+#include <algorithm>
+
 #include "seqmix.cuh"
 
 namespace b200 {
@@ -94,9 +99,6 @@ __global__ void short_conv_state_kernel(const float* __restrict__ x, int ldx, fl
   for (int j = 0; j < P; ++j) sp[static_cast<size_t>(j) * C] = keep[j];
 }
 
-// tokens staged in shared memory per pass; there are two such buffers (static shared memory stays under 48 KB for
-// the widest state): the next pass's rows arrive by cp.async while the current pass's tokens are walked
-constexpr int chunk_for(int rows) { return rows > 128 ? 8 : rows > 64 ? 16 : 32; }
 __device__ __forceinline__ void cp_async4(float* smem, const float* gmem) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(smem))),
                "l"(gmem)
@@ -111,234 +113,683 @@ __device__ __forceinline__ void cp_async16(float* smem, const float* gmem) {
 template <int N> __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
-constexpr int kRowSplit = 8;       // lanes that share one column of S (each holds every 8th row)
-constexpr int kScanThreads = 128, kScanCols = kScanThreads / kRowSplit;      // columns of S per block
+// two fp32 values in a 64-bit register, one instruction for both
+using f2 = unsigned long long;
+__device__ __forceinline__ f2 pack2(float lo, float hi) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float sum2(f2 v) {
+  float lo, hi;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+  return lo + hi;
+}
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
+  f2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack2(f2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
 
-// grid = (column blocks, heads, sequences); block = 128 threads = 16 columns x kRowSplit lanes.  DK = compile-time
-// bound of `dim`; a lane holds the rows i = j * kRowSplit + part of its column.
-// CHAN: the decay is one value per head, key channel and token, read ready-made from chan_decay [T, heads, dim] (row
-// stride ld_decay; a_raw, a_log and dt_bias are not used); otherwise one value per head and token computed here.
-template <int DK, bool CHAN>
-__global__ void __launch_bounds__(128)
-delta_rule_kernel(float* __restrict__ out, const float* __restrict__ q, const float* __restrict__ k,
-                  const float* __restrict__ v, int ld, const float* __restrict__ b_raw,
-                  const float* __restrict__ a_raw, int ld_ba, const float* __restrict__ a_log,
-                  const float* __restrict__ dt_bias, const float* __restrict__ chan_decay, int ld_decay,
-                  float* __restrict__ state, const int32_t* __restrict__ slots,
-                  const uint32_t* __restrict__ cu, const uint32_t* __restrict__ ctx, int heads, int kv_heads, int dim,
-                  int vdim) {
-  // a third staged row set halves the tokens per pass where the rows are long (static shared memory stays under 48 KB)
-  constexpr int RS = kRowSplit, NR = DK / RS, kChunk = (CHAN && DK >= 64) ? chunk_for(DK) / 2 : chunk_for(DK);
-  __shared__ float ks[2][kChunk][DK], qs[2][kChunk][DK], vs[2][kChunk][kScanCols], gs[2][kChunk], bs[2][kChunk];
-  __shared__ float as[CHAN ? 2 : 1][CHAN ? kChunk : 1][CHAN ? DK : 1];
-  const int h = blockIdx.y, b = blockIdx.z;
-  const int part = threadIdx.x % RS;
-  const int col = blockIdx.x * (blockDim.x / RS) + threadIdx.x / RS;
-  const bool live = col < vdim;
-  const int t0 = cu[b], t1 = cu[b + 1];
-  if (t1 <= t0) return;
-  const bool fresh = static_cast<int>(ctx[b]) == t1 - t0;
-  const int hk = h / (heads / kv_heads);
-  float* sp = state + ((static_cast<size_t>(slots[b]) * heads + h) * dim) * vdim + col;
-  float s[NR];
+constexpr int kScanCols = 16;                  // columns of S per block of threads
+constexpr int kBT = 8;                         // tokens per block of the recurrence
+constexpr int kRing = 4;                       // blocks of tokens in shared memory: walked, prepared, two on their way
+constexpr int kDelta = 0, kDecay = 1, kSsd = 2;
+
+struct ScanArgs {
+  float* out;
+  const float *q, *k, *v;          // delta: q, k, v; ssd: C, B, x
+  int ld;
+  const float *b_raw, *a_raw;      // delta: write strength and decay logits; ssd: a_raw = dt_raw
+  int ld_ba;
+  const float *a_log, *dt_bias, *d_skip, *head_decay, *chan_decay;
+  int ld_decay;
+  float q_scale, k_scale;
+  int act;
+  float* state;
+  const int32_t* slots;
+  const uint32_t *cu, *ctx;
+  int heads, kv_heads, dim, vdim;
+};
+
+template <int DK, bool CHAN> struct ScanSmem {
+  static constexpr int kRows = kBT * DK;                                        // floats of one array of token rows
+  static constexpr int kV = (CHAN ? 3 : 2) * kRows;                             // k | q | decays | v | scalars | T, P (8 x 8 each) | ..
+  static constexpr int kG = kV + kBT * kScanCols, kMat = kG + 4 * kBT;          // decay, strength, G_t, W_t per token
+  static constexpr int kGend = kMat + 2 * kBT * kBT;                            // CHAN: [DK] decays over the block
+  static constexpr int kBuf = kGend + (CHAN ? DK : 0);
+  static constexpr int kU = kRing * kBuf;                                       // [4 warps][8 tokens][4 columns]
+  static constexpr int kBars = kU + 4 * kBT * 4;
+  static constexpr int kBytes = kBars * 4 + 2 * kRing * 8 + 16;
+};
+// CH floats from shared memory
+template <int CH> __device__ __forceinline__ void ldv(float (&x)[CH], const float* p) {
+  if constexpr (CH % 4 == 0) {
 #pragma unroll
-  for (int j = 0; j < NR; ++j) {
-    const int i = j * RS + part;
-    s[j] = (!fresh && live && i < dim) ? sp[static_cast<size_t>(i) * vdim] : 0.f;
-  }
-  const float neg_a = CHAN ? 0.f : -expf(a_log[h]), dtb = CHAN ? 0.f : dt_bias[h];
-  const float qscale = rsqrtf(static_cast<float>(dim));
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  if (dim < DK)                                                           // the padding past `dim` stays zero
-    for (int e = threadIdx.x; e < 2 * kChunk * DK; e += kScanThreads) {
-      (&ks[0][0][0])[e] = (&qs[0][0][0])[e] = 0.f;
-      if (CHAN) (&as[0][0][0])[e] = 0.f;
+    for (int i = 0; i < CH; i += 4) {
+      const float4 v = *reinterpret_cast<const float4*>(p + i);
+      x[i] = v.x; x[i + 1] = v.y; x[i + 2] = v.z; x[i + 3] = v.w;
     }
-  for (int e = threadIdx.x; e < 2 * kChunk * kScanCols; e += kScanThreads) (&vs[0][0][0])[e] = 0.f;
+  } else {
+    const float2 v = *reinterpret_cast<const float2*>(p);
+    x[0] = v.x; x[1] = v.y;
+  }
+}
+template <int CH> __device__ __forceinline__ void stv(float* p, const float (&x)[CH]) {
+  if constexpr (CH % 4 == 0) {
+#pragma unroll
+    for (int i = 0; i < CH; i += 4) *reinterpret_cast<float4*>(p + i) = make_float4(x[i], x[i + 1], x[i + 2], x[i + 3]);
+  } else {
+    *reinterpret_cast<float2*>(p) = make_float2(x[0], x[1]);
+  }
+}
+template <int CH> __device__ __forceinline__ void ldv2(f2 (&x)[CH / 2], const float* p) {
+  if constexpr (CH % 4 == 0) {
+#pragma unroll
+    for (int i = 0; i < CH; i += 4) {
+      const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p + i);
+      x[i / 2] = v.x; x[i / 2 + 1] = v.y;
+    }
+  } else {
+    x[0] = *reinterpret_cast<const f2*>(p);
+  }
+}
+// 32 values per lane -> lane l holds the sum over the lanes of value l: a butterfly that halves the values
+__device__ __forceinline__ float meet32(float (&x)[32], int lane) {
+#pragma unroll
+  for (int w = 16; w > 0; w >>= 1) {
+    const bool up = lane & w;
+#pragma unroll
+    for (int i = 0; i < w; ++i) {
+      const float keep = up ? x[i + w] : x[i], send = up ? x[i] : x[i + w];
+      x[i] = keep + __shfl_xor_sync(0xffffffffu, send, w);
+    }
+  }
+  return x[0];
+}
+
+// Portions of two tokens and more.  grid = (column blocks, heads, runs of sequences); a block walks its sequences one after
+// another.  Warps 0-3 each own four columns of S: a lane holds DK / 32 neighbouring rows of them in registers, so that a key or
+// query row is read once from shared memory for four columns (one column per lane made these reads the bound: 512 bytes of
+// registers per load and warp).  Warps 4-7 fetch the token rows (cp.async, two blocks of eight tokens ahead), norm or
+// activate them and prepare the block's triangles under the walk of the block before.
+// 4096 tokens, 16 heads of 128 x 128: BEFORE us token by token (1020 cycles per token), AFTER us.
+template <int DK, int MODE, bool CHAN>
+__global__ void __launch_bounds__(256, 2)
+scan_kernel(const ScanArgs a, int num_seqs, int* err) {
+  using SM = ScanSmem<DK, CHAN>;
+  constexpr int CH = DK / 32;
+  extern __shared__ __align__(16) float sm[];
+  uint64_t* ready = reinterpret_cast<uint64_t*>(sm + SM::kBars);
+  uint64_t* done = ready + kRing;
+  volatile int* fail = reinterpret_cast<volatile int*>(done + kRing);
+  const int h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, col0 = blockIdx.x * kScanCols;
+  const int dim = a.dim, vdim = a.vdim, hk = MODE == kDecay ? h : h / (a.heads / a.kv_heads);
+  if (tid == 0) {
+    for (int i = 0; i < kRing; ++i) { mbar_init(&ready[i], 4); mbar_init(&done[i], 4); }
+    *fail = 0;
+    fence_barrier_init();
+  }
+  for (int e = tid; e < kRing * SM::kBuf; e += 256) sm[e] = 0.f;       // padding past `dim` is zero and stays it
   __syncthreads();
-  // raw rows of one pass -> buffer `buf` (asynchronous; committed as one group)
-  auto fetch = [&](int c0, int buf) {
-    const int n = min(kChunk, t1 - c0);
-    for (int e = threadIdx.x; e < n * dim; e += kScanThreads) {
-      const int r = e / dim, i = e - r * dim;
-      cp_async4(&ks[buf][r][i], k + static_cast<size_t>(c0 + r) * ld + hk * dim + i);
-      cp_async4(&qs[buf][r][i], q + static_cast<size_t>(c0 + r) * ld + hk * dim + i);
-      if (CHAN) cp_async4(&as[buf][r][i], chan_decay + static_cast<size_t>(c0 + r) * ld_decay + h * dim + i);
-    }
-    for (int e = threadIdx.x; e < n * kScanCols; e += kScanThreads) {
-      const int r = e / kScanCols, c = blockIdx.x * kScanCols + e % kScanCols;
-      if (c < vdim) cp_async4(&vs[buf][r][e % kScanCols], v + static_cast<size_t>(c0 + r) * ld + h * vdim + c);
-    }
-    if (threadIdx.x < n) {
-      cp_async4(&bs[buf][threadIdx.x], b_raw + static_cast<size_t>(c0 + threadIdx.x) * ld_ba + h);
-      if (!CHAN) cp_async4(&gs[buf][threadIdx.x], a_raw + static_cast<size_t>(c0 + threadIdx.x) * ld_ba + h);
-    }
-    cp_async_commit();
-  };
-  fetch(t0, 0);
-  int buf = 0;
-  for (int c0 = t0; c0 < t1; c0 += kChunk, buf ^= 1) {
-    const int n = min(kChunk, t1 - c0);
-    if (c0 + kChunk < t1) {
-      fetch(c0 + kChunk, buf ^ 1);         // the other buffer's tokens were walked before the last barrier
-      cp_async_wait<1>();
-    } else {
+  int blocks = 0;                                                      // blocks of tokens so far, over all sequences
+  for (int b = blockIdx.z; b < num_seqs; b += gridDim.z) {
+    const int t0 = a.cu[b], t1 = a.cu[b + 1], nblk = (t1 - t0 + kBT - 1) / kBT;
+    if (t1 - t0 < 2) continue;                                         // (scan_one_kernel)
+    const bool fresh = static_cast<int>(a.ctx[b]) == t1 - t0;
+    if (warp >= 4) {
+      // ---------------------------------------------------------- token rows
+      const int pt = tid - 128, pw = warp - 4;
+      const bool wide = dim % 4 == 0 && a.ld % 4 == 0 && (!CHAN || a.ld_decay % 4 == 0) &&
+                        ((reinterpret_cast<uintptr_t>(a.q) | reinterpret_cast<uintptr_t>(a.k) |
+                          (CHAN ? reinterpret_cast<uintptr_t>(a.chan_decay) : 0)) & 15) == 0;
+      const bool wide_v = vdim % 4 == 0 && a.ld % 4 == 0 && (reinterpret_cast<uintptr_t>(a.v) & 15) == 0;
+      auto fetch = [&](int i) {                                        // block i of the sequence; one group in any case
+        if (i < nblk) {
+          const int g = blocks + i;
+          if (g >= kRing) mbar_wait_limited(&done[g % kRing], (g / kRing - 1) & 1, fail, err);
+          float* B = sm + g % kRing * SM::kBuf;
+          const int c0 = t0 + i * kBT, n = min(kBT, t1 - c0);
+          const float* kg = a.k + static_cast<size_t>(c0) * a.ld + hk * dim;
+          const float* qg = a.q + static_cast<size_t>(c0) * a.ld + hk * dim;
+          const float* ag = CHAN ? a.chan_decay + static_cast<size_t>(c0) * a.ld_decay + h * dim : nullptr;
+          if (wide) {
+            const int d4 = dim / 4;
+            for (int e = pt; e < n * d4; e += 128) {
+              const int r = e / d4, x = (e - r * d4) * 4, o = r * DK + x;
+              cp_async16(B + o, kg + static_cast<size_t>(r) * a.ld + x);
+              cp_async16(B + SM::kRows + o, qg + static_cast<size_t>(r) * a.ld + x);
+              if (CHAN) cp_async16(B + 2 * SM::kRows + o, ag + static_cast<size_t>(r) * a.ld_decay + x);
+            }
+          } else {
+            for (int e = pt; e < n * dim; e += 128) {
+              const int r = e / dim, x = e - r * dim, o = r * DK + x;
+              cp_async4(B + o, kg + static_cast<size_t>(r) * a.ld + x);
+              cp_async4(B + SM::kRows + o, qg + static_cast<size_t>(r) * a.ld + x);
+              if (CHAN) cp_async4(B + 2 * SM::kRows + o, ag + static_cast<size_t>(r) * a.ld_decay + x);
+            }
+          }
+          const float* vg = a.v + static_cast<size_t>(c0) * a.ld + h * vdim + col0;
+          if (wide_v) {
+            const int r = pt >> 2, c = (pt & 3) * 4;
+            if (r < n && col0 + c < vdim) cp_async16(B + SM::kV + r * kScanCols + c, vg + static_cast<size_t>(r) * a.ld + c);
+          } else {
+            const int r = pt >> 4, c = pt & 15;
+            if (r < n && col0 + c < vdim) cp_async4(B + SM::kV + pt, vg + static_cast<size_t>(r) * a.ld + c);
+          }
+          if (pt < n) {
+            const size_t o = static_cast<size_t>(c0 + pt) * a.ld_ba + h;
+            if (MODE == kDelta) cp_async4(B + SM::kG + kBT + pt, a.b_raw + o);
+            if (MODE == kSsd || (MODE == kDelta && !CHAN)) cp_async4(B + SM::kG + pt, a.a_raw + o);
+          }
+        }
+        cp_async_commit();
+      };
+      auto sync = [] {                                 // of these four warps
+        __syncwarp();
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+      };
+      const float neg_a = MODE == kDecay || CHAN ? 0.f : -expf(a.a_log[h]), dtb = MODE == kDecay || CHAN ? 0.f : a.dt_bias[h];
+      const float hd = MODE == kDecay && !CHAN ? a.head_decay[h] : 1.f;
+      const float qn = rsqrtf(static_cast<float>(dim));
+      fetch(0);
+      fetch(1);
+      for (int i = 0; i < nblk; ++i) {
+        fetch(i + 2);
+        cp_async_wait<2>();
+        sync();
+        float* B = sm + (blocks + i) % kRing * SM::kBuf;
+        float* G = B + SM::kG;
+        const int n = min(kBT, t1 - t0 - i * kBT);
+        // ---- two tokens per warp: norms or activation, in place; past the end: no key, no value, decay one
+#pragma unroll
+        for (int z = 0; z < 2; ++z) {
+          const int r = pw * 2 + z;
+          float* kr = B + r * DK + lane * CH;
+          float* qr = kr + SM::kRows;
+          float kx[CH], qx[CH];
+          if (r < n) {
+            if (MODE == kDelta || (MODE == kDecay && a.act)) {
+              ldv<CH>(kx, kr);
+              ldv<CH>(qx, qr);
+              if (MODE == kDelta) {
+                float sk = 0.f, sq = 0.f;
+#pragma unroll
+                for (int j = 0; j < CH; ++j) {
+                  sk += kx[j] * kx[j];
+                  sq += qx[j] * qx[j];
+                }
+                sk = lanes_sum(sk);
+                sq = lanes_sum(sq);
+                const float ik = 1.f / sqrtf(sk + 1e-6f), iq = qn / sqrtf(sq + 1e-6f);
+#pragma unroll
+                for (int j = 0; j < CH; ++j) {
+                  kx[j] *= ik;
+                  qx[j] *= iq;
+                }
+              } else {
+#pragma unroll
+                for (int j = 0; j < CH; ++j) {
+                  kx[j] = silu_exact(kx[j]);
+                  qx[j] = silu_exact(qx[j]);
+                }
+                if (lane < kScanCols) B[SM::kV + r * kScanCols + lane] = silu_exact(B[SM::kV + r * kScanCols + lane]);
+              }
+              stv<CH>(kr, kx);
+              stv<CH>(qr, qx);
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < CH; ++j) kx[j] = 0.f;
+            stv<CH>(kr, kx);
+            stv<CH>(qr, kx);
+            if (lane < kScanCols) B[SM::kV + r * kScanCols + lane] = 0.f;
+            if (CHAN) {
+#pragma unroll
+              for (int j = 0; j < CH; ++j) kx[j] = 1.f;
+              stv<CH>(kr + 2 * SM::kRows, kx);
+            }
+          }
+        }
+        if (pw == 3 && lane < kBT) {
+          float g = 1.f, w = 0.f;                      // decay; write strength
+          if (lane < n) {
+            if (MODE == kDelta) {
+              w = sigmoid_f(G[kBT + lane]);
+              if (!CHAN) g = expf(neg_a * softplus_f(G[lane] + dtb));
+            } else if (MODE == kSsd) {
+              w = softplus_f(G[lane] + dtb);
+              g = expf(neg_a * w);
+            } else {
+              w = a.k_scale;
+              g = hd;
+            }
+          }
+          float up = g, down = 1.f;                    // products of decays up to a token, and behind it
+#pragma unroll
+          for (int o = 1; o < kBT; o <<= 1) {
+            const float x = __shfl_up_sync(0xffu, up, o);
+            if (lane >= o) up *= x;
+          }
+          float tail = g;
+#pragma unroll
+          for (int o = 1; o < kBT; o <<= 1) {
+            const float x = __shfl_down_sync(0xffu, tail, o);
+            if (lane + o < kBT) tail *= x;
+          }
+          const float after = __shfl_down_sync(0xffu, tail, 1);
+          if (lane + 1 < kBT) down = after;
+          G[lane] = g;
+          G[kBT + lane] = w;
+          G[2 * kBT + lane] = up;
+          G[3 * kBT + lane] = down;
+        }
+        sync();
+        // ---- warp 0: P (t, j) = decayed q_t . k_j, j <= t.  warp 1 (delta): M (t, j) = beta_t times the decayed k_t . k_j, j < t,
+        // and T = (1 + M)^-1.  A lane holds its rows of all eight tokens.
+        if (pw == 0 || (pw == 1 && MODE == kDelta)) {
+          float y[kBT][CH], x[64];
+#pragma unroll
+          for (int t = 0; t < kBT; ++t) ldv<CH>(y[t], B + t * DK + lane * CH);
+#pragma unroll
+          for (int t = 0; t < kBT; ++t) {
+            float xt[CH], dt[CH];
+            ldv<CH>(xt, B + (pw == 0 ? SM::kRows : 0) + t * DK + lane * CH);
+            if (CHAN) {                                // y[j] becomes k_j decayed up to token t
+              ldv<CH>(dt, B + 2 * SM::kRows + t * DK + lane * CH);
+#pragma unroll
+              for (int j = 0; j < kBT; ++j)
+                if (j < t) {
+#pragma unroll
+                  for (int c = 0; c < CH; ++c) y[j][c] *= dt[c];
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < kBT; ++j) {
+              float acc = 0.f;
+              if (j <= t) {
+#pragma unroll
+                for (int c = 0; c < CH; ++c) acc += xt[c] * y[j][c];
+              }
+              x[t * kBT + j] = acc;
+            }
+          }
+          // sums over the lanes: lane l gets entries l and l + 32
+          float lo[32], hi[32];
+#pragma unroll
+          for (int e = 0; e < 32; ++e) {
+            lo[e] = x[e];
+            hi[e] = x[32 + e];
+          }
+          float ent[2] = {meet32(lo, lane), meet32(hi, lane)};
+          float* out = B + SM::kMat + (pw == 0 ? kBT * kBT : 0);
+#pragma unroll
+          for (int z = 0; z < 2; ++z) {
+            const int t = (lane >> 3) + z * 4, j = lane & 7;
+            float v = ent[z];
+            for (int m = j + 1; m <= t; ++m) v *= G[m];
+            if (pw == 1) v = t > j ? v * G[kBT + t] : 0.f;
+            out[t * kBT + j] = v;
+          }
+          if (pw == 1) {                               // column c of T by forward substitution, one lane each
+            __syncwarp();
+            float tc[kBT];
+            if (lane < kBT) {
+#pragma unroll
+              for (int t = 0; t < kBT; ++t) {
+                float acc = t == lane ? 1.f : 0.f;
+#pragma unroll
+                for (int j = 0; j < t; ++j) acc -= out[t * kBT + j] * tc[j];
+                tc[t] = acc;
+              }
+            }
+            __syncwarp();
+            if (lane < kBT) {
+#pragma unroll
+              for (int t = 0; t < kBT; ++t) out[t * kBT + lane] = tc[t];
+            }
+          }
+        }
+        if (CHAN) {
+          // k <- G_t k_t, q <- G_t q_t, decays <- W_t k_t, per channel; the block's whole decay
+          sync();
+          for (int e = pt; e < DK; e += 128) {
+            float kr[kBT], d[kBT], g = 1.f;
+#pragma unroll
+            for (int t = 0; t < kBT; ++t) {
+              kr[t] = B[t * DK + e];
+              d[t] = e < dim ? B[2 * SM::kRows + t * DK + e] : 1.f;
+              g *= d[t];
+              B[t * DK + e] = kr[t] * g;
+              B[SM::kRows + t * DK + e] *= g;
+            }
+            B[SM::kGend + e] = g;
+            g = 1.f;
+#pragma unroll
+            for (int t = kBT - 1; t >= 0; --t) {
+              B[2 * SM::kRows + t * DK + e] = kr[t] * g;
+              g *= d[t];
+            }
+          }
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&ready[(blocks + i) % kRing]);
+      }
       cp_async_wait<0>();
-    }
-    __syncthreads();
-    // unit-normalise q, k of the pass in place: one warp per token row
-    for (int r = warp; r < n; r += nw) {
-      float sk = 0.f, sq = 0.f;
-      for (int i = lane; i < dim; i += 32) {
-        sk += ks[buf][r][i] * ks[buf][r][i];
-        sq += qs[buf][r][i] * qs[buf][r][i];
-      }
-      sk = lanes_sum(sk);
-      sq = lanes_sum(sq);
-      const float ik = 1.f / sqrtf(sk + 1e-6f), iq = qscale / sqrtf(sq + 1e-6f);
-      for (int i = lane; i < dim; i += 32) {
-        ks[buf][r][i] *= ik;
-        qs[buf][r][i] *= iq;
-      }
-      if (lane == 0) {
-        bs[buf][r] = sigmoid_f(bs[buf][r]);
-        if (!CHAN) gs[buf][r] = expf(neg_a * softplus_f(gs[buf][r] + dtb));
-      }
-    }
-    __syncthreads();
-    for (int r = 0; r < n; ++r) {          // every lane runs the shuffles; dead columns carry zeros
-      const float vv = vs[buf][r][threadIdx.x / RS];
-      const float g = CHAN ? 0.f : gs[buf][r];
-      float d0 = 0.f, d1 = 0.f;
+    } else {
+      // ---------------------------------------------------------- the walk
+      const int colw = col0 + warp * 4;                // this warp's first column
+      float* sp = a.state + ((static_cast<size_t>(a.slots[b]) * a.heads + h) * dim) * vdim + colw;
+      const bool wide_s = vdim % 4 == 0 && (reinterpret_cast<uintptr_t>(a.state) & 15) == 0;
+      const float skip = MODE == kSsd && a.d_skip ? a.d_skip[h] : 0.f;
+      f2 s[4][CH / 2];                                 // [column][pair of rows]
+      {
+        float x[CH][4];
 #pragma unroll
-      for (int j = 0; j < NR; j += 2) {
-        s[j] *= CHAN ? as[CHAN ? buf : 0][CHAN ? r : 0][CHAN ? j * RS + part : 0] : g;
-        d0 += ks[buf][r][j * RS + part] * s[j];
-        if (j + 1 < NR) {
-          s[j + 1] *= CHAN ? as[CHAN ? buf : 0][CHAN ? r : 0][CHAN ? (j + 1) * RS + part : 0] : g;
-          d1 += ks[buf][r][(j + 1) * RS + part] * s[j + 1];
+        for (int r = 0; r < CH; ++r) {
+          const int i = lane * CH + r;
+#pragma unroll
+          for (int c = 0; c < 4; ++c) x[r][c] = 0.f;
+          if (!fresh && i < dim) {
+            const float* src = sp + static_cast<size_t>(i) * vdim;
+            if (wide_s && colw < vdim) {
+              const float4 v = *reinterpret_cast<const float4*>(src);
+              x[r][0] = v.x; x[r][1] = v.y; x[r][2] = v.z; x[r][3] = v.w;
+            } else {
+#pragma unroll
+              for (int c = 0; c < 4; ++c)
+                if (colw + c < vdim) x[r][c] = src[c];
+            }
+          }
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+          for (int r = 0; r < CH; r += 2) s[c][r / 2] = pack2(x[r][c], x[r + 1][c]);
+      }
+      float* us = sm + SM::kU + warp * kBT * 4;
+      const int tt = lane >> 2, c4 = lane & 3;         // the token and column whose sums this lane gets
+      for (int i = 0; i < nblk; ++i) {
+        const int g = blocks + i;
+        mbar_wait_limited(&ready[g % kRing], (g / kRing) & 1, fail, err);
+        __syncwarp();
+        const float* B = sm + g % kRing * SM::kBuf;
+        const float* G = B + SM::kG;
+        // a row's products with the state, summed over the lanes
+        auto dots = [&](const float* rows) {
+          float x[32];
+#pragma unroll
+          for (int t = 0; t < kBT; ++t) {
+            f2 y[CH / 2];
+            ldv2<CH>(y, rows + t * DK + lane * CH);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              f2 acc = mul2(y[0], s[c][0]);
+#pragma unroll
+              for (int r = 1; r < CH / 2; ++r) acc = fma2(y[r], s[c][r], acc);
+              x[t * 4 + c] = sum2(acc);
+            }
+          }
+          return meet32(x, lane);
+        };
+        const float gt = CHAN ? 1.f : G[2 * kBT + tt];
+        const float vt = B[SM::kV + tt * kScanCols + warp * 4 + c4], wt = G[kBT + tt];
+        float u = vt * wt;
+        if (MODE == kDelta) {
+          const float r = wt * (vt - gt * dots(B));
+          const float4 ta = *reinterpret_cast<const float4*>(B + SM::kMat + tt * kBT), tb = *reinterpret_cast<const float4*>(B + SM::kMat + tt * kBT + 4);
+          const float T[kBT] = {ta.x, ta.y, ta.z, ta.w, tb.x, tb.y, tb.z, tb.w};
+          u = 0.f;
+#pragma unroll
+          for (int j = 0; j < kBT; ++j) u += T[j] * __shfl_sync(0xffffffffu, r, j * 4 + c4);
+        }
+        us[lane] = CHAN ? u : u * G[3 * kBT + tt];
+        const float e = dots(B + SM::kRows);
+        {
+          const float4 pa = *reinterpret_cast<const float4*>(B + SM::kMat + kBT * kBT + tt * kBT);
+          const float4 pb = *reinterpret_cast<const float4*>(B + SM::kMat + kBT * kBT + tt * kBT + 4);
+          const float P[kBT] = {pa.x, pa.y, pa.z, pa.w, pb.x, pb.y, pb.z, pb.w};
+          float o = gt * e;
+#pragma unroll
+          for (int j = 0; j < kBT; ++j) o += P[j] * __shfl_sync(0xffffffffu, u, j * 4 + c4);
+          if (MODE == kDecay) o *= a.q_scale;
+          if (MODE == kSsd) o += skip * vt;
+          const int t = t0 + i * kBT + tt;
+          if (t < t1 && colw + c4 < vdim) a.out[(static_cast<size_t>(t) * a.heads + h) * vdim + colw + c4] = o;
+        }
+        if (CHAN) {
+          f2 ge[CH / 2];
+          ldv2<CH>(ge, B + SM::kGend + lane * CH);
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+#pragma unroll
+            for (int r = 0; r < CH / 2; ++r) s[c][r] = mul2(s[c][r], ge[r]);
+        } else {
+          const float ge = G[3 * kBT - 1];
+          const f2 g2 = pack2(ge, ge);
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+#pragma unroll
+            for (int r = 0; r < CH / 2; ++r) s[c][r] = mul2(s[c][r], g2);
+        }
+        __syncwarp();
+        const float* kd = B + (CHAN ? 2 * SM::kRows : 0) + lane * CH;       // keys as they enter the state
+#pragma unroll
+        for (int t = 0; t < kBT; ++t) {
+          f2 y[CH / 2];
+          ldv2<CH>(y, kd + t * DK);
+          const float4 uu = *reinterpret_cast<const float4*>(us + t * 4);
+          const f2 u0 = pack2(uu.x, uu.x), u1 = pack2(uu.y, uu.y), u2 = pack2(uu.z, uu.z), u3 = pack2(uu.w, uu.w);
+#pragma unroll
+          for (int r = 0; r < CH / 2; ++r) {
+            s[0][r] = fma2(y[r], u0, s[0][r]);
+            s[1][r] = fma2(y[r], u1, s[1][r]);
+            s[2][r] = fma2(y[r], u2, s[2][r]);
+            s[3][r] = fma2(y[r], u3, s[3][r]);
+          }
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&done[g % kRing]);
+      }
+#pragma unroll
+      for (int r = 0; r < CH; r += 2) {
+        float x[2][4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) unpack2(s[c][r / 2], x[0][c], x[1][c]);
+#pragma unroll
+        for (int z = 0; z < 2; ++z) {
+          const int i = lane * CH + r + z;
+          if (i >= dim) continue;
+          float* dst = sp + static_cast<size_t>(i) * vdim;
+          if (wide_s && colw < vdim) {
+            *reinterpret_cast<float4*>(dst) = make_float4(x[z][0], x[z][1], x[z][2], x[z][3]);
+          } else {
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+              if (colw + c < vdim) dst[c] = x[z][c];
+          }
         }
       }
-      float dot = d0 + d1;
-#pragma unroll
-      for (int o = 1; o < RS; o <<= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-      const float u = bs[buf][r] * (vv - dot);
-      float o0 = 0.f, o1 = 0.f;
-#pragma unroll
-      for (int j = 0; j < NR; j += 2) {
-        s[j] += ks[buf][r][j * RS + part] * u;
-        o0 += qs[buf][r][j * RS + part] * s[j];
-        if (j + 1 < NR) {
-          s[j + 1] += ks[buf][r][(j + 1) * RS + part] * u;
-          o1 += qs[buf][r][(j + 1) * RS + part] * s[j + 1];
-        }
-      }
-      float o = o0 + o1;
-#pragma unroll
-      for (int x = 1; x < RS; x <<= 1) o += __shfl_xor_sync(0xffffffffu, o, x);
-      if (live && part == 0) out[(static_cast<size_t>(c0 + r) * heads + h) * vdim + col] = o;
     }
-    __syncthreads();                       // this buffer is refilled by the next pass's fetch
-  }
-  if (live) {
-#pragma unroll
-    for (int j = 0; j < NR; ++j) {
-      const int i = j * RS + part;
-      if (i < dim) sp[static_cast<size_t>(i) * vdim] = s[j];
-    }
+    blocks += nblk;
   }
 }
 
-template <int NS>
+// Sequences that bring one token.  grid = (column blocks, heads, sequences); 128 threads = 32 rows x 4 columns of 4; bound by the
+// state's way in and out, which are whole 64-byte rows here.
+template <int DK, int MODE, bool CHAN>
 __global__ void __launch_bounds__(128)
-ssd_scan_kernel(float* __restrict__ out, const float* __restrict__ x, const float* __restrict__ Bm,
-                const float* __restrict__ Cm, int ld, const float* __restrict__ dt_raw, int ld_dt,
-                const float* __restrict__ a_log, const float* __restrict__ dt_bias, const float* __restrict__ d_skip,
-                float* __restrict__ state, const int32_t* __restrict__ slots, const uint32_t* __restrict__ cu,
-                const uint32_t* __restrict__ ctx, int heads, int groups, int nstate, int vdim) {
-  constexpr int RS = kRowSplit, NR = NS / RS, kChunk = chunk_for(NS);
-  __shared__ float Bs[2][kChunk][NS], Cs[2][kChunk][NS], xs[2][kChunk][kScanCols], dts[2][kChunk], das[2][kChunk];
-  const int h = blockIdx.y, b = blockIdx.z;
-  const int part = threadIdx.x % RS;
-  const int col = blockIdx.x * (blockDim.x / RS) + threadIdx.x / RS;
-  const bool live = col < vdim;
-  const int t0 = cu[b], t1 = cu[b + 1];
-  if (t1 <= t0) return;
-  const bool fresh = static_cast<int>(ctx[b]) == t1 - t0;
-  const int g = h / (heads / groups);
-  float* sp = state + ((static_cast<size_t>(slots[b]) * heads + h) * nstate) * vdim + col;
-  float s[NR];
+scan_one_kernel(const ScanArgs a) {
+  constexpr int NR = DK / 32;
+  __shared__ float ks[DK], qs[DK], red[2][4][kScanCols], sums[4][2];
+  const int h = blockIdx.y, b = blockIdx.z, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int t = a.cu[b];
+  if (static_cast<int>(a.cu[b + 1]) - t != 1) return;
+  const bool fresh = a.ctx[b] == 1;
+  const int dim = a.dim, vdim = a.vdim, hk = MODE == kDecay ? h : h / (a.heads / a.kv_heads);
+  const int c = (tid & 3) * 4, col = blockIdx.x * kScanCols + c, row = tid >> 2;
+  float* sp = a.state + ((static_cast<size_t>(a.slots[b]) * a.heads + h) * dim) * vdim + col;
+  const bool wide = vdim % 4 == 0 && (reinterpret_cast<uintptr_t>(a.state) & 15) == 0;
+  float s[NR][4];
 #pragma unroll
-  for (int j = 0; j < NR; ++j) {
-    const int i = j * RS + part;
-    s[j] = (!fresh && live && i < nstate) ? sp[static_cast<size_t>(i) * vdim] : 0.f;
-  }
-  const float neg_a = -expf(a_log[h]), dtb = dt_bias[h], dsk = d_skip ? d_skip[h] : 0.f;
-  if (nstate < NS)                                                        // the padding past `nstate` stays zero
-    for (int e = threadIdx.x; e < 2 * kChunk * NS; e += kScanThreads) (&Bs[0][0][0])[e] = (&Cs[0][0][0])[e] = 0.f;
-  for (int e = threadIdx.x; e < 2 * kChunk * kScanCols; e += kScanThreads) (&xs[0][0][0])[e] = 0.f;
-  __syncthreads();
-  // raw rows of one pass -> buffer `buf` (asynchronous; committed as one group)
-  auto fetch = [&](int c0, int buf) {
-    const int n = min(kChunk, t1 - c0);
-    for (int e = threadIdx.x; e < n * nstate; e += kScanThreads) {
-      const int r = e / nstate, i = e - r * nstate;
-      cp_async4(&Bs[buf][r][i], Bm + static_cast<size_t>(c0 + r) * ld + g * nstate + i);
-      cp_async4(&Cs[buf][r][i], Cm + static_cast<size_t>(c0 + r) * ld + g * nstate + i);
-    }
-    for (int e = threadIdx.x; e < n * kScanCols; e += kScanThreads) {
-      const int r = e / kScanCols, c = blockIdx.x * kScanCols + e % kScanCols;
-      if (c < vdim) cp_async4(&xs[buf][r][e % kScanCols], x + static_cast<size_t>(c0 + r) * ld + h * vdim + c);
-    }
-    if (threadIdx.x < n) cp_async4(&dts[buf][threadIdx.x], dt_raw + static_cast<size_t>(c0 + threadIdx.x) * ld_dt + h);
-    cp_async_commit();
-  };
-  fetch(t0, 0);
-  int buf = 0;
-  for (int c0 = t0; c0 < t1; c0 += kChunk, buf ^= 1) {
-    const int n = min(kChunk, t1 - c0);
-    if (c0 + kChunk < t1) {
-      fetch(c0 + kChunk, buf ^ 1);         // the other buffer's tokens were walked before the last barrier
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
-    }
-    __syncthreads();
-    if (threadIdx.x < n) {
-      const float dt = softplus_f(dts[buf][threadIdx.x] + dtb);
-      dts[buf][threadIdx.x] = dt;
-      das[buf][threadIdx.x] = expf(neg_a * dt);
-    }
-    __syncthreads();
-    for (int r = 0; r < n; ++r) {
-      const float xv = xs[buf][r][threadIdx.x / RS];
-      const float a = das[buf][r], dx = dts[buf][r] * xv;
-      float y0 = 0.f, y1 = 0.f;
+  for (int r = 0; r < NR; ++r) {
+    const int i = row + r * 32;
+    s[r][0] = s[r][1] = s[r][2] = s[r][3] = 0.f;
+    if (!fresh && i < dim && col < vdim) {
+      const float* src = sp + static_cast<size_t>(i) * vdim;
+      if (wide) {
+        const float4 v = *reinterpret_cast<const float4*>(src);
+        s[r][0] = v.x; s[r][1] = v.y; s[r][2] = v.z; s[r][3] = v.w;
+      } else {
 #pragma unroll
-      for (int j = 0; j < NR; j += 2) {
-        s[j] = a * s[j] + dx * Bs[buf][r][j * RS + part];
-        y0 += Cs[buf][r][j * RS + part] * s[j];
-        if (j + 1 < NR) {
-          s[j + 1] = a * s[j + 1] + dx * Bs[buf][r][(j + 1) * RS + part];
-          y1 += Cs[buf][r][(j + 1) * RS + part] * s[j + 1];
-        }
+        for (int x = 0; x < 4; ++x)
+          if (col + x < vdim) s[r][x] = src[x];
       }
-      float y = y0 + y1;
-#pragma unroll
-      for (int o = 1; o < RS; o <<= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
-      if (live && part == 0) out[(static_cast<size_t>(c0 + r) * heads + h) * vdim + col] = y + dsk * xv;
     }
-    __syncthreads();                       // this buffer is refilled by the next pass's fetch
   }
-  if (live) {
-#pragma unroll
-    for (int j = 0; j < NR; ++j) {
-      const int i = j * RS + part;
-      if (i < nstate) sp[static_cast<size_t>(i) * vdim] = s[j];
+  const float* kg = a.k + static_cast<size_t>(t) * a.ld + hk * dim;
+  const float* qg = a.q + static_cast<size_t>(t) * a.ld + hk * dim;
+  float sk = 0.f, sq = 0.f;
+  for (int i = tid; i < DK; i += 128) {
+    float kv = i < dim ? kg[i] : 0.f, qv = i < dim ? qg[i] : 0.f;
+    if (MODE == kDecay && a.act) {
+      kv = silu_exact(kv);
+      qv = silu_exact(qv);
     }
+    ks[i] = kv;
+    qs[i] = qv;
+    sk += kv * kv;
+    sq += qv * qv;
+  }
+  if (MODE == kDelta) {
+    sk = lanes_sum(sk);
+    sq = lanes_sum(sq);
+    if (lane == 0) {
+      sums[warp][0] = sk;
+      sums[warp][1] = sq;
+    }
+  }
+  const size_t ba = static_cast<size_t>(t) * a.ld_ba + h;
+  float g = 1.f, w = a.k_scale;                        // decay; write strength
+  if (MODE == kDelta) {
+    w = sigmoid_f(a.b_raw[ba]);
+    if (!CHAN) g = expf(-expf(a.a_log[h]) * softplus_f(a.a_raw[ba] + a.dt_bias[h]));
+  } else if (MODE == kSsd) {
+    w = softplus_f(a.a_raw[ba] + a.dt_bias[h]);
+    g = expf(-expf(a.a_log[h]) * w);
+  } else if (!CHAN) {
+    g = a.head_decay[h];
+  }
+  float v[4];
+#pragma unroll
+  for (int x = 0; x < 4; ++x) {
+    v[x] = col + x < vdim ? a.v[static_cast<size_t>(t) * a.ld + h * vdim + col + x] : 0.f;
+    if (MODE == kDecay && a.act) v[x] = silu_exact(v[x]);
+  }
+  __syncthreads();
+  float ik = 1.f, iq = MODE == kDecay ? a.q_scale : 1.f;
+  if (MODE == kDelta) {
+    ik = 1.f / sqrtf(sums[0][0] + sums[1][0] + sums[2][0] + sums[3][0] + 1e-6f);
+    iq = rsqrtf(static_cast<float>(dim)) / sqrtf(sums[0][1] + sums[1][1] + sums[2][1] + sums[3][1] + 1e-6f);
+  }
+  // sums over the rows of four columns: lanes of the same columns, then the warps
+  auto meet = [&](float (&x)[4], int slot) {
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1)
+#pragma unroll
+      for (int z = 0; z < 4; ++z) x[z] += __shfl_xor_sync(0xffffffffu, x[z], o);
+    if (lane < 4) {
+#pragma unroll
+      for (int z = 0; z < 4; ++z) red[slot][warp][c + z] = x[z];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int z = 0; z < 4; ++z) x[z] = (red[slot][0][c + z] + red[slot][1][c + z]) + (red[slot][2][c + z] + red[slot][3][c + z]);
+  };
+  float u[4];
+#pragma unroll
+  for (int r = 0; r < NR; ++r) {
+    const int i = row + r * 32;
+    const float d = CHAN ? (i < dim ? a.chan_decay[static_cast<size_t>(t) * a.ld_decay + h * dim + i] : 1.f) : g;
+#pragma unroll
+    for (int x = 0; x < 4; ++x) s[r][x] *= d;
+  }
+  if (MODE == kDelta) {
+    float d[4] = {};
+#pragma unroll
+    for (int r = 0; r < NR; ++r) {
+      const float kv = ks[row + r * 32] * ik;
+#pragma unroll
+      for (int x = 0; x < 4; ++x) d[x] += kv * s[r][x];
+    }
+    meet(d, 0);
+#pragma unroll
+    for (int x = 0; x < 4; ++x) u[x] = w * (v[x] - d[x]);
+  } else {
+#pragma unroll
+    for (int x = 0; x < 4; ++x) u[x] = v[x] * w;
+  }
+  float o[4] = {};
+#pragma unroll
+  for (int r = 0; r < NR; ++r) {
+    const int i = row + r * 32;
+    const float kv = ks[i] * ik, qv = qs[i];
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      s[r][x] += kv * u[x];
+      o[x] += qv * s[r][x];
+    }
+    if (i < dim && col < vdim) {
+      float* dst = sp + static_cast<size_t>(i) * vdim;
+      if (wide) {
+        *reinterpret_cast<float4*>(dst) = make_float4(s[r][0], s[r][1], s[r][2], s[r][3]);
+      } else {
+#pragma unroll
+        for (int x = 0; x < 4; ++x)
+          if (col + x < vdim) dst[x] = s[r][x];
+      }
+    }
+  }
+  meet(o, 1);
+  const float skip = MODE == kSsd && a.d_skip ? a.d_skip[h] : 0.f;
+  if (warp == 0 && lane < 4) {
+#pragma unroll
+    for (int x = 0; x < 4; ++x)
+      if (col + x < vdim) a.out[(static_cast<size_t>(t) * a.heads + h) * vdim + col + x] = o[x] * iq + skip * v[x];
   }
 }
 
+template <int DK, int MODE, bool CHAN>
+static void launch_scan_dk(const ScanArgs& a, int num_seqs, cudaStream_t st_) {
+  const int cols = (a.vdim + kScanCols - 1) / kScanCols;
+  int* err = wait_error_flag();
+  if (!err) {
+    set_error(2, "scan: no host-visible memory");
+    return;
+  }
+  scan_one_kernel<DK, MODE, CHAN><<<dim3(cols, a.heads, num_seqs), 128, 0, st_>>>(a);
+  B200_CUDA_LAUNCH_CHECK();
+  auto kern = scan_kernel<DK, MODE, CHAN>;
+  constexpr int smem = ScanSmem<DK, CHAN>::kBytes;
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  // portions: a few blocks per SM, each taking every so many sequences (a step of decoded tokens is over at once)
+  const int z = std::max(1, std::min(num_seqs, 4 * sm_count() / (cols * a.heads)));
+  kern<<<dim3(cols, a.heads, z), 256, smem, st_>>>(a, num_seqs, err);
+  B200_CUDA_LAUNCH_CHECK();
+}
+// dim: rows of the state; at most 256 (the caller has checked)
+template <int MODE, bool CHAN>
+static void launch_scan(const ScanArgs& a, int num_seqs, cudaStream_t st_) {
+  if (a.dim <= 64) launch_scan_dk<64, MODE, CHAN>(a, num_seqs, st_);
+  else if (a.dim <= 128) launch_scan_dk<128, MODE, CHAN>(a, num_seqs, st_);
+  else launch_scan_dk<256, MODE, CHAN>(a, num_seqs, st_);
+}
 
 // out[t, c] = sigmoid(z)^(1 / tau) with z = bias[c] + sum_r w2[c, r] * low[t, r]: the per-channel decay of gated linear
 // attention from the low-rank half of its projection.  Computed as exp(log sigmoid(z) / tau), all fp32.
@@ -380,156 +831,6 @@ lowrank_decay_kernel(float* __restrict__ out, const float* __restrict__ low, int
   }
 }
 
-// tokens per pass of the decayed-state scan (two buffers of this many; a per-channel decay stages a third row set)
-constexpr int decay_chunk_for(int rows, bool chan) { return (chan ? 8 : 16) / (rows > 128 ? 2 : 1); }
-constexpr int kDecayPad = 4;       // floats between the row segments of two lanes: 16-byte loads without bank conflicts
-
-// grid = (column blocks, heads, sequences); block = 128 threads = 16 columns x kRowSplit lanes.  Unlike the scans above
-// a lane holds NR = DK / 8 CONSECUTIVE rows of its column (rows part * NR ..), and a token's k / q / decay rows lie in
-// shared memory as eight padded segments, so a lane reads its segment with 16-byte loads; four tokens are walked per
-// round so that their read-out reductions (shuffles) overlap the next tokens' state updates.
-// CHAN: the decay is per key channel and token (chan_decay [T, heads, dim], row stride ld_decay); otherwise one
-// constant per head (head_decay [heads]).
-template <int DK, bool CHAN>
-__global__ void __launch_bounds__(128)
-decay_attn_kernel(float* __restrict__ out, const float* __restrict__ q, const float* __restrict__ k,
-                  const float* __restrict__ v, int ld, const float* __restrict__ head_decay,
-                  const float* __restrict__ chan_decay, int ld_decay, float q_scale, float k_scale, int act,
-                  float* __restrict__ state, const int32_t* __restrict__ slots, const uint32_t* __restrict__ cu,
-                  const uint32_t* __restrict__ ctx, int heads, int dim, int vdim) {
-  constexpr int RS = kRowSplit, NR = DK / RS, SEG = NR + kDecayPad, DKP = RS * SEG, kChunk = decay_chunk_for(DK, CHAN);
-  constexpr int UN = 4;              // tokens per round of the walk
-  __shared__ __align__(16) float ks[2][kChunk][DKP], qs[2][kChunk][DKP],
-      as[CHAN ? 2 : 1][CHAN ? kChunk : 1][CHAN ? DKP : 4], vs[2][kChunk][kScanCols];
-  const int h = blockIdx.y, b = blockIdx.z;
-  const int part = threadIdx.x % RS;
-  const int col = blockIdx.x * (blockDim.x / RS) + threadIdx.x / RS;
-  const bool live = col < vdim;
-  const int t0 = cu[b], t1 = cu[b + 1];
-  if (t1 <= t0) return;
-  const bool fresh = static_cast<int>(ctx[b]) == t1 - t0;
-  float* sp = state + ((static_cast<size_t>(slots[b]) * heads + h) * dim) * vdim + col;
-  float s[NR];
-#pragma unroll
-  for (int j = 0; j < NR; ++j) {
-    const int i = part * NR + j;
-    s[j] = (!fresh && live && i < dim) ? sp[static_cast<size_t>(i) * vdim] : 0.f;
-  }
-  const float hd = CHAN ? 0.f : head_decay[h];
-  if (dim < DK)                          // rows past `dim` stay zero (the padding between segments is never read)
-    for (int e = threadIdx.x; e < 2 * kChunk * DKP; e += kScanThreads) {
-      (&ks[0][0][0])[e] = (&qs[0][0][0])[e] = 0.f;
-      if (CHAN) (&as[0][0][0])[e] = 0.f;
-    }
-  for (int e = threadIdx.x; e < 2 * kChunk * kScanCols; e += kScanThreads) (&vs[0][0][0])[e] = 0.f;
-  __syncthreads();
-  auto at = [](int i) { return i + (i / NR) * kDecayPad; };       // place of row i in a padded token row
-  // 16-byte copies where four consecutive rows share a segment and every source address is 16-byte aligned
-  const bool wide = NR % 4 == 0 && dim % 4 == 0 && ld % 4 == 0 && (!CHAN || ld_decay % 4 == 0) &&
-                    ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) |
-                      (CHAN ? reinterpret_cast<uintptr_t>(chan_decay) : 0)) & 15) == 0;
-  auto fetch = [&](int c0, int buf) {
-    const int n = min(kChunk, t1 - c0);
-    if (wide) {
-      const int d4 = dim / 4;
-      for (int e = threadIdx.x; e < n * d4; e += kScanThreads) {
-        const int r = e / d4, i = (e - r * d4) * 4;
-        cp_async16(&ks[buf][r][at(i)], k + static_cast<size_t>(c0 + r) * ld + h * dim + i);
-        cp_async16(&qs[buf][r][at(i)], q + static_cast<size_t>(c0 + r) * ld + h * dim + i);
-        if (CHAN) cp_async16(&as[buf][r][at(i)], chan_decay + static_cast<size_t>(c0 + r) * ld_decay + h * dim + i);
-      }
-    } else {
-      for (int e = threadIdx.x; e < n * dim; e += kScanThreads) {
-        const int r = e / dim, i = e - r * dim;
-        cp_async4(&ks[buf][r][at(i)], k + static_cast<size_t>(c0 + r) * ld + h * dim + i);
-        cp_async4(&qs[buf][r][at(i)], q + static_cast<size_t>(c0 + r) * ld + h * dim + i);
-        if (CHAN) cp_async4(&as[buf][r][at(i)], chan_decay + static_cast<size_t>(c0 + r) * ld_decay + h * dim + i);
-      }
-    }
-    for (int e = threadIdx.x; e < n * kScanCols; e += kScanThreads) {
-      const int r = e / kScanCols, c = blockIdx.x * kScanCols + e % kScanCols;
-      if (c < vdim) cp_async4(&vs[buf][r][e % kScanCols], v + static_cast<size_t>(c0 + r) * ld + h * vdim + c);
-    }
-    cp_async_commit();
-  };
-  // NR floats of a lane's segment: 16-byte loads where the segment is a whole number of them
-  auto load_seg = [&](float* dst, const float* src) {
-    if constexpr (NR % 4 == 0) {
-#pragma unroll
-      for (int j = 0; j < NR; j += 4) {
-        const float4 x = *reinterpret_cast<const float4*>(src + j);
-        dst[j] = x.x; dst[j + 1] = x.y; dst[j + 2] = x.z; dst[j + 3] = x.w;
-      }
-    } else {
-#pragma unroll
-      for (int j = 0; j < NR; ++j) dst[j] = src[j];
-    }
-  };
-  fetch(t0, 0);
-  int buf = 0;
-  for (int c0 = t0; c0 < t1; c0 += kChunk, buf ^= 1) {
-    const int n = min(kChunk, t1 - c0);
-    if (c0 + kChunk < t1) {
-      fetch(c0 + kChunk, buf ^ 1);         // the other buffer's tokens were walked before the last barrier
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
-    }
-    __syncthreads();
-    // activation of the pass, in place
-    if (act) {
-      for (int e = threadIdx.x; e < n * dim; e += kScanThreads) {
-        const int r = e / dim, i = at(e - r * dim);
-        ks[buf][r][i] = silu_exact(ks[buf][r][i]);
-        qs[buf][r][i] = silu_exact(qs[buf][r][i]);
-      }
-      for (int e = threadIdx.x; e < n * kScanCols; e += kScanThreads)
-        vs[buf][e / kScanCols][e % kScanCols] = silu_exact(vs[buf][e / kScanCols][e % kScanCols]);
-      __syncthreads();
-    }
-    for (int r = 0; r < n; r += UN) {      // n is the same in every thread: the guards below do not diverge
-      float y[UN];
-#pragma unroll
-      for (int u = 0; u < UN; ++u) {
-        y[u] = 0.f;
-        if (r + u < n) {
-          float kr[NR], qr[NR], ar[CHAN ? NR : 1];
-          load_seg(kr, &ks[buf][r + u][part * SEG]);
-          load_seg(qr, &qs[buf][r + u][part * SEG]);
-          if (CHAN) load_seg(ar, &as[buf][r + u][part * SEG]);
-          const float vv = vs[buf][r + u][threadIdx.x / RS] * k_scale;      // (s k) v^T = k (s v)^T: one factor, not `dim`
-          float y0 = 0.f, y1 = 0.f;
-#pragma unroll
-          for (int j = 0; j < NR; j += 2) {
-            s[j] = (CHAN ? ar[j] : hd) * s[j] + kr[j] * vv;
-            y0 += qr[j] * s[j];
-            if (j + 1 < NR) {
-              s[j + 1] = (CHAN ? ar[CHAN ? j + 1 : 0] : hd) * s[j + 1] + kr[j + 1] * vv;
-              y1 += qr[j + 1] * s[j + 1];
-            }
-          }
-          y[u] = (y0 + y1) * q_scale;
-        }
-      }
-#pragma unroll
-      for (int o = 1; o < RS; o <<= 1)
-#pragma unroll
-        for (int u = 0; u < UN; ++u) y[u] += __shfl_xor_sync(0xffffffffu, y[u], o);
-#pragma unroll
-      for (int u = 0; u < UN; ++u)           // lane `u` of the column stores token r + u
-        if (live && part == u && r + u < n) out[(static_cast<size_t>(c0 + r + u) * heads + h) * vdim + col] = y[u];
-    }
-    __syncthreads();                       // this buffer is refilled by the next pass's fetch
-  }
-  if (live) {
-#pragma unroll
-    for (int j = 0; j < NR; ++j) {
-      const int i = part * NR + j;
-      if (i < dim) sp[static_cast<size_t>(i) * vdim] = s[j];
-    }
-  }
-}
-
 void launch_short_conv_silu(float* out, int ldo, const float* x, int ldx, const float* taps_w, const float* bias,
                             float* state, const int32_t* slots, const uint32_t* cu, const uint32_t* ctx, int num_seqs,
                             int num_rows, int C, int taps, cudaStream_t st_) {
@@ -561,28 +862,14 @@ void launch_delta_rule(float* out, const float* q, const float* k, const float* 
                        int ld_decay, float* state, const int32_t* slots, const uint32_t* cu, const uint32_t* ctx,
                        int num_seqs, int heads, int kv_heads, int dim, int vdim, cudaStream_t st_) {
   if (num_seqs <= 0) return;
-  const int th = kScanThreads;
-  const dim3 grid((vdim + kScanCols - 1) / kScanCols, heads, num_seqs);
-#define B200_DELTA2(DK, CH)                                                                                        \
-  delta_rule_kernel<DK, CH><<<grid, th, 0, st_>>>(out, q, k, v, ld, b_raw, a_raw, ld_ba, a_log, dt_bias, chan_decay, \
-                                                  ld_decay, state, slots, cu, ctx, heads, kv_heads, dim, vdim)
-#define B200_DELTA(DK)                     \
-  {                                        \
-    if (chan_decay) B200_DELTA2(DK, true); \
-    else B200_DELTA2(DK, false);           \
-  }
-  if (dim <= 16) B200_DELTA(16)
-  else if (dim <= 32) B200_DELTA(32)
-  else if (dim <= 64) B200_DELTA(64)
-  else if (dim <= 128) B200_DELTA(128)
-  else if (dim <= 256) B200_DELTA(256)
-  else {
+  if (dim > 256) {
     set_error(1, "delta_rule: key dimension above 256 is not supported");
     return;
   }
-#undef B200_DELTA
-#undef B200_DELTA2
-  B200_CUDA_LAUNCH_CHECK();
+  const ScanArgs s{out, q, k, v, ld, b_raw, a_raw, ld_ba, a_log, dt_bias, nullptr, nullptr, chan_decay, ld_decay, 1.f, 1.f, 0,
+                   state, slots, cu, ctx, heads, kv_heads, dim, vdim};
+  if (chan_decay) launch_scan<kDelta, true>(s, num_seqs, st_);
+  else launch_scan<kDelta, false>(s, num_seqs, st_);
 }
 
 void launch_ssd_scan(float* out, const float* x, const float* Bm, const float* Cm, int ld, const float* dt_raw,
@@ -590,24 +877,14 @@ void launch_ssd_scan(float* out, const float* x, const float* Bm, const float* C
                      const int32_t* slots, const uint32_t* cu, const uint32_t* ctx, int num_seqs, int heads, int groups,
                      int nstate, int vdim, cudaStream_t st_) {
   if (num_seqs <= 0) return;
-  const int th = kScanThreads;
-  const dim3 grid((vdim + kScanCols - 1) / kScanCols, heads, num_seqs);
-#define B200_SSD(NS)                                                                                               \
-  ssd_scan_kernel<NS><<<grid, th, 0, st_>>>(out, x, Bm, Cm, ld, dt_raw, ld_dt, a_log, dt_bias, d_skip, state, slots, \
-                                            cu, ctx, heads, groups, nstate, vdim)
-  if (nstate <= 16) B200_SSD(16);
-  else if (nstate <= 32) B200_SSD(32);
-  else if (nstate <= 64) B200_SSD(64);
-  else if (nstate <= 128) B200_SSD(128);
-  else if (nstate <= 256) B200_SSD(256);
-  else {
+  if (nstate > 256) {
     set_error(1, "ssd_scan: state size above 256 is not supported");
     return;
   }
-#undef B200_SSD
-  B200_CUDA_LAUNCH_CHECK();
+  const ScanArgs s{out, Cm, Bm, x, ld, nullptr, dt_raw, ld_dt, a_log, dt_bias, d_skip, nullptr, nullptr, 0, 1.f, 1.f, 0,
+                   state, slots, cu, ctx, heads, groups, nstate, vdim};
+  launch_scan<kSsd, false>(s, num_seqs, st_);
 }
-
 
 void launch_lowrank_decay(float* out, const float* low, int ld_low, const float* w2, const float* bias, float tau,
                           const float* a_log, int a_period, int T, int C, int rank, cudaStream_t st_) {
@@ -627,28 +904,14 @@ void launch_decay_attn(float* out, const float* q, const float* k, const float* 
                        const int32_t* slots, const uint32_t* cu, const uint32_t* ctx, int num_seqs, int heads, int dim,
                        int vdim, cudaStream_t st_) {
   if (num_seqs <= 0) return;
-  const int th = kScanThreads;
-  const dim3 grid((vdim + kScanCols - 1) / kScanCols, heads, num_seqs);
-#define B200_DECAY2(DK, CH)                                                                                          \
-  decay_attn_kernel<DK, CH><<<grid, th, 0, st_>>>(out, q, k, v, ld, head_decay, chan_decay, ld_decay, q_scale, k_scale, \
-                                                  act, state, slots, cu, ctx, heads, dim, vdim)
-#define B200_DECAY(DK)          \
-  {                             \
-    if (chan_decay) B200_DECAY2(DK, true); \
-    else B200_DECAY2(DK, false);           \
-  }
-  if (dim <= 16) B200_DECAY(16)
-  else if (dim <= 32) B200_DECAY(32)
-  else if (dim <= 64) B200_DECAY(64)
-  else if (dim <= 128) B200_DECAY(128)
-  else if (dim <= 256) B200_DECAY(256)
-  else {
+  if (dim > 256) {
     set_error(1, "decay_attn: key dimension above 256 is not supported");
     return;
   }
-#undef B200_DECAY
-#undef B200_DECAY2
-  B200_CUDA_LAUNCH_CHECK();
+  const ScanArgs s{out, q, k, v, ld, nullptr, nullptr, 0, nullptr, nullptr, nullptr, head_decay, chan_decay, ld_decay,
+                   q_scale, k_scale, act, state, slots, cu, ctx, heads, heads, dim, vdim};
+  if (chan_decay) launch_scan<kDecay, true>(s, num_seqs, st_);
+  else launch_scan<kDecay, false>(s, num_seqs, st_);
 }
 
 }  // namespace b200
