@@ -28,6 +28,7 @@
 // never quotients.  All fp32.
 #include "../../include/b200_vllm.h"
 #include <algorithm>
+#include <type_traits>
 
 #include "seqmix.cuh"
 
@@ -162,7 +163,8 @@ template <int DK, bool CHAN> struct ScanSmem {
   static constexpr int kRows = kBT * DK;                                        // floats of one array of token rows
   static constexpr int kV = (CHAN ? 3 : 2) * kRows;                             // k | q | decays | v | scalars | T, P (8 x 8 each) | ..
   static constexpr int kG = kV + kBT * kScanCols, kMat = kG + 4 * kBT;          // decay, strength, G_t, W_t per token
-  static constexpr int kGend = kMat + 2 * kBT * kBT;                            // CHAN: [DK] decays over the block
+  static constexpr int kRat = kMat + 2 * kBT * kBT;                             // [t][j] decay from token j to token t
+  static constexpr int kGend = kRat + kBT * kBT;                                // CHAN: [DK] decays over the block
   static constexpr int kBuf = kGend + (CHAN ? DK : 0);
   static constexpr int kU = kRing * kBuf;                                       // [4 warps][8 tokens][4 columns]
   static constexpr int kBars = kU + 4 * kBT * 4;
@@ -259,20 +261,24 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
           const float* kg = a.k + static_cast<size_t>(c0) * a.ld + hk * dim;
           const float* qg = a.q + static_cast<size_t>(c0) * a.ld + hk * dim;
           const float* ag = CHAN ? a.chan_decay + static_cast<size_t>(c0) * a.ld_decay + h * dim : nullptr;
-          if (wide) {
-            const int d4 = dim / 4;
-            for (int e = pt; e < n * d4; e += 128) {
-              const int r = e / d4, x = (e - r * d4) * 4, o = r * DK + x;
-              cp_async16(B + o, kg + static_cast<size_t>(r) * a.ld + x);
-              cp_async16(B + SM::kRows + o, qg + static_cast<size_t>(r) * a.ld + x);
+          constexpr int TPR = DK / 4, RPS = 128 / TPR;                 // threads per row, rows at a time
+          const int x = pt % TPR * 4;
+#pragma unroll
+          for (int r = pt / TPR; r < kBT; r += RPS) {
+            if (r >= n || x >= dim) continue;
+            const int o = r * DK + x;
+            const float* ks_ = kg + static_cast<size_t>(r) * a.ld + x;
+            const float* qs_ = qg + static_cast<size_t>(r) * a.ld + x;
+            if (wide) {
+              cp_async16(B + o, ks_);
+              cp_async16(B + SM::kRows + o, qs_);
               if (CHAN) cp_async16(B + 2 * SM::kRows + o, ag + static_cast<size_t>(r) * a.ld_decay + x);
-            }
-          } else {
-            for (int e = pt; e < n * dim; e += 128) {
-              const int r = e / dim, x = e - r * dim, o = r * DK + x;
-              cp_async4(B + o, kg + static_cast<size_t>(r) * a.ld + x);
-              cp_async4(B + SM::kRows + o, qg + static_cast<size_t>(r) * a.ld + x);
-              if (CHAN) cp_async4(B + 2 * SM::kRows + o, ag + static_cast<size_t>(r) * a.ld_decay + x);
+            } else {
+              for (int z = 0; z < min(4, dim - x); ++z) {
+                cp_async4(B + o + z, ks_ + z);
+                cp_async4(B + SM::kRows + o + z, qs_ + z);
+                if (CHAN) cp_async4(B + 2 * SM::kRows + o + z, ag + static_cast<size_t>(r) * a.ld_decay + x + z);
+              }
             }
           }
           const float* vg = a.v + static_cast<size_t>(c0) * a.ld + h * vdim + col0;
@@ -282,11 +288,6 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
           } else {
             const int r = pt >> 4, c = pt & 15;
             if (r < n && col0 + c < vdim) cp_async4(B + SM::kV + pt, vg + static_cast<size_t>(r) * a.ld + c);
-          }
-          if (pt < n) {
-            const size_t o = static_cast<size_t>(c0 + pt) * a.ld_ba + h;
-            if (MODE == kDelta) cp_async4(B + SM::kG + kBT + pt, a.b_raw + o);
-            if (MODE == kSsd || (MODE == kDelta && !CHAN)) cp_async4(B + SM::kG + pt, a.a_raw + o);
           }
         }
         cp_async_commit();
@@ -298,156 +299,187 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
       const float neg_a = MODE == kDecay || CHAN ? 0.f : -expf(a.a_log[h]), dtb = MODE == kDecay || CHAN ? 0.f : a.dt_bias[h];
       const float hd = MODE == kDecay && !CHAN ? a.head_decay[h] : 1.f;
       const float qn = rsqrtf(static_cast<float>(dim));
+      // The scalars of a block, by warp 3, one block ahead: raw values in registers, then decays, strengths, products.
+      float raw_b = 0.f, raw_a = 0.f;
+      auto read_scalars = [&](int i) {
+        const int t = t0 + i * kBT + lane;
+        if (lane >= kBT || t >= t1) return;
+        const size_t o = static_cast<size_t>(t) * a.ld_ba + h;
+        if (MODE == kDelta) raw_b = a.b_raw[o];
+        if (MODE == kSsd || (MODE == kDelta && !CHAN)) raw_a = a.a_raw[o];
+      };
+      auto make_scalars = [&](int i) {
+        float* G = sm + (blocks + i) % kRing * SM::kBuf + SM::kG;
+        float g = 1.f, w = 0.f;                        // decay; write strength
+        if (lane < kBT && t0 + i * kBT + lane < t1) {
+          if (MODE == kDelta) {
+            w = sigmoid_f(raw_b);
+            if (!CHAN) g = expf(neg_a * softplus_f(raw_a + dtb));
+          } else if (MODE == kSsd) {
+            w = softplus_f(raw_a + dtb);
+            g = expf(neg_a * w);
+          } else {
+            w = a.k_scale;
+            g = hd;
+          }
+        }
+        // decay from token j to token t: the products g_(j+1) .. g_t; from the block's start, and to its end
+        float* R = G + (SM::kRat - SM::kG);
+#pragma unroll
+        for (int z = 0; z < 2; ++z) {
+          const int t = (lane >> 3) + z * 4, j = lane & 7;
+          float r = 1.f;
+#pragma unroll
+          for (int m = 1; m < kBT; ++m) {
+            const float gm = __shfl_sync(0xffffffffu, g, m);
+            if (m > j && m <= t) r *= gm;
+          }
+          R[t * kBT + j] = r;
+          if (j == 0) G[2 * kBT + t] = r * __shfl_sync(0x01010101u, g, 0);
+          if (t == kBT - 1) G[3 * kBT + j] = r;
+        }
+        if (lane < kBT) {
+          G[lane] = g;
+          G[kBT + lane] = w;
+        }
+      };
+      // which entry of a triangle, row after row, this lane gets: M (rows 1 .., j < t) for warp 1, P (j <= t) from row 4 on for warp
+      // 0, of rows 0 - 3 for warp 2
+      int et = pw == 1 ? 1 : pw == 0 ? 4 : 0, ej = lane;
+      const int et_end = pw == 2 ? 4 : kBT;
+      while (et < et_end && ej >= (pw == 1 ? et : et + 1)) {
+        ej -= pw == 1 ? et : et + 1;
+        ++et;
+      }
       fetch(0);
       fetch(1);
+      if (pw == 3) {
+        read_scalars(0);
+        make_scalars(0);
+      }
       for (int i = 0; i < nblk; ++i) {
         fetch(i + 2);
+        if (pw == 3) read_scalars(i + 1);
         cp_async_wait<2>();
         sync();
         float* B = sm + (blocks + i) % kRing * SM::kBuf;
-        float* G = B + SM::kG;
+        const float* G = B + SM::kG;
         const int n = min(kBT, t1 - t0 - i * kBT);
         // ---- two tokens per warp: norms or activation, in place; past the end: no key, no value, decay one
-#pragma unroll
-        for (int z = 0; z < 2; ++z) {
-          const int r = pw * 2 + z;
-          float* kr = B + r * DK + lane * CH;
-          float* qr = kr + SM::kRows;
-          float kx[CH], qx[CH];
-          if (r < n) {
-            if (MODE == kDelta || (MODE == kDecay && a.act)) {
-              ldv<CH>(kx, kr);
-              ldv<CH>(qx, qr);
-              if (MODE == kDelta) {
-                float sk = 0.f, sq = 0.f;
-#pragma unroll
-                for (int j = 0; j < CH; ++j) {
-                  sk += kx[j] * kx[j];
-                  sq += qx[j] * qx[j];
-                }
-                sk = lanes_sum(sk);
-                sq = lanes_sum(sq);
-                const float ik = 1.f / sqrtf(sk + 1e-6f), iq = qn / sqrtf(sq + 1e-6f);
-#pragma unroll
-                for (int j = 0; j < CH; ++j) {
-                  kx[j] *= ik;
-                  qx[j] *= iq;
-                }
-              } else {
-#pragma unroll
-                for (int j = 0; j < CH; ++j) {
-                  kx[j] = silu_exact(kx[j]);
-                  qx[j] = silu_exact(qx[j]);
-                }
-                if (lane < kScanCols) B[SM::kV + r * kScanCols + lane] = silu_exact(B[SM::kV + r * kScanCols + lane]);
-              }
-              stv<CH>(kr, kx);
-              stv<CH>(qr, qx);
-            }
-          } else {
-#pragma unroll
-            for (int j = 0; j < CH; ++j) kx[j] = 0.f;
-            stv<CH>(kr, kx);
-            stv<CH>(qr, kx);
-            if (lane < kScanCols) B[SM::kV + r * kScanCols + lane] = 0.f;
-            if (CHAN) {
-#pragma unroll
-              for (int j = 0; j < CH; ++j) kx[j] = 1.f;
-              stv<CH>(kr + 2 * SM::kRows, kx);
-            }
-          }
-        }
-        if (pw == 3 && lane < kBT) {
-          float g = 1.f, w = 0.f;                      // decay; write strength
-          if (lane < n) {
-            if (MODE == kDelta) {
-              w = sigmoid_f(G[kBT + lane]);
-              if (!CHAN) g = expf(neg_a * softplus_f(G[lane] + dtb));
-            } else if (MODE == kSsd) {
-              w = softplus_f(G[lane] + dtb);
-              g = expf(neg_a * w);
-            } else {
-              w = a.k_scale;
-              g = hd;
-            }
-          }
-          float up = g, down = 1.f;                    // products of decays up to a token, and behind it
-#pragma unroll
-          for (int o = 1; o < kBT; o <<= 1) {
-            const float x = __shfl_up_sync(0xffu, up, o);
-            if (lane >= o) up *= x;
-          }
-          float tail = g;
-#pragma unroll
-          for (int o = 1; o < kBT; o <<= 1) {
-            const float x = __shfl_down_sync(0xffu, tail, o);
-            if (lane + o < kBT) tail *= x;
-          }
-          const float after = __shfl_down_sync(0xffu, tail, 1);
-          if (lane + 1 < kBT) down = after;
-          G[lane] = g;
-          G[kBT + lane] = w;
-          G[2 * kBT + lane] = up;
-          G[3 * kBT + lane] = down;
-        }
-        sync();
-        // ---- warp 0: P (t, j) = decayed q_t . k_j, j <= t.  warp 1 (delta): M (t, j) = beta_t times the decayed k_t . k_j, j < t,
-        // and T = (1 + M)^-1.  A lane holds its rows of all eight tokens.
-        if (pw == 0 || (pw == 1 && MODE == kDelta)) {
-          float y[kBT][CH], x[64];
-#pragma unroll
-          for (int t = 0; t < kBT; ++t) ldv<CH>(y[t], B + t * DK + lane * CH);
-#pragma unroll
-          for (int t = 0; t < kBT; ++t) {
-            float xt[CH], dt[CH];
-            ldv<CH>(xt, B + (pw == 0 ? SM::kRows : 0) + t * DK + lane * CH);
-            if (CHAN) {                                // y[j] becomes k_j decayed up to token t
-              ldv<CH>(dt, B + 2 * SM::kRows + t * DK + lane * CH);
-#pragma unroll
-              for (int j = 0; j < kBT; ++j)
-                if (j < t) {
-#pragma unroll
-                  for (int c = 0; c < CH; ++c) y[j][c] *= dt[c];
-                }
-            }
-#pragma unroll
-            for (int j = 0; j < kBT; ++j) {
-              float acc = 0.f;
-              if (j <= t) {
-#pragma unroll
-                for (int c = 0; c < CH; ++c) acc += xt[c] * y[j][c];
-              }
-              x[t * kBT + j] = acc;
-            }
-          }
-          // sums over the lanes: lane l gets entries l and l + 32
-          float lo[32], hi[32];
-#pragma unroll
-          for (int e = 0; e < 32; ++e) {
-            lo[e] = x[e];
-            hi[e] = x[32 + e];
-          }
-          float ent[2] = {meet32(lo, lane), meet32(hi, lane)};
-          float* out = B + SM::kMat + (pw == 0 ? kBT * kBT : 0);
+        if (MODE == kDelta || (MODE == kDecay && a.act) || n < kBT) {
+          float kx[2][CH], qx[2][CH], sk[2] = {0.f, 0.f}, sq[2] = {0.f, 0.f};
+          float* kr = B + pw * 2 * DK + lane * CH;
 #pragma unroll
           for (int z = 0; z < 2; ++z) {
-            const int t = (lane >> 3) + z * 4, j = lane & 7;
-            float v = ent[z];
-            for (int m = j + 1; m <= t; ++m) v *= G[m];
-            if (pw == 1) v = t > j ? v * G[kBT + t] : 0.f;
-            out[t * kBT + j] = v;
+            ldv<CH>(kx[z], kr + z * DK);
+            ldv<CH>(qx[z], kr + SM::kRows + z * DK);
+#pragma unroll
+            for (int j = 0; j < CH; ++j) {
+              if (MODE == kDelta) {
+                sk[z] += kx[z][j] * kx[z][j];
+                sq[z] += qx[z][j] * qx[z][j];
+              } else if (MODE == kDecay && a.act) {
+                kx[z][j] = silu_exact(kx[z][j]);
+                qx[z][j] = silu_exact(qx[z][j]);
+              }
+            }
           }
-          if (pw == 1) {                               // column c of T by forward substitution, one lane each
+          float ik[2] = {1.f, 1.f}, iq[2] = {1.f, 1.f};
+          if (MODE == kDelta) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+              for (int z = 0; z < 2; ++z) {
+                sk[z] += __shfl_xor_sync(0xffffffffu, sk[z], o);
+                sq[z] += __shfl_xor_sync(0xffffffffu, sq[z], o);
+              }
+#pragma unroll
+            for (int z = 0; z < 2; ++z) {
+              ik[z] = 1.f / sqrtf(sk[z] + 1e-6f);
+              iq[z] = qn / sqrtf(sq[z] + 1e-6f);
+            }
+          }
+#pragma unroll
+          for (int z = 0; z < 2; ++z) {
+            const int r = pw * 2 + z;
+            const bool in = r < n;
+#pragma unroll
+            for (int j = 0; j < CH; ++j) {
+              kx[z][j] = in ? kx[z][j] * ik[z] : 0.f;
+              qx[z][j] = in ? qx[z][j] * iq[z] : 0.f;
+            }
+            stv<CH>(kr + z * DK, kx[z]);
+            stv<CH>(kr + SM::kRows + z * DK, qx[z]);
+            if (CHAN && !in) {
+#pragma unroll
+              for (int j = 0; j < CH; ++j) kx[z][j] = 1.f;
+              stv<CH>(kr + 2 * SM::kRows + z * DK, kx[z]);
+            }
+            if (lane < kScanCols) {
+              float* v = B + SM::kV + r * kScanCols + lane;
+              if (!in) *v = 0.f;
+              else if (MODE == kDecay && a.act) *v = silu_exact(*v);
+            }
+          }
+        }
+        sync();
+        // ---- P (t, j) = decayed q_t . k_j, j <= t, and (delta) M (t, j) = beta_t times the decayed k_t . k_j, j < t, then
+        // T = (1 + M)^-1.  A lane holds its rows of all eight tokens; the sums over the lanes go an entry to a lane.
+        if (pw == 3) {
+          if (i + 1 < nblk) make_scalars(i + 1);
+        } else if (pw != 1 || MODE == kDelta) {
+          auto entries = [&](auto first, auto last, auto strict, const float* rows) {
+            constexpr int F = decltype(first)::value, L = decltype(last)::value, ST = decltype(strict)::value;
+            float y[kBT][CH], x[32];
+#pragma unroll
+            for (int e = 0; e < 32; ++e) x[e] = 0.f;
+            int e = 0;
+#pragma unroll
+            for (int t = 0; t < L; ++t) {
+              ldv<CH>(y[t], B + t * DK + lane * CH);
+              if (CHAN) {                              // y[j] becomes k_j decayed up to token t
+                float dt[CH];
+                ldv<CH>(dt, B + 2 * SM::kRows + t * DK + lane * CH);
+#pragma unroll
+                for (int j = 0; j < t; ++j)
+#pragma unroll
+                  for (int c = 0; c < CH; ++c) y[j][c] *= dt[c];
+              }
+              if (t < F) continue;
+              float xt[CH];
+              ldv<CH>(xt, rows + t * DK + lane * CH);
+#pragma unroll
+              for (int j = 0; j <= t - ST; ++j) {
+                float acc = xt[0] * y[j][0];
+#pragma unroll
+                for (int c = 1; c < CH; ++c) acc += xt[c] * y[j][c];
+                x[e++] = acc;
+              }
+            }
+            return meet32(x, lane);
+          };
+          using std::integral_constant;
+          const float* K = B;
+          const float* Q = B + SM::kRows;
+          float v = pw == 1   ? entries(integral_constant<int, 1>{}, integral_constant<int, kBT>{}, integral_constant<int, 1>{}, K)
+                    : pw == 0 ? entries(integral_constant<int, 4>{}, integral_constant<int, kBT>{}, integral_constant<int, 0>{}, Q)
+                              : entries(integral_constant<int, 0>{}, integral_constant<int, 4>{}, integral_constant<int, 0>{}, Q);
+          float* out = B + SM::kMat + (pw == 1 ? 0 : kBT * kBT);
+          if (et < et_end) {
+            v *= B[SM::kRat + et * kBT + ej];
+            out[et * kBT + ej] = pw == 1 ? v * G[kBT + et] : v;
+          }
+          if (pw == 1) {                               // column `lane` of T by forward substitution
             __syncwarp();
             float tc[kBT];
-            if (lane < kBT) {
 #pragma unroll
-              for (int t = 0; t < kBT; ++t) {
-                float acc = t == lane ? 1.f : 0.f;
+            for (int t = 0; t < kBT; ++t) {
+              const float4 ma = *reinterpret_cast<const float4*>(out + t * kBT), mb = *reinterpret_cast<const float4*>(out + t * kBT + 4);
+              const float m[kBT] = {ma.x, ma.y, ma.z, ma.w, mb.x, mb.y, mb.z, mb.w};
+              float acc = t == lane ? 1.f : 0.f;
 #pragma unroll
-                for (int j = 0; j < t; ++j) acc -= out[t * kBT + j] * tc[j];
-                tc[t] = acc;
-              }
+              for (int j = 0; j < t; ++j) acc -= m[j] * tc[j];
+              tc[t] = acc;
             }
             __syncwarp();
             if (lane < kBT) {
