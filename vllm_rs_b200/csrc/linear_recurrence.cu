@@ -141,6 +141,7 @@ __device__ __forceinline__ void unpack2(f2 v, float& lo, float& hi) { asm("mov.b
 constexpr int kScanCols = 16;                  // columns of S per block of threads
 constexpr int kBT = 8;                         // tokens per block of the recurrence
 constexpr int kRing = 4;                       // blocks of tokens in shared memory: walked, prepared, two on their way
+constexpr int kScanThreads = 384;
 constexpr int kDelta = 0, kDecay = 1, kSsd = 2;
 
 struct ScanArgs {
@@ -219,11 +220,11 @@ __device__ __forceinline__ float meet32(float (&x)[32], int lane) {
 // Portions of two tokens and more.  grid = (column blocks, heads, runs of sequences); a block walks its sequences one after
 // another.  Warps 0-3 each own four columns of S: a lane holds DK / 32 neighbouring rows of them in registers, so that a key or
 // query row is read once from shared memory for four columns (one column per lane made these reads the bound: 512 bytes of
-// registers per load and warp).  Warps 4-7 fetch the token rows (cp.async, two blocks of eight tokens ahead), norm or
-// activate them and prepare the block's triangles under the walk of the block before.
-// 4096 tokens, 16 heads of 128 x 128: BEFORE us token by token (1020 cycles per token), AFTER us.
+// registers per load and warp).  Warps 4-7 and 8-11 take turns at fetching a block's token rows (cp.async, a block ahead of
+// each), norming or activating them and preparing its triangles under the walks of the blocks before; one such group takes
+// longer than a walk (3300 against 1950 cycles for the delta rule), two do not.
 template <int DK, int MODE, bool CHAN>
-__global__ void __launch_bounds__(256, 2)
+__global__ void __launch_bounds__(kScanThreads, 1)
 scan_kernel(const ScanArgs a, int num_seqs, int* err) {
   using SM = ScanSmem<DK, CHAN>;
   constexpr int CH = DK / 32;
@@ -238,7 +239,7 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
     *fail = 0;
     fence_barrier_init();
   }
-  for (int e = tid; e < kRing * SM::kBuf; e += 256) sm[e] = 0.f;       // padding past `dim` is zero and stays it
+  for (int e = tid; e < kRing * SM::kBuf; e += kScanThreads) sm[e] = 0.f;       // padding past `dim` is zero and stays it
   __syncthreads();
   int blocks = 0;                                                      // blocks of tokens so far, over all sequences
   for (int b = blockIdx.z; b < num_seqs; b += gridDim.z) {
@@ -247,7 +248,7 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
     const bool fresh = static_cast<int>(a.ctx[b]) == t1 - t0;
     if (warp >= 4) {
       // ---------------------------------------------------------- token rows
-      const int pt = tid - 128, pw = warp - 4;
+      const int pt = tid & 127, pw = warp & 3, grp = (warp >> 2) - 1;
       const bool wide = dim % 4 == 0 && a.ld % 4 == 0 && (!CHAN || a.ld_decay % 4 == 0) &&
                         ((reinterpret_cast<uintptr_t>(a.q) | reinterpret_cast<uintptr_t>(a.k) |
                           (CHAN ? reinterpret_cast<uintptr_t>(a.chan_decay) : 0)) & 15) == 0;
@@ -292,14 +293,14 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
         }
         cp_async_commit();
       };
-      auto sync = [] {                                 // of these four warps
+      auto sync = [&] {                                // of these four warps
         __syncwarp();
-        asm volatile("bar.sync 1, 128;" ::: "memory");
+        asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory");
       };
       const float neg_a = MODE == kDecay || CHAN ? 0.f : -expf(a.a_log[h]), dtb = MODE == kDecay || CHAN ? 0.f : a.dt_bias[h];
       const float hd = MODE == kDecay && !CHAN ? a.head_decay[h] : 1.f;
       const float qn = rsqrtf(static_cast<float>(dim));
-      // The scalars of a block, by warp 3, one block ahead: raw values in registers, then decays, strengths, products.
+      // The scalars of a block, by the group's last warp, a block ahead: raw values in registers, then decays, strengths, products.
       float raw_b = 0.f, raw_a = 0.f;
       auto read_scalars = [&](int i) {
         const int t = t0 + i * kBT + lane;
@@ -351,16 +352,15 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
         ej -= pw == 1 ? et : et + 1;
         ++et;
       }
-      fetch(0);
-      fetch(1);
-      if (pw == 3) {
-        read_scalars(0);
-        make_scalars(0);
+      fetch(grp);
+      if (pw == 3 && grp < nblk) {
+        read_scalars(grp);
+        make_scalars(grp);
       }
-      for (int i = 0; i < nblk; ++i) {
+      for (int i = grp; i < nblk; i += 2) {
         fetch(i + 2);
-        if (pw == 3) read_scalars(i + 1);
-        cp_async_wait<2>();
+        if (pw == 3) read_scalars(i + 2);
+        cp_async_wait<1>();
         sync();
         float* B = sm + (blocks + i) % kRing * SM::kBuf;
         const float* G = B + SM::kG;
@@ -426,7 +426,7 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
         // ---- P (t, j) = decayed q_t . k_j, j <= t, and (delta) M (t, j) = beta_t times the decayed k_t . k_j, j < t, then
         // T = (1 + M)^-1.  A lane holds its rows of all eight tokens; the sums over the lanes go an entry to a lane.
         if (pw == 3) {
-          if (i + 1 < nblk) make_scalars(i + 1);
+          if (i + 2 < nblk) make_scalars(i + 2);
         } else if (pw != 1 || MODE == kDelta) {
           auto entries = [&](auto first, auto last, auto strict, const float* rows) {
             constexpr int F = decltype(first)::value, L = decltype(last)::value, ST = decltype(strict)::value;
@@ -812,7 +812,7 @@ static void launch_scan_dk(const ScanArgs& a, int num_seqs, cudaStream_t st_) {
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   // portions: a few blocks per SM, each taking every so many sequences (a step of decoded tokens is over at once)
   const int z = std::max(1, std::min(num_seqs, 4 * sm_count() / (cols * a.heads)));
-  kern<<<dim3(cols, a.heads, z), 256, smem, st_>>>(a, num_seqs, err);
+  kern<<<dim3(cols, a.heads, z), kScanThreads, smem, st_>>>(a, num_seqs, err);
   B200_CUDA_LAUNCH_CHECK();
 }
 // dim: rows of the state; at most 256 (the caller has checked)
