@@ -138,10 +138,9 @@ __device__ __forceinline__ f2 mul2(f2 a, f2 b) {
 }
 __device__ __forceinline__ void unpack2(f2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
 
-constexpr int kScanCols = 16;                  // columns of S per block of threads
+constexpr int kOneCols = 16;                   // columns of S per block of threads: single tokens
 constexpr int kBT = 8;                         // tokens per block of the recurrence
 constexpr int kRing = 4;                       // blocks of tokens in shared memory: walked, prepared, two on their way
-constexpr int kScanThreads = 384;
 constexpr int kDelta = 0, kDecay = 1, kSsd = 2;
 
 struct ScanArgs {
@@ -160,15 +159,15 @@ struct ScanArgs {
   int heads, kv_heads, dim, vdim;
 };
 
-template <int DK, bool CHAN> struct ScanSmem {
+template <int DK, bool CHAN, int WW> struct ScanSmem {         // WW: walking warps, four columns each
   static constexpr int kRows = kBT * DK;                                        // floats of one array of token rows
   static constexpr int kV = (CHAN ? 3 : 2) * kRows;                             // k | q | decays | v | scalars | T, P (8 x 8 each) | ..
-  static constexpr int kG = kV + kBT * kScanCols, kMat = kG + 4 * kBT;          // decay, strength, G_t, W_t per token
+  static constexpr int kCols = WW * 4, kG = kV + kBT * kCols, kMat = kG + 4 * kBT;          // decay, strength, G_t, W_t per token
   static constexpr int kRat = kMat + 2 * kBT * kBT;                             // [t][j] decay from token j to token t
   static constexpr int kGend = kRat + kBT * kBT;                                // CHAN: [DK] decays over the block
   static constexpr int kBuf = kGend + (CHAN ? DK : 0);
-  static constexpr int kU = kRing * kBuf;                                       // [4 warps][8 tokens][4 columns]
-  static constexpr int kBars = kU + 4 * kBT * 4;
+  static constexpr int kU = kRing * kBuf;                                       // [WW][8 tokens][4 columns]
+  static constexpr int kBars = kU + WW * kBT * 4;
   static constexpr int kBytes = kBars * 4 + 2 * kRing * 8 + 16;
 };
 // CH floats from shared memory
@@ -218,37 +217,38 @@ __device__ __forceinline__ float meet32(float (&x)[32], int lane) {
 }
 
 // Portions of two tokens and more.  grid = (column blocks, heads, runs of sequences); a block walks its sequences one after
-// another.  Warps 0-3 each own four columns of S: a lane holds DK / 32 neighbouring rows of them in registers, so that a key or
-// query row is read once from shared memory for four columns (one column per lane made these reads the bound: 512 bytes of
-// registers per load and warp).  Warps 4-7 and 8-11 take turns at fetching a block's token rows (cp.async, a block ahead of
-// each), norming or activating them and preparing its triangles under the walks of the blocks before; one such group takes
-// longer than a walk (3300 against 1950 cycles for the delta rule), two do not.
-template <int DK, int MODE, bool CHAN>
-__global__ void __launch_bounds__(kScanThreads, 1)
+// another.  The first WW warps each own four columns of S: a lane holds DK / 32 neighbouring rows of them in registers, so that
+// a key or query row is read once from shared memory for four columns (one column per lane made these reads the bound: 512
+// bytes of registers per load and warp).  Two groups of four warps take turns at fetching a block's token rows (cp.async, a
+// block ahead of each), norming or activating them and preparing its triangles under the walks of the blocks before; one such
+// group takes longer than a walk (3300 against 1950 cycles for the delta rule), two do not.
+// WW = 8 lets two walking warps share a scheduler and a prepared block, WW = 4 spreads few columns over more SMs.
+template <int DK, int MODE, bool CHAN, int WW>
+__global__ void __launch_bounds__(WW * 32 + 256, 1)
 scan_kernel(const ScanArgs a, int num_seqs, int* err) {
-  using SM = ScanSmem<DK, CHAN>;
-  constexpr int CH = DK / 32;
+  using SM = ScanSmem<DK, CHAN, WW>;
+  constexpr int CH = DK / 32, COLS = SM::kCols;
   extern __shared__ __align__(16) float sm[];
   uint64_t* ready = reinterpret_cast<uint64_t*>(sm + SM::kBars);
   uint64_t* done = ready + kRing;
   volatile int* fail = reinterpret_cast<volatile int*>(done + kRing);
-  const int h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, col0 = blockIdx.x * kScanCols;
+  const int h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, col0 = blockIdx.x * COLS;
   const int dim = a.dim, vdim = a.vdim, hk = MODE == kDecay ? h : h / (a.heads / a.kv_heads);
   if (tid == 0) {
-    for (int i = 0; i < kRing; ++i) { mbar_init(&ready[i], 4); mbar_init(&done[i], 4); }
+    for (int i = 0; i < kRing; ++i) { mbar_init(&ready[i], 4); mbar_init(&done[i], WW); }
     *fail = 0;
     fence_barrier_init();
   }
-  for (int e = tid; e < kRing * SM::kBuf; e += kScanThreads) sm[e] = 0.f;       // padding past `dim` is zero and stays it
+  for (int e = tid; e < kRing * SM::kBuf; e += WW * 32 + 256) sm[e] = 0.f;       // padding past `dim` is zero and stays it
   __syncthreads();
   int blocks = 0;                                                      // blocks of tokens so far, over all sequences
   for (int b = blockIdx.z; b < num_seqs; b += gridDim.z) {
     const int t0 = a.cu[b], t1 = a.cu[b + 1], nblk = (t1 - t0 + kBT - 1) / kBT;
     if (t1 - t0 < 2) continue;                                         // (scan_one_kernel)
     const bool fresh = static_cast<int>(a.ctx[b]) == t1 - t0;
-    if (warp >= 4) {
+    if (warp >= WW) {
       // ---------------------------------------------------------- token rows
-      const int pt = tid & 127, pw = warp & 3, grp = (warp >> 2) - 1;
+      const int pt = tid & 127, pw = warp & 3, grp = (warp - WW) >> 2;
       const bool wide = dim % 4 == 0 && a.ld % 4 == 0 && (!CHAN || a.ld_decay % 4 == 0) &&
                         ((reinterpret_cast<uintptr_t>(a.q) | reinterpret_cast<uintptr_t>(a.k) |
                           (CHAN ? reinterpret_cast<uintptr_t>(a.chan_decay) : 0)) & 15) == 0;
@@ -284,11 +284,13 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
           }
           const float* vg = a.v + static_cast<size_t>(c0) * a.ld + h * vdim + col0;
           if (wide_v) {
-            const int r = pt >> 2, c = (pt & 3) * 4;
-            if (r < n && col0 + c < vdim) cp_async16(B + SM::kV + r * kScanCols + c, vg + static_cast<size_t>(r) * a.ld + c);
+            const int r = pt / (COLS / 4), c = pt % (COLS / 4) * 4;
+            if (r < n && col0 + c < vdim) cp_async16(B + SM::kV + r * COLS + c, vg + static_cast<size_t>(r) * a.ld + c);
           } else {
-            const int r = pt >> 4, c = pt & 15;
-            if (r < n && col0 + c < vdim) cp_async4(B + SM::kV + pt, vg + static_cast<size_t>(r) * a.ld + c);
+            for (int e = pt; e < n * COLS; e += 128) {
+              const int r = e / COLS, c = e % COLS;
+              if (col0 + c < vdim) cp_async4(B + SM::kV + e, vg + static_cast<size_t>(r) * a.ld + c);
+            }
           }
         }
         cp_async_commit();
@@ -415,8 +417,8 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
               for (int j = 0; j < CH; ++j) kx[z][j] = 1.f;
               stv<CH>(kr + 2 * SM::kRows + z * DK, kx[z]);
             }
-            if (lane < kScanCols) {
-              float* v = B + SM::kV + r * kScanCols + lane;
+            if (lane < COLS) {
+              float* v = B + SM::kV + r * COLS + lane;
               if (!in) *v = 0.f;
               else if (MODE == kDecay && a.act) *v = silu_exact(*v);
             }
@@ -571,7 +573,7 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
           return meet32(x, lane);
         };
         const float gt = CHAN ? 1.f : G[2 * kBT + tt];
-        const float vt = B[SM::kV + tt * kScanCols + warp * 4 + c4], wt = G[kBT + tt];
+        const float vt = B[SM::kV + tt * COLS + warp * 4 + c4], wt = G[kBT + tt];
         float u = vt * wt;
         if (MODE == kDelta) {
           const float r = wt * (vt - gt * dots(B));
@@ -659,13 +661,13 @@ template <int DK, int MODE, bool CHAN>
 __global__ void __launch_bounds__(128)
 scan_one_kernel(const ScanArgs a) {
   constexpr int NR = DK / 32;
-  __shared__ float ks[DK], qs[DK], red[2][4][kScanCols], sums[4][2];
+  __shared__ float ks[DK], qs[DK], red[2][4][kOneCols], sums[4][2];
   const int h = blockIdx.y, b = blockIdx.z, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int t = a.cu[b];
   if (static_cast<int>(a.cu[b + 1]) - t != 1) return;
   const bool fresh = a.ctx[b] == 1;
   const int dim = a.dim, vdim = a.vdim, hk = MODE == kDecay ? h : h / (a.heads / a.kv_heads);
-  const int c = (tid & 3) * 4, col = blockIdx.x * kScanCols + c, row = tid >> 2;
+  const int c = (tid & 3) * 4, col = blockIdx.x * kOneCols + c, row = tid >> 2;
   float* sp = a.state + ((static_cast<size_t>(a.slots[b]) * a.heads + h) * dim) * vdim + col;
   const bool wide = vdim % 4 == 0 && (reinterpret_cast<uintptr_t>(a.state) & 15) == 0;
   float s[NR][4];
@@ -797,23 +799,29 @@ scan_one_kernel(const ScanArgs a) {
   }
 }
 
+template <int DK, int MODE, bool CHAN, int WW>
+static void launch_scan_ww(const ScanArgs& a, int num_seqs, int* err, cudaStream_t st_) {
+  using SM = ScanSmem<DK, CHAN, WW>;
+  auto kern = scan_kernel<DK, MODE, CHAN, WW>;
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SM::kBytes);
+  const int cols = (a.vdim + SM::kCols - 1) / SM::kCols;
+  // a few blocks per SM, each taking every so many sequences (a step of decoded tokens is over at once)
+  const int z = std::max(1, std::min(num_seqs, 4 * sm_count() / (cols * a.heads)));
+  kern<<<dim3(cols, a.heads, z), WW * 32 + 256, SM::kBytes, st_>>>(a, num_seqs, err);
+  B200_CUDA_LAUNCH_CHECK();
+}
 template <int DK, int MODE, bool CHAN>
 static void launch_scan_dk(const ScanArgs& a, int num_seqs, cudaStream_t st_) {
-  const int cols = (a.vdim + kScanCols - 1) / kScanCols;
   int* err = wait_error_flag();
   if (!err) {
     set_error(2, "scan: no host-visible memory");
     return;
   }
-  scan_one_kernel<DK, MODE, CHAN><<<dim3(cols, a.heads, num_seqs), 128, 0, st_>>>(a);
+  scan_one_kernel<DK, MODE, CHAN><<<dim3((a.vdim + kOneCols - 1) / kOneCols, a.heads, num_seqs), 128, 0, st_>>>(a);
   B200_CUDA_LAUNCH_CHECK();
-  auto kern = scan_kernel<DK, MODE, CHAN>;
-  constexpr int smem = ScanSmem<DK, CHAN>::kBytes;
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  // portions: a few blocks per SM, each taking every so many sequences (a step of decoded tokens is over at once)
-  const int z = std::max(1, std::min(num_seqs, 4 * sm_count() / (cols * a.heads)));
-  kern<<<dim3(cols, a.heads, z), kScanThreads, smem, st_>>>(a, num_seqs, err);
-  B200_CUDA_LAUNCH_CHECK();
+  // 16 columns per block while that leaves a block per SM at most, 32 beyond
+  if ((a.vdim + 15) / 16 * a.heads * num_seqs <= sm_count()) launch_scan_ww<DK, MODE, CHAN, 4>(a, num_seqs, err, st_);
+  else launch_scan_ww<DK, MODE, CHAN, 8>(a, num_seqs, err, st_);
 }
 // dim: rows of the state; at most 256 (the caller has checked)
 template <int MODE, bool CHAN>

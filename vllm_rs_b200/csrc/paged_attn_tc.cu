@@ -7,9 +7,9 @@
 // that hold kept tokens outside the window, then the window.
 //   S  = Q K^T    fp32 [128 x 64] in TMEM.  Q was rounded to bf16 once: in shared memory (SW128, K-major) or, where the key
 //                 rows are so long that Q and the page ring do not fit together, its first q_tm blocks of 64 in TMEM
-//   P  = softmax  thread = row: options and mask on the fp32 scores, lazy running maximum (the accumulator is rescaled
-//                 when the maximum grows by more than 2^8; exact, since the last division uses the same reference),
-//                 bf16 P to TMEM
+//   P  = softmax  thread = row: options and mask on the fp32 scores, running maximum (the accumulator is rescaled whenever a
+//                 row's maximum grows: letting it lag by up to 2^8 saves 3 - 10 % of the time, but the largest weight of a
+//                 row then is not 1 and is rounded like the others, 4 - 8 % more error against 64 bits), bf16 P to TMEM
 //   O += P V      fp32 [128 x up to 256] in TMEM; V = page as an MN-major operand
 // Warp 0 fetches pages by block-table index (TMA, K ring | V ring), warp 1 issues the MMAs (S of page j + 1 before P V of
 // page j), warps 2-5 own the rows.  Latent rows (kv_rank 512: O would need all 512 TMEM columns) are walked in passes of up to
@@ -33,7 +33,6 @@ constexpr int kTailBlk = kTok * 64;       // the last 32 columns: 64 rows of 64 
 constexpr int kQBlk = kRows * 128, kQTail = kRows * 64;
 constexpr int kMaxStages = 4;
 constexpr float kLog2e = 1.4426950408889634f, kLn2 = 0.6931471805599453f;
-constexpr float kRescale = 8.f;           // log2 units
 constexpr float kNone = -1e30f;           // a reference maximum before any key was seen
 
 struct Args {
@@ -540,7 +539,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
         const float mx = max3(mx0, mx1, fmaxf(x[kTok - 2], x[kTok - 1])) * mult;
         float corr = 1.f;
         bool grow = false;
-        if (mx - m_ref > kRescale) {
+        if (mx > m_ref) {
           corr = ex2(m_ref - mx);
           m_ref = mx;
           grow = true;
