@@ -68,6 +68,18 @@ __device__ __forceinline__ void tmem_st_x32(uint32_t taddr, const uint32_t (&v)[
       : "memory");
 }
 
+// 2^x, zero below 2^-126 (exp2f spends three more instructions on denormal results, which fp16 weights do not have)
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+
 struct Args {
   __half* out;
   const uint32_t* cu_seqlens_q;
@@ -250,8 +262,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_co
         tc_wait_ld();
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
-          x[i] = __uint_as_float(v0[i]) * a.scale_log2;
-          x[32 + i] = __uint_as_float(v1[i]) * a.scale_log2;
+          x[i] = __uint_as_float(v0[i]);
+          x[32 + i] = __uint_as_float(v1[i]);
         }
       }
       tc_fence_before();
@@ -261,16 +273,21 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_co
 #pragma unroll
         for (int i = 0; i < kTok; ++i) x[i] = (page_base + i <= qpos) ? x[i] : -INFINITY;
       }
-      float mx = x[0];
+      // maxima of the unscaled scores (the scale is positive); scale and reference meet in the exponent's multiply-add
+      float mx0 = max3(x[0], x[1], x[2]), mx1 = max3(x[3], x[4], x[5]);
 #pragma unroll
-      for (int i = 1; i < kTok; ++i) mx = fmaxf(mx, x[i]);
+      for (int i = 6; i < kTok - 2; i += 4) {
+        mx0 = max3(mx0, x[i], x[i + 1]);
+        mx1 = max3(mx1, x[i + 2], x[i + 3]);
+      }
+      const float mx = max3(mx0, mx1, fmaxf(x[kTok - 2], x[kTok - 1])) * a.scale_log2;
       // lazy rescale: keep the reference max unless the true max outgrew it by 2^8
       float corr = 1.f;
       bool grow = false;
       if (j == 0) {
         m_ref = (mx == -INFINITY) ? 0.f : mx;
       } else if (mx - m_ref > kRescaleThreshold) {
-        corr = exp2f(m_ref - mx);
+        corr = ex2(m_ref - mx);
         m_ref = mx;
         grow = true;
       }
@@ -278,7 +295,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_co
       uint32_t pk[32];
 #pragma unroll
       for (int i = 0; i < 32; ++i) {
-        const float p0 = exp2f(x[2 * i] - m_ref), p1 = exp2f(x[2 * i + 1] - m_ref);
+        const float p0 = ex2(fmaf(x[2 * i], a.scale_log2, -m_ref)), p1 = ex2(fmaf(x[2 * i + 1], a.scale_log2, -m_ref));
         psum += p0 + p1;
         pk[i] = pack16x2<BF>(p0, p1);
       }
@@ -380,7 +397,7 @@ bool launch_attn_prefill_tc(const AttnMaps& maps, void* out, const void* q, int 
                             cudaStream_t st, bool bf16) {
   using namespace pft;
   if (mode < 0) mode = prefill_attn_mode();
-  if (mode == 0 || D != kD) return false;
+  if (mode == 0 || D != kD || !(scale > 0.f)) return false;
   const int G = H / Hkv;
   if (kRows % G != 0 || (q_stride * 2) % 16 != 0 || (reinterpret_cast<uintptr_t>(q) & 15)) return false;
   const int TQ = kRows / G;

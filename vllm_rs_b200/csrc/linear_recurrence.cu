@@ -140,7 +140,7 @@ __device__ __forceinline__ void unpack2(f2 v, float& lo, float& hi) { asm("mov.b
 
 constexpr int kOneCols = 16;                   // columns of S per block of threads: single tokens
 constexpr int kBT = 8;                         // tokens per block of the recurrence
-constexpr int kRing = 4;                       // blocks of tokens in shared memory: walked, prepared, two on their way
+constexpr int kRing = 8;                       // blocks of tokens in shared memory (with four, fetching waited for the walk)
 constexpr int kDelta = 0, kDecay = 1, kSsd = 2;
 
 struct ScanArgs {
@@ -803,7 +803,8 @@ template <int DK, int MODE, bool CHAN, int WW>
 static void launch_scan_ww(const ScanArgs& a, int num_seqs, int* err, cudaStream_t st_) {
   using SM = ScanSmem<DK, CHAN, WW>;
   auto kern = scan_kernel<DK, MODE, CHAN, WW>;
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SM::kBytes);
+  static const cudaError_t sized = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SM::kBytes);
+  (void)sized;
   const int cols = (a.vdim + SM::kCols - 1) / SM::kCols;
   // a few blocks per SM, each taking every so many sequences (a step of decoded tokens is over at once)
   const int z = std::max(1, std::min(num_seqs, 4 * sm_count() / (cols * a.heads)));

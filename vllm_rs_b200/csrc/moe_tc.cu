@@ -287,7 +287,8 @@ static void launch(void* out, const void* a, const void* w, const int32_t* off, 
     return;
   }
   auto kern = grouped_linear_tc_kernel<ACT, BN>;
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BN>::kSmem);
+  static const cudaError_t sized = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BN>::kSmem);
+  (void)sized;
   const int most = std::min(pairs, E + pairs / kM) * g.ntiles_n;        // no step has more tiles
   kern<<<std::min(most, sm_count()), kThreads, Cfg<BN>::kSmem, st>>>(amap, wmap, g);
   B200_CUDA_LAUNCH_CHECK();

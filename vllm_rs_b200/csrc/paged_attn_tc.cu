@@ -739,7 +739,12 @@ void launch_attn_tc(const AttnTcProblem& p, cudaStream_t st) {
   const bool cap = p.softcap > 0.f, bias = p.slopes || p.dist_bias;
   auto kern = cap ? (bias ? attn_tc_kernel<true, true> : attn_tc_kernel<true, false>)
                   : (bias ? attn_tc_kernel<false, true> : attn_tc_kernel<false, false>);
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  static const bool sized = [] {
+    for (auto k : {attn_tc_kernel<true, true>, attn_tc_kernel<true, false>, attn_tc_kernel<false, true>, attn_tc_kernel<false, false>})
+      cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
+    return true;
+  }();
+  (void)sized;
   kern<<<grid, kThreads, smem, st>>>(kmap, tmap, vmap, a);
   B200_CUDA_LAUNCH_CHECK();
 }
