@@ -860,6 +860,20 @@ void b200_lowrank_decay(float* out, const float* low, int32_t ld_low, const floa
 void b200_lowrank_decay_ex(float* out, const float* low, int32_t ld_low, const float* w2, const float* bias, float tau,
                            int32_t kind, const float* a_log, int32_t a_period, int32_t num_tokens, int32_t channels,
                            int32_t rank, int64_t stream);
+/* The recurrent scans with a row stride per operand.  kind 0 the gated delta rule (strength, and either decay_raw with a_log and
+ * dt_bias or chan_decay), 1 decayed linear attention (head_decay or chan_decay; q_scale, k_scale, act), 2 the state-space scan
+ * (q = C, k = B, v = x, decay_raw = dt; d_skip or NULL).  strength and decay_raw fp32 [T, heads] (row stride ld_s), everything
+ * else as in the entry point of that scan.                                                                           */
+typedef struct b200_scan_args {
+  float* out;
+  const float *q, *k, *v, *strength, *decay_raw, *a_log, *dt_bias, *d_skip, *head_decay, *chan_decay;
+  float* state;
+  const int32_t* state_slots;
+  const uint32_t *cu_seqlens_q, *context_lens;
+  int32_t num_seqs, ld_q, ld_k, ld_v, ld_s, ld_decay, heads, kv_heads, dim, vdim, act;
+  float q_scale, k_scale;
+} b200_scan_args;
+void b200_scan(const b200_scan_args* args, int32_t kind, int64_t stream);
 /* Linear attention with a decayed state: S <- diag(a_t) S + (k_scale k_t) v_t^T, o_t = S^T (q_scale q_t).  q, k fp32
  * [T, heads, dim], v [T, heads, vdim] (row stride ld); exactly one of head_decay fp32 [heads] (a constant per head)
  * and chan_decay fp32 [T, heads, dim] (row stride ld_decay); act != 0: SiLU on q, k and v first; out fp32

@@ -102,6 +102,15 @@ class ExpertAct(C.Structure):
     _fields_ = [("kind", c_i32)] + [(n, c_f32) for n in ("limit", "alpha", "up_add")]
 
 
+class ScanArgs(C.Structure):
+    """b200_scan_args (include/b200_vllm.h)."""
+
+    _fields_ = [(n, c_vp) for n in ("out", "q", "k", "v", "strength", "decay_raw", "a_log", "dt_bias", "d_skip", "head_decay",
+                                    "chan_decay", "state", "state_slots", "cu_seqlens_q", "context_lens")] + \
+               [(n, c_i32) for n in ("num_seqs", "ld_q", "ld_k", "ld_v", "ld_s", "ld_decay", "heads", "kv_heads", "dim", "vdim",
+                                     "act")] + [(n, c_f32) for n in ("q_scale", "k_scale")]
+
+
 class KvCachePlan(C.Structure):
     """b200_kvcache_plan (include/b200_vllm.h)."""
 
@@ -286,6 +295,7 @@ _SIGS = {
     "b200_latent_prep_queries": (None, [c_vp, c_i32, c_vp, c_vp, c_vp, c_f32, c_vp] + [c_i32] * 7 + [c_i64]),
     "b200_latent_attn_gated": (None, [c_vp] * 5 + [c_i32] + [c_vp] * 3 + [c_i32] * 7 + [c_f32, c_i32, c_vp, c_i64]),
     "b200_short_conv_silu": (None, [c_vp, c_i32, c_vp, c_i32] + [c_vp] * 6 + [c_i32] * 4 + [c_i64]),
+    "b200_scan": (None, [C.POINTER(ScanArgs), c_i32, c_i64]),
     "b200_delta_rule": (None, [c_vp] * 4 + [c_i32, c_vp, c_vp, c_i32] + [c_vp] * 6 + [c_i32] * 5 + [c_i64]),
     "b200_ssd_scan": (None, [c_vp] * 4 + [c_i32, c_vp, c_i32] + [c_vp] * 7 + [c_i32] * 5 + [c_i64]),
     "b200_moe_route": (None, [c_vp, c_i32, c_i32, c_i32, c_f32, c_vp, c_vp, c_i64]),

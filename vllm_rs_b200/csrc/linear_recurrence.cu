@@ -143,21 +143,7 @@ constexpr int kBT = 8;                         // tokens per block of the recurr
 constexpr int kRing = 8;                       // blocks of tokens in shared memory (with four, fetching waited for the walk)
 constexpr int kDelta = 0, kDecay = 1, kSsd = 2;
 
-struct ScanArgs {
-  float* out;
-  const float *q, *k, *v;          // delta: q, k, v; ssd: C, B, x
-  int ld;
-  const float *b_raw, *a_raw;      // delta: write strength and decay logits; ssd: a_raw = dt_raw
-  int ld_ba;
-  const float *a_log, *dt_bias, *d_skip, *head_decay, *chan_decay;
-  int ld_decay;
-  float q_scale, k_scale;
-  int act;
-  float* state;
-  const int32_t* slots;
-  const uint32_t *cu, *ctx;
-  int heads, kv_heads, dim, vdim;
-};
+using ScanArgs = b200_scan_args;
 
 template <int DK, bool CHAN, int WW> struct ScanSmem {         // WW: walking warps, four columns each
   static constexpr int kRows = kBT * DK;                                        // floats of one array of token rows
@@ -223,6 +209,9 @@ __device__ __forceinline__ float meet32(float (&x)[32], int lane) {
 // block ahead of each), norming or activating them and preparing its triangles under the walks of the blocks before; one such
 // group takes longer than a walk (3300 against 1950 cycles for the delta rule), two do not.
 // WW = 8 lets two walking warps share a scheduler and a prepared block, WW = 4 spreads few columns over more SMs.
+// Bound: the chain of blocks, one walk after another, of fp32 FMAs and a butterfly over the lanes; HBM and the FMA units would
+// take 16 and 89 us for 4096 tokens of 16 heads of 128 x 128.  Measured there, token by token (eight lanes per column, four
+// chained shuffles per token) -> in blocks: delta rule 2255 -> 654 us; decayed state of 8 heads of 128 x 256: 909 -> 445 us.
 template <int DK, int MODE, bool CHAN, int WW>
 __global__ void __launch_bounds__(WW * 32 + 256, 1)
 scan_kernel(const ScanArgs a, int num_seqs, int* err) {
@@ -243,24 +232,24 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
   __syncthreads();
   int blocks = 0;                                                      // blocks of tokens so far, over all sequences
   for (int b = blockIdx.z; b < num_seqs; b += gridDim.z) {
-    const int t0 = a.cu[b], t1 = a.cu[b + 1], nblk = (t1 - t0 + kBT - 1) / kBT;
+    const int t0 = a.cu_seqlens_q[b], t1 = a.cu_seqlens_q[b + 1], nblk = (t1 - t0 + kBT - 1) / kBT;
     if (t1 - t0 < 2) continue;                                         // (scan_one_kernel)
-    const bool fresh = static_cast<int>(a.ctx[b]) == t1 - t0;
+    const bool fresh = static_cast<int>(a.context_lens[b]) == t1 - t0;
     if (warp >= WW) {
       // ---------------------------------------------------------- token rows
       const int pt = tid & 127, pw = warp & 3, grp = (warp - WW) >> 2;
-      const bool wide = dim % 4 == 0 && a.ld % 4 == 0 && (!CHAN || a.ld_decay % 4 == 0) &&
+      const bool wide = dim % 4 == 0 && (a.ld_q | a.ld_k) % 4 == 0 && (!CHAN || a.ld_decay % 4 == 0) &&
                         ((reinterpret_cast<uintptr_t>(a.q) | reinterpret_cast<uintptr_t>(a.k) |
                           (CHAN ? reinterpret_cast<uintptr_t>(a.chan_decay) : 0)) & 15) == 0;
-      const bool wide_v = vdim % 4 == 0 && a.ld % 4 == 0 && (reinterpret_cast<uintptr_t>(a.v) & 15) == 0;
+      const bool wide_v = vdim % 4 == 0 && a.ld_v % 4 == 0 && (reinterpret_cast<uintptr_t>(a.v) & 15) == 0;
       auto fetch = [&](int i) {                                        // block i of the sequence; one group in any case
         if (i < nblk) {
           const int g = blocks + i;
           if (g >= kRing) mbar_wait_limited(&done[g % kRing], (g / kRing - 1) & 1, fail, err);
           float* B = sm + g % kRing * SM::kBuf;
           const int c0 = t0 + i * kBT, n = min(kBT, t1 - c0);
-          const float* kg = a.k + static_cast<size_t>(c0) * a.ld + hk * dim;
-          const float* qg = a.q + static_cast<size_t>(c0) * a.ld + hk * dim;
+          const float* kg = a.k + static_cast<size_t>(c0) * a.ld_k + hk * dim;
+          const float* qg = a.q + static_cast<size_t>(c0) * a.ld_q + hk * dim;
           const float* ag = CHAN ? a.chan_decay + static_cast<size_t>(c0) * a.ld_decay + h * dim : nullptr;
           constexpr int TPR = DK / 4, RPS = 128 / TPR;                 // threads per row, rows at a time
           const int x = pt % TPR * 4;
@@ -268,8 +257,8 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
           for (int r = pt / TPR; r < kBT; r += RPS) {
             if (r >= n || x >= dim) continue;
             const int o = r * DK + x;
-            const float* ks_ = kg + static_cast<size_t>(r) * a.ld + x;
-            const float* qs_ = qg + static_cast<size_t>(r) * a.ld + x;
+            const float* ks_ = kg + static_cast<size_t>(r) * a.ld_k + x;
+            const float* qs_ = qg + static_cast<size_t>(r) * a.ld_q + x;
             if (wide) {
               cp_async16(B + o, ks_);
               cp_async16(B + SM::kRows + o, qs_);
@@ -282,14 +271,14 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
               }
             }
           }
-          const float* vg = a.v + static_cast<size_t>(c0) * a.ld + h * vdim + col0;
+          const float* vg = a.v + static_cast<size_t>(c0) * a.ld_v + h * vdim + col0;
           if (wide_v) {
             const int r = pt / (COLS / 4), c = pt % (COLS / 4) * 4;
-            if (r < n && col0 + c < vdim) cp_async16(B + SM::kV + r * COLS + c, vg + static_cast<size_t>(r) * a.ld + c);
+            if (r < n && col0 + c < vdim) cp_async16(B + SM::kV + r * COLS + c, vg + static_cast<size_t>(r) * a.ld_v + c);
           } else {
             for (int e = pt; e < n * COLS; e += 128) {
               const int r = e / COLS, c = e % COLS;
-              if (col0 + c < vdim) cp_async4(B + SM::kV + e, vg + static_cast<size_t>(r) * a.ld + c);
+              if (col0 + c < vdim) cp_async4(B + SM::kV + e, vg + static_cast<size_t>(r) * a.ld_v + c);
             }
           }
         }
@@ -307,9 +296,9 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
       auto read_scalars = [&](int i) {
         const int t = t0 + i * kBT + lane;
         if (lane >= kBT || t >= t1) return;
-        const size_t o = static_cast<size_t>(t) * a.ld_ba + h;
-        if (MODE == kDelta) raw_b = a.b_raw[o];
-        if (MODE == kSsd || (MODE == kDelta && !CHAN)) raw_a = a.a_raw[o];
+        const size_t o = static_cast<size_t>(t) * a.ld_s + h;
+        if (MODE == kDelta) raw_b = a.strength[o];
+        if (MODE == kSsd || (MODE == kDelta && !CHAN)) raw_a = a.decay_raw[o];
       };
       auto make_scalars = [&](int i) {
         float* G = sm + (blocks + i) % kRing * SM::kBuf + SM::kG;
@@ -519,7 +508,7 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
     } else {
       // ---------------------------------------------------------- the walk
       const int colw = col0 + warp * 4;                // this warp's first column
-      float* sp = a.state + ((static_cast<size_t>(a.slots[b]) * a.heads + h) * dim) * vdim + colw;
+      float* sp = a.state + ((static_cast<size_t>(a.state_slots[b]) * a.heads + h) * dim) * vdim + colw;
       const bool wide_s = vdim % 4 == 0 && (reinterpret_cast<uintptr_t>(a.state) & 15) == 0;
       const float skip = MODE == kSsd && a.d_skip ? a.d_skip[h] : 0.f;
       f2 s[4][CH / 2];                                 // [column][pair of rows]
@@ -655,7 +644,8 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
   }
 }
 
-// Sequences that bring one token.  grid = (column blocks, heads, sequences); 128 threads = 32 rows x 4 columns of 4; bound by the
+// Sequences that bring one token: 16 columns per block, so that a single sequence of 16 heads of 128 still makes 128 blocks.
+// 32 sequences of 16 heads of 128 x 128 move 67 MB; the call, with the other kernel's launch, is bound by its host side.  grid = (column blocks, heads, sequences); 128 threads = 32 rows x 4 columns of 4; bound by the
 // state's way in and out, which are whole 64-byte rows here.
 template <int DK, int MODE, bool CHAN>
 __global__ void __launch_bounds__(128)
@@ -663,12 +653,12 @@ scan_one_kernel(const ScanArgs a) {
   constexpr int NR = DK / 32;
   __shared__ float ks[DK], qs[DK], red[2][4][kOneCols], sums[4][2];
   const int h = blockIdx.y, b = blockIdx.z, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int t = a.cu[b];
-  if (static_cast<int>(a.cu[b + 1]) - t != 1) return;
-  const bool fresh = a.ctx[b] == 1;
+  const int t = a.cu_seqlens_q[b];
+  if (static_cast<int>(a.cu_seqlens_q[b + 1]) - t != 1) return;
+  const bool fresh = a.context_lens[b] == 1;
   const int dim = a.dim, vdim = a.vdim, hk = MODE == kDecay ? h : h / (a.heads / a.kv_heads);
   const int c = (tid & 3) * 4, col = blockIdx.x * kOneCols + c, row = tid >> 2;
-  float* sp = a.state + ((static_cast<size_t>(a.slots[b]) * a.heads + h) * dim) * vdim + col;
+  float* sp = a.state + ((static_cast<size_t>(a.state_slots[b]) * a.heads + h) * dim) * vdim + col;
   const bool wide = vdim % 4 == 0 && (reinterpret_cast<uintptr_t>(a.state) & 15) == 0;
   float s[NR][4];
 #pragma unroll
@@ -687,8 +677,8 @@ scan_one_kernel(const ScanArgs a) {
       }
     }
   }
-  const float* kg = a.k + static_cast<size_t>(t) * a.ld + hk * dim;
-  const float* qg = a.q + static_cast<size_t>(t) * a.ld + hk * dim;
+  const float* kg = a.k + static_cast<size_t>(t) * a.ld_k + hk * dim;
+  const float* qg = a.q + static_cast<size_t>(t) * a.ld_q + hk * dim;
   float sk = 0.f, sq = 0.f;
   for (int i = tid; i < DK; i += 128) {
     float kv = i < dim ? kg[i] : 0.f, qv = i < dim ? qg[i] : 0.f;
@@ -709,13 +699,13 @@ scan_one_kernel(const ScanArgs a) {
       sums[warp][1] = sq;
     }
   }
-  const size_t ba = static_cast<size_t>(t) * a.ld_ba + h;
+  const size_t ba = static_cast<size_t>(t) * a.ld_s + h;
   float g = 1.f, w = a.k_scale;                        // decay; write strength
   if (MODE == kDelta) {
-    w = sigmoid_f(a.b_raw[ba]);
-    if (!CHAN) g = expf(-expf(a.a_log[h]) * softplus_f(a.a_raw[ba] + a.dt_bias[h]));
+    w = sigmoid_f(a.strength[ba]);
+    if (!CHAN) g = expf(-expf(a.a_log[h]) * softplus_f(a.decay_raw[ba] + a.dt_bias[h]));
   } else if (MODE == kSsd) {
-    w = softplus_f(a.a_raw[ba] + a.dt_bias[h]);
+    w = softplus_f(a.decay_raw[ba] + a.dt_bias[h]);
     g = expf(-expf(a.a_log[h]) * w);
   } else if (!CHAN) {
     g = a.head_decay[h];
@@ -723,7 +713,7 @@ scan_one_kernel(const ScanArgs a) {
   float v[4];
 #pragma unroll
   for (int x = 0; x < 4; ++x) {
-    v[x] = col + x < vdim ? a.v[static_cast<size_t>(t) * a.ld + h * vdim + col + x] : 0.f;
+    v[x] = col + x < vdim ? a.v[static_cast<size_t>(t) * a.ld_v + h * vdim + col + x] : 0.f;
     if (MODE == kDecay && a.act) v[x] = silu_exact(v[x]);
   }
   __syncthreads();
@@ -907,8 +897,8 @@ void launch_delta_rule(float* out, const float* q, const float* k, const float* 
     set_error(1, "delta_rule: key dimension above 256 is not supported");
     return;
   }
-  const ScanArgs s{out, q, k, v, ld, b_raw, a_raw, ld_ba, a_log, dt_bias, nullptr, nullptr, chan_decay, ld_decay, 1.f, 1.f, 0,
-                   state, slots, cu, ctx, heads, kv_heads, dim, vdim};
+  const ScanArgs s{out, q, k, v, b_raw, a_raw, a_log, dt_bias, nullptr, nullptr, chan_decay, state, slots, cu, ctx, num_seqs,
+                   ld, ld, ld, ld_ba, ld_decay, heads, kv_heads, dim, vdim, 0, 1.f, 1.f};
   if (chan_decay) launch_scan<kDelta, true>(s, num_seqs, st_);
   else launch_scan<kDelta, false>(s, num_seqs, st_);
 }
@@ -922,8 +912,8 @@ void launch_ssd_scan(float* out, const float* x, const float* Bm, const float* C
     set_error(1, "ssd_scan: state size above 256 is not supported");
     return;
   }
-  const ScanArgs s{out, Cm, Bm, x, ld, nullptr, dt_raw, ld_dt, a_log, dt_bias, d_skip, nullptr, nullptr, 0, 1.f, 1.f, 0,
-                   state, slots, cu, ctx, heads, groups, nstate, vdim};
+  const ScanArgs s{out, Cm, Bm, x, nullptr, dt_raw, a_log, dt_bias, d_skip, nullptr, nullptr, state, slots, cu, ctx, num_seqs,
+                   ld, ld, ld, ld_dt, 0, heads, groups, nstate, vdim, 0, 1.f, 1.f};
   launch_scan<kSsd, false>(s, num_seqs, st_);
 }
 
@@ -949,15 +939,38 @@ void launch_decay_attn(float* out, const float* q, const float* k, const float* 
     set_error(1, "decay_attn: key dimension above 256 is not supported");
     return;
   }
-  const ScanArgs s{out, q, k, v, ld, nullptr, nullptr, 0, nullptr, nullptr, nullptr, head_decay, chan_decay, ld_decay,
-                   q_scale, k_scale, act, state, slots, cu, ctx, heads, heads, dim, vdim};
+  const ScanArgs s{out, q, k, v, nullptr, nullptr, nullptr, nullptr, nullptr, head_decay, chan_decay, state, slots, cu, ctx,
+                   num_seqs, ld, ld, ld, 0, ld_decay, heads, heads, dim, vdim, act, q_scale, k_scale};
   if (chan_decay) launch_scan<kDecay, true>(s, num_seqs, st_);
   else launch_scan<kDecay, false>(s, num_seqs, st_);
+}
+
+void launch_scan_args(const b200_scan_args& a, int kind, cudaStream_t st_) {
+  if (a.num_seqs <= 0) return;
+  if (a.dim > 256) {
+    set_error(1, "scan: key dimension (state size) above 256 is not supported");
+    return;
+  }
+  if (kind == kSsd) launch_scan<kSsd, false>(a, a.num_seqs, st_);
+  else if (kind == kDelta && a.chan_decay) launch_scan<kDelta, true>(a, a.num_seqs, st_);
+  else if (kind == kDelta) launch_scan<kDelta, false>(a, a.num_seqs, st_);
+  else if (a.chan_decay) launch_scan<kDecay, true>(a, a.num_seqs, st_);
+  else launch_scan<kDecay, false>(a, a.num_seqs, st_);
 }
 
 }  // namespace b200
 
 extern "C" {
+void b200_scan(const b200_scan_args* a, int32_t kind, int64_t stream) {
+  B200_CHECK_ARG(a && a->out && a->q && a->k && a->v && a->state && a->state_slots && a->cu_seqlens_q && a->context_lens &&
+                     a->heads > 0 && a->kv_heads > 0 && a->heads % a->kv_heads == 0 && a->dim > 0 && a->vdim > 0 &&
+                     kind >= b200::kDelta && kind <= b200::kSsd &&
+                     (kind == b200::kDecay ? (a->head_decay != nullptr) != (a->chan_decay != nullptr) && a->kv_heads == a->heads
+                      : kind == b200::kSsd ? a->decay_raw && a->a_log && a->dt_bias
+                                           : a->strength && (a->chan_decay || (a->decay_raw && a->a_log && a->dt_bias))),
+                 "scan: bad arguments");
+  b200::launch_scan_args(*a, kind, reinterpret_cast<cudaStream_t>(stream));
+}
 void b200_short_conv_silu(float* out, int32_t ldo, const float* x, int32_t ldx, const float* taps_w, const float* bias,
                           float* state, const int32_t* state_slots, const uint32_t* cu_seqlens_q,
                           const uint32_t* context_lens, int32_t num_seqs, int32_t num_tokens, int32_t channels,
