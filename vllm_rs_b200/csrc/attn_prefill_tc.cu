@@ -18,7 +18,9 @@
 // Warp roles: warp 0 TMA producer (2-stage K|V ring), warp 1 MMA issuer (QK^T of page j+1 is issued
 // before PV of page j, so it runs under the softmax of page j), warps 2-5 softmax / correction /
 // epilogue.  96 KB of shared memory and 256 TMEM columns per CTA: two CTAs share an SM and fill each
-// other's softmax bubbles.  Tensor-bound (4 * 128 * ctx flop per row) with MUFU.EX2 as co-limit.
+// other's softmax bubbles.  Tensor-bound (4 * 128 * ctx flop per row) with MUFU.EX2 and the softmax warps' issue
+// slots as co-limits: without exp2f's guard for denormal results, a multiplication per score and two-input maxima 32 heads
+// over 3 sequences of 8192 rows together take 421 us instead of 441.
 #include <cstdlib>
 #include <cstring>
 

@@ -19,6 +19,9 @@
 //
 // Bound: tensor cores for prompts (per page 2 * 128 * 64 * (dim * passes + vdim) flop against 64 * dim * 2 bytes from L2),
 // HBM for steps of few rows, whose keys are split over blocks; window_attn_merge / latent_attn_merge then finish.
+// Measured, mma.sync kernels -> here: window 1024, 4096 rows, 16 heads of 128 over 4: 622 -> 99 us (303 TFLOP/s; what bounds it
+// is the softmax warps' issue slots, then the start and the drain of 128 blocks); latent, 2 x 2048 rows, 32 heads, rank 512:
+// 7766 -> 690 us (433 TFLOP/s useful, 656 issued); 32 tokens over 2048 keys, 32 heads over 8: 317 -> 59 us (35 at HBM rate).
 #include "paged_attn_tc.cuh"
 
 #include <algorithm>
