@@ -211,7 +211,9 @@ __device__ __forceinline__ float meet32(float (&x)[32], int lane) {
 // WW = 8 lets two walking warps share a scheduler and a prepared block, WW = 4 spreads few columns over more SMs.
 // Bound: the chain of blocks, one walk after another, of fp32 FMAs and a butterfly over the lanes; HBM and the FMA units would
 // take 16 and 89 us for 4096 tokens of 16 heads of 128 x 128.  Measured there, token by token (eight lanes per column, four
-// chained shuffles per token) -> in blocks: delta rule 2255 -> 654 us; decayed state of 8 heads of 128 x 256: 909 -> 445 us.
+// chained shuffles per token) -> in blocks: delta rule 2278 -> 613 us; decayed state of 8 heads of 128 x 256: 909 -> 388 us.  The state's update does not wait for the
+// read-out's sums: the queries' products are taken before the correction's sums meet, and meet under the update (665 and 424
+// us with both in turn).
 template <int DK, int MODE, bool CHAN, int WW>
 __global__ void __launch_bounds__(WW * 32 + 256, 1)
 scan_kernel(const ScanArgs a, int num_seqs, int* err) {
@@ -544,9 +546,8 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
         __syncwarp();
         const float* B = sm + g % kRing * SM::kBuf;
         const float* G = B + SM::kG;
-        // a row's products with the state, summed over the lanes
-        auto dots = [&](const float* rows) {
-          float x[32];
+        // the rows' products with this lane's part of the state
+        auto dots = [&](float (&x)[32], const float* rows) {
 #pragma unroll
           for (int t = 0; t < kBT; ++t) {
             f2 y[CH / 2];
@@ -559,13 +560,15 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
               x[t * 4 + c] = sum2(acc);
             }
           }
-          return meet32(x, lane);
         };
         const float gt = CHAN ? 1.f : G[2 * kBT + tt];
         const float vt = B[SM::kV + tt * COLS + warp * 4 + c4], wt = G[kBT + tt];
-        float u = vt * wt;
+        float u = vt * wt, xq[32];
+        dots(xq, B + SM::kRows);
         if (MODE == kDelta) {
-          const float r = wt * (vt - gt * dots(B));
+          float xk[32];
+          dots(xk, B);
+          const float r = wt * (vt - gt * meet32(xk, lane));
           const float4 ta = *reinterpret_cast<const float4*>(B + SM::kMat + tt * kBT), tb = *reinterpret_cast<const float4*>(B + SM::kMat + tt * kBT + 4);
           const float T[kBT] = {ta.x, ta.y, ta.z, ta.w, tb.x, tb.y, tb.z, tb.w};
           u = 0.f;
@@ -573,7 +576,8 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
           for (int j = 0; j < kBT; ++j) u += T[j] * __shfl_sync(0xffffffffu, r, j * 4 + c4);
         }
         us[lane] = CHAN ? u : u * G[3 * kBT + tt];
-        const float e = dots(B + SM::kRows);
+        __syncwarp();
+        const float e = meet32(xq, lane);              // (in no one's way: the state's update does not need it)
         {
           const float4 pa = *reinterpret_cast<const float4*>(B + SM::kMat + kBT * kBT + tt * kBT);
           const float4 pb = *reinterpret_cast<const float4*>(B + SM::kMat + kBT * kBT + tt * kBT + 4);
@@ -601,7 +605,6 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
 #pragma unroll
             for (int r = 0; r < CH / 2; ++r) s[c][r] = mul2(s[c][r], g2);
         }
-        __syncwarp();
         const float* kd = B + (CHAN ? 2 * SM::kRows : 0) + lane * CH;       // keys as they enter the state
 #pragma unroll
         for (int t = 0; t < kBT; ++t) {
@@ -810,7 +813,8 @@ static void launch_scan_dk(const ScanArgs& a, int num_seqs, cudaStream_t st_) {
   }
   scan_one_kernel<DK, MODE, CHAN><<<dim3((a.vdim + kOneCols - 1) / kOneCols, a.heads, num_seqs), 128, 0, st_>>>(a);
   B200_CUDA_LAUNCH_CHECK();
-  // 16 columns per block while that leaves a block per SM at most, 32 beyond
+  // 16 columns per block while that leaves a block per SM at most, 32 beyond: one sequence of 4096 tokens of 16 heads of
+  // 128 x 128 (128 or 64 blocks) 634 and 883 us, four of 1000 (512 or 256 blocks) 655 and 539 us
   if ((a.vdim + 15) / 16 * a.heads * num_seqs <= sm_count()) launch_scan_ww<DK, MODE, CHAN, 4>(a, num_seqs, err, st_);
   else launch_scan_ww<DK, MODE, CHAN, 8>(a, num_seqs, err, st_);
 }
