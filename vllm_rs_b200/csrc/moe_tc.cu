@@ -10,10 +10,13 @@
 // gathers of four rows (~90 cycles each) as by cp.async, whose blocks need a wait and a fence on their way to the tensor core
 // (prompt of 4096 rows, 16 experts, first product: 183 us and 103-139 us).
 //
-// Measured, mma.sync kernel -> here (whole call): 4096 rows of 2048, 16 experts of 512, 4 chosen: 705 -> 201 us; 32 rows 71 -> 58;
+// Measured, mma.sync kernel -> here (whole call): 4096 rows of 2048, 16 experts of 512, 4 chosen: 705 -> 201 us; 32 rows 71 -> 46;
 // 4096 wide, 32 experts of 1024: 3000 rows 1903 -> 406 us, 32 rows 198 -> 142.  The calls with few rows are the five launches.
-// Bound: tensor cores where experts get hundreds of rows, HBM (every hit expert's weights once) where they get few; BN is the
-// largest of 256 / 128 / 64 that gives every SM two tiles (fewer tiles leave SMs without weights to fetch).
+// Bound: tensor cores where experts get hundreds of rows, HBM (every hit expert's weights once) where they get few; BN is 256
+// where that gives every SM two tiles, else 128 where that gives three SMs in four one (below that the launches are the bound),
+// else 64.  Whole calls with BN = 64 / 128 / 256, 2048 wide, 16 experts of 512: 2 rows 47.8 / 47.5 / 49.2 us (128 / 64 / 32 tiles
+// in the first product), 8 rows 56.0 / 45.6 / 48.5 (256 / 128 / 64), 300 rows 69.6 / 52.6 / 63.0, 4096 rows 388 / 243 / 187;
+// 4096 wide, 32 experts of 1024: 32 rows 198 / 142 / 150 us, 300 rows 295 / 185 / 177, 3000 rows 1027 / 573 / 405.
 #include "../../include/b200_vllm.h"
 #include "moe_tc.cuh"
 
@@ -301,9 +304,8 @@ static void launch_bn(void* out, const void* a, const void* w, const int32_t* of
                       const b200_expert_act& act, cudaStream_t st) {
   constexpr int G = ACT == 1 || ACT == 3 ? 2 : 1;
   const int row_tiles = std::max(std::min(E, pairs), pairs / kM);
-  const int want = 2 * sm_count();
-  if (row_tiles * ((N * G + 255) / 256) >= want) launch<ACT, 256>(out, a, w, off, pairs, E, K, N, act, st);
-  else if (row_tiles * ((N * G + 127) / 128) >= want) launch<ACT, 128>(out, a, w, off, pairs, E, K, N, act, st);
+  if (row_tiles * ((N * G + 255) / 256) >= 2 * sm_count()) launch<ACT, 256>(out, a, w, off, pairs, E, K, N, act, st);
+  else if (row_tiles * ((N * G + 127) / 128) >= sm_count() * 3 / 4) launch<ACT, 128>(out, a, w, off, pairs, E, K, N, act, st);
   else launch<ACT, 64>(out, a, w, off, pairs, E, K, N, act, st);
 }
 
