@@ -77,3 +77,25 @@ def test_scans(lib, kind, H, G, d, e, lens):
     # fp32 sums of up to d terms, thousands of them below 2^-24 of the largest entries each
     assert (got.double().cpu() - want).abs().max() <= 1e-5 * want.abs().max()
     assert (dev_state.double().cpu() - want_state).abs().max() <= 1e-5 * want_state.abs().max()
+
+
+def test_operands_as_they_lie(lib):
+    """Views with other strides and one row per token (the form that mixed types take) give the same bits as packed operands."""
+    from vllm_rs_b200 import _lib, ops
+    T, G, H, d, e = 21, 2, 4, 36, 20
+    g = torch.Generator().manual_seed(5)
+    r = lambda *s: torch.randn(*s, generator=g).cuda()                        # noqa: E731
+    q, k, v, b, a, alog, dtb, state = r(T, G, d), r(T, G, d), r(T, H, e), r(T, H), r(T, H), r(H), r(H), r(2, H, d, e)
+    tail = (_i32([1]), _i32([0, T]), _i32([T + 3]))
+    states = [state.clone() for _ in range(3)]
+    want = ops.delta_rule(q, k, v, b, a, alog, dtb, states[0], *tail)
+    lie = lambda t: torch.stack([t, t + 1], -1).transpose(0, 1).contiguous().transpose(0, 1)[..., 0]      # noqa: E731
+    views = ops.delta_rule(lie(q), lie(k), lie(v), lie(b), lie(a), alog, dtb, states[1], *tail)
+    row = torch.cat([t.reshape(T, -1) for t in (q, k, v, b, a)], 1).contiguous()
+    out, at, n = torch.empty_like(want), row.data_ptr(), G * d
+    _lib.lib().b200_delta_rule(out.data_ptr(), at, at + 4 * n, at + 8 * n, row.shape[1], at + 4 * (2 * n + H * e),
+                               at + 4 * (2 * n + H * e + H), row.shape[1], alog.data_ptr(), dtb.data_ptr(), states[2].data_ptr(),
+                               *(t.data_ptr() for t in tail), 1, H, G, d, e, torch.cuda.current_stream().cuda_stream)
+    _lib.check()
+    for o, s in ((views, states[1]), (out, states[2])):
+        assert torch.equal(o, want) and torch.equal(s, states[0])

@@ -167,7 +167,7 @@ def kernel_table(size, prefill, batch, ctx, peaks):
         if phase == "decode":
             add("delta_rule", phase, ms, 6.0 * T * Hd * dk * dv, B * Hd * dk * dv * 8.0, "hbm", "bytes = state read + write")
         else:
-            add("delta_rule", phase, ms, 6.0 * T * Hd * dk * dv, 0.0, "fp32", "token-serial recurrence")
+            add("delta_rule", phase, ms, 6.0 * T * Hd * dk * dv, 0.0, "fp32", "recurrence in blocks of eight tokens")
         # SSD scan
         ss = s["ssd"]
         Hs, G, N, P = ss["heads"], ss["groups"], ss["state"], ss["vdim"]
@@ -178,7 +178,7 @@ def kernel_table(size, prefill, batch, ctx, peaks):
         if phase == "decode":
             add("ssd_scan", phase, ms, 4.0 * T * Hs * N * P, B * Hs * N * P * 8.0, "hbm", "bytes = state read + write")
         else:
-            add("ssd_scan", phase, ms, 4.0 * T * Hs * N * P, 0.0, "fp32", "token-serial recurrence")
+            add("ssd_scan", phase, ms, 4.0 * T * Hs * N * P, 0.0, "fp32", "recurrence in blocks of eight tokens")
         # routed experts (sort + grouped gate|up + grouped down + combine)
         mo, D = s["moe"], s["width"]
         E, top, F = mo["experts"], mo["top"], mo["ff"]

@@ -7,7 +7,7 @@ Per size: prefill tokens/s (one prompt of `prefill` tokens in one step) and deco
 context `ctx`, one token each) of the three models, CUDA events after warm-up, and a table of the new design's kernels
 timed alone at the same shapes (as replays of a CUDA graph of several calls, so that small kernels are not timed at the
 rate of Python's launches) with their algorithmic bytes / flops against the measured copy bandwidth and cuBLAS bf16 peak
-(the token-serial scans against the nominal fp32 FMA rate).  Every row is followed by a `like` row: the same kernel at the
+(the scans against the nominal fp32 FMA rate).  Every row is followed by a `like` row: the same kernel at the
 same shape with the new options off, or the closest kernel of the other models."""
 from __future__ import annotations
 
@@ -195,7 +195,7 @@ def kernel_table(size, prefill, batch, ctx, peaks):
                          ("like: decayed scan (decay per key channel)", dict(chan_decay=chan))):
             add(name, phase, lambda: ops.decay_attn(qr, kr, vr, state, slots, cu, cl, **kw), 4.0 * T * H * dk * dv,
                 B * H * dk * dv * 8.0, "hbm" if dec else "fp32",
-                "bytes = state read + write; ops packs the rows first" if dec else "token-serial scan; ops packs the rows first")
+                "bytes = state read + write" if dec else "scan in blocks of eight tokens")
         y, gg = rnd(T, H * dv), rnd(T, H * dv)
         add("head norm + SiLU gate (no weight)", phase, lambda: ops.gated_group_norm(y, gg, None, dv, 1e-6, False), 0.0, T * H * dv * 10.0)
         wv = rnd(dv)

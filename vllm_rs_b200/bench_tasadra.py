@@ -6,7 +6,7 @@ runner), at equal width and depth: `python bench.py --config tasadra`.
 Per size: prefill tokens/s (one prompt of `prefill` tokens in one step) and decode tokens/s (`batch` sequences at
 context `ctx`, one token each) of both models, CUDA events after warm-up, and a table of the new design's kernels timed
 alone at the same shapes with their algorithmic bytes / flops against the measured copy bandwidth and cuBLAS bf16 peak
-(the token-serial scans against the nominal fp32 FMA rate).  Every row of a kernel that gained an option, and every new
+(the scans against the nominal fp32 FMA rate).  Every row of a kernel that gained an option, and every new
 kernel, is followed by a `like` row: the same kernel at the same shape with the option off, or the closest kernel the
 other models use."""
 from __future__ import annotations
@@ -206,7 +206,7 @@ def kernel_table(size, prefill, batch, ctx, peaks):
             if phase == "decode":
                 add(name, phase, ms, 6.0 * T * H * dk * dv, sbytes, "hbm", "bytes = state read + write")
             else:
-                add(name, phase, ms, 6.0 * T * H * dk * dv, 0.0, "fp32", "token-serial scan")
+                add(name, phase, ms, 6.0 * T * H * dk * dv, 0.0, "fp32", "scan in blocks of eight tokens")
         del state, decay, qd, kd, vd
         # ---- the row kernels of the layer
         x, w, b, sh = rnd(T, D), rnd(D), rnd(D), torch.rand(D, generator=g, device=dev)

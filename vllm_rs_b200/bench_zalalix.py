@@ -143,7 +143,7 @@ def kernel_table(size, prefill, batch, ctx, peaks):
             if phase == "decode":
                 add(name, phase, ms, 4.0 * T * Hd * ddk * ddv, B * Hd * ddk * ddv * 8.0, "hbm", "bytes = state read + write")
             else:
-                add(name, phase, ms, 4.0 * T * Hd * ddk * ddv, 0.0, "fp32", "token-serial recurrence")
+                add(name, phase, ms, 4.0 * T * Hd * ddk * ddv, 0.0, "fp32", "recurrence in blocks of eight tokens")
         ri = s["right"]
         C, rk = ri["heads"] * ri["dim"], ri["rank"]
         low, w2, b2 = rnd(T, rk), rnd(C, rk), rnd(C)
