@@ -91,6 +91,8 @@ def test_grouped_heads(lib, H, G, Gv, dk, dv, opt, lens, ctxs):
     f = lambda name, *shape: torch.randn(*shape, generator=g) if opt.get(name) else None      # noqa: E731
     sink, slopes = f("sink", H), f("slopes", H)
     slopes = slopes.abs() * 0.02 if slopes is not None else None
+    if "low" in opt:
+        sink[::2] = opt["low"]
     table = torch.randn(H, opt["table"], generator=g) if opt.get("table") else None
     gate = {"head": torch.randn(T, H, generator=g), "elem": torch.randn(T, H * dv, generator=g)}.get(opt.get("gate"))
     scale, window, keep, chunk, cap = dk ** -0.5, opt.get("window", 0), opt.get("keep", 0), opt.get("chunk", 0), opt.get("cap", 0.0)
@@ -117,13 +119,15 @@ def test_grouped_heads(lib, H, G, Gv, dk, dv, opt, lens, ctxs):
 @pytest.mark.parametrize("lens,ctxs", LENS + [([420], [420])])
 @pytest.mark.parametrize("H,rank,rot,window", [(16, 256, 32, 100), (32, 512, 32, 0), (24, 512, 64, 129), (20, 320, 32, 64),
                                                (3, 64, 0, 1), (128, 128, 32, 77), (9, 448, 32, 0)])
-def test_latent_rows(lib, H, rank, rot, window, lens, ctxs):
+def test_latent_rows(lib, H, rank, rot, window, lens, ctxs, low=None):
     from vllm_rs_b200 import ops
     g = torch.Generator().manual_seed(H * rank + sum(ctxs))
     R, T = rank + rot, sum(lens)
     cache, bt, put = _pages(g, ctxs, (R,))
     q = (torch.randn(T, H, R, generator=g) * 0.7).bfloat16()
     sink, gate = torch.randn(H, generator=g), torch.randn(T, H, generator=g)
+    if low is not None:
+        sink[::2] = low
     want, mag, at = [], [], 0
     for b, (n, c) in enumerate(zip(lens, ctxs)):
         k = torch.randn(c, R, generator=g).bfloat16()
@@ -139,3 +143,13 @@ def test_latent_rows(lib, H, rank, rot, window, lens, ctxs):
         out = ops.latent_attn(q.float().cuda(), cache.cuda(), sink.cuda(), cu, _i32(ctxs), bt.cuda(), kv_rank=rank, rot_dim=rot,
                               window=window, scale=0.1, split=split, gate=gate.cuda())
         _check(out, torch.cat(want), torch.cat(mag))
+
+
+@pytest.mark.parametrize("low", [-math.inf, torch.finfo(torch.float32).min])
+@pytest.mark.parametrize("lens,ctxs", [([1, 1], [64, 700]), ([70], [333]), ([130, 257], [130, 300])])
+def test_sinks_below_all_scores(lib, low, lens, ctxs):
+    """A sink that weighs nothing: heads that have it are heads without one, also where a row's first page holds no key that
+    it sees (windows and chunks that start inside a page, for the later tokens of a tile)."""
+    for opt in (dict(window=100), dict(window=65, keep=3, cap=9.0, gate="head"), dict(chunk=96, slopes=True)):
+        test_grouped_heads(lib, 16, 4, 4, 128, 128, dict(opt, sink=True, low=low), lens, ctxs)
+    test_latent_rows(lib, 8, 256, 32, 100, lens, ctxs, low)

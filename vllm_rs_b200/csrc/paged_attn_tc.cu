@@ -467,7 +467,12 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
     int it = 0;
     const int passes = q4 < nwarps ? a.ppc : 0;              // a warp without rows is done
     for (int pi = 0; pi < passes; ++pi) {
+      // A sink below every score that counts is no sink (and -inf as a reference makes NaN of a page without a visible key).
       float m_ref = with_sink && valid ? p.sink[h] * kLog2e : kNone, l = with_sink ? 1.f : 0.f;
+      if (m_ref < kNone) {
+        m_ref = kNone;
+        l = 0.f;
+      }
       const int vn = v_count(pass0 + pi);
       for (int j = 0; j < n; ++j, ++it) {
         const int base = page_of(j0 + j) * kTok;
