@@ -12,7 +12,7 @@
 // learned per-head sink logit that joins the softmax denominator without a key or value, and a per-head output gate
 // (head h's result times sigmoid(gate[t, h]); the gate commutes with the value expansion that follows).  A layer may
 // read ANOTHER layer's cache (latent_prep with no cache: queries only), with its own W_uk / W_uv folded in around it.
-// bf16 caches with kv_rank a multiple of 64 and kv_rank + rot_dim a multiple of 32 take paged_attn_tc.cu (tcgen05; prompt
+// bf16 caches with kv_rank a multiple of 64 up to 512 and kv_rank + rot_dim a multiple of 32 take paged_attn_tc.cu (tcgen05; prompt
 // 4096, 32 heads, rank 512, window 2048: 7766 -> 690 us against the kernel here).  For the other sizes: an fp32 FMA form (any
 // sizes, both dtypes; rows of small steps split their keys over several blocks and merge) and an mma.sync form for steps
 // of many rows (kv_rank a multiple of 64 up to 512, kv_rank + rot_dim a multiple of 16).  Beside paged_attn_decode.cu / attn_prefill*.cu (per-head K / V caches, fp16 / bf16, no window
@@ -522,8 +522,9 @@ void launch_latent_attn(void* out, const float* q_full, const void* cache, const
                         int max_blocks, int num_seqs, int T, int heads, int kv_rank, int rot_dim, int window, float scale,
                         int dt, void* workspace, cudaStream_t st_) {
   if (T <= 0) return;
-  // bf16: the tcgen05 form takes ranks that are multiples of 64 (rows: of 32) and up to 128 heads
-  if (!dt && latent_mma_enabled()) {
+  // bf16: the tcgen05 form takes ranks that are multiples of 64 (rows: of 32) and up to 128 heads, among the sizes that have a
+  // tensor-core form at all: ranks past 512 keep their queries and weights in fp32, in the FMA form.
+  if (!dt && latent_mma_enabled() && latent_mma_shape_ok(kv_rank, rot_dim)) {
     const int nsplit = few_rows(T) && workspace ? attn_tc_splits(T, 1, kv_rank, 1, window, 0) : 1;
     float* po = reinterpret_cast<float*>(workspace);
     const AttnTcProblem p{out, q_full, cache, nullptr, sink, gate, ld_gate, 0, cu, ctx, block_tables, max_blocks, num_seqs, T,

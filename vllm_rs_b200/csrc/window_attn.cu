@@ -35,7 +35,7 @@
 // that size; NULL: no norm), rotates the first rot_dims entries of every q and k head as interleaved pairs (2i, 2i+1)
 // by the angle position * freq[i] (angles in double), writes the K and V rows at the token's slot and the query in fp32.
 //
-// Attention kernels: bf16 caches with dim a multiple of 32 (64 at least) and vdim a multiple of 64 take paged_attn_tc.cu
+// Attention kernels: bf16 caches with dim a multiple of 32 (64 at least) and vdim a multiple of 64 up to 256 take paged_attn_tc.cu
 // (tcgen05; prompt 4096 x 16 heads of 128, window 1024: 622 -> 99 us; 32 decoded tokens over 2048 keys, 32 heads: 317 -> 59 us
 // against the kernels here).  For the other sizes: an fp32 FMA form (any sizes, both dtypes; the rows of small steps split
 // their keys over several blocks and merge) and mma.sync forms: for steps of many rows 64 token rows per block with the
@@ -944,9 +944,13 @@ void launch_window_attn(void* out, const float* q, const void* k_cache, const vo
     set_error(1, "window_attn: kv_heads is a multiple of v_heads");
     return;
   }
-  // bf16: the tcgen05 form takes key sizes that are multiples of 32 and value sizes that are multiples of 64
-  if (!dt && window_mma_enabled()) {
-    const int nsplit = few_rows(T) && workspace ? attn_tc_splits(T, kv_heads, vdim, 0, window, keep_first) : 1;
+  // bf16: the tcgen05 form takes key sizes that are multiples of 32 and value sizes that are multiples of 64, among the sizes
+  // that have a tensor-core form at all: the others (values wider than 256, more score maps at decode than fit) keep their
+  // queries and weights in fp32, in the FMA form.
+  const bool hrows = few_rows(T);
+  const bool tensor = !dt && window_mma_enabled() && window_mma_shape_ok(dim, vdim, hrows ? kv_heads / v_heads : 1);
+  if (tensor) {
+    const int nsplit = hrows && workspace ? attn_tc_splits(T, kv_heads, vdim, 0, window, keep_first) : 1;
     float* po = reinterpret_cast<float*>(workspace);
     const AttnTcProblem p{out, q, k_cache, v_cache, sink, gate, ld_gate, gate_elems, cu, ctx, block_tables, max_blocks, num_seqs,
                           T, heads, kv_heads, v_heads, dim, vdim, window, keep_first, chunk, scale, softcap, slopes, dist_bias,
@@ -962,7 +966,7 @@ void launch_window_attn(void* out, const float* q, const void* k_cache, const vo
     }
   }
   // other sizes, steps of many rows, value sizes up to 128: the mma.sync form with 64 token rows per block
-  if (!dt && window_mma_enabled() && !few_rows(T) && window_rows_enabled() && dim % 16 == 0 && vdim % 16 == 0 &&
+  if (!dt && window_mma_enabled() && !hrows && window_rows_enabled() && dim % 16 == 0 && vdim % 16 == 0 &&
       vdim <= 128) {
     const int stage_bias = dist_bias && dist_n <= 2048;
     const size_t smem = (static_cast<size_t>(WKT + RQ) * (dim + 8) + static_cast<size_t>(WKT) * (vdim + 8)) * 2 +
@@ -997,8 +1001,7 @@ void launch_window_attn(void* out, const float* q, const void* k_cache, const vo
     }
   }
   // bf16: the tensor-core kernel; steps of few rows take its heads-as-rows form with the keys split over blocks
-  const bool hrows = few_rows(T);
-  if (!dt && window_mma_enabled() && window_mma_shape_ok(dim, vdim, hrows ? kv_heads / v_heads : 1)) {
+  if (tensor) {
     const size_t smem = window_mma_smem(dim, vdim, hrows ? kv_heads / v_heads : 1);
     const int nsplit = hrows && workspace ? window_attn_mma_splits(T, heads, kv_heads, window, keep_first, v_heads) : 1;
     float* part_o = reinterpret_cast<float*>(workspace);
