@@ -99,3 +99,44 @@ def test_operands_as_they_lie(lib):
     _lib.check()
     for o, s in ((views, states[1]), (out, states[2])):
         assert torch.equal(o, want) and torch.equal(s, states[0])
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), -float("inf")])
+@pytest.mark.parametrize("kind", ["delta", "delta_chan", "decay", "decay_chan", "ssd"])
+def test_non_finite_tokens_stay_behind(lib, kind, bad):
+    """An entry that is not finite, in a key, a query, a value, a strength or a decay of one token, leaves the outputs before that
+    token as they are, wherever in a block of eight it stands."""
+    from vllm_rs_b200 import ops
+    T, H, d, e = 40, 2, 64, 32
+    g = torch.Generator().manual_seed(11)
+    r = lambda *s: torch.randn(*s, generator=g).cuda()                        # noqa: E731
+    q, k, v, b, a, dec = r(T, H, d), r(T, H, d), r(T, H, e), r(T, H), r(T, H), torch.sigmoid(r(T, H, d) + 2)
+    alog, dtb, state, tail = r(H) * 0.5, r(H), r(1, H, d, e), (_i32([0]), _i32([0, T]), _i32([T + 3]))
+
+    def run(**x):
+        o = dict(q=q, k=k, v=v, b=b, a=a, dec=dec)
+        o.update(x)
+        s = state.clone()
+        if kind == "delta":
+            return ops.delta_rule(o["q"], o["k"], o["v"], o["b"], o["a"], alog, dtb, s, *tail)
+        if kind == "delta_chan":
+            return ops.delta_rule_chan(o["q"], o["k"], o["v"], o["b"], o["dec"], s, *tail)
+        if kind == "ssd":
+            return ops.ssd_scan(o["v"], o["k"], o["q"], o["a"], alog, dtb, r(H), s, *tail)
+        kw = dict(chan_decay=o["dec"]) if kind == "decay_chan" else dict(head_decay=torch.full((H,), 0.9, device="cuda"))
+        return ops.decay_attn(o["q"], o["k"], o["v"], s, *tail, **kw)
+
+    g.manual_seed(12)
+    want = run()
+    assert torch.isfinite(want).all()
+    names = {"delta": "qkvba", "delta_chan": ["q", "k", "v", "b", "dec"], "ssd": "qkva", "decay": "qkv",
+             "decay_chan": ["q", "k", "v", "dec"]}[kind]
+    for name in names:
+        for t in (1, 7, 11, 12, 38):
+            x = dict(q=q, k=k, v=v, b=b, a=a, dec=dec)[name].clone()
+            x[t].view(-1)[5 % x[t].numel()] = bad
+            g.manual_seed(12)
+            got = run(**{name: x})
+            assert torch.equal(got[:t], want[:t]), (name, t)
+            if name == "v" and bad != bad:
+                assert not torch.isfinite(got[t]).all()

@@ -540,6 +540,11 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
       }
       float* us = sm + SM::kU + warp * kBT * 4;
       const int tt = lane >> 2, c4 = lane & 3;         // the token and column whose sums this lane gets
+      // The lane that holds token j's part.  For the tokens after tt, which the triangles have zeros for, this lane's own: a
+      // later token may be infinite or NaN, and zero times that would reach back (leaving them out by a branch: 617 -> 666 us).
+      int from[kBT];
+#pragma unroll
+      for (int j = 0; j < kBT; ++j) from[j] = min(j, tt) * 4 + c4;
       for (int i = 0; i < nblk; ++i) {
         const int g = blocks + i;
         mbar_wait_limited(&ready[g % kRing], (g / kRing) & 1, fail, err);
@@ -573,7 +578,7 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
           const float T[kBT] = {ta.x, ta.y, ta.z, ta.w, tb.x, tb.y, tb.z, tb.w};
           u = 0.f;
 #pragma unroll
-          for (int j = 0; j < kBT; ++j) u += T[j] * __shfl_sync(0xffffffffu, r, j * 4 + c4);
+          for (int j = 0; j < kBT; ++j) u += T[j] * __shfl_sync(0xffffffffu, r, from[j]);
         }
         us[lane] = CHAN ? u : u * G[3 * kBT + tt];
         __syncwarp();
@@ -584,7 +589,7 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
           const float P[kBT] = {pa.x, pa.y, pa.z, pa.w, pb.x, pb.y, pb.z, pb.w};
           float o = gt * e;
 #pragma unroll
-          for (int j = 0; j < kBT; ++j) o += P[j] * __shfl_sync(0xffffffffu, u, j * 4 + c4);
+          for (int j = 0; j < kBT; ++j) o += P[j] * __shfl_sync(0xffffffffu, u, from[j]);
           if (MODE == kDecay) o *= a.q_scale;
           if (MODE == kSsd) o += skip * vt;
           const int t = t0 + i * kBT + tt;
