@@ -552,14 +552,14 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
           m_ref = mx;
           grow = true;
         }
-        // the sum takes the weights as the product does, rounded to bf16: their roundings cancel in the quotient
         float sum[4] = {0.f, 0.f, 0.f, 0.f};
         uint32_t pk[32];
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
-          pk[i] = pack16x2<true>(ex2(fmaf(x[2 * i], mult, -m_ref)), ex2(fmaf(x[2 * i + 1], mult, -m_ref)));
-          sum[(2 * i) & 3] += __uint_as_float(pk[i] << 16);
-          sum[(2 * i + 1) & 3] += __uint_as_float(pk[i] & 0xFFFF0000u);
+          const float p0 = ex2(fmaf(x[2 * i], mult, -m_ref)), p1 = ex2(fmaf(x[2 * i + 1], mult, -m_ref));
+          pk[i] = pack16x2<true>(p0, p1);
+          sum[(2 * i) & 3] += p0;
+          sum[(2 * i + 1) & 3] += p1;
         }
         l = fmaf(l, corr, (sum[0] + sum[1]) + (sum[2] + sum[3]));
         // Value rows past the sequence's end may hold anything, and 0 * NaN is no 0; a single token does not even meet the
