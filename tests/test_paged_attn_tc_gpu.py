@@ -172,3 +172,28 @@ def test_sizes_without_a_tensor_core_form(lib, lens, ctxs):
     if sum(lens) <= 74:
         test_grouped_heads(lib, 12, 12, 1, 128, 64, dict(f32=True, q32=True), lens, ctxs)
     test_latent_rows(lib, 5, 576, 32, 100, lens, ctxs, q32=True)
+
+
+@pytest.mark.parametrize("n", [1, 5])
+def test_largest_weight_of_a_page_is_exact(lib, n):
+    """Steps of few rows: one key per page counts, and each page's weight lies half way between two bf16 numbers relative to the
+    first page's.  Relative to its own page it is one, so that nothing but fp32 sums is left (no split: one reference per row)."""
+    from vllm_rs_b200 import ops
+    pages, dk, dv = 6, 64, 64
+    k = torch.zeros(pages * 64, 1, dk)
+    k[:, 0, 0] = -30.0                                                        # weight 2^-43 at most
+    step = math.log(2 ** -1 * (1 + 3 * 2.0 ** -9))                            # 3 x 2^-9: bf16 rounds the weight by 2^-9
+    q = torch.zeros(n, 1, dk)
+    q[:, 0, 0], q[:, 0, 1] = 1.0, step
+    for p in range(pages):
+        k[p * 64, 0, 0], k[p * 64, 0, 1] = 0.0, 1.0 if p else 0.0
+    q = q.bfloat16().float()
+    scale = step / q[0, 0, 1].item()                                          # the second entry's product is `step` again
+    g = torch.Generator().manual_seed(3)
+    v = torch.randn(pages * 64, 1, dv, generator=g).bfloat16()
+    want, mag = _want(q.double(), k.double(), v.double(), torch.arange(pages * 64 - n, pages * 64), scale, 0, 0, 0, 0.0, None, None,
+                      None, None)
+    out = ops.window_attn(q.cuda(), k.bfloat16().cuda().reshape(pages, 64, 1, dk), v.cuda().reshape(pages, 64, 1, dv), None, None,
+                          _i32([0, n]), _i32([pages * 64]), _i32([list(range(pages))]), window=0, keep_first=0, scale=scale,
+                          split=False, out_f32=True)
+    assert bool(((out.double().cpu() - want).abs() <= 2e-5 * mag).all())

@@ -25,6 +25,8 @@ struct AttnTcProblem {
   int nsplit;                      // key splits; > 1: unnormalised parts [T, heads, nsplit, vdim] and (max, sum) pairs
   float *part_o, *part_ml;
 };
+// steps of few rows (decoding): the keys of a row are split over several blocks
+inline bool attn_few_rows(int T) { return T <= 2 * sm_count() / 4; }
 // whether these sizes and pointers are taken (bf16 caches only)
 bool attn_tc_takes(const AttnTcProblem& p);
 // key splits that fill the chip for a step of T rows of which every sequence brings few (1: no split)

@@ -889,8 +889,6 @@ static size_t window_mma_smem(int dim, int vdim, int maps = 1) {
 static bool window_mma_shape_ok(int dim, int vdim, int maps = 1) {
   return dim % 16 == 0 && vdim % 32 == 0 && vdim <= 256 && maps <= WQ && window_mma_smem(dim, vdim, maps) <= 200 * 1024;
 }
-// steps of few rows (decoding): the keys of a row are split over several blocks
-static bool few_rows(int T) { return T <= 2 * sm_count() / 4; }
 // blocks per token of the heads-as-rows form: a value head's group takes ceil(per_group / hpg) blocks
 static int window_mma_row_blocks(int heads, int kv_heads, int v_heads) {
   const int maps = std::max(1, kv_heads / v_heads), per_group = heads / kv_heads;
@@ -920,7 +918,7 @@ size_t window_attn_workspace_bytes(int T, int heads, int kv_heads, int vdim, int
   if (v_heads <= 0 || kv_heads % v_heads != 0) v_heads = kv_heads;
   const int n = std::max({window_attn_splits(T, heads, kv_heads, window, keep_first),
                           window_attn_mma_splits(T, heads, kv_heads, window, keep_first, v_heads),
-                          few_rows(T) ? attn_tc_splits(T, kv_heads, vdim, 0, window, keep_first) : 1});
+                          attn_few_rows(T) ? attn_tc_splits(T, kv_heads, vdim, 0, window, keep_first) : 1});
   return n == 1 ? 0 : static_cast<size_t>(T) * heads * n * (vdim + 2) * 4;
 }
 
@@ -947,7 +945,7 @@ void launch_window_attn(void* out, const float* q, const void* k_cache, const vo
   // bf16: the tcgen05 form takes key sizes that are multiples of 32 and value sizes that are multiples of 64, among the sizes
   // that have a tensor-core form at all: the others (values wider than 256, more score maps at decode than fit) keep their
   // queries and weights in fp32, in the FMA form.
-  const bool hrows = few_rows(T);
+  const bool hrows = attn_few_rows(T);
   const bool tensor = !dt && window_mma_enabled() && window_mma_shape_ok(dim, vdim, hrows ? kv_heads / v_heads : 1);
   if (tensor) {
     const int nsplit = hrows && workspace ? attn_tc_splits(T, kv_heads, vdim, 0, window, keep_first) : 1;
