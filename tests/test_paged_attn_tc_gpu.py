@@ -197,3 +197,24 @@ def test_largest_weight_of_a_page_is_exact(lib, n):
                           _i32([0, n]), _i32([pages * 64]), _i32([list(range(pages))]), window=0, keep_first=0, scale=scale,
                           split=False, out_f32=True)
     assert bool(((out.double().cpu() - want).abs() <= 2e-5 * mag).all())
+
+
+@pytest.mark.parametrize("n", [1, 90])
+def test_capped_scores_in_other_company(lib, n):
+    """A head's bits do not depend on the scores of the heads and tokens beside it (small arguments of tanh take another form)."""
+    from vllm_rs_b200 import ops
+    ctx, H, G, d = 200, 8, 2, 64
+    g = torch.Generator().manual_seed(n)
+    k, v = (torch.randn(4, 64, G, d, generator=g).bfloat16().cuda() for _ in range(2))
+    q = torch.randn(n, H, d, generator=g).cuda()
+    other = q.clone()
+    other[:, 1] *= 40.0
+    other[1:, 5] *= 40.0
+    args = (None, None, _i32([0, n]), _i32([ctx]), _i32([[2, 0, 3, 1]]))
+    a, b = (ops.window_attn(x, k, v, *args, window=0, keep_first=0, scale=0.3, softcap=9.0, out_f32=True) for x in (q, other))
+    same = torch.ones(n, H, dtype=torch.bool)
+    same[:, 1] = same[1:, 5] = False
+    assert torch.equal(a[same.cuda()], b[same.cuda()])
+    _check(a, *_want(q.bfloat16().double().cpu(), *(t[[2, 0, 3, 1]].reshape(256, G, d)[:ctx].double().cpu() for t in (k, v)),
+                     torch.arange(ctx - n, ctx), 0.3, 0, 0, 0, 9.0, None, None, None, None))
+    assert not torch.equal(a[:, 1], b[:, 1])

@@ -106,7 +106,7 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
   asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
   return r;
 }
-// tanh(y) = y P(y^2) for |y| <= kTanhMax: minimax fit of tanh(y) / y in y^2, relative error 3e-8 before rounding
+// tanh(y) = y P(y^2) for |y| <= kTanhMax: fit of tanh(y) / y in y^2, relative error 6.6e-8 before rounding
 constexpr float kTanhMax = 0.75f;
 constexpr float kT0 = 1.f, kT1 = -0.33332958817481995f, kT2 = 0.1332540661096573f, kT3 = -0.05334442853927612f,
                 kT4 = 0.019582903012633324f, kT5 = -0.004716253839433193f;
@@ -508,22 +508,29 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
           }
           big0 = max3(big0, fabsf(x[kTok - 2]), fabsf(x[kTok - 1]));
           mult = cap2;
+          auto near = [&](float& lo, float& hi) {              // two arguments up to kTanhMax
+            const f2 y = mul2(pack2(lo, hi), pack2(sl, sl)), t = mul2(y, y);
+            f2 q = fma2(t, pack2(kT5, kT5), pack2(kT4, kT4));
+            q = fma2(t, q, pack2(kT3, kT3));
+            q = fma2(t, q, pack2(kT2, kT2));
+            q = fma2(t, q, pack2(kT1, kT1));
+            q = mul2(y, fma2(t, q, pack2(kT0, kT0)));
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(q));
+          };
           if (__all_sync(0xffffffffu, fmaxf(big0, big1) * sl <= kTanhMax)) {
 #pragma unroll
-            for (int i = 0; i < kTok; i += 2) {
-              const f2 y = mul2(pack2(x[i], x[i + 1]), pack2(sl, sl)), t = mul2(y, y);
-              f2 q = fma2(t, pack2(kT5, kT5), pack2(kT4, kT4));
-              q = fma2(t, q, pack2(kT3, kT3));
-              q = fma2(t, q, pack2(kT2, kT2));
-              q = fma2(t, q, pack2(kT1, kT1));
-              q = mul2(y, fma2(t, q, pack2(kT0, kT0)));
-              asm("mov.b64 {%0, %1}, %2;" : "=f"(x[i]), "=f"(x[i + 1]) : "l"(q));
-            }
+            for (int i = 0; i < kTok; i += 2) near(x[i], x[i + 1]);
           } else {
-            // tanh(y) = 1 - 2 / (e^(2 y) + 1)
+            // tanh(y) = 1 - 2 / (e^(2 y) + 1) past kTanhMax.  Which form a score takes is its own affair: a row's bits do not
+            // depend on the rows and heads that share its warp.
             const float e2 = sl * (2.f * kLog2e);
 #pragma unroll
-            for (int i = 0; i < kTok; ++i) x[i] = fmaf(-2.f, rcp(ex2(x[i] * e2) + 1.f), 1.f);
+            for (int i = 0; i < kTok; i += 2) {
+              float a0 = x[i], a1 = x[i + 1];
+              near(a0, a1);
+              x[i] = fabsf(x[i]) * sl <= kTanhMax ? a0 : fmaf(-2.f, rcp(ex2(x[i] * e2) + 1.f), 1.f);
+              x[i + 1] = fabsf(x[i + 1]) * sl <= kTanhMax ? a1 : fmaf(-2.f, rcp(ex2(x[i + 1] * e2) + 1.f), 1.f);
+            }
           }
         }
         if (BIAS) {
