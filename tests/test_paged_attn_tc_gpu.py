@@ -218,3 +218,25 @@ def test_capped_scores_in_other_company(lib, n):
     _check(a, *_want(q.bfloat16().double().cpu(), *(t[[2, 0, 3, 1]].reshape(256, G, d)[:ctx].double().cpu() for t in (k, v)),
                      torch.arange(ctx - n, ctx), 0.3, 0, 0, 0, 9.0, None, None, None, None))
     assert not torch.equal(a[:, 1], b[:, 1])
+
+
+@pytest.mark.parametrize("bad", [math.nan, math.inf])
+@pytest.mark.parametrize("H,G,tile", [(16, 4, 32), (8, 8, 128), (32, 1, 4)])
+def test_later_tokens_of_a_page_stay_out(lib, H, G, tile, bad):
+    """A key and a value that are not finite leave the tiles before their token alone, also where tiles end inside a page."""
+    from vllm_rs_b200 import ops
+    n, d, past = 300, 64, 20
+    g = torch.Generator().manual_seed(tile)
+    pages = -(-(n + past) // 64)
+    k, v = (torch.randn(pages * 64, G, d, generator=g).bfloat16().cuda() for _ in range(2))
+    q = torch.randn(n, H, d, generator=g).cuda()
+    args = (None, None, _i32([0, n]), _i32([n + past]), _i32([list(range(pages))]))
+    run = lambda: ops.window_attn(q, *(t.reshape(pages, 64, G, d) for t in (k, v)), *args, window=0, keep_first=0, scale=0.2)  # noqa: E731
+    want = run()
+    for t in (tile, 2 * tile + 1, n - 1):
+        kept = k[past + t].clone(), v[past + t].clone()
+        k[past + t], v[past + t] = bad, bad
+        got = run()
+        clean = t // tile * tile
+        assert torch.equal(got[:clean], want[:clean]) and not torch.isfinite(got[t]).all()
+        k[past + t], v[past + t] = kept

@@ -575,9 +575,9 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
           sum[(2 * i + 1) & 3] += p1;
         }
         l = fmaf(l, corr, (sum[0] + sum[1]) + (sum[2] + sum[3]));
-        // Value rows past the sequence's end may hold anything, and 0 * NaN is no 0; a single token does not even meet the
-        // rows before its window.
-        const int v_end = p_ctx - base, v_lo = nt == 1 && base + kTok > p.keep_first ? key_lo - base : 0;
+        // Value rows past the tile's last token may hold anything (later tokens, and what lies behind the sequence), and 0 * NaN
+        // is no 0; a single token does not even meet the rows before its window.
+        const int v_end = pos_last + 1 - base, v_lo = nt == 1 && base + kTok > p.keep_first ? key_lo - base : 0;
         if (v_end < kTok || v_lo > 0) {
           mbar_wait_limited(&v_full[vr.s], vr.ph, fail, a.err);
           uint8_t* vt = v_smem + vr.s * a.v_stage + (r & 7) * 16;
