@@ -801,8 +801,8 @@ template <int DK, int MODE, bool CHAN, int WW>
 static void launch_scan_ww(const ScanArgs& a, int num_seqs, int* err, cudaStream_t st_) {
   using SM = ScanSmem<DK, CHAN, WW>;
   auto kern = scan_kernel<DK, MODE, CHAN, WW>;
-  static const cudaError_t sized = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SM::kBytes);
-  (void)sized;
+  static OncePerDevice sized;
+  if (!allow_smem(sized, kern, SM::kBytes)) return;
   const int cols = (a.vdim + SM::kCols - 1) / SM::kCols;
   // a few blocks per SM, each taking every so many sequences (a step of decoded tokens is over at once)
   const int z = std::max(1, std::min(num_seqs, 4 * sm_count() / (cols * a.heads)));

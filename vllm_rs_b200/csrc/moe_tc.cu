@@ -292,8 +292,8 @@ static void launch(void* out, const void* a, const void* w, const int32_t* off, 
     return;
   }
   auto kern = grouped_linear_tc_kernel<ACT, BN>;
-  static const cudaError_t sized = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BN>::kSmem);
-  (void)sized;
+  static OncePerDevice sized;
+  if (!allow_smem(sized, kern, Cfg<BN>::kSmem)) return;
   const int most = std::min(pairs, E + pairs / kM) * g.ntiles_n;        // no step has more tiles
   kern<<<std::min(most, sm_count()), kThreads, Cfg<BN>::kSmem, st>>>(amap, wmap, g);
   B200_CUDA_LAUNCH_CHECK();

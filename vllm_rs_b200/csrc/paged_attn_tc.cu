@@ -761,12 +761,8 @@ void launch_attn_tc(const AttnTcProblem& p, cudaStream_t st) {
   const bool cap = p.softcap > 0.f, bias = p.slopes || p.dist_bias;
   auto kern = cap ? (bias ? attn_tc_kernel<true, true> : attn_tc_kernel<true, false>)
                   : (bias ? attn_tc_kernel<false, true> : attn_tc_kernel<false, false>);
-  static const bool sized = [] {
-    for (auto k : {attn_tc_kernel<true, true>, attn_tc_kernel<true, false>, attn_tc_kernel<false, true>, attn_tc_kernel<false, false>})
-      cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
-    return true;
-  }();
-  (void)sized;
+  static OncePerDevice sized[4];
+  if (!allow_smem(sized[cap * 2 + bias], kern, kSmemMax)) return;
   kern<<<grid, kThreads, smem, st>>>(kmap, tmap, vmap, a);
   B200_CUDA_LAUNCH_CHECK();
 }

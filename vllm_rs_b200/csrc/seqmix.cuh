@@ -14,8 +14,21 @@
 
 #include "../../include/b200_vllm.h"
 #include "common.cuh"
+#include "host/per_device.hpp"
 
 namespace b200 {
+
+// Lets `kern` use `bytes` of dynamic shared memory on the current device; false (and an error): it cannot.
+template <typename Kern>
+inline bool allow_smem(OncePerDevice& once, Kern kern, int bytes) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = once(dev, [&] { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); });
+  if (e == cudaSuccess) return true;
+  cudaGetLastError();
+  set_error(2, cudaGetErrorString(e));
+  return false;
+}
 namespace seqmix {
 
 constexpr int kPage = 64;          // tokens per cache page (the block manager's block size)
