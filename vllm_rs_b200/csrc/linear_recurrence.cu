@@ -417,7 +417,12 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
         }
         sync();
         // ---- P (t, j) = decayed q_t . k_j, j <= t, and (delta) M (t, j) = beta_t times the decayed k_t . k_j, j < t, then
-        // T = (1 + M)^-1.  A lane holds its rows of all eight tokens; the sums over the lanes go an entry to a lane.
+        // T = (1 + M)^-1.  A lane holds its rows of all eight tokens; the sums over the lanes go an entry to a lane.  Rows of P and
+        // T are stored from the diagonal back (entry d: token t - d; zero past the first), so that the walk reaches token t - d
+        // by a shuffle from d tokens below.  For tokens before the block that gives a lane's own part, never a later token's,
+        // which may be infinite or NaN and reach back through its zero.  (Two other ways to leave later tokens out: a branch,
+        // 617 -> 666 us for 4096 tokens of 16 heads of 128 x 128; source lanes in registers, 955 -> 1114 us for 32 heads with a
+        // decay per channel.)
         if (pw == 3) {
           if (i + 2 < nblk) make_scalars(i + 2);
         } else if (pw != 1 || MODE == kDelta) {
@@ -460,7 +465,7 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
           float* out = B + SM::kMat + (pw == 1 ? 0 : kBT * kBT);
           if (et < et_end) {
             v *= B[SM::kRat + et * kBT + ej];
-            out[et * kBT + ej] = pw == 1 ? v * G[kBT + et] : v;
+            out[et * kBT + (pw == 1 ? ej : et - ej)] = pw == 1 ? v * G[kBT + et] : v;
           }
           if (pw == 1) {                               // column `lane` of T by forward substitution
             __syncwarp();
@@ -477,7 +482,7 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
             __syncwarp();
             if (lane < kBT) {
 #pragma unroll
-              for (int t = 0; t < kBT; ++t) out[t * kBT + lane] = tc[t];
+              for (int t = 0; t < kBT; ++t) out[t * kBT + ((t - lane) & (kBT - 1))] = tc[t];
             }
           }
         }
@@ -540,11 +545,6 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
       }
       float* us = sm + SM::kU + warp * kBT * 4;
       const int tt = lane >> 2, c4 = lane & 3;         // the token and column whose sums this lane gets
-      // The lane that holds token j's part.  For the tokens after tt, which the triangles have zeros for, this lane's own: a
-      // later token may be infinite or NaN, and zero times that would reach back (leaving them out by a branch: 617 -> 666 us).
-      int from[kBT];
-#pragma unroll
-      for (int j = 0; j < kBT; ++j) from[j] = min(j, tt) * 4 + c4;
       for (int i = 0; i < nblk; ++i) {
         const int g = blocks + i;
         mbar_wait_limited(&ready[g % kRing], (g / kRing) & 1, fail, err);
@@ -578,7 +578,7 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
           const float T[kBT] = {ta.x, ta.y, ta.z, ta.w, tb.x, tb.y, tb.z, tb.w};
           u = 0.f;
 #pragma unroll
-          for (int j = 0; j < kBT; ++j) u += T[j] * __shfl_sync(0xffffffffu, r, from[j]);
+          for (int d = 0; d < kBT; ++d) u += T[d] * __shfl_up_sync(0xffffffffu, r, d * 4);
         }
         us[lane] = CHAN ? u : u * G[3 * kBT + tt];
         __syncwarp();
@@ -589,7 +589,7 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
           const float P[kBT] = {pa.x, pa.y, pa.z, pa.w, pb.x, pb.y, pb.z, pb.w};
           float o = gt * e;
 #pragma unroll
-          for (int j = 0; j < kBT; ++j) o += P[j] * __shfl_sync(0xffffffffu, u, from[j]);
+          for (int d = 0; d < kBT; ++d) o += P[d] * __shfl_up_sync(0xffffffffu, u, d * 4);
           if (MODE == kDecay) o *= a.q_scale;
           if (MODE == kSsd) o += skip * vt;
           const int t = t0 + i * kBT + tt;
