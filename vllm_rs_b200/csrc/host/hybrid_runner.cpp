@@ -493,7 +493,7 @@ static void mixer_delta(b200_hybrid* r, const b200_hybrid_layer& l, const uint32
     launch_lowrank_decay(decay, low_a, n_in, (const float*)l.w_decay2, (const float*)l.dt_bias, 1.f, (const float*)l.a_log,
                          l.dim, T, nd, l.chan_rank, st);
     launch_delta_rule(r->aux, q, k, v, nconv, b_raw, nullptr, n_in, nullptr, nullptr, decay, nd, (float*)l.rec_state,
-                      state_slots, cu, ctx, B, H, Hk, l.dim, l.vdim, st);
+                      state_slots, cu, ctx, B, H, Hk, l.dim, l.vdim, st, T);
     gemm_f32out(low_g, n_in, 0, l.w_gate2, l.gate_rank, 0, gate2, nv, 0, T, nv, l.gate_rank, 1, 0.f, 0, 1, st);
     launch_gated_group_norm(r->opa, r->aux, nv, gate2, nv, (const float*)l.out_norm_w, l.vdim, T, nv, l.vdim, c.norm_eps,
                             0, 1, c.dt, st);
@@ -503,7 +503,7 @@ static void mixer_delta(b200_hybrid* r, const b200_hybrid_layer& l, const uint32
   const float* a_raw = b_raw + H;
   const float* gate = a_raw + H;
   launch_delta_rule(r->aux, q, k, v, nconv, b_raw, a_raw, n_in, (const float*)l.a_log, (const float*)l.dt_bias, nullptr,
-                    0, (float*)l.rec_state, state_slots, cu, ctx, B, H, Hk, l.dim, l.vdim, st);
+                    0, (float*)l.rec_state, state_slots, cu, ctx, B, H, Hk, l.dim, l.vdim, st, T);
   launch_gated_group_norm(r->opa, r->aux, nv, gate, n_in, (const float*)l.out_norm_w, l.vdim, T, nv, l.vdim, c.norm_eps,
                           0, 0, c.dt, st);
   gemm_f32out_scaled(r->opa, nv, 0, l.w_o, nv, 0, dst, c.width, 0, T, c.width, nv, 1, alpha, beta, 0, c.dt, st);
@@ -520,7 +520,7 @@ static void mixer_ssd(b200_hybrid* r, const b200_hybrid_layer& l, const uint32_t
                          (float*)l.conv_state, state_slots, cu, ctx, B, T, nconv, l.conv_taps, st);
   launch_ssd_scan(r->aux, xbc, xbc + inner, xbc + inner + G * N, nconv, r->proj + inner + nconv, n_in, (const float*)l.a_log,
                   (const float*)l.dt_bias, (const float*)l.d_skip, (float*)l.rec_state, state_slots, cu, ctx, B, H, G, N,
-                  l.vdim, st);
+                  l.vdim, st, T);
   launch_gated_group_norm(r->opa, r->aux, inner, r->proj, n_in, (const float*)l.out_norm_w, inner, T, inner,
                           inner / l.norm_groups, c.norm_eps, 1, 0, c.dt, st);
   gemm_f32out_scaled(r->opa, inner, 0, l.w_o, inner, 0, dst, c.width, 0, T, c.width, inner, 1, alpha, beta, 0, c.dt, st);
@@ -591,7 +591,7 @@ static void mixer_decay(b200_hybrid* r, const b200_hybrid_layer& l, const int64_
     chan = r->conv;
   }
   launch_decay_attn(r->aux, q, k, v, n_in, chan ? nullptr : (const float*)l.head_decay, chan, nk, l.q_scale, l.k_scale,
-                    l.qkv_act, (float*)l.rec_state, state_slots, cu, ctx, B, H, l.dim, l.vdim, st);
+                    l.qkv_act, (float*)l.rec_state, state_slots, cu, ctx, B, H, l.dim, l.vdim, st, T);
   launch_gated_group_norm(r->opa, r->aux, nv, gate, n_in, (const float*)(l.out_norm_period ? l.out_norm_w : nullptr),
                           l.out_norm_period ? l.out_norm_period : 1, T, nv, nv / l.norm_groups, c.norm_eps, 0, l.gate_act,
                           c.dt, st);

@@ -19,7 +19,7 @@
 //                     one value per key channel and token (gated linear attention; lowrank_decay makes it from a
 //                     low-rank projection: sigmoid(z)^(1/tau)).  Optional SiLU on q, k, v and scales on q and k.
 //                     state [slots, heads, dim, vdim].
-// The three scans share two kernels.  scan_one_kernel takes the sequences that bring one token.  scan_kernel walks longer portions
+// The three scans share two kernels.  scan_short_kernel takes the sequences that bring few tokens.  scan_kernel walks longer portions
 // in blocks of eight tokens, within which the recurrence is unrolled exactly: with G_t the product of the block's decays up to
 // token t and S0 the state before it,
 //   k_t^T S_(t-1) = G_t k_t^T S0 + sum_(j<t) (G_t / G_j) (k_t . k_j) u_j,   S_t^T q_t likewise,   S_8 = G_8 S0 + sum_j (G_8 / G_j) k_j u_j^T
@@ -202,7 +202,7 @@ __device__ __forceinline__ float meet32(float (&x)[32], int lane) {
   return x[0];
 }
 
-// Portions of two tokens and more.  grid = (column blocks, heads, runs of sequences); a block walks its sequences one after
+// Portions of more than `most` tokens.  grid = (column blocks, heads, runs of sequences); a block walks its sequences one after
 // another.  The first WW warps each own four columns of S: a lane holds DK / 32 neighbouring rows of them in registers, so that
 // a key or query row is read once from shared memory for four columns (one column per lane made these reads the bound: 512
 // bytes of registers per load and warp).  Two groups of four warps take turns at fetching a block's token rows (cp.async, a
@@ -216,7 +216,7 @@ __device__ __forceinline__ float meet32(float (&x)[32], int lane) {
 // us with both in turn).
 template <int DK, int MODE, bool CHAN, int WW>
 __global__ void __launch_bounds__(WW * 32 + 256, 1)
-scan_kernel(const ScanArgs a, int num_seqs, int* err) {
+scan_kernel(const ScanArgs a, int num_seqs, int most, int* err) {
   using SM = ScanSmem<DK, CHAN, WW>;
   constexpr int CH = DK / 32, COLS = SM::kCols;
   extern __shared__ __align__(16) float sm[];
@@ -225,17 +225,29 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
   volatile int* fail = reinterpret_cast<volatile int*>(done + kRing);
   const int h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, col0 = blockIdx.x * COLS;
   const int dim = a.dim, vdim = a.vdim, hk = MODE == kDecay ? h : h / (a.heads / a.kv_heads);
+  constexpr int kAll = WW * 32 + 256;
+  {
+    int mine = 0;                                                      // a sequence for this kernel among the block's
+    for (int b = blockIdx.z + tid * gridDim.z; b < num_seqs; b += kAll * gridDim.z)
+      mine |= static_cast<int>(a.cu_seqlens_q[b + 1] - a.cu_seqlens_q[b]) > most;
+    if (!__syncthreads_or(mine)) return;
+  }
   if (tid == 0) {
     for (int i = 0; i < kRing; ++i) { mbar_init(&ready[i], 4); mbar_init(&done[i], WW); }
     *fail = 0;
     fence_barrier_init();
   }
-  for (int e = tid; e < kRing * SM::kBuf; e += WW * 32 + 256) sm[e] = 0.f;       // padding past `dim` is zero and stays it
+  // What no token writes is zero and stays it: padding past `dim` and `vdim`, the triangles' upper halves.
+  if (dim < DK || col0 + COLS > vdim) {
+    for (int e = tid; e < kRing * SM::kBuf; e += kAll) sm[e] = 0.f;
+  } else {
+    for (int e = tid; e < kRing * 2 * kBT * kBT; e += kAll) sm[e / (2 * kBT * kBT) * SM::kBuf + SM::kMat + e % (2 * kBT * kBT)] = 0.f;
+  }
   __syncthreads();
   int blocks = 0;                                                      // blocks of tokens so far, over all sequences
   for (int b = blockIdx.z; b < num_seqs; b += gridDim.z) {
     const int t0 = a.cu_seqlens_q[b], t1 = a.cu_seqlens_q[b + 1], nblk = (t1 - t0 + kBT - 1) / kBT;
-    if (t1 - t0 < 2) continue;                                         // (scan_one_kernel)
+    if (t1 - t0 <= most) continue;                                     // (scan_short_kernel)
     const bool fresh = static_cast<int>(a.context_lens[b]) == t1 - t0;
     if (warp >= WW) {
       // ---------------------------------------------------------- token rows
@@ -652,22 +664,25 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
   }
 }
 
-// Sequences that bring one token: 16 columns per block, so that a single sequence of 16 heads of 128 still makes 128 blocks.
-// 32 sequences of 16 heads of 128 x 128 move 67 MB; the call, with the other kernel's launch, is bound by its host side.  grid = (column blocks, heads, sequences); 128 threads = 32 rows x 4 columns of 4; bound by the
-// state's way in and out, which are whole 64-byte rows here.
+// Portions of up to `most` tokens, token by token.  grid = (column blocks, heads, sequences); 128 threads = 32 rows x 4 columns of
+// 4.  16 columns per block, so that a single sequence of 16 heads of 128 still makes 128 blocks, and small blocks, of which an
+// SM holds many.  Single tokens are bound by the state's way in and out, which are whole 64-byte rows here, more tokens by
+// instructions and, for the delta rule, a barrier per token; their rows are staged and normed together, CT tokens at a time.
 template <int DK, int MODE, bool CHAN>
-__global__ void __launch_bounds__(128)
-scan_one_kernel(const ScanArgs a) {
-  constexpr int NR = DK / 32;
-  __shared__ float ks[DK], qs[DK], red[2][4][kOneCols], sums[4][2];
-  const int h = blockIdx.y, b = blockIdx.z, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int t = a.cu_seqlens_q[b];
-  if (static_cast<int>(a.cu_seqlens_q[b + 1]) - t != 1) return;
-  const bool fresh = a.context_lens[b] == 1;
+__global__ void __launch_bounds__(128, DK <= 128 ? 8 : 5)
+scan_short_kernel(const ScanArgs a, int most) {
+  constexpr int NR = DK / 32, CT = DK * (CHAN ? 2 : 1) <= 128 ? 16 : 8;
+  __shared__ __align__(16) float ks[CT][DK], qs[CT][DK], ds[CHAN ? CT : 1][CHAN ? DK : 4], vs[CT][kOneCols];
+  __shared__ __align__(16) float red[2][4][kOneCols], sums[CT][4][kOneCols];
+  __shared__ float sc[CT][3];                          // decay, write strength, what the read-out is multiplied by
+  const int h = blockIdx.y, b = blockIdx.z, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, col0 = blockIdx.x * kOneCols;
+  const int t0 = a.cu_seqlens_q[b], n = static_cast<int>(a.cu_seqlens_q[b + 1]) - t0;
+  if (n < 1 || n > most) return;
+  const bool fresh = static_cast<int>(a.context_lens[b]) == n;
   const int dim = a.dim, vdim = a.vdim, hk = MODE == kDecay ? h : h / (a.heads / a.kv_heads);
-  const int c = (tid & 3) * 4, col = blockIdx.x * kOneCols + c, row = tid >> 2;
+  const int c = (tid & 3) * 4, col = col0 + c, row = tid >> 2;
   float* sp = a.state + ((static_cast<size_t>(a.state_slots[b]) * a.heads + h) * dim) * vdim + col;
-  const bool wide = vdim % 4 == 0 && (reinterpret_cast<uintptr_t>(a.state) & 15) == 0;
+  const bool wide_s = vdim % 4 == 0 && (reinterpret_cast<uintptr_t>(a.state) & 15) == 0;
   float s[NR][4];
 #pragma unroll
   for (int r = 0; r < NR; ++r) {
@@ -675,7 +690,7 @@ scan_one_kernel(const ScanArgs a) {
     s[r][0] = s[r][1] = s[r][2] = s[r][3] = 0.f;
     if (!fresh && i < dim && col < vdim) {
       const float* src = sp + static_cast<size_t>(i) * vdim;
-      if (wide) {
+      if (wide_s) {
         const float4 v = *reinterpret_cast<const float4*>(src);
         s[r][0] = v.x; s[r][1] = v.y; s[r][2] = v.z; s[r][3] = v.w;
       } else {
@@ -685,101 +700,150 @@ scan_one_kernel(const ScanArgs a) {
       }
     }
   }
-  const float* kg = a.k + static_cast<size_t>(t) * a.ld_k + hk * dim;
-  const float* qg = a.q + static_cast<size_t>(t) * a.ld_q + hk * dim;
-  float sk = 0.f, sq = 0.f;
-  for (int i = tid; i < DK; i += 128) {
-    float kv = i < dim ? kg[i] : 0.f, qv = i < dim ? qg[i] : 0.f;
-    if (MODE == kDecay && a.act) {
-      kv = silu_exact(kv);
-      qv = silu_exact(qv);
+  const bool wide = dim % 4 == 0 && (a.ld_q | a.ld_k) % 4 == 0 && (!CHAN || a.ld_decay % 4 == 0) &&
+                    ((reinterpret_cast<uintptr_t>(a.q) | reinterpret_cast<uintptr_t>(a.k) |
+                      (CHAN ? reinterpret_cast<uintptr_t>(a.chan_decay) : 0)) & 15) == 0;
+  const float skip = MODE == kSsd && a.d_skip ? a.d_skip[h] : 0.f;
+  // sums over the rows: four columns' of a thread over the lanes of these columns (halving the values), then over the warps
+  auto meet = [&](const float (&x)[4], float (*to)[kOneCols]) {
+    const bool up = lane & 16, up8 = lane & 8;
+    float a0 = up ? x[2] : x[0], a1 = up ? x[3] : x[1];
+    a0 += __shfl_xor_sync(0xffffffffu, up ? x[0] : x[2], 16);
+    a1 += __shfl_xor_sync(0xffffffffu, up ? x[1] : x[3], 16);
+    float y = up8 ? a1 : a0;
+    y += __shfl_xor_sync(0xffffffffu, up8 ? a0 : a1, 8);
+    y += __shfl_xor_sync(0xffffffffu, y, 4);
+    if (!(lane & 4)) to[warp][c + (up ? 2 : 0) + (up8 ? 1 : 0)] = y;
+  };
+  for (int c0 = 0; c0 < n; c0 += CT) {
+    const int m = min(CT, n - c0);
+    if (c0 > 0) __syncthreads();                       // the tokens before are stored
+    constexpr int TPR = DK / 4, RPS = 128 / TPR;       // threads per row, rows at a time
+    const int x = tid % TPR * 4;
+    for (int r = tid / TPR; r < m; r += RPS) {
+      const size_t t = t0 + c0 + r;
+      const float* kg = a.k + t * a.ld_k + hk * dim + x;
+      const float* qg = a.q + t * a.ld_q + hk * dim + x;
+      const float* ag = CHAN ? a.chan_decay + t * a.ld_decay + h * dim + x : nullptr;
+      if (wide && x < dim) {
+        cp_async16(&ks[r][x], kg);
+        cp_async16(&qs[r][x], qg);
+        if (CHAN) cp_async16(&ds[CHAN ? r : 0][CHAN ? x : 0], ag);
+      } else {
+#pragma unroll
+        for (int z = 0; z < 4; ++z) {
+          const bool in = x + z < dim;                 // the padding past `dim`: no key, no query, decay one
+          ks[r][x + z] = in ? kg[z] : 0.f;
+          qs[r][x + z] = in ? qg[z] : 0.f;
+          if (CHAN) ds[CHAN ? r : 0][CHAN ? x + z : 0] = in ? ag[z] : 1.f;
+        }
+      }
     }
-    ks[i] = kv;
-    qs[i] = qv;
-    sk += kv * kv;
-    sq += qv * qv;
-  }
-  if (MODE == kDelta) {
-    sk = lanes_sum(sk);
-    sq = lanes_sum(sq);
-    if (lane == 0) {
-      sums[warp][0] = sk;
-      sums[warp][1] = sq;
+    cp_async_commit();
+    for (int e = tid; e < m * kOneCols; e += 128) {
+      const int r = e / kOneCols, cc = e % kOneCols;
+      float v = col0 + cc < vdim ? a.v[static_cast<size_t>(t0 + c0 + r) * a.ld_v + h * vdim + col0 + cc] : 0.f;
+      vs[r][cc] = MODE == kDecay && a.act ? silu_exact(v) : v;
     }
-  }
-  const size_t ba = static_cast<size_t>(t) * a.ld_s + h;
-  float g = 1.f, w = a.k_scale;                        // decay; write strength
-  if (MODE == kDelta) {
-    w = sigmoid_f(a.strength[ba]);
-    if (!CHAN) g = expf(-expf(a.a_log[h]) * softplus_f(a.decay_raw[ba] + a.dt_bias[h]));
-  } else if (MODE == kSsd) {
-    w = softplus_f(a.decay_raw[ba] + a.dt_bias[h]);
-    g = expf(-expf(a.a_log[h]) * w);
-  } else if (!CHAN) {
-    g = a.head_decay[h];
-  }
-  float v[4];
+    if (tid < m) {
+      const size_t o = static_cast<size_t>(t0 + c0 + tid) * a.ld_s + h;
+      float g = 1.f, w = a.k_scale;
+      if (MODE == kDelta) {
+        w = sigmoid_f(a.strength[o]);
+        if (!CHAN) g = expf(-expf(a.a_log[h]) * softplus_f(a.decay_raw[o] + a.dt_bias[h]));
+      } else if (MODE == kSsd) {
+        w = softplus_f(a.decay_raw[o] + a.dt_bias[h]);
+        g = expf(-expf(a.a_log[h]) * w);
+      } else if (!CHAN) {
+        g = a.head_decay[h];
+      }
+      sc[tid][0] = g;
+      sc[tid][1] = w;
+      if (MODE != kDelta) sc[tid][2] = MODE == kDecay ? a.q_scale : 1.f;
+    }
+    cp_async_wait<0>();
+    __syncthreads();
+    if (MODE == kDelta) {                              // a warp per token: unit keys; the query's norm goes to the read-out
+      for (int r = warp; r < m; r += 4) {
+        float kx[NR], sk = 0.f, sq = 0.f;
 #pragma unroll
-  for (int x = 0; x < 4; ++x) {
-    v[x] = col + x < vdim ? a.v[static_cast<size_t>(t) * a.ld_v + h * vdim + col + x] : 0.f;
-    if (MODE == kDecay && a.act) v[x] = silu_exact(v[x]);
-  }
-  __syncthreads();
-  float ik = 1.f, iq = MODE == kDecay ? a.q_scale : 1.f;
-  if (MODE == kDelta) {
-    ik = 1.f / sqrtf(sums[0][0] + sums[1][0] + sums[2][0] + sums[3][0] + 1e-6f);
-    iq = rsqrtf(static_cast<float>(dim)) / sqrtf(sums[0][1] + sums[1][1] + sums[2][1] + sums[3][1] + 1e-6f);
-  }
-  // sums over the rows of four columns: lanes of the same columns, then the warps
-  auto meet = [&](float (&x)[4], int slot) {
+        for (int i = 0; i < NR; ++i) {
+          kx[i] = ks[r][lane + i * 32];
+          const float qx = qs[r][lane + i * 32];
+          sk += kx[i] * kx[i];
+          sq += qx * qx;
+        }
+        sk = lanes_sum(sk);
+        sq = lanes_sum(sq);
+        const float ik = 1.f / sqrtf(sk + 1e-6f);
 #pragma unroll
-    for (int o = 4; o < 32; o <<= 1)
+        for (int i = 0; i < NR; ++i) ks[r][lane + i * 32] = kx[i] * ik;
+        if (lane == 0) sc[r][2] = rsqrtf(static_cast<float>(dim)) / sqrtf(sq + 1e-6f);
+      }
+      __syncthreads();
+    } else if (MODE == kDecay && a.act) {
+      for (int e = tid; e < m * DK; e += 128) {
+        ks[e / DK][e % DK] = silu_exact(ks[e / DK][e % DK]);
+        qs[e / DK][e % DK] = silu_exact(qs[e / DK][e % DK]);
+      }
+      __syncthreads();
+    }
+    for (int t = 0; t < m; ++t) {
+      const float g = sc[t][0], w = sc[t][1];
+      const float4 vv = *reinterpret_cast<const float4*>(&vs[t][c]);
+      const float v[4] = {vv.x, vv.y, vv.z, vv.w};
+      float kv[NR], u[4], o[4] = {};
 #pragma unroll
-      for (int z = 0; z < 4; ++z) x[z] += __shfl_xor_sync(0xffffffffu, x[z], o);
-    if (lane < 4) {
+      for (int r = 0; r < NR; ++r) {
+        kv[r] = ks[t][row + r * 32];
+        const float d = CHAN ? ds[CHAN ? t : 0][CHAN ? row + r * 32 : 0] : g;
 #pragma unroll
-      for (int z = 0; z < 4; ++z) red[slot][warp][c + z] = x[z];
+        for (int z = 0; z < 4; ++z) s[r][z] *= d;
+      }
+      if (MODE == kDelta) {
+        float d[4] = {};
+#pragma unroll
+        for (int r = 0; r < NR; ++r)
+#pragma unroll
+          for (int z = 0; z < 4; ++z) d[z] += kv[r] * s[r][z];
+        meet(d, red[t & 1]);
+        __syncthreads();
+        float4 y[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) y[i] = *reinterpret_cast<const float4*>(&red[t & 1][i][c]);
+        u[0] = w * (v[0] - ((y[0].x + y[1].x) + (y[2].x + y[3].x)));
+        u[1] = w * (v[1] - ((y[0].y + y[1].y) + (y[2].y + y[3].y)));
+        u[2] = w * (v[2] - ((y[0].z + y[1].z) + (y[2].z + y[3].z)));
+        u[3] = w * (v[3] - ((y[0].w + y[1].w) + (y[2].w + y[3].w)));
+      } else {
+#pragma unroll
+        for (int z = 0; z < 4; ++z) u[z] = v[z] * w;
+      }
+#pragma unroll
+      for (int r = 0; r < NR; ++r) {
+        const float qv = qs[t][row + r * 32];
+#pragma unroll
+        for (int z = 0; z < 4; ++z) {
+          s[r][z] += kv[r] * u[z];
+          o[z] += qv * s[r][z];
+        }
+      }
+      meet(o, sums[t]);
     }
     __syncthreads();
-#pragma unroll
-    for (int z = 0; z < 4; ++z) x[z] = (red[slot][0][c + z] + red[slot][1][c + z]) + (red[slot][2][c + z] + red[slot][3][c + z]);
-  };
-  float u[4];
+    for (int e = tid; e < m * kOneCols; e += 128) {
+      const int r = e / kOneCols, cc = e % kOneCols;
+      if (col0 + cc < vdim)
+        a.out[(static_cast<size_t>(t0 + c0 + r) * a.heads + h) * vdim + col0 + cc] =
+            ((sums[r][0][cc] + sums[r][1][cc]) + (sums[r][2][cc] + sums[r][3][cc])) * sc[r][2] + skip * vs[r][cc];
+    }
+  }
 #pragma unroll
   for (int r = 0; r < NR; ++r) {
     const int i = row + r * 32;
-    const float d = CHAN ? (i < dim ? a.chan_decay[static_cast<size_t>(t) * a.ld_decay + h * dim + i] : 1.f) : g;
-#pragma unroll
-    for (int x = 0; x < 4; ++x) s[r][x] *= d;
-  }
-  if (MODE == kDelta) {
-    float d[4] = {};
-#pragma unroll
-    for (int r = 0; r < NR; ++r) {
-      const float kv = ks[row + r * 32] * ik;
-#pragma unroll
-      for (int x = 0; x < 4; ++x) d[x] += kv * s[r][x];
-    }
-    meet(d, 0);
-#pragma unroll
-    for (int x = 0; x < 4; ++x) u[x] = w * (v[x] - d[x]);
-  } else {
-#pragma unroll
-    for (int x = 0; x < 4; ++x) u[x] = v[x] * w;
-  }
-  float o[4] = {};
-#pragma unroll
-  for (int r = 0; r < NR; ++r) {
-    const int i = row + r * 32;
-    const float kv = ks[i] * ik, qv = qs[i];
-#pragma unroll
-    for (int x = 0; x < 4; ++x) {
-      s[r][x] += kv * u[x];
-      o[x] += qv * s[r][x];
-    }
     if (i < dim && col < vdim) {
       float* dst = sp + static_cast<size_t>(i) * vdim;
-      if (wide) {
+      if (wide_s) {
         *reinterpret_cast<float4*>(dst) = make_float4(s[r][0], s[r][1], s[r][2], s[r][3]);
       } else {
 #pragma unroll
@@ -788,47 +852,48 @@ scan_one_kernel(const ScanArgs a) {
       }
     }
   }
-  meet(o, 1);
-  const float skip = MODE == kSsd && a.d_skip ? a.d_skip[h] : 0.f;
-  if (warp == 0 && lane < 4) {
-#pragma unroll
-    for (int x = 0; x < 4; ++x)
-      if (col + x < vdim) a.out[(static_cast<size_t>(t) * a.heads + h) * vdim + col + x] = o[x] * iq + skip * v[x];
-  }
 }
 
 template <int DK, int MODE, bool CHAN, int WW>
-static void launch_scan_ww(const ScanArgs& a, int num_seqs, int* err, cudaStream_t st_) {
+static void launch_scan_ww(const ScanArgs& a, int z, int most, int* err, cudaStream_t st_) {
   using SM = ScanSmem<DK, CHAN, WW>;
   auto kern = scan_kernel<DK, MODE, CHAN, WW>;
   static OncePerDevice sized;
   if (!allow_smem(sized, kern, SM::kBytes)) return;
   const int cols = (a.vdim + SM::kCols - 1) / SM::kCols;
-  // a few blocks per SM, each taking every so many sequences (a step of decoded tokens is over at once)
-  const int z = std::max(1, std::min(num_seqs, 4 * sm_count() / (cols * a.heads)));
-  kern<<<dim3(cols, a.heads, z), WW * 32 + 256, SM::kBytes, st_>>>(a, num_seqs, err);
+  // a few blocks per SM, each taking every so many sequences
+  z = std::max(1, std::min(z, 4 * sm_count() / (cols * a.heads)));
+  kern<<<dim3(cols, a.heads, z), WW * 32 + 256, SM::kBytes, st_>>>(a, a.num_seqs, most, err);
   B200_CUDA_LAUNCH_CHECK();
 }
 template <int DK, int MODE, bool CHAN>
-static void launch_scan_dk(const ScanArgs& a, int num_seqs, cudaStream_t st_) {
+static void launch_scan_dk(const ScanArgs& a, int num_tokens, cudaStream_t st_) {
   int* err = wait_error_flag();
   if (!err) {
     set_error(2, "scan: no host-visible memory");
     return;
   }
-  scan_one_kernel<DK, MODE, CHAN><<<dim3((a.vdim + kOneCols - 1) / kOneCols, a.heads, num_seqs), 128, 0, st_>>>(a);
-  B200_CUDA_LAUNCH_CHECK();
   // 16 columns per block while that leaves a block per SM at most, 32 beyond: one sequence of 4096 tokens of 16 heads of
   // 128 x 128 (128 or 64 blocks) 634 and 883 us, four of 1000 (512 or 256 blocks) 655 and 539 us
-  if ((a.vdim + 15) / 16 * a.heads * num_seqs <= sm_count()) launch_scan_ww<DK, MODE, CHAN, 4>(a, num_seqs, err, st_);
-  else launch_scan_ww<DK, MODE, CHAN, 8>(a, num_seqs, err, st_);
+  const bool narrow = (a.vdim + 15) / 16 * a.heads * a.num_seqs <= sm_count();
+  // Token by token up to 16 tokens where the blocks of eight all run at once, up to 32 where they take turns on the SMs (they
+  // are one to an SM).  Delta rule, heads of 128 x 128, token by token and in blocks: one sequence of 17 tokens of 16 heads
+  // 11.8 and 10.2 us, two of 16 11.9 and about 10; two of 17 of 32 heads 17.4 and 20.5, four of 32 38 and 44, 32 of 17 148 and 214.
+  const int most = narrow || (a.vdim + 31) / 32 * a.heads * a.num_seqs <= sm_count() ? 16 : 32;
+  scan_short_kernel<DK, MODE, CHAN><<<dim3((a.vdim + kOneCols - 1) / kOneCols, a.heads, a.num_seqs), 128, 0, st_>>>(a, most);
+  B200_CUDA_LAUNCH_CHECK();
+  // sequences that can be longer than that: none in a step of few tokens, as of decoded ones
+  const int longer = num_tokens > 0 ? std::min(a.num_seqs, num_tokens / (most + 1)) : a.num_seqs;
+  if (longer == 0) return;
+  if (narrow) launch_scan_ww<DK, MODE, CHAN, 4>(a, longer, most, err, st_);
+  else launch_scan_ww<DK, MODE, CHAN, 8>(a, longer, most, err, st_);
 }
 // dim: rows of the state; at most 256 (the caller has checked)
 template <int MODE, bool CHAN>
-static void launch_scan(const ScanArgs& a, int num_seqs, cudaStream_t st_) {
-  if (a.dim <= 64) launch_scan_dk<64, MODE, CHAN>(a, num_seqs, st_);
-  else if (a.dim <= 128) launch_scan_dk<128, MODE, CHAN>(a, num_seqs, st_);
-  else launch_scan_dk<256, MODE, CHAN>(a, num_seqs, st_);
+static void launch_scan(const ScanArgs& a, int num_tokens, cudaStream_t st_) {
+  if (a.dim <= 64) launch_scan_dk<64, MODE, CHAN>(a, num_tokens, st_);
+  else if (a.dim <= 128) launch_scan_dk<128, MODE, CHAN>(a, num_tokens, st_);
+  else launch_scan_dk<256, MODE, CHAN>(a, num_tokens, st_);
 }
 
 // out[t, c] = sigmoid(z)^(1 / tau) with z = bias[c] + sum_r w2[c, r] * low[t, r]: the per-channel decay of gated linear
@@ -900,7 +965,7 @@ void launch_short_conv_silu(float* out, int ldo, const float* x, int ldx, const 
 void launch_delta_rule(float* out, const float* q, const float* k, const float* v, int ld, const float* b_raw,
                        const float* a_raw, int ld_ba, const float* a_log, const float* dt_bias, const float* chan_decay,
                        int ld_decay, float* state, const int32_t* slots, const uint32_t* cu, const uint32_t* ctx,
-                       int num_seqs, int heads, int kv_heads, int dim, int vdim, cudaStream_t st_) {
+                       int num_seqs, int heads, int kv_heads, int dim, int vdim, cudaStream_t st_, int num_tokens) {
   if (num_seqs <= 0) return;
   if (dim > 256) {
     set_error(1, "delta_rule: key dimension above 256 is not supported");
@@ -908,14 +973,14 @@ void launch_delta_rule(float* out, const float* q, const float* k, const float* 
   }
   const ScanArgs s{out, q, k, v, b_raw, a_raw, a_log, dt_bias, nullptr, nullptr, chan_decay, state, slots, cu, ctx, num_seqs,
                    ld, ld, ld, ld_ba, ld_decay, heads, kv_heads, dim, vdim, 0, 1.f, 1.f};
-  if (chan_decay) launch_scan<kDelta, true>(s, num_seqs, st_);
-  else launch_scan<kDelta, false>(s, num_seqs, st_);
+  if (chan_decay) launch_scan<kDelta, true>(s, num_tokens, st_);
+  else launch_scan<kDelta, false>(s, num_tokens, st_);
 }
 
 void launch_ssd_scan(float* out, const float* x, const float* Bm, const float* Cm, int ld, const float* dt_raw,
                      int ld_dt, const float* a_log, const float* dt_bias, const float* d_skip, float* state,
                      const int32_t* slots, const uint32_t* cu, const uint32_t* ctx, int num_seqs, int heads, int groups,
-                     int nstate, int vdim, cudaStream_t st_) {
+                     int nstate, int vdim, cudaStream_t st_, int num_tokens) {
   if (num_seqs <= 0) return;
   if (nstate > 256) {
     set_error(1, "ssd_scan: state size above 256 is not supported");
@@ -923,7 +988,7 @@ void launch_ssd_scan(float* out, const float* x, const float* Bm, const float* C
   }
   const ScanArgs s{out, Cm, Bm, x, nullptr, dt_raw, a_log, dt_bias, d_skip, nullptr, nullptr, state, slots, cu, ctx, num_seqs,
                    ld, ld, ld, ld_dt, 0, heads, groups, nstate, vdim, 0, 1.f, 1.f};
-  launch_scan<kSsd, false>(s, num_seqs, st_);
+  launch_scan<kSsd, false>(s, num_tokens, st_);
 }
 
 void launch_lowrank_decay(float* out, const float* low, int ld_low, const float* w2, const float* bias, float tau,
@@ -942,7 +1007,7 @@ void launch_lowrank_decay(float* out, const float* low, int ld_low, const float*
 void launch_decay_attn(float* out, const float* q, const float* k, const float* v, int ld, const float* head_decay,
                        const float* chan_decay, int ld_decay, float q_scale, float k_scale, int act, float* state,
                        const int32_t* slots, const uint32_t* cu, const uint32_t* ctx, int num_seqs, int heads, int dim,
-                       int vdim, cudaStream_t st_) {
+                       int vdim, cudaStream_t st_, int num_tokens) {
   if (num_seqs <= 0) return;
   if (dim > 256) {
     set_error(1, "decay_attn: key dimension above 256 is not supported");
@@ -950,8 +1015,8 @@ void launch_decay_attn(float* out, const float* q, const float* k, const float* 
   }
   const ScanArgs s{out, q, k, v, nullptr, nullptr, nullptr, nullptr, nullptr, head_decay, chan_decay, state, slots, cu, ctx,
                    num_seqs, ld, ld, ld, 0, ld_decay, heads, heads, dim, vdim, act, q_scale, k_scale};
-  if (chan_decay) launch_scan<kDecay, true>(s, num_seqs, st_);
-  else launch_scan<kDecay, false>(s, num_seqs, st_);
+  if (chan_decay) launch_scan<kDecay, true>(s, num_tokens, st_);
+  else launch_scan<kDecay, false>(s, num_tokens, st_);
 }
 
 void launch_scan_args(const b200_scan_args& a, int kind, cudaStream_t st_) {
@@ -960,11 +1025,11 @@ void launch_scan_args(const b200_scan_args& a, int kind, cudaStream_t st_) {
     set_error(1, "scan: key dimension (state size) above 256 is not supported");
     return;
   }
-  if (kind == kSsd) launch_scan<kSsd, false>(a, a.num_seqs, st_);
-  else if (kind == kDelta && a.chan_decay) launch_scan<kDelta, true>(a, a.num_seqs, st_);
-  else if (kind == kDelta) launch_scan<kDelta, false>(a, a.num_seqs, st_);
-  else if (a.chan_decay) launch_scan<kDecay, true>(a, a.num_seqs, st_);
-  else launch_scan<kDecay, false>(a, a.num_seqs, st_);
+  if (kind == kSsd) launch_scan<kSsd, false>(a, 0, st_);
+  else if (kind == kDelta && a.chan_decay) launch_scan<kDelta, true>(a, 0, st_);
+  else if (kind == kDelta) launch_scan<kDelta, false>(a, 0, st_);
+  else if (a.chan_decay) launch_scan<kDecay, true>(a, 0, st_);
+  else launch_scan<kDecay, false>(a, 0, st_);
 }
 
 }  // namespace b200

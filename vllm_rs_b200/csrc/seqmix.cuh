@@ -153,14 +153,15 @@ void launch_short_conv_silu(float* out, int ldo, const float* x, int ldx, const 
                             int num_rows, int C, int taps, cudaStream_t st);
 // chan_decay (may be NULL): ready-made decays per head and key channel [T, heads, dim] (row stride ld_decay); with it
 // a_raw, a_log and dt_bias are not used
+// (the scans' num_tokens: rows of the step, where they are known on the host; 0: they are not)
 void launch_delta_rule(float* out, const float* q, const float* k, const float* v, int ld, const float* b_raw,
                        const float* a_raw, int ld_ba, const float* a_log, const float* dt_bias, const float* chan_decay,
                        int ld_decay, float* state, const int32_t* slots, const uint32_t* cu, const uint32_t* ctx,
-                       int num_seqs, int heads, int kv_heads, int dim, int vdim, cudaStream_t st);
+                       int num_seqs, int heads, int kv_heads, int dim, int vdim, cudaStream_t st, int num_tokens = 0);
 void launch_ssd_scan(float* out, const float* x, const float* Bm, const float* Cm, int ld, const float* dt_raw,
                      int ld_dt, const float* a_log, const float* dt_bias, const float* d_skip, float* state,
                      const int32_t* slots, const uint32_t* cu, const uint32_t* ctx, int num_seqs, int heads, int groups,
-                     int nstate, int vdim, cudaStream_t st);
+                     int nstate, int vdim, cudaStream_t st, int num_tokens = 0);
 
 // a_log (may be NULL): the delta rule's decay exp(-exp(a_log[c / a_period]) softplus(z)) instead of sigmoid(z)^(1/tau)
 void launch_lowrank_decay(float* out, const float* low, int ld_low, const float* w2, const float* bias, float tau,
@@ -168,7 +169,7 @@ void launch_lowrank_decay(float* out, const float* low, int ld_low, const float*
 void launch_decay_attn(float* out, const float* q, const float* k, const float* v, int ld, const float* head_decay,
                        const float* chan_decay, int ld_decay, float q_scale, float k_scale, int act, float* state,
                        const int32_t* slots, const uint32_t* cu, const uint32_t* ctx, int num_seqs, int heads, int dim,
-                       int vdim, cudaStream_t st);
+                       int vdim, cudaStream_t st, int num_tokens = 0);
 
 // score 0 softmax, 1 sigmoid, 2 logits + bias with a softmax over the chosen ones; group_top: a group's score sums its 1 or
 // 2 best members; renorm: weights / (their sum + 1e-20)
