@@ -219,6 +219,7 @@ __global__ void __launch_bounds__(WW * 32 + 256, 1)
 scan_kernel(const ScanArgs a, int num_seqs, int most, int* err) {
   using SM = ScanSmem<DK, CHAN, WW>;
   constexpr int CH = DK / 32, COLS = SM::kCols;
+  constexpr bool BACK = MODE != kDelta || WW == 8;                     // rows of the triangles from the diagonal back (below)
   extern __shared__ __align__(16) float sm[];
   uint64_t* ready = reinterpret_cast<uint64_t*>(sm + SM::kBars);
   uint64_t* done = ready + kRing;
@@ -429,12 +430,13 @@ scan_kernel(const ScanArgs a, int num_seqs, int most, int* err) {
         }
         sync();
         // ---- P (t, j) = decayed q_t . k_j, j <= t, and (delta) M (t, j) = beta_t times the decayed k_t . k_j, j < t, then
-        // T = (1 + M)^-1.  A lane holds its rows of all eight tokens; the sums over the lanes go an entry to a lane.  Rows of P and
-        // T are stored from the diagonal back (entry d: token t - d; zero past the first), so that the walk reaches token t - d
-        // by a shuffle from d tokens below.  For tokens before the block that gives a lane's own part, never a later token's,
-        // which may be infinite or NaN and reach back through its zero.  (Two other ways to leave later tokens out: a branch,
-        // 617 -> 666 us for 4096 tokens of 16 heads of 128 x 128; source lanes in registers, 955 -> 1114 us for 32 heads with a
-        // decay per channel.)
+        // T = (1 + M)^-1.  A lane holds its rows of all eight tokens; the sums over the lanes go an entry to a lane.
+        // A walking lane must not meet a later token's part, which may be infinite or NaN and reach back through its zero of the
+        // triangle; in its place it takes its own.  BACK: rows are stored from the diagonal back (entry d: token t - d, zero past
+        // the first), and a shuffle from d tokens below gives a lane's own part where there is none.  Otherwise as they are, with
+        // the source lanes in registers, which eight walking warps do not have.  Delta rule, 4096 tokens of heads of 128 x 128:
+        // 16 heads 650 us with BACK, 590 without (a branch instead: 666); 32 heads, a decay per channel 907 - 965 and 1114.
+        // Decayed state, 8 heads of 128 x 256: 384 and 397.
         if (pw == 3) {
           if (i + 2 < nblk) make_scalars(i + 2);
         } else if (pw != 1 || MODE == kDelta) {
@@ -477,7 +479,7 @@ scan_kernel(const ScanArgs a, int num_seqs, int most, int* err) {
           float* out = B + SM::kMat + (pw == 1 ? 0 : kBT * kBT);
           if (et < et_end) {
             v *= B[SM::kRat + et * kBT + ej];
-            out[et * kBT + (pw == 1 ? ej : et - ej)] = pw == 1 ? v * G[kBT + et] : v;
+            out[et * kBT + (pw != 1 && BACK ? et - ej : ej)] = pw == 1 ? v * G[kBT + et] : v;
           }
           if (pw == 1) {                               // column `lane` of T by forward substitution
             __syncwarp();
@@ -494,7 +496,7 @@ scan_kernel(const ScanArgs a, int num_seqs, int most, int* err) {
             __syncwarp();
             if (lane < kBT) {
 #pragma unroll
-              for (int t = 0; t < kBT; ++t) out[t * kBT + ((t - lane) & (kBT - 1))] = tc[t];
+              for (int t = 0; t < kBT; ++t) out[t * kBT + (BACK ? (t - lane) & (kBT - 1) : lane)] = tc[t];
             }
           }
         }
@@ -557,6 +559,11 @@ scan_kernel(const ScanArgs a, int num_seqs, int most, int* err) {
       }
       float* us = sm + SM::kU + warp * kBT * 4;
       const int tt = lane >> 2, c4 = lane & 3;         // the token and column whose sums this lane gets
+      int from[kBT];
+#pragma unroll
+      for (int j = 0; j < kBT; ++j) from[j] = min(j, tt) * 4 + c4;
+      // what entry j of a row of the triangles is multiplied by
+      auto part = [&](float x, int j) { return BACK ? __shfl_up_sync(0xffffffffu, x, j * 4) : __shfl_sync(0xffffffffu, x, from[j]); };
       for (int i = 0; i < nblk; ++i) {
         const int g = blocks + i;
         mbar_wait_limited(&ready[g % kRing], (g / kRing) & 1, fail, err);
@@ -590,7 +597,7 @@ scan_kernel(const ScanArgs a, int num_seqs, int most, int* err) {
           const float T[kBT] = {ta.x, ta.y, ta.z, ta.w, tb.x, tb.y, tb.z, tb.w};
           u = 0.f;
 #pragma unroll
-          for (int d = 0; d < kBT; ++d) u += T[d] * __shfl_up_sync(0xffffffffu, r, d * 4);
+          for (int j = 0; j < kBT; ++j) u += T[j] * part(r, j);
         }
         us[lane] = CHAN ? u : u * G[3 * kBT + tt];
         __syncwarp();
@@ -601,7 +608,7 @@ scan_kernel(const ScanArgs a, int num_seqs, int most, int* err) {
           const float P[kBT] = {pa.x, pa.y, pa.z, pa.w, pb.x, pb.y, pb.z, pb.w};
           float o = gt * e;
 #pragma unroll
-          for (int d = 0; d < kBT; ++d) o += P[d] * __shfl_up_sync(0xffffffffu, u, d * 4);
+          for (int j = 0; j < kBT; ++j) o += P[j] * part(u, j);
           if (MODE == kDecay) o *= a.q_scale;
           if (MODE == kSsd) o += skip * vt;
           const int t = t0 + i * kBT + tt;
