@@ -140,3 +140,17 @@ def test_non_finite_tokens_stay_behind(lib, kind, bad):
             assert torch.equal(got[:t], want[:t]), (name, t)
             if name == "v" and bad != bad:
                 assert not torch.isfinite(got[t]).all()
+
+
+def test_operands_the_row_form_judges(lib):
+    """More value heads than query heads (the first ones count), and tensors whose sign is pending, take the row form."""
+    from vllm_rs_b200 import ops
+    T, H, d, e = 13, 2, 16, 8
+    g = torch.Generator().manual_seed(6)
+    r = lambda *s: torch.randn(*s, generator=g).cuda()                        # noqa: E731
+    q, k, v, state, hd = r(T, H, d), r(T, H, d), r(T, H + 2, e), r(1, H, d, e), torch.full((H,), 0.8, device="cuda")
+    tail = (_i32([0]), _i32([0, T]), _i32([T + 2]))
+    run = lambda q, k, v: ops.decay_attn(q, k, v, state.clone(), *tail, head_decay=hd)      # noqa: E731
+    want = run(q, k, v[:, :H])
+    assert torch.equal(run(q, k, v), want)
+    assert torch.equal(run(q, torch._neg_view(-k), v[:, :H]), want)

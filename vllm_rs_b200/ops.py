@@ -449,14 +449,16 @@ SCAN_DELTA, SCAN_DECAY, SCAN_SSD = 0, 1, 2
 def _scan(kind, q, k, v, state, state_slots, cu_seqlens_q, context_lens, *, strength=None, decay_raw=None, q_scale=1.0,
           k_scale=1.0, act=False, **params):
     """b200_scan on operands as they lie, one row stride each.  Laying them out as one row per token first (torch.cat) took
-    9 us of 675 for 4096 tokens of 16 heads of 128 x 128, and 12 us of host time of the 45 that a call of one token takes.  None for operands that are not
-    fp32 or whose shapes the concatenation has to judge: the callers then go that way."""
+    9 us of 675 for 4096 tokens of 16 heads of 128 x 128, and 12 us of host time of the 45 that a call of one token takes.
+    None for operands that are not plain fp32 or whose shapes the concatenation has to judge: the callers then go that way."""
     T, kv_heads, dim = q.shape
     heads, vdim = v.shape[1:]
     rows = (q, k, v, strength, decay_raw)
     for t, shape in zip(rows, (q.shape, q.shape, (T, heads, vdim), (T, heads), (T, heads))):
-        if t is not None and (t.dtype != torch.float32 or t.shape != shape or t.device != q.device):
+        if t is not None and (t.dtype != torch.float32 or t.shape != shape or t.device != q.device or t.is_neg()):
             return None
+    if kind == SCAN_DECAY and heads != kv_heads:             # (the row form takes the first value heads)
+        return None
     if T == 0 or kv_heads == 0 or heads % kv_heads or q.numel() == 0 or v.numel() == 0:
         return None
     q, k, v, strength, decay_raw = rows = [t if t is None else t.contiguous() for t in rows]
