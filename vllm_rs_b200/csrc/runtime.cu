@@ -48,7 +48,9 @@ int sm_count() {
   return cached;
 }
 
-static int* g_wait_host = nullptr;      // pinned; written by kernels through its device address
+// Pinned; written by kernels through its device address, on any stream and device.  Like every error of work that is still
+// running, a wait that gave up shows at the first question after it, which latches it for the whole process.
+static std::atomic<int*> g_wait_host{nullptr};
 int* wait_error_flag() {
   static std::once_flag once;
   static int* dev = nullptr;
@@ -60,8 +62,11 @@ int* wait_error_flag() {
     if (cudaHostAlloc(&h, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) == cudaSuccess &&
         cudaHostGetDevicePointer(&d, h, 0) == cudaSuccess) {
       *static_cast<volatile int*>(h) = 0;
-      g_wait_host = static_cast<int*>(h);
       dev = static_cast<int*>(d);
+      g_wait_host.store(static_cast<int*>(h), std::memory_order_release);
+    } else {
+      cudaFreeHost(h);
+      cudaGetLastError();
     }
     cudaThreadExchangeStreamCaptureMode(&mode);
   });
@@ -96,8 +101,9 @@ CUresult encode_tensor_map(CUtensorMap* map, CUtensorMapDataType dt, uint32_t ra
 
 extern "C" {
 int b200_last_error(void) {
-  if (b200::g_wait_host && *static_cast<volatile int*>(b200::g_wait_host)) {
-    *static_cast<volatile int*>(b200::g_wait_host) = 0;
+  int* gave_up = b200::g_wait_host.load(std::memory_order_acquire);
+  // one asking thread takes the word, so that it is neither told twice nor lost between a look and a reset
+  if (gave_up && *static_cast<volatile int*>(gave_up) && __atomic_exchange_n(gave_up, 0, __ATOMIC_ACQ_REL)) {
     b200::set_error(3, "a kernel gave up waiting for its data; the results of that launch are not valid");
   }
   std::lock_guard<std::mutex> lk(b200::g_err_mu);
