@@ -1,5 +1,6 @@
 """The tcgen05 grouped products of routed experts against 64-bit experts: buckets that are empty, hold one row, end inside a tile
-or take several; features and inner sizes that end inside a tile; every activation; identity experts; all three tile widths."""
+or take several; features and inner sizes that end inside a tile; every activation; identity experts; all three tile widths of
+both products (on 148 SMs 256 columns where that makes 296 tiles, 128 where it makes 111, else 64)."""
 import pytest
 import torch
 
@@ -9,7 +10,10 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("act", ["silu_gate", "relu2", "clamped"])
 @pytest.mark.parametrize("T,E,top,D,F,skew", [
     (1, 4, 2, 64, 32, 0), (37, 5, 3, 72, 40, 0), (3, 64, 1, 512, 8, 0), (300, 3, 2, 136, 264, 0), (700, 16, 4, 64, 520, 3),
-    (513, 2, 1, 264, 1032, 0), (2100, 20, 2, 96, 4100 // 8 * 8, 0), (129, 1, 1, 8, 16, 0)])
+    (513, 2, 1, 264, 1032, 0), (2100, 20, 2, 96, 4100 // 8 * 8, 0), (129, 1, 1, 8, 16, 0),
+    (350, 16, 2, 2056, 40, 0),             # second product: 16 row tiles x 17 of 128 columns, the last one 8 wide
+    (600, 20, 4, 4104, 72, 0),             # 20 x 17 of 256 columns, the last one 8 wide
+    (300, 16, 2, 72, 1032, 0)])            # first product without a gate: 16 x 9 of 128 columns
 def test_experts(lib, act, T, E, top, D, F, skew):
     from vllm_rs_b200 import ops
     g = torch.Generator().manual_seed(T * E + F)

@@ -240,3 +240,17 @@ def test_later_tokens_of_a_page_stay_out(lib, H, G, tile, bad):
         clean = t // tile * tile
         assert torch.equal(got[:clean], want[:clean]) and not torch.isfinite(got[t]).all()
         k[past + t], v[past + t] = kept
+
+
+@pytest.mark.parametrize("H,rank,rot,window,lens,ctxs", [
+    (128, 320, 32, 0, [170, 130], [170, 199]), (128, 512, 0, 70, [160, 150], [222, 150]), (64, 448, 64, 100, [300, 311], [300, 340])])
+def test_passes_of_one_block(lib, H, rank, rot, window, lens, ctxs):
+    """Two passes over the value columns in one block, equal and unequal: enough tiles (128 / heads tokens each) for two per SM."""
+    assert sum(-(-n // (128 // H)) for n in lens) + 1 > 2 * 148
+    test_latent_rows(lib, H, rank, rot, window, lens, ctxs)
+
+
+def test_several_maps_over_one_set_of_values_at_decode(lib):
+    """Key head g reads value head g % v_heads: maps that share the values, in the tensor-core form's sizes."""
+    for H, G, Gv in ((8, 4, 2), (12, 6, 1), (16, 8, 4)):
+        test_grouped_heads(lib, H, G, Gv, 64, 128, dict(window=90, sink=True), [1, 1, 1], [64, 129, 700])

@@ -1,6 +1,6 @@
 """The recurrent scans (gated delta rule, decayed linear attention, state-space scan) against the recurrence token by token in 64
-bits: sequences that end at, just before and just after a block of eight tokens and a staged pass of sixteen, single tokens
-on a kept state, sizes with padding, unaligned rows, decays near zero and one, several sequences at once."""
+bits: sequences that end at, just before and just after a block of eight tokens and the sixteen up to which they are walked token
+by token, single tokens on a kept state, sizes with padding, unaligned rows, decays near zero and one, several sequences at once."""
 import pytest
 import torch
 
@@ -69,6 +69,8 @@ def test_scans(lib, kind, H, G, d, e, lens):
                              **(dict(chan_decay=c(chan)) if act else dict(head_decay=c(hd))))
     want, want_state, at = torch.empty(T, H, e, dtype=D), state.double().clone(), 0
     for i, m in enumerate(lens):
+        if m == 0:                                                            # its state stays
+            continue
         sl, s = slice(at, at + m), int(slots[i])
         S0 = state[s].double() if past[i] else torch.zeros(H, d, e, dtype=D)
         want[sl], want_state[s] = _walk(Q[sl], K[sl], V[sl], dec[sl], w[sl], S0, corrected)
@@ -77,6 +79,24 @@ def test_scans(lib, kind, H, G, d, e, lens):
     # fp32 sums of up to d terms, thousands of them below 2^-24 of the largest entries each
     assert (got.double().cpu() - want).abs().max() <= 1e-5 * want.abs().max()
     assert (dev_state.double().cpu() - want_state).abs().max() <= 1e-5 * want_state.abs().max()
+
+
+# More column blocks x heads x sequences than the chip has SMs: 32 columns per block, and blocks that walk several sequences (16
+# heads of 128 x 128: 4 x 16 x 9 blocks for 24 sequences), odd and even numbers of blocks of eight tokens one after another.
+MANY = [17, 2, 24, 70, 1, 25, 0, 33, 40, 16, 9, 18]
+
+
+@pytest.mark.parametrize("e", [128, 40])
+@pytest.mark.parametrize("kind", ["delta", "delta_chan", "decay", "decay_chan", "ssd"])
+def test_many_sequences(lib, kind, e):
+    test_scans(lib, kind, 16, 8, 128, e, MANY + [m + 1 if m > 16 else m for m in MANY[::-1]])
+
+
+@pytest.mark.parametrize("H,G,d,e", [(2, 1, 128, 128), (3, 3, 20, 50), (1, 1, 200, 36)])
+@pytest.mark.parametrize("kind", ["delta", "delta_chan", "decay", "decay_chan", "ssd"])
+def test_ends_of_blocks(lib, kind, H, G, d, e):
+    test_scans(lib, kind, H, G, d, e, [23, 24, 25])
+    test_scans(lib, kind, H, G, d, e, [0, 6, 0, 31, 32])
 
 
 def test_operands_as_they_lie(lib):
