@@ -508,28 +508,31 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
           }
           big0 = max3(big0, fabsf(x[kTok - 2]), fabsf(x[kTok - 1]));
           mult = cap2;
-          auto near = [&](float& lo, float& hi) {              // two arguments up to kTanhMax
-            const f2 y = mul2(pack2(lo, hi), pack2(sl, sl)), t = mul2(y, y);
-            f2 q = fma2(t, pack2(kT5, kT5), pack2(kT4, kT4));
-            q = fma2(t, q, pack2(kT3, kT3));
-            q = fma2(t, q, pack2(kT2, kT2));
-            q = fma2(t, q, pack2(kT1, kT1));
-            q = mul2(y, fma2(t, q, pack2(kT0, kT0)));
-            asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(q));
-          };
           if (__all_sync(0xffffffffu, fmaxf(big0, big1) * sl <= kTanhMax)) {
 #pragma unroll
-            for (int i = 0; i < kTok; i += 2) near(x[i], x[i + 1]);
+            for (int i = 0; i < kTok; i += 2) {
+              const f2 y = mul2(pack2(x[i], x[i + 1]), pack2(sl, sl)), t = mul2(y, y);
+              f2 q = fma2(t, pack2(kT5, kT5), pack2(kT4, kT4));
+              q = fma2(t, q, pack2(kT3, kT3));
+              q = fma2(t, q, pack2(kT2, kT2));
+              q = fma2(t, q, pack2(kT1, kT1));
+              q = mul2(y, fma2(t, q, pack2(kT0, kT0)));
+              asm("mov.b64 {%0, %1}, %2;" : "=f"(x[i]), "=f"(x[i + 1]) : "l"(q));
+            }
           } else {
-            // tanh(y) = 1 - 2 / (e^(2 y) + 1) past kTanhMax.  Which form a score takes is its own affair: a row's bits do not
-            // depend on the rows and heads that share its warp.
+            // The same products one by one, and tanh(y) = 1 - 2 / (e^(2 y) + 1) past kTanhMax.  Which form a score takes is its
+            // own affair: a row's bits do not depend on the rows and heads that share its warp.  (The packed products here too,
+            // or a choice per row, made the path above slower: 101 and 107 instead of 99 us for a prompt of 4096.)
             const float e2 = sl * (2.f * kLog2e);
 #pragma unroll
-            for (int i = 0; i < kTok; i += 2) {
-              float a0 = x[i], a1 = x[i + 1];
-              near(a0, a1);
-              x[i] = fabsf(x[i]) * sl <= kTanhMax ? a0 : fmaf(-2.f, rcp(ex2(x[i] * e2) + 1.f), 1.f);
-              x[i + 1] = fabsf(x[i + 1]) * sl <= kTanhMax ? a1 : fmaf(-2.f, rcp(ex2(x[i + 1] * e2) + 1.f), 1.f);
+            for (int i = 0; i < kTok; ++i) {
+              const float y = __fmul_rn(x[i], sl), t = __fmul_rn(y, y);
+              float q = fmaf(t, kT5, kT4);
+              q = fmaf(t, q, kT3);
+              q = fmaf(t, q, kT2);
+              q = fmaf(t, q, kT1);
+              q = __fmul_rn(y, fmaf(t, q, kT0));
+              x[i] = fabsf(y) <= kTanhMax ? q : fmaf(-2.f, rcp(ex2(x[i] * e2) + 1.f), 1.f);
             }
           }
         }
