@@ -31,17 +31,31 @@ def test_row_norms(lib, n, dtype):
 @pytest.mark.parametrize("gate_first,act", [(True, "silu"), (False, "sigmoid")])
 @pytest.mark.parametrize("C,group,wn", [(24, 8, 8), (30, 6, 30), (256, 128, 128), (1024, 512, 1024), (2048, 2048, 2048),
                                         (4160, 1040, 0), (8192, 8192, 8192)])
-def test_gated_group_norm(lib, C, group, wn, gate_first, act, dtype):
+def test_gated_group_norm(lib, C, group, wn, gate_first, act, dtype, T=7):
     from vllm_rs_b200 import ops
     g = torch.Generator().manual_seed(C + group)
-    y, gate = torch.randn(7, C, generator=g), torch.randn(7, C, generator=g) * 2
+    y, gate = torch.randn(T, C, generator=g), torch.randn(T, C, generator=g) * 2
     w = torch.randn(wn, generator=g) if wn else None
     G, Y = gate.double(), y.double()
     s = torch.sigmoid(G) * (G if act == "silu" else 1.0)
-    u = (Y * s if gate_first else Y).reshape(7, -1, group)
-    want = (u / torch.sqrt((u * u).mean(-1, keepdim=True) + 1e-6)).reshape(7, C)
+    u = (Y * s if gate_first else Y).reshape(T, -1, group)
+    want = (u / torch.sqrt((u * u).mean(-1, keepdim=True) + 1e-6)).reshape(T, C)
     if w is not None:
         want = want * w.double().repeat(C // wn)
     want = want if gate_first else want * s
     got = ops.gated_group_norm(y.cuda(), gate.cuda(), None if w is None else w.cuda(), group, 1e-6, gate_first, dtype, act)
     _close(got, want, dtype)
+
+
+@pytest.mark.parametrize("C,group", [(1024, 256), (2048, 512), (1040, 260), (768, 192), (768, 384)])
+def test_gated_group_norm_of_few_and_many_groups(lib, C, group):
+    """Rows on both sides of the line between several warps per group and one, a last block that is not full; and the same bits."""
+    from vllm_rs_b200 import ops
+    many = 3 * torch.cuda.get_device_properties(0).multi_processor_count * group // 128
+    for T in (-(-many // (C // group)) - 1, -(-many // (C // group)) + 1):
+        test_gated_group_norm(lib, C, group, C, True, "silu", torch.float32, T)
+        test_gated_group_norm(lib, C, group, group, False, "sigmoid", torch.bfloat16, T)
+    y, gate, w = (torch.randn(n, C, device="cuda") for n in (many, many, 1))
+    for first in (True, False):
+        run = lambda n: ops.gated_group_norm(y[:n], gate[:n], w[0], group, 1e-6, first, torch.float32, "silu")      # noqa: E731
+        assert torch.equal(run(many)[:5], run(5))

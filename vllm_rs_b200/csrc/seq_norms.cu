@@ -162,6 +162,38 @@ gated_group_norm_vec_kernel(T* __restrict__ out, const float* __restrict__ y, in
     st4(out + static_cast<size_t>(t) * C + g0 + d, o);
   }
 }
+// The same with W = 2 or 4 warps per group, a vector per lane: where groups are few, W vectors in turn are what a group waits for.
+// The sums are those of the form with a warp per group and NV = W, to the bit.
+template <typename T, int W>
+__global__ void __launch_bounds__(256)
+gated_group_norm_split_kernel(T* __restrict__ out, const float* __restrict__ y, int ldy, const float* __restrict__ gate, int ldg,
+                              const float* __restrict__ w, int w_period, int C, int group, int units, float eps, int gate_first,
+                              int gate_act) {
+  __shared__ float part[8][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, first = warp / W * W;
+  const int unit = blockIdx.x * (8 / W) + warp / W, per = C / group, d = ((warp - first) * 32 + lane) * 4;
+  const bool live = unit < units && d < group;
+  const int t = live ? unit / per : 0, g0 = live ? (unit - t * per) * group : 0;
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f), s = v;
+  if (live) {
+    auto act = [&](float z) { return gate_act ? sigmoid_f(z) : silu_exact(z); };
+    v = ld4(y + static_cast<size_t>(t) * ldy + g0 + d);
+    const float4 g = ld4(gate + static_cast<size_t>(t) * ldg + g0 + d);
+    s = make_float4(act(g.x), act(g.y), act(g.z), act(g.w));
+    if (gate_first) v = make_float4(v.x * s.x, v.y * s.y, v.z * s.z, v.w * s.w);
+  }
+  part[warp][lane] = dot4(v);
+  __syncthreads();
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < W; ++i) ss += part[first + i][lane];
+  ss = lanes_sum(ss);
+  if (!live) return;
+  const float inv = 1.f / sqrtf(ss / static_cast<float>(group) + eps);
+  float4 o = scaled4(v, inv, w ? ld4(w + (g0 + d) % w_period) : make_float4(1.f, 1.f, 1.f, 1.f), 0.f);
+  if (!gate_first) o = make_float4(o.x * s.x, o.y * s.y, o.z * s.z, o.w * s.w);
+  st4(out + static_cast<size_t>(t) * C + g0 + d, o);
+}
 // grid = (runs of 1024 entries, rows)
 template <typename T>
 __global__ void __launch_bounds__(256)
@@ -607,9 +639,21 @@ void launch_gated_group_norm(void* out, const float* y, int ldy, const float* ga
       gated_group_norm_vec_kernel<TO, NT, NV><<<(units + 256 / NT - 1) / (256 / NT), 256, 0, st_>>>(
           o, y, ldy, gate, ldg, w, w_period, C, group, units, eps, gate_first, gate_act);
     };
-    const bool warp = group <= 512;                    // up to 16 entries per lane
+    // A warp per group up to 512 entries, which waits for no other warp, and where groups are few a warp per 128 entries of one.
+    // us for rows of 2048, by warps and split: 8 rows of groups of 256 SPLIT_A, 100 rows SPLIT_B, 300 rows SPLIT_C; groups of 512: 8
+    // rows SPLIT_D, 300 rows SPLIT_E, 1000 rows SPLIT_F.
+    const bool warp = group <= 512, split = warp && group > 128 && units < 3 * sm_count() * group / 128;
     auto pick = [&](auto nv) {
+      constexpr int NV = decltype(nv)::value;
       auto both = [&](auto* o) {
+        if constexpr (NV > 1) {
+          if (split) {
+            using TO = std::remove_pointer_t<decltype(o)>;
+            gated_group_norm_split_kernel<TO, NV><<<(units + 8 / NV - 1) / (8 / NV), 256, 0, st_>>>(
+                o, y, ldy, gate, ldg, w, w_period, C, group, units, eps, gate_first, gate_act);
+            return;
+          }
+        }
         if (warp) run(o, std::integral_constant<int, 32>{}, nv);
         else run(o, std::integral_constant<int, 256>{}, nv);
       };
