@@ -1,4 +1,4 @@
-"""The tcgen05 grouped products of routed experts against 64-bit experts: buckets that are empty, hold one row, end inside a tile
+"""The grouped products of routed experts, on tcgen05 and (short rows) on mma.sync, against 64-bit experts: buckets that are empty, hold one row, end inside a tile
 or take several; features and inner sizes that end inside a tile; every activation; identity experts; all three tile widths of
 both products (on 148 SMs 256 columns where that makes 296 tiles, 128 where it makes 111, else 64)."""
 import pytest
@@ -13,7 +13,10 @@ pytestmark = pytest.mark.gpu
     (513, 2, 1, 264, 1032, 0), (2100, 20, 2, 96, 4100 // 8 * 8, 0), (129, 1, 1, 8, 16, 0),
     (350, 16, 2, 2056, 40, 0),             # second product: 16 row tiles x 17 of 128 columns, the last one 8 wide
     (600, 20, 4, 4104, 72, 0),             # 20 x 17 of 256 columns, the last one 8 wide
-    (300, 16, 2, 72, 1032, 0)])            # first product without a gate: 16 x 9 of 128 columns
+    (300, 16, 2, 72, 1032, 0),             # 16 x 9 of 128 columns without a gate
+    # rows long enough for tcgen05 in both products, whatever their number
+    (1, 4, 2, 776, 264, 0), (37, 5, 3, 776, 264, 0), (3, 64, 1, 1032, 256, 0), (700, 16, 4, 776, 520, 3), (513, 2, 1, 840, 1032, 0),
+    (300, 16, 2, 776, 1032, 0), (2100, 20, 2, 776, 296, 0)])
 def test_experts(lib, act, T, E, top, D, F, skew):
     from vllm_rs_b200 import ops
     g = torch.Generator().manual_seed(T * E + F)
@@ -58,3 +61,21 @@ def test_experts(lib, act, T, E, top, D, F, skew):
     out = ops.moe_experts_ex(c(x), c(h), c(idx.int()), c(w), c(wu), c(wd), act=act, identity=ident, **kw)
     err = (out.double() - want).abs()
     assert bool((err <= 1.02 * tol + 1e-5 * want.abs().clamp(min=1.0)).all()), (err - tol).max().item()
+
+
+@pytest.mark.parametrize("act", ["silu_gate", "relu2"])
+@pytest.mark.parametrize("E,D,F", [(8, 512, 128), (4, 256, 256), (8, 128, 1024)])
+def test_same_bits_in_steps_of_any_size(lib, act, E, D, F):
+    """Steps of few rows take mma.sync for these sizes and steps of many tcgen05: a row's result does not tell which."""
+    from vllm_rs_b200 import ops
+    g = torch.Generator().manual_seed(D)
+    c = lambda t: t.cuda().contiguous()                                      # noqa: E731
+    wu = c((torch.randn(E, F if act == "relu2" else 2 * F, D, generator=g) / D ** 0.5).bfloat16())
+    wd = c((torch.randn(E, D, F, generator=g) / F ** 0.5).bfloat16())
+    T = 6000
+    h, z, x = c(torch.randn(T, D, generator=g).bfloat16()), torch.randn(T, E, generator=g), torch.zeros(T, D).cuda()
+    w, idx = torch.softmax(z, 1).topk(2, 1)
+    w, idx = c(w), c(idx.int())
+    run = lambda n: ops.moe_experts_ex(x[:n].clone(), h[:n], idx[:n], w[:n], wu, wd, act=act)      # noqa: E731
+    few, many = run(70), run(T)
+    assert torch.equal(few, many[:70])

@@ -504,6 +504,20 @@ static bool use_mma() {
   return v == 1;
 }
 
+// Whether the tcgen05 form is the faster one.  Its tiles are 128 rows and it gathers, starts and drains in 4 - 6 us more than the
+// mma.sync form takes for short rows, which the products have to win back (the gated activation takes longest, as few warps
+// have one tile's).  us for a whole call with mma.sync and with tcgen05 for the first product (second alike): 256 x 256, 2 of 8 gated:
+// 1 row 16 and 21, 2048 rows 26 and 27, 4096 rows 40 and 36; 512 x 512: 1 row 20.5 and 23, 2048 rows 51 and 36; 128 x 1024: 512
+// rows 25 and 30, 2048 rows 43 and 39; 768 x 256: 1 row 22.8 and 23.6, 512 rows 31 and 27; ungated 256 x 256: 1 row 14.4 and 14.9, 2048 rows
+// 23 and 22; 512 x 128: 17.5 and 16.2.  Second product: 2048 x 64 (64 wide rows), 1 row 38 and 39, 2048 rows 70 and 63; 256 x 256 16.5
+// and 15.9.  Both give the same bits.
+static bool tc_pays(int act, int pairs, int K, int N) {
+  const double work = static_cast<double>(pairs) * K * N;
+  if (act == 0) return K >= 256 || work > 1 << 27;
+  if (act == 2) return K >= 512 || work >= 1 << 28;
+  return K >= 768 || work >= 1 << 29;
+}
+
 template <int ACT>
 static void grouped_linear(void* out, const void* a, const void* w, const int32_t* off, const int32_t* pair_of_slot,
                            void* rows, int pairs, int top, int E, int K, int N, int dt, cudaStream_t st_,
@@ -513,7 +527,8 @@ static void grouped_linear(void* out, const void* a, const void* w, const int32_
   if (dt) {
     grouped_linear_fma_kernel<float, ACT><<<dim3(tiles, (N + TN - 1) / TN), 256, 0, st_>>>(
         out, (const float*)a, (const float*)w, off, pair_of_slot, top, E, K, N, act);
-  } else if (use_mma() && grouped_linear_tc(ACT, out, a, w, off, pair_of_slot, rows, pairs, top, E, K, N, act, st_)) {
+  } else if (use_mma() && tc_pays(ACT, pairs, K, N) &&
+             grouped_linear_tc(ACT, out, a, w, off, pair_of_slot, rows, pairs, top, E, K, N, act, st_)) {
     return;
   } else if (use_mma()) {
     grouped_linear_mma_kernel<ACT><<<dim3(tiles, (N + MN - 1) / MN), 128, 0, st_>>>(
