@@ -15,3 +15,20 @@ def test_tanh_fit():
     y = np.linspace(1e-6, top, 400001)
     err = np.abs(y * np.polynomial.polynomial.polyval(y * y, c) / np.tanh(y) - 1).max()
     assert 0.5 * said < err <= said
+
+
+def test_parts_never_grow_with_fewer_pages():
+    """The workspace of split keys is sized for the longest context; a rule restated from the source has to keep to it."""
+    src = (CSRC / "paged_attn_tc.cu").read_text()
+    body = src[src.index("int attn_tc_splits("):]
+    body = body[:body.index("\n}\n")]
+    assert "pages <= 4 && blocks > 64" in body and "pages <= 4 ? pages : std::max(4, (pages + 1) / 2), 16" in body
+
+    def parts(n, blocks, pages):
+        if pages <= 4 and blocks > 64:
+            return 1
+        return max(1, min(n, pages if pages <= 4 else max(4, (pages + 1) // 2), 16))
+    for n in range(1, 20):
+        for blocks in (1, 64, 65, 500):
+            got = [parts(n, blocks, p) for p in range(1, 70)]
+            assert got == sorted(got)

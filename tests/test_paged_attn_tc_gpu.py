@@ -254,3 +254,11 @@ def test_several_maps_over_one_set_of_values_at_decode(lib):
     """Key head g reads value head g % v_heads: maps that share the values, in the tensor-core form's sizes."""
     for H, G, Gv in ((8, 4, 2), (12, 6, 1), (16, 8, 4)):
         test_grouped_heads(lib, H, G, Gv, 64, 128, dict(window=90, sink=True), [1, 1, 1], [64, 129, 700])
+
+
+@pytest.mark.parametrize("lens,ctxs", [([1], [256]), ([1], [257]), ([1] * 20, [300] * 20), ([3, 1], [64, 1100])])
+def test_parts_of_a_few_pages(lib, lens, ctxs):
+    """Key splits of one and two pages per part, an odd page left over, and contexts shorter than the longest (empty parts)."""
+    test_grouped_heads(lib, 16, 4, 4, 64, 64, dict(sink=True, gate="head"), lens, ctxs)
+    test_grouped_heads(lib, 6, 2, 2, 96, 64, dict(window=200, keep=70, f32=True), lens, ctxs)
+    test_latent_rows(lib, 4, 64, 32, 0, lens, ctxs)

@@ -511,7 +511,7 @@ int latent_attn_splits(int T, int heads, int window) {
 }
 size_t latent_attn_workspace_bytes(int T, int heads, int kv_rank, int window) {
   const int n = std::max({latent_attn_splits(T, heads, window), latent_attn_mma_splits(T, heads, window),
-                          attn_few_rows(T) ? attn_tc_splits(T, 1, kv_rank, 1, window, 0) : 1});
+                          attn_few_rows(T) ? attn_tc_splits(T, 1, kv_rank, 1, window, 0, 0) : 1});
   return n == 1 ? 0 : static_cast<size_t>(T) * heads * n * (kv_rank + 2) * 4;
 }
 
@@ -523,7 +523,7 @@ void launch_latent_attn(void* out, const float* q_full, const void* cache, const
   // bf16: the tcgen05 form takes ranks that are multiples of 64 (rows: of 32) and up to 128 heads, among the sizes that have a
   // tensor-core form at all: ranks past 512 keep their queries and weights in fp32, in the FMA form.
   if (!dt && latent_mma_enabled() && latent_mma_shape_ok(kv_rank, rot_dim)) {
-    const int nsplit = attn_few_rows(T) && workspace ? attn_tc_splits(T, 1, kv_rank, 1, window, 0) : 1;
+    const int nsplit = attn_few_rows(T) && workspace ? attn_tc_splits(T, 1, kv_rank, 1, window, 0, max_blocks) : 1;
     float* po = reinterpret_cast<float*>(workspace);
     const AttnTcProblem p{out, q_full, cache, nullptr, sink, gate, ld_gate, 0, cu, ctx, block_tables, max_blocks, num_seqs, T,
                           heads, 1, 1, kv_rank + rot_dim, kv_rank, window, 0, 0, scale, 0.f, nullptr, nullptr, 0, 0, nsplit,

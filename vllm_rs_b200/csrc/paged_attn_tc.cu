@@ -729,13 +729,20 @@ bool attn_tc_takes(const AttnTcProblem& p) {
   return (ptrs & 15) == 0 && p.scale > 0.f && hat::plan(p, a);
 }
 
-int attn_tc_splits(int T, int kv_heads, int vdim, int shared_kv, int window, int keep_first) {
+int attn_tc_splits(int T, int kv_heads, int vdim, int shared_kv, int window, int keep_first, int max_blocks) {
   // every row is a tile of its own (one token per sequence), or a few of one sequence share one; a block per pass
   const int passes = shared_kv ? (vdim + 255) / 256 : 1;
   const int blocks = T * kv_heads * passes;
   int n = ((shared_kv ? 1 : 2) * sm_count()) / std::max(1, blocks);
-  if (window > 0) n = std::min(n, (window + std::max(keep_first, 0) + hat::kTok - 1) / hat::kTok + 1);
-  return std::max(1, std::min(n, 16));
+  int pages = max_blocks > 0 ? max_blocks : 1 << 20;
+  if (window > 0) pages = std::min(pages, (window + std::max(keep_first, 0) + hat::kTok - 1) / hat::kTok + 1);
+  // A part that holds no page still costs its block and its place in the merge (one row on 30 keys, 16 parts 12 us, one 9 us), and the
+  // merge costs more than a few pages in turn once there are many rows: up to four pages make one part, or, in small steps, one
+  // each, more pages two each.  us for one row on 700 keys, 16 heads of 64 with 16 parts of one page 16.8, with 6 of two pages 12.8;
+  // 32 rows on a window of 100, 12 heads of 128 x 192: two parts 22.8, one 14.3; one row on 200 keys, 16 heads over 4: one part 13.9, four 12.4.
+  // Never more parts for fewer pages: the workspace is sized without knowing max_blocks.
+  if (pages <= 4 && blocks > 64) return 1;
+  return std::max(1, std::min({n, pages <= 4 ? pages : std::max(4, (pages + 1) / 2), 16}));
 }
 
 void launch_attn_tc(const AttnTcProblem& p, cudaStream_t st) {

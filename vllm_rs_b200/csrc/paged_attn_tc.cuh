@@ -29,8 +29,9 @@ struct AttnTcProblem {
 inline bool attn_few_rows(int T) { return T <= 2 * sm_count() / 4; }
 // whether these sizes and pointers are taken (bf16 caches only)
 bool attn_tc_takes(const AttnTcProblem& p);
-// key splits that fill the chip for a step of T rows of which every sequence brings few (1: no split)
-int attn_tc_splits(int T, int kv_heads, int vdim, int shared_kv, int window, int keep_first);
+// key splits that fill the chip for a step of T rows of which every sequence brings few (1: no split); max_blocks: pages of the
+// longest context, 0 where that is not known
+int attn_tc_splits(int T, int kv_heads, int vdim, int shared_kv, int window, int keep_first, int max_blocks);
 void launch_attn_tc(const AttnTcProblem& p, cudaStream_t st);
 
 }  // namespace b200

@@ -918,7 +918,7 @@ size_t window_attn_workspace_bytes(int T, int heads, int kv_heads, int vdim, int
   if (v_heads <= 0 || kv_heads % v_heads != 0) v_heads = kv_heads;
   const int n = std::max({window_attn_splits(T, heads, kv_heads, window, keep_first),
                           window_attn_mma_splits(T, heads, kv_heads, window, keep_first, v_heads),
-                          attn_few_rows(T) ? attn_tc_splits(T, kv_heads, vdim, 0, window, keep_first) : 1});
+                          attn_few_rows(T) ? attn_tc_splits(T, kv_heads, vdim, 0, window, keep_first, 0) : 1});
   return n == 1 ? 0 : static_cast<size_t>(T) * heads * n * (vdim + 2) * 4;
 }
 
@@ -948,7 +948,7 @@ void launch_window_attn(void* out, const float* q, const void* k_cache, const vo
   const bool hrows = attn_few_rows(T);
   const bool tensor = !dt && window_mma_enabled() && window_mma_shape_ok(dim, vdim, hrows ? kv_heads / v_heads : 1);
   if (tensor) {
-    const int nsplit = hrows && workspace ? attn_tc_splits(T, kv_heads, vdim, 0, window, keep_first) : 1;
+    const int nsplit = hrows && workspace ? attn_tc_splits(T, kv_heads, vdim, 0, window, keep_first, max_blocks) : 1;
     float* po = reinterpret_cast<float*>(workspace);
     const AttnTcProblem p{out, q, k_cache, v_cache, sink, gate, ld_gate, gate_elems, cu, ctx, block_tables, max_blocks, num_seqs,
                           T, heads, kv_heads, v_heads, dim, vdim, window, keep_first, chunk, scale, softcap, slopes, dist_bias,
