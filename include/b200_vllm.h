@@ -874,6 +874,8 @@ typedef struct b200_scan_args {
   float q_scale, k_scale;
 } b200_scan_args;
 void b200_scan(const b200_scan_args* args, int32_t kind, int64_t stream);
+/* The same where the rows of the step are known: steps of few rows need one launch less.                                  */
+void b200_scan_rows(const b200_scan_args* args, int32_t kind, int32_t num_tokens, int64_t stream);
 /* Linear attention with a decayed state: S <- diag(a_t) S + (k_scale k_t) v_t^T, o_t = S^T (q_scale q_t).  q, k fp32
  * [T, heads, dim], v [T, heads, vdim] (row stride ld); exactly one of head_decay fp32 [heads] (a constant per head)
  * and chan_decay fp32 [T, heads, dim] (row stride ld_decay); act != 0: SiLU on q, k and v first; out fp32

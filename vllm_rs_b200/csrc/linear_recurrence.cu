@@ -790,6 +790,7 @@ scan_short_kernel(const ScanArgs a, int most) {
       __syncthreads();
     } else if (MODE == kDecay && a.act) {
       for (int e = tid; e < m * DK; e += 128) {
+        if (e % DK >= dim) continue;
         ks[e / DK][e % DK] = silu_exact(ks[e / DK][e % DK]);
         qs[e / DK][e % DK] = silu_exact(qs[e / DK][e % DK]);
       }
@@ -886,8 +887,11 @@ static void launch_scan_dk(const ScanArgs& a, int num_tokens, cudaStream_t st_) 
   // Token by token up to 16 tokens where the blocks of eight all run at once, up to 32 where they take turns on the SMs (they
   // are one to an SM).  Delta rule, heads of 128 x 128, token by token and in blocks: one sequence of 17 tokens of 16 heads
   // 11.8 and 10.2 us, two of 16 11.9 and about 10; two of 17 of 32 heads 17.4 and 20.5, four of 32 38 and 44, 32 of 17 148 and 214.
-  const int most = narrow || (a.vdim + 31) / 32 * a.heads * a.num_seqs <= sm_count() ? 16 : 32;
-  scan_short_kernel<DK, MODE, CHAN><<<dim3((a.vdim + kOneCols - 1) / kOneCols, a.heads, a.num_seqs), 128, 0, st_>>>(a, most);
+  // An activation makes a block of eight wait longer for its rows (20 tokens of 4 heads of 16 x 16: 9.4 us, token by token 7).
+  const bool at_once = narrow || (a.vdim + 31) / 32 * a.heads * a.num_seqs <= sm_count();
+  const int most = at_once && !(MODE == kDecay && a.act) ? 16 : 32;
+  auto brief = DK == 64 && a.dim <= 32 ? scan_short_kernel<DK == 64 ? 32 : DK, MODE, CHAN> : scan_short_kernel<DK, MODE, CHAN>;
+  brief<<<dim3((a.vdim + kOneCols - 1) / kOneCols, a.heads, a.num_seqs), 128, 0, st_>>>(a, most);
   B200_CUDA_LAUNCH_CHECK();
   // sequences that can be longer than that: none in a step of few tokens, as of decoded ones
   const int longer = num_tokens > 0 ? std::min(a.num_seqs, num_tokens / (most + 1)) : a.num_seqs;
@@ -1026,23 +1030,24 @@ void launch_decay_attn(float* out, const float* q, const float* k, const float* 
   else launch_scan<kDecay, false>(s, num_tokens, st_);
 }
 
-void launch_scan_args(const b200_scan_args& a, int kind, cudaStream_t st_) {
+void launch_scan_args(const b200_scan_args& a, int kind, int num_tokens, cudaStream_t st_) {
   if (a.num_seqs <= 0) return;
   if (a.dim > 256) {
     set_error(1, "scan: key dimension (state size) above 256 is not supported");
     return;
   }
-  if (kind == kSsd) launch_scan<kSsd, false>(a, 0, st_);
-  else if (kind == kDelta && a.chan_decay) launch_scan<kDelta, true>(a, 0, st_);
-  else if (kind == kDelta) launch_scan<kDelta, false>(a, 0, st_);
-  else if (a.chan_decay) launch_scan<kDecay, true>(a, 0, st_);
-  else launch_scan<kDecay, false>(a, 0, st_);
+  if (kind == kSsd) launch_scan<kSsd, false>(a, num_tokens, st_);
+  else if (kind == kDelta && a.chan_decay) launch_scan<kDelta, true>(a, num_tokens, st_);
+  else if (kind == kDelta) launch_scan<kDelta, false>(a, num_tokens, st_);
+  else if (a.chan_decay) launch_scan<kDecay, true>(a, num_tokens, st_);
+  else launch_scan<kDecay, false>(a, num_tokens, st_);
 }
 
 }  // namespace b200
 
 extern "C" {
-void b200_scan(const b200_scan_args* a, int32_t kind, int64_t stream) {
+void b200_scan(const b200_scan_args* a, int32_t kind, int64_t stream) { b200_scan_rows(a, kind, 0, stream); }
+void b200_scan_rows(const b200_scan_args* a, int32_t kind, int32_t num_tokens, int64_t stream) {
   B200_CHECK_ARG(a && a->out && a->q && a->k && a->v && a->state && a->state_slots && a->cu_seqlens_q && a->context_lens &&
                      a->heads > 0 && a->kv_heads > 0 && a->heads % a->kv_heads == 0 && a->dim > 0 && a->vdim > 0 &&
                      kind >= b200::kDelta && kind <= b200::kSsd &&
@@ -1050,7 +1055,7 @@ void b200_scan(const b200_scan_args* a, int32_t kind, int64_t stream) {
                       : kind == b200::kSsd ? a->decay_raw && a->a_log && a->dt_bias
                                            : a->strength && (a->chan_decay || (a->decay_raw && a->a_log && a->dt_bias))),
                  "scan: bad arguments");
-  b200::launch_scan_args(*a, kind, reinterpret_cast<cudaStream_t>(stream));
+  b200::launch_scan_args(*a, kind, num_tokens, reinterpret_cast<cudaStream_t>(stream));
 }
 void b200_short_conv_silu(float* out, int32_t ldo, const float* x, int32_t ldx, const float* taps_w, const float* bias,
                           float* state, const int32_t* state_slots, const uint32_t* cu_seqlens_q,

@@ -448,7 +448,7 @@ SCAN_DELTA, SCAN_DECAY, SCAN_SSD = 0, 1, 2
 
 def _scan(kind, q, k, v, state, state_slots, cu_seqlens_q, context_lens, *, strength=None, decay_raw=None, q_scale=1.0,
           k_scale=1.0, act=False, **params):
-    """b200_scan on operands as they lie, one row stride each.  Laying them out as one row per token first (torch.cat) took
+    """b200_scan_rows on operands as they lie, one row stride each.  Laying them out as one row per token first (torch.cat) took
     9 us of 675 for 4096 tokens of 16 heads of 128 x 128, and 12 us of host time of the 45 that a call of one token takes.
     None for operands that are not plain fp32 or whose shapes the concatenation has to judge: the callers then go that way."""
     T, kv_heads, dim = q.shape
@@ -470,7 +470,7 @@ def _scan(kind, q, k, v, state, state_slots, cu_seqlens_q, context_lens, *, stre
                       ld_decay=heads * dim, heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim,
                       act=int(bool(act)), q_scale=float(q_scale), k_scale=float(k_scale),
                       **{n: _p(t) for n, t in params.items()})
-    _lib.lib().b200_scan(C.byref(a), kind, _stream())
+    _lib.lib().b200_scan_rows(C.byref(a), kind, T, _stream())
     _lib.check()
     return out
 
