@@ -174,3 +174,35 @@ def test_operands_the_row_form_judges(lib):
     want = run(q, k, v[:, :H])
     assert torch.equal(run(q, k, v), want)
     assert torch.equal(run(q, torch._neg_view(-k), v[:, :H]), want)
+
+
+@pytest.mark.parametrize("kind", ["delta", "delta_chan", "decay", "ssd"])
+def test_bits_do_not_tell_the_company(lib, kind):
+    """A sequence alone (16 columns per block, its own launch) and among others (32 columns, blocks that walk several)."""
+    from vllm_rs_b200 import ops
+    H, d, e = 8, 128, 128
+    lens = [40, 5, 1, 17, 70, 16, 33, 2, 24, 90]
+    T, n = sum(lens), len(lens)
+    g = torch.Generator().manual_seed(4)
+    r = lambda *s: torch.randn(*s, generator=g).cuda()                        # noqa: E731
+    q, k, v, b, a, dec = r(T, H, d), r(T, H, d), r(T, H, e), r(T, H), r(T, H), torch.sigmoid(r(T, H, d) + 2)
+    alog, dtb, dsk, state = r(H) * 0.5, r(H), r(H), r(n, H, d, e)
+
+    def run(rows, slots, ns):
+        s, tail = state.clone(), (_i32(slots), _i32([0] + [sum(ns[:i + 1]) for i in range(len(ns))]), _i32([m + 3 for m in ns]))
+        x = [t[rows].contiguous() for t in (q, k, v, b, a, dec)]
+        if kind == "delta":
+            o = ops.delta_rule(x[0], x[1], x[2], x[3], x[4], alog, dtb, s, *tail)
+        elif kind == "delta_chan":
+            o = ops.delta_rule_chan(x[0], x[1], x[2], x[3], x[5], s, *tail)
+        elif kind == "ssd":
+            o = ops.ssd_scan(x[2], x[1], x[0], x[4], alog, dtb, dsk, s, *tail)
+        else:
+            o = ops.decay_attn(x[0], x[1], x[2], s, *tail, head_decay=torch.full((H,), 0.9, device="cuda"), act=True)
+        return o, s
+    out, after = run(slice(0, T), list(range(n)), lens)
+    at = 0
+    for i, m in enumerate(lens):
+        o, s = run(slice(at, at + m), [i], [m])
+        assert torch.equal(o, out[at:at + m]) and torch.equal(s[i], after[i]), (i, m)
+        at += m

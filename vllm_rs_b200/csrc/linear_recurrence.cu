@@ -141,6 +141,7 @@ __device__ __forceinline__ void unpack2(f2 v, float& lo, float& hi) { asm("mov.b
 constexpr int kOneCols = 16;                   // columns of S per block of threads: single tokens
 constexpr int kBT = 8;                         // tokens per block of the recurrence
 constexpr int kRing = 8;                       // blocks of tokens in shared memory (with four, fetching waited for the walk)
+constexpr int kShort = 16;                     // tokens of a sequence up to which it is walked token by token
 constexpr int kDelta = 0, kDecay = 1, kSsd = 2;
 
 using ScanArgs = b200_scan_args;
@@ -202,7 +203,7 @@ __device__ __forceinline__ float meet32(float (&x)[32], int lane) {
   return x[0];
 }
 
-// Portions of more than `most` tokens.  grid = (column blocks, heads, runs of sequences); a block walks its sequences one after
+// Portions of more than kShort tokens.  grid = (column blocks, heads, runs of sequences); a block walks its sequences one after
 // another.  The first WW warps each own four columns of S: a lane holds DK / 32 neighbouring rows of them in registers, so that
 // a key or query row is read once from shared memory for four columns (one column per lane made these reads the bound: 512
 // bytes of registers per load and warp).  Two groups of four warps take turns at fetching a block's token rows (cp.async, a
@@ -216,7 +217,7 @@ __device__ __forceinline__ float meet32(float (&x)[32], int lane) {
 // us with both in turn).
 template <int DK, int MODE, bool CHAN, int WW>
 __global__ void __launch_bounds__(WW * 32 + 256, 1)
-scan_kernel(const ScanArgs a, int num_seqs, int most, int* err) {
+scan_kernel(const ScanArgs a, int num_seqs, int* err) {
   using SM = ScanSmem<DK, CHAN, WW>;
   constexpr int CH = DK / 32, COLS = SM::kCols;
   constexpr bool BACK = MODE != kDelta || WW == 8;                     // rows of the triangles from the diagonal back (below)
@@ -230,7 +231,7 @@ scan_kernel(const ScanArgs a, int num_seqs, int most, int* err) {
   {
     int mine = 0;                                                      // a sequence for this kernel among the block's
     for (int b = blockIdx.z + tid * gridDim.z; b < num_seqs; b += kAll * gridDim.z)
-      mine |= static_cast<int>(a.cu_seqlens_q[b + 1] - a.cu_seqlens_q[b]) > most;
+      mine |= static_cast<int>(a.cu_seqlens_q[b + 1] - a.cu_seqlens_q[b]) > kShort;
     if (!__syncthreads_or(mine)) return;
   }
   if (tid == 0) {
@@ -248,7 +249,7 @@ scan_kernel(const ScanArgs a, int num_seqs, int most, int* err) {
   int blocks = 0;                                                      // blocks of tokens so far, over all sequences
   for (int b = blockIdx.z; b < num_seqs; b += gridDim.z) {
     const int t0 = a.cu_seqlens_q[b], t1 = a.cu_seqlens_q[b + 1], nblk = (t1 - t0 + kBT - 1) / kBT;
-    if (t1 - t0 <= most) continue;                                     // (scan_short_kernel)
+    if (t1 - t0 <= kShort) continue;                                   // (scan_short_kernel)
     const bool fresh = static_cast<int>(a.context_lens[b]) == t1 - t0;
     if (warp >= WW) {
       // ---------------------------------------------------------- token rows
@@ -562,7 +563,8 @@ scan_kernel(const ScanArgs a, int num_seqs, int most, int* err) {
       int from[kBT];
 #pragma unroll
       for (int j = 0; j < kBT; ++j) from[j] = min(j, tt) * 4 + c4;
-      // what entry j of a row of the triangles is multiplied by
+      // what entry j of a row of the triangles is multiplied by; from this token back in both forms, so that their bits are equal
+      auto entry = [](int i) { return BACK ? i : kBT - 1 - i; };
       auto part = [&](float x, int j) { return BACK ? __shfl_up_sync(0xffffffffu, x, j * 4) : __shfl_sync(0xffffffffu, x, from[j]); };
       for (int i = 0; i < nblk; ++i) {
         const int g = blocks + i;
@@ -592,12 +594,12 @@ scan_kernel(const ScanArgs a, int num_seqs, int most, int* err) {
         if (MODE == kDelta) {
           float xk[32];
           dots(xk, B);
-          const float r = wt * (vt - gt * meet32(xk, lane));
+          const float r = wt * fmaf(-gt, meet32(xk, lane), vt);
           const float4 ta = *reinterpret_cast<const float4*>(B + SM::kMat + tt * kBT), tb = *reinterpret_cast<const float4*>(B + SM::kMat + tt * kBT + 4);
           const float T[kBT] = {ta.x, ta.y, ta.z, ta.w, tb.x, tb.y, tb.z, tb.w};
           u = 0.f;
 #pragma unroll
-          for (int j = 0; j < kBT; ++j) u += T[j] * part(r, j);
+          for (int z = 0; z < kBT; ++z) u = fmaf(T[entry(z)], part(r, entry(z)), u);
         }
         us[lane] = CHAN ? u : u * G[3 * kBT + tt];
         __syncwarp();
@@ -606,9 +608,9 @@ scan_kernel(const ScanArgs a, int num_seqs, int most, int* err) {
           const float4 pa = *reinterpret_cast<const float4*>(B + SM::kMat + kBT * kBT + tt * kBT);
           const float4 pb = *reinterpret_cast<const float4*>(B + SM::kMat + kBT * kBT + tt * kBT + 4);
           const float P[kBT] = {pa.x, pa.y, pa.z, pa.w, pb.x, pb.y, pb.z, pb.w};
-          float o = gt * e;
+          float o = __fmul_rn(gt, e);
 #pragma unroll
-          for (int j = 0; j < kBT; ++j) o += P[j] * part(u, j);
+          for (int z = 0; z < kBT; ++z) o = fmaf(P[entry(z)], part(u, entry(z)), o);
           if (MODE == kDecay) o *= a.q_scale;
           if (MODE == kSsd) o += skip * vt;
           const int t = t0 + i * kBT + tt;
@@ -671,20 +673,20 @@ scan_kernel(const ScanArgs a, int num_seqs, int most, int* err) {
   }
 }
 
-// Portions of up to `most` tokens, token by token.  grid = (column blocks, heads, sequences); 128 threads = 32 rows x 4 columns of
+// Portions of up to kShort tokens, token by token.  grid = (column blocks, heads, sequences); 128 threads = 32 rows x 4 columns of
 // 4.  16 columns per block, so that a single sequence of 16 heads of 128 still makes 128 blocks, and small blocks, of which an
 // SM holds many.  Single tokens are bound by the state's way in and out, which are whole 64-byte rows here, more tokens by
 // instructions and, for the delta rule, a barrier per token; their rows are staged and normed together, CT tokens at a time.
 template <int DK, int MODE, bool CHAN>
-__global__ void __launch_bounds__(128, DK <= 128 ? 8 : 5)
-scan_short_kernel(const ScanArgs a, int most) {
+__global__ void __launch_bounds__(128)
+scan_short_kernel(const ScanArgs a) {
   constexpr int NR = DK / 32, CT = DK * (CHAN ? 2 : 1) <= 128 ? 16 : 8;
   __shared__ __align__(16) float ks[CT][DK], qs[CT][DK], ds[CHAN ? CT : 1][CHAN ? DK : 4], vs[CT][kOneCols];
   __shared__ __align__(16) float red[2][4][kOneCols], sums[CT][4][kOneCols];
   __shared__ float sc[CT][3];                          // decay, write strength, what the read-out is multiplied by
   const int h = blockIdx.y, b = blockIdx.z, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, col0 = blockIdx.x * kOneCols;
   const int t0 = a.cu_seqlens_q[b], n = static_cast<int>(a.cu_seqlens_q[b + 1]) - t0;
-  if (n < 1 || n > most) return;
+  if (n < 1 || n > kShort) return;
   const bool fresh = static_cast<int>(a.context_lens[b]) == n;
   const int dim = a.dim, vdim = a.vdim, hk = MODE == kDecay ? h : h / (a.heads / a.kv_heads);
   const int c = (tid & 3) * 4, col = col0 + c, row = tid >> 2;
@@ -863,7 +865,7 @@ scan_short_kernel(const ScanArgs a, int most) {
 }
 
 template <int DK, int MODE, bool CHAN, int WW>
-static void launch_scan_ww(const ScanArgs& a, int z, int most, int* err, cudaStream_t st_) {
+static void launch_scan_ww(const ScanArgs& a, int z, int* err, cudaStream_t st_) {
   using SM = ScanSmem<DK, CHAN, WW>;
   auto kern = scan_kernel<DK, MODE, CHAN, WW>;
   static OncePerDevice sized;
@@ -871,7 +873,7 @@ static void launch_scan_ww(const ScanArgs& a, int z, int most, int* err, cudaStr
   const int cols = (a.vdim + SM::kCols - 1) / SM::kCols;
   // a few blocks per SM, each taking every so many sequences
   z = std::max(1, std::min(z, 4 * sm_count() / (cols * a.heads)));
-  kern<<<dim3(cols, a.heads, z), WW * 32 + 256, SM::kBytes, st_>>>(a, a.num_seqs, most, err);
+  kern<<<dim3(cols, a.heads, z), WW * 32 + 256, SM::kBytes, st_>>>(a, a.num_seqs, err);
   B200_CUDA_LAUNCH_CHECK();
 }
 template <int DK, int MODE, bool CHAN>
@@ -884,20 +886,18 @@ static void launch_scan_dk(const ScanArgs& a, int num_tokens, cudaStream_t st_) 
   // 16 columns per block while that leaves a block per SM at most, 32 beyond: one sequence of 4096 tokens of 16 heads of
   // 128 x 128 (128 or 64 blocks) 634 and 883 us, four of 1000 (512 or 256 blocks) 655 and 539 us
   const bool narrow = (a.vdim + 15) / 16 * a.heads * a.num_seqs <= sm_count();
-  // Token by token up to 16 tokens where the blocks of eight all run at once, up to 32 where they take turns on the SMs (they
-  // are one to an SM).  Delta rule, heads of 128 x 128, token by token and in blocks: one sequence of 17 tokens of 16 heads
-  // 11.8 and 10.2 us, two of 16 11.9 and about 10; two of 17 of 32 heads 17.4 and 20.5, four of 32 38 and 44, 32 of 17 148 and 214.
-  // An activation makes a block of eight wait longer for its rows (20 tokens of 4 heads of 16 x 16: 9.4 us, token by token 7).
-  const bool at_once = narrow || (a.vdim + 31) / 32 * a.heads * a.num_seqs <= sm_count();
-  const int most = at_once && !(MODE == kDecay && a.act) ? 16 : 32;
+  // Which kernel walks a sequence is a matter of its own length, so that its bits do not depend on the step's other sequences.  Up to
+  // kShort tokens, whatever their number, token by token is as fast or faster.  Delta rule, heads of 128 x 128, token by token and
+  // in blocks: 1 sequence of 16 tokens of 16 heads 9.2 and 9.4 us, 2 10.8 and 10.1, 8 22 and 31, 32 of 12 tokens 51 and 78; of 20
+  // tokens 1 sequence 11.5 and 10.5, 4 18.6 and 20.8.  In a step with longer sequences its walk stands before theirs.
   auto brief = DK == 64 && a.dim <= 32 ? scan_short_kernel<DK == 64 ? 32 : DK, MODE, CHAN> : scan_short_kernel<DK, MODE, CHAN>;
-  brief<<<dim3((a.vdim + kOneCols - 1) / kOneCols, a.heads, a.num_seqs), 128, 0, st_>>>(a, most);
+  brief<<<dim3((a.vdim + kOneCols - 1) / kOneCols, a.heads, a.num_seqs), 128, 0, st_>>>(a);
   B200_CUDA_LAUNCH_CHECK();
   // sequences that can be longer than that: none in a step of few tokens, as of decoded ones
-  const int longer = num_tokens > 0 ? std::min(a.num_seqs, num_tokens / (most + 1)) : a.num_seqs;
+  const int longer = num_tokens > 0 ? std::min(a.num_seqs, num_tokens / (kShort + 1)) : a.num_seqs;
   if (longer == 0) return;
-  if (narrow) launch_scan_ww<DK, MODE, CHAN, 4>(a, longer, most, err, st_);
-  else launch_scan_ww<DK, MODE, CHAN, 8>(a, longer, most, err, st_);
+  if (narrow) launch_scan_ww<DK, MODE, CHAN, 4>(a, longer, err, st_);
+  else launch_scan_ww<DK, MODE, CHAN, 8>(a, longer, err, st_);
 }
 // dim: rows of the state; at most 256 (the caller has checked)
 template <int MODE, bool CHAN>
