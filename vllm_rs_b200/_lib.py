@@ -11,7 +11,7 @@ import re
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
-# B200_LIB_PATH: load an instrumented build instead (tools/dec_trace.py builds one with -DB200_DEC_TRACE)
+# B200_LIB_PATH: load an instrumented build instead (-DB200_DEC_TRACE, wna16_tc_dec.cu)
 LIB_PATH = Path(os.environ["B200_LIB_PATH"]) if os.environ.get("B200_LIB_PATH") else PKG / "libb200_vllm.so"
 # the subset library of the fp32-residual hybrid decoders (build.py --target hybrid): loaded when the full one is absent
 HYBRID_LIB_PATH = PKG / "libb200_hybrid.so"

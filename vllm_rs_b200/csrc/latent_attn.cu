@@ -13,7 +13,7 @@
 // (head h's result times sigmoid(gate[t, h]); the gate commutes with the value expansion that follows).  A layer may
 // read ANOTHER layer's cache (latent_prep with no cache: queries only), with its own W_uk / W_uv folded in around it.
 // bf16 caches with kv_rank a multiple of 64 up to 512 and kv_rank + rot_dim a multiple of 32 take paged_attn_tc.cu (tcgen05; prompt
-// 4096, 32 heads, rank 512, window 2048: 7766 -> 690 us against the kernel here).  For the other sizes: an fp32 FMA form (any
+// 4096, 32 heads, rank 512, window 2048: 7766 -> 678 us against the kernel here).  For the other sizes: an fp32 FMA form (any
 // sizes, both dtypes; rows of small steps split their keys over several blocks and merge) and an mma.sync form for steps
 // of many rows (kv_rank a multiple of 64 up to 512, kv_rank + rot_dim a multiple of 16).  Beside paged_attn_decode.cu / attn_prefill*.cu (per-head K / V caches, fp16 / bf16, no window
 // over prompts).

@@ -10,8 +10,9 @@
 // gathers of four rows (~90 cycles each) as by cp.async, whose blocks need a wait and a fence on their way to the tensor core
 // (prompt of 4096 rows, 16 experts, first product: 183 us and 103-139 us).
 //
-// Measured, mma.sync kernel -> here (whole call): 4096 rows of 2048, 16 experts of 512, 4 chosen: 705 -> 201 us; 32 rows 71 -> 46;
-// 4096 wide, 32 experts of 1024: 3000 rows 1903 -> 406 us, 32 rows 198 -> 142.  The calls with few rows are the five launches.
+// Measured, mma.sync kernel -> here (whole call): 4096 rows of 2048, 16 experts of 512, 4 chosen: 709 -> 195 us, 32 rows, device time,
+// 67 -> 36; 4096 wide, 32 experts of 1024: 3000 rows 1903 -> 406 us, 32 rows, device time, 202 -> 159.  moe.cu says which products are
+// long enough to come here.
 // Bound: tensor cores where experts get hundreds of rows, HBM (every hit expert's weights once) where they get few; BN is 256
 // where that gives every SM two tiles, else 128 where that gives three SMs in four one (below that the launches are the bound),
 // else 64.  Whole calls with BN = 64 / 128 / 256, 2048 wide, 16 experts of 512: 2 rows 47.8 / 47.5 / 49.2 us (128 / 64 / 32 tiles

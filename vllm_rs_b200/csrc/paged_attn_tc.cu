@@ -22,9 +22,10 @@
 //
 // Bound: tensor cores for prompts (per page 2 * 128 * 64 * (dim * passes + vdim) flop against 64 * dim * 2 bytes from L2),
 // HBM for steps of few rows, whose keys are split over blocks; window_attn_merge / latent_attn_merge then finish.
-// Measured, mma.sync kernels -> here: window 1024, 4096 rows, 16 heads of 128 over 4: 622 -> 99 us (303 TFLOP/s; what bounds it
+// Measured, mma.sync kernels -> here: window 1024, 4096 rows, 16 heads of 128 over 4: 622 -> 98 us (305 TFLOP/s; what bounds it
 // is the softmax warps' issue slots, then the start and the drain of 128 blocks); latent, 2 x 2048 rows, 32 heads, rank 512:
-// 7766 -> 690 us (433 TFLOP/s useful, 656 issued); 32 tokens over 2048 keys, 32 heads over 8: 317 -> 59 us (35 at HBM rate).
+// 7766 -> 678 us (441 TFLOP/s useful, 668 issued); 32 tokens over 2048 keys, 32 heads over 8: 317 -> 62 us (35 at HBM rate): 256 blocks
+// of 33 pages in turn, with four rows in one of the four row warps.
 #include "paged_attn_tc.cuh"
 
 #include <algorithm>

@@ -640,8 +640,8 @@ void launch_gated_group_norm(void* out, const float* y, int ldy, const float* ga
           o, y, ldy, gate, ldg, w, w_period, C, group, units, eps, gate_first, gate_act);
     };
     // A warp per group up to 512 entries, which waits for no other warp, and where groups are few a warp per 128 entries of one.
-    // us for rows of 2048, by warps and split: 8 rows of groups of 256 SPLIT_A, 100 rows SPLIT_B, 300 rows SPLIT_C; groups of 512: 8
-    // rows SPLIT_D, 300 rows SPLIT_E, 1000 rows SPLIT_F.
+    // us for rows of 2048, by warps and split: 8 rows of groups of 256 3.2 and 2.5, 100 rows 3.3 and 2.7 (150 rows, by warps again, 3.4);
+    // groups of 512: 8 rows 4.8 and 2.5, 300 rows 5.2 and 3.6 (500 rows, by warps again, 5.2).
     const bool warp = group <= 512, split = warp && group > 128 && units < 3 * sm_count() * group / 128;
     auto pick = [&](auto nv) {
       constexpr int NV = decltype(nv)::value;

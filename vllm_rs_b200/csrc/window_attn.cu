@@ -36,7 +36,7 @@
 // by the angle position * freq[i] (angles in double), writes the K and V rows at the token's slot and the query in fp32.
 //
 // Attention kernels: bf16 caches with dim a multiple of 32 (64 at least) and vdim a multiple of 64 up to 256 take paged_attn_tc.cu
-// (tcgen05; prompt 4096 x 16 heads of 128, window 1024: 622 -> 99 us; 32 decoded tokens over 2048 keys, 32 heads: 317 -> 59 us
+// (tcgen05; prompt 4096 x 16 heads of 128, window 1024: 622 -> 98 us; 32 decoded tokens over 2048 keys, 32 heads: 317 -> 62 us
 // against the kernels here).  For the other sizes: an fp32 FMA form (any sizes, both dtypes; the rows of small steps split
 // their keys over several blocks and merge) and mma.sync forms: for steps of many rows 64 token rows per block with the
 // softmax in the accumulator registers (dim and vdim multiples of 16, vdim up to 128; otherwise 16 rows per block, vdim a

@@ -385,7 +385,7 @@ __device__ __forceinline__ void push_signal(const FusedEpi& fe, int tid, int nth
 // epilogue.  lane = 4 channels, warp = row phase.  ALL loads of a batch (2 rows x up to 4 splits
 // x float4) are issued before the first add: an in-order warp that meets a dependent add between
 // two loads pays an L2 round trip per add -- the previous scalar version took 3 us for 32 loads,
-// the longest piece of every GEMM's serial tail (tools/dec_trace.py).
+// the longest piece of every GEMM's serial tail (profiles/r1_v7_dec_gemm_trace.txt).
 template <int EPI>
 __device__ __forceinline__ void split_reduce_rows(const SplitOut& o, int nt, int tid, int nthreads,
                                                   int m_lo, int m_hi) {

@@ -25,7 +25,7 @@ namespace b200 {
 namespace dec {
 
 #ifdef B200_DEC_TRACE
-// Pipeline trace (tools/dec_trace.py): SM clock of each role's events for CTA (0,0), one slot per
+// Pipeline trace: SM clock of each role's events for CTA (0,0), one slot per
 // (event, chunk).  Compiled only with -DB200_DEC_TRACE; production builds carry none of it.
 __device__ uint32_t* g_dec_trace = nullptr;
 #define DEC_TR(ev, i)                                                                        \
@@ -70,7 +70,7 @@ struct Cfg {
   static constexpr int kWBytes = kTileN * kChunkK * BITS / 8;            // one (tile, 64-K chunk)
   static constexpr int kXBytes = NT * kChunkK * 2;
   // Copies move SUPER-chunks of 4 consecutive K chunks (one per dequant group): the pipeline
-  // trace (tools/dec_trace.py) showed one producer thread needs ~400 cycles per copy it issues,
+  // trace (profiles/r1_v7_dec_gemm_trace.txt) showed one producer thread needs ~400 cycles per copy it issues,
   // which with 4 KB copies WAS the chunk period of the whole kernel.
   static constexpr int kSuper = kGroups;
   static constexpr int kWSBytes = kSuper * kWBytes;                       // 16 KB (4-bit) / 32 KB
