@@ -150,10 +150,10 @@ using ScanArgs = b200_scan_args;
 template <int DK, bool CHAN, int WW> struct ScanSmem {         // WW: walking warps, four columns each
   static constexpr int kRows = kBT * DK;                                        // floats of one array of token rows
   static constexpr int kV = (CHAN ? 3 : 2) * kRows;                             // k | q | decays | v | scalars | T, P (8 x 8 each) | ..
-  static constexpr int kCols = WW * 4, kG = kV + kBT * kCols, kMat = kG + 4 * kBT;          // decay, strength, G_t, W_t per token
+  static constexpr int kCols = WW * 4, kG = kV + kBT * kCols, kMat = kG + 4 * kBT;          // rest of G_7, strength, G_t, W_t per token
   static constexpr int kRat = kMat + 2 * kBT * kBT;                             // [t][j] decay from token j to token t
-  static constexpr int kGend = kRat + kBT * kBT;                                // CHAN: [DK] decays over the block
-  static constexpr int kBuf = kGend + (CHAN ? DK : 0);
+  static constexpr int kGend = kRat + kBT * kBT;                                // CHAN: [DK] decays over the block, [DK] their rests
+  static constexpr int kGrest = kGend + (CHAN ? DK : 0), kBuf = kGrest + (CHAN ? DK : 0);
   static constexpr int kU = kRing * kBuf;                                       // [WW][8 tokens][4 columns]
   static constexpr int kBars = kU + WW * kBT * 4;
   static constexpr int kBytes = kBars * 4 + 2 * kRing * 8 + 16;
@@ -213,7 +213,7 @@ __device__ __forceinline__ float meet32(float (&x)[32], int lane) {
 // WW = 8 lets two walking warps share a scheduler and a prepared block, WW = 4 spreads few columns over more SMs.
 // Bound: the chain of blocks, one walk after another, of fp32 FMAs and a butterfly over the lanes; HBM and the FMA units would
 // take 16 and 89 us for 4096 tokens of 16 heads of 128 x 128.  Measured there, token by token (eight lanes per column, four
-// chained shuffles per token) -> in blocks: delta rule 2278 -> 610 us; decayed state of 8 heads of 128 x 256: 909 -> 388 us.  The
+// chained shuffles per token) -> in blocks: delta rule 2278 -> 610 us; decayed state of 8 heads of 128 x 256: 909 -> 391 us.  The
 // state's update does not wait for the read-out's sums: the queries' products are taken before the correction's sums meet, and
 // meet under the update (665 and 424 us with both in turn).
 template <int DK, int MODE, bool CHAN, int WW>
@@ -337,20 +337,28 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
 #pragma unroll
         for (int z = 0; z < 2; ++z) {
           const int t = (lane >> 3) + z * 4, j = lane & 7;
-          float r = 1.f;
+          float r = 1.f, rest = 0.f;                   // the product and what its roundings left
+          auto times = [&](float x) {
+            const float p = __fmul_rn(r, x);
+            if (MODE == kDecay) rest = fmaf(rest, x, fmaf(r, x, -p));
+            r = p;
+          };
 #pragma unroll
           for (int m = 1; m < kBT; ++m) {
             const float gm = __shfl_sync(0xffffffffu, g, m);
-            if (m > j && m <= t) r *= gm;
+            if (m > j && m <= t) times(gm);
           }
-          R[t * kBT + j] = r;
-          if (j == 0) G[2 * kBT + t] = r * __shfl_sync(0x01010101u, g, 0);
-          if (t == kBT - 1) G[3 * kBT + j] = r;
+          R[t * kBT + j] = r + rest;
+          if (t == kBT - 1) G[3 * kBT + j] = r + rest;
+          const float g0 = __shfl_sync(0xffffffffu, g, 0);
+          if (j == 0) {
+            times(g0);
+            const float whole = r + rest;
+            G[2 * kBT + t] = whole;
+            if (t == kBT - 1) G[0] = rest - (whole - r);
+          }
         }
-        if (lane < kBT) {
-          G[lane] = g;
-          G[kBT + lane] = w;
-        }
+        if (lane < kBT) G[kBT + lane] = w;
       };
       // which entry of a triangle, row after row, this lane gets: M (rows 1 .., j < t) for warp 1, P (j <= t) from row 4 on for warp
       // 0, of rows 0 - 3 for warp 2
@@ -506,14 +514,25 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
           // k <- G_t k_t, q <- G_t q_t, decays <- W_t k_t, per channel; the block's whole decay
           sync();
           for (int e = pt; e < DK; e += 128) {
-            float kr[kBT], d[kBT], g = 1.f;
+            float kr[kBT], d[kBT], g = 1.f, rest = 0.f;
 #pragma unroll
             for (int t = 0; t < kBT; ++t) {
               kr[t] = B[t * DK + e];
               d[t] = e < dim ? B[2 * SM::kRows + t * DK + e] : 1.f;
-              g *= d[t];
+              if (MODE == kDecay) {                    // (with what the products' roundings leave)
+                const float p = __fmul_rn(g, d[t]);
+                rest = fmaf(rest, d[t], fmaf(g, d[t], -p));
+                g = p;
+              } else {
+                g *= d[t];
+              }
               B[t * DK + e] = kr[t] * g;
               B[SM::kRows + t * DK + e] *= g;
+            }
+            if (MODE == kDecay) {
+              const float whole = g + rest;
+              B[SM::kGrest + e] = rest - (whole - g);
+              g = whole;
             }
             B[SM::kGend + e] = g;
             g = 1.f;
@@ -564,8 +583,8 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
       int from[kBT];
 #pragma unroll
       for (int j = 0; j < kBT; ++j) from[j] = min(j, tt) * 4 + c4;
-      // what entry j of a row of the triangles is multiplied by; from this token back in both forms, so that their bits are equal
-      auto entry = [](int i) { return BACK ? i : kBT - 1 - i; };
+      // what entry j of a row of the triangles is multiplied by; the oldest token first in both forms, so that their bits are equal
+      auto entry = [](int i) { return BACK ? kBT - 1 - i : i; };
       auto part = [&](float x, int j) { return BACK ? __shfl_up_sync(0xffffffffu, x, j * 4) : __shfl_sync(0xffffffffu, x, from[j]); };
       for (int i = 0; i < nblk; ++i) {
         const int g = blocks + i;
@@ -617,20 +636,27 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
           const int t = t0 + i * kBT + tt;
           if (t < t1 && colw + c4 < vdim) a.out[(static_cast<size_t>(t) * a.heads + h) * vdim + colw + c4] = o;
         }
+        // The block's decay meets the first token's part in one rounding, as eight tokens' decays would.  A state that only decays takes
+        // it with what its own rounding left, which would otherwise be the same in every block and add up (heads of 128 x 128, 500
+        // tokens of one decay and sign: 2.6e-7 off against 64 bits without, 0.7e-7 token by token).
+        // (The corrected form with a decay per channel, short of registers, decays first: 2.8e-7, 3.0e-7 token by token.)
+        constexpr bool REST = MODE == kDecay, FIRST = MODE == kDelta && CHAN;
+        f2 ge[CH / 2], gl[CH / 2];
         if (CHAN) {
-          f2 ge[CH / 2];
           ldv2<CH>(ge, B + SM::kGend + lane * CH);
+          if (FIRST) {
 #pragma unroll
-          for (int c = 0; c < 4; ++c)
+            for (int c = 0; c < 4; ++c)
 #pragma unroll
-            for (int r = 0; r < CH / 2; ++r) s[c][r] = mul2(s[c][r], ge[r]);
+              for (int r = 0; r < CH / 2; ++r) s[c][r] = mul2(s[c][r], ge[r]);
+          }
+          if (REST) ldv2<CH>(gl, B + SM::kGrest + lane * CH);
         } else {
-          const float ge = G[3 * kBT - 1];
-          const f2 g2 = pack2(ge, ge);
 #pragma unroll
-          for (int c = 0; c < 4; ++c)
-#pragma unroll
-            for (int r = 0; r < CH / 2; ++r) s[c][r] = mul2(s[c][r], g2);
+          for (int r = 0; r < CH / 2; ++r) {
+            ge[r] = pack2(G[3 * kBT - 1], G[3 * kBT - 1]);
+            if (REST) gl[r] = pack2(G[0], G[0]);
+          }
         }
         const float* kd = B + (CHAN ? 2 * SM::kRows : 0) + lane * CH;       // keys as they enter the state
 #pragma unroll
@@ -638,14 +664,14 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
           f2 y[CH / 2];
           ldv2<CH>(y, kd + t * DK);
           const float4 uu = *reinterpret_cast<const float4*>(us + t * 4);
-          const f2 u0 = pack2(uu.x, uu.x), u1 = pack2(uu.y, uu.y), u2 = pack2(uu.z, uu.z), u3 = pack2(uu.w, uu.w);
+          const f2 u[4] = {pack2(uu.x, uu.x), pack2(uu.y, uu.y), pack2(uu.z, uu.z), pack2(uu.w, uu.w)};
 #pragma unroll
-          for (int r = 0; r < CH / 2; ++r) {
-            s[0][r] = fma2(y[r], u0, s[0][r]);
-            s[1][r] = fma2(y[r], u1, s[1][r]);
-            s[2][r] = fma2(y[r], u2, s[2][r]);
-            s[3][r] = fma2(y[r], u3, s[3][r]);
-          }
+          for (int r = 0; r < CH / 2; ++r)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              if (t == 0 && !FIRST) s[c][r] = fma2(s[c][r], ge[r], REST ? fma2(y[r], u[c], mul2(s[c][r], gl[r])) : mul2(y[r], u[c]));
+              else s[c][r] = fma2(y[r], u[c], s[c][r]);
+            }
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(&done[g % kRing]);
