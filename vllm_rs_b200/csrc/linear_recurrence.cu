@@ -142,6 +142,7 @@ __device__ __forceinline__ void unpack2(f2 v, float& lo, float& hi) { asm("mov.b
 constexpr int kOneCols = 16;                   // columns of S per block of threads: single tokens
 constexpr int kBT = 8;                         // tokens per block of the recurrence
 constexpr int kRing = 8;                       // blocks of tokens in shared memory (with four, fetching waited for the walk)
+constexpr int kSorted = 64;                    // sequences up to which a step's longest go first
 constexpr int kShort = 16;                     // tokens of a sequence up to which it is walked token by token
 constexpr int kDelta = 0, kDecay = 1, kSsd = 2;
 
@@ -229,10 +230,26 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
   const int h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, col0 = blockIdx.x * COLS;
   const int dim = a.dim, vdim = a.vdim, hk = MODE == kDecay ? h : h / (a.heads / a.kv_heads);
   constexpr int kAll = WW * 32 + 256;
+  // Longest sequences first: where not all blocks fit the chip at once, the last to start have the least to do.  Three sequences
+  // of 500, 1000 and 1501 tokens, 8 heads of 128 x 256 (192 blocks): 2001 tokens in a row before, 1501 now; the four scans of a
+  // hybrid step take 960 us instead of 1.24 ms.
+  __shared__ uint8_t order[kSorted];
+  const bool sorted = num_seqs <= kSorted;
+  if (sorted && tid < num_seqs) {
+    const uint32_t n = a.cu_seqlens_q[tid + 1] - a.cu_seqlens_q[tid];
+    int rank = 0;
+    for (int i = 0; i < num_seqs; ++i) {
+      const uint32_t m = a.cu_seqlens_q[i + 1] - a.cu_seqlens_q[i];
+      rank += m > n || (m == n && i < tid);
+    }
+    order[rank] = static_cast<uint8_t>(tid);
+  }
+  __syncthreads();
+  auto seq = [&](int z) { return sorted ? static_cast<int>(order[z]) : z; };
   {
     int mine = 0;                                                      // a sequence for this kernel among the block's
-    for (int b = blockIdx.z + tid * gridDim.z; b < num_seqs; b += kAll * gridDim.z)
-      mine |= static_cast<int>(a.cu_seqlens_q[b + 1] - a.cu_seqlens_q[b]) > kShort;
+    for (int z = blockIdx.z + tid * gridDim.z; z < num_seqs; z += kAll * gridDim.z)
+      mine |= static_cast<int>(a.cu_seqlens_q[seq(z) + 1] - a.cu_seqlens_q[seq(z)]) > kShort;
     if (!__syncthreads_or(mine)) return;
   }
   if (tid == 0) {
@@ -248,8 +265,8 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
   }
   __syncthreads();
   int blocks = 0;                                                      // blocks of tokens so far, over all sequences
-  for (int b = blockIdx.z; b < num_seqs; b += gridDim.z) {
-    const int t0 = a.cu_seqlens_q[b], t1 = a.cu_seqlens_q[b + 1], nblk = (t1 - t0 + kBT - 1) / kBT;
+  for (int z = blockIdx.z; z < num_seqs; z += gridDim.z) {
+    const int b = seq(z), t0 = a.cu_seqlens_q[b], t1 = a.cu_seqlens_q[b + 1], nblk = (t1 - t0 + kBT - 1) / kBT;
     if (t1 - t0 <= kShort) continue;                                   // (scan_short_kernel)
     const bool fresh = static_cast<int>(a.context_lens[b]) == t1 - t0;
     if (warp >= WW) {
