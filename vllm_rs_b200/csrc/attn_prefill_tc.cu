@@ -15,12 +15,14 @@
 //                  written back to TMEM with tcgen05.st
 //   O += P V       tcgen05.mma TS: A = P from TMEM, B = V page as an MN-major operand (D contiguous),
 //                  fp32 [128 x 128] in TMEM for the whole walk
-// Warp roles: warp 0 TMA producer (2-stage K|V ring), warp 1 MMA issuer (QK^T of page j+1 is issued
+// Warp roles: warp 0 TMA producer (two places for K, two for V), warp 1 MMA issuer (QK^T of page j+1 is issued
 // before PV of page j, so it runs under the softmax of page j), warps 2-5 softmax / correction /
 // epilogue.  96 KB of shared memory and 256 TMEM columns per CTA: two CTAs share an SM and fill each
-// other's softmax bubbles.  Tensor-bound (4 * 128 * ctx flop per row) with MUFU.EX2 and the softmax warps' issue
-// slots as co-limits: without exp2f's guard for denormal results, a multiplication per score and two-input maxima 32 heads
-// over 3 sequences of 8192 rows together take 421 us instead of 441.
+// other's softmax bubbles.  Bound: the chain of a page's softmax (its waits, TMEM's latencies, 64 exponentials per row);
+// tensor cores (4 * 128 * ctx flop per row) and MUFU.EX2 are half idle.  So K's place is given back as soon as the scores
+// are made and fetched again under two softmaxes (K and V in one place: the next scores waited for PV and the fetch), P
+// has two places, so that its store need not wait for the last PV, the next scores come out of TMEM while P is stored, and
+// scaling and sums are two values per instruction.  32 heads over 3 sequences of 8192 rows together: 418 -> 361 us.
 #include <cstdlib>
 #include <cstring>
 
@@ -42,7 +44,7 @@ constexpr int kBarOff = kQBytes + kStages * kStageBytes;
 constexpr int kTmemPtrOff = kBarOff + 16 * 8;
 constexpr int kAlloc = kTmemPtrOff + 16 + 1024;
 constexpr int kTmemCols = 256;
-constexpr int kSCol = 0, kPCol = 64, kOCol = 128;
+constexpr int kSCol = 0, kPCol = 64, kOCol = 128;   // P: two places of 32 columns, for even and odd pages
 constexpr float kRescaleThreshold = 8.f;         // log2 units
 
 // MN-major SWIZZLE_128B operand: rows of 128 B hold 64 consecutive MN elements of ONE K index;
@@ -79,6 +81,25 @@ __device__ __forceinline__ float ex2(float x) {
 __device__ __forceinline__ float max3(float a, float b, float c) {
   float r;
   asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+
+// two fp32 values in a 64-bit register, one instruction for both
+using f2 = unsigned long long;
+__device__ __forceinline__ f2 pack2(float lo, float hi) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack2(f2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f2 add2(f2 a, f2 b) {
+  f2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
 
@@ -130,24 +151,29 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_co
                                              ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kBarOff);
   uint64_t* q_full = bars;
-  uint64_t* kv_full = bars + 1;        // [2]
-  uint64_t* kv_empty = bars + 3;       // [2]
-  uint64_t* s_full = bars + 5;
-  uint64_t* s_free = bars + 6;
-  uint64_t* p_full = bars + 7;
-  uint64_t* pv_done = bars + 8;
+  uint64_t* k_full = bars + 1;         // [2]: K and V of a page are free at different times, K as soon as its scores are made
+  uint64_t* k_empty = bars + 3;        // [2]
+  uint64_t* v_full = bars + 5;         // [2]
+  uint64_t* v_empty = bars + 7;        // [2]
+  uint64_t* s_full = bars + 9;
+  uint64_t* s_free = bars + 10;
+  uint64_t* p_full = bars + 11;
+  uint64_t* pv_done = bars + 12;       // [2], of even and odd pages
   uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(smem + kTmemPtrOff);
 
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
     for (int s = 0; s < kStages; ++s) {
-      mbar_init(&kv_full[s], 1);
-      mbar_init(&kv_empty[s], 1);
+      mbar_init(&k_full[s], 1);
+      mbar_init(&k_empty[s], 1);
+      mbar_init(&v_full[s], 1);
+      mbar_init(&v_empty[s], 1);
     }
     mbar_init(s_full, 1);
     mbar_init(s_free, 4);
     mbar_init(p_full, 4);
-    mbar_init(pv_done, 1);
+    mbar_init(&pv_done[0], 1);
+    mbar_init(&pv_done[1], 1);
     fence_barrier_init();
     prefetch_tmap(&qmap);
     prefetch_tmap(&kmap);
@@ -174,27 +200,40 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_co
       tma_load_3d(q_smem + kRows * 128, &qmap, q_full, 64, hkv * G, row0 + q0);
     }
     const uint32_t* bt = a.block_tables + static_cast<size_t>(b) * a.max_blocks;
-    for (int base = 0; base < npages; base += 32) {
+    // V of a page goes behind K of the next: it is wanted a softmax later, and its place comes free later
+    int last = 0;                      // page number of the page before
+    for (int base = 0; base <= npages; base += 32) {
       const int mine = base + lane < npages ? static_cast<int>(bt[base + lane]) : 0;
-      const int cnt = min(32, npages - base);
+      const int cnt = min(32, npages + 1 - base);
       for (int jj = 0; jj < cnt; ++jj) {
         const int blk = __shfl_sync(0xffffffffu, mine, jj);
         if (lane == 0) {
           const int j = base + jj, s = j & 1;
-          mbar_wait_bounded(&kv_empty[s], ((j >> 1) & 1) ^ 1);
-          mbar_arrive_expect_tx(&kv_full[s], kStageBytes);
-          uint8_t* kdst = kv_smem + s * kStageBytes;
-          uint8_t* vdst = kdst + kTileBytes;
-          if (L1) {
-            tma_load_4d(kdst, &kmap, &kv_full[s], 0, 0, hkv, blk);
-            tma_load_4d(vdst, &vmap, &kv_full[s], 0, 0, hkv, blk);
-          } else {
-            tma_load_4d(kdst, &kmap, &kv_full[s], 0, hkv, 0, blk);
-            tma_load_4d(kdst + kTok * 128, &kmap, &kv_full[s], 64, hkv, 0, blk);
-            tma_load_4d(vdst, &vmap, &kv_full[s], 0, hkv, 0, blk);
-            tma_load_4d(vdst + kTok * 128, &vmap, &kv_full[s], 64, hkv, 0, blk);
+          if (j < npages) {
+            mbar_wait_bounded(&k_empty[s], ((j >> 1) & 1) ^ 1);
+            mbar_arrive_expect_tx(&k_full[s], kTileBytes);
+            uint8_t* kdst = kv_smem + s * kStageBytes;
+            if (L1) {
+              tma_load_4d(kdst, &kmap, &k_full[s], 0, 0, hkv, blk);
+            } else {
+              tma_load_4d(kdst, &kmap, &k_full[s], 0, hkv, 0, blk);
+              tma_load_4d(kdst + kTok * 128, &kmap, &k_full[s], 64, hkv, 0, blk);
+            }
+          }
+          if (j > 0) {
+            const int i = j - 1, t = i & 1;
+            mbar_wait_bounded(&v_empty[t], ((i >> 1) & 1) ^ 1);
+            mbar_arrive_expect_tx(&v_full[t], kTileBytes);
+            uint8_t* vdst = kv_smem + t * kStageBytes + kTileBytes;
+            if (L1) {
+              tma_load_4d(vdst, &vmap, &v_full[t], 0, 0, hkv, last);
+            } else {
+              tma_load_4d(vdst, &vmap, &v_full[t], 0, hkv, 0, last);
+              tma_load_4d(vdst + kTok * 128, &vmap, &v_full[t], 64, hkv, 0, last);
+            }
           }
         }
+        last = blk;
       }
     }
   } else if (warp == 1) {
@@ -207,7 +246,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_co
       const uint32_t q_addr = smem_u32(q_smem);
       auto issue_qk = [&](int j) {
         const int s = j & 1;
-        mbar_wait_bounded(&kv_full[s], (j >> 1) & 1);
+        mbar_wait_bounded(&k_full[s], (j >> 1) & 1);
         if (j > 0) mbar_wait_bounded(s_free, (j - 1) & 1);      // softmax holds S of page j-1 in registers
         tc_fence_after();
         const uint32_t k_addr = smem_u32(kv_smem + s * kStageBytes);
@@ -220,6 +259,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_co
                                     : make_smem_desc_sw128(k_addr + (ks >> 2) * (kTok * 128) + off);
           tc_mma_ss(s_tmem, adesc, bdesc, idesc_s, ks > 0 ? 1u : 0u);
         }
+        tc_commit(&k_empty[s]);
         tc_commit(s_full);
       };
       mbar_wait_bounded(q_full, 0);
@@ -228,6 +268,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_co
         if (j + 1 < npages) issue_qk(j + 1);
         const int s = j & 1;
         mbar_wait_bounded(p_full, j & 1);
+        mbar_wait_bounded(&v_full[s], (j >> 1) & 1);
         tc_fence_after();
         const uint32_t v_addr = smem_u32(kv_smem + s * kStageBytes + kTileBytes);
 #pragma unroll
@@ -235,10 +276,10 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_co
           const uint64_t bdesc = L1 ? make_smem_desc_sw128(v_addr + ks * 32)
                                  : (a.dbg & 1) ? make_smem_desc_mn_sw128(v_addr + ks * 2048, 1024, kTok * 128)
                                                : make_smem_desc_mn_sw128(v_addr + ks * 2048, kTok * 128, 1024);
-          tc_mma_ts(o_tmem, p_tmem + ks * 8, bdesc, idesc_o, (j > 0 || ks > 0) ? 1u : 0u);
+          tc_mma_ts(o_tmem, p_tmem + s * 32 + ks * 8, bdesc, idesc_o, (j > 0 || ks > 0) ? 1u : 0u);
         }
-        tc_commit(&kv_empty[s]);
-        tc_commit(pv_done);
+        tc_commit(&v_empty[s]);
+        tc_commit(&pv_done[s]);
       }
     }
   } else {
@@ -252,25 +293,37 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_co
     const int qpos = cached + tq;                         // last visible key of this row
     const int first_limit = cached + q0;                  // smallest limit in the CTA
     float m_ref = -INFINITY, l_run = 0.f;
-    for (int j = 0; j < npages; ++j) {
-      const int page_base = j * kTok;
-      mbar_wait_bounded(s_full, j & 1);
+    // S of a page is on its way from TMEM while the page before is stored: asked for by ask(), there after take()
+    uint32_t v0[32], v1[32];
+    auto ask = [&] {
       tc_fence_after();
-      float x[kTok];
-      {
-        uint32_t v0[32], v1[32];
-        tmem_ld_x32(tmem_base + lane_base + kSCol, v0);
-        tmem_ld_x32(tmem_base + lane_base + kSCol + 32, v1);
-        tc_wait_ld();
+      tmem_ld_x32(tmem_base + lane_base + kSCol, v0);
+      tmem_ld_x32(tmem_base + lane_base + kSCol + 32, v1);
+    };
+    auto take = [&] {
+      tc_wait_ld();
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          x[i] = __uint_as_float(v0[i]);
-          x[32 + i] = __uint_as_float(v1[i]);
-        }
+      for (int i = 0; i < 32; i += 8) {                   // (no use of these registers moves before the wait)
+        asm volatile("" : "+r"(v0[i]), "+r"(v0[i + 1]), "+r"(v0[i + 2]), "+r"(v0[i + 3]), "+r"(v0[i + 4]), "+r"(v0[i + 5]),
+                          "+r"(v0[i + 6]), "+r"(v0[i + 7]));
+        asm volatile("" : "+r"(v1[i]), "+r"(v1[i + 1]), "+r"(v1[i + 2]), "+r"(v1[i + 3]), "+r"(v1[i + 4]), "+r"(v1[i + 5]),
+                          "+r"(v1[i + 6]), "+r"(v1[i + 7]));
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(s_free);                 // S may be overwritten by QK^T of page j+1
+      if (lane == 0) mbar_arrive(s_free);                 // S may be overwritten by QK^T of the next page
+    };
+    mbar_wait_bounded(s_full, 0);
+    ask();
+    take();
+    for (int j = 0; j < npages; ++j) {
+      const int page_base = j * kTok;
+      float x[kTok];
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        x[i] = __uint_as_float(v0[i]);
+        x[32 + i] = __uint_as_float(v1[i]);
+      }
       if (page_base + kTok - 1 > first_limit) {           // diagonal page: causal mask
 #pragma unroll
         for (int i = 0; i < kTok; ++i) x[i] = (page_base + i <= qpos) ? x[i] : -INFINITY;
@@ -293,18 +346,25 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_co
         m_ref = mx;
         grow = true;
       }
-      float psum = 0.f;
+      f2 sum0 = 0, sum1 = 0;                              // (bits of two zeros)
+      const f2 sc2 = pack2(a.scale_log2, a.scale_log2), mr2 = pack2(-m_ref, -m_ref);
       uint32_t pk[32];
 #pragma unroll
       for (int i = 0; i < 32; ++i) {
-        const float p0 = ex2(fmaf(x[2 * i], a.scale_log2, -m_ref)), p1 = ex2(fmaf(x[2 * i + 1], a.scale_log2, -m_ref));
-        psum += p0 + p1;
+        float p0, p1;
+        unpack2(fma2(pack2(x[2 * i], x[2 * i + 1]), sc2, mr2), p0, p1);
+        p0 = ex2(p0);
+        p1 = ex2(p1);
+        if (i & 1) sum1 = add2(sum1, pack2(p0, p1));
+        else sum0 = add2(sum0, pack2(p0, p1));
         pk[i] = pack16x2<BF>(p0, p1);
       }
-      l_run = l_run * corr + psum;
+      float s0, s1;
+      unpack2(add2(sum0, sum1), s0, s1);
+      l_run = l_run * corr + (s0 + s1);
       // stale V rows past the context (uninitialised cache memory) must not meet the MMA: 0 * NaN
       if (page_base + kTok > ctx) {
-        mbar_wait_bounded(&kv_full[j & 1], (j >> 1) & 1);
+        mbar_wait_bounded(&v_full[j & 1], (j >> 1) & 1);
         uint8_t* vt = kv_smem + (j & 1) * kStageBytes + kTileBytes;
         const int first_bad = ctx - page_base;             // rows [first_bad, 64) of both D halves
         if (L1) {
@@ -327,29 +387,44 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_co
         }
         fence_proxy_async();                               // generic-proxy writes -> tensor-core reads
       }
-      if (j > 0) {
-        mbar_wait_bounded(pv_done, (j - 1) & 1);           // PV of page j-1 retired: P and O are ours
-        tc_fence_after();
-        if (__any_sync(0xffffffffu, grow)) {
+      auto store = [&] {
+        if (j > 1) mbar_wait_bounded(&pv_done[j & 1], ((j - 2) >> 1) & 1);       // PV of page j-2 retired: its P is ours
+        if (j > 0 && __any_sync(0xffffffffu, grow)) {
+          mbar_wait_bounded(&pv_done[(j - 1) & 1], ((j - 1) >> 1) & 1);          // O is ours
+          tc_fence_after();
 #pragma unroll 1
-          for (int c0 = 0; c0 < kD; c0 += 32) {
-            uint32_t o[32];
-            tmem_ld_x32(tmem_base + lane_base + kOCol + c0, o);
+          for (int c0 = 0; c0 < kD; c0 += 16) {
+            uint32_t o[16];
+            tmem_ld_x16(tmem_base + lane_base + kOCol + c0, o);
             tc_wait_ld();
 #pragma unroll
-            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * corr);
-            tmem_st_x32(tmem_base + lane_base + kOCol + c0, o);
+            for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * corr);
+            tmem_st_x16(tmem_base + lane_base + kOCol + c0, o);
           }
         }
+        tc_fence_after();
+        tmem_st_x32(tmem_base + lane_base + kPCol + (j & 1) * 32, pk);
+        tc_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(p_full);
+      };
+      // (asking and taking stay in one branch: nothing is copied between)
+      if (j + 1 == npages) {
+        store();
+      } else if (__all_sync(0xffffffffu, mbar_probe_addr(smem_u32(s_full), (j + 1) & 1))) {
+        ask();
+        store();
+        take();
+      } else {
+        store();
+        mbar_wait_bounded(s_full, (j + 1) & 1);
+        ask();
+        take();
       }
-      tmem_st_x32(tmem_base + lane_base + kPCol, pk);
-      tc_wait_st();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(p_full);
     }
     // ---- epilogue: O / l -> fp16
-    mbar_wait_bounded(pv_done, (npages - 1) & 1);
+    mbar_wait_bounded(&pv_done[(npages - 1) & 1], ((npages - 1) >> 1) & 1);
     tc_fence_after();
     const float inv_l = valid ? 1.f / l_run : 0.f;
     __half* dst = a.out + (static_cast<size_t>(row0 + tq) * a.H + hkv * G + g) * kD;
