@@ -283,6 +283,66 @@ def test_wna16_streamk_decode(ops, fmt, bits, K, N, M, group, epi, variant):
         assert e_new <= e_old + 5e-4, (e_new, e_old)
 
 
+def _wna_run(ops, fmt, bits, K, N, M, group, epi, seed):
+    """(call with a variant, reference, exact product as a function) of one quantised projection."""
+    qw, qz, s, W, x = _wna_case(K, N, M, fmt, bits, seed=seed, group=group)
+    qwd = torch.from_numpy(qw).cuda()
+    packed = ops.awq_prepack(qwd) if fmt == "awq" else ops.gptq_prepack(qwd, bits)
+    ws = ops.wna16_workspace(max(M, 16), N)
+    sd, zd = torch.from_numpy(s).cuda(), None if qz is None else torch.from_numpy(qz).cuda()
+    bias = torch.randn(N).to(F16) if epi == "bias" else None
+    kw = dict(k=K, n=N, bits=bits, group_size=group, qfmt=ops.QFMT_AWQ if fmt == "awq" else ops.QFMT_GPTQ,
+              epilogue=ops.EPI_SILU_MUL if epi == "silu" else ops.EPI_NONE, bias=None if bias is None else bias.cuda())
+    full = om.linear(x, W, bias)
+    ref = om.silu_mul(full[:, :N // 2], full[:, N // 2:]) if epi == "silu" else full
+
+    def call(variant):
+        y = ops.wna16_gemm(x.cuda(), packed, sd, zd, ws, variant=variant, **kw)
+        assert int(ws[:16384].view(torch.int32).abs().sum()) == 0      # arrival counters back at rest
+        return y
+
+    def truth():
+        q = oq.unpack_awq(qw) if fmt == "awq" else oq.unpack_gptq(qw, bits)
+        z = oq.unpack_awq(qz).astype(np.int32) if fmt == "awq" else oq.unpack_gptq_zeros(qz, bits)
+        g = np.arange(K) // group
+        return torch.from_numpy(x.numpy().astype(np.float64) @ ((q.astype(np.float64) - z[g]) * s[g].astype(np.float64)))
+
+    return call, ref, truth
+
+
+@pytest.mark.parametrize("fmt,bits,K,N,M,group,epi", [
+    ("awq", 4, 128, 128, 1, 128, "none"),          # one unit: the second group of warps has none
+    ("awq", 4, 384, 256, 9, 128, "silu"),          # three units per tile, pairs of gate and up
+    ("gptq", 4, 640, 384, 8, 640, "bias"),         # one quantisation group; tiles of five units
+    ("gptq_sym", 4, 2048, 1536, 16, 256, "none"),  # no zero points, two units per group
+    ("awq", 4, 4096, 28672, 3, 128, "silu"),       # ranges cut anywhere: two tiles in a block
+    ("awq", 4, 256, 40960, 5, 128, "none"),        # more tiles than blocks, whole tiles and parts in one block
+    ("awq", 4, 14336, 4096, 2, 128, "none"),       # eight parts per tile
+    ("awq", 4, 2048, 34816, 16, 128, "none"),      # as many units as the sixteen tokens want
+])
+def test_wna16_decode_of_few_tokens(ops, fmt, bits, K, N, M, group, epi):
+    """wna16_mma.cu (variant 7, and what variant 0 takes at up to 16 tokens)."""
+    call, ref, truth = _wna_run(ops, fmt, bits, K, N, M, group, epi, K + N + M)
+    y = call(7)
+    _close(y, ref, 2e-3, 4e-3 if epi == "silu" else 2e-3)          # the bound of the other variants: fp32 sums, fp16 results
+    assert torch.equal(call(7), y)                 # parts are summed in the order of K
+    if M <= 8 or K // 128 * (N // 128) >= 4096:
+        assert torch.equal(call(0), y)
+    if epi == "none" and "sym" not in fmt:
+        t = truth()
+        e_new, e_old = ((v.cpu().double() - t).norm() for v in (y, call(2)))
+        assert e_new <= e_old * 1.05, (e_new, e_old)               # the same weights, sums in another order
+
+
+@pytest.mark.parametrize("K,N,M,group", [(4096, 9728, 17, 64), (8192, 9728, 33, 64), (8192, 1280, 64, 128)])
+def test_wna16_decode_of_many_groups(ops, K, N, M, group):
+    """wna16_tc_dec.cu where one K piece has exactly as many quantisation groups as are staged, and where it takes more pieces."""
+    call, ref, _ = _wna_run(ops, "awq", 4, K, N, M, group, "none", K + N + M)
+    y = call(2)
+    _close(y, ref, 2e-3, 2e-3)
+    assert torch.equal(call(0), y)
+
+
 def _tc_available(ops):
     from vllm_rs_b200 import _lib
     rng = np.random.default_rng(0)

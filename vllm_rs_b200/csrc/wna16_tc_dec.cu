@@ -568,28 +568,43 @@ wna16_tc_dec_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_const
   }
 }
 
+// K pieces per tile, 64-K chunks of a piece, quantisation groups that a piece touches.
+struct Split { int splits, chunks, groups; };
+static Split split_of(const WnaParams& p) {
+  const int KC = p.K / kChunkK, tiles = p.N / kTileN;
+  const bool grouped = p.group_size < p.K;
+  auto cut = [&](int splits) {
+    Split s;
+    s.chunks = (KC + splits - 1) / splits;
+    s.splits = (KC + s.chunks - 1) / s.chunks;
+    const int k = s.chunks * kChunkK;         // one group more where pieces may start inside a group
+    s.groups = !grouped ? 1 : (k + p.group_size - 1) / p.group_size + (s.splits > 1 && k % p.group_size ? 1 : 0);
+    return s;
+  };
+  if (p.no_split) return cut(1);
+  // more than eight K pieces per tile cost more at the meeting point than they save in the main loop (TP-rank
+  // shapes, profiles/r2_ad_tp_shape_splits.txt: qkv at TP = 8, 6 tiles x 16 pieces 7.7 us -> x 8 pieces 6.5 us)
+  static const int cap_env = getenv("B200_DEC_MAX_SPLITS") ? atoi(getenv("B200_DEC_MAX_SPLITS")) : 8;
+  const int cap = cap_env > 0 ? cap_env : KC;
+  int splits = sm_count() / tiles;
+  if (splits < 1) splits = 1;
+  if (splits > KC / 4) splits = KC / 4 > 0 ? KC / 4 : 1;
+  if (splits > cap) splits = cap;
+  while (splits > 1 && static_cast<long>(splits) * p.N > kMaxSplitCols) --splits;
+  // long K: as many more pieces as the staging of the scales asks for (the kernel for other shapes is far slower here)
+  while (cut(splits).groups > kSZGroups && splits < cap && (splits + 1L) * p.N <= kMaxSplitCols) ++splits;
+  return cut(splits);
+}
+
 template <int BITS, int NT, int EPI>
 static bool launch_epi(const WnaParams& p, cudaStream_t st) {
   using C = Cfg<BITS, NT>;
   const int KC = p.K / kChunkK;
   const int tiles = p.N / kTileN;
-  int splits = sm_count() / tiles;
-  if (splits < 1) splits = 1;
-  if (splits > KC / 4) splits = KC / 4 > 0 ? KC / 4 : 1;
-  {
-    // more than eight K pieces per tile cost more at the meeting point than they save in the main loop (TP-rank
-    // shapes, profiles/r2_ad_tp_shape_splits.txt: qkv at TP = 8, 6 tiles x 16 pieces 7.7 us -> x 8 pieces 6.5 us)
-    static const int cap = getenv("B200_DEC_MAX_SPLITS") ? atoi(getenv("B200_DEC_MAX_SPLITS")) : 8;
-    if (cap > 0 && splits > cap) splits = cap;
-  }
-  while (splits > 1 && static_cast<long>(splits) * p.N > kMaxSplitCols) --splits;
-  if (p.no_split) splits = 1;
-  int cps = (KC + splits - 1) / splits;
-  splits = (KC + cps - 1) / cps;
+  const Split sp = split_of(p);
+  const int cps = sp.chunks, splits = sp.splits, sz_rows = sp.groups;
   const bool grouped = p.group_size < p.K;
   const int total_groups = grouped ? p.K / p.group_size : 1;
-  int sz_rows = grouped ? (cps * kChunkK + p.group_size - 1) / p.group_size + 1 : 1;
-  if (sz_rows > kSZGroups) sz_rows = kSZGroups;
   // activations as a 3-D tensor {64 K elements, M rows, K/64 chunks}: one TMA box brings 4 chunks,
   // each landing as its own [NT rows][128 B] swizzled tile (the MMA B operand of one chunk)
   CUtensorMap xmap, smap, zmap;
@@ -683,16 +698,7 @@ bool launch_wna16_tc_dec(const WnaParams& p, cudaStream_t st) {
   if (p.M > 64) return false;
   const bool pow2 = p.group_size >= p.K || (p.group_size & (p.group_size - 1)) == 0;
   if (!pow2) return false;
-  // scale / zero staging covers 64 quantisation groups of the CTA's K range
-  const int KC = p.K / kChunkK;
-  int splits = sm_count() / (p.N / kTileN);
-  if (splits < 1) splits = 1;
-  if (splits > KC / 4) splits = KC / 4 > 0 ? KC / 4 : 1;
-  if (splits > 8) splits = 8;                 // same cap as launch_epi
-  if (p.no_split) splits = 1;
-  const int cps = (KC + splits - 1) / splits;
-  const int groups_per_cta = p.group_size >= p.K ? 1 : (cps * kChunkK + p.group_size - 1) / p.group_size + 1;
-  if (groups_per_cta > dec::kSZGroups) return false;
+  if (dec::split_of(p).groups > dec::kSZGroups) return false;      // staged in shared memory
   if (p.epilogue == B200_EPI_SILU_MUL && ((p.N / kTileN) & 1)) return false;
   if (p.epilogue == kEpiRopeKv && p.fe && (kTileN % p.fe->D) != 0) return false;
 #if B200_DEC_GROUPS > 4
