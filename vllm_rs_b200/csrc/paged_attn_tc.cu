@@ -7,7 +7,7 @@
 // that hold kept tokens outside the window, then the window.
 //   S  = Q K^T    fp32 [128 x 64] in TMEM.  Q was rounded to bf16 once: in shared memory (SW128, K-major) or, where the key
 //                 rows are so long that Q and the page ring do not fit together, its first q_tm blocks of 64 in TMEM
-//   P  = softmax  thread = row: options and mask on the fp32 scores, running maximum (the accumulator is rescaled whenever a
+//   P  = softmax  two threads per row, half of a page's keys each: options and mask on the fp32 scores, running maximum (the accumulator is rescaled whenever a
 //                 row's maximum grows: letting it lag by up to 2^8 saves 3 - 10 % of the time, but the largest weight of a
 //                 row then is not 1 and is rounded like the others, 4 - 8 % more error against 64 bits), bf16 P to TMEM.
 //                 Steps of few rows take every page's own maximum: its largest weight is exact then, as the largest of every
@@ -15,17 +15,19 @@
 //                 0.00280 with the running maximum, 0.00276 with 16 splits, 0.00268 here; 59 -> 62 us)
 //   O += P V      fp32 [128 x up to 256] in TMEM; V = page as an MN-major operand
 // Warp 0 fetches pages by block-table index (TMA, K ring | V ring), warp 1 issues the MMAs (S of page j + 1 before P V of
-// page j), warps 2-5 own the rows.  Latent rows (kv_rank 512: O would need all 512 TMEM columns) are walked in passes of up to
+// page j), warps 2-9 own the rows: two warps share 32 of them, exchange their halves' maxima in shared memory at a barrier of the
+// two, and rescale and write half of the columns each.  (One thread per row has a page's 64 scores in one chain of waits: 98 / 62 / 680
+// us for the three cases below where two take 90 / 58 / 577.  More warps also stage the queries faster.)  Latent rows (kv_rank 512: O would need all 512 TMEM columns) are walked in passes of up to
 // 256 value columns; the scores are computed again in every pass (1.5x the products, still far from the 8 mma.sync
 // warps' rate that made 128-row tiles of 16 rows x 1 head re-read every page 64 times).  In a pass the page blocks that are
 // also values stay until P V has read them (V ring), the rest is released after S (K ring).
 //
 // Bound: tensor cores for prompts (per page 2 * 128 * 64 * (dim * passes + vdim) flop against 64 * dim * 2 bytes from L2),
 // HBM for steps of few rows, whose keys are split over blocks; window_attn_merge / latent_attn_merge then finish.
-// Measured, mma.sync kernels -> here: window 1024, 4096 rows, 16 heads of 128 over 4: 622 -> 98 us (305 TFLOP/s; what bounds it
-// is the softmax warps' issue slots, then the start and the drain of 128 blocks); latent, 2 x 2048 rows, 32 heads, rank 512:
-// 7766 -> 678 us (441 TFLOP/s useful, 668 issued); 32 tokens over 2048 keys, 32 heads over 8: 317 -> 62 us (35 at HBM rate): 256 blocks
-// of 33 pages in turn, with four rows in one of the four row warps.
+// Measured, mma.sync kernels -> here: window 1024, 4096 rows, 16 heads of 128 over 4: 622 -> 90 us (332 TFLOP/s; what bounds it
+// is the softmax warps, then the start and the drain of 128 blocks); latent, 2 x 2048 rows, 32 heads, rank 512:
+// 7766 -> 577 us (518 TFLOP/s useful, 785 issued); 32 tokens over 2048 keys, 32 heads over 8: 317 -> 58 us (35 at HBM rate): 256 blocks
+// of 33 pages in turn, with four rows in one pair of the row warps.
 #include "paged_attn_tc.cuh"
 
 #include <algorithm>
@@ -34,7 +36,8 @@ namespace b200 {
 using namespace seqmix;
 namespace hat {
 
-constexpr int kRows = 128, kTok = 64, kThreads = 192;
+constexpr int kRows = 128, kTok = 64, kRowWarps = 8, kThreads = 64 + kRowWarps * 32;
+constexpr int kHalf = kTok / 2;           // keys of a page (and half of a pass's columns) that one of a row's two threads has
 constexpr int kBlk = kTok * 128;          // a page's 64 x 64 block: 64 swizzled rows of 128 bytes
 constexpr int kTailBlk = kTok * 64;       // the last 32 columns: 64 rows of 64 bytes
 constexpr int kQBlk = kRows * 128, kQTail = kRows * 64;
@@ -197,12 +200,12 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
   const int nwarps = (nrows + 31) / 32;                      // row warps that have a row
   const int vcols = a.vblk * 64;                             // value columns of a pass (the last one may have fewer)
 
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* q_smem = smem;
   uint8_t* k_smem = q_smem + a.q_bytes;
   uint8_t* v_smem = k_smem + a.sk * a.k_stage;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(v_smem + a.sv * a.v_stage);
+  float* s_max = reinterpret_cast<float*>(v_smem + a.sv * a.v_stage);       // [page parity][half of the keys][row]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(s_max + 4 * kRows);
   uint64_t* k_full = bars;
   uint64_t* k_empty = k_full + kMaxStages;
   uint64_t* v_full = k_empty + kMaxStages;
@@ -216,6 +219,10 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
   uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(q_full + 6);
   volatile int* fail = reinterpret_cast<volatile int*>(tmem_ptr + 1);
 
+  if (smem_u32(smem) & 1023) {             // the swizzles' atoms; dynamic shared memory without static one begins on them
+    if (threadIdx.x == 0) *reinterpret_cast<volatile int*>(a.err) = 1;
+    return;
+  }
   if (n <= 0) {                            // a split without keys leaves an empty part
     for (int e = threadIdx.x; e < nrows * a.ppc * vcols; e += kThreads) {
       const int r = e / (a.ppc * vcols), c = pass0 * vcols + e % (a.ppc * vcols);
@@ -232,10 +239,10 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
   if (threadIdx.x == 0) {
     for (int s = 0; s < a.sk; ++s) { mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 1); }
     for (int s = 0; s < a.sv; ++s) { mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 1); }
-    mbar_init(q_full, 4);
+    mbar_init(q_full, kRowWarps);
     mbar_init(s_full, 1);
-    mbar_init(s_free, nwarps);
-    mbar_init(p_full, nwarps);
+    mbar_init(s_free, 2 * nwarps);
+    mbar_init(p_full, 2 * nwarps);
     mbar_init(pv_done, 1);
     mbar_init(drained, 1);
     *fail = 0;
@@ -382,13 +389,16 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
     __syncwarp();
   } else {
     // ------------------------------------------------------------ rows
-    const int q4 = warp & 3, r = q4 * 32 + lane;             // row = TMEM lane
+    // row = TMEM lane; the warps q4 and q4 + 4 share 32 rows: a thread has half of a page's keys and half of the columns
+    const int q4 = warp & 3, hf = (warp - 2) >> 2, r = q4 * 32 + lane;
+    auto meet = [&] { asm volatile("bar.sync %0, 64;" ::"r"(2 + q4) : "memory"); };
+    constexpr int kRowThreads = kRowWarps * 32;
     const int tid = threadIdx.x - 64;
     const uint32_t lane_base = static_cast<uint32_t>(q4 * 32) << 16;
     // ---- stage Q as bf16: coalesced 32-byte reads, chunks of 8 entries
     {
       const int cpr = p.dim / 8;
-      const int dr = kRows / cpr, dc = kRows % cpr;          // what 128 chunks on are: dr rows and dc chunks
+      const int dr = kRowThreads / cpr, dc = kRowThreads % cpr;          // what 256 chunks on are: dr rows and dc chunks
       int row = tid / cpr, c = tid % cpr;
       while (row < kRows) {
         constexpr int U = 8;                                 // chunks in flight per thread: 32 KB per block
@@ -432,8 +442,8 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
       }
       __syncwarp();
       if (a.q_tm) {
-        asm volatile("bar.sync 1, 128;" ::: "memory");
-        for (int blk = 0; blk < a.q_tm; ++blk) {
+        asm volatile("bar.sync 1, %0;" ::"n"(kRowThreads) : "memory");
+        for (int blk = hf; blk < a.q_tm; blk += 2) {
           uint32_t w[32];
           const uint8_t* src = k_smem + blk * kQBlk + r * 128;          // (eight lanes' rows lie in different banks)
 #pragma unroll
@@ -473,7 +483,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
     const int passes = q4 < nwarps ? a.ppc : 0;              // a warp without rows is done
     for (int pi = 0; pi < passes; ++pi) {
       // A sink below every score that counts is no sink (and -inf as a reference makes NaN of a page without a visible key).
-      float m_ref = with_sink && valid ? p.sink[h] * kLog2e : kNone, l = with_sink ? 1.f : 0.f;
+      float m_ref = with_sink && valid ? p.sink[h] * kLog2e : kNone, l = with_sink && hf == 0 ? 1.f : 0.f;      // (l: of this half)
       if (m_ref < kNone) {
         m_ref = kNone;
         l = 0.f;
@@ -481,37 +491,33 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
       float m_top = m_ref;                                   // the largest score so far; m_ref where the reference never falls
       const int vn = v_count(pass0 + pi);
       for (int j = 0; j < n; ++j, ++it) {
-        const int base = page_of(j0 + j) * kTok;
+        const int page0 = page_of(j0 + j) * kTok, base = page0 + hf * kHalf;        // first key of the page, of this half
         mbar_wait_limited(s_full, it & 1, fail, a.err);
         __syncwarp();
         tc_fence_after();
-        uint32_t v0[32], v1[32];
-        tmem_ld_x32(s_tm + lane_base, v0);
-        tmem_ld_x32(s_tm + lane_base + 32, v1);
+        uint32_t v0[kHalf];
+        tmem_ld_x32(s_tm + lane_base + hf * kHalf, v0);
         tc_wait_ld();
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(s_free);
-        float x[kTok];
+        float x[kHalf];
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          x[i] = __uint_as_float(v0[i]);
-          x[32 + i] = __uint_as_float(v1[i]);
-        }
+        for (int i = 0; i < kHalf; ++i) x[i] = __uint_as_float(v0[i]);
         // x times `mult` is the score; keys outside the mask become -inf
         float mult = sl;
         if (CAP) {
           float big0 = fabsf(x[0]), big1 = fabsf(x[1]);
 #pragma unroll
-          for (int i = 2; i < kTok - 2; i += 4) {
+          for (int i = 2; i < kHalf - 2; i += 4) {
             big0 = max3(big0, fabsf(x[i]), fabsf(x[i + 1]));
             big1 = max3(big1, fabsf(x[i + 2]), fabsf(x[i + 3]));
           }
-          big0 = max3(big0, fabsf(x[kTok - 2]), fabsf(x[kTok - 1]));
+          big0 = max3(big0, fabsf(x[kHalf - 2]), fabsf(x[kHalf - 1]));
           mult = cap2;
           if (__all_sync(0xffffffffu, fmaxf(big0, big1) * sl <= kTanhMax)) {
 #pragma unroll
-            for (int i = 0; i < kTok; i += 2) {
+            for (int i = 0; i < kHalf; i += 2) {
               const f2 y = mul2(pack2(x[i], x[i + 1]), pack2(sl, sl)), t = mul2(y, y);
               f2 q = fma2(t, pack2(kT5, kT5), pack2(kT4, kT4));
               q = fma2(t, q, pack2(kT3, kT3));
@@ -523,10 +529,10 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
           } else {
             // The same products one by one, and tanh(y) = 1 - 2 / (e^(2 y) + 1) past kTanhMax.  Which form a score takes is its
             // own affair: a row's bits do not depend on the rows and heads that share its warp.  (The packed products here too,
-            // or a choice per row, made the path above slower: 101 and 107 instead of 99 us for a prompt of 4096.)
+            // or a choice per row, made the path above slower: 101 and 107 instead of 99 us for a prompt of 4096, with one thread per row.)
             const float e2 = sl * (2.f * kLog2e);
 #pragma unroll
-            for (int i = 0; i < kTok; ++i) {
+            for (int i = 0; i < kHalf; ++i) {
               const float y = __fmul_rn(x[i], sl), t = __fmul_rn(y, y);
               float q = fmaf(t, kT5, kT4);
               q = fmaf(t, q, kT3);
@@ -539,28 +545,33 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
         }
         if (BIAS) {
           const float d0 = static_cast<float>(pos - base);
-          if (table && pos - (base + kTok - 1) < p.dist_n - 1) {
+          if (table && pos - (base + kHalf - 1) < p.dist_n - 1) {
 #pragma unroll
-            for (int i = 0; i < kTok; ++i)
+            for (int i = 0; i < kHalf; ++i)
               x[i] = fmaf(x[i], mult, fmaf(-slope, d0 - i, __ldg(table + max(0, min(pos - base - i, p.dist_n - 1))) * kLog2e));
           } else {
 #pragma unroll
-            for (int i = 0; i < kTok; ++i) x[i] = fmaf(x[i], mult, fmaf(-slope, d0 - i, far_bias));
+            for (int i = 0; i < kHalf; ++i) x[i] = fmaf(x[i], mult, fmaf(-slope, d0 - i, far_bias));
           }
           mult = 1.f;
         }
-        if (base + kTok - 1 > pos0 || base < lo_last) {       // the diagonal, the window's edge, kept tokens
+        if (page0 + kTok - 1 > pos0 || page0 < lo_last) {       // the diagonal, the window's edge, kept tokens
           const int last = pos - base, first = lo - base, kept = p.keep_first - base;
 #pragma unroll
-          for (int i = 0; i < kTok; ++i) x[i] = i <= last && (i >= first || i < kept) ? x[i] : -INFINITY;
+          for (int i = 0; i < kHalf; ++i) x[i] = i <= last && (i >= first || i < kept) ? x[i] : -INFINITY;
         }
         float mx0 = max3(x[0], x[1], x[2]), mx1 = max3(x[3], x[4], x[5]);
 #pragma unroll
-        for (int i = 6; i < kTok - 2; i += 4) {
+        for (int i = 6; i < kHalf - 2; i += 4) {
           mx0 = max3(mx0, x[i], x[i + 1]);
           mx1 = max3(mx1, x[i + 2], x[i + 3]);
         }
-        const float mx = max3(mx0, mx1, fmaxf(x[kTok - 2], x[kTok - 1])) * mult;
+        // of both halves (a place is written again two pages later, behind the barrier of the page between)
+        const float own = max3(mx0, mx1, fmaxf(x[kHalf - 2], x[kHalf - 1]));
+        float* const top = s_max + (it & 1) * 2 * kRows + r;
+        top[hf * kRows] = own;
+        meet();
+        const float mx = fmaxf(own, top[(hf ^ 1) * kRows]) * mult;
         float corr = 1.f;
         bool grow = false;
         m_top = fmaxf(m_top, mx);
@@ -570,9 +581,9 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
           grow = true;
         }
         float sum[4] = {0.f, 0.f, 0.f, 0.f};
-        uint32_t pk[32];
+        uint32_t pk[kHalf / 2];
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
+        for (int i = 0; i < kHalf / 2; ++i) {
           const float p0 = ex2(fmaf(x[2 * i], mult, -m_ref)), p1 = ex2(fmaf(x[2 * i + 1], mult, -m_ref));
           pk[i] = pack16x2<true>(p0, p1);
           sum[(2 * i) & 3] += p0;
@@ -581,12 +592,12 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
         l = fmaf(l, corr, (sum[0] + sum[1]) + (sum[2] + sum[3]));
         // Value rows past the tile's last token may hold anything (later tokens, and what lies behind the sequence), and 0 * NaN
         // is no 0; a single token does not even meet the rows before its window.
-        const int v_end = pos_last + 1 - base, v_lo = nt == 1 && base + kTok > p.keep_first ? key_lo - base : 0;
+        const int v_end = pos_last + 1 - page0, v_lo = nt == 1 && page0 + kTok > p.keep_first ? key_lo - page0 : 0;
         if (v_end < kTok || v_lo > 0) {
           mbar_wait_limited(&v_full[vr.s], vr.ph, fail, a.err);
           uint8_t* vt = v_smem + vr.s * a.v_stage + (r & 7) * 16;
-          for (int row = r >> 3; row < kTok; row += nwarps * 4)
-            if (row >= v_end || (row < v_lo && base + row >= p.keep_first))
+          for (int row = (r >> 3) + hf * nwarps * 4; row < kTok; row += nwarps * 8)
+            if (row >= v_end || (row < v_lo && page0 + row >= p.keep_first))
               for (int i = 0; i < vn; ++i) *reinterpret_cast<uint4*>(vt + i * kBlk + row * 128) = make_uint4(0, 0, 0, 0);
           fence_proxy_async();
         }
@@ -597,7 +608,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
           tc_fence_after();
           if (j > 0 && __any_sync(0xffffffffu, grow)) {
 #pragma unroll 1
-            for (int c0 = 0; c0 < vn * 64; c0 += 32) {
+            for (int c0 = hf * vn * 32; c0 < (hf + 1) * vn * 32; c0 += 32) {
               uint32_t o[32];
               tmem_ld_x32(o_tm + lane_base + c0, o);
               tc_wait_ld();
@@ -607,7 +618,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
             }
           }
         }
-        tmem_st32(p_tm + lane_base, pk);
+        tmem_st_x16(p_tm + lane_base + hf * (kHalf / 2), pk);
         tc_wait_st();
         tc_fence_before();
         __syncwarp();
@@ -619,11 +630,16 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
       // ---- the pass's columns of this row
       const size_t trow = static_cast<size_t>(row0 + tl), orow = trow * p.heads + h;
       const int col0 = v_first(pass0 + pi) * 64;
+      float* const sums = s_max + (it & 1) * 2 * kRows + r;              // (last read before the last page's barrier)
+      sums[hf * kRows] = l;
+      meet();
+      l = sums[0] + sums[kRows];
+      meet();
       float inv = l > 0.f ? 1.f / l : 0.f;
       if (p.nsplit == 1 && p.gate && !p.gate_elems && valid) inv *= sigmoid_f(p.gate[trow * p.ld_gate + h]);
       const float* ge = p.gate && p.gate_elems ? p.gate + trow * p.ld_gate + static_cast<size_t>(h) * p.vdim + col0 : nullptr;
 #pragma unroll 1
-      for (int c0 = 0; c0 < vn * 64; c0 += 32) {
+      for (int c0 = hf * vn * 32; c0 < (hf + 1) * vn * 32; c0 += 32) {
         uint32_t o[32];
         tmem_ld_x32(o_tm + lane_base + c0, o);
         tc_wait_ld();
@@ -657,7 +673,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
         }
         __syncwarp();
       }
-      if (p.nsplit > 1 && valid && col0 == 0) {
+      if (p.nsplit > 1 && valid && col0 == 0 && hf == 0) {
         float* ml = p.part_ml + (orow * p.nsplit + sp) * 2;
         ml[0] = m_ref * kLn2;
         ml[1] = l;
@@ -673,7 +689,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
   }
 }
 
-constexpr int kSmemMax = 227 * 1024, kBarBytes = 256, kAlign = 1024;
+constexpr int kSmemMax = 227 * 1024, kBarBytes = 256 + 4 * kRows * 4;       // (and the rows' maxima)
 
 // Sizes of one launch; false: the shape does not fit.
 static bool plan(const AttnTcProblem& p, Args& a) {
@@ -701,7 +717,7 @@ static bool plan(const AttnTcProblem& p, Args& a) {
       a.sk = 2;
       a.q_bytes = (a.kblk - a.q_tm) * kQBlk + a.tail * kQTail;
       const int rings = a.sk * a.k_stage + a.sv * a.v_stage;
-      if (a.q_bytes + rings + kBarBytes + kAlign > kSmemMax) continue;
+      if (a.q_bytes + rings + kBarBytes > kSmemMax) continue;
       if (a.q_tm * kQBlk > rings) continue;
       const int cols = a.vblk * 64 + 96 + a.q_tm * 32;
       a.tmem_cols = cols <= 128 ? 128 : (cols <= 256 ? 256 : 512);
@@ -763,7 +779,7 @@ void launch_attn_tc(const AttnTcProblem& p, cudaStream_t st) {
     set_error(2, "attn_tc: cuTensorMapEncodeTiled failed");
     return;
   }
-  const int smem = a.q_bytes + a.sk * a.k_stage + a.sv * a.v_stage + kBarBytes + kAlign;
+  const int smem = a.q_bytes + a.sk * a.k_stage + a.sv * a.v_stage + kBarBytes;
   const int tiles = (p.T + a.tq - 1) / a.tq + p.num_seqs;
   // all passes in one block (Q is staged once) where that still gives every SM two blocks; otherwise a block per pass
   a.page_ref = attn_few_rows(p.T);
