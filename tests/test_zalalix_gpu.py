@@ -228,6 +228,42 @@ def test_window_attention_prep_op(lib):
         assert torch.allclose(vc.cpu()[s // 64, s % 64].double(), wv[t], atol=2e-5)
 
 
+@pytest.mark.parametrize("T,H,G,dk,dv,rd,bias,norm,bf16,vk,extra", [
+    (37, 16, 4, 128, 128, 64, True, True, True, False, 16),       # the rows a hybrid step has, part of a head rotated
+    (5, 32, 8, 128, 128, 128, True, True, True, False, 0),        # four queries of a thread, the largest table of rotations
+    (9, 4, 2, 64, 96, 34, False, True, False, False, 4),          # half a group of four rotated
+    (3, 8, 8, 32, 32, 30, True, False, True, True, 8),            # values taken from the keys
+    (1, 2, 1, 4, 8, 2, False, False, False, False, 0),            # threads without an entry
+    (64, 12, 12, 64, 64, 0, True, True, True, False, 0)])         # no rotation
+def test_window_attn_prep_aligned_rows_match_unaligned(lib, T, H, G, dk, dv, rd, bias, norm, bf16, vk, extra):
+    """Projections that lie on 16 bytes are read four entries at a time; a view that starts one float further on takes the
+    general form.  The sums of squares meet in another order, so fp32 may differ by a few roundings of them (2e-6 of an entry of
+    up to the largest value) and bf16 by one step of the larger entry (2^-7)."""
+    from vllm_rs_b200 import ops
+    g = torch.Generator().manual_seed(T)
+    nq, nk, nv = H * dk, G * dk, 0 if vk else G * dv
+    n, ld, dt = nq + nk + nv, nq + nk + nv + extra, torch.bfloat16 if bf16 else torch.float32
+    proj = torch.randn(T, ld, generator=g).cuda()
+    b = torch.randn(n, generator=g).cuda() if bias else None
+    qn, kn = (torch.randn(nq, generator=g).cuda(), torch.randn(nk, generator=g).cuda()) if norm else (None, None)
+    f = 10000.0 ** (-torch.arange(max(1, rd // 2), dtype=torch.float64) / max(1, rd // 2)).cuda()
+    pos, slots = torch.randint(0, 5000, (T,), generator=g).cuda(), torch.randperm(128, generator=g)[:T]
+    if T > 4:
+        slots[3] = -1                                             # a row that is not kept
+    got = []
+    for off in (0, 1):
+        at = torch.empty(T * ld + 1, device="cuda")[off:off + T * ld].view(T, ld)
+        at.copy_(proj)
+        kc = torch.zeros(2, 64, G, dk, device="cuda", dtype=dt)
+        vc = torch.zeros(2, 64, G, dv, device="cuda", dtype=dt)
+        q = ops.window_attn_prep(at, b, qn, kn, f, pos, slots.cuda(), kc, vc, heads=H, rot_dims=rd, eps=1e-6,
+                                 v_from_k=vk, q_temp=(0.3, 100), rot_mag=1.1)
+        got.append((q, kc, vc))
+    for x, y in zip(*got):
+        top = max(1.0, y.float().abs().max().item())
+        assert (x.float() - y.float()).abs().max().item() <= (2.0 ** -7 if x.dtype == torch.bfloat16 else 2e-6) * top
+
+
 @pytest.mark.parametrize("window,keep", [(3, 2), (64, 5), (65, 64)])
 def test_model_edges_show_in_logits(lib, window, keep):
     """A one-layer model whose recurrent side is switched off: replacing the token at one place changes the last row's
