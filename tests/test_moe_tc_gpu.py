@@ -79,3 +79,21 @@ def test_same_bits_in_steps_of_any_size(lib, act, E, D, F):
     run = lambda n: ops.moe_experts_ex(x[:n].clone(), h[:n], idx[:n], w[:n], wu, wd, act=act)      # noqa: E731
     few, many = run(70), run(T)
     assert torch.equal(few, many[:70])
+
+
+@pytest.mark.parametrize("T,E,top", [(4096, 33, 4), (4097, 33, 4), (13000, 70, 3)])
+def test_buckets_of_many_pairs(lib, T, E, top):
+    """The sort keeps up to 16 384 pairs in registers and walks more of them in several rounds: every row of a large step has the
+    bits that it has in a portion of 1000 rows, as sums are taken in the order of a token's choices."""
+    from vllm_rs_b200 import ops
+    g = torch.Generator().manual_seed(T)
+    c = lambda t: t.cuda().contiguous()                                      # noqa: E731
+    D, F = 64, 32
+    wu, wd = c(torch.randn(E, 2 * F, D, generator=g).bfloat16()), c(torch.randn(E, D, F, generator=g).bfloat16())
+    h, z, x = c(torch.randn(T, D, generator=g).bfloat16()), torch.randn(T, E, generator=g), torch.zeros(T, D).cuda()
+    w, idx = torch.softmax(z, 1).topk(top, 1)
+    w, idx = c(w), c(idx.int())
+    run = lambda a, b: ops.moe_experts_ex(x[a:b].clone(), h[a:b], idx[a:b], w[a:b], wu, wd, act="silu_gate")      # noqa: E731
+    whole = run(0, T)
+    assert torch.equal(whole, torch.cat([run(a, min(a + 1000, T)) for a in range(0, T, 1000)]))
+    assert whole.abs().sum() > 0
