@@ -66,7 +66,8 @@ __device__ __forceinline__ void commit(uint32_t lead, uint64_t* bar) {
 // ACT as in moe.cu: 0 plain product, fp32 out; 1 SiLU gate, 2 squared ReLU, 3 clamped gate, bf16 out.  Rows in bucket order.  After a wait has given up (*fail) all others return at once and the loops run out.
 template <int ACT, int BN>
 __global__ void __launch_bounds__(kThreads, 1)
-grouped_linear_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap wmap, const Args a) {
+grouped_linear_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap tilemap,
+                         const __grid_constant__ CUtensorMap wmap, const Args a) {
   constexpr bool GATED = ACT == 1 || ACT == 3;
   constexpr int FN = GATED ? BN / 2 : BN;          // output features of a tile
   using C = Cfg<BN>;
@@ -89,6 +90,7 @@ grouped_linear_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_
     *fail = 0;
     fence_barrier_init();
     prefetch_tmap(&amap);
+    prefetch_tmap(&tilemap);
     prefetch_tmap(&wmap);
   }
   if (warp == 1) {
@@ -151,7 +153,9 @@ grouped_linear_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_
           } else {
             tma_load_2d(wd, &wmap, &full[s], kb * kK, wrow);
           }
-          for (int i = 0; i < boxes; ++i) tma_load_2d(ad + i * (kBox * 128), &amap, &full[s], kb * kK, w.s0 + i * kBox);
+          if (boxes == kM / kBox) tma_load_2d(ad, &tilemap, &full[s], kb * kK, w.s0);      // a copy costs its issue, whatever its size
+          else
+            for (int i = 0; i < boxes; ++i) tma_load_2d(ad + i * (kBox * 128), &amap, &full[s], kb * kK, w.s0 + i * kBox);
         }
         ++armed;
         if (++s == C::kStages) { s = 0; ph ^= 1; }
@@ -286,8 +290,9 @@ static void launch(void* out, const void* a, const void* w, const int32_t* off, 
   constexpr bool GATED = ACT == 1 || ACT == 3;
   constexpr int FN = GATED ? BN / 2 : BN;
   Args g{out, off, E, (K + kK - 1) / kK, N, (N + FN - 1) / FN, act, wait_error_flag()};
-  CUtensorMap amap, wmap;
-  const bool ok = map_2d(&amap, a, pairs, K, kBox) && map_2d(&wmap, w, static_cast<uint64_t>(E) * (GATED ? 2 : 1) * N, K, FN);
+  CUtensorMap amap, tilemap, wmap;
+  const bool ok = map_2d(&amap, a, pairs, K, kBox) && map_2d(&tilemap, a, pairs, K, kM) &&
+                  map_2d(&wmap, w, static_cast<uint64_t>(E) * (GATED ? 2 : 1) * N, K, FN);
   if (!ok || !g.err) {
     set_error(2, "grouped_linear_tc: cuTensorMapEncodeTiled failed");
     return;
@@ -296,7 +301,7 @@ static void launch(void* out, const void* a, const void* w, const int32_t* off, 
   static OncePerDevice sized;
   if (!allow_smem(sized, kern, Cfg<BN>::kSmem)) return;
   const int most = std::min(pairs, E + pairs / kM) * g.ntiles_n;        // no step has more tiles
-  kern<<<std::min(most, sm_count()), kThreads, Cfg<BN>::kSmem, st>>>(amap, wmap, g);
+  kern<<<std::min(most, sm_count()), kThreads, Cfg<BN>::kSmem, st>>>(amap, tilemap, wmap, g);
   B200_CUDA_LAUNCH_CHECK();
 }
 
