@@ -2,15 +2,16 @@
 // formulas, the buckets and the fp32 / odd-size forms).
 //
 // Persistent blocks, one per SM, walk tiles of 128 slots (rows of ONE expert's bucket) x BN weight rows.  Warp 0 fetches 64-wide
-// K blocks of both operands by TMA, of the rows only as many 32-row boxes as the bucket has.  Warp 1 issues the products into
+// K blocks of both operands by TMA, of the rows only as many 32-row boxes as the bucket has, a full tile as one
+// box (the two products of the prompt below: 75 / 52 -> 71 / 51 us).  Warp 1 issues the products into
 // one of two TMEM accumulators, warps 2-9 apply the activation and store, through shared memory so that rows leave in whole
 // sectors, under the products of the next tile.  A gated tile holds BN / 2 gate and BN / 2 up rows of the same features side by
 // side, so the activation needs no second pass.  Token rows are first gathered into bucket order by a copy of their own (in
 // space that the second product's results take later): gathering inside the product took longer than the product, by TMA
 // gathers of four rows (~90 cycles each) as by cp.async, whose blocks need a wait and a fence on their way to the tensor core
-// (prompt of 4096 rows, 16 experts, first product: 183 us and 103-139 us).
+// (prompt of 4096 rows, 16 experts, first product: 183 us and 103-139 us).  Pairs of blocks on 256 x 256 tiles: 67.5 / 55.4 us.
 //
-// Measured, mma.sync kernel -> here (whole call): 4096 rows of 2048, 16 experts of 512, 4 chosen: 709 -> 195 us, 32 rows, device time,
+// Measured, mma.sync kernel -> here (whole call): 4096 rows of 2048, 16 experts of 512, 4 chosen: 709 -> 194 us, 32 rows, device time,
 // 67 -> 36; 4096 wide, 32 experts of 1024: 3000 rows 1903 -> 406 us, 32 rows, device time, 202 -> 159.  moe.cu says which products are
 // long enough to come here.
 // Bound: tensor cores where experts get hundreds of rows, HBM (every hit expert's weights once) where they get few; BN is 256
