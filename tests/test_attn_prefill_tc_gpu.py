@@ -91,3 +91,39 @@ def test_attn_prefill_tc_lazy_rescale_and_long_rows(ops):
     assert bool((err <= 3e-3 + 3e-3 * ref.float().abs()).all()), float(err.max())
     # the default dispatch is the tcgen05 kernel: identical bits
     assert torch.equal(out, ops.attention_prefill(*args).float().cpu())
+
+
+@pytest.mark.parametrize("warp", range(4))
+@pytest.mark.parametrize("dt,l1", [(F16, False), (F16, True), (torch.bfloat16, False), (torch.bfloat16, True)])
+def test_attn_prefill_tc_one_warp_rescales_at_every_page(ops, dt, l1, warp):
+    """Every tile's rows of ONE softmax warp (8 of 32 tokens, four heads each) meet keys whose scores grow by some 2^10 a page,
+    so that this warp rescales at every page; the other rows' queries are at right angles to what grows, and their warps run ahead.
+    fp64 reference from the rounded operands; the bounds of the other tests of this kernel (weights and results of 16 bits)."""
+    H, Hkv, D, n, past = 32, 8, 128, 323, 1000
+    ctx, scale = n + past, 1.0 / math.sqrt(D)
+    pages = -(-ctx // 64)
+    g = torch.Generator().manual_seed(warp)
+    u = torch.randn(D, generator=g)
+    u /= u.norm()
+    q, k = torch.randn(n, H, D, generator=g), torch.randn(ctx, Hkv, D, generator=g)
+    q -= (q @ u)[..., None] * u
+    q[torch.arange(n) % 32 // 8 == warp] += 32 * u
+    k += (2.5 * (torch.arange(ctx) // 64))[:, None, None] * u
+    q, k, v = q.to(dt), k.to(dt), torch.randn(ctx, Hkv, D, generator=g).to(dt)
+    s = torch.einsum("thd,chd->htc", q.double(), k.double().repeat_interleave(H // Hkv, 1)) * scale
+    s += torch.full((n, ctx), float("-inf"), dtype=torch.float64).triu(past + 1)
+    ref = torch.einsum("htc,chd->thd", torch.softmax(s, -1), v.double().repeat_interleave(H // Hkv, 1))
+    order = torch.randperm(pages + 2, generator=g)[:pages]
+    kc, vc = (torch.full((pages + 2, 64, Hkv, D), float("nan"), dtype=dt) for _ in range(2))
+    for at, t in ((kc, k), (vc, v)):
+        for p in range(pages):
+            rows = t[p * 64:(p + 1) * 64]
+            at[order[p], :len(rows)] = rows
+    if l1:
+        kc, vc = om.to_l1_layout(kc, vc)
+    out = ops.attention_prefill(q.cuda(), kc.cuda(), vc.cuda(), torch.tensor([0, n], dtype=torch.int32).cuda(),
+                                torch.tensor([ctx], dtype=torch.int32).cuda(), order.int()[None].contiguous().cuda(), n, scale,
+                                mode=ops.ATTN_TC).double().cpu()
+    tol = 2e-3 if dt == F16 else 1.6e-2
+    assert not torch.isnan(out).any()
+    assert bool(((out - ref).abs() <= tol + tol * ref.abs()).all()), float((out - ref).abs().max())

@@ -157,8 +157,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_co
   uint64_t* v_empty = bars + 7;        // [2]
   uint64_t* s_full = bars + 9;
   uint64_t* s_free = bars + 10;
-  uint64_t* p_full = bars + 11;
-  uint64_t* pv_done = bars + 12;       // [2], of even and odd pages
+  uint64_t* p_full = bars + 11;        // [2], of even and odd pages: a row warp stores P of a page while another one is still at the
+                                       // page before, and on one barrier would count twice in its phase
+  uint64_t* pv_done = bars + 13;       // [2]
   uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(smem + kTmemPtrOff);
 
   if (threadIdx.x == 0) {
@@ -171,9 +172,10 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_co
     }
     mbar_init(s_full, 1);
     mbar_init(s_free, 4);
-    mbar_init(p_full, 4);
-    mbar_init(&pv_done[0], 1);
-    mbar_init(&pv_done[1], 1);
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&p_full[s], 4);
+      mbar_init(&pv_done[s], 1);
+    }
     fence_barrier_init();
     prefetch_tmap(&qmap);
     prefetch_tmap(&kmap);
@@ -267,7 +269,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_co
       for (int j = 0; j < npages; ++j) {
         if (j + 1 < npages) issue_qk(j + 1);
         const int s = j & 1;
-        mbar_wait_bounded(p_full, j & 1);
+        mbar_wait_bounded(&p_full[s], (j >> 1) & 1);
         mbar_wait_bounded(&v_full[s], (j >> 1) & 1);
         tc_fence_after();
         const uint32_t v_addr = smem_u32(kv_smem + s * kStageBytes + kTileBytes);
@@ -407,7 +409,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_co
         tc_wait_st();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(p_full);
+        if (lane == 0) mbar_arrive(&p_full[j & 1]);
       };
       // (asking and taking stay in one branch: nothing is copied between)
       if (j + 1 == npages) {
