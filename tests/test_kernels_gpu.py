@@ -334,6 +334,30 @@ def test_wna16_decode_of_few_tokens(ops, fmt, bits, K, N, M, group, epi):
         assert e_new <= e_old * 1.05, (e_new, e_old)               # the same weights, sums in another order
 
 
+@pytest.mark.parametrize("M", [1, 16])
+def test_wna16_decode_of_more_than_65536_units(ops, M):
+    """Sizes at which a product by the number of all units does not fit 32 bits (wna16_mma.cu, ranges cut anywhere): every tile is
+    written, and the counters are back at rest.  fp32 sums of the weights rounded to fp16, a group of 128 K at a time."""
+    K, N = 34944, 30848
+    g = torch.Generator(device="cuda").manual_seed(M)
+    words = lambda r: torch.randint(-2 ** 31, 2 ** 31, (r, N // 8), generator=g, device="cuda", dtype=torch.int64).int()      # noqa: E731
+    qw, qz = words(K), words(K // 128)
+    s = (0.005 + 0.01 * torch.rand(K // 128, N, generator=g, device="cuda")).to(F16)
+    x = (0.05 * torch.randn(M, K, generator=g, device="cuda")).to(F16)
+    at = torch.tensor([4 * j for j in (0, 4, 1, 5, 2, 6, 3, 7)], device="cuda", dtype=torch.int32)      # nibble of output 8 c + i
+    nib = lambda w: ((w[..., None] >> at) & 15).reshape(w.shape[0], N)              # noqa: E731
+    ref = torch.zeros(M, N, device="cuda", dtype=torch.float64)
+    for i in range(K // 128):
+        rows = slice(i * 128, i * 128 + 128)
+        w = ((nib(qw[rows]) - nib(qz[i:i + 1])).to(F16) * s[i]).float()
+        ref += (x[:, rows].float() @ w).double()
+    packed, ws = ops.awq_prepack(qw), ops.wna16_workspace(16, N)
+    for variant in (7, 0):
+        y = ops.wna16_gemm(x, packed, s, qz, ws, k=K, n=N, bits=4, group_size=128, qfmt=ops.QFMT_AWQ, variant=variant)
+        _close(y, ref.cpu(), 2e-3, 2e-3)
+        assert int(ws[:16384].view(torch.int32).abs().sum()) == 0
+
+
 @pytest.mark.parametrize("K,N,M,group", [(4096, 9728, 17, 64), (8192, 9728, 33, 64), (8192, 1280, 64, 128)])
 def test_wna16_decode_of_many_groups(ops, K, N, M, group):
     """wna16_tc_dec.cu where one K piece has exactly as many quantisation groups as are staged, and where it takes more pieces."""

@@ -22,6 +22,7 @@
 #include <cstring>
 
 #include "host/per_device.hpp"
+#include "host/unit_cut.hpp"
 #include "wna16.cuh"
 
 namespace b200 {
@@ -60,26 +61,6 @@ struct Cfg {
   static_assert(kAlloc <= 220 * 1024, "shared memory");
 };
 
-// x / d by one multiplication: m = ceil(2^32 / d) is exact for x * d < 2^32 (the launcher checks); d = 1: m = 0.
-struct Div {
-  uint32_t m;
-  __device__ __forceinline__ int operator()(int x) const { return m ? static_cast<int>(__umulhi(x, m)) : x; }
-};
-// The cut of the units: every `period` of them (a tile, or all there are) goes to `parts` blocks, of which the first `rest`
-// have share + 1 units and the others `share`.
-struct Cut {
-  int period, parts, share, rest;
-  Div by_period, by_parts, by_share, by_more;
-  __device__ __forceinline__ int start(int i) const {
-    const int q = by_parts(i), j = i - q * parts;
-    return q * period + j * share + min(j, rest);
-  }
-  __device__ __forceinline__ int block_of(int unit) const {
-    const int q = by_period(unit), j = unit - q * period, head = rest * (share + 1);
-    return q * parts + (j < head ? by_more(j) : rest + by_share(j - head));
-  }
-};
-
 struct Args {
   const uint8_t* bp;
   const __half* scales;
@@ -90,8 +71,8 @@ struct Args {
   int M, K, N, qfmt;
   int gshift;            // log2(group_size / 128); 30: one group
   int U;                 // units per tile
-  Cut cut;
-  Div by_U;
+  UnitCut cut;
+  UnitDiv by_U;
   int hd_shift;          // log2(head_dim / 2) of the rotated epilogue
   SplitOut o;
 };
@@ -595,32 +576,11 @@ static bool launch_epi(const WnaParams& p, cudaStream_t st) {
       if ((kUnitK << s) == p.group_size) a.gshift = s;
   const int tiles = p.N / kTileN;
   a.U = p.K / kUnitK;
-  const int total = tiles * a.U;
   int grid = sm_count() * C::kBlocks;
   if (grid > kSkSlotCols / (2 * kTileN)) grid = kSkSlotCols / (2 * kTileN);        // two parts per block
-  // Every tile in the same number of parts, at most eight, where that leaves few blocks out: no block has then two tiles.
-  // 4096 x 4096, one token: 8 parts 5.4 us, 4 parts 7.1.  Otherwise ranges cut anywhere.
-  int splits = grid / tiles;
-  if (splits > a.U / kKG) splits = a.U / kKG;
-  if (splits > 8) splits = 8;
-  a.cut.period = total;
-  if (splits >= 1 && (tiles * splits * 100 >= grid * 85 || total < grid * kKG || tiles * 8 < grid)) {
-    grid = tiles * splits;
-    a.cut.period = a.U;
-  }
-  if (grid > total) grid = total;
-  a.cut.parts = a.cut.period == total ? grid : splits;
-  a.cut.share = a.cut.period / a.cut.parts;
-  a.cut.rest = a.cut.period % a.cut.parts;
-  // Div is exact for these
-  const long long widest = a.U > a.cut.share + 1 ? a.U : a.cut.share + 1;
-  if (total * widest >= 1LL << 31 || static_cast<long long>(grid) * a.cut.parts >= 1LL << 31) return false;
-  auto div = [](int d) { return Div{d > 1 ? static_cast<uint32_t>(((1ull << 32) + d - 1) / d) : 0u}; };
-  a.cut.by_period = div(a.cut.period);
-  a.cut.by_parts = div(a.cut.parts);
-  a.cut.by_share = div(a.cut.share);
-  a.cut.by_more = div(a.cut.share + 1);
-  a.by_U = div(a.U);
+  grid = cut_units(tiles, a.U, grid, kKG, a.cut);
+  if (grid == 0) return false;
+  a.by_U = unit_div(a.U);
   a.hd_shift = 6;
   if (p.fe && p.epilogue == kEpiRopeKv) a.hd_shift = p.fe->D == 128 ? 6 : p.fe->D == 64 ? 5 : 4;
   a.o.partials = a.partials; a.o.counters = a.counters; a.o.bias = p.bias; a.o.c = p.c;
