@@ -334,6 +334,24 @@ def test_wna16_decode_of_few_tokens(ops, fmt, bits, K, N, M, group, epi):
         assert e_new <= e_old * 1.05, (e_new, e_old)               # the same weights, sums in another order
 
 
+@pytest.mark.parametrize("off_bias,off_y", [(1, 0), (0, 1), (2, 2)])
+def test_wna16_bias_and_result_off_four_bytes(ops, off_bias, off_y):
+    """As many tiles as SMs: the tile-split kernel writes results one by one, wherever bias and result begin."""
+    K, N, M = 512, 19456, 3
+    qw, qz, s, W, x = _wna_case(K, N, M, "awq", 4, seed=5)
+    bias = torch.randn(N).to(F16)
+    at = torch.zeros(N + 4, dtype=F16)
+    at[off_bias:off_bias + N] = bias
+    y = torch.zeros(M * N + 4, dtype=F16).cuda()
+    ops.wna16_gemm(x.cuda(), ops.awq_prepack(torch.from_numpy(qw).cuda()), torch.from_numpy(s).cuda(), torch.from_numpy(qz).cuda(),
+                   ops.wna16_workspace(16, N), k=K, n=N, bias=at.cuda()[off_bias:off_bias + N],
+                   out=y[off_y:off_y + M * N].view(M, N))
+    _close(y[off_y:off_y + M * N].view(M, N), om.linear(x, W, bias), 2e-3, 2e-3)
+    rest = torch.ones(M * N + 4, dtype=torch.bool)
+    rest[off_y:off_y + M * N] = False
+    assert not y.cpu()[rest].any()
+
+
 @pytest.mark.parametrize("M", [1, 16])
 def test_wna16_decode_of_more_than_65536_units(ops, M):
     """Sizes at which a product by the number of all units does not fit 32 bits (wna16_mma.cu, ranges cut anywhere): every tile is

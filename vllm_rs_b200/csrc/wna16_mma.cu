@@ -643,6 +643,8 @@ bool launch_wna16_mma(const WnaParams& p, cudaStream_t st, bool force) {
                         reinterpret_cast<uintptr_t>(p.qzeros) | reinterpret_cast<uintptr_t>(p.a) |
                         reinterpret_cast<uintptr_t>(p.workspace);
   if (low & 15) return false;                // 16-byte copies
+  // pairs of fp16 (the tile-split kernel's unsplit form goes by single values; fused operands lie on 8 bytes for every kernel)
+  if ((reinterpret_cast<uintptr_t>(p.bias) | reinterpret_cast<uintptr_t>(p.c)) & 3) return false;
   if (p.epilogue == B200_EPI_SILU_MUL && ((p.N / kTileN) & 1)) return false;
   if (p.epilogue == kEpiRopeKv && p.fe && !(p.fe->D == 32 || p.fe->D == 64 || p.fe->D == 128)) return false;
   return p.M <= 8 ? wm::launch_nt<1>(p, st) : wm::launch_nt<2>(p, st);
