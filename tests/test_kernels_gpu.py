@@ -352,6 +352,20 @@ def test_wna16_bias_and_result_off_four_bytes(ops, off_bias, off_y):
     assert not y.cpu()[rest].any()
 
 
+@pytest.mark.parametrize("M,off_s,off_z", [(1, 1, 0), (9, 0, 1), (16, 3, 2)])
+def test_wna16_scales_and_zeros_off_sixteen_bytes(ops, M, off_s, off_z):
+    """Large 4-bit products of few tokens whose scales or zero points begin anywhere (views of fused ones): the stream-K kernel, as
+    the others copy them by 16 bytes."""
+    K, N = 4096, 28672
+    qw, qz, s, W, x = _wna_case(K, N, M, "awq", 4, seed=M)
+    at = lambda a, n: torch.cat([torch.zeros(n, dtype=a.dtype), a.flatten()]).cuda()[n:].view(a.shape)      # noqa: E731
+    args = (x.cuda(), ops.awq_prepack(torch.from_numpy(qw).cuda()), at(torch.from_numpy(s), off_s), at(torch.from_numpy(qz), off_z),
+            ops.wna16_workspace(16, N))
+    y = ops.wna16_gemm(*args, k=K, n=N)
+    _close(y, om.linear(x, W, None), 2e-3, 2e-3)
+    assert torch.equal(y, ops.wna16_gemm(*args, k=K, n=N, variant=5))
+
+
 @pytest.mark.parametrize("M", [1, 16])
 def test_wna16_decode_of_more_than_65536_units(ops, M):
     """Sizes at which a product by the number of all units does not fit 32 bits (wna16_mma.cu, ranges cut anywhere): every tile is

@@ -495,6 +495,7 @@ __device__ __forceinline__ void split_arrive_and_reduce(const SplitOut& o, int n
 void launch_wna16_gemv(const WnaParams& p, cudaStream_t st);
 bool launch_wna16_tc(const WnaParams& p, cudaStream_t st);   // false: shape unsupported
 bool launch_wna16_tc_dec(const WnaParams& p, cudaStream_t st);   // decode shapes (M <= 64)
+bool wna16_mma_takes(const WnaParams& p, bool force = false);
 bool launch_wna16_mma(const WnaParams& p, cudaStream_t st, bool force = false);      // 4-bit decode shapes (M <= 16)
 // stream-K decode kernel (M <= 32); bf16: A, scales and C are bf16 (plain epilogue, 4-bit only)
 bool launch_wna16_sk(const WnaParams& p, cudaStream_t st, bool force = false, bool bf16 = false, int flavour = -1);

@@ -559,6 +559,13 @@ wna16_mma_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
   }
 }
 
+template <int NT>
+static int cut_of(const WnaParams& p, UnitCut& cut) {
+  int most = sm_count() * Cfg<NT>::kBlocks;
+  if (most > kSkSlotCols / (2 * kTileN)) most = kSkSlotCols / (2 * kTileN);        // two parts per block
+  return cut_units(p.N / kTileN, p.K / kUnitK, most, kKG, cut);
+}
+
 template <int NT, int EPI>
 static bool launch_epi(const WnaParams& p, cudaStream_t st) {
   using C = Cfg<NT>;
@@ -574,12 +581,8 @@ static bool launch_epi(const WnaParams& p, cudaStream_t st) {
   if (p.group_size < p.K)
     for (int s = 0; s < 24; ++s)
       if ((kUnitK << s) == p.group_size) a.gshift = s;
-  const int tiles = p.N / kTileN;
   a.U = p.K / kUnitK;
-  int grid = sm_count() * C::kBlocks;
-  if (grid > kSkSlotCols / (2 * kTileN)) grid = kSkSlotCols / (2 * kTileN);        // two parts per block
-  grid = cut_units(tiles, a.U, grid, kKG, a.cut);
-  if (grid == 0) return false;
+  const int grid = cut_of<NT>(p, a.cut);
   a.by_U = unit_div(a.U);
   a.hd_shift = 6;
   if (p.fe && p.epilogue == kEpiRopeKv) a.hd_shift = p.fe->D == 128 ? 6 : p.fe->D == 64 ? 5 : 4;
@@ -625,13 +628,13 @@ static bool launch_nt(const WnaParams& p, cudaStream_t st) {
 
 }  // namespace wm
 
-// Decode batches of 4-bit weights: false when the shape needs another kernel.  `force`: whether or not it is the faster one.
+// Decode batches of 4-bit weights: false when the call needs another kernel.  `force`: whether or not it is the faster one.
 // Up to 8 tokens it is at every size measured, at 9 - 16, where the products take twice the issue slots, from 4096 units on.
 // us at 1 / 16 tokens, here and the faster of the other two: 4096 x 6144 7.2 / 9.3 and 8.5 / 8.9, 4096 x 4096 5.7 / 7.6 and
 // 7.1 / 7.5, 4096 x 28672 21.0 / 24.9 and 25.7 / 29.1, 14336 x 4096 12.2 / 14.8 and 13.8 / 14.3, 2048 x 2560 4.5 / 6.2 and 5.4 / 6.0,
 // 5632 x 2048 6.5 / 8.2 and 6.2 / 6.6, 8192 x 10240 15.6 / 18.1 and 17.9 / 20.0, 8192 x 57344 65 / 75 and 100 / 102, 28672 x 8192
 // 35.8 / 41.5 and 38.3 / 41.0.  (8-bit weights stay with those: a unit is twice the bytes, one block per SM: 4096 x 28672 35 and 28.)
-bool launch_wna16_mma(const WnaParams& p, cudaStream_t st, bool force) {
+bool wna16_mma_takes(const WnaParams& p, bool force) {
   if (p.bits != 4 || p.M > 16 || p.K % wm::kUnitK != 0 || p.N % kTileN != 0) return false;
   if (!force && p.M > 8 && static_cast<long>(p.N / kTileN) * (p.K / wm::kUnitK) < 4096) return false;
   if (p.group_size < p.K) {                  // a unit lies in one group, whose index is a shift of the unit's
@@ -647,6 +650,12 @@ bool launch_wna16_mma(const WnaParams& p, cudaStream_t st, bool force) {
   if ((reinterpret_cast<uintptr_t>(p.bias) | reinterpret_cast<uintptr_t>(p.c)) & 3) return false;
   if (p.epilogue == B200_EPI_SILU_MUL && ((p.N / kTileN) & 1)) return false;
   if (p.epilogue == kEpiRopeKv && p.fe && !(p.fe->D == 32 || p.fe->D == 64 || p.fe->D == 128)) return false;
+  UnitCut cut;
+  return (p.M <= 8 ? wm::cut_of<1>(p, cut) : wm::cut_of<2>(p, cut)) > 0;
+}
+
+bool launch_wna16_mma(const WnaParams& p, cudaStream_t st, bool force) {
+  if (!wna16_mma_takes(p, force)) return false;
   return p.M <= 8 ? wm::launch_nt<1>(p, st) : wm::launch_nt<2>(p, st);
 }
 

@@ -911,8 +911,8 @@ wna16_sk_kernel(const __grid_constant__ CUtensorMap xmap, const Args a) {
   }
 }
 
-// B200_DEC_SK: 0 = never, 1 = every shape the kernel takes (M <= 32), 2 (default) = 8-bit weights (4-bit ones of so few tokens
-// are faster in wna16_mma.cu) where it measured faster than the
+// B200_DEC_SK: 0 = never, 1 = every shape the kernel takes (M <= 32), 2 (default) = what wna16_mma.cu does not take (4-bit weights
+// of so few tokens are faster there; 8-bit ones, and operands off its 16 bytes, come here) where it measured faster than the
 // tile-split kernel on B200 IN THE DECODE STEP (profiles/r2_ai_sk_policy_ab.txt, same-box A/B): at most 16 tokens on
 // projections with at least 32 units per CTA (gate|up): b=1 2.55 -> 2.44 ms per step.  At 32 tokens the kernel is
 // faster in isolation (gate|up 31.2 vs 32.4 us) but the step gets SLOWER (5.05 -> 5.20 ms): a persistent grid ends on
@@ -1019,7 +1019,8 @@ bool launch_wna16_sk(const WnaParams& p, cudaStream_t st, bool force, bool bf16,
   if (p.M > 32) return false;
   if (!force && sk::sk_mode() == 2) {
     const long units = static_cast<long>(p.N / kTileN) * (p.K / sk::kUnitK);
-    if (p.bits != 8 || p.M > 16 || units < 32L * sm_count()) return false;
+    if (p.M > 16 || units < 32L * sm_count() || wna16_mma_takes(p)) return false;
+    if ((reinterpret_cast<uintptr_t>(p.bias) | reinterpret_cast<uintptr_t>(p.c)) & 7) return false;      // four channels at a time
   }
   if (p.K % sk::kUnitK != 0) return false;
   if (p.group_size < p.K) {                             // a 128-K unit must lie inside one quantisation group,
