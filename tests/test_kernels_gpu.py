@@ -366,6 +366,19 @@ def test_wna16_scales_and_zeros_off_sixteen_bytes(ops, M, off_s, off_z):
     assert torch.equal(y, ops.wna16_gemm(*args, k=K, n=N, variant=5))
 
 
+@pytest.mark.parametrize("K,N,M,group,off_s,off_z", [(8192, 9728, 33, 64, 1, 0), (4096, 9728, 17, 64, 0, 1), (16384, 1280, 64, 32, 1, 1)])
+def test_wna16_many_groups_off_sixteen_bytes(ops, K, N, M, group, off_s, off_z):
+    """Scales or zero points that begin anywhere, of more groups than the tile-split kernel stages for one piece of K: the general
+    kernel, which reads them one by one."""
+    qw, qz, s, W, x = _wna_case(K, N, M, "awq", 4, seed=M, group=group)
+    at = lambda a, n: torch.cat([torch.zeros(n, dtype=a.dtype), a.flatten()]).cuda()[n:].view(a.shape)      # noqa: E731
+    args = (x.cuda(), ops.awq_prepack(torch.from_numpy(qw).cuda()), at(torch.from_numpy(s), off_s), at(torch.from_numpy(qz), off_z),
+            ops.wna16_workspace(64, N))
+    y = ops.wna16_gemm(*args, k=K, n=N, group_size=group)
+    _close(y, om.linear(x, W, None), 2e-3, 2e-3)
+    assert torch.equal(y, ops.wna16_gemm(*args, k=K, n=N, group_size=group, variant=4))
+
+
 @pytest.mark.parametrize("M", [1, 16])
 def test_wna16_decode_of_more_than_65536_units(ops, M):
     """Sizes at which a product by the number of all units does not fit 32 bits (wna16_mma.cu, ranges cut anywhere): every tile is

@@ -573,12 +573,15 @@ struct Split { int splits, chunks, groups; };
 static Split split_of(const WnaParams& p) {
   const int KC = p.K / kChunkK, tiles = p.N / kTileN;
   const bool grouped = p.group_size < p.K;
+  // Scales and zero points come by tensor maps.  Where they do not lie on 16 bytes, long K is left to the general kernel, which reads
+  // them one by one (groups counted as for pieces that start anywhere, no pieces added).
+  const bool mapped = ((reinterpret_cast<uintptr_t>(p.scales) | reinterpret_cast<uintptr_t>(p.qzeros)) & 15) == 0;
   auto cut = [&](int splits) {
     Split s;
     s.chunks = (KC + splits - 1) / splits;
     s.splits = (KC + s.chunks - 1) / s.chunks;
     const int k = s.chunks * kChunkK;         // one group more where pieces may start inside a group
-    s.groups = !grouped ? 1 : (k + p.group_size - 1) / p.group_size + (s.splits > 1 && k % p.group_size ? 1 : 0);
+    s.groups = !grouped ? 1 : (k + p.group_size - 1) / p.group_size + (!mapped || (s.splits > 1 && k % p.group_size) ? 1 : 0);
     return s;
   };
   if (p.no_split) return cut(1);
@@ -592,7 +595,7 @@ static Split split_of(const WnaParams& p) {
   if (splits > cap) splits = cap;
   while (splits > 1 && static_cast<long>(splits) * p.N > kMaxSplitCols) --splits;
   // long K: as many more pieces as the staging of the scales asks for (the kernel for other shapes is far slower here)
-  while (cut(splits).groups > kSZGroups && splits < cap && (splits + 1L) * p.N <= kMaxSplitCols) ++splits;
+  while (mapped && cut(splits).groups > kSZGroups && splits < cap && (splits + 1L) * p.N <= kMaxSplitCols) ++splits;
   return cut(splits);
 }
 
