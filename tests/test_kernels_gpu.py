@@ -334,17 +334,18 @@ def test_wna16_decode_of_few_tokens(ops, fmt, bits, K, N, M, group, epi):
         assert e_new <= e_old * 1.05, (e_new, e_old)               # the same weights, sums in another order
 
 
+@pytest.mark.parametrize("K,N,M,group", [(512, 19456, 3, 128),          # as many tiles as SMs: no kernel splits them
+                                         (8192, 9728, 33, 64)])         # more groups than an unsplit tile of wna16_tc_dec.cu stages
 @pytest.mark.parametrize("off_bias,off_y", [(1, 0), (0, 1), (2, 2)])
-def test_wna16_bias_and_result_off_four_bytes(ops, off_bias, off_y):
-    """As many tiles as SMs: the tile-split kernel writes results one by one, wherever bias and result begin."""
-    K, N, M = 512, 19456, 3
-    qw, qz, s, W, x = _wna_case(K, N, M, "awq", 4, seed=5)
+def test_wna16_bias_and_result_off_eight_bytes(ops, K, N, M, group, off_bias, off_y):
+    """Where a kernel writes a tile's results one by one, they and the bias may begin anywhere."""
+    qw, qz, s, W, x = _wna_case(K, N, M, "awq", 4, seed=5, group=group)
     bias = torch.randn(N).to(F16)
     at = torch.zeros(N + 4, dtype=F16)
     at[off_bias:off_bias + N] = bias
     y = torch.zeros(M * N + 4, dtype=F16).cuda()
     ops.wna16_gemm(x.cuda(), ops.awq_prepack(torch.from_numpy(qw).cuda()), torch.from_numpy(s).cuda(), torch.from_numpy(qz).cuda(),
-                   ops.wna16_workspace(16, N), k=K, n=N, bias=at.cuda()[off_bias:off_bias + N],
+                   ops.wna16_workspace(64, N), k=K, n=N, group_size=group, bias=at.cuda()[off_bias:off_bias + N],
                    out=y[off_y:off_y + M * N].view(M, N))
     _close(y[off_y:off_y + M * N].view(M, N), om.linear(x, W, bias), 2e-3, 2e-3)
     rest = torch.ones(M * N + 4, dtype=torch.bool)

@@ -594,8 +594,10 @@ static Split split_of(const WnaParams& p) {
   if (splits > KC / 4) splits = KC / 4 > 0 ? KC / 4 : 1;
   if (splits > cap) splits = cap;
   while (splits > 1 && static_cast<long>(splits) * p.N > kMaxSplitCols) --splits;
-  // long K: as many more pieces as the staging of the scales asks for (the kernel for other shapes is far slower here)
-  while (mapped && cut(splits).groups > kSZGroups && splits < cap && (splits + 1L) * p.N <= kMaxSplitCols) ++splits;
+  // Long K: as many more pieces as the staging of the scales asks for (the kernel for other shapes is far slower here).  Where
+  // pieces meet, results and bias go four at a time; off 8 bytes an unsplit tile stays unsplit (there or here: one by one).
+  const bool fours = ((reinterpret_cast<uintptr_t>(p.bias) | reinterpret_cast<uintptr_t>(p.c)) & 7) == 0;
+  while (mapped && (fours || splits > 1) && cut(splits).groups > kSZGroups && splits < cap && (splits + 1L) * p.N <= kMaxSplitCols) ++splits;
   return cut(splits);
 }
 
