@@ -404,6 +404,24 @@ def test_wna16_decode_of_more_than_65536_units(ops, M):
         assert int(ws[:16384].view(torch.int32).abs().sum()) == 0
 
 
+@pytest.mark.parametrize("M", [1, 16])
+def test_wna16_decode_repeats_itself(ops, M):
+    """The same bits from every call: no warp reads a place of the ring that a later unit's copies are on their way to.  Weights that
+    have just been written keep the activations out of L2, so that copies take their longest."""
+    K, N = 34944, 30848
+    g = torch.Generator(device="cuda").manual_seed(M)
+    words = lambda r: torch.randint(-2 ** 31, 2 ** 31, (r, N // 8), generator=g, device="cuda", dtype=torch.int64).int()      # noqa: E731
+    qw, qz = words(K), words(K // 128)
+    s = (0.005 + 0.01 * torch.rand(K // 128, N, generator=g, device="cuda")).to(F16)
+    x = (0.05 * torch.randn(M, K, generator=g, device="cuda")).to(F16)
+    ws, first, differ = ops.wna16_workspace(16, N), None, 0
+    for _ in range(500):
+        y = ops.wna16_gemm(x, ops.awq_prepack(qw), s, qz, ws, k=K, n=N, variant=7)
+        first = y if first is None else first
+        differ += int((y != first).any())
+    assert differ == 0
+
+
 @pytest.mark.parametrize("K,N,M,group", [(4096, 9728, 17, 64), (8192, 9728, 33, 64), (8192, 1280, 64, 128)])
 def test_wna16_decode_of_many_groups(ops, K, N, M, group):
     """wna16_tc_dec.cu where one K piece has exactly as many quantisation groups as are staged, and where it takes more pieces."""
