@@ -92,3 +92,22 @@ def test_product_path_never_touches_the_oracle():
             assert not pat.search(p.read_text()), p
     src = (root / "vllm_rs_b200" / "_lib.py").read_text()
     assert "B200Error" in src and "libb200_vllm.so" in src
+
+
+def test_current_stream_with_and_without_the_private_call(monkeypatch):
+    import importlib
+    from types import SimpleNamespace
+
+    import torch
+
+    from vllm_rs_b200 import ops
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 3)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda: SimpleNamespace(cuda_stream=11))
+    try:
+        monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda device: 100 + device, raising=False)
+        assert importlib.reload(ops)._stream() == 103
+        monkeypatch.delattr(torch._C, "_cuda_getCurrentRawStream")
+        assert importlib.reload(ops)._stream() == 11
+    finally:
+        monkeypatch.undo()
+        importlib.reload(ops)

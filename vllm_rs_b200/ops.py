@@ -17,9 +17,15 @@ EPI_NONE, EPI_SILU_MUL = 0, 1
 VARIANT_AUTO, VARIANT_GEMV, VARIANT_TC = 0, 1, 2
 
 
+# torch.cuda.current_stream() builds an object around the handle, a third of a small call's host time; this call is no public one
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream() -> int:
-    """The current stream's handle; torch.cuda.current_stream() builds an object around it, a third of a small call's host time."""
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+    """The current stream's handle."""
+    if _raw_stream is None:
+        return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(torch.cuda.current_device())
 
 
 def _p(t):
