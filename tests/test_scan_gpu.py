@@ -208,6 +208,35 @@ def test_bits_do_not_tell_the_company(lib, kind):
         at += m
 
 
+@pytest.mark.parametrize("n", [2, 63, 64, 65])
+@pytest.mark.parametrize("kind", ["delta", "decay"])
+def test_bits_do_not_tell_the_order(lib, kind, n):
+    """Up to 64 sequences of a step are walked longest first, more as they come: every one has the bits that it has alone, in steps of
+    equal lengths, short ones and several per block (at most 18 blocks of 32 columns share a head's sequences here)."""
+    from vllm_rs_b200 import ops
+    H, d, e = 8, 128, 128
+    lens = [[40, 5, 90, 17, 16, 1, 40, 33][i % 8] + (i * 29) % 23 * (i % 3) for i in range(n)]
+    assert n < 8 or (len(set(lens)) < n and min(lens) <= 16 < 4 * 148 // 32 < sum(m > 16 for m in lens))
+    T, at = sum(lens), [sum(lens[:i]) for i in range(n + 1)]
+    g = torch.Generator().manual_seed(n)
+    r = lambda *s: torch.randn(*s, generator=g).cuda()                        # noqa: E731
+    q, k, v, b, a = r(T, H, d), r(T, H, d), r(T, H, e), r(T, H), r(T, H)
+    alog, dtb, state, past = r(H) * 0.5, r(H), r(n, H, d, e), [0 if i % 5 == 2 else 3 for i in range(n)]
+
+    def run(first, last):
+        rows, ids = slice(at[first], at[last]), list(range(first, last))
+        s, tail = state.clone(), (_i32(ids), _i32([at[i] - at[first] for i in range(first, last + 1)]),
+                                  _i32([lens[i] + past[i] for i in ids]))
+        x = [t[rows].contiguous() for t in (q, k, v, b, a)]
+        if kind == "delta":
+            return ops.delta_rule(*x, alog, dtb, s, *tail), s
+        return ops.decay_attn(*x[:3], s, *tail, head_decay=torch.full((H,), 0.9, device="cuda"), act=True), s
+    out, after = run(0, n)
+    for i in range(n):
+        o, s = run(i, i + 1)
+        assert torch.equal(o, out[at[i]:at[i + 1]]) and torch.equal(s[i], after[i]), (i, lens[i])
+
+
 def test_one_decay_for_long(lib):
     """Hundreds of tokens of one decay and one sign: what a block's decay is off by may not add up from block to block.  Outputs of
     the walk token by token are 0.7e-7 off in the 2-norm, a block's rounded decay by itself made it 2.6e-7."""

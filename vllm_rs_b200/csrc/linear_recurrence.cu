@@ -232,8 +232,7 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
   constexpr int kAll = WW * 32 + 256;
   // Longest sequences first: where not all blocks fit the chip at once, the last to start have the least to do.  Three sequences
   // of 500, 1000 and 1501 tokens, 8 heads of 128 x 256 (192 blocks): 2001 tokens in a row before, 1501 now; the four scans of a
-  // hybrid step take 960 us instead of 1256.  One sequence has no order to look up (4096 tokens, 16 heads of 128: 612 us at first, 599
-  // so; with the order 3 us above the first).
+  // hybrid step take 960 us instead of 1256.  One sequence has no order to look up.
   __shared__ uint8_t order[kSorted];
   const bool sorted = num_seqs > 1 && num_seqs <= kSorted;
   if (sorted && tid < num_seqs) {
