@@ -4,6 +4,7 @@ Bars: integer/byte outputs bit-exact (prepack, argmax, cache contents); floating
 the tolerance written in each test (north star: logits within 1e-3 in fp16 terms; single ops
 are held to ~1 fp16 ulp of their output scale).
 """
+import ctypes
 import math
 
 import numpy as np
@@ -420,6 +421,70 @@ def test_wna16_decode_repeats_itself(ops, M):
         first = y if first is None else first
         differ += int((y != first).any())
     assert differ == 0
+
+
+class _FusedEpi(ctypes.Structure):                   # wna16.cuh, FusedEpi
+    _fields_ = ([("ssq_in", ctypes.c_void_p), ("ssq_tiles", ctypes.c_int), ("inv_dim", ctypes.c_float), ("eps", ctypes.c_float)] +
+                [(n, ctypes.c_void_p) for n in ("resid", "norm_w", "ssq_out", "positions", "slots", "cos", "sin", "k_cache", "v_cache")] +
+                [(n, ctypes.c_int) for n in ("H", "Hkv", "D", "kv_fp8")] +
+                [("push", ctypes.c_void_p * 8), ("push_cnt", ctypes.c_void_p * 8), ("push_world", ctypes.c_int), ("out_bf16", ctypes.c_int)])
+
+
+class _WnaParams(ctypes.Structure):                  # wna16.cuh, WnaParams
+    _fields_ = ([(n, ctypes.c_void_p) for n in ("a", "bp", "scales", "qzeros", "bias", "c")] +
+                [(n, ctypes.c_int) for n in ("M", "K", "N", "bits", "group_size", "qfmt", "epilogue", "no_split")] +
+                [("workspace", ctypes.c_void_p), ("fe", ctypes.c_void_p)])
+
+
+def _same_members(cls, struct):
+    """The header's struct has these members in this order (a launch with others would be one with wrong addresses)."""
+    import re
+    from pathlib import Path
+    text = (Path(__file__).resolve().parent.parent / "vllm_rs_b200" / "csrc" / "wna16.cuh").read_text()
+    body = re.sub(r"//[^\n]*", "", text[text.index(f"struct {struct} {{"):].split("{", 1)[1].split("};", 1)[0])
+    kind = {"int": ctypes.c_int, "float": ctypes.c_float}
+    got = []
+    for decl in filter(None, (d.strip() for d in body.split(";"))):
+        base, names = re.fullmatch(r"(?:const )?(?:struct )?(\w+)(.*)", decl, re.S).groups()
+        for n in names.split(","):
+            size = re.search(r"\[kMaxTpRanks\]", n)
+            got.append((re.search(r"\w+", n).group(), ctypes.c_void_p * 8 if size else ctypes.c_void_p if "*" in n else kind[base]))
+    assert "constexpr int kMaxTpRanks = 8;" in text and got == cls._fields_
+
+
+@pytest.mark.parametrize("kernel,M", [("mma", 1), ("mma", 8), ("mma", 9), ("mma", 16), ("dec", 9), ("dec", 17), ("dec", 33), ("dec", 64)])
+def test_wna16_push_to_peers(ops, kernel, M):
+    """The epilogue of a tensor-parallel rank's row-parallel products: the fp16 partial in every rank's receive buffer, one count per
+    tile and rank.  Nothing waits for the counts here, so the three receive areas lie on this GPU."""
+    from vllm_rs_b200 import _lib
+    _same_members(_FusedEpi, "FusedEpi")
+    _same_members(_WnaParams, "WnaParams")
+    K, N, world = 1024, 2048, 3
+    qw, qz, s, W, x = _wna_case(K, N, M, "awq", 4, seed=M)
+    xd, packed, sd, zd = x.cuda(), ops.awq_prepack(torch.from_numpy(qw).cuda()), torch.from_numpy(s).cuda(), torch.from_numpy(qz).cuda()
+    ws = ops.wna16_workspace(64, N)
+    recv, cnt = torch.full((world, 64, N), float("nan"), dtype=F16, device="cuda"), torch.zeros(world, 16, dtype=torch.int32, device="cuda")
+    fe, p = _FusedEpi(), _WnaParams()
+    for r in range(world):
+        fe.push[r], fe.push_cnt[r] = recv[r].data_ptr(), cnt[r, 5:].data_ptr()
+    fe.push_world = world
+    for n, v in dict(a=xd.data_ptr(), bp=packed.data_ptr(), scales=sd.data_ptr(), qzeros=zd.data_ptr(), M=M, K=K, N=N, bits=4,
+                     group_size=128, qfmt=ops.QFMT_AWQ, epilogue=4, workspace=ws.data_ptr(), fe=ctypes.addressof(fe)).items():
+        setattr(p, n, v)
+    name, more = {"mma": ("_ZN4b20016launch_wna16_mmaERKNS_9WnaParamsEP11CUstream_stb", (ctypes.c_bool(True),)),
+                  "dec": ("_ZN4b20019launch_wna16_tc_decERKNS_9WnaParamsEP11CUstream_st", ())}[kernel]
+    launch = getattr(_lib.lib(), name)
+    launch.restype = ctypes.c_bool
+    for calls in (1, 2):
+        assert launch(ctypes.byref(p), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream), *more)
+        _lib.check()
+        want = torch.zeros(world, 16, dtype=torch.int32)
+        want[:, 5] = calls * (N // 128)
+        assert torch.equal(cnt.cpu(), want)
+        for r in range(world):
+            _close(recv[r, :M], om.linear(x, W, None), 2e-3, 2e-3)
+            assert recv[r, M:].isnan().all()
+        assert int(ws[:16384].view(torch.int32).abs().sum()) == 0
 
 
 @pytest.mark.parametrize("K,N,M,group", [(4096, 9728, 17, 64), (8192, 9728, 33, 64), (8192, 1280, 64, 128)])

@@ -381,8 +381,8 @@ def test_engine_loop_with_prefix_cache(lib):
 @pytest.mark.parametrize("nseq", [1, 2, 4])
 @pytest.mark.parametrize("plan", ["fused", "classic"])
 def test_decode_small_batches(lib, nseq, plan):
-    """Batches of 1-4 sequences (BASELINE: "batch 1-64") run the tcgen05 decode GEMM with a 16-token tile since
-    the GEMV lost its M <= 4 slot (B200_GEMV_MAX_M): same parity bars as the larger batches, two steps."""
+    """Batches of 1-4 sequences run the per-warp 4-bit product of eight tokens (wna16_mma.cu): same parity bars as the larger
+    batches, two steps."""
     from vllm_rs_b200 import engine
     cfg = _toy_cfg()
     NB, MAXB, MAXBLK = 32, 4, 8
@@ -431,6 +431,65 @@ def test_decode_small_batches(lib, nseq, plan):
         osch.postprocess(ids, toks)
         csch.postprocess(ids, toks)
         _sync_cache_to_gpu(oracle, runner)
+
+
+_D64 = dict(num_heads=8, num_kv_heads=2, head_dim=64)
+_D128 = dict(num_heads=4, num_kv_heads=2, head_dim=128)
+
+
+@pytest.mark.parametrize("nseq,shape", [
+    # the tile-split kernel's finalisers, 17 to 64 tokens
+    (17, dict(hidden=512, inter=1024, num_layers=2, **_D64)), (32, dict(hidden=512, inter=1024, num_layers=2, **_D128)),
+    (32, dict(hidden=512, inter=1024, num_layers=2, **_D64)), (48, dict(hidden=512, inter=1024, num_layers=2, **_D128)),
+    # the per-warp kernel's, 9 to 16 tokens: projections of at least 4096 units of 128 x 128 (q|k|v 5120, o 4096; gate|up 4096)
+    (12, dict(hidden=8192, inter=1024, num_layers=2, num_heads=64, num_kv_heads=8, head_dim=128)),
+    (12, dict(hidden=8192, inter=4096, num_layers=1, num_heads=128, num_kv_heads=16, head_dim=64)),
+])
+def test_decode_step_of_larger_batches(lib, nseq, shape):
+    """The fused plan's products (RoPE and cache write, residual and sums of squares, folded norms, SiLU) for the batches that
+    neither the small toys nor the rank shapes above reach: one step, the bars of the other decode tests."""
+    from vllm_rs_b200 import engine
+    cfg = om.ModelConfig(vocab=1024, rope_theta=10000.0, rms_eps=1e-5, max_pos=2048, qkv_bias=nseq == 17, **shape)
+    NB, MAXBLK = 2 * nseq + 2, 2
+    oracle, runner = _build(cfg, "awq", seed=nseq, num_blocks=NB, max_batch=nseq, max_blocks=MAXBLK)
+    with om.exact_mode():
+        exact = om.LlamaOracle(cfg, oracle.w, NB)
+    osch, csch = osched.Scheduler(NB, 64, nseq), engine.Scheduler(NB, 64, nseq)
+    rng = np.random.default_rng(nseq)
+    for i in range(nseq):
+        toks = rng.integers(0, cfg.vocab, size=(3, 17, 64, 70, 1, 33)[i % 6]).tolist()
+        osch.add(osched.Sequence(toks, 64, max_tokens=8))
+        csch.add(toks, 8)
+    ids, _ = osch.schedule()
+    csch.schedule()
+    pmeta = osched.prepare_prefill([osch.running[i] for i in ids], 64)
+    first = oracle.prefill(pmeta).argmax(-1).tolist()
+    with om.exact_mode():
+        exact.prefill(pmeta)
+    for s in (osch, csch):
+        _, fin = s.filter_prefill_finished(ids)
+        s.postprocess(fin, first)
+    _sync_cache_to_gpu(oracle, runner)
+    ids, _ = osch.schedule()
+    csch.schedule()
+    assert len(ids) == nseq
+    mo, mc = osched.prepare_decode([osch.running[i] for i in ids], 64), csch.prepare_decode(ids, max_blocks_cap=MAXBLK)
+    ref = oracle.decode(mo)
+    with om.exact_mode():
+        truth = exact.decode(mo)
+    bt = torch.zeros(nseq, MAXBLK, dtype=torch.int32)
+    bt[:, :mc["max_blocks"]] = torch.from_numpy(mc["block_tables"].astype(np.int32))
+    got = runner.decode_device(
+        torch.from_numpy(mc["input_ids"].astype(np.int32)).cuda(), torch.from_numpy(mc["positions"]).cuda(),
+        torch.from_numpy(mc["slot_mapping"]).cuda(), bt.cuda(),
+        torch.from_numpy(mc["context_lens"].astype(np.int32)).cuda())[0].cpu()
+    noise = (ref - truth).abs().max().item()
+    assert (got - truth).abs().max().item() <= 3 * noise + 2e-3
+    assert (got - ref).abs().max().item() <= 3 * noise + 2e-3
+    for l in range(cfg.num_layers):                  # every row's keys and values, where the step has put them
+        for mine, theirs in ((runner.k_cache, oracle.k_cache), (runner.v_cache, oracle.v_cache)):
+            a, b = (c[l].cpu().float().view(-1, cfg.num_kv_heads, cfg.head_dim)[mo["slot_mapping"]] for c in (mine, theirs))
+            assert (a - b).abs().max() < 2e-2
 
 
 def test_runner_parity_with_the_streamk_gemm_forced():
