@@ -6,6 +6,7 @@ warps, every one of which may find at any page that its rows' maximum grows or d
 before or after it has stored its weights.
 """
 import re
+import subprocess
 from pathlib import Path
 
 import pytest
@@ -181,3 +182,14 @@ def test_the_walk_finds_one_barrier_for_all_pages():
     p["p_wait"], p["p_arrive"] = [lambda j: ("p_full", 0), lambda j: j & 1], [lambda j: ("p_full", 0)]
     fault, _ = walk(p, 3, 2)
     assert "before every warp" in fault or "nobody" in fault
+
+
+def test_no_register_of_a_page_is_spilled(tmp_path):
+    """A page's scores are on their way from tensor memory into registers while the page before is stored: none of these may go
+    through memory in between."""
+    from vllm_rs_b200 import build
+    src = build.CSRC / "attn_prefill_tc.cu"
+    r = subprocess.run([build.NVCC, *build.NVCC_FLAGS, "-Xptxas", "-v", "-cubin", "-o", str(tmp_path / "k.cubin"), str(src)],
+                       capture_output=True, text=True, check=True)
+    frames = re.findall(r"(\d+) bytes stack frame, (\d+) bytes spill stores, (\d+) bytes spill loads", r.stdout + r.stderr)
+    assert frames == [("0", "0", "0")] * 4, frames

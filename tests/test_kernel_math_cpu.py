@@ -32,3 +32,10 @@ def test_parts_never_grow_with_fewer_pages():
         for blocks in (1, 64, 65, 500):
             got = [parts(n, blocks, p) for p in range(1, 70)]
             assert got == sorted(got)
+
+
+def test_swizzled_places_begin_the_shared_memory():
+    """attn_tc_kernel has no room for a round-up to its swizzles' 1024 bytes: dynamic shared memory begins on them as long as there is
+    no static one in front."""
+    src = (CSRC / "paged_attn_tc.cu").read_text()
+    assert re.findall(r"^.*__shared__.*$", src, re.M) == ["  extern __shared__ __align__(1024) uint8_t smem[];"]
