@@ -37,7 +37,7 @@ for name, (K, N, epi) in shapes.items():
         e1.record(st); st.synchronize()
     us = e0.elapsed_time(e1) * 1e3 / (reps * copies)
     out[name] = (us, K * N / 2 / us / 1e3)
-print(f"M={M} variant={variant} dbg={os.environ.get('B200_TC_DBG','0')} pdl={os.environ.get('B200_PDL','1')}: " +
+print(f"M={M} variant={variant} pdl={os.environ.get('B200_PDL','1')}: " +
       "  ".join(f"{k}: {v[0]:.1f}us {v[1]:.0f}GB/s" for k, v in out.items()) +
       f"  | sum {sum(v[0] for v in out.values()):.1f}us")
 

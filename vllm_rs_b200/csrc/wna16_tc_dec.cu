@@ -44,9 +44,6 @@ __device__ uint32_t* g_dec_trace = nullptr;
 #define DEC_TRE(k) do { } while (0)
 #endif
 
-#ifndef B200_DEC_EXP
-#define B200_DEC_EXP 0            // timing experiments (side builds only; results are wrong on purpose): bit 0 no TMEM
-#endif                            // stores, bit 1 no MMAs, bit 2 no activation loads
 #ifndef B200_DEC_PROBE
 #define B200_DEC_PROBE 0          // 1 = early non-blocking probes of afree / wfull: measured neutral (profiles/r2_v_*)
 #endif
@@ -201,12 +198,8 @@ wna16_tc_dec_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_const
         const int xs = j % C::kSXS;
         mbar_wait(&xempty[xs], ((j / C::kSXS) & 1) ^ 1);
         DEC_TR(6, j * C::kSuper);
-#if B200_DEC_EXP & 4           // TIMING EXPERIMENT bit 2: the stage is declared full without loading anything
-        mbar_arrive(&xfull[xs]);
-#else
         mbar_arrive_expect_tx(&xfull[xs], C::kXSBytes);       // TMA zero-fills rows >= M / chunks >= KC
         tma_load_3d(smem + C::kXOff + xs * C::kXSBytes, &xmap, &xfull[xs], 0, 0, c0 + j * C::kSuper);
-#endif
       }
     }
   } else if (warp >= kDqWarps + 2) {
@@ -235,12 +228,10 @@ wna16_tc_dec_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_const
         const uint32_t a_tmem = tmem_base + C::kACol0 + as * 32;
         const uint64_t bdesc =
             make_smem_desc_sw128(smem_u32(smem + C::kXOff + xs * C::kXSBytes + grp * C::kXBytes));
-#if !(B200_DEC_EXP & 2)      // TIMING EXPERIMENT bit 1 (side builds): no MMAs (commits only)
 #pragma unroll
         for (int ks = 0; ks < kChunkK / 16; ++ks)
           tc_mma_ts(d_tmem, a_tmem + ks * 8, bdesc + static_cast<uint64_t>(ks * 2), idesc,
                     (it > 0 || ks > 0) ? 1u : 0u);
-#endif
         tc_commit(&xempty[xs]);
         tc_commit(&afree[as]);
         if (i + kGroups >= nchunks) tc_commit(&gdone[grp]);      // the group's last chunk
@@ -472,11 +463,7 @@ wna16_tc_dec_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_const
         if (!af_ok) bar_wait(s_afree + as * 8, as_phase);
         tc_fence_after();
         if (q4 == 0 && lane == 0) DEC_TR(3, i);
-#if !(B200_DEC_EXP & 1)      // TIMING EXPERIMENT bit 0 (side builds): no TMEM stores
         tmem_st_x16(a_tmem + lane_base, lo);
-#else
-        asm volatile("" ::"r"(lo[0]), "r"(lo[5]), "r"(lo[10]), "r"(lo[15]));
-#endif
 #if B200_DEC_PROBE
         const uint32_t wf_ok = (i + kGroups < nchunks) ? mbar_probe_addr(s_wfull + ss * 8, ss_phase) : 0;
 #else
@@ -484,11 +471,7 @@ wna16_tc_dec_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_const
 #endif
         dequant_half(i, 1, hi);
         if (i + kGroups < nchunks) load_words(cur, i + kGroups, wf_ok);
-#if !(B200_DEC_EXP & 1)
         tmem_st_x16(a_tmem + lane_base + 16, hi);
-#else
-        asm volatile("" ::"r"(hi[0]), "r"(hi[5]), "r"(hi[10]), "r"(hi[15]));
-#endif
         pending_as = as;
         if (++as_l == kAS) { as_l = 0; as_phase ^= 1; }
       }
