@@ -31,6 +31,7 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "f32x2.cuh"
 #include "seqmix.cuh"
 
 namespace b200 {
@@ -115,29 +116,11 @@ __device__ __forceinline__ void cp_async16(float* smem, const float* gmem) {
 template <int N> __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
-// two fp32 values in a 64-bit register, one instruction for both
-using f2 = unsigned long long;
-__device__ __forceinline__ f2 pack2(float lo, float hi) {
-  f2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
 __device__ __forceinline__ float sum2(f2 v) {
   float lo, hi;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+  unpack2(v, lo, hi);
   return lo + hi;
 }
-__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
-  f2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
-  f2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ void unpack2(f2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
 
 constexpr int kOneCols = 16;                   // columns of S per block of threads: single tokens
 constexpr int kBT = 8;                         // tokens per block of the recurrence

@@ -29,6 +29,7 @@
 // 7766 -> 577 us (518 TFLOP/s useful, 785 issued); 32 tokens over 2048 keys, 32 heads over 8: 317 -> 58 us (35 at HBM rate): 256 blocks
 // of 33 pages in turn, with four rows in one pair of the row warps.
 #include "paged_attn_tc.cuh"
+#include "f32x2.cuh"
 
 #include <algorithm>
 
@@ -87,28 +88,6 @@ __device__ __forceinline__ void commit(uint32_t lead, uint64_t* bar) {
       "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%1];\n\t}\n" ::"r"(lead),
       "r"(smem_u32(bar))
       : "memory");
-}
-// two fp32 values in a 64-bit register, one instruction for both
-using f2 = unsigned long long;
-__device__ __forceinline__ f2 pack2(float lo, float hi) {
-  f2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
-  f2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
-  f2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ float max3(float a, float b, float c) {
-  float r;
-  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-  return r;
 }
 // tanh(y) = y P(y^2) for |y| <= kTanhMax: fit of tanh(y) / y in y^2, relative error 6.6e-8 before rounding
 constexpr float kTanhMax = 0.75f;
