@@ -3,7 +3,7 @@
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl reference] [--config NAME]
 
-Configs (BASELINE.json `configs`):
+Configs:
   decode8b        [1] Llama-3-8B AWQ-int4 decode, batch 32, context 4096 (the headline; TP = N under torchrun,
                       strong scaling).  One "step" = one decode step of the whole model (32 layers + lm_head +
                       greedy sampling).  The N = 1 line also carries `prefill` ([2] as written: fp16 weights,
@@ -56,8 +56,8 @@ Keys of the JSON line:
   step_roofline  algorithmic bytes of the whole step (per rank) / step time.
   tp_parity      (N > 1) before timing: TP prefill + 4 decode steps of a 2-layer model of the same per-rank layer
                  shapes vs the unsharded CPU oracle on rank 0 (tests/parity_util.py).
-  cpu_baseline   oracle/c/decode_ref.c (C + OpenMP port of the same step; the reference has no CPU path for AWQ,
-                 SURVEY F3) -- a whole step: 32 layer passes (over 2 layers' worth of distinct tensors) + lm_head.
+  cpu_baseline   oracle/c/decode_ref.c (C + OpenMP port of the same step; the reference has no CPU path for
+                 AWQ) -- a whole step: 32 layer passes (over 2 layers' worth of distinct tensors) + lm_head.
 """
 from __future__ import annotations
 
@@ -245,7 +245,7 @@ def cpu_baseline(batch, ctx, steps=1, model="llama3-8b", distinct_layers=2):
 
 def run_reference(args):
     """The reference arm for this tier: the reference's own CPU implementation of the path cannot be built
-    here (Rust, un-vendored kernels; and it has no CPU path for AWQ at all, SURVEY F2/F3), so this times the
+    here (Rust, un-vendored kernels; and it has no CPU path for AWQ at all), so this times the
     oracle PORT (kind "port") on every host core, on the b200 arm's metric / config."""
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
@@ -595,7 +595,7 @@ def prefill_flops(shape, L, seq_lens):
 
 
 def run_prefill_leg(args, cx: Ctx, fmt, seqs, tokens_per_seq, reps=2):
-    """One prefill step of `seqs` sequences x `tokens_per_seq` tokens (BASELINE configs[2]: fp16 weights, 8 x 8192
+    """One prefill step of `seqs` sequences x `tokens_per_seq` tokens (fp16 weights, 8 x 8192
     in one step = 65 536 tokens, causal varlen attention over the paged cache, last-token lm_head)."""
     import numpy as np
     import torch
@@ -640,8 +640,8 @@ def run_prefill_leg(args, cx: Ctx, fmt, seqs, tokens_per_seq, reps=2):
 
 
 def run_fp8_leg(args, cx: Ctx, K, W, peak):
-    """The same decode step with the FP8 KV cache (`--fp8-kvcache`, SURVEY 8(f) rank 1): NOT the headline
-    configuration (BASELINE.json's metric is the default fp16 cache) -- reported beside it."""
+    """The same decode step with the FP8 KV cache (`--fp8-kvcache`): NOT the headline
+    configuration (that one has the default fp16 cache) -- reported beside it."""
     import torch
     from vllm_rs_b200 import synthetic
     model = "llama3-8b"

@@ -1,7 +1,7 @@
 /*
  * b200_vllm.h -- C ABI of the B200-native (sm_100a) forward hot path for vllm.rs.
  *
- * Drop-in boundary (SURVEY.md section 8b).  Every symbol below replaces one call the
+ * Drop-in boundary.  Every symbol below replaces one call the
  * reference crate makes into its un-vendored native dependency `attention-rs`
  * (or composes several of them into one fused launch).  Conventions are the
  * reference's own (src/utils/gptq.rs:100-200, 314-333):

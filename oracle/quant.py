@@ -2,7 +2,7 @@
 
 TEST INFRASTRUCTURE (see oracle/__init__.py).  Formats as implied by the reference loader
 src/models/layers/wna16.rs:56-83,127-152 (tensor names / shapes / shard dims)
-and the public AutoGPTQ / AutoAWQ packing (SURVEY.md appendix A.4):
+and the public AutoGPTQ / AutoAWQ packing:
 
   GPTQ  qweight i32 [K/pack, N]  element (k,n) = (w[k//pack, n] >> bits*(k%pack)) & mask
         qzeros  i32 [K/G, N/pack] zero(g,n)    = ((z[g, n//pack] >> bits*(n%pack)) & mask) + 1
@@ -105,7 +105,7 @@ def dequant_gptq(qweight, qzeros, scales, group_size, bits):
 
 
 def random_awq(rng: np.random.Generator, K: int, N: int, group_size: int = 128):
-    """Synthetic AWQ layer per SURVEY 8(d) config 2: uniform nibbles, scales
+    """Synthetic AWQ layer: uniform nibbles, scales
     U(0.5,1.5) * (2/15) / sqrt(K) so activations stay O(1)."""
     q = rng.integers(0, 16, size=(K, N), dtype=np.uint8)
     z = rng.integers(0, 16, size=(K // group_size, N), dtype=np.uint8)

@@ -1,4 +1,4 @@
-"""Device sampler timing (SURVEY 8(f) rank 3): sample_topk_topp / penalties / argmax at the Llama-3 vocabulary,
+"""Device sampler timing: sample_topk_topp / penalties / argmax at the Llama-3 vocabulary,
 CUDA events over graph replays; logits rotated over copies larger than L2.  python tools/sampler_bench.py [B]"""
 import os, sys
 sys.path.insert(0, os.path.dirname(os.path.dirname(os.path.abspath(__file__))))

@@ -12,8 +12,8 @@
 // query tokens of ONE kv head, so a K/V page is staged once for the whole GQA group.  8 consumer
 // warps x 16 rows; a producer warp walks the block table 32 entries at a time and issues the
 // 4-D TMA boxes into a 4-stage mbarrier ring.  fp32 online softmax, causal mask per row,
-// P rounded to fp16 for the PV MMA.  Compute-bound on the legacy tensor path (HMMA); a tcgen05
-// version is the next step for this row of SURVEY section 8.
+// P rounded to fp16 for the PV MMA.  Compute-bound on the legacy tensor path (HMMA); heads of
+// 128 go to the tcgen05 kernel (attn_prefill_tc.cu).
 #include "../../include/b200_vllm.h"
 #include "attn.cuh"
 

@@ -2,7 +2,7 @@
 // fp16 or fp32 output, optional bias.
 //
 // Replaces the cuBLAS call behind Linear::forward (src/models/layers/linear.rs:75-123)
-// for fp16 checkpoints (BASELINE.json configs[2]: Llama-3-8B fp16 chunked prefill), the lm_head
+// for fp16 checkpoints (Llama-3-8B fp16 chunked prefill), the lm_head
 // (src/models/llama.rs:311-320) and -- together with wna16_dequant_kernel below --
 // the W4A16 / W8A16 linears of large prefill steps, where dequantising a layer's weights ONCE into an
 // fp16 scratch and running this kernel beats re-dequantising them for every 256-token tile

@@ -10,7 +10,7 @@
 // TensorParallelRowLinear src/models/layers/distributed.rs:438-454
 // GraphCapturer           src/utils/graph.rs:370-377,448-835
 //
-// Launch plan per layer (5 kernels + 2 small ones, vs 17-22 in the reference, SURVEY 3.4):
+// Launch plan per layer (5 kernels + 2 small ones, vs 17-22 in the reference):
 //   [add+]rmsnorm -> fused qkv W4A16 GEMM (+bias) -> RoPE + KV write -> paged attention
 //   (+ split merge) -> o_proj GEMM [-> all-reduce] -> add+rmsnorm -> gate|up GEMM with
 //   SiLU*mul epilogue -> down GEMM [-> all-reduce]

@@ -13,7 +13,7 @@
 // move or release KV blocks (KVCacheSwap, FinishDecode, ClearBlocks), and the trivial ones a runner must recognise
 // (Heartbeat, Shutdown).  RunPrefill carries whole `Sequence` structs: scheduler.cpp reads / writes it
 // (b200_scheduler_load_run_prefill / _frame_run_prefill), next to the Sequence mirror it fills.  Init / RunEmbed
-// (EngineConfig, embedding strategies) stay with the Rust host (control plane, SURVEY 8 out of scope).
+// (EngineConfig, embedding strategies) stay with the Rust host (control plane).
 #include <cstdint>
 #include <cstring>
 

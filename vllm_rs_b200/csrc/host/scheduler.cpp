@@ -13,7 +13,7 @@
 //        reference-counted sharing, eviction); scheduler.rs:288-337,1167-1175 (eviction under pressure)
 //   CPU swap of running sequences (block_manager.rs:255-272,878-1000; scheduler.rs:303-337,830-954): the
 //        bookkeeping only -- the block copies are handed to the host as (src, dst) lists for b200_swap_blocks
-// Out of scope here (SURVEY.md section 8): session ("Cached") sequences, PD transfer, mamba state, image seeds,
+// Out of scope here: session ("Cached") sequences, PD transfer, mamba state, image seeds,
 // tool-call end detection (EOS, max_tokens and stop_token_ids sequences are handled).
 #include <algorithm>
 #include <cstdint>

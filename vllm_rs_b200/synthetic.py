@@ -1,7 +1,6 @@
 """Synthetic (random-init) checkpoints in the reference's on-disk formats, for benches and
 parity tests (there is no network for real checkpoints).  Shapes / packing follow
-src/models/layers/wna16.rs:56-83,127-152; value distributions follow SURVEY.md section 8(d)
-config 2: uniform int4 codes and zero points, scales U(0.5,1.5)*(2/15)/sqrt(K).
+src/models/layers/wna16.rs:56-83,127-152; values: uniform int4 codes and zero points, scales U(0.5,1.5)*(2/15)/sqrt(K).
 """
 from __future__ import annotations
 
@@ -115,12 +114,12 @@ def build_runner(name="llama3-8b", fmt="awq", *, num_blocks, max_blocks_per_seq,
 
 
 def build_awq_runner(name="llama3-8b", **kw) -> ModelRunner:
-    """Random AWQ-int4 model (BASELINE.json configs[1]); see build_runner."""
+    """Random AWQ-int4 model; see build_runner."""
     return build_runner(name, "awq", **kw)
 
 
 def fill_kv_random(r: ModelRunner, seed=1):
-    """KV cache ~ N(0,1) fp16 (SURVEY 8(d) config 2) without a huge temporary."""
+    """KV cache ~ N(0,1) fp16 without a huge temporary."""
     gen = torch.Generator(device=r.device).manual_seed(seed)
     for kc, vc in zip(r.k_cache, r.v_cache):
         if kc.dtype == torch.uint8:          # --fp8-kvcache: e4m3 bytes of the same N(0,1) values
@@ -133,7 +132,7 @@ def fill_kv_random(r: ModelRunner, seed=1):
 
 
 def decode_algorithmic_bytes(shape: dict, batch: int, ctx: int, bits=None, kv_bytes=2) -> dict:
-    """Algorithmic HBM bytes of one decode step of ONE rank (SURVEY.md 8(d) / BASELINE.md section 4)."""
+    """Algorithmic HBM bytes of one decode step of ONE rank."""
     h, L, H, Hkv, D, inter, V, G = (shape[k] for k in
                                     ("hidden", "L", "H", "Hkv", "D", "inter", "vocab", "group"))
     bits = bits or shape.get("bits", 4)

@@ -44,8 +44,8 @@ def shard_column(qweight, qzeros, scales, idx, n):
 
 
 def shard_row(qweight, qzeros, scales, idx, n, group_size):
-    """In-dim shard: tensor dim 0; K/n must be a multiple of the group size (SURVEY section 7:
-    Qwen2-72B inter 29568 / 4 is not -> pad to 29696)."""
+    """In-dim shard: tensor dim 0; K/n must be a multiple of the group size (Qwen2-72B:
+    inter 29568 / 4 is not -> pad to 29696)."""
     k_groups = scales.shape[0]
     assert k_groups % n == 0, f"{k_groups} groups (K={k_groups * group_size}) not divisible by {n}"
     return (_chunk(qweight, 0, idx, n), None if qzeros is None else _chunk(qzeros, 0, idx, n),
