@@ -264,6 +264,29 @@ def test_window_attn_prep_aligned_rows_match_unaligned(lib, T, H, G, dk, dv, rd,
         assert (x.float() - y.float()).abs().max().item() <= (2.0 ** -7 if x.dtype == torch.bfloat16 else 2e-6) * top
 
 
+@pytest.mark.parametrize("H", [8, 16, 32])
+def test_window_attn_prep_norms_are_as_exact_in_both_forms(lib, H):
+    """Normed queries of aligned rows (sums of squares of four entries a thread) against 64 bits, beside the general form's.  The rows'
+    common factor is what the sum's order moves: over 8 x 4096 rows its error is known to half a percent."""
+    from vllm_rs_b200 import ops
+    T, dk, off = 4096, 128, [0.0, 0.0]
+    slots, f = torch.full((T,), -1, device="cuda"), torch.zeros(1, dtype=torch.float64, device="cuda")
+    kc = torch.zeros(1, 64, 1, dk, device="cuda")
+    one = torch.ones(H * dk, device="cuda")
+    for seed in range(8):
+        g = torch.Generator(device="cuda").manual_seed(seed)
+        proj = torch.randn(T, (H + 2) * dk, generator=g, device="cuda")
+        x = proj[:, :H * dk].double()
+        want = x / torch.sqrt((x * x).mean(1, keepdim=True) + 1e-6)
+        for i in (0, 1):
+            at = torch.empty(proj.numel() + 1, device="cuda")[i:i + proj.numel()].view(proj.shape)
+            at.copy_(proj)
+            q = ops.window_attn_prep(at, None, one, one[:dk], f, slots, slots, kc, kc.clone(), heads=H, rot_dims=0, eps=1e-6)
+            off[i] += float(((q.reshape(T, -1).double() - want) ** 2).sum() / (want ** 2).sum())
+    print(H, [(e / 8) ** 0.5 for e in off])
+    assert (off[0] / off[1]) ** 0.5 <= 1.01, [(e / 8) ** 0.5 for e in off]
+
+
 @pytest.mark.parametrize("window,keep", [(3, 2), (64, 5), (65, 64)])
 def test_model_edges_show_in_logits(lib, window, keep):
     """A one-layer model whose recurrent side is switched off: replacing the token at one place changes the last row's
