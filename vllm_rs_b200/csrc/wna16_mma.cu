@@ -239,14 +239,15 @@ __device__ __forceinline__ void finish_tile(const SplitOut& o, int tile, int w, 
 }
 
 // A wait that gives up after some 2^24 polls (or when another one of the block has) and says so.
-__device__ __forceinline__ void wait(uint32_t bar, uint32_t parity, volatile int* fail, int* err) {
+__device__ __forceinline__ bool wait(uint32_t bar, uint32_t parity, volatile int* fail, int* err) {
 #pragma unroll 1
   for (int i = 0; !mbar_try_wait_addr(bar, parity); ++i)
     if (*fail || i > (1 << 24)) {
       *fail = 1;
       *reinterpret_cast<volatile int*>(err) = 1;
-      break;
+      return false;
     }
+  return true;
 }
 
 template <int NT, int EPI>
@@ -397,6 +398,8 @@ wna16_mma_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
 
   int st = 0, done = 0, at = u0 + kg;        // place of the unit at hand, units done, the unit
   uint32_t ph = 0;
+  int refills = 0;                           // by this warp, of one place: (w - kLag) mod S
+  static_assert(S == kGW, "the warps take turns as the places do");
   if (kg == 0) asm volatile("bar.arrive 4, %0;" ::"n"(kThreads) : "memory");
 #pragma unroll 1
   for (int ct = first_tile; ct <= last_tile; ++ct) {
@@ -414,9 +417,11 @@ wna16_mma_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
       if (done >= C::kLag && unit < u1) {
         if ((done & 3) == w) {
           const int ds = st >= C::kLag ? st - C::kLag : st - C::kLag + S;
-          wait(empty + ds * 8, st >= C::kLag ? ph : ph ^ 1, &s_fail, a.err);
-          bring(ds);
-          copy_x(ds, unit - tile * U);
+          if (__all_sync(0xffffffffu, wait(empty + ds * 8, st >= C::kLag ? ph : ph ^ 1, &s_fail, a.err))) {
+            bring(ds);
+            copy_x(ds, unit - tile * U);
+            ++refills;
+          }
         }
         unit += kKG;
       }
@@ -561,6 +566,11 @@ wna16_mma_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
       }
     }
     finish_tile<EPI, NT>(a.o, ct, w, lane, tot, s_rs, s_sq, bar_id, a.hd_shift);
+  }
+  // after a wait has given up: no copy may land in this memory when it is another block's
+  if (*reinterpret_cast<volatile int*>(&s_fail)) {
+    const int at_place = (w + S - C::kLag) % S, fills = refills + (u0 + kg + at_place * kKG < u1 ? 1 : 0);
+    if (fills > 0) mbar_wait_limited(&s_full[kg * S + at_place], (fills - 1) & 1, nullptr, a.err);
   }
 }
 
