@@ -120,7 +120,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_co
   const int cached = ctx - nq;
   const int q_end = min(q0 + TQ, nq);
   const int npages = (cached + q_end - 1) / kTok + 1;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -172,7 +172,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_co
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_arrive_expect_tx(q_full, kQBytes);
       tma_load_3d(q_smem, &qmap, q_full, 0, hkv * G, row0 + q0);
       tma_load_3d(q_smem + kRows * 128, &qmap, q_full, 64, hkv * G, row0 + q0);
@@ -185,7 +185,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_co
       const int cnt = min(32, npages + 1 - base);
       for (int jj = 0; jj < cnt; ++jj) {
         const int blk = __shfl_sync(0xffffffffu, mine, jj);
-        if (lane == 0) {
+        if (elect_one()) {
           const int j = base + jj, s = j & 1;
           if (j < npages) {
             mbar_wait_bounded(&k_empty[s], ((j >> 1) & 1) ^ 1);
@@ -216,7 +216,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_co
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t kFmt = BF ? ((1u << 7) | (1u << 10)) : 0u;          // a_format / b_format = BF16
       const uint32_t idesc_s = make_idesc_f16(kRows, kTok) | kFmt;
       const uint32_t idesc_o = make_idesc_f16(kRows, kD) | (L1 ? 0u : (1u << 16)) | kFmt;   // flash V: MN-major B

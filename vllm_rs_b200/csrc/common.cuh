@@ -152,6 +152,9 @@ __device__ __forceinline__ void cluster_wait() {
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
+// True in one lane of a whole warp.  Single-thread roles (TMA, tcgen05.mma, commit) branch on this and not on lane == 0: those
+// instructions take their operands from the warp, and only behind elect.sync does the compiler know that one lane is there.
+// Eight tcgen05.mma of 128 x 32 x 16 from one warp: 388 cycles under lane == 0, 129 under elect.sync (the tensor core's own time).
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred = 0;
   asm volatile(

@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 dense_gemm_tc_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_constant__ CUtensorMap qmap,
                      const Args a) {
   using C = Cfg<BN, CG>;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const uint32_t rank = CG == 2 ? cluster_ctarank() : 0;
   const int unit = blockIdx.x / CG, nunits = gridDim.x / CG;      // a unit = a CTA or a CTA pair
   const int ntiles = a.tiles_p * a.tiles_q;
@@ -140,7 +140,7 @@ dense_gemm_tc_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_cons
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (every CTA)
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t kit = 0;
       for (int t = unit; t < ntiles; t += nunits) {
         int p, q;
@@ -168,7 +168,7 @@ dense_gemm_tc_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_cons
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (leader CTA)
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && elect_one()) {
       const uint32_t idesc = make_idesc_f16(kBM * CG, BN);
       uint32_t kit = 0;
       int it = 0;

@@ -146,7 +146,7 @@ grouped_linear_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_
         if (!free_) break;                         // a stage that did not come free is not armed again
         uint8_t* ad = smem + s * C::kStage;
         uint8_t* wd = ad + kABytes;
-        if (lane == 0) {
+        if (elect_one()) {
           mbar_arrive_expect_tx(&full[s], boxes * (kBox * 128) + BN * 128);
           if (GATED) {
             tma_load_2d(wd, &wmap, &full[s], kb * kK, wrow);

@@ -259,7 +259,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
         const int cnt = min(32, n - base);
         for (int jj = 0; jj < cnt; ++jj) {
           const int page = __shfl_sync(0xffffffffu, mine, jj);
-          if (lane == 0) {
+          if (elect_one()) {
             free_ = free_ && mbar_wait_limited(&k_empty[kr.s], kr.ph ^ 1, fail, a.err);
             if (free_) {
               uint8_t* kd = k_smem + kr.s * a.k_stage;

@@ -297,7 +297,7 @@ wna16_sk_kernel(const __grid_constant__ CUtensorMap xmap, const Args a) {
   uint32_t tid_o = threadIdx.x;
   asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(s_base + C::kTidOff + tid_o * 4), "r"(tid_o) : "memory");
   asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(tid_o) : "r"(s_base + C::kTidOff + threadIdx.x * 4) : "memory");
-  const int warp = static_cast<int>(tid_o >> 5), lane = static_cast<int>(tid_o & 31);
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(tid_o >> 5), 0), lane = static_cast<int>(tid_o & 31);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::kBarOff);
   uint64_t* wfull = bars;
   uint64_t* wempty = wfull + C::kSWS;
@@ -449,7 +449,7 @@ wna16_sk_kernel(const __grid_constant__ CUtensorMap xmap, const Args a) {
 
   if (warp == kWProdWarp) {
     // ------------------------------------------------------------ weight producer: one contiguous stream
-    if (lane == 0) {
+    if (elect_one()) {
       const uint8_t* src = reinterpret_cast<const uint8_t*>(a.bp) + static_cast<size_t>(u0) * C::kUnitW;
       const int nst = (n + kDG - 1) / kDG;
       for (int s = 0; s < nst; ++s) {
@@ -470,7 +470,7 @@ wna16_sk_kernel(const __grid_constant__ CUtensorMap xmap, const Args a) {
     }
   } else if (warp == kXProdWarp) {
     // ------------------------------------------------------------ activation producer (ring of kDG * kSXS units)
-    if (lane == 0) {
+    if (elect_one()) {
       pdl_wait();      // activations are the previous kernel's output; weights are not
       constexpr int R = kDG * C::kSXS;
       Pos p = pos_of(u0, KP);
@@ -492,7 +492,7 @@ wna16_sk_kernel(const __grid_constant__ CUtensorMap xmap, const Args a) {
     }
   } else if (warp >= kIssWarp0) {
     // ------------------------------------------------------------ MMA issuers (one per dequant group)
-    if (lane == 0) {
+    if (elect_one()) {
       const int grp = warp - kIssWarp0;
       // kind::f16 takes bf16 operands with a_format = b_format = 1 (bits [7,10) and [10,13))
       const uint32_t idesc = make_idesc_f16(128, NT < 16 ? 16 : NT) | (kBf16 ? ((1u << 7) | (1u << 10)) : 0u);

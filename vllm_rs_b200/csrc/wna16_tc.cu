@@ -83,7 +83,7 @@ wna16_tc_kernel(const __grid_constant__ CUtensorMap xmap, const TcArgs a) {
   const int c1 = min(c0 + a.chunks_per_split, KC);
   const int nchunks = c1 - c0;
   const int m0 = blockIdx.z * NT;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int N = a.N, M = a.M;
 
   extern __shared__ uint8_t smem_raw[];
@@ -263,7 +263,7 @@ wna16_tc_kernel(const __grid_constant__ CUtensorMap xmap, const TcArgs a) {
     }
   } else if (warp == kDqWarps) {
     // ------------------------------------------------------------ weight producer
-    if (lane == 0) {
+    if (elect_one()) {
       const uint8_t* src = reinterpret_cast<const uint8_t*>(a.bp) +
                            (static_cast<size_t>(nt) * KC + c0) * Cfg::kWBytes;
       for (int i = 0; i < nchunks; ++i) {
@@ -276,7 +276,7 @@ wna16_tc_kernel(const __grid_constant__ CUtensorMap xmap, const TcArgs a) {
     }
   } else if (warp == kDqWarps + 1) {
     // ------------------------------------------------------------ activation producer
-    if (lane == 0) {
+    if (elect_one()) {
       pdl_wait();      // activations are the previous kernel's output; weights are not
       for (int i = 0; i < nchunks; ++i) {
         const int sx = i % Cfg::kSX;
@@ -287,7 +287,7 @@ wna16_tc_kernel(const __grid_constant__ CUtensorMap xmap, const TcArgs a) {
     }
   } else {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = make_idesc_f16(128, NT < 16 ? 16 : NT);
       for (int i = 0; i < nchunks; ++i) {
         const int sx = i % Cfg::kSX, sa = i % kSA;

@@ -113,7 +113,7 @@ wna16_tc_dec_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_const
   const int c0 = split * a.chunks_per_split;
   const int c1 = min(c0 + a.chunks_per_split, KC);
   const int nchunks = c1 - c0;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int N = a.N, M = a.M;
 
   extern __shared__ uint8_t smem_raw[];
@@ -169,7 +169,7 @@ wna16_tc_dec_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_const
 
   if (warp == kDqWarps) {
     // ------------------------------------------------------------ weight / scale producer
-    if (lane == 0) {
+    if (elect_one()) {
       // scales / zero points of the CTA's K range: one 2-D TMA box each ([groups][128 channels])
       const uint32_t zbytes = a.qzeros ? ZW * 4 : 0;
       mbar_arrive_expect_tx(szfull, static_cast<uint32_t>(a.sz_rows) * (kTileN * 2 + zbytes));
@@ -191,7 +191,7 @@ wna16_tc_dec_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_const
     }
   } else if (warp == kDqWarps + 1) {
     // ------------------------------------------------------------ activation producer
-    if (lane == 0) {
+    if (elect_one()) {
       pdl_wait();      // activations are the previous kernel's output; weights are not
       const int nsuper = (nchunks + C::kSuper - 1) / C::kSuper;
       for (int j = 0; j < nsuper; ++j) {
@@ -207,7 +207,7 @@ wna16_tc_dec_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_const
     // A single in-order issuer for all groups was measured 30% slower (its wait -> issue ->
     // commit loop takes longer per chunk than the dequant of a chunk): four independent issue
     // loops keep the four accumulators busy.
-    if (lane == 0) {
+    if (elect_one()) {
       const int grp = warp - (kDqWarps + 2);
       const uint32_t idesc = make_idesc_f16(128, NT < 16 ? 16 : NT);
       const uint32_t d_tmem = tmem_base + grp * C::kDCols;
