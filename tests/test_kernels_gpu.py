@@ -335,6 +335,34 @@ def test_wna16_decode_of_few_tokens(ops, fmt, bits, K, N, M, group, epi):
         assert e_new <= e_old * 1.05, (e_new, e_old)               # the same weights, sums in another order
 
 
+@pytest.mark.parametrize("fmt,bits,K,N,M,group,epi", [
+    ("awq", 4, 128, 128, 9, 128, "none"),           # one unit: one accumulator, one group of warps
+    ("awq", 4, 384, 256, 17, 128, "silu"),          # three blocks of a unit each meet in a cluster
+    ("gptq", 4, 640, 384, 33, 640, "bias"),         # five units in five blocks; rows that not every block has as many of
+    ("gptq_sym", 4, 2048, 1536, 64, 256, "none"),   # no zero points, two units per group
+    ("awq", 4, 4096, 6144, 11, 128, "bias"),        # two blocks per tile
+    ("awq", 4, 4096, 28672, 32, 128, "silu"),       # ranges cut anywhere: two or three tiles in a block, meetings in memory
+    ("awq", 4, 1280, 40960, 50, 128, "none"),       # whole tiles and parts of an odd number of units in one block
+    ("awq", 4, 14336, 4096, 16, 128, "none"),       # rings that go round many times
+    ("awq", 4, 8192, 1280, 64, 128, "none"),        # seven blocks would meet, but as many clusters do not fit
+    ("gptq", 8, 384, 256, 1, 128, "silu"),
+    ("gptq", 8, 4096, 12288, 32, 128, "none"),
+    ("gptq", 8, 14336, 4096, 9, 128, "bias"),
+])
+def test_wna16_units_cut_evenly(ops, fmt, bits, K, N, M, group, epi):
+    """wna16_ts.cu (variant 8, and what variant 0 takes from 9 tokens on)."""
+    call, ref, truth = _wna_run(ops, fmt, bits, K, N, M, group, epi, K + N + M)
+    y = call(8)
+    _close(y, ref, 2e-3, 4e-3 if epi == "silu" else 2e-3)          # the bound of the other variants: fp32 sums, fp16 results
+    assert all(torch.equal(call(8), y) for _ in range(20))         # parts are summed in the order of K
+    if M > 8:
+        assert torch.equal(call(0), y)
+    if epi == "none" and "sym" not in fmt:
+        t = truth()
+        e_new, e_old = ((v.cpu().double() - t).norm() for v in (y, call(9)))      # 9: wna16_tc_dec.cu
+        assert e_new <= e_old * 1.05, (e_new, e_old)               # the same weights, sums in another order
+
+
 @pytest.mark.parametrize("K,N,M,group", [(512, 19456, 3, 128),          # as many tiles as SMs: no kernel splits them
                                          (8192, 9728, 33, 64)])         # more groups than an unsplit tile of wna16_tc_dec.cu stages
 @pytest.mark.parametrize("off_bias,off_y", [(1, 0), (0, 1), (2, 2)])
@@ -485,6 +513,30 @@ def test_wna16_push_to_peers(ops, kernel, M):
             _close(recv[r, :M], om.linear(x, W, None), 2e-3, 2e-3)
             assert recv[r, M:].isnan().all()
         assert int(ws[:16384].view(torch.int32).abs().sum()) == 0
+
+
+@pytest.mark.parametrize("K,N,M", [(1024, 2048, 9), (1024, 2048, 64), (2048, 20480, 33)])     # parts of a tile; whole tiles as well
+def test_wna16_units_push_to_peers(ops, K, N, M):
+    """test_wna16_push_to_peers for wna16_ts.cu, whose blocks meet in memory here."""
+    from vllm_rs_b200 import _lib
+    qw, qz, s, W, x = _wna_case(K, N, M, "awq", 4, seed=M)
+    hold = [x.cuda(), ops.awq_prepack(torch.from_numpy(qw).cuda()), torch.from_numpy(s).cuda(), torch.from_numpy(qz).cuda()]
+    ws, world = ops.wna16_workspace(64, N), 2
+    recv, cnt = torch.full((world, 64, N), float("nan"), dtype=F16, device="cuda"), torch.zeros(world, 16, dtype=torch.int32, device="cuda")
+    fe, p = _FusedEpi(push_world=world), _WnaParams(M=M, K=K, N=N, bits=4, group_size=128, qfmt=ops.QFMT_AWQ, epilogue=4)
+    for r in range(world):
+        fe.push[r], fe.push_cnt[r] = recv[r].data_ptr(), cnt[r, 5:].data_ptr()
+    p.a, p.bp, p.scales, p.qzeros = (t.data_ptr() for t in hold)
+    p.workspace, p.fe = ws.data_ptr(), ctypes.addressof(fe)
+    launch = getattr(_lib.lib(), "_ZN4b20015launch_wna16_tsERKNS_9WnaParamsEP11CUstream_stb")
+    launch.restype = ctypes.c_bool
+    assert launch(ctypes.byref(p), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream), ctypes.c_bool(True))
+    _lib.check()
+    assert cnt.cpu()[:, 5].tolist() == [N // 128] * world and int(cnt.sum()) == world * (N // 128)
+    for r in range(world):
+        _close(recv[r, :M], om.linear(x, W, None), 2e-3, 2e-3)
+        assert recv[r, M:].isnan().all()
+    assert int(ws[:16384].view(torch.int32).abs().sum()) == 0
 
 
 @pytest.mark.parametrize("K,N,M,group", [(4096, 9728, 17, 64), (8192, 9728, 33, 64), (8192, 1280, 64, 128)])

@@ -40,22 +40,17 @@ struct UnitCut {
   }
 };
 
-// The cut of tiles x U units for at most `most` blocks of `groups` groups each, of which every one takes a unit in turn.  Returns the
-// number of blocks; 0 where a division would not be exact.
-// Every tile in the same number of parts, at most eight, where that leaves few blocks out: no block has then two tiles.
-// 4096 x 4096, one token: 8 parts 5.4 us, 4 parts 7.1.  Otherwise ranges cut anywhere.
-inline int cut_units(int tiles, int U, int most, int groups, UnitCut& c) {
+// tiles x U units in `parts` parts per tile, or (0) in ranges cut anywhere for `grid` blocks.  Returns the number of blocks; 0 where a
+// division would not be exact.
+inline int cut_parts(int tiles, int U, int parts, int grid, UnitCut& c) {
   const int64_t all = static_cast<int64_t>(tiles) * U;
   if (all >= int64_t{1} << 31) return 0;
   const int total = static_cast<int>(all);
-  int grid = most, splits = grid / tiles;
-  if (splits > U / groups) splits = U / groups;
-  if (splits > 8) splits = 8;
-  c.whole = !(splits >= 1 && (tiles * splits * 100 >= grid * 85 || total < grid * groups || tiles * 8 < grid));
-  if (!c.whole) grid = tiles * splits;
+  c.whole = !parts;
+  if (!c.whole) grid = tiles * parts;
   if (grid > total) grid = total;
   c.period = c.whole ? total : U;
-  c.parts = c.whole ? grid : splits;
+  c.parts = c.whole ? grid : parts;
   c.share = c.period / c.parts;
   c.rest = c.period % c.parts;
   // What is divided: units by U (by the kernel, and as `period` where tiles are cut alike); places in a period by share and share + 1;
@@ -67,6 +62,18 @@ inline int cut_units(int tiles, int U, int most, int groups, UnitCut& c) {
   c.by_share = unit_div(c.share);
   c.by_more = unit_div(c.share + 1);
   return grid;
+}
+
+// The cut of tiles x U units for at most `most` blocks of `groups` groups each, of which every one takes a unit in turn.
+// Every tile in the same number of parts, at most eight, where that leaves few blocks out: no block has then two tiles.
+// 4096 x 4096, one token: 8 parts 5.4 us, 4 parts 7.1.  Otherwise ranges cut anywhere.
+inline int cut_units(int tiles, int U, int most, int groups, UnitCut& c) {
+  if (static_cast<int64_t>(tiles) * U >= int64_t{1} << 31) return 0;
+  int splits = most / tiles;
+  if (splits > U / groups) splits = U / groups;
+  if (splits > 8) splits = 8;
+  const bool even = splits >= 1 && (tiles * splits * 100 >= most * 85 || tiles * U < most * groups || tiles * 8 < most);
+  return cut_parts(tiles, U, even ? splits : 0, most, c);
 }
 
 }  // namespace b200

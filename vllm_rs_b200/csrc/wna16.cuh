@@ -206,23 +206,14 @@ __device__ __forceinline__ float ssq_lane_partial(const float* __restrict__ row,
   return v;
 }
 
+// n0: the thread's first column; n1: its partner columns' first (-1: none)
 template <int EPI>
-__device__ __forceinline__ EpiCol epi_col(const SplitOut& o, int nt, int ch) {
+__device__ __forceinline__ EpiCol epi_col_at(const SplitOut& o, int n0, int n1) {
   const FusedEpi& fe = o.fe;
   EpiCol c;
   c.silu = EPI == B200_EPI_SILU_MUL;
-  c.n1 = -1;
-  if (c.silu) {
-    const int half_tiles = (o.N / kTileN) >> 1;
-    c.n0 = (nt % half_tiles) * kTileN + ch;
-    c.n1 = c.n0 + (o.N >> 1);
-  } else {
-    c.n0 = nt * kTileN + ch;
-    if (EPI == kEpiRopeKv && c.n0 < (fe.H + fe.Hkv) * fe.D) {
-      const int d = c.n0 % fe.D, hd = fe.D >> 1;
-      c.n1 = d < hd ? c.n0 + hd : c.n0 - hd;
-    }
-  }
+  c.n0 = n0;
+  c.n1 = n1;
   c.pair = c.n1 >= 0;
   c.kv_col = EPI == kEpiRopeKv && c.n0 >= fe.H * fe.D;
 #pragma unroll
@@ -237,6 +228,21 @@ __device__ __forceinline__ EpiCol epi_col(const SplitOut& o, int nt, int ch) {
   }
   if (EPI == kEpiResidNorm) half4_to_float(fe.norm_w + c.n0, c.nw);
   return c;
+}
+// the other half of a rotated head (-1: a column that is not rotated)
+__device__ __forceinline__ int rope_partner(const FusedEpi& fe, int n0) {
+  if (n0 >= (fe.H + fe.Hkv) * fe.D) return -1;
+  const int d = n0 % fe.D, hd = fe.D >> 1;
+  return d < hd ? n0 + hd : n0 - hd;
+}
+template <int EPI>
+__device__ __forceinline__ EpiCol epi_col(const SplitOut& o, int nt, int ch) {
+  if (EPI == B200_EPI_SILU_MUL) {
+    const int n0 = (nt % ((o.N / kTileN) >> 1)) * kTileN + ch;
+    return epi_col_at<EPI>(o, n0, n0 + (o.N >> 1));
+  }
+  const int n0 = nt * kTileN + ch;
+  return epi_col_at<EPI>(o, n0, EPI == kEpiRopeKv ? rope_partner(o.fe, n0) : -1);
 }
 
 template <int EPI>
@@ -278,13 +284,12 @@ __device__ __forceinline__ void epi_row_prefetch2(const SplitOut& o, const EpiCo
 // a0 / a1: fp32 sums of the thread's 4 columns / partner columns for row m.  Called by whole
 // warps with a warp-uniform m (the sum-of-squares path reduces across the warp = the tile row).
 template <int EPI>
-__device__ __forceinline__ void epi_row_apply(const SplitOut& o, const EpiCol& c, int m, bool valid,
-                                              const float (&a0)[4], const float (&a1)[4],
-                                              const EpiRow& r, int lane) {
+__device__ __forceinline__ void epi_row_finish(const SplitOut& o, const EpiCol& c, int m, bool valid,
+                                               const float (&a0)[4], const float (&a1)[4],
+                                               const EpiRow& r, int lane, float scale) {
   const FusedEpi& fe = o.fe;
   const int N = o.N;
   constexpr int epi = EPI;
-  const float scale = fe.ssq_in ? rsqrtf(warp_sum(r.rs) * fe.inv_dim + fe.eps) : 1.f;
   float v0[4], v1[4], out[4];
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
@@ -298,7 +303,7 @@ __device__ __forceinline__ void epi_row_apply(const SplitOut& o, const EpiCol& c
         // round the two GEMM outputs to fp16 first: the values an unfused pipeline would see
         const float gg = __half2float(__float2half_rn(v0[e]));
         const float uu = __half2float(__float2half_rn(v1[e]));
-        out[e] = gg / (1.f + __expf(-gg)) * uu;
+        out[e] = __fdividef(gg, 1.f + __expf(-gg)) * uu;       // (a division by subroutine is fetched cold: 1000 cycles)
       }
       store_half4(o.c + static_cast<size_t>(m) * (N >> 1) + c.n0, out);
     }
@@ -360,6 +365,14 @@ __device__ __forceinline__ void epi_row_apply(const SplitOut& o, const EpiCol& c
     else
       store_half4(o.c + static_cast<size_t>(m) * N + c.n0, v0);
   }
+}
+
+template <int EPI>
+__device__ __forceinline__ void epi_row_apply(const SplitOut& o, const EpiCol& c, int m, bool valid,
+                                              const float (&a0)[4], const float (&a1)[4],
+                                              const EpiRow& r, int lane) {
+  epi_row_finish<EPI>(o, c, m, valid, a0, a1, r, lane,
+                      o.fe.ssq_in ? rsqrtf(warp_sum(r.rs) * o.fe.inv_dim + o.fe.eps) : 1.f);
 }
 
 // After the finaliser of a kEpiPushPeers tile: make the tile's remote stores visible system-wide,
@@ -487,6 +500,7 @@ bool launch_wna16_tc(const WnaParams& p, cudaStream_t st);   // false: shape uns
 bool launch_wna16_tc_dec(const WnaParams& p, cudaStream_t st);   // decode shapes (M <= 64)
 bool wna16_mma_takes(const WnaParams& p, bool force = false);
 bool launch_wna16_mma(const WnaParams& p, cudaStream_t st, bool force = false);      // 4-bit decode shapes (M <= 16)
+bool launch_wna16_ts(const WnaParams& p, cudaStream_t st, bool force = false);       // decode shapes (M <= 64), units cut evenly over the SMs
 // stream-K decode kernel (M <= 32); bf16: A, scales and C are bf16 (plain epilogue, 4-bit only)
 bool launch_wna16_sk(const WnaParams& p, cudaStream_t st, bool force = false, bool bf16 = false, int flavour = -1);
 // Largest M the automatic dispatch still gives to the flat GEMV (env B200_GEMV_MAX_M, default 0: the tcgen05

@@ -308,10 +308,16 @@ void b200_wna16_gemm_ex(const void* a, const void* b_packed, const void* scales,
     set_error(1, "wna16: shape unsupported by the per-warp decode kernel");
     return;
   }
-  if (variant == 2 || variant == 3 || variant == 4 || (variant == 0 && m > gemv_max_m())) {
+  if (variant == 8) {                                  // units cut evenly over the SMs (wna16_ts.cu)
+    if (launch_wna16_ts(p, st, true)) return;
+    set_error(1, "wna16: shape unsupported by the unit decode kernel");
+    return;
+  }
+  if (variant == 2 || variant == 3 || variant == 4 || variant == 9 || (variant == 0 && m > gemv_max_m())) {
+    if ((variant == 0 || variant == 2) && launch_wna16_ts(p, st)) return;       // units cut evenly over the SMs (M <= 64)
     if (variant == 0 && launch_wna16_sk(p, st)) return;        // persistent stream-K decode kernel (M <= 32)
     if (variant == 0 && launch_wna16_mma(p, st)) return;       // per-warp decode kernel (M <= 16)
-    if (variant != 4 && launch_wna16_tc_dec(p, st)) return;    // tile-split decode kernel (M <= 64; A/B arm: variant 2)
+    if (variant != 4 && launch_wna16_tc_dec(p, st)) return;    // tile-split decode kernel (M <= 64; A/B arm: variant 9)
     if (launch_wna16_tc(p, st)) return;
     if (variant >= 2) { set_error(1, "wna16: shape unsupported by the tcgen05 variant"); return; }
   }
