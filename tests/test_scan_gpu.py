@@ -99,6 +99,15 @@ def test_ends_of_blocks(lib, kind, H, G, d, e):
     test_scans(lib, kind, H, G, d, e, [0, 6, 0, 31, 32])
 
 
+@pytest.mark.parametrize("H,G,d,e,lens", [(2, 1, 128, 128, [300]),            # four blocks of columns share what they prepare
+                                          (2, 2, 64, 96, [65, 66]),            # two do
+                                          (40, 20, 128, 64, [200, 1, 150]),    # two of 32 columns; a short sequence between
+                                          (2, 1, 200, 256, [257]), (3, 1, 128, 40, [130])])      # unaligned rows; alone
+@pytest.mark.parametrize("kind", ["delta", "delta_chan", "decay", "decay_chan", "ssd"])
+def test_shared_preparation(lib, kind, H, G, d, e, lens):
+    test_scans(lib, kind, H, G, d, e, lens)
+
+
 def test_operands_as_they_lie(lib):
     """Views with other strides and one row per token (the form that mixed types take) give the same bits as packed operands."""
     from vllm_rs_b200 import _lib, ops

@@ -124,22 +124,23 @@ __device__ __forceinline__ float sum2(f2 v) {
 
 constexpr int kOneCols = 16;                   // columns of S per block of threads: single tokens
 constexpr int kBT = 8;                         // tokens per block of the recurrence
-constexpr int kRing = 8;                       // blocks of tokens in shared memory (with four, fetching waited for the walk)
+constexpr int kRing = 8;                       // blocks of tokens in shared memory (sixteen are no faster)
 constexpr int kSorted = 64;                    // sequences up to which a step's longest go first
 constexpr int kShort = 16;                     // tokens of a sequence up to which it is walked token by token
 constexpr int kDelta = 0, kDecay = 1, kSsd = 2;
 
 using ScanArgs = b200_scan_args;
 
-template <int DK, bool CHAN, int WW> struct ScanSmem {         // WW: walking warps, four columns each
+constexpr int CW = 4;                          // columns of the state per walking warp
+template <int DK, bool CHAN, int WW> struct ScanSmem {         // WW: walking warps
   static constexpr int kRows = kBT * DK;                                        // floats of one array of token rows
-  static constexpr int kV = (CHAN ? 3 : 2) * kRows;                             // k | q | decays | v | scalars | T, P (8 x 8 each) | ..
-  static constexpr int kCols = WW * 4, kG = kV + kBT * kCols, kMat = kG + 4 * kBT;          // rest of G_7, strength, G_t, W_t per token
+  static constexpr int kG = (CHAN ? 3 : 2) * kRows;                             // k | q | decays | scalars | T, P (8 x 8 each) | ..
+  static constexpr int kCols = WW * CW, kMat = kG + 4 * kBT;                 // rest of G_7, strength, G_t, W_t per token
   static constexpr int kRat = kMat + 2 * kBT * kBT;                             // [t][j] decay from token j to token t
   static constexpr int kGend = kRat + kBT * kBT;                                // CHAN: [DK] decays over the block, [DK] their rests
   static constexpr int kGrest = kGend + (CHAN ? DK : 0), kBuf = kGrest + (CHAN ? DK : 0);
   static constexpr int kU = kRing * kBuf;                                       // [WW][8 tokens][4 columns]
-  static constexpr int kBars = kU + WW * kBT * 4;
+  static constexpr int kBars = kU + WW * kBT * CW;
   static constexpr int kBytes = kBars * 4 + 2 * kRing * 8 + 16;
 };
 // CH floats from shared memory
@@ -187,22 +188,60 @@ __device__ __forceinline__ float meet32(float (&x)[32], int lane) {
   }
   return x[0];
 }
+// The same where lane l has the values of token t (of eight, four columns each) at t ^ (l >> 2): what a lane keeps in the first three
+// exchanges is always the first half, and nothing has to be selected.
+__device__ __forceinline__ float meet32_turned(float (&x)[32], int lane) {
+#pragma unroll
+  for (int w = 16; w > 2; w >>= 1)
+#pragma unroll
+    for (int i = 0; i < w; ++i) x[i] += __shfl_xor_sync(0xffffffffu, x[i + w], w);
+#pragma unroll
+  for (int w = 2; w > 0; w >>= 1) {
+    const bool up = lane & w;
+#pragma unroll
+    for (int i = 0; i < w; ++i) {
+      const float keep = up ? x[i + w] : x[i], send = up ? x[i] : x[i + w];
+      x[i] = keep + __shfl_xor_sync(0xffffffffu, send, w);
+    }
+  }
+  return x[0];
+}
+// The walkers of a whole cluster arrive on the preparing block's barrier.
+__device__ __forceinline__ bool wait_cluster(uint64_t* bar, uint32_t parity, volatile int* fail, int* err) {
+  const uint32_t at = smem_u32(bar);
+#pragma unroll 1
+  for (int i = 0;; ++i) {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred P;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 P, [%1], %2;\n\tselp.u32 %0, 1, 0, P;\n\t}"
+                 : "=r"(ok) : "r"(at), "r"(parity) : "memory");
+    if (ok) return true;
+    if (*fail || i > (1 << 24)) {
+      *reinterpret_cast<volatile int*>(err) = 1;
+      *fail = 1;
+      return false;
+    }
+  }
+}
 
 // Portions of more than kShort tokens.  grid = (column blocks, heads, runs of sequences); a block walks its sequences one after
 // another.  The first WW warps each own four columns of S: a lane holds DK / 32 neighbouring rows of them in registers, so that
 // a key or query row is read once from shared memory for four columns (one column per lane made these reads the bound: 512
-// bytes of registers per load and warp).  Two groups of four warps take turns at fetching a block's token rows (cp.async, a
-// block ahead of each), norming or activating them and preparing its triangles under the walks of the blocks before; one such
-// group takes longer than a walk (3300 against 1950 cycles for the delta rule), two do not.
+// bytes of registers per load and warp).  Two groups of four warps prepare blocks of tokens under the walks of the blocks before: rows read a
+// turn ahead into registers, normed or activated, and the block's triangles.  What they prepare is the same for all columns of a head, so
+// nc neighbouring blocks form a cluster, take turns at it and send it to each other's rings by bulk copies: prepared eight
+// times over, in each of the blocks of a head of 128 columns, it took issue slots from the walk (4096 tokens of 16 heads of 128 x 128:
+// 597 us, 423 for the walk alone).
 // WW = 8 lets two walking warps share a scheduler and a prepared block, WW = 4 spreads few columns over more SMs.
-// Bound: the chain of blocks, one walk after another, of fp32 FMAs and a butterfly over the lanes; HBM and the FMA units would
-// take 16 and 89 us for 4096 tokens of 16 heads of 128 x 128.  Measured there, token by token (eight lanes per column, four
-// chained shuffles per token) -> in blocks: delta rule 2278 -> 610 us; decayed state of 8 heads of 128 x 256: 909 -> 391 us.  The
+// Bound: the chain of blocks, one walk after another; a walk's 78 shuffles (6.3 cycles each from one warp of a scheduler), its 16-byte loads
+// (12) and its packed FMAs (2.7) overlap in part.  HBM and the FMA units would take 16 and 89 us for 4096 tokens of 16 heads of
+// 128 x 128.  Measured there, token by token (eight lanes per column, four chained shuffles per token) -> in blocks -> prepared in turns,
+// and sums that meet without selections (meet32_turned: 510 -> 440): delta rule 2278 -> 597 -> 440 us; decayed state of 8 heads of
+// 128 x 256: 909 -> 398 -> 334 us.  Two columns per warp and twice the warps: slower (shared memory's loads per column double).  The
 // state's update does not wait for the read-out's sums: the queries' products are taken before the correction's sums meet, and
 // meet under the update (665 and 424 us with both in turn).
 template <int DK, int MODE, bool CHAN, int WW>
 __global__ void __launch_bounds__(WW * 32 + 256, 1)
-scan_kernel(const ScanArgs a, int num_seqs, int* err) {
+scan_kernel(const ScanArgs a, int num_seqs, int nc, int* err) {
   using SM = ScanSmem<DK, CHAN, WW>;
   constexpr int CH = DK / 32, COLS = SM::kCols;
   constexpr bool BACK = MODE != kDelta || WW == 8;                     // rows of the triangles from the diagonal back (below)
@@ -210,7 +249,8 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
   uint64_t* ready = reinterpret_cast<uint64_t*>(sm + SM::kBars);
   uint64_t* done = ready + kRing;
   volatile int* fail = reinterpret_cast<volatile int*>(done + kRing);
-  const int h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, col0 = blockIdx.x * COLS;
+  const int h = blockIdx.y, tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31, col0 = blockIdx.x * COLS;
+  const int rank = nc > 1 ? static_cast<int>(cluster_ctarank()) : 0;
   const int dim = a.dim, vdim = a.vdim, hk = MODE == kDecay ? h : h / (a.heads / a.kv_heads);
   constexpr int kAll = WW * 32 + 256;
   // Longest sequences first: where not all blocks fit the chip at once, the last to start have the least to do.  Three sequences
@@ -236,17 +276,17 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
     if (!__syncthreads_or(mine)) return;
   }
   if (tid == 0) {
-    for (int i = 0; i < kRing; ++i) { mbar_init(&ready[i], 4); mbar_init(&done[i], WW); }
+    for (int i = 0; i < kRing; ++i) { mbar_init(&ready[i], 4); mbar_init(&done[i], WW * nc); }
     *fail = 0;
     fence_barrier_init();
   }
-  // What no token writes is zero and stays it: padding past `dim` and `vdim`, the triangles' upper halves.
-  if (dim < DK || col0 + COLS > vdim) {
-    for (int e = tid; e < kRing * SM::kBuf; e += kAll) sm[e] = 0.f;
-  } else {
-    for (int e = tid; e < kRing * 2 * kBT * kBT; e += kAll) sm[e / (2 * kBT * kBT) * SM::kBuf + SM::kMat + e % (2 * kBT * kBT)] = 0.f;
-  }
+  // what no token writes is zero and stays it: the triangles' upper halves
+  for (int e = tid; e < kRing * 2 * kBT * kBT; e += kAll) sm[e / (2 * kBT * kBT) * SM::kBuf + SM::kMat + e % (2 * kBT * kBT)] = 0.f;
   __syncthreads();
+  if (nc > 1) {                                                        // the others' barriers are there
+    cluster_arrive();
+    cluster_wait();
+  }
   int blocks = 0;                                                      // blocks of tokens so far, over all sequences
   for (int z = blockIdx.z; z < num_seqs; z += gridDim.z) {
     const int b = seq(z), t0 = a.cu_seqlens_q[b], t1 = a.cu_seqlens_q[b + 1], nblk = (t1 - t0 + kBT - 1) / kBT;
@@ -258,48 +298,35 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
       const bool wide = dim % 4 == 0 && (a.ld_q | a.ld_k) % 4 == 0 && (!CHAN || a.ld_decay % 4 == 0) &&
                         ((reinterpret_cast<uintptr_t>(a.q) | reinterpret_cast<uintptr_t>(a.k) |
                           (CHAN ? reinterpret_cast<uintptr_t>(a.chan_decay) : 0)) & 15) == 0;
-      const bool wide_v = vdim % 4 == 0 && a.ld_v % 4 == 0 && (reinterpret_cast<uintptr_t>(a.v) & 15) == 0;
-      auto fetch = [&](int i) {                                        // block i of the sequence; one group in any case
-        if (i < nblk) {
-          const int g = blocks + i;
-          if (g >= kRing) mbar_wait_limited(&done[g % kRing], (g / kRing - 1) & 1, fail, err);
-          float* B = sm + g % kRing * SM::kBuf;
-          const int c0 = t0 + i * kBT, n = min(kBT, t1 - c0);
-          const float* kg = a.k + static_cast<size_t>(c0) * a.ld_k + hk * dim;
-          const float* qg = a.q + static_cast<size_t>(c0) * a.ld_q + hk * dim;
-          const float* ag = CHAN ? a.chan_decay + static_cast<size_t>(c0) * a.ld_decay + h * dim : nullptr;
-          constexpr int TPR = DK / 4, RPS = 128 / TPR;                 // threads per row, rows at a time
-          const int x = pt % TPR * 4;
+      // A block of tokens is prepared by one group of one block of the cluster, g being its number over all sequences, in the order of the
+      // ring's places; its rows are read a turn ahead into registers.
+      const int step = 2 * nc, first = (grp * nc + rank - blocks) & (step - 1);
+      constexpr int TPR = DK / 4, RPS = 128 / TPR, NR = kBT / RPS;     // threads per row, rows at a time, rows of a thread
+      constexpr bool kAhead = DK <= 128;                               // (rows of 256 entries do not fit beside the triangles' operands)
+      float4 raw_k[NR], raw_q[NR], raw_d[CHAN ? NR : 1];
+      const int rx = pt % TPR * 4;
+      auto read_rows = [&](int i) {
+        const int c0 = t0 + i * kBT;
 #pragma unroll
-          for (int r = pt / TPR; r < kBT; r += RPS) {
-            if (r >= n || x >= dim) continue;
-            const int o = r * DK + x;
-            const float* ks_ = kg + static_cast<size_t>(r) * a.ld_k + x;
-            const float* qs_ = qg + static_cast<size_t>(r) * a.ld_q + x;
-            if (wide) {
-              cp_async16(B + o, ks_);
-              cp_async16(B + SM::kRows + o, qs_);
-              if (CHAN) cp_async16(B + 2 * SM::kRows + o, ag + static_cast<size_t>(r) * a.ld_decay + x);
-            } else {
-              for (int z = 0; z < min(4, dim - x); ++z) {
-                cp_async4(B + o + z, ks_ + z);
-                cp_async4(B + SM::kRows + o + z, qs_ + z);
-                if (CHAN) cp_async4(B + 2 * SM::kRows + o + z, ag + static_cast<size_t>(r) * a.ld_decay + x + z);
-              }
+        for (int z = 0; z < NR; ++z) {
+          const int t = c0 + pt / TPR + z * RPS;
+          const bool in = i < nblk && t < t1 && rx < dim;
+          auto get = [&](const float* p) {
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (in && wide) {
+              v = __ldg(reinterpret_cast<const float4*>(p));
+            } else if (in) {
+              v.x = __ldg(p);
+              if (rx + 1 < dim) v.y = __ldg(p + 1);
+              if (rx + 2 < dim) v.z = __ldg(p + 2);
+              if (rx + 3 < dim) v.w = __ldg(p + 3);
             }
-          }
-          const float* vg = a.v + static_cast<size_t>(c0) * a.ld_v + h * vdim + col0;
-          if (wide_v) {
-            const int r = pt / (COLS / 4), c = pt % (COLS / 4) * 4;
-            if (r < n && col0 + c < vdim) cp_async16(B + SM::kV + r * COLS + c, vg + static_cast<size_t>(r) * a.ld_v + c);
-          } else {
-            for (int e = pt; e < n * COLS; e += 128) {
-              const int r = e / COLS, c = e % COLS;
-              if (col0 + c < vdim) cp_async4(B + SM::kV + e, vg + static_cast<size_t>(r) * a.ld_v + c);
-            }
-          }
+            return v;
+          };
+          raw_k[z] = get(a.k + static_cast<size_t>(t) * a.ld_k + hk * dim + rx);
+          raw_q[z] = get(a.q + static_cast<size_t>(t) * a.ld_q + hk * dim + rx);
+          if (CHAN) raw_d[z] = get(a.chan_decay + static_cast<size_t>(t) * a.ld_decay + h * dim + rx);
         }
-        cp_async_commit();
       };
       auto sync = [&] {                                // of these four warps
         __syncwarp();
@@ -368,19 +395,24 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
         ej -= pw == 1 ? et : et + 1;
         ++et;
       }
-      fetch(grp);
-      if (pw == 3 && grp < nblk) {
-        read_scalars(grp);
-        make_scalars(grp);
-      }
-      for (int i = grp; i < nblk; i += 2) {
-        fetch(i + 2);
-        if (pw == 3) read_scalars(i + 2);
-        cp_async_wait<1>();
-        sync();
-        float* B = sm + (blocks + i) % kRing * SM::kBuf;
+      if (kAhead) read_rows(first);
+      if (pw == 3) read_scalars(first);
+      for (int i = first; i < nblk; i += step) {
+        const int g = blocks + i, n = min(kBT, t1 - t0 - i * kBT);
+        float* B = sm + g % kRing * SM::kBuf;
         const float* G = B + SM::kG;
-        const int n = min(kBT, t1 - t0 - i * kBT);
+        if (!kAhead) read_rows(i);
+        if (g >= kRing) wait_cluster(&done[g % kRing], (g / kRing - 1) & 1, fail, err);
+        __syncwarp();
+#pragma unroll
+        for (int z = 0; z < NR; ++z) {
+          float* row = B + (pt / TPR + z * RPS) * DK + rx;
+          *reinterpret_cast<float4*>(row) = raw_k[z];
+          *reinterpret_cast<float4*>(row + SM::kRows) = raw_q[z];
+          if (CHAN) *reinterpret_cast<float4*>(row + 2 * SM::kRows) = raw_d[z];
+        }
+        if (kAhead) read_rows(i + step);
+        sync();
         // ---- two tokens per warp: norms or activation, in place; past the end: no key, no value, decay one
         if (MODE == kDelta || (MODE == kDecay && a.act) || n < kBT) {
           float kx[2][CH], qx[2][CH], sk[2] = {0.f, 0.f}, sq[2] = {0.f, 0.f};
@@ -431,11 +463,6 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
               for (int j = 0; j < CH; ++j) kx[z][j] = 1.f;
               stv<CH>(kr + 2 * SM::kRows + z * DK, kx[z]);
             }
-            if (lane < COLS) {
-              float* v = B + SM::kV + r * COLS + lane;
-              if (!in) *v = 0.f;
-              else if (MODE == kDecay && a.act) *v = silu_exact(*v);
-            }
           }
         }
         sync();
@@ -447,8 +474,10 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
         // the source lanes in registers, which eight walking warps do not have.  Delta rule, 4096 tokens of heads of 128 x 128:
         // 16 heads 650 us with BACK, 590 without (a branch instead: 666); 32 heads, a decay per channel 907 - 965 and 1114.
         // Decayed state, 8 heads of 128 x 256: 384 and 397.
+        float v = 0.f;
         if (pw == 3) {
-          if (i + 2 < nblk) make_scalars(i + 2);
+          make_scalars(i);
+          read_scalars(i + step);
         } else if (pw != 1 || MODE == kDelta) {
           auto entries = [&](auto first, auto last, auto strict, const float* rows) {
             constexpr int F = decltype(first)::value, L = decltype(last)::value, ST = decltype(strict)::value;
@@ -483,9 +512,12 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
           using std::integral_constant;
           const float* K = B;
           const float* Q = B + SM::kRows;
-          float v = pw == 1   ? entries(integral_constant<int, 1>{}, integral_constant<int, kBT>{}, integral_constant<int, 1>{}, K)
+          v = pw == 1   ? entries(integral_constant<int, 1>{}, integral_constant<int, kBT>{}, integral_constant<int, 1>{}, K)
                     : pw == 0 ? entries(integral_constant<int, 4>{}, integral_constant<int, kBT>{}, integral_constant<int, 0>{}, Q)
                               : entries(integral_constant<int, 0>{}, integral_constant<int, 4>{}, integral_constant<int, 0>{}, Q);
+        }
+        sync();
+        if (pw != 3 && (pw != 1 || MODE == kDelta)) {
           float* out = B + SM::kMat + (pw == 1 ? 0 : kBT * kBT);
           if (et < et_end) {
             v *= B[SM::kRat + et * kBT + ej];
@@ -544,77 +576,119 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
           }
         }
         __syncwarp();
-        if (lane == 0) mbar_arrive(&ready[(blocks + i) % kRing]);
+        if (lane == 0) mbar_arrive(&ready[g % kRing]);
+        if (nc > 1) {                                  // to the same place of the cluster's other blocks
+          fence_proxy_async();
+          sync();
+          if (pw == 0 && lane < nc && lane != rank)
+            asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                             mapa_shared(smem_u32(B), lane)),
+                         "r"(smem_u32(B)), "r"(SM::kBuf * 4), "r"(mapa_shared(smem_u32(&ready[g % kRing]), lane))
+                         : "memory");
+        }
       }
-      cp_async_wait<0>();
     } else {
       // ---------------------------------------------------------- the walk
-      const int colw = col0 + warp * 4;                // this warp's first column
+      const int colw = col0 + warp * CW;               // this warp's first column
       float* sp = a.state + ((static_cast<size_t>(a.state_slots[b]) * a.heads + h) * dim) * vdim + colw;
       const bool wide_s = vdim % 4 == 0 && (reinterpret_cast<uintptr_t>(a.state) & 15) == 0;
       const float skip = MODE == kSsd && a.d_skip ? a.d_skip[h] : 0.f;
-      f2 s[4][CH / 2];                                 // [column][pair of rows]
+      f2 s[CW][CH / 2];                                // [column][pair of rows]
       {
-        float x[CH][4];
+        float x[CH][CW];
 #pragma unroll
         for (int r = 0; r < CH; ++r) {
           const int i = lane * CH + r;
 #pragma unroll
-          for (int c = 0; c < 4; ++c) x[r][c] = 0.f;
+          for (int c = 0; c < CW; ++c) x[r][c] = 0.f;
           if (!fresh && i < dim) {
             const float* src = sp + static_cast<size_t>(i) * vdim;
             if (wide_s && colw < vdim) {
-              const float4 v = *reinterpret_cast<const float4*>(src);
-              x[r][0] = v.x; x[r][1] = v.y; x[r][2] = v.z; x[r][3] = v.w;
+              ldv<CW>(x[r], src);
             } else {
 #pragma unroll
-              for (int c = 0; c < 4; ++c)
+              for (int c = 0; c < CW; ++c)
                 if (colw + c < vdim) x[r][c] = src[c];
             }
           }
         }
 #pragma unroll
-        for (int c = 0; c < 4; ++c)
+        for (int c = 0; c < CW; ++c)
 #pragma unroll
           for (int r = 0; r < CH; r += 2) s[c][r / 2] = pack2(x[r][c], x[r + 1][c]);
       }
-      float* us = sm + SM::kU + warp * kBT * 4;
-      const int tt = lane >> 2, c4 = lane & 3;         // the token and column whose sums this lane gets
+      float* us = sm + SM::kU + warp * kBT * CW;
+      const int tt = lane >> 2, cc = lane & 3;         // the token and column whose sums this lane gets
       int from[kBT];
 #pragma unroll
-      for (int j = 0; j < kBT; ++j) from[j] = min(j, tt) * 4 + c4;
+      for (int j = 0; j < kBT; ++j) from[j] = min(j, tt) * 4 + cc;
+      // its values, two blocks ahead
+      const bool col_in = colw + cc < vdim;
+      const float* vp = a.v + static_cast<size_t>(t0 + tt) * a.ld_v + h * vdim + colw + cc;
+      const size_t v_step = static_cast<size_t>(kBT) * a.ld_v;
+      int v_left = col_in ? (t1 - t0 - tt + kBT - 1) / kBT : 0;        // blocks in which this lane has a token
+      auto value = [&] {
+        const float v = v_left > 0 ? __ldg(vp) : 0.f;
+        vp += v_step;
+        --v_left;
+        return v;
+      };
+      float v0 = value(), v1 = value();
+      float* op = a.out + (static_cast<size_t>(t0 + tt) * a.heads + h) * vdim + colw + cc;
+      const size_t o_step = static_cast<size_t>(kBT) * a.heads * vdim;
+      // A block that another one prepares arrives by its bytes; who waits for them says so, a block ahead.
+      auto expect = [&](int g) {
+        if (nc > 1 && warp == 0 && lane == 0 && (g & (nc - 1)) != rank) {
+          const uint32_t bar = smem_u32(&ready[g % kRing]);
+          asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(SM::kBuf * 4) : "memory");
+          asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], 4;" ::"r"(bar) : "memory");
+        }
+      };
+      expect(blocks);
       // what entry j of a row of the triangles is multiplied by; the oldest token first in both forms, so that their bits are equal
       auto entry = [](int i) { return BACK ? kBT - 1 - i : i; };
       auto part = [&](float x, int j) { return BACK ? __shfl_up_sync(0xffffffffu, x, j * 4) : __shfl_sync(0xffffffffu, x, from[j]); };
       for (int i = 0; i < nblk; ++i) {
         const int g = blocks + i;
+        if (i + 1 < nblk) expect(g + 1);
+        float vt = v0;
+        v0 = v1;
+        const bool has = v_left > -2;                  // (of the block at hand)
+        v1 = value();
         mbar_wait_limited(&ready[g % kRing], (g / kRing) & 1, fail, err);
         __syncwarp();
         const float* B = sm + g % kRing * SM::kBuf;
         const float* G = B + SM::kG;
         // the rows' products with this lane's part of the state
-        auto dots = [&](float (&x)[32], const float* rows) {
+        constexpr bool KEEP = MODE == kDelta && !CHAN && WW == 4 && DK <= 128;     // keys stay in registers until the update
+        f2 kept[KEEP ? kBT : 1][CH / 2];
+        auto dots = [&](float (&x)[32], const float* rows, auto keep) {
 #pragma unroll
           for (int t = 0; t < kBT; ++t) {
             f2 y[CH / 2];
-            ldv2<CH>(y, rows + t * DK + lane * CH);
+            ldv2<CH>(y, rows + (decltype(keep)::value ? t : t ^ tt) * DK + lane * CH);
+            if (decltype(keep)::value) {
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
+              for (int r = 0; r < CH / 2; ++r) kept[KEEP ? t : 0][r] = y[r];
+            }
+#pragma unroll
+            for (int c = 0; c < CW; ++c) {
               f2 acc = mul2(y[0], s[c][0]);
 #pragma unroll
               for (int r = 1; r < CH / 2; ++r) acc = fma2(y[r], s[c][r], acc);
-              x[t * 4 + c] = sum2(acc);
+              x[t * CW + c] = sum2(acc);
             }
           }
         };
         const float gt = CHAN ? 1.f : G[2 * kBT + tt];
-        const float vt = B[SM::kV + tt * COLS + warp * 4 + c4], wt = G[kBT + tt];
+        const float wt = G[kBT + tt];
+        if (MODE == kDecay && a.act) vt = silu_exact(vt);
         float u = vt * wt, xq[32];
-        dots(xq, B + SM::kRows);
+        dots(xq, B + SM::kRows, std::false_type{});
         if (MODE == kDelta) {
           float xk[32];
-          dots(xk, B);
-          const float r = wt * fmaf(-gt, meet32(xk, lane), vt);
+          dots(xk, B, std::integral_constant<bool, KEEP>{});
+          const float r = wt * fmaf(-gt, KEEP ? meet32(xk, lane) : meet32_turned(xk, lane), vt);
           const float4 ta = *reinterpret_cast<const float4*>(B + SM::kMat + tt * kBT), tb = *reinterpret_cast<const float4*>(B + SM::kMat + tt * kBT + 4);
           const float T[kBT] = {ta.x, ta.y, ta.z, ta.w, tb.x, tb.y, tb.z, tb.w};
           u = 0.f;
@@ -623,7 +697,7 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
         }
         us[lane] = CHAN ? u : u * G[3 * kBT + tt];
         __syncwarp();
-        const float e = meet32(xq, lane);              // (in no one's way: the state's update does not need it)
+        const float e = meet32_turned(xq, lane);              // (in no one's way: the state's update does not need it)
         {
           const float4 pa = *reinterpret_cast<const float4*>(B + SM::kMat + kBT * kBT + tt * kBT);
           const float4 pb = *reinterpret_cast<const float4*>(B + SM::kMat + kBT * kBT + tt * kBT + 4);
@@ -633,8 +707,8 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
           for (int z = 0; z < kBT; ++z) o = fmaf(P[entry(z)], part(u, entry(z)), o);
           if (MODE == kDecay) o *= a.q_scale;
           if (MODE == kSsd) o += skip * vt;
-          const int t = t0 + i * kBT + tt;
-          if (t < t1 && colw + c4 < vdim) a.out[(static_cast<size_t>(t) * a.heads + h) * vdim + colw + c4] = o;
+          if (has) *op = o;
+          op += o_step;
         }
         // The block's decay meets the first token's part in one rounding, as eight tokens' decays would.  A state that only decays takes
         // it with what its own rounding left, which would otherwise be the same in every block and add up (heads of 128 x 128, 500
@@ -646,7 +720,7 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
           ldv2<CH>(ge, B + SM::kGend + lane * CH);
           if (FIRST) {
 #pragma unroll
-            for (int c = 0; c < 4; ++c)
+            for (int c = 0; c < CW; ++c)
 #pragma unroll
               for (int r = 0; r < CH / 2; ++r) s[c][r] = mul2(s[c][r], ge[r]);
           }
@@ -662,41 +736,60 @@ scan_kernel(const ScanArgs a, int num_seqs, int* err) {
 #pragma unroll
         for (int t = 0; t < kBT; ++t) {
           f2 y[CH / 2];
-          ldv2<CH>(y, kd + t * DK);
-          const float4 uu = *reinterpret_cast<const float4*>(us + t * 4);
-          const f2 u[4] = {pack2(uu.x, uu.x), pack2(uu.y, uu.y), pack2(uu.z, uu.z), pack2(uu.w, uu.w)};
+          if constexpr (KEEP) {
+#pragma unroll
+            for (int r = 0; r < CH / 2; ++r) y[r] = kept[t][r];
+          } else {
+            ldv2<CH>(y, kd + t * DK);
+          }
+          float uu[CW];
+          ldv<CW>(uu, us + t * 4);
+          f2 u[CW];
+#pragma unroll
+          for (int c = 0; c < CW; ++c) u[c] = pack2(uu[c], uu[c]);
 #pragma unroll
           for (int r = 0; r < CH / 2; ++r)
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
+            for (int c = 0; c < CW; ++c) {
               if (t == 0 && !FIRST) s[c][r] = fma2(s[c][r], ge[r], REST ? fma2(y[r], u[c], mul2(s[c][r], gl[r])) : mul2(y[r], u[c]));
               else s[c][r] = fma2(y[r], u[c], s[c][r]);
             }
         }
         __syncwarp();
-        if (lane == 0) mbar_arrive(&done[g % kRing]);
+        if (lane == 0) {
+          // (what was read from the place has been used; a release would wait for the outputs' stores, some 700 cycles)
+          if (nc > 1)
+            asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(mapa_shared(smem_u32(&done[g % kRing]), g & (nc - 1))) : "memory");
+          else
+            mbar_arrive(&done[g % kRing]);
+        }
       }
 #pragma unroll
       for (int r = 0; r < CH; r += 2) {
-        float x[2][4];
+        float x[2][CW];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) unpack2(s[c][r / 2], x[0][c], x[1][c]);
+        for (int c = 0; c < CW; ++c) unpack2(s[c][r / 2], x[0][c], x[1][c]);
 #pragma unroll
         for (int z = 0; z < 2; ++z) {
           const int i = lane * CH + r + z;
           if (i >= dim) continue;
           float* dst = sp + static_cast<size_t>(i) * vdim;
           if (wide_s && colw < vdim) {
-            *reinterpret_cast<float4*>(dst) = make_float4(x[z][0], x[z][1], x[z][2], x[z][3]);
+            stv<CW>(dst, x[z]);
           } else {
 #pragma unroll
-            for (int c = 0; c < 4; ++c)
+            for (int c = 0; c < CW; ++c)
               if (colw + c < vdim) dst[c] = x[z][c];
           }
         }
       }
     }
     blocks += nblk;
+  }
+  if (nc > 1) {                                                        // nothing is on its way to, or read from, a block that is gone
+    __syncwarp();
+    cluster_arrive();
+    cluster_wait();
   }
 }
 
@@ -893,8 +986,23 @@ scan_short_kernel(const ScanArgs a) {
   }
 }
 
+template <typename... P, typename... A>
+static void launch_cluster(void (*kern)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st_, int nc, A... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = nc;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st_;
+  cfg.attrs = &attr;
+  cfg.numAttrs = nc > 1 ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
 template <int DK, int MODE, bool CHAN, int WW>
-static void launch_scan_ww(const ScanArgs& a, int z, int* err, cudaStream_t st_) {
+static void launch_scan_ww(const ScanArgs& a, int z, bool short_rows, int* err, cudaStream_t st_) {
   using SM = ScanSmem<DK, CHAN, WW>;
   auto kern = scan_kernel<DK, MODE, CHAN, WW>;
   static OncePerDevice sized;
@@ -902,7 +1010,11 @@ static void launch_scan_ww(const ScanArgs& a, int z, int* err, cudaStream_t st_)
   const int cols = (a.vdim + SM::kCols - 1) / SM::kCols;
   // a few blocks per SM, each taking every so many sequences
   z = std::max(1, std::min(z, 4 * sm_count() / (cols * a.heads)));
-  kern<<<dim3(cols, a.heads, z), WW * 32 + 256, SM::kBytes, st_>>>(a, a.num_seqs, err);
+  // Blocks of a head that share what they prepare.  Portions of a few blocks of tokens end before that pays for the clusters' start and
+  // end: delta rule, 16 heads of 128 x 128, eight sequences of 17 / 64 tokens alone 39 / 68 us, four together 47.5 / 75; 64
+  // tokens 16.6 and 18.6; 4096 tokens 538 and 440.  (The bits are the same.)
+  const int nc = short_rows || cols % 2 ? 1 : cols % 4 ? 2 : 4;
+  launch_cluster(kern, dim3(cols, a.heads, z), WW * 32 + 256, SM::kBytes, st_, nc, a, a.num_seqs, nc, err);
   B200_CUDA_LAUNCH_CHECK();
 }
 template <int DK, int MODE, bool CHAN>
@@ -925,8 +1037,9 @@ static void launch_scan_dk(const ScanArgs& a, int num_tokens, cudaStream_t st_) 
   // sequences that can be longer than that: none in a step of few tokens, as of decoded ones
   const int longer = num_tokens > 0 ? std::min(a.num_seqs, num_tokens / (kShort + 1)) : a.num_seqs;
   if (longer == 0) return;
-  if (narrow) launch_scan_ww<DK, MODE, CHAN, 4>(a, longer, err, st_);
-  else launch_scan_ww<DK, MODE, CHAN, 8>(a, longer, err, st_);
+  const bool short_rows = num_tokens > 0 && num_tokens <= 64 * a.num_seqs;
+  if (narrow) launch_scan_ww<DK, MODE, CHAN, 4>(a, longer, short_rows, err, st_);
+  else launch_scan_ww<DK, MODE, CHAN, 8>(a, longer, short_rows, err, st_);
 }
 // dim: rows of the state; at most 256 (the caller has checked)
 template <int MODE, bool CHAN>
