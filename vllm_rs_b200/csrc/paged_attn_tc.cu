@@ -24,9 +24,9 @@
 //
 // Bound: tensor cores for prompts (per page 2 * 128 * 64 * (dim * passes + vdim) flop against 64 * dim * 2 bytes from L2),
 // HBM for steps of few rows, whose keys are split over blocks; window_attn_merge / latent_attn_merge then finish.
-// Measured, mma.sync kernels -> here: window 1024, 4096 rows, 16 heads of 128 over 4: 622 -> 90 us (332 TFLOP/s; what bounds it
+// Measured, mma.sync kernels -> here: window 1024, 4096 rows, 16 heads of 128 over 4: 622 -> 85 us (352 TFLOP/s; what bounds it
 // is the softmax warps, then the start and the drain of 128 blocks); latent, 2 x 2048 rows, 32 heads, rank 512:
-// 7766 -> 577 us (518 TFLOP/s useful, 785 issued); 32 tokens over 2048 keys, 32 heads over 8: 317 -> 58 us (35 at HBM rate): 256 blocks
+// 7766 -> 512 us (584 TFLOP/s useful, 885 issued); 32 tokens over 2048 keys, 32 heads over 8: 317 -> 58 us (35 at HBM rate): 256 blocks
 // of 33 pages in turn, with four rows in one pair of the row warps.
 #include "paged_attn_tc.cuh"
 #include "f32x2.cuh"
@@ -53,6 +53,8 @@ struct Args {
   int kblk, tail, vblk, passes, ppc;      // 64-wide blocks of a key row (+ 32-wide tail), of a value row; passes; passes per block
   int shared, q_tm, sk, sv;               // values inside the key rows; query blocks in TMEM; ring stages
   int k_stage, v_stage, q_bytes, tmem_cols, page_ref;
+  int wide_q, wide_out;                   // on 32 bytes
+  uint32_t by_group;                      // row / group = row * by_group >> 16 (row < 256)
   int* err;
 };
 
@@ -88,6 +90,26 @@ __device__ __forceinline__ void commit(uint32_t lead, uint64_t* bar) {
       "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%1];\n\t}\n" ::"r"(lead),
       "r"(smem_u32(bar))
       : "memory");
+}
+// 32 bytes of a lane at once: the scattered rows of a warp are a line each to the load and store units
+__device__ __forceinline__ void ld32(float4& lo, float4& hi, const float* p, bool wide) {
+  if (wide)
+    asm volatile("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=f"(lo.x), "=f"(lo.y), "=f"(lo.z), "=f"(lo.w), "=f"(hi.x), "=f"(hi.y), "=f"(hi.z), "=f"(hi.w) : "l"(p));
+  else {
+    lo = __ldg(reinterpret_cast<const float4*>(p));
+    hi = __ldg(reinterpret_cast<const float4*>(p) + 1);
+  }
+}
+__device__ __forceinline__ void st32(void* p, const uint4& lo, const uint4& hi, bool wide) {
+  if (wide)
+    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(lo.x), "r"(lo.y), "r"(lo.z), "r"(lo.w), "r"(hi.x),
+                 "r"(hi.y), "r"(hi.z), "r"(hi.w)
+                 : "memory");
+  else {
+    reinterpret_cast<uint4*>(p)[0] = lo;
+    reinterpret_cast<uint4*>(p)[1] = hi;
+  }
 }
 // tanh(y) = y P(y^2) for |y| <= kTanhMax: fit of tanh(y) / y in y^2, relative error 6.6e-8 before rounding
 constexpr float kTanhMax = 0.75f;
@@ -374,25 +396,22 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
     constexpr int kRowThreads = kRowWarps * 32;
     const int tid = threadIdx.x - 64;
     const uint32_t lane_base = static_cast<uint32_t>(q4 * 32) << 16;
-    // ---- stage Q as bf16: coalesced 32-byte reads, chunks of 8 entries
+    // ---- stage Q as bf16: coalesced 32-byte reads, chunks of 8 entries (128 rows of 544: 26 000 cycles with divisions and 64-bit
+    // addresses per chunk and 16-byte loads, 17 000 without; latent prompt 549 -> 512 us)
     {
       const int cpr = p.dim / 8;
       const int dr = kRowThreads / cpr, dc = kRowThreads % cpr;          // what 256 chunks on are: dr rows and dc chunks
       int row = tid / cpr, c = tid % cpr;
+      const float* const first = p.q + (static_cast<size_t>(row0) * p.heads + kvh * G) * p.dim;
+      const int skip = p.heads - G;                          // heads between a token's rows and the next one's
       while (row < kRows) {
-        constexpr int U = 8;                                 // chunks in flight per thread: 32 KB per block
+        constexpr int U = 8;                                 // chunks in flight per thread: 64 KB per block
         float4 lo[U], hi[U];
         const int row_first = row, c_first = c;
 #pragma unroll
         for (int u = 0; u < U; ++u) {
           lo[u] = hi[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (row < nrows) {
-            const int t = row / G;
-            const float4* src = reinterpret_cast<const float4*>(
-                p.q + (static_cast<size_t>(row0 + t) * p.heads + kvh * G + (row - t * G)) * p.dim + c * 8);
-            lo[u] = __ldg(src);
-            hi[u] = __ldg(src + 1);
-          }
+          if (row < nrows) ld32(lo[u], hi[u], first + ((row + static_cast<int>(row * a.by_group >> 16) * skip) * p.dim + c * 8), a.wide_q);
           row += dr;
           c += dc;
           if (c >= cpr) { c -= cpr; ++row; }
@@ -625,7 +644,8 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
         if (valid && p.nsplit > 1) {
           float* dst = p.part_o + (orow * p.nsplit + sp) * p.vdim + col0 + c0;
 #pragma unroll
-          for (int i = 0; i < 32; i += 4) *reinterpret_cast<uint4*>(dst + i) = make_uint4(o[i], o[i + 1], o[i + 2], o[i + 3]);
+          for (int i = 0; i < 32; i += 8)
+            st32(dst + i, make_uint4(o[i], o[i + 1], o[i + 2], o[i + 3]), make_uint4(o[i + 4], o[i + 5], o[i + 6], o[i + 7]), a.wide_out);
         } else if (valid) {
           if (ge) {
 #pragma unroll
@@ -633,21 +653,20 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
           }
           if (p.out_f32) {
             float* dst = reinterpret_cast<float*>(p.out) + orow * p.vdim + col0 + c0;
+            auto four = [&](int i) {
+              return make_uint4(__float_as_uint(__uint_as_float(o[i]) * inv), __float_as_uint(__uint_as_float(o[i + 1]) * inv),
+                                __float_as_uint(__uint_as_float(o[i + 2]) * inv), __float_as_uint(__uint_as_float(o[i + 3]) * inv));
+            };
 #pragma unroll
-            for (int i = 0; i < 32; i += 4)
-              *reinterpret_cast<float4*>(dst + i) = make_float4(__uint_as_float(o[i]) * inv, __uint_as_float(o[i + 1]) * inv,
-                                                                __uint_as_float(o[i + 2]) * inv, __uint_as_float(o[i + 3]) * inv);
+            for (int i = 0; i < 32; i += 8) st32(dst + i, four(i), four(i + 4), a.wide_out);
           } else {
             __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.out) + orow * p.vdim + col0 + c0;
+            auto eight = [&](int i) {
+              auto two = [&](int k) { return pack16x2<true>(__uint_as_float(o[k]) * inv, __uint_as_float(o[k + 1]) * inv); };
+              return make_uint4(two(i), two(i + 2), two(i + 4), two(i + 6));
+            };
 #pragma unroll
-            for (int i = 0; i < 32; i += 8) {
-              uint4 w;
-              w.x = pack16x2<true>(__uint_as_float(o[i]) * inv, __uint_as_float(o[i + 1]) * inv);
-              w.y = pack16x2<true>(__uint_as_float(o[i + 2]) * inv, __uint_as_float(o[i + 3]) * inv);
-              w.z = pack16x2<true>(__uint_as_float(o[i + 4]) * inv, __uint_as_float(o[i + 5]) * inv);
-              w.w = pack16x2<true>(__uint_as_float(o[i + 6]) * inv, __uint_as_float(o[i + 7]) * inv);
-              *reinterpret_cast<uint4*>(dst + i) = w;
-            }
+            for (int i = 0; i < 32; i += 16) st32(dst + i, eight(i), eight(i + 8), a.wide_out);
           }
         }
         __syncwarp();
@@ -764,6 +783,9 @@ void launch_attn_tc(const AttnTcProblem& p, cudaStream_t st) {
   a.page_ref = attn_few_rows(p.T);
   a.ppc = p.nsplit == 1 && tiles * p.kv_heads >= 2 * sm_count() ? a.passes : 1;
   const dim3 grid(tiles, p.kv_heads, p.nsplit * (a.passes / a.ppc));
+  a.by_group = (65536 + a.group - 1) / a.group;
+  a.wide_q = (reinterpret_cast<uintptr_t>(p.q) & 31) == 0;
+  a.wide_out = ((reinterpret_cast<uintptr_t>(p.out) | reinterpret_cast<uintptr_t>(p.part_o)) & 31) == 0;
   const bool cap = p.softcap > 0.f, bias = p.slopes || p.dist_bias;
   auto kern = cap ? (bias ? attn_tc_kernel<true, true> : attn_tc_kernel<true, false>)
                   : (bias ? attn_tc_kernel<false, true> : attn_tc_kernel<false, false>);
