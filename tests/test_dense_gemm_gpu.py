@@ -99,3 +99,23 @@ def test_wna16_dequant_bit_exact(ops, fmt, bits):
                             k=K, n=N, bits=bits, group_size=G, qfmt=ops.QFMT_AWQ if fmt == "awq" else ops.QFMT_GPTQ)
     want = torch.from_numpy(np.ascontiguousarray(W.T))                 # oracle W is [K, N]
     assert torch.equal(out.cpu(), want)
+
+
+@pytest.mark.parametrize("T,ff,K", [(129, 8, 64), (300, 136, 192), (256, 128, 64), (1000, 5632, 2048)])
+def test_gated_rows(T, ff, K):
+    """dense_gated.cu: gate and up rows behind each other, tiles of 256 rows and 128 channels with ragged ends, bf16 results of fp32 sums."""
+    import ctypes
+    from vllm_rs_b200 import _lib
+    g = torch.Generator().manual_seed(T + ff)
+    x, w = torch.randn(T, K, generator=g).bfloat16(), (torch.randn(2 * ff, K, generator=g) / K ** 0.5).bfloat16()
+    xd, wd, out = x.cuda(), w.cuda(), torch.full((T + 1, ff), float("nan"), dtype=torch.bfloat16, device="cuda")
+    launch = getattr(_lib.lib(), "_ZN4b20018launch_dense_gatedEPKvS1_PviiiiP11CUstream_st")
+    launch.restype = ctypes.c_bool
+    p = lambda t: ctypes.c_void_p(t.data_ptr())                                # noqa: E731
+    assert launch(p(xd), p(wd), p(out), T, ff, K, 0, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    _lib.check()
+    gate, up = (xd.double() @ wd.double().T).chunk(2, 1)
+    ref = torch.nn.functional.silu(gate) * up
+    assert ((out[:T].double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5).all()      # one rounding to bf16; fp32 sums of K terms
+    assert out[T].isnan().all()
+    assert not launch(p(xd), p(wd), p(out), 128, ff, K, 0, None) and not launch(p(xd), p(wd), p(out), T, ff, K, 1, None)

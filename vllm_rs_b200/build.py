@@ -37,7 +37,7 @@ NVCC_FLAGS = [
 
 HYBRID_SOURCES = ["runtime.cu", "glue.cu", "sampler.cu", "seq_norms.cu", "latent_attn.cu", "window_attn.cu", "paged_attn_tc.cu",
                   "linear_recurrence.cu",
-                  "moe.cu", "moe_tc.cu", "gemm_lib.cu", "host/scheduler.cpp", "host/hybrid_runner.cpp"]
+                  "moe.cu", "moe_tc.cu", "gemm_lib.cu", "dense_gated.cu", "host/scheduler.cpp", "host/hybrid_runner.cpp"]
 HYBRID_LIB = PKG / "libb200_hybrid.so"
 
 

@@ -619,9 +619,11 @@ static void run_mixer(b200_hybrid* r, const b200_hybrid_layer& l, const int64_t*
 // dense gated feed-forward of a sandwich layer: y = W_down (silu(W_gate h) * (W_up h))
 static void dense_ffn(b200_hybrid* r, const b200_hybrid_layer& l, int T, cudaStream_t st) {
   const b200_hybrid_config& c = r->cfg;
-  gemm_f32out(r->hin, c.width, 0, l.w_shared_gate_up, c.width, 0, r->sh, 2 * l.shared_ff, 0, T, 2 * l.shared_ff, c.width, 1,
-              0.f, 0, c.dt, st);
-  launch_silu_mul_f32(r->sha, r->sh, T, l.shared_ff, c.dt, st);
+  if (!launch_dense_gated(r->hin, l.w_shared_gate_up, r->sha, T, l.shared_ff, c.width, c.dt, st)) {
+    gemm_f32out(r->hin, c.width, 0, l.w_shared_gate_up, c.width, 0, r->sh, 2 * l.shared_ff, 0, T, 2 * l.shared_ff, c.width, 1,
+                0.f, 0, c.dt, st);
+    launch_silu_mul_f32(r->sha, r->sh, T, l.shared_ff, c.dt, st);
+  }
   gemm_f32out(r->sha, l.shared_ff, 0, l.w_shared_down, l.shared_ff, 0, r->y, c.width, 0, T, c.width, l.shared_ff, 1, 0.f,
               0, c.dt, st);
 }
@@ -656,10 +658,11 @@ static void feed_forward(b200_hybrid* r, const b200_hybrid_layer& l, int T, floa
   if (l.shared_ff > 0) {
     // SiLU-gated: [gate | up] rows; squared ReLU, GELU: up rows, closed by the one row of the token's gate where there is one
     const int rows = l.shared_act == 0 ? 2 * l.shared_ff : l.shared_ff + (l.shared_gated ? 1 : 0);
-    gemm_f32out(r->hin, c.width, 0, l.w_shared_gate_up, c.width, 0, r->sh, rows, 0, T, rows, c.width, 1, 0.f, 0, c.dt, st);
-    if (l.shared_act == 0)
+    const bool gated = l.shared_act == 0 && launch_dense_gated(r->hin, l.w_shared_gate_up, r->sha, T, l.shared_ff, c.width, c.dt, st);
+    if (!gated) gemm_f32out(r->hin, c.width, 0, l.w_shared_gate_up, c.width, 0, r->sh, rows, 0, T, rows, c.width, 1, 0.f, 0, c.dt, st);
+    if (!gated && l.shared_act == 0)
       launch_silu_mul_f32(r->sha, r->sh, T, l.shared_ff, c.dt, st);
-    else
+    else if (!gated)
       launch_ff_act(r->sha, r->sh, rows, T, l.shared_ff, l.shared_gated ? l.shared_ff : -1, (const float*)l.ff_up_bias,
                     l.shared_act, c.dt, st);
     gemm_f32out_scaled(r->sha, l.shared_ff, 0, l.w_shared_down, l.shared_ff, 0, dst, c.width, 0, T, c.width, l.shared_ff,
