@@ -452,3 +452,31 @@ def test_random_configurations_under_random_schedules(lib, seed, dtype):
     tol, q = (F32_TOL, 1.0) if dtype == torch.float32 else (BF16_TOL, 0.9)
     for k, v in reqs.items():
         assert rel_err(d.result(k), ref_logits(cfg, w, v), q) <= tol, (k, kinds)
+
+
+@pytest.mark.parametrize("T,width,off", [(3, 4, 0), (2, 1020, 0), (37, 2048, 0), (5, 4096, 0), (3, 4100, 0), (3, 2047, 0), (4, 512, 1)])
+@pytest.mark.parametrize("dt", [0, 1])
+def test_norm_after_update(T, width, off, dt):
+    """The norm made with the update of the stream against the two launches, aligned or not, wider than the registers or not.  The
+    stream's bits are the same.  The squares meet in the same tree, of at most 16 terms and 8 levels, but not with the same multiplies
+    fused: 24 roundings of 2^-24 on either side, halved by the root, are below 2^-18; bf16 rounds to the neighbour at worst."""
+    import ctypes
+    from vllm_rs_b200 import _lib
+    g = torch.Generator().manual_seed(width)
+    row = lambda *n: torch.randn(*n, generator=g).cuda()                       # noqa: E731
+    rows = torch.randn(T * width + off, generator=g).cuda()
+    x, xs = rows[off:], rows.clone()[off:]                  # both at the same offset: the two sides sum in the same order
+    y, w, w2 = row(T, width), row(width), row(width)
+    outs = [torch.zeros(T, width, dtype=torch.float32 if dt else torch.bfloat16, device="cuda") for _ in range(2)]
+    p = lambda t: None if t is None else ctypes.c_void_p(t.data_ptr())         # noqa: E731
+    f, i, L = ctypes.c_float, ctypes.c_int, _lib.lib()
+    st = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    add = getattr(L, "_ZN4b20024launch_resid_add_rmsnormEPfPKfS2_iiffPvP11CUstream_stS3_S2_i")
+    norm = getattr(L, "_ZN4b20020launch_resid_rmsnormEPvPKfS2_iiffPKjiP11CUstream_sti")
+    add(p(x), p(y), p(w), T, width, f(1e-6), f(1.0), None, st, p(outs[0]), p(w2), i(dt))
+    add(p(xs), p(y), p(w), T, width, f(1e-6), f(1.0), None, st, None, None, i(0))
+    norm(p(outs[1]), p(xs), p(w2), T, width, f(1e-6), f(1.0), None, i(dt), st, i(0))
+    torch.cuda.synchronize()
+    _lib.check()
+    a, b = (o.double() for o in outs)
+    assert torch.equal(x, xs) and ((a - b).abs() <= b.abs() * (2.0 ** -18 if dt else 2.0 ** -7)).all() and float(b.abs().sum()) > 0

@@ -698,6 +698,7 @@ void b200_hybrid_step(b200_hybrid* r, const uint32_t* input_ids, const int64_t* 
     r->x = r->hist + hstride;
   }
   bool h_is_x = first_reads_stream;          // h holds the bf16 rounding of the current x
+  bool normed = false;                       // h holds the norm that the layer starts with
   // hyper-connected streams: the update of the sublayer run last waits for the next read of the streams, which does both
   struct {
     const float *mix = nullptr, *out = nullptr, *y = nullptr, *down = nullptr;
@@ -830,22 +831,28 @@ void b200_hybrid_step(b200_hybrid* r, const uint32_t* input_ids, const int64_t* 
       }
       continue;
     }
-    launch_resid_rmsnorm(r->h, r->x, (const float*)l.norm_w, T, c.width, c.norm_eps, c.norm_weight_offset, nullptr,
-                         c.dt, st);
+    if (!normed)
+      launch_resid_rmsnorm(r->h, r->x, (const float*)l.norm_w, T, c.width, c.norm_eps, c.norm_weight_offset, nullptr,
+                           c.dt, st);
+    normed = false;
     if (l.layout == B200_LAYOUT_SANDWICH) {
+      // the norm that follows an update of the stream is made with it: this layer's, or the next one's where that is its first step
+      const b200_hybrid_layer* next = i + 1 < c.num_layers ? &r->layers[i + 1] : nullptr;
+      if (next && next->layout != B200_LAYOUT_SANDWICH) next = nullptr;
+      const float* next_w = next ? (const float*)next->norm_w : nullptr;
+      normed = next_w != nullptr;
       run_mixer(r, l, positions, slot_mapping, cu, ctx, block_tables, state_slots, max_blocks, B, T, r->y, l.out_scale,
                 0.f, st);
       if (side.heads > 0)
         run_mixer(r, side, positions, slot_mapping, cu, ctx, block_tables, state_slots, max_blocks, B, T, r->y,
                   side.out_scale, 1.f, st);
+      const float* then = l.shared_ff > 0 ? (const float*)l.ff_norm_w : next_w;
       launch_resid_add_rmsnorm(r->x, r->y, (const float*)l.post_norm_w, T, c.width, c.norm_eps, c.norm_weight_offset,
-                               nullptr, st);
+                               nullptr, st, then ? r->h : nullptr, then, c.dt);
       if (l.shared_ff > 0) {
-        launch_resid_rmsnorm(r->h, r->x, (const float*)l.ff_norm_w, T, c.width, c.norm_eps, c.norm_weight_offset, nullptr,
-                             c.dt, st);
         dense_ffn(r, l, T, st);
         launch_resid_add_rmsnorm(r->x, r->y, (const float*)l.ff_post_norm_w, T, c.width, c.norm_eps,
-                                 c.norm_weight_offset, nullptr, st);
+                                 c.norm_weight_offset, nullptr, st, next_w ? r->h : nullptr, next_w, c.dt);
       }
     } else {
       run_mixer(r, l, positions, slot_mapping, cu, ctx, block_tables, state_slots, max_blocks, B, T, r->x, l.out_scale,

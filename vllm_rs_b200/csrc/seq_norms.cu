@@ -93,10 +93,14 @@ resid_rmsnorm_vec_kernel(T* __restrict__ out, const float* __restrict__ x, size_
     if (d < width) st4(out + static_cast<size_t>(r) * width + d, scaled4(v[i], inv, ld4(w + d), w_offset));
   }
 }
-template <int NV>
+// x += norm(y), and where the next step on the stream is its norm (next_out), that from the same registers: the row is not read a
+// second time and a launch goes.  HBM / L2 bound.  A step of 3001 rows of 2048 through four layers, 12.2 + 9.2 us (cold) apart: 2463 us,
+// together: 2437.
+template <typename T, int NV>
 __global__ void __launch_bounds__(256)
 resid_add_rmsnorm_vec_kernel(float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ w, int width, float eps,
-                             float w_offset, __nv_bfloat16* __restrict__ cast_out) {
+                             float w_offset, __nv_bfloat16* __restrict__ cast_out, T* __restrict__ next_out,
+                             const float* __restrict__ next_w) {
   __shared__ float red[33];
   const size_t row = static_cast<size_t>(blockIdx.x) * width;
   float4 v[NV], o[NV];
@@ -118,9 +122,20 @@ resid_add_rmsnorm_vec_kernel(float* __restrict__ x, const float* __restrict__ y,
     const int d = (i * 256 + threadIdx.x) * 4;
     if (d >= width) continue;
     const float4 s = scaled4(v[i], inv, ld4(w + d), w_offset);
-    const float4 n = make_float4(o[i].x + s.x, o[i].y + s.y, o[i].z + s.z, o[i].w + s.w);
-    st4(x + row + d, n);
-    if (cast_out) st4(cast_out + row + d, n);
+    o[i] = make_float4(o[i].x + s.x, o[i].y + s.y, o[i].z + s.z, o[i].w + s.w);
+    st4(x + row + d, o[i]);
+    if (cast_out) st4(cast_out + row + d, o[i]);
+  }
+  if (!next_out) return;
+  ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) ss += dot4(o[i]);
+  ss = block_sum(ss, red);
+  const float next_inv = 1.f / sqrtf(ss / static_cast<float>(width) + eps);
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int d = (i * 256 + threadIdx.x) * 4;
+    if (d < width) st4(next_out + row + d, scaled4(o[i], next_inv, ld4(next_w + d), w_offset));
   }
 }
 // NT threads per group (32: eight groups per block of 256; 256: one), NV vectors each
@@ -677,16 +692,23 @@ void launch_gated_group_norm(void* out, const float* y, int ldy, const float* ga
 }
 
 void launch_resid_add_rmsnorm(float* x, const float* y, const float* w, int T, int width, float eps, float w_offset,
-                              void* cast_out, cudaStream_t st_) {
+                              void* cast_out, cudaStream_t st_, void* next_out, const float* next_w, int dt) {
   if (T <= 0) return;
-  if (width % 4 == 0 && aligned16(x, y, w, cast_out) && with_vectors(width, 1024, [&](auto nv) {
-        resid_add_rmsnorm_vec_kernel<decltype(nv)::value><<<T, 256, 0, st_>>>(x, y, w, width, eps, w_offset, (__nv_bfloat16*)cast_out);
+  if (width % 4 == 0 && aligned16(x, y, w, cast_out) && aligned16(next_out, next_w) && with_vectors(width, 1024, [&](auto nv) {
+        constexpr int NV = decltype(nv)::value;
+        auto run = [&](auto* next) {
+          resid_add_rmsnorm_vec_kernel<std::remove_pointer_t<decltype(next)>, NV><<<T, 256, 0, st_>>>(
+              x, y, w, width, eps, w_offset, (__nv_bfloat16*)cast_out, next, next_w);
+        };
+        if (dt) run((float*)next_out);
+        else run((__nv_bfloat16*)next_out);
       })) {
     B200_CUDA_LAUNCH_CHECK();
     return;
   }
   resid_add_rmsnorm_kernel<<<T, 256, 0, st_>>>(x, y, w, width, eps, w_offset, (__nv_bfloat16*)cast_out);
   B200_CUDA_LAUNCH_CHECK();
+  if (next_out) launch_resid_rmsnorm(next_out, x, next_w, T, width, eps, w_offset, nullptr, dt, st_);
 }
 
 void launch_bias_rows(float* y, const float* bias, float scale, int T, int n, cudaStream_t st_) {

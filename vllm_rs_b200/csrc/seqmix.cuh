@@ -91,9 +91,9 @@ void launch_resid_rmsnorm(void* out, const float* x, const float* w, int T, int 
                           const uint32_t* rows, int dt, cudaStream_t st, int ldx = 0);      // ldx 0: width
 void launch_gated_group_norm(void* out, const float* y, int ldy, const float* gate, int ldg, const float* w, int w_period,
                              int T, int C, int group, float eps, int gate_first, int gate_act, int dt, cudaStream_t st);
-// cast_out (may be NULL): the updated rows rounded to bf16 as well
+// cast_out (may be NULL): the updated rows rounded to bf16 as well; next_out (may be NULL): norm(x) with next_w, of type dt, as well
 void launch_resid_add_rmsnorm(float* x, const float* y, const float* w, int T, int width, float eps, float w_offset,
-                              void* cast_out, cudaStream_t st);
+                              void* cast_out, cudaStream_t st, void* next_out = nullptr, const float* next_w = nullptr, int dt = 0);
 void launch_bias_rows(float* y, const float* bias, float scale, int T, int n, cudaStream_t st);
 void launch_cast_rows(void* out, const float* in, int ld_in, int T, int n, int dt, cudaStream_t st);
 // out [T, n] = in * sigmoid(gate), in fp32 [T, n], gate fp32 with row stride ld_gate
