@@ -480,3 +480,43 @@ def test_norm_after_update(T, width, off, dt):
     _lib.check()
     a, b = (o.double() for o in outs)
     assert torch.equal(x, xs) and ((a - b).abs() <= b.abs() * (2.0 ** -18 if dt else 2.0 ** -7)).all() and float(b.abs().sum()) > 0
+
+
+@pytest.mark.parametrize("T,n,off", [(1, 8, 0), (5, 1032, 0), (300, 2048, 0), (3, 4096, 0), (3, 36, 0), (2, 512, 1)])
+def test_row_kernels_wide_and_not(T, n, off):
+    """Embedding rows and bias rows by wide accesses and by single entries: exact products and one fused multiply-add, so exact
+    against the same in 64 bits rounded once (bias), or in 32 bits (a power of two as scale)."""
+    import ctypes
+    from vllm_rs_b200 import _lib
+    g = torch.Generator().manual_seed(n)
+    L, st = _lib.lib(), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    p = lambda t: None if t is None else ctypes.c_void_p(t.data_ptr())         # noqa: E731
+    f, i = ctypes.c_float, ctypes.c_int
+    embed = getattr(L, "_ZN4b20016launch_embed_f32EPfPKvPKjPKlfiiifiPvP11CUstream_st")
+    ids = torch.randint(0, 12, (T,), generator=g)                             # 11 is out of range: row 0
+    rows = torch.where(ids < 11, ids, torch.zeros_like(ids))
+    for dt, ty in ((0, torch.bfloat16), (1, torch.float32)):
+        table = torch.randn(11 * n + off, generator=g).to(ty).cuda()[off:]
+        x, cast = torch.zeros(T, n, device="cuda"), torch.zeros(T, n, dtype=ty, device="cuda")
+        embed(p(x), p(table), p(_i32(ids.tolist())), None, f(0.0), T, n, 11, f(4.0), i(dt), p(cast), st)
+        want = table.view(11, n)[rows.cuda()].float() * 4
+        assert torch.equal(x, want) and (dt or torch.equal(cast, want.to(ty)))
+    y = torch.randn(T * n + off, generator=g).cuda()[off:]
+    b = torch.randn(n, generator=g).cuda()
+    want = (y.view(T, n).double() + 0.75 * b.double()).float()
+    getattr(L, "_ZN4b20016launch_bias_rowsEPfPKffiiP11CUstream_st")(p(y), p(b), f(0.75), T, n, st)
+    torch.cuda.synchronize()
+    _lib.check()
+    assert torch.equal(y.view(T, n), want)
+
+
+@pytest.mark.parametrize("T,C,rank", [(1, 1, 4), (17, 300, 16), (16, 256, 6), (40, 33, 12)])
+def test_lowrank_decay_tiles(lib, T, C, rank):
+    """Tiles of 16 tokens, rows of w2 by four entries where the rank allows it.  exp and log1p are within 2 units, z within rank + 1
+    roundings of its terms: the bound of the op's other test holds."""
+    from vllm_rs_b200 import ops
+    g = torch.Generator().manual_seed(T * C)
+    low, w2, b = torch.randn(T, rank, generator=g), torch.randn(C, rank, generator=g), torch.randn(C, generator=g) * 4
+    want = torch.sigmoid(low.double() @ w2.double().T + b.double()) ** (1.0 / 16.0)
+    got = ops.lowrank_decay(low.cuda(), w2.cuda(), b.cuda(), 16.0).cpu()
+    assert torch.allclose(got, want.float(), atol=1e-6, rtol=1e-5)

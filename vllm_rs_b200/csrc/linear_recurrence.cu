@@ -1054,16 +1054,19 @@ static void launch_scan(const ScanArgs& a, int num_tokens, cudaStream_t st_) {
 // a_log != NULL (kind 1): out[t, c] = exp(-exp(a_log[c / a_period]) * softplus(z)), the decay of a gated delta rule per
 // head and key channel.
 // grid = (channel blocks, token tiles): a thread owns one channel and kDecayTile tokens; the tokens' low-rank rows sit in
-// shared memory, the channel's row of w2 is read once per tile (each thread whole sectors), the stores are coalesced.
+// shared memory, entry by entry (four tokens per load), the channel's row of w2 is read once per tile (each thread whole sectors),
+// the stores are coalesced.  3001 tokens of 1024 channels, rank 16: 24 us with one token per load, 17 with four.
 constexpr int kDecayTile = 16;
 __global__ void __launch_bounds__(256)
 lowrank_decay_kernel(float* __restrict__ out, const float* __restrict__ low, int ld_low, const float* __restrict__ w2,
                      const float* __restrict__ bias, float inv_tau, const float* __restrict__ a_log, int a_period, int T,
                      int C, int rank) {
-  extern __shared__ float lr[];          // [kDecayTile][rank]
+  extern __shared__ __align__(16) float lr[];          // [rank][kDecayTile]
   const int t0 = blockIdx.y * kDecayTile, nt = min(kDecayTile, T - t0);
-  for (int e = threadIdx.x; e < nt * rank; e += blockDim.x)
-    lr[e] = low[static_cast<size_t>(t0 + e / rank) * ld_low + e % rank];
+  for (int e = threadIdx.x; e < kDecayTile * rank; e += blockDim.x) {
+    const int t = e % kDecayTile;
+    lr[e] = t < nt ? low[static_cast<size_t>(t0 + t) * ld_low + e / kDecayTile] : 0.f;
+  }
   __syncthreads();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= C) return;
@@ -1072,11 +1075,21 @@ lowrank_decay_kernel(float* __restrict__ out, const float* __restrict__ low, int
 #pragma unroll
   for (int i = 0; i < kDecayTile; ++i) z[i] = b;
   const float* w = w2 + static_cast<size_t>(c) * rank;
-  for (int r = 0; r < rank; ++r) {
-    const float wv = w[r];
+  auto add = [&](float wv, int r) {
 #pragma unroll
-    for (int i = 0; i < kDecayTile; ++i) z[i] += wv * lr[(i < nt ? i : 0) * rank + r];
+    for (int i = 0; i < kDecayTile; i += 4) {
+      const float4 l = *reinterpret_cast<const float4*>(lr + r * kDecayTile + i);
+      z[i] += wv * l.x; z[i + 1] += wv * l.y; z[i + 2] += wv * l.z; z[i + 3] += wv * l.w;
+    }
+  };
+  int r = 0;
+  if (rank % 4 == 0 && (reinterpret_cast<uintptr_t>(w2) & 15) == 0) {
+    for (; r < rank; r += 4) {
+      const float4 v = *reinterpret_cast<const float4*>(w + r);
+      add(v.x, r); add(v.y, r + 1); add(v.z, r + 2); add(v.w, r + 3);
+    }
   }
+  for (; r < rank; ++r) add(w[r], r);
 #pragma unroll
   for (int i = 0; i < kDecayTile; ++i) {
     if (i >= nt) break;

@@ -41,6 +41,43 @@ __global__ void embed_f32_kernel(float* __restrict__ x, const T* __restrict__ ta
   }
 }
 
+// The rows alone, eight entries per thread: an entry per access took 16.4 us for 3001 rows of 2048, which HBM
+// moves in 6; this one 10.2.
+template <typename T>
+__global__ void __launch_bounds__(256)
+embed_f32_vec_kernel(float* __restrict__ x, const T* __restrict__ table, const uint32_t* __restrict__ ids, int width, int vocab,
+                     float scale, T* __restrict__ cast_out) {
+  const size_t t = blockIdx.x;
+  uint32_t id = ids[t];
+  if (id >= static_cast<uint32_t>(vocab)) id = 0;
+  const T* row = table + static_cast<size_t>(id) * width;
+  for (int d = threadIdx.x * 8; d < width; d += 256 * 8) {
+    float v[8];
+    if constexpr (std::is_same_v<T, float>) {
+      const float4 a = *reinterpret_cast<const float4*>(row + d), b = *reinterpret_cast<const float4*>(row + d + 4);
+      v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+    } else {
+      const uint4 raw = *reinterpret_cast<const uint4*>(row + d);
+      const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        v[2 * i] = __uint_as_float(w[i] << 16);
+        v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] *= scale;
+    float* o = x + t * width + d;
+    *reinterpret_cast<float4*>(o) = make_float4(v[0], v[1], v[2], v[3]);
+    *reinterpret_cast<float4*>(o + 4) = make_float4(v[4], v[5], v[6], v[7]);
+    if constexpr (!std::is_same_v<T, float>) {
+      if (cast_out)
+        *reinterpret_cast<uint4*>(cast_out + t * width + d) = make_uint4(pack16x2<true>(v[0], v[1]), pack16x2<true>(v[2], v[3]),
+                                                                        pack16x2<true>(v[4], v[5]), pack16x2<true>(v[6], v[7]));
+    }
+  }
+}
+
 // out[r] = x[row(r)] / sqrt(mean(x^2) + eps) * (w_offset + w); rows == nullptr: row(r) = r; ldx: row stride of x
 template <typename T>
 __global__ void resid_rmsnorm_kernel(T* __restrict__ out, const float* __restrict__ x, size_t ldx,
@@ -94,8 +131,8 @@ resid_rmsnorm_vec_kernel(T* __restrict__ out, const float* __restrict__ x, size_
   }
 }
 // x += norm(y), and where the next step on the stream is its norm (next_out), that from the same registers: the row is not read a
-// second time and a launch goes.  HBM / L2 bound.  A step of 3001 rows of 2048 through four layers, 12.2 + 9.2 us (cold) apart: 2463 us,
-// together: 2437.
+// second time and a launch goes.  HBM / L2 bound.  3001 rows of 2048, from HBM: 12.2 + 9.2 us
+// in two launches, 14.4 in one.
 template <typename T, int NV>
 __global__ void __launch_bounds__(256)
 resid_add_rmsnorm_vec_kernel(float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ w, int width, float eps,
@@ -282,6 +319,22 @@ __global__ void resid_add_rmsnorm_kernel(float* __restrict__ x, const float* __r
   }
 }
 
+// The same, four entries per access and a block's entries of the bias in registers over its rows: an entry per access, its column
+// from a 64-bit remainder, took 16.5 us for 3001 rows of 2048 (49 MB: 8 us of HBM);
+// this one 8.
+__global__ void __launch_bounds__(256)
+bias_rows_vec_kernel(float* __restrict__ y, const float* __restrict__ bias, float scale, int n, int T) {
+  const int d = (blockIdx.x * 256 + threadIdx.x) * 4;
+  if (d >= n) return;
+  const float4 b = ld4(bias + d);
+#pragma unroll 4
+  for (int t = blockIdx.y; t < T; t += gridDim.y) {
+    float* p = y + static_cast<size_t>(t) * n + d;
+    float4 v = ld4(p);
+    v.x += scale * b.x; v.y += scale * b.y; v.z += scale * b.z; v.w += scale * b.w;
+    st4(p, v);
+  }
+}
 // y[t, d] += scale * bias[d]
 __global__ void bias_rows_kernel(float* __restrict__ y, const float* __restrict__ bias, float scale, int n, size_t total) {
   for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < total;
@@ -614,6 +667,14 @@ static int flat_grid(size_t total) {
 void launch_embed_f32(float* x, const void* table, const uint32_t* ids, const int64_t* positions, float pos_base, int T,
                       int width, int vocab, float scale, int dt, void* cast_out, cudaStream_t st_) {
   if (T <= 0) return;
+  if (width % 8 == 0 && !(pos_base > 0.f && positions) && aligned16(x, table, cast_out)) {
+    if (dt) embed_f32_vec_kernel<float><<<T, 256, 0, st_>>>(x, (const float*)table, ids, width, vocab, scale, nullptr);
+    else
+      embed_f32_vec_kernel<__nv_bfloat16><<<T, 256, 0, st_>>>(x, (const __nv_bfloat16*)table, ids, width, vocab, scale,
+                                                              (__nv_bfloat16*)cast_out);
+    B200_CUDA_LAUNCH_CHECK();
+    return;
+  }
   if (dt)
     embed_f32_kernel<float><<<T, 256, 0, st_>>>(x, (const float*)table, ids, positions, pos_base, width, vocab, scale,
                                                 nullptr);
@@ -714,6 +775,12 @@ void launch_resid_add_rmsnorm(float* x, const float* y, const float* w, int T, i
 void launch_bias_rows(float* y, const float* bias, float scale, int T, int n, cudaStream_t st_) {
   const size_t total = static_cast<size_t>(T) * n;
   if (total == 0) return;
+  if (n % 4 == 0 && aligned16(y, bias)) {
+    const int per = (n + 1023) / 1024;
+    bias_rows_vec_kernel<<<dim3(per, std::min(T, std::max(1, 8 * sm_count() / per))), 256, 0, st_>>>(y, bias, scale, n, T);
+    B200_CUDA_LAUNCH_CHECK();
+    return;
+  }
   bias_rows_kernel<<<flat_grid(total), 256, 0, st_>>>(y, bias, scale, n, total);
   B200_CUDA_LAUNCH_CHECK();
 }
