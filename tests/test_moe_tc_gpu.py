@@ -97,3 +97,24 @@ def test_buckets_of_many_pairs(lib, T, E, top):
     whole = run(0, T)
     assert torch.equal(whole, torch.cat([run(a, min(a + 1000, T)) for a in range(0, T, 1000)]))
     assert whole.abs().sum() > 0
+
+
+@pytest.mark.parametrize("act", ["silu_gate", "relu2", "clamped"])
+@pytest.mark.parametrize("T,E,skew", [(6000, 3, 0), (5003, 4, 2), (9000, 2, 9)])
+def test_pairs_of_blocks(lib, act, T, E, skew):
+    """Tiles of 256 slots, which two blocks share: buckets that end in either block's half, hold few rows or none, features that end
+    inside a tile.  Every row has the bits that it has in portions of 500 rows, whose tiles are a block's own."""
+    from vllm_rs_b200 import ops
+    g = torch.Generator().manual_seed(T)
+    c = lambda t: t.cuda().contiguous()                                      # noqa: E731
+    D, F = 776, 520
+    wu = c((torch.randn(E, F if act == "relu2" else 2 * F, D, generator=g) / D ** 0.5).bfloat16())
+    wd = c((torch.randn(E, D, F, generator=g) / F ** 0.5).bfloat16())
+    h, x = c(torch.randn(T, D, generator=g).bfloat16()), torch.zeros(T, D).cuda()
+    z = torch.randn(T, E, generator=g) - skew * torch.arange(E).float()
+    w, idx = torch.softmax(z, 1).topk(2 if skew < 9 else 1, 1)
+    w, idx = c(w), c(idx.int())
+    kw = dict(limit=1.5, alpha=1.702, up_add=1.0) if act == "clamped" else {}
+    run = lambda a, b: ops.moe_experts_ex(x[a:b].clone(), h[a:b], idx[a:b], w[a:b], wu, wd, act=act, **kw)      # noqa: E731
+    whole = run(0, T)
+    assert torch.equal(whole, torch.cat([run(a, min(a + 500, T)) for a in range(0, T, 500)])) and float(whole.abs().sum()) > 0

@@ -9,7 +9,8 @@
 // side, so the activation needs no second pass.  Token rows are first gathered into bucket order by a copy of their own (in
 // space that the second product's results take later): gathering inside the product took longer than the product, by TMA
 // gathers of four rows (~90 cycles each) as by cp.async, whose blocks need a wait and a fence on their way to the tensor core
-// (prompt of 4096 rows, 16 experts, first product: 183 us and 103-139 us).  Pairs of blocks on 256 x 256 tiles: 67.5 / 55.4 us.
+// (prompt of 4096 rows, 16 experts, first product: 183 us and 103-139 us).  Two blocks of a cluster may share a tile of 256 slots, each
+// with its own rows and half of the weight rows in shared memory: two thirds of the reads (that prompt's products 71 / 52 -> 66 / 52 us).
 //
 // Measured, mma.sync kernel -> here (whole call): 4096 rows of 2048, 16 experts of 512, 4 chosen: 709 -> 194 us, 32 rows, device time,
 // 67 -> 36; 4096 wide, 32 experts of 1024: 3000 rows 1903 -> 406 us, 32 rows, device time, 202 -> 159.  moe.cu says which products are
@@ -20,6 +21,7 @@
 // in the first product), 8 rows 56.0 / 45.6 / 48.5 (256 / 128 / 64), 300 rows 69.6 / 52.6 / 63.0, 4096 rows 388 / 243 / 187;
 // 4096 wide, 32 experts of 1024: 32 rows 198 / 142 / 150 us, 300 rows 295 / 185 / 177, 3000 rows 1027 / 573 / 405.
 #include "../../include/b200_vllm.h"
+#include <cmath>
 #include "moe_tc.cuh"
 
 namespace b200 {
@@ -31,9 +33,10 @@ constexpr int kABytes = kM * 128;
 constexpr int kPitch = 80, kOutBytes = kEpiWarps * 32 * kPitch;      // a warp's 32 rows x 64 bytes on their way out
 constexpr uint32_t kHiSw128 = (1024 >> 4) | (1u << 14) | (2u << 29);
 
-template <int BN> struct Cfg {
-  static constexpr int kStage = kABytes + BN * 128;
-  static constexpr int kStages = 192 * 1024 / kStage;          // 4 / 6 / 8
+template <int BN, int CG> struct Cfg {                          // CG: blocks that share a tile
+  static constexpr int kWRows = BN / CG;                       // weight rows staged by a block
+  static constexpr int kStage = kABytes + kWRows * 128;
+  static constexpr int kStages = 192 * 1024 / kStage;          // 4 / 6 / 8 (pairs: 6)
   static constexpr int kOutOff = kStages * kStage;
   static constexpr int kBarOff = kOutOff + kOutBytes;
   static constexpr int kSmem = kBarOff + (2 * kStages + 5) * 8 + 16 + (kMaxExperts + 1) * 4 + 1024;
@@ -47,31 +50,51 @@ struct Args {
   int* err;
 };
 
+template <int CG>
 __device__ __forceinline__ void mma_ss(uint32_t lead, uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t acc) {
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"
-      "setp.ne.b32 q, %0, 0;\n\tsetp.ne.b32 p, %6, 0;\n\t"
-      "mov.b64 da, {%2, %5};\n\tmov.b64 db, {%3, %5};\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%1], da, db, %4, p;\n\t}\n" ::"r"(lead),
-      "r"(d), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(kHiSw128), "r"(acc)
-      : "memory");
+  if constexpr (CG == 1)
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"
+        "setp.ne.b32 q, %0, 0;\n\tsetp.ne.b32 p, %6, 0;\n\t"
+        "mov.b64 da, {%2, %5};\n\tmov.b64 db, {%3, %5};\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%1], da, db, %4, p;\n\t}\n" ::"r"(lead),
+        "r"(d), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(kHiSw128), "r"(acc)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"
+        "setp.ne.b32 q, %0, 0;\n\tsetp.ne.b32 p, %6, 0;\n\t"
+        "mov.b64 da, {%2, %5};\n\tmov.b64 db, {%3, %5};\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%1], da, db, %4, p;\n\t}\n" ::"r"(lead),
+        "r"(d), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(kHiSw128), "r"(acc)
+        : "memory");
 }
-__device__ __forceinline__ void commit(uint32_t lead, uint64_t* bar) {
-  asm volatile(
-      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %0, 0;\n\t"
-      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%1];\n\t}\n" ::"r"(lead),
-      "r"(smem_u32(bar))
-      : "memory");
+// on this barrier in the blocks of `mask` (one block: its own)
+template <int CG>
+__device__ __forceinline__ void commit(uint32_t lead, uint64_t* bar, uint16_t mask = 3) {
+  if constexpr (CG == 1)
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %0, 0;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%1];\n\t}\n" ::"r"(lead),
+        "r"(smem_u32(bar))
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %0, 0;\n\t"
+        "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%1], %2;\n\t}\n" ::"r"(lead),
+        "r"(smem_u32(bar)), "h"(mask)
+        : "memory");
 }
 
 // ACT as in moe.cu: 0 plain product, fp32 out; 1 SiLU gate, 2 squared ReLU, 3 clamped gate, bf16 out.  Rows in bucket order.  After a wait has given up (*fail) all others return at once and the loops run out.
-template <int ACT, int BN>
+template <int ACT, int BN, int CG>
 __global__ void __launch_bounds__(kThreads, 1)
 grouped_linear_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap tilemap,
                          const __grid_constant__ CUtensorMap wmap, const Args a) {
   constexpr bool GATED = ACT == 1 || ACT == 3;
   constexpr int FN = GATED ? BN / 2 : BN;          // output features of a tile
-  using C = Cfg<BN>;
+  constexpr int TM = kM * CG;                      // rows of a tile
+  using C = Cfg<BN, CG>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + C::kBarOff);
@@ -83,10 +106,11 @@ grouped_linear_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_
   volatile int* fail = reinterpret_cast<volatile int*>(tmem_ptr + 1);
   int* first = reinterpret_cast<int*>(tmem_ptr + 4);         // [E + 1] first row tile of every expert
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const int rank = CG == 2 ? static_cast<int>(cluster_ctarank()) : 0, unit = blockIdx.x / CG, units = gridDim.x / CG;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::kStages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-    for (int s = 0; s < 2; ++s) { mbar_init(&tfull[s], 1); mbar_init(&tempty[s], kEpiWarps); }
+    for (int s = 0; s < 2; ++s) { mbar_init(&tfull[s], 1); mbar_init(&tempty[s], kEpiWarps * CG); }
     mbar_init(drained, 1);
     *fail = 0;
     fence_barrier_init();
@@ -95,14 +119,19 @@ grouped_linear_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_
     prefetch_tmap(&wmap);
   }
   if (warp == 1) {
-    tmem_alloc(tmem_ptr, 2 * BN);
-    tmem_relinquish();
+    if constexpr (CG == 2) {
+      tmem_alloc_cg2(tmem_ptr, 2 * BN);
+      tmem_relinquish_cg2();
+    } else {
+      tmem_alloc(tmem_ptr, 2 * BN);
+      tmem_relinquish();
+    }
   }
   if (warp == 2) {                                 // row tiles before every expert: a scan over the buckets' sizes
     int before = 0;
     for (int e0 = 0; e0 < a.E; e0 += 32) {
       const int e = e0 + lane;
-      const int mine = e < a.E ? (a.off[e + 1] - a.off[e] + kM - 1) / kM : 0;
+      const int mine = e < a.E ? (a.off[e + 1] - a.off[e] + TM - 1) / TM : 0;
       int inc = mine;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -116,6 +145,10 @@ grouped_linear_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_
   }
   tc_fence_before();
   __syncthreads();
+  if constexpr (CG == 2) {                         // the other block's barriers are there
+    cluster_arrive();
+    cluster_wait();
+  }
   tc_fence_after();
   const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_ptr, 0);
   const int ntiles = first[a.E] * a.ntiles_n;
@@ -129,7 +162,7 @@ grouped_linear_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_
       if (first[mid] <= m) lo = mid; else hi = mid - 1;
     }
     const int b = a.off[lo], k = m - first[lo];
-    return Tile{lo, b + k * kM, min(kM, a.off[lo + 1] - b - k * kM), (t - m * a.ntiles_n) * FN};
+    return Tile{lo, b + k * TM, min(TM, a.off[lo + 1] - b - k * TM), (t - m * a.ntiles_n) * FN};
   };
 
   if (warp == 0) {
@@ -137,43 +170,49 @@ grouped_linear_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_
     int s = 0, armed = 0;
     uint32_t ph = 0;
     bool free_ = true;
-    for (int t = blockIdx.x; t < ntiles && free_; t += gridDim.x) {
+    for (int t = unit; t < ntiles && free_; t += units) {
       const Tile w = tile_at(t);
-      const int boxes = (w.rows + kBox - 1) / kBox;
-      const int wrow = w.e * (GATED ? 2 : 1) * a.N + w.n0;
+      // the boxes of this block's rows, and of the tile; a pair's second block has the up rows, or the second half of the plain ones
+      const int all = (w.rows + kBox - 1) / kBox, boxes = min(max(all - rank * (kM / kBox), 0), kM / kBox), s0 = w.s0 + rank * kM;
+      const int wrow = w.e * (GATED ? 2 : 1) * a.N + w.n0 + rank * (GATED ? a.N : C::kWRows);
       for (int kb = 0; kb < a.KB; ++kb) {
         free_ = __all_sync(0xffffffffu, mbar_wait_limited(&empty[s], ph ^ 1, fail, a.err));
         if (!free_) break;                         // a stage that did not come free is not armed again
         uint8_t* ad = smem + s * C::kStage;
         uint8_t* wd = ad + kABytes;
         if (elect_one()) {
-          mbar_arrive_expect_tx(&full[s], boxes * (kBox * 128) + BN * 128);
-          if (GATED) {
-            tma_load_2d(wd, &wmap, &full[s], kb * kK, wrow);
-            tma_load_2d(wd + FN * 128, &wmap, &full[s], kb * kK, wrow + a.N);
+          if constexpr (CG == 2) {                 // both blocks' bytes count on the first one's barrier
+            if (rank == 0) mbar_arrive_expect_tx(&full[s], all * (kBox * 128) + BN * 128);
+            const uint32_t bar = mapa_shared(smem_u32(&full[s]), 0);
+            tma_load_2d_cg2(wd, &wmap, bar, kb * kK, wrow);
+            if (boxes == kM / kBox) tma_load_2d_cg2(ad, &tilemap, bar, kb * kK, s0);
+            else
+              for (int i = 0; i < boxes; ++i) tma_load_2d_cg2(ad + i * (kBox * 128), &amap, bar, kb * kK, s0 + i * kBox);
           } else {
+            mbar_arrive_expect_tx(&full[s], boxes * (kBox * 128) + BN * 128);
             tma_load_2d(wd, &wmap, &full[s], kb * kK, wrow);
+            if (GATED) tma_load_2d(wd + FN * 128, &wmap, &full[s], kb * kK, wrow + a.N);
+            if (boxes == kM / kBox) tma_load_2d(ad, &tilemap, &full[s], kb * kK, s0);      // a copy costs its issue, whatever its size
+            else
+              for (int i = 0; i < boxes; ++i) tma_load_2d(ad + i * (kBox * 128), &amap, &full[s], kb * kK, s0 + i * kBox);
           }
-          if (boxes == kM / kBox) tma_load_2d(ad, &tilemap, &full[s], kb * kK, w.s0);      // a copy costs its issue, whatever its size
-          else
-            for (int i = 0; i < boxes; ++i) tma_load_2d(ad + i * (kBox * 128), &amap, &full[s], kb * kK, w.s0 + i * kBox);
         }
         ++armed;
         if (++s == C::kStages) { s = 0; ph ^= 1; }
       }
     }
-    if (lane == 0 && *fail)                        // copies in flight land before the block ends
+    if (lane == 0 && rank == 0 && *fail)           // copies in flight land before the block ends (a pair's second waits for its first)
       for (int i = 0; i < C::kStages && i < armed; ++i)
         mbar_wait_limited(&full[i], ((armed - 1 - i) / C::kStages) & 1, nullptr, a.err);
     __syncwarp();
-  } else if (warp == 1) {
+  } else if (warp == 1 && rank == 0) {
     // ------------------------------------------------------------ products
-    constexpr uint32_t idesc = make_idesc_f16(kM, BN) | (1u << 7) | (1u << 10);        // bf16 operands
+    constexpr uint32_t idesc = make_idesc_f16(TM, BN) | (1u << 7) | (1u << 10);        // bf16 operands
     const uint32_t lead = elect_one() ? 1u : 0u;
     const uint32_t base = (smem_u32(smem) >> 4) | (1u << 16);
     int s = 0, it = 0;
     uint32_t ph = 0;
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++it) {
+    for (int t = unit; t < ntiles; t += units, ++it) {
       const int buf = it & 1;
       mbar_wait_limited(&tempty[buf], ((it >> 1) & 1) ^ 1, fail, a.err);
       tc_fence_after();
@@ -183,18 +222,18 @@ grouped_linear_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_
         tc_fence_after();
         const uint32_t a_lo = base + s * (C::kStage >> 4), b_lo = a_lo + (kABytes >> 4);
 #pragma unroll
-        for (int ks = 0; ks < kK / 16; ++ks) mma_ss(lead, d, a_lo + ks * 2, b_lo + ks * 2, idesc, (kb | ks) ? 1u : 0u);
-        commit(lead, &empty[s]);
+        for (int ks = 0; ks < kK / 16; ++ks) mma_ss<CG>(lead, d, a_lo + ks * 2, b_lo + ks * 2, idesc, (kb | ks) ? 1u : 0u);
+        commit<CG>(lead, &empty[s]);
         if (++s == C::kStages) { s = 0; ph ^= 1; }
       }
-      commit(lead, &tfull[buf]);
+      commit<CG>(lead, &tfull[buf]);
     }
     if (*fail) {                                   // products in flight end before TMEM is given back
-      commit(lead, drained);
+      commit<CG>(lead, drained, 1);
       mbar_wait_limited(drained, 0, nullptr, a.err);
     }
     __syncwarp();
-  } else {
+  } else if (warp > 1) {
     // ------------------------------------------------------------ activation and stores
     // A warp reads its quarter of the rows, every other 32 columns; four lanes then write 64 bytes of a row.
     const int q4 = warp & 3;
@@ -202,18 +241,18 @@ grouped_linear_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_
     uint8_t* stage = smem + C::kOutOff + (warp - 2) * 32 * kPitch;
     const int sub = (lane & 3) * 16;
     int it = 0;
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++it) {
+    for (int t = unit; t < ntiles; t += units, ++it) {
       const Tile w = tile_at(t);
       const int buf = it & 1;
       mbar_wait_limited(&tfull[buf], (it >> 1) & 1, fail, a.err);
       __syncwarp();
       tc_fence_after();
       const uint32_t src = tmem + lanes + buf * BN;
-      const int rows = w.rows - q4 * 32;               // of this warp
+      const int rows = w.rows - rank * kM - q4 * 32;               // of this warp
       // the staged rows' bytes [b, b + 64) of a tile row whose first column is n0
       auto store = [&](int b, int elem) {
         __syncwarp();
-        uint8_t* dst = static_cast<uint8_t*>(a.out) + (static_cast<size_t>(w.s0 + q4 * 32) * a.N + w.n0) * elem + b + sub;
+        uint8_t* dst = static_cast<uint8_t*>(a.out) + (static_cast<size_t>(w.s0 + rank * kM + q4 * 32) * a.N + w.n0) * elem + b + sub;
         if (w.n0 * elem + b + sub < a.N * elem) {
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
@@ -266,14 +305,25 @@ grouped_linear_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&tempty[buf]);
+      if (lane == 0) {
+        // (what the products overwrite has been read; a release at cluster scope would wait for the results' stores)
+        if (CG == 2 && rank != 0)
+          asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(mapa_shared(smem_u32(&tempty[buf]), 0)) : "memory");
+        else
+          mbar_arrive(&tempty[buf]);
+      }
     }
   }
   tc_fence_before();
   __syncthreads();
+  if constexpr (CG == 2) {                         // neither block goes while the other can reach its memory
+    cluster_arrive();
+    cluster_wait();
+  }
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem, 2 * BN);
+    if constexpr (CG == 2) tmem_dealloc_cg2(tmem, 2 * BN);
+    else tmem_dealloc(tmem, 2 * BN);
   }
 }
 
@@ -285,7 +335,7 @@ static bool map_2d(CUtensorMap* m, const void* base, uint64_t rows, int K, uint3
 }
 
 // a [pairs, K] in bucket order
-template <int ACT, int BN>
+template <int ACT, int BN, int CG = 1>
 static void launch(void* out, const void* a, const void* w, const int32_t* off, int pairs, int E, int K, int N,
                    const b200_expert_act& act, cudaStream_t st) {
   constexpr bool GATED = ACT == 1 || ACT == 3;
@@ -293,16 +343,27 @@ static void launch(void* out, const void* a, const void* w, const int32_t* off, 
   Args g{out, off, E, (K + kK - 1) / kK, N, (N + FN - 1) / FN, act, wait_error_flag()};
   CUtensorMap amap, tilemap, wmap;
   const bool ok = map_2d(&amap, a, pairs, K, kBox) && map_2d(&tilemap, a, pairs, K, kM) &&
-                  map_2d(&wmap, w, static_cast<uint64_t>(E) * (GATED ? 2 : 1) * N, K, FN);
+                  map_2d(&wmap, w, static_cast<uint64_t>(E) * (GATED ? 2 : 1) * N, K, CG == 2 ? BN / 2 : FN);
   if (!ok || !g.err) {
     set_error(2, "grouped_linear_tc: cuTensorMapEncodeTiled failed");
     return;
   }
-  auto kern = grouped_linear_tc_kernel<ACT, BN>;
+  auto kern = grouped_linear_tc_kernel<ACT, BN, CG>;
   static OncePerDevice sized;
-  if (!allow_smem(sized, kern, Cfg<BN>::kSmem)) return;
-  const int most = std::min(pairs, E + pairs / kM) * g.ntiles_n;        // no step has more tiles
-  kern<<<std::min(most, sm_count()), kThreads, Cfg<BN>::kSmem, st>>>(amap, tilemap, wmap, g);
+  if (!allow_smem(sized, kern, Cfg<BN, CG>::kSmem)) return;
+  const int most = std::min(pairs, E + pairs / (kM * CG)) * g.ntiles_n;        // no step has more tiles
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = CG;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(std::min(most, sm_count() / CG) * CG);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = Cfg<BN, CG>::kSmem;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = CG > 1 ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kern, amap, tilemap, wmap, g);
   B200_CUDA_LAUNCH_CHECK();
 }
 
@@ -311,7 +372,18 @@ static void launch_bn(void* out, const void* a, const void* w, const int32_t* of
                       const b200_expert_act& act, cudaStream_t st) {
   constexpr int G = ACT == 1 || ACT == 3 ? 2 : 1;
   const int row_tiles = std::max(std::min(E, pairs), pairs / kM);
-  if (row_tiles * ((N * G + 255) / 256) >= 2 * sm_count()) launch<ACT, 256>(out, a, w, off, pairs, E, K, N, act, st);
+  // Pairs of blocks where their tiles, twice as high, do not cost more turns: a pair's turn takes 0.8 - 0.9 of a block's (first product
+  // of the prompt above 73 000 and 93 000 cycles for four, second 60 000 and 66 000 for eight).  Whole calls, single blocks and pairs, us:
+  // 4096 rows of 2048, 16 experts of 512: 185 and 181, 8192 rows 329 and 314, 2048 rows 110 and 114 (two turns and three); 64
+  // experts of 1024, 8 chosen of 4096 rows 503 and 487; 4096 wide, 32 experts of 1024: 3000 rows 386 and 382, 300 rows 189 and 193.
+  const auto turns = [&](int rows, int slots) {            // half a tile of every bucket is past its end
+    const double tiles = std::max<double>(std::min(E, pairs), E * 0.5 + static_cast<double>(pairs) / rows) * ((N * G + 255) / 256);
+    return std::ceil(tiles / slots);
+  };
+  if (row_tiles * ((N * G + 255) / 256) >= 2 * sm_count()) {
+    if (0.85 * turns(2 * kM, sm_count() / 2) <= turns(kM, sm_count())) launch<ACT, 256, 2>(out, a, w, off, pairs, E, K, N, act, st);
+    else launch<ACT, 256>(out, a, w, off, pairs, E, K, N, act, st);
+  }
   else if (row_tiles * ((N * G + 127) / 128) >= sm_count() * 3 / 4) launch<ACT, 128>(out, a, w, off, pairs, E, K, N, act, st);
   else launch<ACT, 64>(out, a, w, off, pairs, E, K, N, act, st);
 }
