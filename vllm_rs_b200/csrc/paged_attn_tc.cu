@@ -24,7 +24,7 @@
 //
 // Bound: tensor cores for prompts (per page 2 * 128 * 64 * (dim * passes + vdim) flop against 64 * dim * 2 bytes from L2),
 // HBM for steps of few rows, whose keys are split over blocks; window_attn_merge / latent_attn_merge then finish.
-// Measured, mma.sync kernels -> here: window 1024, 4096 rows, 16 heads of 128 over 4: 622 -> 85 us (352 TFLOP/s; what bounds it
+// Measured, this kernel alone (whole calls in turn with others: 88, 557 and 57.5 us), mma.sync kernels -> here: window 1024, 4096 rows, 16 heads of 128 over 4: 622 -> 85 us (352 TFLOP/s; what bounds it
 // is the softmax warps, then the start and the drain of 128 blocks); latent, 2 x 2048 rows, 32 heads, rank 512:
 // 7766 -> 512 us (584 TFLOP/s useful, 885 issued); 32 tokens over 2048 keys, 32 heads over 8: 317 -> 58 us (35 at HBM rate): 256 blocks
 // of 33 pages in turn, with four rows in one pair of the row warps.

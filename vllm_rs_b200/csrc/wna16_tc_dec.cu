@@ -14,6 +14,8 @@
 //     (no synchronous global loads on the critical path); group indices are shifts.
 //   * the weight producer never waits for the previous kernel (weights do not depend on it), so
 //     under PDL the 48 KB ring is already full when the activations become visible.
+// wna16_ts.cu is faster (its head has both at 32 tokens) and takes what it can; here come 8-bit weights of 33 to 64 tokens, groups that
+// units of 128 K do not fit, and operands off 16 bytes.
 // Measured motivation (profiles/r1_gemm_experiments.txt): v3 spent ~10 us per launch in prologue
 // + epilogue and ~900 cycles per 4 KB chunk with the tensor pipe < 10% busy.
 #include <cstdlib>
@@ -67,8 +69,8 @@ struct Cfg {
   static constexpr int kWBytes = kTileN * kChunkK * BITS / 8;            // one (tile, 64-K chunk)
   static constexpr int kXBytes = NT * kChunkK * 2;
   // Copies move SUPER-chunks of 4 consecutive K chunks (one per dequant group): the pipeline
-  // trace (profiles/r1_v7_dec_gemm_trace.txt) showed one producer thread needs ~400 cycles per copy it issues,
-  // which with 4 KB copies WAS the chunk period of the whole kernel.
+  // trace (profiles/r1_v7_dec_gemm_trace.txt) showed ~400 cycles per copy that one producer thread issues behind
+  // lane == 0, which with 4 KB copies WAS the chunk period of the whole kernel (behind elect.sync it is half of that).
   static constexpr int kSuper = kGroups;
   static constexpr int kWSBytes = kSuper * kWBytes;                       // 16 KB (4-bit) / 32 KB
   static constexpr int kXSBytes = kSuper * kXBytes;
