@@ -130,7 +130,9 @@ __global__ void __launch_bounds__(kSortThreads)
 moe_sort_kernel(const int32_t* __restrict__ top_idx, int pairs, int E, int32_t* __restrict__ expert_off,
                 int32_t* __restrict__ pair_of_slot, int32_t* __restrict__ slot_of_pair) {
   extern __shared__ int cnt[];       // [E] counts, then first slots
+  pdl_trigger();
   for (int e = threadIdx.x; e < E; e += kSortThreads) cnt[e] = 0;
+  pdl_wait();
   __syncthreads();
   int ex[kSortHeld], rank[kSortHeld];
 #pragma unroll 1
@@ -412,6 +414,7 @@ moe_combine_kernel(float* __restrict__ x, const float* __restrict__ down, const 
                    const int32_t* __restrict__ top_idx, const float* __restrict__ top_w, int top, int width, int E,
                    const TI* __restrict__ ident, int accumulate) {
   const int t = blockIdx.x, d = (blockIdx.y * 256 + threadIdx.x) * V;
+  pdl_wait();
   if (d >= width) return;
   float acc[V] = {};
   for (int j = 0; j < top; ++j) {
@@ -475,9 +478,8 @@ void launch_moe_sort(const int32_t* top_idx, int pairs, int E, int32_t* expert_o
     set_error(1, "moe_sort: more than 8192 experts");
     return;
   }
-  (pairs <= kSortHeld * kSortThreads ? moe_sort_kernel<true> : moe_sort_kernel<false>)<<<1, kSortThreads, static_cast<size_t>(E) * 4,
-                                                                                       st_>>>(
-      top_idx, pairs, E, expert_off, pair_of_slot, slot_of_pair);
+  launch_pdl(pairs <= kSortHeld * kSortThreads ? moe_sort_kernel<true> : moe_sort_kernel<false>, dim3(1), dim3(kSortThreads),
+             static_cast<size_t>(E) * 4, st_, top_idx, pairs, E, expert_off, pair_of_slot, slot_of_pair);
   B200_CUDA_LAUNCH_CHECK();
 }
 
@@ -547,7 +549,7 @@ void launch_moe_combine(float* x, const float* down, const int32_t* slot_of_pair
   const bool vec = width % 4 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(down)) & 15) == 0;
   const dim3 grid(T, (width + (vec ? 1024 : 256) - 1) / (vec ? 1024 : 256));
   auto run = [&](auto kern, auto* id) {
-    kern<<<grid, 256, 0, st_>>>(x, down, slot_of_pair, top_idx, top_w, top, width, E, id, accumulate);
+    launch_pdl(kern, grid, dim3(256), 0, st_, x, down, slot_of_pair, top_idx, top_w, top, width, E, id, accumulate);
   };
   if (!ident || ident_f32 || dt)
     run(vec ? moe_combine_kernel<float, 4> : moe_combine_kernel<float, 1>, (const float*)ident);

@@ -11,6 +11,8 @@
 // gathers of four rows (~90 cycles each) as by cp.async, whose blocks need a wait and a fence on their way to the tensor core
 // (prompt of 4096 rows, 16 experts, first product: 183 us and 103-139 us).  Two blocks of a cluster may share a tile of 256 slots, each
 // with its own rows and half of the weight rows in shared memory: two thirds of the reads (that prompt's products 71 / 52 -> 66 / 52 us).
+// All launches of a call depend on each other as programs, so that the next one's start lies under the last one's end: 40 rows 56 -> 49 us,
+// 4096 rows 181 -> 176.
 //
 // Measured, mma.sync kernel -> here (whole call): 4096 rows of 2048, 16 experts of 512, 4 chosen: 709 -> 194 us, 32 rows, device time,
 // 67 -> 36; 4096 wide, 32 experts of 1024: 3000 rows 1903 -> 406 us, 32 rows, device time, 202 -> 159.  moe.cu says which products are
@@ -108,6 +110,7 @@ grouped_linear_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int rank = CG == 2 ? static_cast<int>(cluster_ctarank()) : 0, unit = blockIdx.x / CG, units = gridDim.x / CG;
 
+  pdl_trigger();
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::kStages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
     for (int s = 0; s < 2; ++s) { mbar_init(&tfull[s], 1); mbar_init(&tempty[s], kEpiWarps * CG); }
@@ -127,6 +130,7 @@ grouped_linear_tc_kernel(const __grid_constant__ CUtensorMap amap, const __grid_
       tmem_relinquish();
     }
   }
+  pdl_wait();                                      // buckets and rows come from the kernels before, and results go where they read
   if (warp == 2) {                                 // row tiles before every expert: a scan over the buckets' sizes
     int before = 0;
     for (int e0 = 0; e0 < a.E; e0 += 32) {
@@ -352,18 +356,13 @@ static void launch(void* out, const void* a, const void* w, const int32_t* off, 
   static OncePerDevice sized;
   if (!allow_smem(sized, kern, Cfg<BN, CG>::kSmem)) return;
   const int most = std::min(pairs, E + pairs / (kM * CG)) * g.ntiles_n;        // no step has more tiles
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = CG;
-  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(std::min(most, sm_count() / CG) * CG);
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = Cfg<BN, CG>::kSmem;
-  cfg.stream = st;
-  cfg.attrs = &attr;
-  cfg.numAttrs = CG > 1 ? 1 : 0;
-  cudaLaunchKernelEx(&cfg, kern, amap, tilemap, wmap, g);
+  const dim3 grid(std::min(most, sm_count() / CG) * CG);
+  if constexpr (CG == 1) {
+    launch_pdl(kern, grid, dim3(kThreads), Cfg<BN, CG>::kSmem, st, amap, tilemap, wmap, g);
+  } else {
+    const cudaError_t e = launch_pdl_cluster(kern, grid, dim3(kThreads), Cfg<BN, CG>::kSmem, st, dim3(CG), amap, tilemap, wmap, g);
+    if (e != cudaSuccess) set_error(2, cudaGetErrorString(e));
+  }
   B200_CUDA_LAUNCH_CHECK();
 }
 
@@ -394,6 +393,8 @@ bucket_rows_kernel(uint4* __restrict__ out, const uint4* __restrict__ h, const i
                    int top, int n16) {
   const int per = 256 / 32, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;       // a warp per row
   const int slot = blockIdx.x * per + warp;
+  pdl_trigger();
+  pdl_wait();
   if (slot >= pairs) return;
   const uint4* src = h + static_cast<size_t>(pair_of_slot[slot] / top) * n16;
   uint4* dst = out + static_cast<size_t>(slot) * n16;
@@ -417,8 +418,8 @@ bool grouped_linear_tc(int act_kind, void* out, const void* a, const void* w, co
                          reinterpret_cast<uintptr_t>(rows);
   if (K % 8 != 0 || N % 8 != 0 || E > kMaxExperts || (ptrs & 15) || (act_kind != 0 && !rows)) return false;
   if (act_kind != 0) {
-    bucket_rows_kernel<<<(pairs + 7) / 8, 256, 0, st>>>(static_cast<uint4*>(rows), static_cast<const uint4*>(a), pair_of_slot,
-                                                        pairs, top, K / 8);
+    launch_pdl(bucket_rows_kernel, dim3((pairs + 7) / 8), dim3(256), 0, st, static_cast<uint4*>(rows), static_cast<const uint4*>(a),
+               pair_of_slot, pairs, top, K / 8);
     B200_CUDA_LAUNCH_CHECK();
     a = rows;
   }
