@@ -273,7 +273,10 @@ scan_kernel(const ScanArgs a, int num_seqs, int nc, int* err) {
     int mine = 0;                                                      // a sequence for this kernel among the block's
     for (int z = blockIdx.z + tid * gridDim.z; z < num_seqs; z += kAll * gridDim.z)
       mine |= static_cast<int>(a.cu_seqlens_q[seq(z) + 1] - a.cu_seqlens_q[seq(z)]) > kShort;
-    if (!__syncthreads_or(mine)) return;
+    if (!__syncthreads_or(mine)) {
+      pdl_wait();
+      return;
+    }
   }
   if (tid == 0) {
     for (int i = 0; i < kRing; ++i) { mbar_init(&ready[i], 4); mbar_init(&done[i], WW * nc); }
@@ -791,6 +794,7 @@ scan_kernel(const ScanArgs a, int num_seqs, int nc, int* err) {
     cluster_arrive();
     cluster_wait();
   }
+  pdl_wait();          // the short sequences' kernel, of which nothing is read here, ends before this one does
 }
 
 // Portions of up to kShort tokens, token by token.  grid = (column blocks, heads, sequences); 128 threads = 32 rows x 4 columns of
@@ -807,6 +811,7 @@ scan_short_kernel(const ScanArgs a) {
   __shared__ __align__(16) float red[2][4][kOneCols], sums[CT][4][kOneCols];
   __shared__ float sc[CT][3];                          // decay, write strength, what the read-out is multiplied by
   const int h = blockIdx.y, b = blockIdx.z, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, col0 = blockIdx.x * kOneCols;
+  pdl_trigger();
   const int t0 = a.cu_seqlens_q[b], n = static_cast<int>(a.cu_seqlens_q[b + 1]) - t0;
   if (n < 1 || n > kShort) return;
   const bool fresh = static_cast<int>(a.context_lens[b]) == n;
@@ -988,17 +993,25 @@ scan_short_kernel(const ScanArgs a) {
 
 template <typename... P, typename... A>
 static void launch_cluster(void (*kern)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st_, int nc, A... args) {
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = nc;
-  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cudaLaunchAttribute attr[2]{};
+  int na = 0;
+  if (pdl_enabled()) {
+    attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[na++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (nc > 1) {
+    attr[na].id = cudaLaunchAttributeClusterDimension;
+    attr[na].val.clusterDim.x = nc;
+    attr[na].val.clusterDim.y = attr[na].val.clusterDim.z = 1;
+    ++na;
+  }
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st_;
-  cfg.attrs = &attr;
-  cfg.numAttrs = nc > 1 ? 1 : 0;
+  cfg.attrs = attr;
+  cfg.numAttrs = na;
   cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
 }
 template <int DK, int MODE, bool CHAN, int WW>
@@ -1030,11 +1043,13 @@ static void launch_scan_dk(const ScanArgs& a, int num_tokens, cudaStream_t st_) 
   // Which kernel walks a sequence is a matter of its own length, so that its bits do not depend on the step's other sequences.  Up to
   // kShort tokens, whatever their number, token by token is as fast or faster.  Delta rule, heads of 128 x 128, token by token and
   // in blocks: 1 sequence of 16 tokens of 16 heads 9.2 and 9.4 us, 2 10.8 and 10.1, 8 22 and 31, 32 of 12 tokens 51 and 78; of 20
-  // tokens 1 sequence 11.5 and 10.5, 4 18.6 and 20.8.  In a step with longer sequences its walk stands before theirs.
+  // tokens 1 sequence 11.5 and 10.5, 4 18.6 and 20.8.  In a step with longer sequences its walk stood before theirs.
   auto brief = DK == 64 && a.dim <= 32 ? scan_short_kernel<DK == 64 ? 32 : DK, MODE, CHAN> : scan_short_kernel<DK, MODE, CHAN>;
   brief<<<dim3((a.vdim + kOneCols - 1) / kOneCols, a.heads, a.num_seqs), 128, 0, st_>>>(a);
   B200_CUDA_LAUNCH_CHECK();
-  // sequences that can be longer than that: none in a step of few tokens, as of decoded ones
+  // The walk of the longer sequences starts beside it: they share what they read, and nothing that they write (a sequence of 400 tokens and
+  // 32 of 4, 16 heads of 128 x 128, a decay per channel: 105 us one after the other, 100 so; 4096 tokens of the delta rule 441 and 439).
+  // Sequences that can be longer than that: none in a step of few tokens, as of decoded ones
   const int longer = num_tokens > 0 ? std::min(a.num_seqs, num_tokens / (kShort + 1)) : a.num_seqs;
   if (longer == 0) return;
   const bool short_rows = num_tokens > 0 && num_tokens <= 64 * a.num_seqs;
