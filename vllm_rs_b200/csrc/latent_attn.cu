@@ -188,6 +188,7 @@ __global__ void latent_attn_merge_kernel(T* __restrict__ out, const float* __res
                                          const float* __restrict__ part_ml, const float* __restrict__ sink,
                                          const float* __restrict__ gate, int ld_gate, int heads, int kv_rank,
                                          int nsplit) {
+  pdl_wait();                          // (launched under the attention's end by its tensor-core form)
   const size_t th = blockIdx.x;
   const int h = static_cast<int>(th % heads);
   const float* ml = part_ml + th * nsplit * 2;
@@ -531,8 +532,8 @@ void launch_latent_attn(void* out, const float* q_full, const void* cache, const
     if (attn_tc_takes(p)) {
       launch_attn_tc(p, st_);
       if (nsplit > 1) {
-        latent_attn_merge_kernel<__nv_bfloat16><<<T * heads, kv_rank >= 256 ? 256 : 128, 0, st_>>>(
-            (__nv_bfloat16*)out, p.part_o, p.part_ml, sink, gate, ld_gate, heads, kv_rank, nsplit);
+        launch_pdl(latent_attn_merge_kernel<__nv_bfloat16>, dim3(T * heads), dim3(kv_rank >= 256 ? 256 : 128), 0, st_,
+                   (__nv_bfloat16*)out, p.part_o, p.part_ml, sink, gate, ld_gate, heads, kv_rank, nsplit);
         B200_CUDA_LAUNCH_CHECK();
       }
       return;

@@ -415,6 +415,7 @@ __global__ void window_attn_merge_kernel(T* __restrict__ out, const float* __res
                                          const float* __restrict__ part_ml, const float* __restrict__ sink,
                                          const float* __restrict__ gate, int ld_gate, int heads, int vdim, int nsplit,
                                          int gate_elems, int out_f32) {
+  pdl_wait();                          // (launched under the attention's end by its tensor-core form)
   const size_t th = blockIdx.x;
   const int h = static_cast<int>(th % heads);
   const size_t t = th / heads;
@@ -1084,8 +1085,8 @@ void launch_window_attn(void* out, const float* q, const void* k_cache, const vo
     if (attn_tc_takes(p)) {
       launch_attn_tc(p, st_);
       if (nsplit > 1) {
-        window_attn_merge_kernel<__nv_bfloat16><<<T * heads, vdim >= 128 ? 128 : 64, 0, st_>>>(
-            (__nv_bfloat16*)out, p.part_o, p.part_ml, sink, gate, ld_gate, heads, vdim, nsplit, gate_elems, out_f32);
+        launch_pdl(window_attn_merge_kernel<__nv_bfloat16>, dim3(T * heads), dim3(vdim >= 128 ? 128 : 64), 0, st_,
+                   (__nv_bfloat16*)out, p.part_o, p.part_ml, sink, gate, ld_gate, heads, vdim, nsplit, gate_elems, out_f32);
         B200_CUDA_LAUNCH_CHECK();
       }
       return;
