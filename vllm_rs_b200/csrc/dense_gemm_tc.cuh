@@ -3,6 +3,7 @@
 #include <cstdlib>
 #include <cstring>
 
+#include "host/per_device.hpp"
 #include "wna16.cuh"
 
 namespace b200 {
@@ -351,18 +352,19 @@ static bool launch_cfg(const void* x, const void* w, void* c, const __half* bias
     return true;
   }
   auto kern = dense_gemm_tc_kernel<BN, CG, SWAP, OUT_F32, SILU, GATED>;
-  static bool attr_set = false;
-  static int max_units = 0;
-  if (!attr_set) {
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kAlloc);
-    if (CG == 2) {
-      max_units = max_active_clusters(kern, dim3(sm_count()), dim3(kThreads), C::kAlloc, dim3(2, 1, 1));
-      if (max_units <= 0) max_units = sm_count() / 2;
-    } else {
-      max_units = sm_count();
-    }
-    attr_set = true;
+  static OncePerDevice sized;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const cudaError_t set = sized(dev, [&] { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kAlloc); });
+  if (set != cudaSuccess) {
+    set_error(2, cudaGetErrorString(set));
+    return true;
   }
+  static const int max_units = [&] {
+    if (CG == 1) return sm_count();
+    const int n = max_active_clusters(kern, dim3(sm_count()), dim3(kThreads), C::kAlloc, dim3(2, 1, 1));
+    return n > 0 ? n : sm_count() / 2;
+  }();
   const int ntiles = a.tiles_p * a.tiles_q;
   const int units = ntiles < max_units ? ntiles : max_units;
   const cudaError_t e = launch_pdl_cluster(kern, dim3(units * CG), dim3(kThreads), C::kAlloc, st,
