@@ -345,6 +345,10 @@ def test_wna16_decode_of_few_tokens(ops, fmt, bits, K, N, M, group, epi):
     ("awq", 4, 1280, 40960, 50, 128, "none"),       # whole tiles and parts of an odd number of units in one block
     ("awq", 4, 14336, 4096, 16, 128, "none"),       # rings that go round many times
     ("awq", 4, 8192, 1280, 64, 128, "none"),        # seven blocks would meet, but as many clusters do not fit
+    ("awq", 4, 128, 76800, 17, 128, "none"),        # tiles of one unit, four in a block: the issuers take turns
+    ("awq", 4, 128, 40960, 12, 128, "silu"),
+    ("awq", 4, 256, 29440, 33, 128, "none"),        # first and last parts of one unit beside tiles of two
+    ("gptq", 8, 128, 38400, 9, 128, "bias"),
     ("gptq", 8, 384, 256, 1, 128, "silu"),
     ("gptq", 8, 4096, 12288, 32, 128, "none"),
     ("gptq", 8, 14336, 4096, 9, 128, "bias"),

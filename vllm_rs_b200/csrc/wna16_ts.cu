@@ -221,11 +221,11 @@ wna16_ts_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant_
   constexpr int SP = C::kWPairs, XP = C::kXPairs;
   constexpr bool kSilu = EPI == B200_EPI_SILU_MUL, kPairs = kSilu || EPI == kEpiRopeKv;
   extern __shared__ uint8_t smem_raw[];
-  constexpr int kBars = 2 * SP + 2 * XP + 2 * kPlaces + 7;
+  constexpr int kBars = 2 * SP + 2 * XP + 2 * kPlaces + 8;
   __shared__ uint64_t s_bars[kBars];
   uint64_t *const s_wfull = s_bars, *const s_wempty = s_wfull + SP, *const s_xfull = s_wempty + SP, *const s_xempty = s_xfull + XP,
                   *const s_stored = s_xempty + XP, *const s_free = s_stored + kPlaces, *const s_done = s_free + kPlaces,
-                  *const s_flush = s_done + 2, *const s_taken = s_flush + 2, *const s_drained = s_taken + 1, *const s_written = s_drained + 1;
+                  *const s_flush = s_done + 2, *const s_taken = s_flush + 2, *const s_drained = s_taken + 1, *const s_written = s_drained + 2;
   __shared__ uint32_t s_tmem;
   __shared__ int s_last, s_first_last, s_alone, s_fail;
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
@@ -363,13 +363,15 @@ wna16_ts_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant_
         constexpr uint32_t idesc = make_idesc_f16(128, NT);
         const uint32_t d = tmem + h * C::kDCols;
         Ring p{h, 0}, x{0, 0};
-        int i = h, seg = 0;
+        int i = h, turns = 0;                              // tiles in which this issuer had units
         const uint32_t xfull_at = smem_u32(s_xfull), stored_at = smem_u32(s_stored);
         uint32_t x_ok = 0, s_ok = 0;
 #pragma unroll 1
-        for (int ct = first_tile; ct <= last_tile; ++ct, ++seg) {
+        for (int ct = first_tile; ct <= last_tile; ++ct) {
           const int end = min((ct + 1) * U - u0, n);
-          if (seg > 0) wait(smem_u32(s_drained), (seg - 1) & 1, &s_fail, a.err);
+          // Its own accumulator has been read.  A barrier for both issuers would not do: where a tile has one unit, the other issuer and the
+          // readers end it alone, and a phase that this one has not looked at is followed by another of the same parity.
+          if (turns > 0 && i < end) wait(smem_u32(&s_drained[h]), (turns - 1) & 1, &s_fail, a.err);
           uint32_t acc = 0;
 #pragma unroll 1
           for (; i < end; i += 2) {
@@ -393,7 +395,10 @@ wna16_ts_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant_
             tc_commit(free_);
             tc_commit(empty);
           }
-          if (acc) tc_commit(&s_done[h]);
+          if (acc) {
+            tc_commit(&s_done[h]);
+            ++turns;
+          }
         }
         if (*reinterpret_cast<volatile int*>(&s_fail)) {   // products in flight end before their memory is given back
           tc_commit(&s_flush[h]);
@@ -536,16 +541,19 @@ wna16_ts_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant_
         tc_fence_after();
         float acc[T];
         {
-          uint32_t v[T], w[T];
+          uint32_t v[T], w[T] = {};
           tmem_ld<T>(tmem + (both ? 0 : h0) * C::kDCols + lanes + m0, v);
-          tmem_ld<T>(tmem + C::kDCols + lanes + m0, w);
+          if (both) tmem_ld<T>(tmem + C::kDCols + lanes + m0, w);      // (else the other issuer may be in the next tile)
           tc_wait_ld();
 #pragma unroll
-          for (int j = 0; j < T; ++j) acc[j] = __uint_as_float(v[j]) + (both ? __uint_as_float(w[j]) : 0.f);
+          for (int j = 0; j < T; ++j) acc[j] = __uint_as_float(v[j]) + __uint_as_float(w[j]);
         }
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) arrive(smem_u32(s_drained));
+        if (lane == 0) {
+          if (both || h0 == 0) arrive(smem_u32(&s_drained[0]));
+          if (both || h0 == 1) arrive(smem_u32(&s_drained[1]));
+        }
         __syncwarp();
         if (a.cluster) {
           // ---- the blocks of a cluster finalise some rows each, and send each other theirs
