@@ -285,6 +285,7 @@ scan_kernel(const ScanArgs a, int num_seqs, int nc, int* err) {
   }
   // what no token writes is zero and stays it: the triangles' upper halves
   for (int e = tid; e < kRing * 2 * kBT * kBT; e += kAll) sm[e / (2 * kBT * kBT) * SM::kBuf + SM::kMat + e % (2 * kBT * kBT)] = 0.f;
+  fence_proxy_async();                                                 // before the bulk copies that other blocks send there
   __syncthreads();
   if (nc > 1) {                                                        // the others' barriers are there
     cluster_arrive();
