@@ -308,7 +308,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
         }
       }
     }
-    if (lane == 0 && *fail) {               // copies in flight land before the block ends
+    if (elect_one() && *fail) {             // copies in flight, as the lane that made them counted them, land before the block ends
       for (int s = 0; s < a.sk && s < armed_k; ++s)
         mbar_wait_limited(&k_full[s], ((armed_k - 1 - s) / a.sk) & 1, nullptr, a.err);
       for (int s = 0; s < a.sv && s < armed_v; ++s)
