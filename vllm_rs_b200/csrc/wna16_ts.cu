@@ -638,16 +638,17 @@ wna16_ts_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant_
   }
 }
 
-// Clusters of `size` blocks that fit at once (the same on every B200).
-template <class Kernel>
-static int clusters_at_once(Kernel kernel, size_t smem, int size) {
-  static std::atomic<int> known[9];            // + 1
+// Clusters of `size` blocks of this kernel that fit at once (the same on every B200).  What can't be found out is 0, and asked again.
+template <int BITS, int NT, int EPI>
+static int clusters_at_once(int size) {
+  static std::atomic<int> known[9];
   int v = known[size].load(std::memory_order_relaxed);
   if (!v) {
-    v = max_active_clusters(kernel, dim3(size * (sm_count() / size)), dim3(kThreads), smem, dim3(size, 1, 1)) + 1;
+    v = max_active_clusters(wna16_ts_kernel<BITS, NT, EPI>, dim3(size * (sm_count() / size)), dim3(kThreads), Cfg<BITS, NT>::kAlloc,
+                            dim3(size, 1, 1));
     known[size].store(v, std::memory_order_relaxed);
   }
-  return v - 1;
+  return v;
 }
 
 // Ranges cut anywhere, for what takes no clusters.
@@ -667,7 +668,7 @@ static int plan(const WnaParams& p, UnitCut& cut, int& cluster) {
   // SM idle, but a meeting through the L2 costs as much as kMeet units more than one in a cluster.
   constexpr int kMeet = BITS == 4 ? 9 : 6;
   int parts = U < 8 ? U : 8;
-  while (parts > 1 && clusters_at_once(wna16_ts_kernel<BITS, NT, EPI>, Cfg<BITS, NT>::kAlloc, parts) < tiles) --parts;
+  while (parts > 1 && clusters_at_once<BITS, NT, EPI>(parts) < tiles) --parts;
   if (tiles * parts > sm_count() || (U + parts - 1) / parts > cut.share + (cut.rest ? 1 : 0) + kMeet) return grid;
   cluster = parts > 1 ? parts : 0;
   return cut_parts(tiles, U, parts, 0, cut);
