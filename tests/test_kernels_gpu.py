@@ -367,6 +367,20 @@ def test_wna16_units_cut_evenly(ops, fmt, bits, K, N, M, group, epi):
         assert e_new <= e_old * 1.05, (e_new, e_old)               # the same weights, sums in another order
 
 
+@pytest.mark.parametrize("M,variants", [(3, (0, 1, 2, 4, 5, 6, 7, 8, 9)), (12, (0, 2, 4, 5, 6, 7, 8, 9)), (40, (0, 2, 4, 8, 9))])
+def test_wna16_silu_quotient_is_a_division(ops, M, variants):
+    """silu(-88) is -88 / (1 + e^88), whose denominator is above 2^126: small, not zero, so that an infinite up makes it infinite."""
+    K, N, g = 512, 256, 128
+    q, z, s = np.full((K, N), 7, np.uint8), np.full((K // g, N), 8, np.uint8), np.ones((K // g, N), np.float16)
+    q[:, N // 2:], z[:, N // 2:], s[:, N // 2:] = 15, 5, 100                 # gate weights -1, up weights 1000
+    packed = ops.awq_prepack(torch.from_numpy(oq.pack_awq(q)).cuda())
+    sd, zd, ws = torch.from_numpy(s).cuda(), torch.from_numpy(oq.pack_awq(z)).cuda(), ops.wna16_workspace(64, N)
+    x = torch.full((M, K), 88 / K, dtype=F16, device="cuda")                 # exact: the sums are -88 and 88 000, past fp16
+    for v in variants:
+        y = ops.wna16_gemm(x, packed, sd, zd, ws, k=K, n=N, epilogue=ops.EPI_SILU_MUL, variant=v)
+        assert torch.equal(y, torch.full_like(y, -float("inf"))), v
+
+
 @pytest.mark.parametrize("K,N,M,group", [(512, 19456, 3, 128),          # as many tiles as SMs: no kernel splits them
                                          (8192, 9728, 33, 64)])         # more groups than an unsplit tile of wna16_tc_dec.cu stages
 @pytest.mark.parametrize("off_bias,off_y", [(1, 0), (0, 1), (2, 2)])

@@ -303,7 +303,7 @@ __device__ __forceinline__ void epi_row_finish(const SplitOut& o, const EpiCol& 
         // round the two GEMM outputs to fp16 first: the values an unfused pipeline would see
         const float gg = __half2float(__float2half_rn(v0[e]));
         const float uu = __half2float(__float2half_rn(v1[e]));
-        out[e] = __fdividef(gg, 1.f + __expf(-gg)) * uu;       // (a division by subroutine is fetched cold: 1000 cycles)
+        out[e] = gg / (1.f + __expf(-gg)) * uu;
       }
       store_half4(o.c + static_cast<size_t>(m) * (N >> 1) + c.n0, out);
     }

@@ -8,7 +8,8 @@
 // issuers ask early (test_wait) for what they need next, and a unit is as large as tensor memory allows.  It runs at about 450 per unit
 // (4-bit, 32 tokens; 530 with 64); 8-bit units at 740, which is HBM.  The rest is fixed time per launch, some 3 us: the previous
 // kernel's end, the activations' way to shared memory (1300 cycles beside the weights' copies), the meeting of a tile's parts, and code that
-// runs once, as fast as it is fetched (so the finalisers are short loops; a division by subroutine cost 1000 cycles).
+// runs once, as fast as it is fetched (so the finalisers are short loops; SiLU's division takes 0.4 of
+// 20.8 us at 4096 x 28672).
 //
 // Layout.  Sixteen warps dequantise: four groups take the block's units in turn, a warp has 32 channels (its quarter of the tensor memory's
 // lanes) and writes 128 K of them as the A operand; the activations, by TMA, are the B operand.  Even and odd units have an issuer and an
