@@ -498,6 +498,7 @@ __device__ __forceinline__ void split_arrive_and_reduce(const SplitOut& o, int n
 void launch_wna16_gemv(const WnaParams& p, cudaStream_t st);
 bool launch_wna16_tc(const WnaParams& p, cudaStream_t st);   // false: shape unsupported
 bool launch_wna16_tc_dec(const WnaParams& p, cudaStream_t st);   // decode shapes (M <= 64)
+int wna16_tc_dec_turn(const WnaParams& p);                       // chunks of its blocks, if they all run at once
 bool wna16_mma_takes(const WnaParams& p, bool force = false);
 bool launch_wna16_mma(const WnaParams& p, cudaStream_t st, bool force = false);      // 4-bit decode shapes (M <= 16)
 bool launch_wna16_ts(const WnaParams& p, cudaStream_t st, bool force = false);       // decode shapes (M <= 64), units cut evenly over the SMs

@@ -14,8 +14,8 @@
 //     (no synchronous global loads on the critical path); group indices are shifts.
 //   * the weight producer never waits for the previous kernel (weights do not depend on it), so
 //     under PDL the 48 KB ring is already full when the activations become visible.
-// wna16_ts.cu is faster (its head has both at 32 tokens) and takes what it can; here come 8-bit weights of 33 to 64 tokens, groups that
-// units of 128 K do not fit, and operands off 16 bytes.
+// wna16_ts.cu is faster where its blocks take clearly fewer units or meet in clusters (its launch says where).  Here come the calls that one
+// turn of blocks finishes as soon, 8-bit weights of 33 to 64 tokens, groups that units of 128 K do not fit, and operands off 16 bytes.
 // Measured motivation (profiles/r1_gemm_experiments.txt): v3 spent ~10 us per launch in prologue
 // + epilogue and ~900 cycles per 4 KB chunk with the tensor pipe < 10% busy.
 #include <cstdlib>
@@ -683,16 +683,27 @@ extern "C" void b200_debug_set_dec_trace(void* buf) {
 }
 #endif
 
-// Decode-shape entry: false when the shape needs the general kernel (wna16_tc.cu).
-bool launch_wna16_tc_dec(const WnaParams& p, cudaStream_t st) {
+static bool wna16_tc_dec_takes(const WnaParams& p) {
   if (p.M > 64) return false;
   const bool pow2 = p.group_size >= p.K || (p.group_size & (p.group_size - 1)) == 0;
   if (!pow2) return false;
   if (dec::split_of(p).groups > dec::kSZGroups) return false;      // staged in shared memory
   if (p.epilogue == B200_EPI_SILU_MUL && ((p.N / kTileN) & 1)) return false;
   if (p.epilogue == kEpiRopeKv && p.fe && (kTileN % p.fe->D) != 0) return false;
+  return !(B200_DEC_GROUPS > 4 && (p.M > 32 || p.bits != 4));  // five groups: TMEM / shared memory only fit the 4-bit, 32-token tiles
+}
+
+// 64-K chunks of a block where all blocks of this kernel run at once; 0: they do not, or another kernel takes the call.
+int wna16_tc_dec_turn(const WnaParams& p) {
+  if (!wna16_tc_dec_takes(p) || (p.epilogue == B200_EPI_NONE && p.fe && p.fe->ssq_in)) return 0;
+  const dec::Split s = dec::split_of(p);
+  return static_cast<int64_t>(p.N / kTileN) * s.splits <= sm_count() ? s.chunks : 0;
+}
+
+// Decode-shape entry: false when the shape needs the general kernel (wna16_tc.cu).
+bool launch_wna16_tc_dec(const WnaParams& p, cudaStream_t st) {
+  if (!wna16_tc_dec_takes(p)) return false;
 #if B200_DEC_GROUPS > 4
-  if (p.M > 32 || p.bits != 4) return false;   // five groups: TMEM / shared memory only fit the 4-bit, 32-token tiles
   if (p.M <= 16) return dec::launch_nt<4, 16>(p, st);
   return dec::launch_nt<4, 32>(p, st);
 #else

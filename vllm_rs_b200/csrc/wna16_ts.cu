@@ -675,8 +675,33 @@ static int plan(const WnaParams& p, UnitCut& cut, int& cluster) {
   return cut_parts(tiles, U, parts, 0, cut);
 }
 
+// Whether the tile-split kernel (wna16_tc_dec.cu) is the faster one for a call that would be cut so here.  It is a matter of the units that a
+// block takes there and here: there all blocks run at once or not, a block stores its results itself where a tile is one block's and the
+// epilogue is plain, and parts meet in memory; here parts meet in clusters, or in memory for `gain` units more.  1298 plain products, 1092 with
+// SiLU and 776 with a residual, K 128 - 28672, N 1024 - 65536, 1 - 64 tokens: by this rule 20 take more than 1.025 times the faster of the two
+// (1.09 at most); by this kernel alone 484, 20 and 39 of them (128 x 1024, 9 tokens, here and there 2.4 / 1.9 us; 14336 x 1024, 8-bit, 32
+// tokens 16.4 / 8.6; 4096 x 12800, 32 tokens 14.4 / 13.0; 4096 x 9728 11.9 / 12.1); by the other one 689, 1039 and 723.
 template <int BITS, int NT, int EPI>
-static bool launch_epi(const WnaParams& p, cudaStream_t st) {
+static bool tile_split_is_faster(const WnaParams& p, const UnitCut& cut, int cluster) {
+  const int tiles = p.N / kTileN, U = p.K / kUnitK;
+  // (these would go to wna16_mma.cu and wna16_sk.cu)
+  if (p.M <= 16 && static_cast<int64_t>(tiles) * U >= (BITS == 4 ? 4096 : 32 * sm_count())) return false;
+  const int chunks = wna16_tc_dec_turn(p);
+  if (!chunks) return false;
+  const bool unsplit = chunks * kChunkK >= p.K, direct = unsplit && EPI == B200_EPI_NONE;
+  const int mine = cut.share + (cut.rest ? 1 : 0);
+  const int less = chunks - 2 * mine;                      // half units that a block takes less here than there
+  if (cluster) return direct && mine == 1 && NT <= 32;
+  if (!cut.whole) return direct && (BITS == 8 || (U <= 12 && NT <= 32));      // a tile each, as there
+  if (tiles * 10 < cut.parts) return true;                 // sums of more than ten parts
+  if (EPI == B200_EPI_SILU_MUL) return BITS == 8 && NT == 16 && less < 2 * 11;
+  if (unsplit && !direct) return false;
+  const int gain = direct ? (BITS == 4 ? (NT <= 32 ? 13 : 18) : NT == 16 ? 17 : 22) : BITS == 8 && NT == 32 ? 14 : 10;
+  return less < 2 * gain;
+}
+
+template <int BITS, int NT, int EPI>
+static bool launch_epi(const WnaParams& p, cudaStream_t st, bool force) {
   using C = Cfg<BITS, NT>;
   Args a;
   static OncePerDevice sized;
@@ -700,6 +725,7 @@ static bool launch_epi(const WnaParams& p, cudaStream_t st) {
       if ((kUnitK << s) == p.group_size) a.gshift = s;
   a.U = p.K / kUnitK;
   const int grid = plan<BITS, NT, EPI>(p, a.cut, a.cluster);
+  if (!force && tile_split_is_faster<BITS, NT, EPI>(p, a.cut, a.cluster)) return false;
   a.by_U = unit_div(a.U);
   a.rows = a.cluster ? (p.M + a.cluster - 1) / a.cluster : p.M;
   a.o.counters = reinterpret_cast<uint32_t*>(p.workspace);
@@ -737,13 +763,13 @@ static bool launch_epi(const WnaParams& p, cudaStream_t st) {
 }
 
 template <int BITS, int NT>
-static bool launch_nt(const WnaParams& p, cudaStream_t st) {
+static bool launch_nt(const WnaParams& p, cudaStream_t st, bool force) {
   switch (p.epilogue) {
-    case B200_EPI_SILU_MUL: return launch_epi<BITS, NT, B200_EPI_SILU_MUL>(p, st);
-    case kEpiResidNorm: return launch_epi<BITS, NT, kEpiResidNorm>(p, st);
-    case kEpiRopeKv: return launch_epi<BITS, NT, kEpiRopeKv>(p, st);
-    case kEpiPushPeers: return launch_epi<BITS, NT, kEpiPushPeers>(p, st);
-    default: return launch_epi<BITS, NT, B200_EPI_NONE>(p, st);
+    case B200_EPI_SILU_MUL: return launch_epi<BITS, NT, B200_EPI_SILU_MUL>(p, st, force);
+    case kEpiResidNorm: return launch_epi<BITS, NT, kEpiResidNorm>(p, st, force);
+    case kEpiRopeKv: return launch_epi<BITS, NT, kEpiRopeKv>(p, st, force);
+    case kEpiPushPeers: return launch_epi<BITS, NT, kEpiPushPeers>(p, st, force);
+    default: return launch_epi<BITS, NT, B200_EPI_NONE>(p, st, force);
   }
 }
 
@@ -754,8 +780,10 @@ static bool launch_nt(const WnaParams& p, cudaStream_t st) {
 // 14336 x 4096 11.5 / 12.1, 4096 x 4096 5.9 / 5.9).  From 9 on this kernel is faster at 16 / 32 / 64 tokens (here and the faster of the others:
 // 4096 x 28672 18.4 / 25.5, 19.5 / 30.2, 23.1 / 36.7; 14336 x 4096 11.7 / 13.3, 12.0 / 13.6, 12.8 / 16.7; 2048 x 2048 4.2 / 5.6, 4.5 / 5.9,
 // 5.2 / 9.5), but for many short tiles, where a block finalises two or three (16 tokens: 2048 x 34816 14.8 / 14.4, 512 x 131072 19.9 / 17.0,
-// though 1024 x 65536 15.8 / 16.5; 8-bit, 32 tokens, 2048 x 34816 18.4 / 17.0): those stay where they were.  8-bit weights: 16 / 32 tokens
-// 4096 x 28672 23.5 / 28.6, 24.2 / 30.5, 14336 x 4096 13.3 / 13.3, 13.7 / 14.1; with 64 tokens the rings would be too short (14336 x 4096 19.4 / 17.3).
+// though 1024 x 65536 15.8 / 16.5; 8-bit, 32 tokens, 2048 x 34816 18.4 / 17.0): those stay where they were, at up to 16 tokens with
+// wna16_mma.cu and wna16_sk.cu, which take no others of these by themselves.  8-bit weights, 1 / 16 / 32 tokens: 4096 x 28672 24.1 / 26.9,
+// 25.1 / 28.6, 26.6 / 30.7, 14336 x 4096 14.0 / 15.0, 14.4 / 15.5, 15.0 / 16.7, 4096 x 4096 6.7 / 7.5, 7.0 / 8.0, 7.4 / 8.7; with 64 tokens
+// the rings would be too short (14336 x 4096 19.4 / 17.3).  tile_split_is_faster has the sizes at which it is the tile-split kernel's turn.
 bool launch_wna16_ts(const WnaParams& p, cudaStream_t st, bool force) {
   if (p.M > (p.bits == 4 ? 64 : 32) || p.K % ts::kUnitK != 0 || p.N % kTileN != 0 || p.no_split) return false;
   const int64_t tiles = p.N / kTileN, U = p.K / ts::kUnitK;
@@ -777,8 +805,8 @@ bool launch_wna16_ts(const WnaParams& p, cudaStream_t st, bool force) {
   if (U * p.N >= int64_t{1} << 31) return false;             // offsets of scales
   UnitCut cut;
   if (ts::cut_of(p, cut) <= 0) return false;
-  if (p.bits == 4) return p.M <= 16 ? ts::launch_nt<4, 16>(p, st) : p.M <= 32 ? ts::launch_nt<4, 32>(p, st) : ts::launch_nt<4, 64>(p, st);
-  return p.M <= 16 ? ts::launch_nt<8, 16>(p, st) : ts::launch_nt<8, 32>(p, st);
+  if (p.bits == 4) return p.M <= 16 ? ts::launch_nt<4, 16>(p, st, force) : p.M <= 32 ? ts::launch_nt<4, 32>(p, st, force) : ts::launch_nt<4, 64>(p, st, force);
+  return p.M <= 16 ? ts::launch_nt<8, 16>(p, st, force) : ts::launch_nt<8, 32>(p, st, force);
 }
 
 }  // namespace b200
