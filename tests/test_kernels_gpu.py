@@ -199,8 +199,9 @@ def _wna_case(K, N, M, fmt, bits, seed, group=128):
     return qw, qz, s, torch.from_numpy(W), x
 
 
-# flat GEMV / tile-split tcgen05 decode kernel (M <= 64) / general tcgen05 / stream-K tcgen05 decode kernel (M <= 32)
-@pytest.mark.parametrize("variant", [1, 2, 4, 5, 6])
+# flat GEMV / unit or tile-split tcgen05 decode kernel (M <= 64) / general tcgen05 / stream-K tcgen05 decode kernel (M <= 32), two
+# flavours / unit kernel (8-bit: M <= 32) / tile-split kernel
+@pytest.mark.parametrize("variant", [1, 2, 4, 5, 6, 8, 9])
 @pytest.mark.parametrize("fmt,bits,K,N,M", [
     ("awq", 4, 4096, 1024, 1), ("awq", 4, 4096, 6144, 32), ("awq", 4, 14336, 4096, 5),
     ("gptq", 4, 2048, 256, 3), ("gptq_sym", 4, 1024, 512, 16), ("gptq", 8, 2048, 512, 7),
@@ -209,7 +210,7 @@ def _wna_case(K, N, M, fmt, bits, seed, group=128):
 def test_wna16_gemm(ops, fmt, bits, K, N, M, variant):
     if variant >= 2 and not _tc_available(ops):
         pytest.skip("tcgen05 variant not built yet")
-    if variant >= 5 and M > 32:
+    if variant in (5, 6) and M > 32:
         pytest.skip("the stream-K decode kernel takes M <= 32")
     if variant == 6 and bits != 4:
         pytest.skip("the mma.sync stream-K flavour is 4-bit only")
@@ -278,7 +279,7 @@ def test_wna16_streamk_decode(ops, fmt, bits, K, N, M, group, epi, variant):
         gi = np.arange(K) // group
         wexact = (q.astype(np.float64) - z[gi]) * s[gi].astype(np.float64)
         truth = torch.from_numpy(x.numpy().astype(np.float64) @ wexact)
-        y_old = ops.wna16_gemm(x.cuda(), packed, sd, zd, ws, variant=2, **kw)
+        y_old = ops.wna16_gemm(x.cuda(), packed, sd, zd, ws, variant=9, **kw)
         e_new = (y.cpu().double() - truth).abs().max().item()
         e_old = (y_old.cpu().double() - truth).abs().max().item()
         assert e_new <= e_old + 5e-4, (e_new, e_old)
@@ -322,7 +323,7 @@ def _wna_run(ops, fmt, bits, K, N, M, group, epi, seed):
     ("awq", 4, 2048, 34816, 16, 128, "none"),      # as many units as the sixteen tokens want
 ])
 def test_wna16_decode_of_few_tokens(ops, fmt, bits, K, N, M, group, epi):
-    """wna16_mma.cu (variant 7, and what variant 0 takes at up to 16 tokens)."""
+    """wna16_mma.cu (variant 7, and what variant 0 takes at up to 8 tokens, and to 16 of wide products of short K)."""
     call, ref, truth = _wna_run(ops, fmt, bits, K, N, M, group, epi, K + N + M)
     y = call(7)
     _close(y, ref, 2e-3, 4e-3 if epi == "silu" else 2e-3)          # the bound of the other variants: fp32 sums, fp16 results
@@ -331,7 +332,7 @@ def test_wna16_decode_of_few_tokens(ops, fmt, bits, K, N, M, group, epi):
         assert torch.equal(call(0), y)
     if epi == "none" and "sym" not in fmt:
         t = truth()
-        e_new, e_old = ((v.cpu().double() - t).norm() for v in (y, call(2)))
+        e_new, e_old = ((v.cpu().double() - t).norm() for v in (y, call(9)))
         assert e_new <= e_old * 1.05, (e_new, e_old)               # the same weights, sums in another order
 
 
@@ -561,9 +562,21 @@ def test_wna16_units_push_to_peers(ops, K, N, M):
 def test_wna16_decode_of_many_groups(ops, K, N, M, group):
     """wna16_tc_dec.cu where one K piece has exactly as many quantisation groups as are staged, and where it takes more pieces."""
     call, ref, _ = _wna_run(ops, "awq", 4, K, N, M, group, "none", K + N + M)
-    y = call(2)
+    y = call(9)
     _close(y, ref, 2e-3, 2e-3)
-    assert torch.equal(call(0), y)
+    assert torch.equal(call(9), y)
+    if group < 128:                                                # (of 128 and more wna16_ts.cu takes them)
+        assert torch.equal(call(0), y)
+
+
+@pytest.mark.parametrize("K,N,M,epi", [(2048, 512, 33, "bias"), (14336, 4096, 64, "none"), (4096, 28672, 48, "silu"), (128, 256, 40, "silu"),
+                                       (1024, 20480, 64, "bias"), (4096, 1280, 57, "none")])
+def test_wna16_eight_bits_of_many_tokens(ops, K, N, M, epi):
+    """8-bit weights of 33 to 64 tokens, which are wna16_tc_dec.cu's: pieces that meet, tiles that store themselves, pairs of tiles."""
+    call, ref, _ = _wna_run(ops, "gptq", 8, K, N, M, 128, epi, K + N + M)
+    y = call(9)
+    _close(y, ref, 2e-3, 4e-3 if epi == "silu" else 2e-3)          # the bound of the other variants: fp32 sums, fp16 results
+    assert torch.equal(call(9), y) and torch.equal(call(0), y)
 
 
 @pytest.mark.parametrize("fmt,bits,K,N,M,epi,unit", [

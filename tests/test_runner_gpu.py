@@ -438,20 +438,26 @@ _D128 = dict(num_heads=4, num_kv_heads=2, head_dim=128)
 
 
 @pytest.mark.parametrize("nseq,shape", [
-    # the tile-split kernel's finalisers, 17 to 64 tokens
+    # the unit kernel's finalisers, 9 to 64 tokens of 4-bit weights
     (17, dict(hidden=512, inter=1024, num_layers=2, **_D64)), (32, dict(hidden=512, inter=1024, num_layers=2, **_D128)),
     (32, dict(hidden=512, inter=1024, num_layers=2, **_D64)), (48, dict(hidden=512, inter=1024, num_layers=2, **_D128)),
-    # the per-warp kernel's, 9 to 16 tokens: projections of at least 4096 units of 128 x 128 (q|k|v 5120, o 4096; gate|up 4096)
+    # the same, with projections of at least 4096 units of 128 x 128 (q|k|v 5120, o 4096; gate|up 4096)
     (12, dict(hidden=8192, inter=1024, num_layers=2, num_heads=64, num_kv_heads=8, head_dim=128)),
     (12, dict(hidden=8192, inter=4096, num_layers=1, num_heads=128, num_kv_heads=16, head_dim=64)),
+    # the per-warp kernel's, 9 to 16 tokens: gate|up of at least 4096 units in tiles of at most 16
+    (12, dict(hidden=1024, inter=32768, num_layers=1, **_D64)),
+    # the tile-split kernel's: 8-bit weights of 33 to 64 tokens
+    (33, dict(fmt="gptq8", hidden=512, inter=1024, num_layers=2, **_D64)), (48, dict(fmt="gptq8", hidden=512, inter=1024, num_layers=2, **_D128)),
 ])
 def test_decode_step_of_larger_batches(lib, nseq, shape):
     """The fused plan's products (RoPE and cache write, residual and sums of squares, folded norms, SiLU) for the batches that
     neither the small toys nor the rank shapes above reach: one step, the bars of the other decode tests."""
     from vllm_rs_b200 import engine
+    shape = dict(shape)
+    fmt = shape.pop("fmt", "awq")
     cfg = om.ModelConfig(vocab=1024, rope_theta=10000.0, rms_eps=1e-5, max_pos=2048, qkv_bias=nseq == 17, **shape)
     NB, MAXBLK = 2 * nseq + 2, 2
-    oracle, runner = _build(cfg, "awq", seed=nseq, num_blocks=NB, max_batch=nseq, max_blocks=MAXBLK)
+    oracle, runner = _build(cfg, fmt, seed=nseq, num_blocks=NB, max_batch=nseq, max_blocks=MAXBLK)
     with om.exact_mode():
         exact = om.LlamaOracle(cfg, oracle.w, NB)
     osch, csch = osched.Scheduler(NB, 64, nseq), engine.Scheduler(NB, 64, nseq)

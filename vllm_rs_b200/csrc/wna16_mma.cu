@@ -644,8 +644,8 @@ static bool launch_nt(const WnaParams& p, cudaStream_t st) {
 }  // namespace wm
 
 // Decode batches of 4-bit weights: false when the call needs another kernel.  `force`: whether or not it is the faster one.
-// Up to 8 tokens it is at every size measured, at 9 - 16, where the products take twice the issue slots, from 4096 units on.
-// us at 1 / 16 tokens, here and the faster of the other two: 4096 x 6144 7.2 / 9.3 and 8.5 / 8.9, 4096 x 4096 5.7 / 7.6 and
+// Up to 8 tokens it is at every size measured.  At 9 - 16, where the products take twice the issue slots, from 4096 units on, of which
+// wna16_ts.cu comes first for all but K <= 2048 (N from 32768 on) and results off 8 bytes.  us at 1 / 16 tokens, here and the faster of the other two: 4096 x 6144 7.2 / 9.3 and 8.5 / 8.9, 4096 x 4096 5.7 / 7.6 and
 // 7.1 / 7.5, 4096 x 28672 21.0 / 24.9 and 25.7 / 29.1, 14336 x 4096 12.2 / 14.8 and 13.8 / 14.3, 2048 x 2560 4.5 / 6.2 and 5.4 / 6.0,
 // 5632 x 2048 6.5 / 8.2 and 6.2 / 6.6, 8192 x 10240 15.6 / 18.1 and 17.9 / 20.0, 8192 x 57344 65 / 75 and 100 / 102, 28672 x 8192
 // 35.8 / 41.5 and 38.3 / 41.0.  (8-bit weights stay with those: a unit is twice the bytes, one block per SM: 4096 x 28672 35 and 28.)
