@@ -1,8 +1,10 @@
 """Approximations that kernels use, from their constants in the source, against 64 bits."""
+import ctypes
 import re
 from pathlib import Path
 
 import numpy as np
+import pytest
 
 CSRC = Path(__file__).resolve().parent.parent / "vllm_rs_b200" / "csrc"
 
@@ -39,3 +41,14 @@ def test_swizzled_places_begin_the_shared_memory():
     no static one in front."""
     src = (CSRC / "paged_attn_tc.cu").read_text()
     assert re.findall(r"^.*__shared__.*$", src, re.M) == ["  extern __shared__ __align__(1024) uint8_t smem[];"]
+
+
+@pytest.mark.parametrize("T,ff,K,own", [(3001, 5632, 2048, True), (1000, 5632, 2048, True), (256, 5632, 2048, False), (300, 512, 2048, False),
+                                        (3001, 512, 2048, False), (300, 11008, 2048, False), (512, 11008, 2048, True),
+                                        (1000, 5632, 1024, False), (3001, 5632, 1024, True), (1500, 2816, 4096, True), (129, 8, 64, False)])
+def test_gated_rows_take_the_faster_way(T, ff, K, own):
+    """Sizes whose times stand on the one side or the other, by 5 % at least, of the library's and a pass over its results."""
+    from vllm_rs_b200 import _lib
+    pays = getattr(_lib.lib(), "_ZN4b20016dense_gated_paysEiiii")
+    pays.restype = ctypes.c_bool
+    assert pays(T, ff, K, 74) == own

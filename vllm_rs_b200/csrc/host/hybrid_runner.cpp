@@ -616,10 +616,16 @@ static void run_mixer(b200_hybrid* r, const b200_hybrid_layer& l, const int64_t*
   }
 }
 
+// SiLU-gated rows in one launch where that is the faster way; false: not made
+static bool gated_rows(b200_hybrid* r, const b200_hybrid_layer& l, int T, cudaStream_t st) {
+  const b200_hybrid_config& c = r->cfg;
+  return dense_gated_pays(T, l.shared_ff, c.width, sm_count() / 2) &&
+         launch_dense_gated(r->hin, l.w_shared_gate_up, r->sha, T, l.shared_ff, c.width, c.dt, st);
+}
 // dense gated feed-forward of a sandwich layer: y = W_down (silu(W_gate h) * (W_up h))
 static void dense_ffn(b200_hybrid* r, const b200_hybrid_layer& l, int T, cudaStream_t st) {
   const b200_hybrid_config& c = r->cfg;
-  if (!launch_dense_gated(r->hin, l.w_shared_gate_up, r->sha, T, l.shared_ff, c.width, c.dt, st)) {
+  if (!gated_rows(r, l, T, st)) {
     gemm_f32out(r->hin, c.width, 0, l.w_shared_gate_up, c.width, 0, r->sh, 2 * l.shared_ff, 0, T, 2 * l.shared_ff, c.width, 1,
                 0.f, 0, c.dt, st);
     launch_silu_mul_f32(r->sha, r->sh, T, l.shared_ff, c.dt, st);
@@ -658,7 +664,7 @@ static void feed_forward(b200_hybrid* r, const b200_hybrid_layer& l, int T, floa
   if (l.shared_ff > 0) {
     // SiLU-gated: [gate | up] rows; squared ReLU, GELU: up rows, closed by the one row of the token's gate where there is one
     const int rows = l.shared_act == 0 ? 2 * l.shared_ff : l.shared_ff + (l.shared_gated ? 1 : 0);
-    const bool gated = l.shared_act == 0 && launch_dense_gated(r->hin, l.w_shared_gate_up, r->sha, T, l.shared_ff, c.width, c.dt, st);
+    const bool gated = l.shared_act == 0 && gated_rows(r, l, T, st);
     if (!gated) gemm_f32out(r->hin, c.width, 0, l.w_shared_gate_up, c.width, 0, r->sh, rows, 0, T, rows, c.width, 1, 0.f, 0, c.dt, st);
     if (!gated && l.shared_act == 0)
       launch_silu_mul_f32(r->sha, r->sh, T, l.shared_ff, c.dt, st);

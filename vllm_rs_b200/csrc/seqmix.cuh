@@ -101,6 +101,7 @@ void launch_gate_rows(void* out, const float* in, const float* gate, int ld_gate
 // rotary positions on `heads` heads of `dim` entries in place (fp32 rows with stride ld)
 void launch_rotary_rows(float* x, int ld, const double* rot_freq, float rot_mag, int rot_half, const int64_t* positions,
                         int T, int heads, int dim, int rot_dims, cudaStream_t st);
+bool dense_gated_pays(int T, int ff, int K, int pairs);
 bool launch_dense_gated(const void* x, const void* w, void* out, int T, int ff, int K, int dt, cudaStream_t st);
 void launch_silu_mul_f32(void* out, const float* gate_up, int T, int ff, int dt, cudaStream_t st);
 // out [T, ff] = act(up[t, d] + bias[d]) (* sigmoid(up[t, gate_col]) when gate_col >= 0); act 1: relu(.)^2, 2: exact GELU;
