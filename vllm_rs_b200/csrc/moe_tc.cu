@@ -380,7 +380,8 @@ static void launch_bn(void* out, const void* a, const void* w, const int32_t* of
     return std::ceil(tiles / slots);
   };
   if (row_tiles * ((N * G + 255) / 256) >= 2 * sm_count()) {
-    if (0.85 * turns(2 * kM, sm_count() / 2) <= turns(kM, sm_count())) launch<ACT, 256, 2>(out, a, w, off, pairs, E, K, N, act, st);
+    // (buckets of fewer rows than a pair's tile leave its second block idle: 1000 rows, 8 of 64 experts, 218 single and 236)
+    if (pairs >= 2 * kM * E && 0.85 * turns(2 * kM, sm_count() / 2) <= turns(kM, sm_count())) launch<ACT, 256, 2>(out, a, w, off, pairs, E, K, N, act, st);
     else launch<ACT, 256>(out, a, w, off, pairs, E, K, N, act, st);
   }
   else if (row_tiles * ((N * G + 127) / 128) >= sm_count() * 3 / 4) launch<ACT, 128>(out, a, w, off, pairs, E, K, N, act, st);
