@@ -532,9 +532,8 @@ void launch_latent_attn(void* out, const float* q_full, const void* cache, const
     if (attn_tc_takes(p)) {
       launch_attn_tc(p, st_);
       if (nsplit > 1) {
-        launch_pdl(latent_attn_merge_kernel<__nv_bfloat16>, dim3(T * heads), dim3(kv_rank >= 256 ? 256 : 128), 0, st_,
-                   (__nv_bfloat16*)out, p.part_o, p.part_ml, sink, gate, ld_gate, heads, kv_rank, nsplit);
-        B200_CUDA_LAUNCH_CHECK();
+        launch_attn_merge(latent_attn_merge_kernel<__nv_bfloat16>, T * heads, kv_rank >= 256 ? 256 : 128, st_, (__nv_bfloat16*)out,
+                          p.part_o, p.part_ml, sink, gate, ld_gate, heads, kv_rank, nsplit);
       }
       return;
     }

@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(kThreads, 2)
 attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap tmap,
                const __grid_constant__ CUtensorMap vmap, const __grid_constant__ Args a) {
   const AttnTcProblem& p = a.p;
-  pdl_trigger();       // the merge of split keys may take its place (one decoded token over 2000 keys of 16 heads: 21.5 -> 19.5 us)
+  pdl_trigger();       // the merge of split keys may start (launch_attn_merge)
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int G = a.group, kvh = blockIdx.y, vh = kvh % p.v_heads;
   // ---- which tokens: tile (gridDim.x - 1 - blockIdx.x) of the sequences' tiles, so that the latest (longest) go first

@@ -33,5 +33,14 @@ bool attn_tc_takes(const AttnTcProblem& p);
 // longest context, 0 where that is not known
 int attn_tc_splits(int T, int kv_heads, int vdim, int shared_kv, int window, int keep_first, int max_blocks);
 void launch_attn_tc(const AttnTcProblem& p, cudaStream_t st);
+// The merge of split keys, one block per token and head, right after launch_attn_tc.  Few blocks start under the attention's end (as dependents of
+// it); more would all wait on the SMs that the attention leaves idle, and then share those.  us, plain and as dependents: one token over
+// 2047 latent keys, 32 blocks, 24.9 and 22.8, four tokens, 128 blocks, 26.6 and 30.2; 8 tokens over 2048 keys, 256 blocks, 24.7 and 26.1.
+template <typename... P, typename... A>
+inline void launch_attn_merge(void (*kern)(P...), int blocks, int threads, cudaStream_t st, A... args) {
+  if (blocks <= 64) launch_pdl(kern, dim3(blocks), dim3(threads), 0, st, args...);
+  else kern<<<blocks, threads, 0, st>>>(static_cast<P>(args)...);
+  B200_CUDA_LAUNCH_CHECK();
+}
 
 }  // namespace b200

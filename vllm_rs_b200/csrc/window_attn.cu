@@ -1085,9 +1085,8 @@ void launch_window_attn(void* out, const float* q, const void* k_cache, const vo
     if (attn_tc_takes(p)) {
       launch_attn_tc(p, st_);
       if (nsplit > 1) {
-        launch_pdl(window_attn_merge_kernel<__nv_bfloat16>, dim3(T * heads), dim3(vdim >= 128 ? 128 : 64), 0, st_,
-                   (__nv_bfloat16*)out, p.part_o, p.part_ml, sink, gate, ld_gate, heads, vdim, nsplit, gate_elems, out_f32);
-        B200_CUDA_LAUNCH_CHECK();
+        launch_attn_merge(window_attn_merge_kernel<__nv_bfloat16>, T * heads, vdim >= 128 ? 128 : 64, st_, (__nv_bfloat16*)out,
+                          p.part_o, p.part_ml, sink, gate, ld_gate, heads, vdim, nsplit, gate_elems, out_f32);
       }
       return;
     }
