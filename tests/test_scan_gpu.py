@@ -108,6 +108,32 @@ def test_shared_preparation(lib, kind, H, G, d, e, lens):
     test_scans(lib, kind, H, G, d, e, lens)
 
 
+@pytest.mark.parametrize("d,e", [(128, 128), (256, 64)])
+@pytest.mark.parametrize("kind", ["delta", "decay"])
+def test_long_portion_beside_decoded_tokens(lib, kind, d, e):
+    """Short sequences on average with a long one among them go to two launches by their length, and every one has the bits that it has
+    alone (one launch, shared or not)."""
+    from vllm_rs_b200 import ops
+    lens, H, G = [1, 600, 20, 1, 113, 64, 1, 65, 16, 17, 33, 112, 0, 1] + [1] * 30, 4, 2 if kind == "delta" else 4
+    g = torch.Generator().manual_seed(d)
+    r = lambda *s: torch.randn(*s, generator=g).cuda()                        # noqa: E731
+    T, n = sum(lens), len(lens)
+    q, k, v, b, a, alog, dtb, state = r(T, G, d), r(T, G, d), r(T, H, e), r(T, H), r(T, H), r(H) - 1, r(H), r(n, H, d, e)
+    dec = torch.linspace(0.9, 1.0, H).cuda()
+
+    def run(i, j, st):
+        at, T = sum(lens[:i]), sum(lens[i:j])
+        x = [t[at:at + T] for t in (q, k, v, b, a)]
+        tail = (st, torch.arange(i, j).int().cuda(), _i32([sum(lens[i:m]) for m in range(i, j + 1)]), _i32([m + 3 for m in lens[i:j]]))
+        if kind == "delta":
+            return ops.delta_rule(*x, alog, dtb, *tail)
+        return ops.decay_attn(*x[:3], *tail, head_decay=dec, k_scale=0.1)
+    one, many = state.clone(), state.clone()
+    got = run(0, n, many)
+    want = torch.cat([run(i, i + 1, one) for i in range(n) if lens[i]])
+    assert torch.equal(got, want) and torch.equal(many, one)
+
+
 def test_operands_as_they_lie(lib):
     """Views with other strides and one row per token (the form that mixed types take) give the same bits as packed operands."""
     from vllm_rs_b200 import _lib, ops

@@ -223,7 +223,7 @@ __device__ __forceinline__ bool wait_cluster(uint64_t* bar, uint32_t parity, vol
   }
 }
 
-// Portions of more than kShort tokens.  grid = (column blocks, heads, runs of sequences); a block walks its sequences one after
+// Portions of more than `above` tokens, up to `to`.  grid = (column blocks, heads, runs of sequences); a block walks its sequences one after
 // another.  The first WW warps each own four columns of S: a lane holds DK / 32 neighbouring rows of them in registers, so that
 // a key or query row is read once from shared memory for four columns (one column per lane made these reads the bound: 512
 // bytes of registers per load and warp).  Two groups of four warps prepare blocks of tokens under the walks of the blocks before: rows read a
@@ -241,7 +241,7 @@ __device__ __forceinline__ bool wait_cluster(uint64_t* bar, uint32_t parity, vol
 // meet under the update (665 and 424 us with both in turn).
 template <int DK, int MODE, bool CHAN, int WW>
 __global__ void __launch_bounds__(WW * 32 + 256, 1)
-scan_kernel(const ScanArgs a, int num_seqs, int nc, int* err) {
+scan_kernel(const ScanArgs a, int num_seqs, int above, int to, int nc, int* err) {
   using SM = ScanSmem<DK, CHAN, WW>;
   constexpr int CH = DK / 32, COLS = SM::kCols;
   constexpr bool BACK = MODE != kDelta || WW == 8;                     // rows of the triangles from the diagonal back (below)
@@ -253,6 +253,7 @@ scan_kernel(const ScanArgs a, int num_seqs, int nc, int* err) {
   const int rank = nc > 1 ? static_cast<int>(cluster_ctarank()) : 0;
   const int dim = a.dim, vdim = a.vdim, hk = MODE == kDecay ? h : h / (a.heads / a.kv_heads);
   constexpr int kAll = WW * 32 + 256;
+  if (above > kShort) pdl_trigger();                                   // the launch for shorter sequences follows
   // Longest sequences first: where not all blocks fit the chip at once, the last to start have the least to do.  Three sequences
   // of 500, 1000 and 1501 tokens, 8 heads of 128 x 256 (192 blocks): 2001 tokens in a row before, 1501 now; the four scans of a
   // hybrid step take 960 us instead of 1256.  One sequence has no order to look up.
@@ -268,11 +269,12 @@ scan_kernel(const ScanArgs a, int num_seqs, int nc, int* err) {
     order[rank] = static_cast<uint8_t>(tid);
   }
   __syncthreads();
+  auto of_this = [&](int tokens) { return tokens > above && tokens <= to; };
   auto seq = [&](int z) { return sorted ? static_cast<int>(order[z]) : z; };
   {
     int mine = 0;                                                      // a sequence for this kernel among the block's
     for (int z = blockIdx.z + tid * gridDim.z; z < num_seqs; z += kAll * gridDim.z)
-      mine |= static_cast<int>(a.cu_seqlens_q[seq(z) + 1] - a.cu_seqlens_q[seq(z)]) > kShort;
+      mine |= of_this(static_cast<int>(a.cu_seqlens_q[seq(z) + 1] - a.cu_seqlens_q[seq(z)]));
     if (!__syncthreads_or(mine)) {
       pdl_wait();
       return;
@@ -294,7 +296,7 @@ scan_kernel(const ScanArgs a, int num_seqs, int nc, int* err) {
   int blocks = 0;                                                      // blocks of tokens so far, over all sequences
   for (int z = blockIdx.z; z < num_seqs; z += gridDim.z) {
     const int b = seq(z), t0 = a.cu_seqlens_q[b], t1 = a.cu_seqlens_q[b + 1], nblk = (t1 - t0 + kBT - 1) / kBT;
-    if (t1 - t0 <= kShort) continue;                                   // (scan_short_kernel)
+    if (!of_this(t1 - t0)) continue;                                   // (another launch's)
     const bool fresh = static_cast<int>(a.context_lens[b]) == t1 - t0;
     if (warp >= WW) {
       // ---------------------------------------------------------- token rows
@@ -306,7 +308,8 @@ scan_kernel(const ScanArgs a, int num_seqs, int nc, int* err) {
       // ring's places; its rows are read a turn ahead into registers.
       const int step = 2 * nc, first = (grp * nc + rank - blocks) & (step - 1);
       constexpr int TPR = DK / 4, RPS = 128 / TPR, NR = kBT / RPS;     // threads per row, rows at a time, rows of a thread
-      constexpr bool kAhead = DK <= 128;                               // (rows of 256 entries do not fit beside the triangles' operands)
+      // (rows of 256 entries do not fit beside the triangles' operands but where there are fewer threads and triangles)
+      constexpr bool kAhead = DK <= 128 || (MODE != kDelta && !CHAN && WW == 4);
       float4 raw_k[NR], raw_q[NR], raw_d[CHAN ? NR : 1];
       const int rx = pt % TPR * 4;
       auto read_rows = [&](int i) {
@@ -1018,20 +1021,28 @@ static void launch_cluster(void (*kern)(P...), dim3 grid, int threads, size_t sm
   cfg.numAttrs = na;
   cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
 }
+// Tokens of a sequence above which two, and four, neighbouring blocks of a head share what they prepare; shorter ones end before that pays for the
+// clusters' start, for a place's way around, and, of four, for the wait until as many SMs are free.  us, one / two / four blocks, heads of 128 x 128 but as
+// noted: delta rule, 16 heads, 8 x 64 tokens 65.5 / 68 / 74, 8 x 100 94.4 / 93.1 / 96.2, 64 x 200 1123 / 997 / 1134, 8 x 300 236 / 220 / 216, 1 x 2000 267 /
+// 263 / 219; decayed, 16 heads, 8 x 100 67.7 / 67.9 / 73.8, 64 x 200 804 / 714 / 839, 8 x 300 167 / 157 / 158, 1 x 2000 191 / 174 / 166; delta, a decay per
+// channel, 256 x 256, 32 x 40 330 / 304 / 350, 1 x 128 48.2 / 49.5 / 44.6.  (The bits are the same.)
+template <int DK, int MODE, bool CHAN> struct ScanShare {
+  static constexpr int kTwo = MODE != kDelta ? 112 : DK <= 128 ? 64 : 32;
+  static constexpr int kFour = MODE != kDelta ? (DK <= 128 ? 512 : 256) : CHAN && DK > 128 ? 112 : 256;
+};
+// share: 1, 2 or 4 blocks, where there are as many
 template <int DK, int MODE, bool CHAN, int WW>
-static void launch_scan_ww(const ScanArgs& a, int z, bool short_rows, int* err, cudaStream_t st_) {
+static void launch_scan_ww(const ScanArgs& a, int z, int above, int to, int share, int* err, cudaStream_t st_) {
   using SM = ScanSmem<DK, CHAN, WW>;
   auto kern = scan_kernel<DK, MODE, CHAN, WW>;
   static OncePerDevice sized;
   if (!allow_smem(sized, kern, SM::kBytes)) return;
   const int cols = (a.vdim + SM::kCols - 1) / SM::kCols;
-  // a few blocks per SM, each taking every so many sequences
-  z = std::max(1, std::min(z, 4 * sm_count() / (cols * a.heads)));
-  // Blocks of a head that share what they prepare.  Portions of a few blocks of tokens end before that pays for the clusters' start and
-  // end: delta rule, 16 heads of 128 x 128, eight sequences of 17 / 64 tokens alone 39 / 68 us, four together 47.5 / 75; 64
-  // tokens 16.6 and 18.6; 4096 tokens 538 and 440.  (The bits are the same.)
-  const int nc = short_rows || cols % 2 ? 1 : cols % 4 ? 2 : 4;
-  launch_cluster(kern, dim3(cols, a.heads, z), WW * 32 + 256, SM::kBytes, st_, nc, a, a.num_seqs, nc, err);
+  // a few blocks per SM, each taking every so many sequences; of a launch for long ones only, which may have none, one per SM (32 sequences of 40
+  // tokens, 16 heads of 128 x 128: four waves of blocks that only look took 5 of 111 us)
+  z = std::max(1, std::min(z, (above > kShort ? 1 : 4) * sm_count() / (cols * a.heads)));
+  const int nc = share == 1 || cols % 2 ? 1 : share == 2 || cols % 4 ? 2 : 4;
+  launch_cluster(kern, dim3(cols, a.heads, z), WW * 32 + 256, SM::kBytes, st_, nc, a, a.num_seqs, above, to, nc, err);
   B200_CUDA_LAUNCH_CHECK();
 }
 template <int DK, int MODE, bool CHAN>
@@ -1041,9 +1052,6 @@ static void launch_scan_dk(const ScanArgs& a, int num_tokens, cudaStream_t st_) 
     set_error(2, "scan: no host-visible memory");
     return;
   }
-  // 16 columns per block while that leaves a block per SM at most, 32 beyond: one sequence of 4096 tokens of 16 heads of
-  // 128 x 128 (128 or 64 blocks) 634 and 883 us, four of 1000 (512 or 256 blocks) 655 and 539 us
-  const bool narrow = (a.vdim + 15) / 16 * a.heads * a.num_seqs <= sm_count();
   // Which kernel walks a sequence is a matter of its own length, so that its bits do not depend on the step's other sequences.  Up to
   // kShort tokens, whatever their number, token by token is as fast or faster.  Delta rule, heads of 128 x 128, token by token and
   // in blocks: 1 sequence of 16 tokens of 16 heads 9.2 and 9.4 us, 2 10.8 and 10.1, 8 22 and 31, 32 of 12 tokens 51 and 78; of 20
@@ -1052,13 +1060,31 @@ static void launch_scan_dk(const ScanArgs& a, int num_tokens, cudaStream_t st_) 
   brief<<<dim3((a.vdim + kOneCols - 1) / kOneCols, a.heads, a.num_seqs), 128, 0, st_>>>(a);
   B200_CUDA_LAUNCH_CHECK();
   // The walk of the longer sequences starts beside it: they share what they read, and nothing that they write (a sequence of 400 tokens and
-  // 32 of 4, 16 heads of 128 x 128, a decay per channel: 105 us one after the other, 100 so; 4096 tokens of the delta rule 441 and 439).
-  // Sequences that can be longer than that: none in a step of few tokens, as of decoded ones
-  const int longer = num_tokens > 0 ? std::min(a.num_seqs, num_tokens / (kShort + 1)) : a.num_seqs;
-  if (longer == 0) return;
-  const bool short_rows = num_tokens > 0 && num_tokens <= 64 * a.num_seqs;
-  if (narrow) launch_scan_ww<DK, MODE, CHAN, 4>(a, longer, short_rows, err, st_);
-  else launch_scan_ww<DK, MODE, CHAN, 8>(a, longer, short_rows, err, st_);
+  // 32 of 4, 16 heads of 128 x 128, a decay per channel: 105 us one after the other, 100 so).  It writes before it waits for the kernel
+  // in front (at its end), so the first launch above has to stay a plain one, and nothing may come between.
+  auto walk = [&](int above, int to, int share) {
+    // sequences that can be that long: none in a step of few tokens, as of decoded ones
+    const int most = num_tokens > 0 ? std::min(a.num_seqs, num_tokens / (above + 1)) : a.num_seqs;
+    if (most == 0) return;
+    // 16 columns per block while that leaves a block per SM at most, 32 beyond: one sequence of 4096 tokens of 16 heads of
+    // 128 x 128 (128 or 64 blocks) 634 and 883 us, four of 1000 (512 or 256 blocks) 655 and 539 us
+    const bool narrow = (a.vdim + 15) / 16 * a.heads * (above > kShort ? most : a.num_seqs) <= sm_count();
+    if (narrow) launch_scan_ww<DK, MODE, CHAN, 4>(a, most, above, to, share, err, st_);
+    else launch_scan_ww<DK, MODE, CHAN, 8>(a, most, above, to, share, err, st_);
+  };
+  using Share = ScanShare<DK, MODE, CHAN>;
+  constexpr int kAny = 1 << 30;
+  const int mean = num_tokens > 0 ? num_tokens / a.num_seqs : kAny;
+  if (mean > Share::kTwo) {
+    walk(kShort, kAny, mean > Share::kFour ? 4 : 2);
+  } else if (num_tokens <= std::max(256, 4 * Share::kTwo)) {
+    walk(kShort, kAny, 1);
+  } else {
+    // Short sequences on average, among them perhaps the long portion of a prompt beside decoded tokens: each in the launch for its length.
+    // A prompt of 2000 tokens and 32 single ones, all in the form for short ones and so, us: delta rule, 16 heads of 128 x 128 372 and 344, decayed 288 and 257.
+    walk(Share::kTwo, kAny, 4);
+    walk(kShort, Share::kTwo, 1);
+  }
 }
 // dim: rows of the state; at most 256 (the caller has checked)
 template <int MODE, bool CHAN>
