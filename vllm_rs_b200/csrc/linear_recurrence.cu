@@ -587,7 +587,7 @@ scan_kernel(const ScanArgs a, int num_seqs, int above, int to, int nc, int* err)
         if (nc > 1) {                                  // to the same place of the cluster's other blocks
           fence_proxy_async();
           sync();
-          if (pw == 0 && lane < nc && lane != rank)
+          if (pw == 0 && lane < nc && lane != rank && !*fail)          // (after a wait gave up, nothing more is sent)
             asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
                              mapa_shared(smem_u32(B), lane)),
                          "r"(smem_u32(B)), "r"(SM::kBuf * 4), "r"(mapa_shared(smem_u32(&ready[g % kRing]), lane))
@@ -1057,11 +1057,12 @@ static void launch_scan_dk(const ScanArgs& a, int num_tokens, cudaStream_t st_) 
   // in blocks: 1 sequence of 16 tokens of 16 heads 9.2 and 9.4 us, 2 10.8 and 10.1, 8 22 and 31, 32 of 12 tokens 51 and 78; of 20
   // tokens 1 sequence 11.5 and 10.5, 4 18.6 and 20.8.  In a step with longer sequences its walk stood before theirs.
   auto brief = DK == 64 && a.dim <= 32 ? scan_short_kernel<DK == 64 ? 32 : DK, MODE, CHAN> : scan_short_kernel<DK, MODE, CHAN>;
+  // (a plain launch: the walks below start under it and write before they wait for it)
   brief<<<dim3((a.vdim + kOneCols - 1) / kOneCols, a.heads, a.num_seqs), 128, 0, st_>>>(a);
   B200_CUDA_LAUNCH_CHECK();
   // The walk of the longer sequences starts beside it: they share what they read, and nothing that they write (a sequence of 400 tokens and
   // 32 of 4, 16 heads of 128 x 128, a decay per channel: 105 us one after the other, 100 so).  It writes before it waits for the kernel
-  // in front (at its end), so the first launch above has to stay a plain one, and nothing may come between.
+  // in front, at its end, which is only right behind a plain launch, or another of its own kind, that has begun after all earlier ones ended.
   auto walk = [&](int above, int to, int share) {
     // sequences that can be that long: none in a step of few tokens, as of decoded ones
     const int most = num_tokens > 0 ? std::min(a.num_seqs, num_tokens / (above + 1)) : a.num_seqs;
