@@ -235,8 +235,8 @@ __device__ __forceinline__ bool wait_cluster(uint64_t* bar, uint32_t parity, vol
 // Bound: the chain of blocks, one walk after another; a walk's 78 shuffles (6.3 cycles each from one warp of a scheduler), its 16-byte loads
 // (12) and its packed FMAs (2.7) overlap in part.  HBM and the FMA units would take 16 and 89 us for 4096 tokens of 16 heads of
 // 128 x 128.  Measured there, token by token (eight lanes per column, four chained shuffles per token) -> in blocks -> prepared in turns,
-// and sums that meet without selections (meet32_turned: 510 -> 440): delta rule 2278 -> 597 -> 440 us; decayed state of 8 heads of
-// 128 x 256: 909 -> 398 -> 334 us.  Two columns per warp and twice the warps: slower (shared memory's loads per column double).  The
+// and sums that meet without selections (meet32_turned: 510 -> 440): delta rule 2278 -> 597 -> 445 us; decayed state of 8 heads of
+// 128 x 256: 909 -> 398 -> 337 us.  Two columns per warp and twice the warps: slower (shared memory's loads per column double).  The
 // state's update does not wait for the read-out's sums: the queries' products are taken before the correction's sums meet, and
 // meet under the update (665 and 424 us with both in turn).
 template <int DK, int MODE, bool CHAN, int WW>
@@ -1061,7 +1061,7 @@ static void launch_scan_dk(const ScanArgs& a, int num_tokens, cudaStream_t st_) 
   brief<<<dim3((a.vdim + kOneCols - 1) / kOneCols, a.heads, a.num_seqs), 128, 0, st_>>>(a);
   B200_CUDA_LAUNCH_CHECK();
   // The walk of the longer sequences starts beside it: they share what they read, and nothing that they write (a sequence of 400 tokens and
-  // 32 of 4, 16 heads of 128 x 128, a decay per channel: 105 us one after the other, 100 so).  It writes before it waits for the kernel
+  // 32 of 4, 16 heads of 128 x 128, a decay per channel: 101.5 so; 105 one after the other).  It writes before it waits for the kernel
   // in front, at its end, which is only right behind a plain launch, or another of its own kind, that has begun after all earlier ones ended.
   auto walk = [&](int above, int to, int share) {
     // sequences that can be that long: none in a step of few tokens, as of decoded ones

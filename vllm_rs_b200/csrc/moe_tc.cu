@@ -11,10 +11,10 @@
 // gathers of four rows (~90 cycles each) as by cp.async, whose blocks need a wait and a fence on their way to the tensor core
 // (prompt of 4096 rows, 16 experts, first product: 183 us and 103-139 us).  Two blocks of a cluster may share a tile of 256 slots, each
 // with its own rows and half of the weight rows in shared memory: two thirds of the reads (that prompt's products 71 / 52 -> 66 / 52 us).
-// All launches of a call depend on each other as programs, so that the next one's start lies under the last one's end: 40 rows 56 -> 49 us,
-// 4096 rows 181 -> 176.
+// The launches of a call, but for the sum of the choices, depend on each other as programs, so that the next one's start lies under
+// the last one's end.  Replayed as a graph, without pairs and dependent launches and with both: 40 rows 41.5 -> 33.8 us, 4096 rows 172 -> 158.5.
 //
-// Measured, mma.sync kernel -> here (whole call): 4096 rows of 2048, 16 experts of 512, 4 chosen: 709 -> 194 us, 32 rows, device time,
+// Measured, mma.sync kernel -> here (whole public call): 4096 rows of 2048, 16 experts of 512, 4 chosen: 709 -> 183 us, 32 rows, device time,
 // 67 -> 36; 4096 wide, 32 experts of 1024: 3000 rows 1903 -> 406 us, 32 rows, device time, 202 -> 159.  moe.cu says which products are
 // long enough to come here.
 // Bound: tensor cores where experts get hundreds of rows, HBM (every hit expert's weights once) where they get few; BN is 256
@@ -372,9 +372,9 @@ static void launch_bn(void* out, const void* a, const void* w, const int32_t* of
   constexpr int G = ACT == 1 || ACT == 3 ? 2 : 1;
   const int row_tiles = std::max(std::min(E, pairs), pairs / kM);
   // Pairs of blocks where their tiles, twice as high, do not cost more turns: a pair's turn takes 0.8 - 0.9 of a block's (first product
-  // of the prompt above 73 000 and 93 000 cycles for four, second 60 000 and 66 000 for eight).  Whole calls, single blocks and pairs, us:
-  // 4096 rows of 2048, 16 experts of 512: 185 and 181, 8192 rows 329 and 314, 2048 rows 110 and 114 (two turns and three); 64
-  // experts of 1024, 8 chosen of 4096 rows 503 and 487; 4096 wide, 32 experts of 1024: 3000 rows 386 and 382, 300 rows 189 and 193.
+  // of the prompt above 73 000 and 93 000 cycles for four, second 60 000 and 66 000 for eight).  Calls replayed
+  // as a graph, single blocks and pairs, us: 16 experts of 512, 2048 wide, 2000 rows 95.4 and 99.1 (two turns and three), 2500 rows 121 and 116, 4096
+  // rows 174 and 165, 8000 rows 302 and 299; 64 experts of 1024, 8 chosen, 2500 rows 363 and 338, 4096 rows 516 and 497.
   const auto turns = [&](int rows, int slots) {            // half a tile of every bucket is past its end
     const double tiles = std::max<double>(std::min(E, pairs), E * 0.5 + static_cast<double>(pairs) / rows) * ((N * G + 255) / 256);
     return std::ceil(tiles / slots);

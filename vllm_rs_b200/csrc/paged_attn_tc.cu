@@ -17,16 +17,16 @@
 // Warp 0 fetches pages by block-table index (TMA, K ring | V ring), warp 1 issues the MMAs (S of page j + 1 before P V of
 // page j), warps 2-9 own the rows: two warps share 32 of them, exchange their halves' maxima in shared memory at a barrier of the
 // two, and rescale and write half of the columns each.  (One thread per row has a page's 64 scores in one chain of waits: 98 / 62 / 680
-// us for the three cases below where two take 90 / 58 / 577.  More warps also stage the queries faster.)  Latent rows (kv_rank 512: O would need all 512 TMEM columns) are walked in passes of up to
+// us for the three cases below, in turn with others, where two took 90 / 58 / 577.  More warps also stage the queries faster.)  Latent rows (kv_rank 512: O would need all 512 TMEM columns) are walked in passes of up to
 // 256 value columns; the scores are computed again in every pass (1.5x the products, still far from the 8 mma.sync
 // warps' rate that made 128-row tiles of 16 rows x 1 head re-read every page 64 times).  In a pass the page blocks that are
 // also values stay until P V has read them (V ring), the rest is released after S (K ring).
 //
 // Bound: tensor cores for prompts (per page 2 * 128 * 64 * (dim * passes + vdim) flop against 64 * dim * 2 bytes from L2),
 // HBM for steps of few rows, whose keys are split over blocks; window_attn_merge / latent_attn_merge then finish.
-// Measured, this kernel alone (whole calls in turn with others: 88, 557 and 57.5 us), mma.sync kernels -> here: window 1024, 4096 rows, 16 heads of 128 over 4: 622 -> 85 us (352 TFLOP/s; what bounds it
-// is the softmax warps, then the start and the drain of 128 blocks); latent, 2 x 2048 rows, 32 heads, rank 512:
-// 7766 -> 512 us (584 TFLOP/s useful, 885 issued); 32 tokens over 2048 keys, 32 heads over 8: 317 -> 58 us (35 at HBM rate): 256 blocks
+// Measured, whole calls in turn with others, mma.sync kernels -> here: window 1024, 4096 rows, 16 heads of 128 over 4: 622 -> 88 us
+// (340 TFLOP/s; what bounds it is the softmax warps, then the start and the drain of 128 blocks); latent, 2 x 2048 rows, 32 heads, rank 512:
+// 7766 -> 561 us (533 TFLOP/s useful, 810 issued); 32 tokens over 2048 keys, 32 heads over 8: 317 -> 57.6 us (35 at HBM rate): 256 blocks
 // of 33 pages in turn, with four rows in one pair of the row warps.
 #include "paged_attn_tc.cuh"
 #include "f32x2.cuh"
@@ -398,7 +398,8 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__
     const int tid = threadIdx.x - 64;
     const uint32_t lane_base = static_cast<uint32_t>(q4 * 32) << 16;
     // ---- stage Q as bf16: coalesced 32-byte reads, chunks of 8 entries (128 rows of 544: 26 000 cycles with divisions and 64-bit
-    // addresses per chunk and 16-byte loads, 17 000 without; latent prompt 549 -> 512 us)
+    // addresses per chunk and 16-byte loads, 17 000 without; latent prompt 580 -> 561 us, with the issue
+    // behind elect.sync)
     {
       const int cpr = p.dim / 8;
       const int dr = kRowThreads / cpr, dc = kRowThreads % cpr;          // what 256 chunks on are: dr rows and dc chunks

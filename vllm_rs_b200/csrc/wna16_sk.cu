@@ -1014,6 +1014,8 @@ static int skm_mode() {
 
 // Decode-shape entry (M <= 32): false when the shape needs another kernel.  `force` skips the B200_DEC_SK switch
 // (b200_wna16_gemm_ex variant 5, the bf16 entry points).
+// By itself it comes after wna16_ts.cu and wna16_mma.cu: up to 16 tokens and from 32 units per SM on, 8-bit products of K <= 2048, and
+// 4-bit ones whose scales or zero points lie off 16 bytes.
 bool launch_wna16_sk(const WnaParams& p, cudaStream_t st, bool force, bool bf16, int flavour) {
   if (!force && sk::sk_mode() == 0) return false;
   if (p.M > 32) return false;
