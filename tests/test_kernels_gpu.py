@@ -558,6 +558,24 @@ def test_wna16_units_push_to_peers(ops, K, N, M):
     assert int(ws[:16384].view(torch.int32).abs().sum()) == 0
 
 
+def test_wna16_streamk_switch():
+    """B200_DEC_SK=1 gives the stream-K kernel every product of up to 32 tokens that it takes, before all others (read once per process)."""
+    import os
+    import subprocess
+    import sys
+    program = """
+import test_kernels_gpu as t
+from vllm_rs_b200 import ops
+for fmt, bits, M in (("awq", 4, 3), ("awq", 4, 16), ("awq", 4, 32), ("gptq", 8, 1), ("gptq", 8, 32)):
+    call, _, _ = t._wna_run(ops, fmt, bits, 2048, 1536, M, 128, "none", M)
+    assert t.torch.equal(call(0), call(5)), (bits, M)
+print("equal")
+"""
+    env = dict(os.environ, B200_DEC_SK="1", PYTHONPATH=os.pathsep.join([os.path.dirname(os.path.abspath(__file__))] + sys.path))
+    r = subprocess.run([sys.executable, "-c", program], env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "equal" in r.stdout, r.stdout[-2000:] + r.stderr[-2000:]
+
+
 @pytest.mark.parametrize("K,N,M,group", [(4096, 9728, 17, 64), (8192, 9728, 33, 64), (8192, 1280, 64, 128)])
 def test_wna16_decode_of_many_groups(ops, K, N, M, group):
     """wna16_tc_dec.cu where one K piece has exactly as many quantisation groups as are staged, and where it takes more pieces."""

@@ -502,6 +502,7 @@ int wna16_tc_dec_turn(const WnaParams& p);                       // chunks of it
 bool wna16_mma_takes(const WnaParams& p, bool force = false);
 bool launch_wna16_mma(const WnaParams& p, cudaStream_t st, bool force = false);      // 4-bit decode shapes (M <= 16)
 bool launch_wna16_ts(const WnaParams& p, cudaStream_t st, bool force = false);       // decode shapes (M <= 64), units cut evenly over the SMs
+bool wna16_sk_first();
 // stream-K decode kernel (M <= 32); bf16: A, scales and C are bf16 (plain epilogue, 4-bit only)
 bool launch_wna16_sk(const WnaParams& p, cudaStream_t st, bool force = false, bool bf16 = false, int flavour = -1);
 // Largest M the automatic dispatch still gives to the flat GEMV (env B200_GEMV_MAX_M, default 0: the tcgen05

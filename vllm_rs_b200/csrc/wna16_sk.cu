@@ -1012,6 +1012,9 @@ static int skm_mode() {
 
 }  // namespace sk
 
+// B200_DEC_SK=1: before every other kernel
+bool wna16_sk_first() { return sk::sk_mode() == 1; }
+
 // Decode-shape entry (M <= 32): false when the shape needs another kernel.  `force` skips the B200_DEC_SK switch
 // (b200_wna16_gemm_ex variant 5, the bf16 entry points).
 // By itself it comes after wna16_ts.cu and wna16_mma.cu: up to 16 tokens and from 32 units per SM on, 8-bit products of K <= 2048, and

@@ -787,7 +787,7 @@ static bool launch_nt(const WnaParams& p, cudaStream_t st, bool force) {
 bool launch_wna16_ts(const WnaParams& p, cudaStream_t st, bool force) {
   if (p.M > (p.bits == 4 ? 64 : 32) || p.K % ts::kUnitK != 0 || p.N % kTileN != 0 || p.no_split) return false;
   const int64_t tiles = p.N / kTileN, U = p.K / ts::kUnitK;
-  if (!force && ((p.bits == 4 && p.M <= 8) || (U <= 16 && tiles * U >= 4096))) return false;
+  if (!force && ((p.bits == 4 && p.M <= 8) || (U <= 16 && tiles * U >= 4096) || (p.M <= 32 && wna16_sk_first()))) return false;
   if (p.group_size < p.K) {                  // a unit lies in one group, whose index is a shift of the unit's
     bool ok = false;
     for (int s = 0; s < 24; ++s) ok = ok || (ts::kUnitK << s) == p.group_size;
