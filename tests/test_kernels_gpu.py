@@ -558,6 +558,27 @@ def test_wna16_units_push_to_peers(ops, K, N, M):
     assert int(ws[:16384].view(torch.int32).abs().sum()) == 0
 
 
+@pytest.mark.parametrize("variant,bits,K,N,M,epi", [(9, 8, 4096, 28672, 48, "silu"), (9, 8, 14336, 4096, 64, "none"), (9, 4, 4096, 28672, 64, "none"),
+                                                    (4, 8, 4096, 8192, 64, "none"), (4, 4, 8192, 4096, 200, "none"),
+                                                    (5, 8, 4096, 28672, 16, "silu"), (5, 4, 14336, 4096, 32, "none"), (6, 4, 8192, 8192, 16, "none")])
+def test_wna16_rings_repeat_themselves(ops, variant, bits, K, N, M, epi):
+    """The same bits from 400 calls of the kernels whose warps read packed weights from a ring of copies, weights cold and not."""
+    g = torch.Generator(device="cuda").manual_seed(M)
+    words = lambda n: torch.randint(-2 ** 31, 2 ** 31, (n,), generator=g, device="cuda", dtype=torch.int64).int()      # noqa: E731
+    packed, qz = words(K * N * bits // 32), words(K // 128 * N * bits // 32).view(K // 128, -1)
+    s = (0.005 + 0.01 * torch.rand(K // 128, N, generator=g, device="cuda")).to(F16) / 2 ** (bits - 4)
+    x = (0.05 * torch.randn(M, K, generator=g, device="cuda")).to(F16)
+    ws, cold = ops.wna16_workspace(M, N), torch.empty(64 << 20, device="cuda")
+    kw = dict(k=K, n=N, bits=bits, qfmt=ops.QFMT_AWQ if bits == 4 else ops.QFMT_GPTQ, variant=variant,
+              epilogue=ops.EPI_SILU_MUL if epi == "silu" else ops.EPI_NONE)
+    first, differ = ops.wna16_gemm(x, packed, s, qz, ws, **kw), torch.zeros((), dtype=torch.int64, device="cuda")
+    for i in range(400):
+        if i % 8 == 0:
+            cold.zero_()
+        differ += (ops.wna16_gemm(x, packed, s, qz, ws, **kw).view(torch.int16) != first.view(torch.int16)).any()
+    assert int(differ) == 0
+
+
 def test_wna16_streamk_switch():
     """B200_DEC_SK=1 gives the stream-K kernel every product of up to 32 tokens that it takes, before all others (read once per process)."""
     import os

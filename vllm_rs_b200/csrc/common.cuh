@@ -198,6 +198,12 @@ __device__ __forceinline__ void fence_barrier_init() {
 __device__ __forceinline__ void fence_proxy_async() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
+// Before a warp gives back a place that bulk copies overwrite: what it has asked for there, through the generic proxy, has arrived.  An
+// arrival alone does not wait for reads that are still on their way, nor order them before another proxy's writes.
+__device__ __forceinline__ void reads_done() {
+  __threadfence_block();
+  fence_proxy_async();
+}
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }

@@ -462,8 +462,7 @@ wna16_mma_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
           // The last read of the unit's place.  What was read has to be there before the copies of a later unit may be asked for, and
           // these write by another proxy: without the two fences one warp in some 10^7 read the last activations after them (seen
           // at 9 - 16 tokens, 34944 x 30848: one call in 100).  They cost nothing: four projections, one token 47.1 -> 46.7 us.
-          __threadfence_block();
-          fence_proxy_async();
+          reads_done();
           __syncwarp();
           if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(empty + st * 8) : "memory");
         }

@@ -687,6 +687,7 @@ wna16_sk_kernel(const __grid_constant__ CUtensorMap xmap, const Args a) {
               }
           }
         }
+        reads_done();
         __syncwarp();
         if (lane0) {
           arrive_bar(s_wempty + wslot * 8);              // this warp's part of the stage has been consumed
@@ -861,6 +862,7 @@ wna16_sk_kernel(const __grid_constant__ CUtensorMap xmap, const Args a) {
           if (cc == 0) {
             load_chunk(cur, wslot, 1);
           } else {
+            reads_done();
             __syncwarp();
             if (lane0) arrive_bar(s_wempty + wslot * 8);   // this warp's quarter of the stage is in registers
             if (++wslot == C::kSWS) { wslot = 0; wphase ^= 1; }

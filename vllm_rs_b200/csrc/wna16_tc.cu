@@ -166,6 +166,7 @@ wna16_tc_kernel(const __grid_constant__ CUtensorMap xmap, const TcArgs a) {
         asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
                      : "=r"(dst[sub * 4]), "=r"(dst[sub * 4 + 1]), "=r"(dst[sub * 4 + 2]), "=r"(dst[sub * 4 + 3])
                      : "r"(addr + sub * kTileN * 16));
+      reads_done();
       __syncwarp();
       if (lane == 0) mbar_arrive(&wempty[sw]);        // packed bytes are in registers
     };

@@ -274,6 +274,7 @@ wna16_tc_dec_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_const
         asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
                      : "=r"(dst[sub * 4]), "=r"(dst[sub * 4 + 1]), "=r"(dst[sub * 4 + 2]), "=r"(dst[sub * 4 + 3])
                      : "r"(addr + sub * kTileN * 16));
+      reads_done();
       __syncwarp();
       if (lane == 0) bar_arrive(s_wempty + ss * 8);   // packed bytes are in registers
       if (++ss == C::kSWS) { ss = 0; ss_phase ^= 1; }
@@ -418,6 +419,7 @@ wna16_tc_dec_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_const
               asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
                            : "=r"(cur[sub * 4]), "=r"(cur[sub * 4 + 1]), "=r"(cur[sub * 4 + 2]), "=r"(cur[sub * 4 + 3])
                            : "r"(s_wq + ssn * C::kWSBytes + sub * kTileN * 16));
+            reads_done();
             __syncwarp();
             if (lane0) bar_arrive(s_wempty + ssn * 8);
           }
