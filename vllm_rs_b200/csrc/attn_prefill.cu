@@ -248,6 +248,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_const
         }
       }
     }
+    reads_done();
     __syncwarp();
     if (lane == 0) mbar_arrive(&empty_bar[s]);
   }

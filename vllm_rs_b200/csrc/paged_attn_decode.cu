@@ -358,6 +358,7 @@ paged_attn_decode_body(const CUtensorMap& kmap, const CUtensorMap& vmap,
             }
           }
         }
+        reads_done();
         __syncwarp();
         if (lane == 0) {
 #pragma unroll
@@ -453,6 +454,7 @@ paged_attn_decode_body(const CUtensorMap& kmap, const CUtensorMap& vmap,
           mma_16816_t<BF>(o_acc[2 * jj + 1], pa, r[2], r[3]);
         }
       }
+      reads_done();
       __syncwarp();
       if (lane == 0) mbar_arrive(&empty_bar[s]);
     }
